@@ -10,8 +10,8 @@
 // totals to the policy.
 //
 // Used where a three-launch partition over n items (histogram, one-block scan,
-// scatter) was spending most of its time in launch gaps: run heads of a sorted
-// batch, their per-class numbering, the list of cache misses of a batch.
+// scatter) was spending most of its time in launch gaps: the list of cache misses
+// of a batch.
 #pragma once
 
 #include "launch.cuh"
@@ -68,37 +68,14 @@ __device__ __forceinline__ void bump4(int4& c, int cls) {
   c.w += cls == 3;
 }
 
-// The classes of a thread's 8 consecutive items.  A policy may bring its own
-// classify8(base, n, cls) (e.g. vector loads of the 8 keys); otherwise classify(i) is asked
-// item by item.
-template <typename Policy>
-__device__ __forceinline__ auto classify_items(const Policy& pol, int64_t base, int64_t n, int* cls, int)
-    -> decltype(pol.classify8(base, n, cls), void()) {
-  pol.classify8(base, n, cls);
-}
-template <typename Policy>
-__device__ __forceinline__ void classify_items(const Policy& pol, int64_t base, int64_t n, int* cls, long) {
-#pragma unroll
-  for (int k = 0; k < kCompItems; ++k) cls[k] = base + k < n ? pol.classify(base + k) : -1;
-}
-
-// A policy may ask for the number of kept items ahead of every thread's 8 items
-// (thread_begin(base, before)), e.g. to leave a coarse index of the compaction behind.
-template <typename Policy>
-__device__ __forceinline__ auto thread_begin_hook(const Policy& pol, int64_t base, const int4& before, int)
-    -> decltype(pol.thread_begin(base, before), void()) {
-  pol.thread_begin(base, before);
-}
-template <typename Policy>
-__device__ __forceinline__ void thread_begin_hook(const Policy&, int64_t, const int4&, long) {}
-
 template <typename Policy>
 __global__ void __launch_bounds__(kCompBlock) compact_count_kernel(Policy pol, CompactPlan p) {
   __shared__ int4 s_warp[kCompBlock / 32];
   const int64_t base = (int64_t)blockIdx.x * kCompTile + (int64_t)threadIdx.x * kCompItems;
   int4 c = make_int4(0, 0, 0, 0);
   int cls[kCompItems];
-  classify_items(pol, base, p.n, cls, 0);
+#pragma unroll
+  for (int k = 0; k < kCompItems; ++k) cls[k] = base + k < p.n ? pol.classify(base + k) : -1;
 #pragma unroll
   for (int k = 0; k < kCompItems; ++k) bump4(c, cls[k]);
   const int4 t = block_sum4(c, s_warp);
@@ -162,7 +139,8 @@ __global__ void __launch_bounds__(kCompBlock) compact_scatter_kernel(Policy pol,
   const int64_t base = tile * kCompTile + (int64_t)threadIdx.x * kCompItems;
   int cls[kCompItems];
   int4 mine = make_int4(0, 0, 0, 0);
-  classify_items(pol, base, p.n, cls, 0);
+#pragma unroll
+  for (int k = 0; k < kCompItems; ++k) cls[k] = base + k < p.n ? pol.classify(base + k) : -1;
 #pragma unroll
   for (int k = 0; k < kCompItems; ++k) bump4(mine, cls[k]);
   // exclusive scan of the per-thread counts over the block
@@ -184,7 +162,6 @@ __global__ void __launch_bounds__(kCompBlock) compact_scatter_kernel(Policy pol,
     run.x += x.x; run.y += x.y; run.z += x.z; run.w += x.w;
   }
   run.x += inc.x - mine.x; run.y += inc.y - mine.y; run.z += inc.z - mine.z; run.w += inc.w - mine.w;
-  if (base < p.n) thread_begin_hook(pol, base, run, 0);
 #pragma unroll
   for (int k = 0; k < kCompItems; ++k) {
     if (cls[k] >= 0) {

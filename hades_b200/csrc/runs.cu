@@ -12,13 +12,12 @@
 //                           the batch position whose output row holds their embedding
 //                           (the uncached cold ids sent to the server, dist_emb.py:218-259)
 // The backward aggregation (segsum.cu) and the LRU ageing (index.cu) take the same runs.
-#include <cub/device/device_radix_sort.cuh>
-
 #include "a2a.cuh"
 #include "compact.cuh"
 #include "index.cuh"
 #include "runs.cuh"
 #include "shard.cuh"
+#include "sortcore.cuh"
 
 namespace hb {
 int* device_error_word();  // runtime.cu
@@ -27,58 +26,42 @@ namespace {
 
 constexpr int kBlock = 256;
 
-size_t sort_temp_bytes(int64_t n) {
-  size_t b64 = 0, b32 = 0;
-  cub::DoubleBuffer<int64_t> k(nullptr, nullptr);
-  cub::DoubleBuffer<uint32_t> k32(nullptr, nullptr);
-  cub::DoubleBuffer<uint32_t> v(nullptr, nullptr);
-  cub::DeviceRadixSort::SortPairs(nullptr, b64, k, v, (int)n, 0, 64, (cudaStream_t)0);
-  cub::DeviceRadixSort::SortPairs(nullptr, b32, k32, v, (int)n, 0, 32, (cudaStream_t)0);
-  return b64 > b32 ? b64 : b32;
-}
-
-// number of valid entries of a segmented input = sum of the segment counts
-__global__ void sum_counts_kernel(const int64_t* __restrict__ seg_counts, int64_t num_segs,
-                                  int64_t seg_cap, int64_t* __restrict__ out) {
-  if (threadIdx.x || blockIdx.x) return;
-  int64_t t = 0;
-  for (int64_t k = 0; k < num_segs; ++k) {
-    const int64_t c = seg_counts[k];
-    t += c < 0 ? 0 : (c > seg_cap ? seg_cap : c);
-  }
-  *out = t;
-}
-
-// keys = ids (entries at and beyond the device count, or beyond their segment's count, get
-// the largest key of id_bits bits, so they sort last), perm = 0..n-1.  A valid id that does
-// not fit below that key raises HB_ERR_INVALID in the device status word: it would collide
-// with another id or with the padding.
-template <typename KeyT>
-__global__ void prepare_keys_kernel(const int64_t* __restrict__ ids, int64_t n,
-                                    const int64_t* __restrict__ n_dev,
-                                    const int64_t* __restrict__ seg_counts, int64_t seg_cap,
-                                    int64_t sentinel, KeyT* __restrict__ keys,
-                                    uint32_t* __restrict__ perm, int* __restrict__ err) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const bool keep = seg_counts ? (i % seg_cap) < seg_counts[i / seg_cap] : (!n_dev || i < *n_dev);
-  int64_t id = keep ? ids[i] : sentinel;
-  if (keep && (id < 0 || id >= sentinel)) {
-    atomicExch(err, HB_ERR_INVALID);
-    id = sentinel;
-  }
-  keys[i] = (KeyT)id;
-  perm[i] = (uint32_t)i;
-}
-
-// run heads of the sorted keys, numbered over all runs and inside their class
-template <typename KeyT>
-struct HeadPolicy {
-  const KeyT* keys;
-  const int64_t* n_dev;
+// The ids of a batch as sort keys.  Entries at and beyond the device count are left out; entries
+// beyond their segment's count sort last.  So does a valid id that is negative or does not fit below
+// `sentinel` (2^id_bits - 1): it raises HB_ERR_INVALID in the device status word.
+struct IdSource {
+  const int64_t* ids;
   int64_t n;
+  const int64_t* n_dev;
+  const int64_t* seg_counts;
+  uint32_t seg_cap;
+  int64_t sentinel;
+  int* err;
+  __device__ __forceinline__ int64_t count() const {
+    if (!n_dev) return n;
+    const int64_t d = *n_dev;
+    return d < n ? (d > 0 ? d : 0) : n;
+  }
+  __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
+    if (seg_counts) {
+      const uint32_t seg = (uint32_t)i / seg_cap;
+      if ((int64_t)((uint32_t)i - seg * seg_cap) >= seg_counts[seg]) return false;
+    }
+    const int64_t id = __ldg(ids + i);
+    if (id < 0 || id >= sentinel) {
+      atomicExch(err, HB_ERR_INVALID);
+      return false;
+    }
+    key = (unsigned long long)id;
+    return true;
+  }
+};
+
+// Runs of equal ids in the sorted order, numbered over all runs and inside the class of their id.
+struct RunsFinish {
   const int8_t* table;   // nullable: no classes
   int64_t table_len;
+  uint32_t* perm;        // [n]
   uint8_t* head;
   int64_t* uniq;
   int64_t* uniq2;        // nullable second copy (the caller's buffer)
@@ -91,81 +74,214 @@ struct HeadPolicy {
   int64_t* class_counts;
   int64_t* class_counts2;
   int32_t* base8;        // [ceil(n / 8)] runs that start before entry 8k
-  __device__ __forceinline__ void thread_begin(int64_t base, const int4& before) const {
-    base8[base >> 3] = before.x + before.y + before.z + before.w;
-  }
-  __device__ __forceinline__ int64_t valid_entries() const {
-    if (!n_dev) return n;
-    const int64_t d = *n_dev;
-    return d < n ? (d > 0 ? d : 0) : n;
-  }
-  __device__ __forceinline__ int classify(int64_t i) const {
-    const bool is_head = i < valid_entries() && (i == 0 || __ldg(keys + i - 1) != __ldg(keys + i));
-    head[i] = is_head;
-    if (!is_head) return -1;
-    if (!table) return 0;
-    const int64_t id = (int64_t)__ldg(keys + i);
-    if (id >= table_len) return 3;
-    const int8_t v = __ldg(table + id);
-    return (v >= 0 && v <= 2) ? (int)v : 3;
-  }
-  // the 8 items of a thread at once: their keys come in two 16-byte loads (32-bit keys) and
-  // the head flags leave in one 8-byte store
-  __device__ __forceinline__ void classify8(int64_t base, int64_t n_items, int* cls) const {
-    const int64_t ne = valid_entries();
-    if (base + 8 > n_items || sizeof(KeyT) != 4) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) cls[k] = base + k < n_items ? classify(base + k) : -1;
-      return;
+  int64_t* n_valid;      // number of valid entries of a segmented input
+
+  template <class Ctx>
+  __device__ __forceinline__ void run(Ctx& ctx, const IdSource& src) const {
+    constexpr int T = Ctx::kThreads, W = T / 32;
+    __shared__ int4 s_sum[2 * W + 1];
+    __shared__ unsigned long long s_valid;
+    const int lane = threadIdx.x & 31;
+    int ne = ctx.count;
+    if (src.seg_counts) {
+      // valid entries are scattered over the segments; their number becomes the device count
+      if (threadIdx.x == 0) s_valid = 0ull;
+      __syncthreads();
+      unsigned long long t = 0;
+      for (int64_t k = threadIdx.x; k < src.n / src.seg_cap; k += T) {
+        const int64_t c = src.seg_counts[k];
+        t += (unsigned long long)(c < 0 ? 0 : (c > (int64_t)src.seg_cap ? (int64_t)src.seg_cap : c));
+      }
+      if (t) atomicAdd(&s_valid, t);
+      __syncthreads();
+      ne = (int)s_valid;
+      if (ctx.rank == 0 && threadIdx.x == 0) *n_valid = ne;
     }
-    uint32_t key[9];
-    key[0] = base > 0 ? (uint32_t)__ldg(keys + base - 1) : 0u;
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(keys + base));
-    const uint4 b = __ldg(reinterpret_cast<const uint4*>(keys + base) + 1);
-    key[1] = a.x; key[2] = a.y; key[3] = a.z; key[4] = a.w;
-    key[5] = b.x; key[6] = b.y; key[7] = b.z; key[8] = b.w;
-    unsigned long long flags = 0ull;
+    const int begin = ctx.chunk_begin(), end = ctx.chunk_end();
+    // id of an entry of the narrow kind (entries that sort last: the sentinel)
+    auto narrow_id = [&](uint32_t key) -> int64_t {
+      return key == kSortNone && ctx.none ? src.sentinel : (int64_t)key;
+    };
+    auto wide_id = [&](uint32_t pos) -> int64_t {
+      unsigned long long key;
+      return src.load(pos, key) ? (int64_t)key : src.sentinel;
+    };
+    // A thread takes 8 consecutive entries (whole vectors of positions and head flags to
+    // write, one entry of base8, no votes), the CTA 8 * T in a strip.
+    uint32_t code = 0u;  // per entry 3 bits: 4 | class (3: none) where a run starts, else 0
+    auto classify = [&](int j0, bool write) -> int4 {
+      int4 c = make_int4(0, 0, 0, 0);
+      code = 0u;
+      uint2 e[8];
+      e[7] = make_uint2(0u, 0u);
+      if (j0 < end) ctx.get8(j0, e);
+      uint32_t before = __shfl_up_sync(0xffffffffu, e[7].x, 1);
+      if (j0 >= end) return c;
+      if (lane == 0 && j0 > 0) before = ctx.get(j0 - 1).x;
+      unsigned heads = 0u;
+      if (!ctx.wide) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int64_t i = base + k;
-      const bool is_head = i < ne && (i == 0 || key[k] != key[k + 1]);
-      flags |= (unsigned long long)is_head << (8 * k);
-      int c = -1;
-      if (is_head) {
-        c = 0;
-        if (table) {
-          const int64_t id = (int64_t)key[k + 1];
-          c = 3;
-          if (id < table_len) {
-            const int8_t v = __ldg(table + id);
-            if (v >= 0 && v <= 2) c = (int)v;
-          }
+        for (int x = 0; x < 8; ++x) {
+          heads |= (unsigned)(j0 + x < ne && (j0 + x == 0 || e[x].x != before)) << x;
+          before = e[x].x;
+        }
+      } else {
+        int64_t was = j0 > 0 ? wide_id(ctx.get(j0 - 1).y) : -1;
+#pragma unroll 1
+        for (int x = 0; x < 8 && j0 + x < end; ++x) {
+          const int64_t id = wide_id(ctx.get(j0 + x).y);
+          heads |= (unsigned)(j0 + x < ne && id != was) << x;
+          was = id;
         }
       }
-      cls[k] = c;
+      if (write) {
+        if (j0 + 8 <= end) {
+          uint4* p = reinterpret_cast<uint4*>(perm + j0);
+          p[0] = make_uint4(e[0].y, e[1].y, e[2].y, e[3].y);
+          p[1] = make_uint4(e[4].y, e[5].y, e[6].y, e[7].y);
+        } else {
+#pragma unroll
+          for (int x = 0; x < 8; ++x)
+            if (j0 + x < end) perm[j0 + x] = e[x].y;
+        }
+        // one byte per entry (the allocation holds whole groups of 8)
+        const uint32_t lo = (heads & 1u) | ((heads & 2u) << 7) | ((heads & 4u) << 14) | ((heads & 8u) << 21);
+        const uint32_t h4 = heads >> 4;
+        const uint32_t hi = (h4 & 1u) | ((h4 & 2u) << 7) | ((h4 & 4u) << 14) | ((h4 & 8u) << 21);
+        *reinterpret_cast<uint2*>(head + j0) = make_uint2(lo, hi);
+      }
+      if (!table) {
+#pragma unroll
+        for (int x = 0; x < 8; ++x) code |= ((heads >> x) & 1u) << (3 * x + 2);
+        c.x = __popc(heads);
+        return c;
+      }
+      int8_t cls[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        cls[x] = 3;
+        if ((heads >> x) & 1u) {
+          const int64_t id = ctx.wide ? wide_id(e[x].y) : narrow_id(e[x].x);
+          if (id < table_len) cls[x] = __ldg(table + id);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        if (!((heads >> x) & 1u)) continue;
+        const int k = cls[x] >= 0 && cls[x] <= 2 ? cls[x] : 3;
+        code |= (4u | k) << (3 * x);
+        c.x += k == 0;
+        c.y += k == 1;
+        c.z += k == 2;
+        c.w += k == 3;
+      }
+      return c;
+    };
+    // a thread's counts -> those of the threads ahead in its warp and of the whole warp
+    auto scan_warp = [&](const int4& c, int4& total) -> int4 {
+      const unsigned long long v = (unsigned long long)(uint32_t)(c.x | (c.y << 16)) | ((unsigned long long)(uint32_t)(c.z | (c.w << 16)) << 32);
+      unsigned long long inc = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+      }
+      const unsigned long long t = __shfl_sync(0xffffffffu, inc, 31);
+      total = make_int4((int)(t & 0xffff), (int)((t >> 16) & 0xffff), (int)((t >> 32) & 0xffff), (int)(t >> 48));
+      inc -= v;
+      return make_int4((int)(inc & 0xffff), (int)((inc >> 16) & 0xffff), (int)((inc >> 32) & 0xffff), (int)(inc >> 48));
+    };
+    uint32_t kept = 0u;  // the codes of the first of two strips
+    const int strips = (end - begin + 8 * T - 1) / (8 * T);
+    int4 mine = make_int4(0, 0, 0, 0), lanes = mine, warps, cta, ahead, all;
+#pragma unroll 1
+    for (int q = 0; q < strips; ++q) {
+      const int4 c = classify(begin + q * (8 * T) + threadIdx.x * 8, true);
+      int4 total;
+      lanes = scan_warp(c, total);
+      mine.x += total.x; mine.y += total.y; mine.z += total.z; mine.w += total.w;
+      if (q == 0) kept = code;
     }
-    *reinterpret_cast<unsigned long long*>(head + base) = flags;
-  }
-  __device__ __forceinline__ void emit(int64_t i, int cls, const int4& before) const {
-    const int64_t u = (int64_t)before.x + before.y + before.z + before.w;
-    const int64_t id = (int64_t)keys[i];
-    uniq[u] = id;
-    if (uniq2) uniq2[u] = id;
-    run_start[u] = i;
-    if (table) {
-      const int pos = cls == 0 ? before.x : (cls == 1 ? before.y : (cls == 2 ? before.z : before.w));
-      dclass[u] = cls < 3 ? (int8_t)cls : (int8_t)-1;
-      dpos[u] = pos;
-      if (cls < 3 && out_ids[cls]) out_ids[cls][pos] = id;
+    sort_warp_sums<W>(mine, s_sum, warps, cta);
+    if (!ctx.prefix(cta, ahead, all)) return;
+#pragma unroll 1
+    for (int q = 0; q < strips; ++q) {
+      const int strip = begin + q * (8 * T);
+      const int j0 = strip + threadIdx.x * 8;
+      if (strips > 1) {
+        int4 total, c = make_int4(0, 0, 0, 0);
+        if (strips > 2) {
+          c = classify(j0, false);
+        } else {
+          const uint32_t last = code;  // strip 1 was classified last: its codes stay for the next turn
+          if (q == 0) code = kept;
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            const uint32_t v = (code >> (3 * x)) & 7u;
+            c.x += v == 4u;
+            c.y += v == 5u;
+            c.z += v == 6u;
+            c.w += v == 7u;
+          }
+          if (q == 0) kept = last;
+        }
+        lanes = scan_warp(c, total);
+        __syncthreads();
+        sort_warp_sums<W>(total, s_sum, warps, cta);
+      }
+      // The runs of the strip as a list in shared memory, so that what is written per run leaves in
+      // whole sectors: 13 bits place in the strip, 2 class, 14 number inside the class and strip.
+      int4 run = make_int4(warps.x + lanes.x, warps.y + lanes.y, warps.z + lanes.z, warps.w + lanes.w);
+      const int before = ahead.x + ahead.y + ahead.z + ahead.w;
+      if (j0 < end) base8[j0 >> 3] = before + run.x + run.y + run.z + run.w;
+      if (code) {
+        int at = run.x + run.y + run.z + run.w;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+          const uint32_t c = (code >> (3 * x)) & 7u;
+          if (!c) continue;
+          const uint32_t k = c & 3u;
+          const int pos = k == 0 ? run.x : (k == 1 ? run.y : (k == 2 ? run.z : run.w));
+          ctx.scratch[at++] = (threadIdx.x * 8 + x) | (k << 13) | ((uint32_t)pos << 15);
+          run.x += k == 0;
+          run.y += k == 1;
+          run.z += k == 2;
+          run.w += k == 3;
+        }
+      }
+      __syncthreads();
+      const int runs = cta.x + cta.y + cta.z + cta.w;
+#pragma unroll 2
+      for (int r = threadIdx.x; r < runs; r += T) {
+        const uint32_t w = ctx.scratch[r];
+        const int j = strip + (int)(w & 8191u);
+        const uint2 e = ctx.get(j);
+        const int64_t id = ctx.wide ? wide_id(e.y) : narrow_id(e.x);
+        const int u = before + r;
+        uniq[u] = id;
+        if (uniq2) uniq2[u] = id;
+        run_start[u] = j;
+        if (table) {
+          const int k = (int)(w >> 13) & 3;
+          const int pos = (int)(w >> 15) + (k == 0 ? ahead.x : (k == 1 ? ahead.y : (k == 2 ? ahead.z : ahead.w)));
+          dclass[u] = k < 3 ? (int8_t)k : (int8_t)-1;
+          dpos[u] = pos;
+          int64_t* to = k == 0 ? out_ids[0] : (k == 1 ? out_ids[1] : (k == 2 ? out_ids[2] : nullptr));
+          if (to) to[pos] = id;
+        }
+      }
+      if (strips > 1) __syncthreads();
+      if (strips == 2) code = kept;
+      ahead.x += cta.x; ahead.y += cta.y; ahead.z += cta.z; ahead.w += cta.w;
     }
-  }
-  __device__ __forceinline__ void finish(const int4& tot) const {
-    const int64_t u = (int64_t)tot.x + tot.y + tot.z + tot.w;
-    *num_runs = u;
-    if (num_runs2) *num_runs2 = u;
-    run_start[u] = valid_entries();
-    class_counts[0] = tot.x; class_counts[1] = tot.y; class_counts[2] = tot.z; class_counts[3] = tot.w;
-    if (class_counts2) { class_counts2[0] = tot.x; class_counts2[1] = tot.y; class_counts2[2] = tot.z; }
+    if (ctx.rank == 0 && threadIdx.x == 0) {
+      const int64_t u = (int64_t)all.x + all.y + all.z + all.w;
+      *num_runs = u;
+      if (num_runs2) *num_runs2 = u;
+      run_start[u] = ne;
+      class_counts[0] = all.x; class_counts[1] = all.y; class_counts[2] = all.z; class_counts[3] = all.w;
+      if (class_counts2) { class_counts2[0] = all.x; class_counts2[1] = all.y; class_counts2[2] = all.z; }
+    }
   }
 };
 
@@ -480,14 +596,10 @@ RunsPlan make_runs_plan(void* ws, int64_t n) {
   RunsPlan s;
   Carver cv(ws ? ws : (void*)256);  // a null workspace still yields the sizes
   const int64_t m = n > 0 ? n : 1;
-  s.k0 = cv.take<int64_t>(m);
-  s.k1 = cv.take<int64_t>(m);
-  s.p0 = cv.take<uint32_t>(m);
-  s.p1 = cv.take<uint32_t>(m);
-  s.sort_temp_bytes = sort_temp_bytes(m);
-  s.sort_temp = cv.take<char>(s.sort_temp_bytes);
+  s.perm = cv.take<uint32_t>(m);
+  s.sort_ws = cv.take<char>(sort_grid_bytes(m));
   s.run_start = cv.take<int64_t>(m + 1);
-  s.head = cv.take<uint8_t>(m + 1);
+  s.head = cv.take<uint8_t>(m + 8);
   s.n_valid = cv.take<int64_t>(1);
   s.num_runs = cv.take<int64_t>(1);
   s.class_counts = cv.take<int64_t>(4);
@@ -495,8 +607,6 @@ RunsPlan make_runs_plan(void* ws, int64_t n) {
   s.dpos = cv.take<int32_t>(m + 1);
   s.uniq = cv.take<int64_t>(m + 1);
   s.base8 = cv.take<int32_t>(m / 8 + 2);
-  s.compact_ws_bytes = compact_workspace_bytes(m);
-  s.compact_ws = cv.take<char>(s.compact_ws_bytes);
   s.total = cv.used() + 256;
   return s;
 }
@@ -545,47 +655,17 @@ int hb_runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int
     if (class_counts_out) HB_CUDA(cudaMemsetAsync(class_counts_out, 0, 3 * sizeof(int64_t), st));
     return HB_OK;
   }
-  if (seg_counts) {
-    // valid entries are scattered over the segments; their number becomes the device count
-    HB_LAUNCH(sum_counts_kernel, 1, 32, 0, st, seg_counts, n / seg_cap, seg_cap, s.n_valid);
-    n_dev = s.n_valid;
-  }
-  runs_out->n_dev = n_dev;
+  runs_out->n_dev = seg_counts ? s.n_valid : n_dev;
   const int64_t sentinel = id_bits >= 63 ? INT64_MAX : (((int64_t)1 << id_bits) - 1);
-  cub::DoubleBuffer<uint32_t> perm(s.p0, s.p1);
-  int rc;
-  int64_t* cls_out[3] = {class_ids_out ? class_ids_out[0] : nullptr, class_ids_out ? class_ids_out[1] : nullptr,
-                         class_ids_out ? class_ids_out[2] : nullptr};
-  if (id_bits <= 32) {
-    uint32_t* k0 = reinterpret_cast<uint32_t*>(s.k0);
-    uint32_t* k1 = reinterpret_cast<uint32_t*>(s.k1);
-    HB_LAUNCH(prepare_keys_kernel<uint32_t>, (int)ceil_div(n, kBlock), kBlock, 0, st, ids, n, n_dev,
-              seg_counts, seg_cap, sentinel, k0, s.p0, device_error_word());
-    cub::DoubleBuffer<uint32_t> keys(k0, k1);
-    HB_CUDA(cub::DeviceRadixSort::SortPairs(s.sort_temp, s.sort_temp_bytes, keys, perm, (int)n, 0,
-                                            id_bits, st));
-    HeadPolicy<uint32_t> pol{keys.Current(), n_dev, n, class_table, table_len, s.head, s.uniq, uniq_ids_out,
-                             s.run_start, s.dclass, s.dpos, {cls_out[0], cls_out[1], cls_out[2]},
-                             s.num_runs, num_unique_out, s.class_counts, class_counts_out, s.base8};
-    rc = run_compact(pol, n, s.compact_ws, s.compact_ws_bytes, st);
-    runs_out->keys = keys.Current();
-    runs_out->key_bytes = 4;
-  } else {
-    HB_LAUNCH(prepare_keys_kernel<int64_t>, (int)ceil_div(n, kBlock), kBlock, 0, st, ids, n, n_dev,
-              seg_counts, seg_cap, sentinel, s.k0, s.p0, device_error_word());
-    cub::DoubleBuffer<int64_t> keys(s.k0, s.k1);
-    HB_CUDA(cub::DeviceRadixSort::SortPairs(s.sort_temp, s.sort_temp_bytes, keys, perm, (int)n, 0,
-                                            id_bits, st));
-    HeadPolicy<int64_t> pol{keys.Current(), n_dev, n, class_table, table_len, s.head, s.uniq, uniq_ids_out,
-                            s.run_start, s.dclass, s.dpos, {cls_out[0], cls_out[1], cls_out[2]},
-                            s.num_runs, num_unique_out, s.class_counts, class_counts_out, s.base8};
-    rc = run_compact(pol, n, s.compact_ws, s.compact_ws_bytes, st);
-    runs_out->keys = keys.Current();
-    runs_out->key_bytes = 8;
-  }
-  count_library_launches(1 + (id_bits + 7) / 8);
-  runs_out->perm = perm.Current();
-  return rc;
+  runs_out->perm = s.perm;
+  IdSource src{ids, n, seg_counts ? nullptr : n_dev, seg_counts, (uint32_t)(seg_counts ? seg_cap : 1), sentinel,
+               device_error_word()};
+  RunsFinish fin{class_table, table_len, s.perm, s.head, s.uniq, uniq_ids_out, s.run_start,
+                 s.dclass, s.dpos,
+                 {class_ids_out ? class_ids_out[0] : nullptr, class_ids_out ? class_ids_out[1] : nullptr,
+                  class_ids_out ? class_ids_out[2] : nullptr},
+                 s.num_runs, num_unique_out, s.class_counts, class_counts_out, s.base8, s.n_valid};
+  return sort_run(src, fin, n, s.sort_ws, st);
 }
 
 namespace {

@@ -9,12 +9,10 @@ namespace hb {
 
 // carve of the workspace behind hb_runs_build
 struct RunsPlan {
-  int64_t *k0, *k1;     // sort keys (uint32 view when the ids fit 32 bits)
-  uint32_t *p0, *p1;    // positions
-  void* sort_temp;
-  size_t sort_temp_bytes;
+  uint32_t* perm;       // [m] positions
+  void* sort_ws;
   int64_t* run_start;   // [m + 1]
-  uint8_t* head;        // [m + 1]
+  uint8_t* head;        // [m + 8]
   int64_t* n_valid;     // [1]
   int64_t* num_runs;    // [1]
   int64_t* class_counts;  // [4]
@@ -22,8 +20,6 @@ struct RunsPlan {
   int32_t* dpos;        // [m + 1]
   int64_t* uniq;        // [m + 1]
   int32_t* base8;       // [m / 8 + 2]
-  void* compact_ws;
-  size_t compact_ws_bytes;
   size_t total;
 };
 

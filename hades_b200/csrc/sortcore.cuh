@@ -1,0 +1,849 @@
+// Stable sort of (key, position) pairs, fused with whatever works on the sorted order.
+//
+// A source says how many entries there are (a number that may only be known on the device) and
+// what the key of entry i is; a finish takes the sorted chunk of every CTA and does the rest (run
+// heads and classes of a batch, the walk over the cache sets, the LRU ageing) without another
+// launch.  Least significant digit first, every pass
+//   rank      warp by warp with match_any: how many earlier entries of the warp, of the CTA and of
+//             the earlier CTAs have the same digit
+//   scatter   to base[digit] + rank
+// so that equal keys keep the order of the input.
+//
+// What bounds it: latency.  A batch of 65,536 ids is half a megabyte, one of 2,000,000 is 16 MB and
+// stays in L2; with one launch per pass the time goes into launches, cold starts and the chain of
+// look-backs.  So
+//  * the passes of one sort run in ONE launch, separated by barriers;
+//  * digits are as wide as 10 bits and as few as the largest key needs, found on the device from
+//    the OR of the keys (ids of a table of 20 M rows: 25 bits, three passes; a caller that says
+//    nothing about its ids would pay eight passes of 8 bits otherwise);
+//  * up to 65,536 entries a cluster of 1 to 16 CTAs does it all in (distributed) shared memory:
+//    its barrier costs well under a microsecond and its digit counts are read from the peers' shared
+//    memory directly;
+//  * above that a cooperative grid, one CTA per SM, keeps its keys and ranks in registers between
+//    the counting and the scatter of a pass and goes through L2; barriers are counters in the
+//    workspace with bounded waits.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "launch.cuh"
+
+namespace hb {
+int* device_error_word();  // runtime.cu
+
+constexpr int kClusterT = 512;         // threads per CTA of the cluster version
+constexpr int kClusterDigit = 8;       // its bits per pass: counts are exchanged between all CTAs
+constexpr int kClusterMaxItems = 8;
+constexpr int64_t kSortClusterMax = 16 * (int64_t)kClusterT * kClusterMaxItems;  // its largest input
+constexpr int kGridT = 1024;           // threads per CTA of the grid version
+constexpr int kGridDigit = 10;
+constexpr int kGridBins = 1 << kGridDigit;
+
+// scratch of the grid version
+struct SortGridBufs {
+  uint2* kv0;          // [n]
+  uint2* kv1;          // [n]
+  uint32_t* hist;      // [grid][bins]
+  uint32_t* total;     // [bins]
+  unsigned* partial;   // [grid][4] OR of the keys (low, high), sentinel seen
+  int4* exchange;      // [grid]
+  unsigned* barrier;   // [1], zero before the launch
+};
+
+static inline int sort_grid_ctas(int64_t n) {
+  // fewer CTAs where the chunks would get short: a barrier over few CTAs is quicker
+  int64_t g = ceil_div(n, 2048);
+  const int64_t cap = sm_count();
+  return (int)(g > cap ? cap : (g < 1 ? 1 : g));
+}
+
+static inline size_t sort_grid_bytes(int64_t n) {
+  if (n <= kSortClusterMax) return 0;
+  const size_t g = (size_t)sm_count();
+  return 2 * align_up((size_t)n * sizeof(uint2), 256) + align_up(g * kGridBins * 4, 256) +
+         align_up(kGridBins * 4, 256) + align_up(g * 16, 256) + align_up(g * sizeof(int4), 256) + 256 + 256;
+}
+
+static inline SortGridBufs sort_grid_bufs(void* ws, int64_t n) {
+  SortGridBufs b;
+  Carver cv(ws);
+  const size_t g = (size_t)sm_count();
+  b.kv0 = cv.take<uint2>(n);
+  b.kv1 = cv.take<uint2>(n);
+  b.hist = cv.take<uint32_t>(g * kGridBins);
+  b.total = cv.take<uint32_t>(kGridBins);
+  b.partial = cv.take<unsigned>(g * 4);
+  b.exchange = cv.take<int4>(g);
+  b.barrier = cv.take<unsigned>(1);
+  return b;
+}
+
+#ifdef __CUDACC__
+
+namespace cg = cooperative_groups;
+
+// key of an entry that takes no part: larger than any other at every width (all ones)
+constexpr uint32_t kSortNone = 0xffffffffu;
+
+struct SortDigits {
+  int passes, width, bits;
+  bool wide;  // keys of more than 32 bits: digits come from the source, by position
+};
+
+__device__ __forceinline__ SortDigits sort_digits(unsigned lo, unsigned hi, bool none_seen, int max_width) {
+  SortDigits d;
+  int bits = hi ? 64 - __clz(hi) : 32 - __clz(lo);
+  if (none_seen) bits += 1;  // the all-ones key stays above every other
+  if (bits < 1) bits = 1;
+  if (bits > 64) bits = 64;
+  d.wide = bits > 32;
+  d.bits = bits;
+  d.passes = (bits + max_width - 1) / max_width;
+  d.width = (bits + d.passes - 1) / d.passes;
+  return d;
+}
+
+// exclusive scan over the first `bins` threads of the CTA (bins <= 1024, a multiple of 32 or below
+// 32); s_warp: [32].  All threads call it.
+__device__ __forceinline__ uint32_t sort_block_exscan(uint32_t v, int bins, uint32_t* s_warp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool on = warp * 32 < bins;
+  uint32_t inc = v;
+  if (on) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+  }
+  __syncthreads();
+  uint32_t before = 0;
+  if (on) before = __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[lane] : 0u);
+  return before + inc - v;
+}
+
+// sums over the CTA's warps: `mine` is the same in every lane of a warp; before = the warps ahead.
+// s4: [2 * W + 1].  A lane of four warps scans one component (a shuffle tree in every warp would
+// take the CTA's shuffle unit a thousand cycles).
+template <int W>
+__device__ __forceinline__ void sort_warp_sums(const int4& mine, int4* s4, int4& before, int4& all) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) s4[warp] = mine;
+  __syncthreads();
+  if (warp < 4) {
+    const int v = lane < W ? reinterpret_cast<const int*>(s4 + lane)[warp] : 0;
+    int inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane < W) reinterpret_cast<int*>(s4 + W + lane)[warp] = inc - v;
+    if (lane == 31) reinterpret_cast<int*>(s4 + 2 * W)[warp] = inc;
+  }
+  __syncthreads();
+  before = s4[W + warp];
+  all = s4[2 * W];
+}
+
+// zero_masks: the words of sort_rank_warp too (they stay zero from then on)
+template <int T>
+__device__ __forceinline__ void sort_zero_counts(uint16_t* wcnt, uint32_t* wmask, int bins, int zero_masks) {
+  uint32_t* w32 = reinterpret_cast<uint32_t*>(wcnt);
+  const int words = (T / 32) * bins / 2;
+  for (int k = threadIdx.x; k < words; k += T) w32[k] = 0u;
+  for (int k = threadIdx.x; k < zero_masks; k += T) wmask[k] = 0u;
+}
+
+// rank of a warp's items among the earlier ones of the same digit in the warp; leaves the warp's
+// digit counts in wc[0..bins).  wm[0..bins): one word per digit, zero before and after.
+// The lanes that share a digit find each other through an atomic OR into wm: measured at 32 warps
+// per SM 14 cycles per 32 items whose digits are scattered, against 60 for match.any (a turn for
+// every distinct value) and 2.8 per vote for digit bits taken one by one.  Same-address atomics
+// take turns, so neighbours that agree (popular ids once the lower digits are sorted) send one
+// OR together.
+template <int I>
+__device__ __forceinline__ void sort_rank_warp(const uint32_t (&k)[I], int left, int shift,
+                                               int width, uint16_t* wc, uint32_t* wm,
+                                               uint32_t (&rank)[(I + 1) / 2]) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t mask = (1u << width) - 1u;
+  if (left + lane <= 0) return;  // the whole warp
+#pragma unroll
+  for (int i = 0; i < I; ++i) {
+    const bool valid = i * 32 < left;
+    const uint32_t d = valid ? (k[i] >> shift) & mask : ~0u;
+    const uint32_t up = __shfl_up_sync(0xffffffffu, d, 1);
+    const bool lead = lane == 0 || up != d;
+    const unsigned leads = __ballot_sync(0xffffffffu, lead);
+    if (lead && valid) {
+      const unsigned later = leads & ~(lt | (1u << lane));
+      const unsigned upto = later ? (later & (0u - later)) - 1u : ~0u;
+      atomicOr(wm + d, upto & ~lt);
+    }
+    __syncwarp();
+    uint32_t pre = 0, same = 0;
+    if (valid) {
+      pre = wc[d];
+      same = wm[d];
+    }
+    __syncwarp();
+    if (valid && (same & lt) == 0u) {
+      wc[d] = (uint16_t)(pre + __popc(same));
+      wm[d] = 0u;
+    }
+    __syncwarp();
+    const uint32_t r = pre + __popc(same & lt);
+    if (i & 1) rank[i >> 1] |= r << 16; else rank[i >> 1] = r;
+  }
+}
+
+// counts per warp -> offsets of the warps inside the CTA, two digits per thread in one word (a
+// CTA holds fewer than 65,536 entries); the CTA's counts go to total[0..bins)
+template <int T>
+__device__ __forceinline__ void sort_scan_warps(uint16_t* wcnt, int bins, uint32_t* total) {
+  constexpr int W = T / 32;
+  uint32_t* w32 = reinterpret_cast<uint32_t*>(wcnt);
+  const int words = bins >> 1;
+  for (int d = threadIdx.x; d < words; d += T) {
+    uint32_t run = 0;
+#pragma unroll
+    for (int w0 = 0; w0 < W; w0 += 8) {
+      uint32_t c[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) c[w] = w32[(w0 + w) * words + d];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        w32[(w0 + w) * words + d] = run;
+        run += c[w];
+      }
+    }
+    total[2 * d] = run & 0xffffu;
+    total[2 * d + 1] = run >> 16;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Cluster version: I entries per thread, chunk kClusterT * I per CTA, 1 to 16 CTAs of one cluster.
+// ------------------------------------------------------------------------------------------------
+struct SortClusterSmem {
+  uint2* kv;         // [kClusterT * I]
+  uint16_t* wcnt;    // [warps][bins]
+  uint32_t* wmask;   // [warps][bins]
+  uint32_t* total;   // [bins] read by the peers
+  uint32_t* base;    // [bins]
+  uint32_t* warp;    // [32]
+  int4* sums;        // [2 * warps + 1]
+  int4* cta4;        // [3]: [0] read by the peers, [1..2] sums of the peers
+  uint4* seen;       // [2]: [0] read by the peers
+};
+
+static inline size_t sort_cluster_smem_bytes(int items) {
+  constexpr int W = kClusterT / 32, B = 1 << kClusterDigit;
+  return (size_t)kClusterT * items * sizeof(uint2) + (size_t)W * B * 6 + 2 * B * 4 + 32 * 4 + (2 * W + 1) * sizeof(int4) +
+         3 * sizeof(int4) + 2 * sizeof(uint4);
+}
+
+// what a finish sees: the sorted entries chunk by chunk, barriers and exchanges between the CTAs
+template <int ITEMS>
+struct ClusterCtx {
+  static constexpr int kThreads = kClusterT;
+  static constexpr int kItems = ITEMS;
+  static constexpr int kChunk = kClusterT * ITEMS;
+  SortClusterSmem s;
+  int count;   // entries that were sorted
+  uint32_t* scratch;  // shared memory, 8 * kThreads words, free after the sort
+  int rank, ctas;
+  bool wide;       // keys of more than 32 bits: .x of the entries is undefined
+  bool none;       // some entries take no part (kSortNone)
+  // (positions are 32-bit: at most 2^31 entries)
+  // first entry of this lane (a warp takes 32 * kItems consecutive ones); item i is at + 32 * i
+  __device__ __forceinline__ int first() const {
+    return rank * kChunk + (threadIdx.x >> 5) * (32 * ITEMS) + (threadIdx.x & 31);
+  }
+  __device__ __forceinline__ int chunk_begin() const { return rank * kChunk; }
+  __device__ __forceinline__ int chunk_end() const {
+    const int e = chunk_begin() + kChunk;
+    return e < count ? e : count;
+  }
+  // a sorted entry of this chunk, or the last one of the chunk before
+  __device__ __forceinline__ uint2 get(int j) const {
+    const int at = j - chunk_begin();
+    if (at >= 0) return s.kv[at];
+    return *cg::this_cluster().map_shared_rank(s.kv + (kChunk + at), rank - 1);
+  }
+  // 8 consecutive ones of this chunk from a multiple of 8 on (those at and beyond `count` are undefined)
+  __device__ __forceinline__ void get8(int j, uint2 (&e)[8]) const {
+    const uint4* p = reinterpret_cast<const uint4*>(s.kv + j - chunk_begin());
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 x = p[q];
+      e[2 * q] = make_uint2(x.x, x.y);
+      e[2 * q + 1] = make_uint2(x.z, x.w);
+    }
+  }
+  // sums over the CTAs: `mine` of the CTAs ahead and of all
+  __device__ __forceinline__ bool prefix(const int4& mine, int4& before, int4& all) {
+    if (ctas == 1) {
+      before = make_int4(0, 0, 0, 0);
+      all = mine;
+      return true;
+    }
+    if (threadIdx.x == 0) s.cta4[0] = mine;
+    sync();
+    if (threadIdx.x < 32) {
+      const int lane = threadIdx.x;
+      int4 v = make_int4(0, 0, 0, 0);
+      if (lane < ctas) v = *cg::this_cluster().map_shared_rank(s.cta4, lane);
+      int4 a, b;
+      a.x = __reduce_add_sync(0xffffffffu, v.x);
+      a.y = __reduce_add_sync(0xffffffffu, v.y);
+      a.z = __reduce_add_sync(0xffffffffu, v.z);
+      a.w = __reduce_add_sync(0xffffffffu, v.w);
+      if (lane >= rank) v = make_int4(0, 0, 0, 0);
+      b.x = __reduce_add_sync(0xffffffffu, v.x);
+      b.y = __reduce_add_sync(0xffffffffu, v.y);
+      b.z = __reduce_add_sync(0xffffffffu, v.z);
+      b.w = __reduce_add_sync(0xffffffffu, v.w);
+      if (lane == 0) {
+        s.cta4[1] = b;
+        s.cta4[2] = a;
+      }
+    }
+    __syncthreads();
+    before = s.cta4[1];
+    all = s.cta4[2];
+    return true;
+  }
+  // shared memory written before it, the peers' too, is seen after it
+  __device__ __forceinline__ void sync() const {
+    if (ctas > 1) cg::this_cluster().sync(); else __syncthreads();
+  }
+  // the same for global memory (read with __ldcg after it)
+  __device__ __forceinline__ bool barrier() {
+    if (ctas > 1) __threadfence();
+    sync();
+    return true;
+  }
+  // before a CTA leaves: no peer reads its shared memory any more
+  __device__ __forceinline__ void leave() {
+    if (ctas > 1) cg::this_cluster().sync();
+  }
+};
+
+template <class Src, class Fin, int I>
+__global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin fin) {
+  constexpr int T = kClusterT, W = T / 32, B = 1 << kClusterDigit;
+  extern __shared__ __align__(16) char smem[];
+  ClusterCtx<I> ctx;
+  SortClusterSmem& s = ctx.s;
+  {
+    char* p = smem;
+    s.kv = reinterpret_cast<uint2*>(p); p += (size_t)T * I * sizeof(uint2);
+    s.wcnt = reinterpret_cast<uint16_t*>(p); p += (size_t)W * B * 2;
+    s.wmask = reinterpret_cast<uint32_t*>(p); p += (size_t)W * B * 4;
+    s.total = reinterpret_cast<uint32_t*>(p); p += B * 4;
+    s.base = reinterpret_cast<uint32_t*>(p); p += B * 4;
+    s.warp = reinterpret_cast<uint32_t*>(p); p += 32 * 4;
+    s.sums = reinterpret_cast<int4*>(p); p += (2 * W + 1) * sizeof(int4);
+    s.cta4 = reinterpret_cast<int4*>(p); p += 3 * sizeof(int4);
+    s.seen = reinterpret_cast<uint4*>(p);
+  }
+  auto cluster = cg::this_cluster();
+  ctx.scratch = s.wmask;
+  ctx.rank = (int)cluster.block_rank();
+  ctx.ctas = (int)cluster.num_blocks();
+  const int n = (int)src.count();
+  ctx.count = n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first = ctx.first();
+  uint32_t k[I], v[I];
+  SortDigits dig;
+  {
+    unsigned lo = 0, hi = 0, none = 0;
+#pragma unroll
+    for (int i = 0; i < I; ++i) {
+      const int j = first + i * 32;
+      k[i] = kSortNone;
+      v[i] = (uint32_t)j;
+      if (j < n) {
+        unsigned long long key;
+        if (src.load(j, key)) {
+          k[i] = (uint32_t)key;
+          lo |= (unsigned)key;
+          hi |= (unsigned)(key >> 32);
+        } else {
+          none = 1u;
+        }
+      }
+    }
+    lo = __reduce_or_sync(0xffffffffu, lo);
+    hi = __reduce_or_sync(0xffffffffu, hi);
+    none = __reduce_or_sync(0xffffffffu, none);
+    uint4* per_warp = reinterpret_cast<uint4*>(s.sums);
+    if (lane == 0) per_warp[warp] = make_uint4(lo, hi, none, 0u);
+    __syncthreads();
+    if (warp == 0) {
+      const uint4 x = lane < W ? per_warp[lane] : make_uint4(0u, 0u, 0u, 0u);
+      lo = __reduce_or_sync(0xffffffffu, x.x);
+      hi = __reduce_or_sync(0xffffffffu, x.y);
+      none = __reduce_or_sync(0xffffffffu, x.z);
+      if (lane == 0) s.seen[0] = make_uint4(lo, hi, none, 0u);
+    }
+    ctx.sync();
+    if (ctx.ctas > 1) {
+      if (warp == 0) {
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (lane < ctx.ctas) x = *cluster.map_shared_rank(s.seen, lane);
+        lo = __reduce_or_sync(0xffffffffu, x.x);
+        hi = __reduce_or_sync(0xffffffffu, x.y);
+        none = __reduce_or_sync(0xffffffffu, x.z);
+        if (lane == 0) s.seen[1] = make_uint4(lo, hi, none, 0u);
+      }
+      __syncthreads();
+    }
+    const uint4 x = s.seen[ctx.ctas > 1 ? 1 : 0];
+    dig = sort_digits(x.x, x.y, x.z != 0u, kClusterDigit);
+    ctx.wide = dig.wide;
+    ctx.none = x.z != 0u;
+  }
+  for (int pass = 0; pass < dig.passes; ++pass) {
+    const int bit = pass * dig.width;
+    const int width = dig.bits - bit < dig.width ? dig.bits - bit : dig.width;
+    const int bins = 1 << width;
+    sort_zero_counts<T>(s.wcnt, s.wmask, bins, pass == 0 ? W * bins : 0);
+    if (pass > 0) {
+#pragma unroll
+      for (int i = 0; i < I; ++i) {
+        if (first + i * 32 < n) {
+          const uint2 e = s.kv[warp * (32 * I) + i * 32 + lane];
+          k[i] = e.x;
+          v[i] = e.y;
+        }
+      }
+    }
+    if (dig.wide) {
+#pragma unroll
+      for (int i = 0; i < I; ++i)
+        if (first + i * 32 < n) {
+          unsigned long long key;
+          k[i] = src.load(v[i], key) ? (uint32_t)(key >> bit) : kSortNone;
+        }
+    }
+    const int shift = dig.wide ? 0 : bit;
+    __syncthreads();
+    uint32_t rank[(I + 1) / 2];
+    uint16_t* wc = s.wcnt + warp * bins;
+    sort_rank_warp<I>(k, n - first, shift, width, wc, s.wmask + warp * bins, rank);
+    __syncthreads();
+    sort_scan_warps<T>(s.wcnt, bins, s.total);
+    ctx.sync();
+    uint32_t pre = 0, all = 0;
+    if ((int)threadIdx.x < bins) {
+      if (ctx.ctas > 1) {
+        uint32_t t[16];  // all sixteen on their way at once
+#pragma unroll
+        for (int c = 0; c < 16; ++c) t[c] = c < ctx.ctas ? *cluster.map_shared_rank(s.total + threadIdx.x, c) : 0u;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          if (c < ctx.rank) pre += t[c];
+          all += t[c];
+        }
+      } else {
+        all = s.total[threadIdx.x];
+      }
+    }
+    const uint32_t start = sort_block_exscan(all, bins, s.warp);
+    if ((int)threadIdx.x < bins) s.base[threadIdx.x] = start + pre;
+    __syncthreads();
+    const uint32_t mask = bins - 1;
+#pragma unroll
+    for (int i = 0; i < I; ++i) {
+      if (first + i * 32 < n) {
+        const uint32_t d = (k[i] >> shift) & mask;
+        const uint32_t to = s.base[d] + wc[d] + ((rank[i >> 1] >> (16 * (i & 1))) & 0xffffu);
+        uint2* at = s.kv + (to & (T * I - 1));
+        if (ctx.ctas > 1) at = cluster.map_shared_rank(at, to / (T * I));
+        *at = make_uint2(k[i], v[i]);
+      }
+    }
+    ctx.sync();
+  }
+  fin.run(ctx, src);
+  ctx.leave();
+}
+
+// ------------------------------------------------------------------------------------------------
+// Grid version: a cooperative launch, chunk of the input per CTA, scratch in global memory.
+// ------------------------------------------------------------------------------------------------
+template <int ITEMS>
+struct GridCtx {
+  static constexpr int kThreads = kGridT;
+  static constexpr int kItems = ITEMS;
+  const uint2* kv;     // the sorted entries
+  uint32_t* scratch;   // shared memory, 8 * kThreads words, free after the sort
+  int4* exchange;
+  unsigned* bar;
+  int4* s_pref;        // shared memory [2]
+  int* s_flag;         // shared memory [1]
+  int* err;
+  int count;
+  int chunk;       // entries per CTA
+  int rank, ctas, ntiles;
+  unsigned arrived;    // barriers passed so far
+  bool wide, none, alive;
+  __device__ __forceinline__ int chunk_begin() const {
+    const int b = rank * chunk;
+    return b < count ? b : count;
+  }
+  __device__ __forceinline__ int chunk_end() const {
+    const int e = rank * chunk + chunk;
+    return e < count ? e : count;
+  }
+  // a tile is kGridT * kItems entries (the last one fewer), a warp takes 32 * kItems consecutive ones
+  __device__ __forceinline__ int first(int t) const {
+    return rank * chunk + t * (kGridT * kItems) + (threadIdx.x >> 5) * (32 * kItems) + (threadIdx.x & 31);
+  }
+  __device__ __forceinline__ void get8(int j, uint2 (&e)[8]) const {
+    const uint4* p = reinterpret_cast<const uint4*>(kv + j);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 x = __ldcg(p + q);
+      e[2 * q] = make_uint2(x.x, x.y);
+      e[2 * q + 1] = make_uint2(x.z, x.w);
+    }
+  }
+  __device__ __forceinline__ uint2 get(int j) const { return __ldcg(kv + j); }
+  __device__ __forceinline__ bool barrier() {
+    ++arrived;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      bool ok = alive;
+      if (ok) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        const unsigned want = arrived * (unsigned)ctas;
+        ok = false;
+        for (int it = 0; it < (1 << 21); ++it) {  // bounded: a second or two, then the call reports a time-out
+          unsigned seen;
+          asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+          if (seen >= want) { ok = true; break; }
+          if (it > 4096) __nanosleep(64);
+        }
+        __threadfence();
+        if (!ok && err) atomicExch(err, HB_ERR_TIMEOUT);
+      }
+      *s_flag = ok;
+    }
+    __syncthreads();
+    alive = *s_flag != 0;
+    return alive;
+  }
+  __device__ __forceinline__ bool prefix(const int4& mine, int4& before, int4& all) {
+    if (threadIdx.x == 0) __stcg(exchange + rank, mine);
+    if (!barrier()) return false;
+    if (threadIdx.x < 32) {
+      int4 v = make_int4(0, 0, 0, 0), w = v;
+      for (int c = threadIdx.x; c < ctas; c += 32) {
+        const int4 x = __ldcg(exchange + c);
+        if (c < rank) { v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w; }
+        w.x += x.x; w.y += x.y; w.z += x.z; w.w += x.w;
+      }
+      int4 a, t;
+      a.x = __reduce_add_sync(0xffffffffu, v.x);
+      a.y = __reduce_add_sync(0xffffffffu, v.y);
+      a.z = __reduce_add_sync(0xffffffffu, v.z);
+      a.w = __reduce_add_sync(0xffffffffu, v.w);
+      t.x = __reduce_add_sync(0xffffffffu, w.x);
+      t.y = __reduce_add_sync(0xffffffffu, w.y);
+      t.z = __reduce_add_sync(0xffffffffu, w.z);
+      t.w = __reduce_add_sync(0xffffffffu, w.w);
+      if (threadIdx.x == 0) {
+        s_pref[0] = a;
+        s_pref[1] = t;
+      }
+    }
+    __syncthreads();
+    before = s_pref[0];
+    all = s_pref[1];
+    return true;
+  }
+};
+
+static inline size_t sort_grid_smem_bytes() {
+  return (size_t)(kGridT / 32) * kGridBins * 6 + 2 * (size_t)kGridBins * 4 + (kGridT / 32) * 4 + 2 * sizeof(int4) + 32;
+}
+
+template <class Src, class Fin, int I>
+__global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, SortGridBufs b, int max_digit, int* err) {
+  extern __shared__ __align__(16) char smem[];
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(smem);
+  uint32_t* wmask = reinterpret_cast<uint32_t*>(smem + (size_t)(kGridT / 32) * kGridBins * 2);
+  uint32_t* s_base = wmask + (kGridT / 32) * kGridBins;
+  uint32_t* s_tot = s_base + kGridBins;
+  int4* s_pref = reinterpret_cast<int4*>(s_tot + kGridBins);
+  uint32_t* s_warp = reinterpret_cast<uint32_t*>(s_pref + 2);
+  unsigned* s_seen = s_warp + (kGridT / 32);
+  int* s_flag = reinterpret_cast<int*>(s_seen + 4);
+  GridCtx<I> ctx;
+  ctx.scratch = wmask;
+  ctx.exchange = b.exchange;
+  ctx.bar = b.barrier;
+  ctx.s_pref = s_pref;
+  ctx.s_flag = s_flag;
+  ctx.err = err;
+  ctx.rank = blockIdx.x;
+  ctx.ctas = gridDim.x;
+  ctx.arrived = 0;
+  ctx.alive = true;
+  const int n = (int)src.count();
+  ctx.count = n;
+  {
+    const int per = (n + ctx.ctas - 1) / ctx.ctas;
+    ctx.chunk = (per + kGridT - 1) / kGridT * kGridT;  // whole rounds of the CTA
+  }
+  ctx.ntiles = ((ctx.chunk + kGridT * I - 1) / (kGridT * I));
+  if (ctx.ntiles < 1) ctx.ntiles = 1;
+  const int nt = ctx.ntiles;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int end = ctx.chunk_end();
+  uint32_t k[I];
+  uint32_t rank[(I + 1) / 2];
+  SortDigits dig;
+  {
+    unsigned lo = 0, hi = 0;
+    bool none = false;
+    for (int t = 0; t < nt; ++t) {
+      const int first = ctx.first(t);
+#pragma unroll
+      for (int i = 0; i < I; ++i) {
+        const int j = first + i * 32;
+        k[i] = kSortNone;
+        if (j < end) {
+          unsigned long long key;
+          if (src.load(j, key)) {
+            k[i] = (uint32_t)key;
+            lo |= (unsigned)key;
+            hi |= (unsigned)(key >> 32);
+          } else {
+            none = true;
+          }
+        }
+      }
+    }
+    lo = __reduce_or_sync(0xffffffffu, lo);
+    hi = __reduce_or_sync(0xffffffffu, hi);
+    none = __any_sync(0xffffffffu, none);
+    if (threadIdx.x < 4) s_seen[threadIdx.x] = 0u;
+    __syncthreads();
+    if (lane == 0) {
+      if (lo) atomicOr(s_seen, lo);
+      if (hi) atomicOr(s_seen + 1, hi);
+      if (none) atomicOr(s_seen + 2, 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) __stcg(reinterpret_cast<uint4*>(b.partial) + ctx.rank, make_uint4(s_seen[0], s_seen[1], s_seen[2], 0u));
+    if (!ctx.barrier()) return;
+    lo = hi = 0;
+    unsigned nn = 0;
+    for (int c = lane; c < ctx.ctas; c += 32) {
+      const uint4 p = __ldcg(reinterpret_cast<const uint4*>(b.partial) + c);
+      lo |= p.x; hi |= p.y; nn |= p.z;
+    }
+    lo = __reduce_or_sync(0xffffffffu, lo);
+    hi = __reduce_or_sync(0xffffffffu, hi);
+    nn = __reduce_or_sync(0xffffffffu, nn);
+    dig = sort_digits(lo, hi, nn != 0, max_digit);
+    ctx.wide = dig.wide;
+    ctx.none = nn != 0;
+  }
+  const uint2* in = nullptr;
+  uint2* out = b.kv0;
+  for (int pass = 0; pass < dig.passes; ++pass) {
+    const int bit = pass * dig.width;
+    const int width = dig.bits - bit < dig.width ? dig.bits - bit : dig.width;
+    const int bins = 1 << width;
+    const uint32_t mask = bins - 1;
+    const int shift = dig.wide ? 0 : bit;
+    uint16_t* wc = wcnt + warp * bins;
+    // keys of a tile into k[] (already there for the first pass of a chunk of one tile)
+    auto load_tile = [&](int t) {
+      const int first = ctx.first(t);
+#pragma unroll
+      for (int i = 0; i < I; ++i) {
+        const int j = first + i * 32;
+        if (j >= end) continue;
+        unsigned long long key;
+        if (dig.wide)
+          k[i] = src.load(in ? (int)__ldcg(&in[j].y) : j, key) ? (uint32_t)(key >> bit) : kSortNone;
+        else if (in)
+          k[i] = __ldcg(&in[j].x);
+        else if (nt > 1)
+          k[i] = src.load(j, key) ? (uint32_t)key : kSortNone;
+      }
+    };
+    auto rank_tile = [&](int t) -> uint32_t {  // the tile's count of digit threadIdx.x
+      __syncthreads();
+      sort_zero_counts<kGridT>(wcnt, wmask, bins, pass == 0 && t == 0 ? (kGridT / 32) * bins : 0);
+      load_tile(t);
+      __syncthreads();
+      sort_rank_warp<I>(k, end - ctx.first(t), shift, width, wc, wmask + warp * bins, rank);
+      __syncthreads();
+      sort_scan_warps<kGridT>(wcnt, bins, s_tot);
+      __syncthreads();
+      return (int)threadIdx.x < bins ? s_tot[threadIdx.x] : 0u;
+    };
+    uint32_t mine = 0, last = 0;
+    for (int t = 0; t < nt; ++t) {
+      last = rank_tile(t);
+      mine += last;
+    }
+    if ((int)threadIdx.x < bins) __stcg(b.hist + ctx.rank * bins + threadIdx.x, mine);
+    if (!ctx.barrier()) return;
+    // every CTA turns the counts of its share of the digits into offsets, a warp per digit
+    {
+      const int per = (bins + ctx.ctas - 1) / ctx.ctas;
+      const int d0 = ctx.rank * per;
+      const int d1 = d0 + per < bins ? d0 + per : bins;
+      for (int d = d0 + warp; d < d1; d += (kGridT / 32)) {
+        uint32_t run = 0;
+        for (int c0 = 0; c0 < ctx.ctas; c0 += 32 * 5) {
+          uint32_t x[5];
+#pragma unroll
+          for (int q = 0; q < 5; ++q) {
+            const int c = c0 + q * 32 + lane;
+            x[q] = c < ctx.ctas ? __ldcg(b.hist + c * bins + d) : 0u;
+          }
+#pragma unroll
+          for (int q = 0; q < 5; ++q) {
+            const int c = c0 + q * 32 + lane;
+            uint32_t inc = x[q];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+              if (lane >= o) inc += y;
+            }
+            if (c < ctx.ctas) __stcg(b.hist + c * bins + d, run + inc - x[q]);
+            run += __shfl_sync(0xffffffffu, inc, 31);
+          }
+        }
+        if (lane == 0) __stcg(b.total + d, run);
+      }
+    }
+    if (!ctx.barrier()) return;
+    {
+      const uint32_t all = (int)threadIdx.x < bins ? __ldcg(b.total + threadIdx.x) : 0u;
+      const uint32_t pre = (int)threadIdx.x < bins ? __ldcg(b.hist + ctx.rank * bins + threadIdx.x) : 0u;
+      const uint32_t start = sort_block_exscan(all, bins, s_warp);
+      if ((int)threadIdx.x < bins) s_base[threadIdx.x] = start + pre;
+    }
+    for (int t = 0; t < nt; ++t) {
+      if (nt > 1) last = rank_tile(t);
+      __syncthreads();
+      const int first = ctx.first(t);
+#pragma unroll
+      for (int i = 0; i < I; ++i) {
+        const int j = first + i * 32;
+        if (j < end) {
+          const uint32_t d = (k[i] >> shift) & mask;
+          const uint32_t to = s_base[d] + wc[d] + ((rank[i >> 1] >> (16 * (i & 1))) & 0xffffu);
+          __stcg(out + to, make_uint2(k[i], in ? __ldcg(&in[j].y) : (uint32_t)j));
+        }
+      }
+      if (nt > 1) {
+        __syncthreads();
+        if ((int)threadIdx.x < bins) s_base[threadIdx.x] += last;
+      }
+    }
+    if (!ctx.barrier()) return;
+    in = out;
+    out = out == b.kv0 ? b.kv1 : b.kv0;
+  }
+  ctx.kv = in;
+  fin.run(ctx, src);
+}
+
+// ---- launches ------------------------------------------------------------------------------------
+template <class Src, class Fin, int I>
+int sort_launch_cluster(const Src& src, const Fin& fin, int ctas, cudaStream_t st) {
+  const size_t smem = sort_cluster_smem_bytes(I);
+  auto kernel = sort_cluster_kernel<Src, Fin, I>;
+  static thread_local int ready_dev = -1;
+  int dev = 0;
+  HB_CUDA(cudaGetDevice(&dev));
+  if (ready_dev != dev) {
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    ready_dev = dev;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kClusterT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, src, fin));
+  count_launch();
+  return HB_OK;
+}
+
+template <class Src, class Fin, int I>
+int sort_launch_grid(const Src& src, const Fin& fin, int64_t n, int max_digit, void* ws, cudaStream_t st) {
+  SortGridBufs b = sort_grid_bufs(ws, n);
+  const size_t smem = sort_grid_smem_bytes();
+  auto kernel = sort_grid_kernel<Src, Fin, I>;
+  static thread_local int ready_dev = -1;
+  int dev = 0;
+  HB_CUDA(cudaGetDevice(&dev));
+  if (ready_dev != dev) {
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ready_dev = dev;
+  }
+  HB_CUDA(cudaMemsetAsync(b.barrier, 0, sizeof(unsigned), st));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sort_grid_ctas(n));
+  cfg.blockDim = dim3(kGridT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, src, fin, b, max_digit, device_error_word()));
+  count_launch();
+  return HB_OK;
+}
+
+// n: most entries the source can have; ws: sort_grid_bytes(n) bytes, 256-byte aligned (none needed for
+// n <= kSortClusterMax)
+template <class Src, class Fin>
+int sort_run(const Src& src, const Fin& fin, int64_t n, void* ws, cudaStream_t st) {
+  // First more CTAs, then longer chunks: what a pass issues (votes, counts, stores) is bound by one
+  // SM's units, and the barrier of a larger cluster costs little more.
+  if (n <= kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 1, st);
+  if (n <= 2 * kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 2, st);
+  if (n <= 4 * kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 4, st);
+  if (n <= 8 * kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 8, st);
+  if (n <= 16 * kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 16, st);
+  if (n <= 32 * kClusterT) return sort_launch_cluster<Src, Fin, 2>(src, fin, 16, st);
+  if (n <= 64 * kClusterT) return sort_launch_cluster<Src, Fin, 4>(src, fin, 16, st);
+  if (n <= kSortClusterMax) return sort_launch_cluster<Src, Fin, 8>(src, fin, 16, st);
+  const int64_t per = ceil_div(n, sort_grid_ctas(n));
+  if (per <= 2 * kGridT) return sort_launch_grid<Src, Fin, 2>(src, fin, n, kGridDigit, ws, st);
+  if (per <= 4 * kGridT) return sort_launch_grid<Src, Fin, 4>(src, fin, n, kGridDigit, ws, st);
+  if (per <= 8 * kGridT) return sort_launch_grid<Src, Fin, 8>(src, fin, n, kGridDigit, ws, st);
+  return sort_launch_grid<Src, Fin, 16>(src, fin, n, kGridDigit, ws, st);
+}
+
+#endif  // __CUDACC__
+
+}  // namespace hb

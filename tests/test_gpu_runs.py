@@ -51,6 +51,41 @@ def test_runs_build_matches_numpy_unique(cuda_lib, n, space, id_bits):
     assert head.sum() == U and np.array_equal(np.nonzero(head)[0], run_start[:U])
 
 
+# one CTA / clusters of 2 to 16 CTAs / longer chunks per CTA / the grid version with one and with
+# several tiles per CTA, at their edges and one beyond; ids of few and of many digits, equal to the
+# padding key of 32 bits, and wider than 32 bits
+@pytest.mark.parametrize("n", [511, 513, 1024, 1025, 8193, 16385, 32769, 65536, 65537, 131_073, 300_001, 1_212_417,
+                               2_424_833])
+@pytest.mark.parametrize("low,space", [(0, 1), (0, 900), (0, 20_000_000), (2**32 - 3, 3), (2**40, 10**12)])
+def test_runs_build_at_the_edges_of_the_sort(cuda_lib, n, low, space):
+    from hades_b200 import EmbCacheLib as E
+    from hades_b200.exchange import _as_tensor
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + space)
+    ids = low + (torch.rand(n, device="cuda", generator=g, dtype=torch.float64) ** 3 * space).long()
+    classes = torch.randint(0, 4, (min(low + space, 1 << 20),), device="cuda", generator=g).to(torch.int8)
+    for kw in ({}, {"n_dev": torch.tensor([n // 3], device="cuda")}):
+        runs = E.cudaRunsBuild(ids, 64, classes, want_uniq=True, **kw)
+        m = n // 3 if kw else n
+        want, order = torch.sort(ids[:m], stable=True)
+        u, counts = torch.unique(want, return_counts=True)
+        U = u.numel()
+        assert int(runs.num_unique.item()) == U and torch.equal(runs.uniq_ids[:U], u)
+        assert torch.equal(_as_tensor(runs.desc.perm, (n,), "<i4", ids.device)[:m].long(), order)
+        start = _as_tensor(runs.desc.run_start, (U + 1,), "<i8", ids.device)
+        assert torch.equal(start[1:] - start[:-1], counts) and int(start[0]) == 0
+        head = _as_tensor(runs.desc.head, (n,), "|u1", ids.device)[:m].long()
+        base8 = _as_tensor(runs.desc.base8, ((m + 7) // 8,), "<i4", ids.device).long()
+        assert int(head.sum()) == U and bool((head[start[:-1]] == 1).all())
+        assert torch.equal(base8, (torch.cumsum(head, 0) - head)[::8])
+        cls = torch.where(u < classes.numel(), classes[u.clamp(max=classes.numel() - 1)], torch.tensor(3, device="cuda", dtype=torch.int8))
+        for c in range(3):
+            ids_c = u[cls == c]
+            assert int(runs.class_counts[c]) == ids_c.numel()
+            assert torch.equal(runs.class_ids[c][: ids_c.numel()], ids_c)
+
+
 def test_runs_build_prefix_count_and_segments(cuda_lib):
     from hades_b200 import EmbCacheLib as E
 
