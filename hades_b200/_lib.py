@@ -77,6 +77,8 @@ PROTOTYPES: dict[str, tuple] = {
     "hb_runs_build": (_int, [_p, _i64, _p, _p, _i64, _int, _p, _i64, _p, _p, _p, _p, _p, _sz, _p, _p]),
     "hb_segsum_runs_workspace_bytes": (_sz, [_i64, _i64]),
     "hb_segsum_runs_f32": (_int, [_p, _p, _p, _i64, _int, _p, _p, _p, _p, _sz, _p]),
+    "hb_segsum_update_f32": (_int, [_p, _p, _p, _i64, _int, _p, _p, _sz, _p]),
+    "hb_unique_update_f32": (_int, [_p, _p, _p, _i64, _p, _p, _i64, _i64, _int, _int, _p, _p, _sz, _p]),
     "hb_lookup_fetch_runs_workspace_bytes": (_sz, [_i64, _i64, _int]),
     "hb_lookup_fetch_runs": (_int, [_p, _p, _p, _p, _i64, _p, _i64, _p, _p, _p, _p, _int, _p, _sz, _p]),
     "hb_runs_resolve_requests": (_int, [_p, _p, _p, _p, _i64, _p, _i64, _p, _p, _p, _int, _p, _sz, _p]),
@@ -134,6 +136,13 @@ class ClassSplitDesc(C.Structure):
     """hb_class_split_t"""
     _fields_ = [("table", _p), ("table_len", _i64), ("out_ids", _p * 3), ("out_rows", _p * 3),
                 ("out_cnt", _p * 3), ("class_counts", _p)]
+
+
+class OptimDesc(C.Structure):
+    """hb_optim_t"""
+    _fields_ = [("kind", _int), ("emb_elem_bytes", _int), ("emb", _p), ("s0", _p), ("s1", _p), ("step", _p),
+                ("id_offset", _i64), ("id_stride", _i64), ("rows", _i64), ("lr", C.c_double), ("beta1", C.c_double),
+                ("beta2", C.c_double), ("eps", C.c_double)]
 
 
 class StagingDesc(C.Structure):

@@ -4,9 +4,8 @@
 // sum += g*g; emb -= lr * g / (sqrt(sum) + eps)).  State, gradient and embedding
 // rows are read and written once, in one kernel; the reference moves state
 // through cached fetch/set kernels and the embedding through a CPU write.
-#include <cuda_fp16.h>
-
 #include "launch.cuh"
+#include "optim.cuh"
 
 namespace hb {
 namespace {
@@ -18,45 +17,6 @@ __device__ __forceinline__ int64_t effective_n(int64_t n, const int64_t* n_dev) 
   const int64_t d = *n_dev;
   return d < n ? d : n;
 }
-
-struct RowMap {
-  int64_t offset, stride, rows;
-  __device__ __forceinline__ int64_t operator()(int64_t id) const {
-    if (id < offset) return -1;
-    const int64_t r = (id - offset) / stride;
-    return r < rows ? r : -1;
-  }
-};
-
-template <typename E> struct EmbIO;
-template <> struct EmbIO<float> {
-  static __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-  static __device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-  static __device__ __forceinline__ float load(const float* p) { return *p; }
-  static __device__ __forceinline__ void store(float* p, float v) { *p = v; }
-};
-template <> struct EmbIO<__half> {
-  static __device__ __forceinline__ float4 load4(const __half* p) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
-    const __half2 a = *reinterpret_cast<const __half2*>(&raw.x);
-    const __half2 b = *reinterpret_cast<const __half2*>(&raw.y);
-    const float2 fa = __half22float2(a), fb = __half22float2(b);
-    return make_float4(fa.x, fa.y, fb.x, fb.y);
-  }
-  static __device__ __forceinline__ void store4(__half* p, float4 v) {
-    const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
-    uint2 raw;
-    raw.x = *reinterpret_cast<const unsigned*>(&a);
-    raw.y = *reinterpret_cast<const unsigned*>(&b);
-    *reinterpret_cast<uint2*>(p) = raw;
-  }
-  static __device__ __forceinline__ float load(const __half* p) { return __half2float(*p); }
-  static __device__ __forceinline__ void store(__half* p, float v) { *p = __float2half_rn(v); }
-};
-
-struct AdamParams {
-  float lr, beta1, beta2, eps, one_minus_beta1, one_minus_beta2;
-};
 
 __device__ __forceinline__ float adam_elem(float g, float& m, float& v, float bias1, float bias2,
                                            const AdamParams& p) {
@@ -99,6 +59,7 @@ __global__ void __launch_bounds__(kBlock, 4) sparse_adam_kernel(
       if (row[r] >= 0 && sub == 0) {
         // state_step = state_step + 1 (per row), sparse_optim.py:624-626
         const float t = step[row[r]] + 1.0f;
+        step[row[r]] = t;  // no other lane looks at it: ids are distinct
         b1 = 1.0f - powf(p.beta1, t);
         b2 = 1.0f - powf(p.beta2, t);
         cc = cnt ? (float)__ldg(cnt + i) : 1.0f;  // grad / cnt, sparse_optim.py:608-611
@@ -154,14 +115,12 @@ __global__ void __launch_bounds__(kBlock, 4) sparse_adam_kernel(
 // rows per round: lane l works out the per-row scalars of row l once (for Adam the two bias
 // corrections, whose powf would otherwise be issued for every 16 bytes of the row), then the
 // warp walks the rows, G lanes per row and kOptRows rows in flight, taking the scalars by
-// shuffle.  Divisions by per-row scalars are multiplications by their reciprocals (one ulp,
-// far inside the 1e-5 the parity tests allow); the element-wise division and the square root
-// are IEEE.
+// shuffle.
 template <typename E, bool ADAM>
 __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
     const int64_t* __restrict__ ids, const float* __restrict__ grads,
     const int64_t* __restrict__ cnt, int64_t n, const int64_t* __restrict__ n_dev, int64_t dim,
-    RowMap map, const float* __restrict__ step, float* __restrict__ s0, float* __restrict__ s1,
+    RowMap map, float* __restrict__ step, float* __restrict__ s0, float* __restrict__ s1,
     E* __restrict__ emb, AdamParams p, int glog2, int rpw) {
   // rpw: rows a warp takes per round (32, or fewer so that a short list still fills the GPU)
   n = effective_n(n, n_dev);
@@ -179,6 +138,7 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
       if (ADAM) {
         // state_step = state_step + 1 (per row), sparse_optim.py:624-626
         const float t = step[row] + 1.0f;
+        step[row] = t;  // no other lane looks at it: ids are distinct
         ra = 1.0f / (1.0f - powf(p.beta1, t));
         rb = 1.0f / (1.0f - powf(p.beta2, t));
       }
@@ -218,14 +178,8 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float g = cnt ? g4[j] * c[u] : g4[j];
-              if (ADAM) {
-                m4[j] = p.beta1 * m4[j] + p.one_minus_beta1 * g;
-                v4[j] = p.beta2 * v4[j] + p.one_minus_beta2 * (g * g);
-                e4[j] -= p.lr * (m4[j] * a[u]) / (sqrtf(v4[j] * b[u]) + p.eps);  // sparse_optim.py:654-655
-              } else {
-                m4[j] += g * g;
-                e4[j] -= p.lr * g / (sqrtf(m4[j]) + p.eps);
-              }
+              if (ADAM) adam_value(g, m4[j], v4[j], e4[j], a[u], b[u], p);
+              else adagrad_value(g, m4[j], e4[j], p);
             }
             reinterpret_cast<float4*>(s0 + rw[u] * dim)[k] = mm[u];
             if (ADAM) reinterpret_cast<float4*>(s1 + rw[u] * dim)[k] = vv[u];
@@ -250,18 +204,6 @@ int grid_for_warps(int64_t n, int rpw) {
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
   return blocks < 1 ? 1 : (int)blocks;
-}
-
-// step[row] += 1 for every updated row; a launch of its own so that no lane of
-// the update kernel can see the new step of its own row.
-__global__ void bump_step_kernel(const int64_t* __restrict__ ids, int64_t n,
-                                 const int64_t* __restrict__ n_dev, RowMap map,
-                                 float* __restrict__ step) {
-  n = effective_n(n, n_dev);
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t row = map(__ldg(ids + i));
-  if (row >= 0) step[row] += 1.0f;
 }
 
 template <typename E, bool VEC4>
@@ -360,7 +302,6 @@ int hb_sparse_adam(const int64_t* ids, const float* grads, const int64_t* cnt, i
   }
 #undef HB_ADAM_VEC
 #undef HB_ADAM
-  HB_LAUNCH(bump_step_kernel, (int)ceil_div(n, kBlock), kBlock, 0, st, ids, n, n_dev, map, step);
   return HB_OK;
 }
 

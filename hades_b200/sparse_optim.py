@@ -13,6 +13,8 @@ ships rows over PCIe and RPC).
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 import torch.distributed as dist
 
@@ -127,6 +129,23 @@ class _SparseOptimizer:
         return idx.contiguous(), grad.contiguous(), None if cnt is None else cnt.contiguous()
 
 
+    def _update_merging(self, idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap) -> bool:
+        """unique_grads (sparse_optim.py:611) and the row update of what it returns in one pass over
+        the gradients; False: rows too wide or too many for that (``hb_segsum_update_f32``)."""
+        n, dim = idx.numel(), grad.size(1)
+        w = self.emb.weight
+        desc = self._desc()
+        aligned = (w.data_ptr() | grad.data_ptr() | (desc.s0 or 0) | (desc.s1 or 0)) & 15 == 0
+        if dim > (512 if dim % 4 == 0 and aligned else 128) or self.emb.rows >= 1 << 30:
+            return False
+        lib = _lib.load()
+        ws = _lib.workspace(lib.hb_unique_segsum_workspace_bytes(n, dim))
+        _lib.check(lib.hb_unique_update_f32(idx.data_ptr(), grad.data_ptr(), _lib.ptr(cnt), n, _lib.ptr(n_dev),
+                                            _lib.ptr(seg_counts), int(seg_cap), dim, int(id_bits), 1, C.byref(desc),
+                                            ws.data_ptr(), ws.numel(), _lib.stream_ptr()))
+        return True
+
+
 class SparseAdam(_SparseOptimizer):
     """SparseAdam of the reference (sparse_optim.py:531-702) on this rank's shard.
 
@@ -165,6 +184,13 @@ class SparseAdam(_SparseOptimizer):
         self.state_step = torch.zeros(emb.rows, dtype=torch.float32, device=dev)
         self.state_mem = torch.zeros((emb.rows, dim), dtype=torch.float32, device=dev)
         self.state_power = torch.zeros((emb.rows, dim), dtype=torch.float32, device=dev)
+
+    def _desc(self):
+        """hb_optim_t of the state in HBM (its tensors keep their addresses; lr may change)."""
+        w, e = self.emb.weight, self.emb
+        return _lib.OptimDesc(0, w.element_size(), w.data_ptr(), self.state_mem.data_ptr(), self.state_power.data_ptr(),
+                              self.state_step.data_ptr(), e.rank, e.world, e.rows, self._lr, self._beta1, self._beta2,
+                              self._eps)
 
     def full_state(self):
         """(step, mem, power) of the whole shard as CUDA tensors, whichever tier the rows are in."""
@@ -215,6 +241,8 @@ class SparseAdam(_SparseOptimizer):
         every segment holds strictly ascending ids (merge instead of sort)."""
         idx, grad, cnt = self._args(idx, grad, cnt)
         if not is_unique:
+            if self.state_cache is None and self._update_merging(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap):
+                return
             idx, grad, n_dev = _merge_duplicates(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap, sorted_segments)
             cnt = None
         if self.state_cache is not None:
@@ -238,6 +266,12 @@ class SparseAdagrad(_SparseOptimizer):
         self.state_sum = torch.zeros((emb.rows, emb.embedding_dim), dtype=torch.float32,
                                      device=emb.weight.device)
 
+    def _desc(self):
+        """hb_optim_t of the state (its tensors keep their addresses; lr may change)."""
+        w, e = self.emb.weight, self.emb
+        return _lib.OptimDesc(1, w.element_size(), w.data_ptr(), self.state_sum.data_ptr(), None, None, e.rank, e.world,
+                              e.rows, self._lr, 0.0, 0.0, self._eps)
+
     def update(self, idx, grad, cnt=None, is_unique: bool = False, n_dev: torch.Tensor | None = None,
                id_bits: int = 64, seg_counts: torch.Tensor | None = None, seg_cap: int = 0,
                sorted_segments: bool = False) -> None:
@@ -246,6 +280,8 @@ class SparseAdagrad(_SparseOptimizer):
         every segment holds strictly ascending ids (merge instead of sort)."""
         idx, grad, cnt = self._args(idx, grad, cnt)
         if not is_unique:
+            if self._update_merging(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap):
+                return
             idx, grad, n_dev = _merge_duplicates(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap, sorted_segments)
             cnt = None
         lib = _lib.load()

@@ -391,6 +391,38 @@ int hb_segsum_runs_f32(const hb_runs_t* runs /* host */, const float* grads,
                        int64_t* counts /* nullable */, const hb_class_split_t* split /* nullable */,
                        void* workspace, size_t workspace_bytes, hb_stream_t stream);
 
+/* A sparse optimiser and the shard it updates, for the calls that update rows as their gradients
+ * become complete (the rules of hb_sparse_adam / hb_sparse_adagrad): row of an id =
+ * (id - id_offset) / id_stride when that is below `rows`, other ids are skipped. */
+#define HB_OPT_ADAM 0
+#define HB_OPT_ADAGRAD 1
+typedef struct hb_optim {
+  int kind;
+  int emb_elem_bytes;      /* 4 = fp32, 2 = fp16 */
+  void* emb;               /* [rows][dim] */
+  float* s0;               /* Adam: mem; Adagrad: sum of squares, [rows][dim] */
+  float* s1;               /* Adam: power */
+  float* step;             /* Adam: [rows] */
+  int64_t id_offset, id_stride, rows;
+  double lr, beta1, beta2, eps;
+} hb_optim_t;
+
+/* hb_segsum_runs_f32 with the optimiser's update as its output: the merged row of every distinct id
+ * updates the state and the table row directly (SparseAdam.update on ids that repeat,
+ * python/EmbCache/sparse_optim.py:608-681), no merged rows in memory.  Rows of up to 512 columns (128
+ * when dim is not a multiple of 4 or a buffer not 16-byte aligned), else HB_ERR_UNSUPPORTED.
+ * Workspace: hb_segsum_runs_workspace_bytes. */
+int hb_segsum_update_f32(const hb_runs_t* runs /* host */, const float* grads,
+                         const int64_t* cnt_in /* nullable */, int64_t dim, int mean,
+                         const hb_optim_t* opt /* host */, void* workspace, size_t workspace_bytes,
+                         hb_stream_t stream);
+/* hb_runs_build + hb_segsum_update_f32; ids, n_dev, seg_counts, seg_cap, id_bits as for
+ * hb_unique_segsum_f32.  Workspace: hb_unique_segsum_workspace_bytes. */
+int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* cnt_in /* nullable */, int64_t n,
+                         const int64_t* n_dev /* nullable */, const int64_t* seg_counts /* nullable */,
+                         int64_t seg_cap, int64_t dim, int id_bits, int mean, const hb_optim_t* opt /* host */,
+                         void* workspace, size_t workspace_bytes, hb_stream_t stream);
+
 /* hb_lookup_fetch (or hb_lookup_fetch_sharded when `table` is given) over a batch that
  * hb_runs_build has sorted: same outputs at the same batch positions (locs, found,
  * out_rows), in two launches (three with a sharded table).  The first works per DISTINCT id:

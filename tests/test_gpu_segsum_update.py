@@ -1,0 +1,71 @@
+"""Aggregation with the optimiser's update as its output (hb_unique_update_f32, what
+``SparseAdam.update`` / ``SparseAdagrad.update`` run on ids that repeat) against a float64
+restatement of unique_grads + the update rule (python/EmbCache/sparse_optim.py:142-157,590-685), at
+the edges of pieces, CTAs and column layouts."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+LR, B1, B2 = 0.01, 0.9, 0.999
+
+
+def _reference(kind, ids, grads, cnt, w, s0, s1, step, rank, world):
+    u, inv = torch.unique(ids, return_inverse=True)
+    sums = torch.zeros((u.numel(), grads.size(1)), dtype=torch.float64, device="cuda").index_add_(0, inv, grads.double())
+    div = torch.zeros(u.numel(), dtype=torch.float64, device="cuda").index_add_(
+        0, inv, torch.ones_like(inv, dtype=torch.float64) if cnt is None else cnt.double())
+    g = sums / (div if cnt is None else div + 1)[:, None]
+    r = (u - rank) // world
+    if kind == "adam":
+        step[r] += 1
+        s0[r] = B1 * s0[r] + (1 - B1) * g
+        s1[r] = B2 * s1[r] + (1 - B2) * g * g
+        m, v = s0[r] / (1 - B1 ** step[r])[:, None], s1[r] / (1 - B2 ** step[r])[:, None]
+        w[r] -= LR * m / (v.sqrt() + 1e-8)
+    else:
+        s0[r] += g * g
+        w[r] -= LR * g / (s0[r].sqrt() + 1e-10)
+    return r
+
+
+@pytest.mark.parametrize("kind,dtype", [("adam", torch.float32), ("adam", torch.float16), ("adagrad", torch.float32),
+                                        ("adagrad", torch.float16)])
+@pytest.mark.parametrize("n,dim", [(1, 128), (7, 4), (8, 16), (129, 32), (257, 128), (2049, 47), (4097, 100), (6000, 3),
+                                   (70_001, 64), (9_001, 256), (3_001, 512), (40_000, 128), (3_000, 520)])
+def test_update_of_repeated_ids(cuda_lib, kind, dtype, n, dim):
+    from hades_b200.sparse_optim import ShardedEmbedding, SparseAdagrad, SparseAdam
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n + dim)
+    rank, world, num = 1, 3, 30_000
+    emb = ShardedEmbedding(num, dim, rank, world, dtype=dtype, init_sigma=0.01, seed=n)
+    opt = (SparseAdam if kind == "adam" else SparseAdagrad)(emb, lr=LR)
+    w = emb.weight.double()
+    s0, s1 = torch.zeros_like(w), torch.zeros_like(w)
+    step = torch.zeros(emb.rows, dtype=torch.float64, device="cuda")
+    for it in range(3):
+        # one id with a third of the rows (it crosses CTAs), one with a few, the rest nearly distinct
+        rows = torch.randint(0, emb.rows, (n,), device="cuda", generator=gen)
+        rows[torch.rand(n, device="cuda", generator=gen) < 0.33] = 17
+        rows[:12] = 18
+        ids = rows * world + rank
+        # values whose sums do not nearly cancel: the first updates of a row are lr * g / |g|
+        grads = (1 + torch.rand((n, dim), device="cuda", generator=gen)) * 1e-3
+        cnt = torch.randint(1, 5, (n,), device="cuda", generator=gen) if it == 1 else None
+        opt.update(ids, grads, cnt, **({"id_bits": 20} if it else {}))
+        touched = _reference(kind, ids, grads, cnt, w, s0, s1, step, rank, world)
+        if dtype == torch.float16:
+            w[touched] = w[touched].half().double()  # the table is rounded after every update
+        # fp32 sums of n rows and a few roundings: 1e-5 of the state and of an update (LR); a table
+        # value then differs by 1e-5 * LR = 1e-4 of 1e-3 (the floor below).  fp16 table: one unit in the
+        # last place (2^-10 relative, 2^-9 below the floor's binade) where the exact value lies between two.
+        tol = 1e-5
+        state0 = opt.state_mem if kind == "adam" else opt.state_sum
+        assert float((state0.double() - s0).abs().max() / s0.abs().max()) < tol
+        err = (emb.weight.double() - w).abs() / w.abs().clamp(min=1e-3)
+        assert float(err.max()) < (2e-3 if dtype == torch.float16 else 1e-4), float(err.max())
+        if kind == "adam":
+            assert torch.equal(opt.state_step.double(), step)
+            assert float((opt.state_power.double() - s1).abs().max() / s1.abs().max()) < tol
+        w = emb.weight.double()  # from here on the same table
