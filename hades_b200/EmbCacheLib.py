@@ -191,8 +191,9 @@ class IndexCache:
         """CPU lookup of the reference (src/cache/cache.h:213-222): returns the slots and
         applies the LRU side effect of every hit, in batch order."""
         dev = self._to_dev(ids)
-        locs = self.cudalookup(dev)
-        self.cuda_touch_lru(locs)
+        locs = torch.empty_like(dev)
+        _lib.check(self._lib.hb_index_lookup_touch(self._h, dev.data_ptr(), dev.numel(), locs.data_ptr(),
+                                                   self.lookup_mode, _lib.stream_ptr()))
         return locs if ids.is_cuda else locs.cpu()
 
     def reset(self, ids: torch.Tensor) -> None:

@@ -8,6 +8,7 @@
 
 #include "index.cuh"
 #include "launch.cuh"
+#include "sortcore.cuh"
 
 namespace hb {
 namespace {
@@ -27,47 +28,40 @@ __global__ void fill_i32_kernel(int32_t* p, int64_t n, int32_t v) {
 }
 
 // ---- add ---------------------------------------------------------------------
-// key = set of the id (or `lines` for an unusable id), value = position in batch.
-__global__ void add_keys_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t lines,
-                                uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t id = ids[i];
-  keys[i] = id >= 0 ? (uint32_t)mod_nonneg(id, lines) : (uint32_t)lines;
-  vals[i] = (uint32_t)i;
-}
-
-// One thread per set that appears in the batch: it owns the line, applies the
-// batch's ids for that set in input order (keys were stably sorted, so vals are
-// ascending inside a set).  Placement policy: src/cache/cache.h:51-88 with
+// The line of one set in registers.  Placement policy: src/cache/cache.h:51-88 with
 // find_or_empty_entry (cache_line.h:67-78) and find_lru (cache_line.h:92-103).
-__global__ void add_walk_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t lines,
-                                const uint32_t* __restrict__ keys,
-                                const uint32_t* __restrict__ vals, int64_t* __restrict__ line_ids,
-                                int32_t* __restrict__ lru, int64_t* __restrict__ locs,
-                                uint8_t* __restrict__ last_writer) {
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t line = keys[j];
-  if ((int64_t)line >= lines) {              // unusable ids (negative: padding) sort last
-    locs[vals[j]] = -1;                      // every thread answers for its own entry
-    if (last_writer) last_writer[vals[j]] = 0;
-    return;
-  }
-  if (j > 0 && keys[j - 1] == line) return;  // not the head of its segment
-  int64_t last_k[kWays];  // sorted position of the last id of the batch placed in each way
-#pragma unroll
-  for (int w = 0; w < kWays; ++w) last_k[w] = -1;
+struct LineState {
   int64_t lid[kWays];
   int32_t cnt[kWays];
+  int last[kWays];  // which id of the batch was placed in each way last, -1 = none
+
+  __device__ __forceinline__ void load(const int64_t* line_ids, const int32_t* lru, int64_t line) {
+    const longlong2* p = reinterpret_cast<const longlong2*>(line_ids + line * kWays);
+    const int4* q = reinterpret_cast<const int4*>(lru + line * kWays);
 #pragma unroll
-  for (int w = 0; w < kWays; ++w) {
-    lid[w] = line_ids[(int64_t)line * kWays + w];
-    cnt[w] = lru[(int64_t)line * kWays + w];
+    for (int w = 0; w < kWays; w += 2) {
+      const longlong2 v = p[w / 2];
+      lid[w] = v.x;
+      lid[w + 1] = v.y;
+    }
+#pragma unroll
+    for (int w = 0; w < kWays; w += 4) {
+      const int4 v = q[w / 4];
+      cnt[w] = v.x; cnt[w + 1] = v.y; cnt[w + 2] = v.z; cnt[w + 3] = v.w;
+    }
+#pragma unroll
+    for (int w = 0; w < kWays; ++w) last[w] = -1;
   }
-  for (int64_t k = j; k < n && keys[k] == line; ++k) {
-    const uint32_t pos = vals[k];
-    const int64_t id = ids[pos];
+  __device__ __forceinline__ void store(int64_t* line_ids, int32_t* lru, int64_t line) const {
+    longlong2* p = reinterpret_cast<longlong2*>(line_ids + line * kWays);
+    int4* q = reinterpret_cast<int4*>(lru + line * kWays);
+#pragma unroll
+    for (int w = 0; w < kWays; w += 2) p[w / 2] = make_longlong2(lid[w], lid[w + 1]);
+#pragma unroll
+    for (int w = 0; w < kWays; w += 4) q[w / 4] = make_int4(cnt[w], cnt[w + 1], cnt[w + 2], cnt[w + 3]);
+  }
+  // places the k-th id of the batch for this set; the way, -1 = refused
+  __device__ __forceinline__ int place(int64_t id, int k) {
     int way = -1;
     bool exists = false;
 #pragma unroll
@@ -87,40 +81,220 @@ __global__ void add_walk_kernel(const int64_t* __restrict__ ids, int64_t n, int6
       }
       way = tmp == 0 ? -1 : best;
     }
-    if (way >= 0) {
-      if (!exists) {
 #pragma unroll
-        for (int w = 0; w < kWays; ++w) {
-          if (w == way) { lid[w] = id; cnt[w] = 0; }  // set_id zeroes the counter
-        }
+    for (int w = 0; w < kWays; ++w)
+      if (w == way) {
+        if (!exists) { lid[w] = id; cnt[w] = 0; }  // set_id zeroes the counter
+        last[w] = k;
       }
-      locs[pos] = (int64_t)line * kWays + way;
+    return way;
+  }
+  __device__ __forceinline__ bool is_last(int64_t loc, int k) const {
+    if (loc < 0) return false;
+    const int way = (int)(loc & (kWays - 1));
+    bool yes = false;
 #pragma unroll
-      for (int w = 0; w < kWays; ++w)
-        if (w == way) last_k[w] = k;
-    } else {
-      locs[pos] = -1;
+    for (int w = 0; w < kWays; ++w)
+      if (w == way) yes = last[w] == k;
+    return yes;
+  }
+};
+
+// Two ways to the ids of a set in input order.
+//
+// (1) Sorted by set (sortcore.cuh), input order kept inside a set; one thread per set walks them.  For
+//     small batches (one launch), for batches of many ids per set, and (LONG_LISTS) for the sets that
+//     (2) leaves behind, usually none.
+constexpr uint32_t kLongList = 0xffffffffu;  // in place of the entry: the set's list is long
+
+template <bool LONG_LISTS>
+struct SetSource {
+  static constexpr bool kSkips = LONG_LISTS;
+  const int64_t* ids;
+  int64_t n;
+  int64_t lines;
+  const unsigned long long* heads;
+  const int32_t* batch;
+  __device__ __forceinline__ int64_t count() const { return !LONG_LISTS || batch[4] == batch[2] ? n : 0; }
+  __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
+    const int64_t x = __ldg(ids + i);
+    if (x < 0) return false;  // unusable (padding)
+    key = (unsigned long long)mod_nonneg(x, lines);
+    return !LONG_LISTS || heads[key] == (((unsigned long long)(uint32_t)batch[2] << 32) | kLongList);
+  }
+};
+
+template <bool LONG_LISTS>
+__device__ __forceinline__ void add_sorted_set(int j, int n, const uint2* kv, const int64_t* ids, int64_t* line_ids,
+                                               int32_t* lru, int64_t* locs, uint8_t* last_writer) {
+  const uint2 e = __ldcg(kv + j);
+  if (e.x == kSortNone) {  // every thread answers for its own entry
+    if (LONG_LISTS) return;
+    locs[e.y] = -1;
+    if (last_writer) last_writer[e.y] = 0;
+    return;
+  }
+  if (j > 0 && __ldcg(&kv[j - 1].x) == e.x) return;  // not the head of its segment
+  const int64_t line = e.x;
+  LineState st;
+  st.load(line_ids, lru, line);
+  int k = j;
+  uint2 x = e;
+  while (true) {
+    const int way = st.place(__ldg(ids + x.y), k);
+    locs[x.y] = way >= 0 ? line * kWays + way : -1;
+    ++k;
+    if (k >= n) break;
+    x = __ldcg(kv + k);
+    if (x.x != e.x) break;
+  }
+  st.store(line_ids, lru, line);
+  if (last_writer)
+    for (int m = j; m < k; ++m) {
+      const uint32_t pos = __ldcg(&kv[m].y);
+      last_writer[pos] = st.is_last(locs[pos], m);
     }
+}
+
+struct AddFinish {
+  int64_t* line_ids;
+  int32_t* lru;
+  int64_t* locs;           // [n]
+  uint8_t* last_writer;    // nullable [n]: of several ids that received one slot, the last
+  uint2* sorted;           // [n] scratch
+  bool walk_later;         // by a launch of its own
+  template <class Ctx, class Src>
+  __device__ __forceinline__ void run(Ctx& ctx, const Src& src) const {
+    const uint2* kv = ctx.publish(sorted);
+    if (walk_later) return;
+    for (int j = ctx.chunk_begin() + threadIdx.x; j < ctx.chunk_end(); j += Ctx::kThreads)
+      add_sorted_set<Src::kSkips>(j, ctx.count, kv, src.ids, line_ids, lru, locs, last_writer);
   }
-#pragma unroll
-  for (int w = 0; w < kWays; ++w) {
-    line_ids[(int64_t)line * kWays + w] = lid[w];
-    lru[(int64_t)line * kWays + w] = cnt[w];
+};
+
+__global__ void __launch_bounds__(kBlock) add_sorted_walk_kernel(const int64_t* ids, int n, AddFinish f) {
+  const int j = blockIdx.x * kBlock + threadIdx.x;
+  if (j < n) add_sorted_set<false>(j, n, f.sorted, ids, f.line_ids, f.lru, f.locs, f.last_writer);
+}
+
+// (2) Every id puts itself on the list of its set (one atomic exchange); the thread whose id ended up
+//     in front owns the set, brings the list into input order and walks it.  No sort.  Lists of more
+//     than 32 ids (copies of one id, ids in strides of the number of sets) go to (1).
+__global__ void __launch_bounds__(kBlock) add_push_kernel(const int64_t* __restrict__ ids, int64_t n, AddLists lists,
+                                                          int64_t* __restrict__ locs, uint8_t* __restrict__ last_writer) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t id = __ldg(ids + i);
+  if (id >= 0) {
+    lists.push(id, i);
+  } else {
+    locs[i] = -1;
+    if (last_writer) last_writer[i] = 0;
   }
-  if (last_writer) {
-    for (int64_t k = j; k < n && keys[k] == line; ++k) {
-      const uint32_t pos = vals[k];
-      const int64_t loc = locs[pos];
-      bool last = false;
-      if (loc >= 0) {
-        const int way = (int)(loc & (kWays - 1));
+}
+
+constexpr int kListShort = 32;  // ids of a set that are put in order in a thread's own memory
+
+// where the first `cap` listed entries end (a block finds it together); the usual case: nothing to cut
+__device__ __forceinline__ int64_t add_cut(const AddEntries& e, int64_t n) {
+  __shared__ long long s_cut[2];
+  if (!e.total || (int64_t)*e.total <= e.cap) return n;
+  __shared__ int s_warp[kBlock / 32];
+  const int64_t chunks = (n + 31) / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t left = e.cap;  // listed entries still allowed
+  for (int64_t c0 = 0; c0 < chunks; c0 += kBlock * 16) {
+    const int64_t c = c0 + threadIdx.x * 16;
+    int mine = 0;
+    for (int x = 0; x < 16; ++x)
+      if (c + x < chunks) mine += __ldg(e.chunk_listed + c + x);
+    int inc = mine;
 #pragma unroll
-        for (int w = 0; w < kWays; ++w)
-          if (w == way) last = last_k[w] == k;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    if (threadIdx.x == 0) s_cut[0] = -1;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < kBlock / 32; ++w) {
+      if (w < warp) before += s_warp[w];
+      all += s_warp[w];
+    }
+    const int64_t first = before + inc - mine;  // listed entries of this round ahead of this thread's
+    if (left >= first && left < first + mine) {
+      int64_t need = left - first;
+      int x = 0;
+      while (need >= __ldg(e.chunk_listed + c + x)) { need -= __ldg(e.chunk_listed + c + x); ++x; }
+      int64_t i = (c + x) * 32;
+      while (true) {
+        if (e.listed[i]) { if (need == 0) break; --need; }
+        ++i;
       }
-      last_writer[pos] = last;
+      s_cut[0] = i;
     }
+    __syncthreads();
+    const int64_t cut = s_cut[0];
+    if (cut >= 0) return cut;
+    left -= all;
+    __syncthreads();
   }
+  return n;
+}
+
+__global__ void __launch_bounds__(kBlock) add_walk_kernel(AddEntries e, unsigned long long* __restrict__ heads,
+                                                          int32_t* batch, const uint32_t* __restrict__ next, int64_t lines,
+                                                          int64_t* __restrict__ line_ids, int32_t* __restrict__ lru,
+                                                          int64_t* __restrict__ locs, uint8_t* __restrict__ last_writer) {
+  const uint32_t number = batch_number(batch + 2);
+  int64_t n = e.n;
+  if (e.n_dev && *e.n_dev < n) n = *e.n_dev;
+  const int64_t cut = add_cut(e, n);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const bool listed = e.listed ? e.listed[i] != 0 : true;
+    if (!listed) continue;
+    const int64_t id = __ldg(e.ids + i);
+    if (id < 0) continue;
+    const int64_t line = mod_nonneg(id, lines);
+    if (heads[line] != (((unsigned long long)number << 32) | (unsigned long long)(i + 1))) continue;
+    LineState st;
+    st.load(line_ids, lru, line);
+    uint32_t behind = next[i];
+    if (!behind) {  // the usual case: one id for the set
+      const bool taken = i < cut;
+      const int way = taken ? st.place(id, 0) : -1;
+      locs[i] = way >= 0 ? line * kWays + way : -1;
+      if (last_writer) last_writer[i] = way >= 0;
+      if (way >= 0) st.store(line_ids, lru, line);
+      continue;
+    }
+    uint32_t order[kListShort];
+    int len = 0;
+    uint32_t at = (uint32_t)i + 1u;
+    for (; at && len < kListShort; at = next[at - 1]) {
+      int k = len++;
+      for (; k > 0 && order[k - 1] > at; --k) order[k] = order[k - 1];
+      order[k] = at;
+    }
+    if (at) {
+      heads[line] = ((unsigned long long)number << 32) | kLongList;
+      batch[4] = (int32_t)number;
+      continue;
+    }
+    for (int k = 0; k < len; ++k) {
+      const int64_t x = (int64_t)order[k] - 1;
+      const int way = x < cut ? st.place(__ldg(e.ids + x), k) : -1;
+      locs[x] = way >= 0 ? line * kWays + way : -1;
+    }
+    if (last_writer)
+      for (int k = 0; k < len; ++k) {
+        const int64_t x = (int64_t)order[k] - 1;
+        last_writer[x] = st.is_last(locs[x], k);
+      }
+    st.store(line_ids, lru, line);
+  }
+  batch_done(batch + 2, number);
 }
 
 // ---- lookup ------------------------------------------------------------------
@@ -147,160 +321,145 @@ __global__ void __launch_bounds__(kBlock) lookup_kernel(IndexView v, const int64
 }
 
 // ---- LRU touch ---------------------------------------------------------------
-__global__ void touch_keys_kernel(const int64_t* __restrict__ locs, int64_t n, int64_t capacity,
-                                  uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t s = locs[i];
-  keys[i] = (s >= 0 && s < capacity) ? (uint32_t)s : (uint32_t)capacity;
-  vals[i] = (uint32_t)i;
-}
-
-__device__ __forceinline__ int64_t lower_bound_u32(const uint32_t* a, int64_t lo, int64_t hi,
-                                                   uint32_t key) {
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (a[mid] < key) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
-// keys = hit slots sorted ascending (stable, so batch positions ascend inside a
-// slot).  The thread at the head of each line's segment computes the counters
-// that the sequential rule "all counters of the line += 1, hit way = 0"
-// (cache_line.h:80-86) leaves after the whole batch:
+// The sequential rule "all counters of the line += 1, hit way = 0" (cache_line.h:80-86) leaves after a
+// whole batch
 //   way hit in the batch   -> number of hits on the line after its last hit
 //   way not hit            -> old counter + hits on the line
-__global__ void touch_apply_kernel(const uint32_t* __restrict__ keys,
-                                   const uint32_t* __restrict__ vals, int64_t n, int64_t capacity,
-                                   int32_t* __restrict__ lru) {
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t key = keys[j];
-  if ((int64_t)key >= capacity) return;  // misses sort last
-  const uint32_t line = key >> 3;
-  if (j > 0 && (keys[j - 1] >> 3) == line) return;
-  // run boundaries of the 8 ways inside this line's segment
-  int64_t rb[kWays + 1];
-  rb[0] = j;
-  // first position whose key belongs to a later line (or a miss)
-  int64_t seg_hi = n;
-  {
-    // gallop to bound the binary search by the segment length, not by n
-    int64_t step = 8;
-    int64_t hi = j + 1;
-    const uint32_t next = (line + 1) << 3;
-    while (hi < n && keys[hi] < next) { hi = (hi + step < n) ? hi + step : n; step <<= 1; }
-    seg_hi = lower_bound_u32(keys, j, hi, next);
+// Three passes over the batch positions, no sort: the last hit of every slot and the hits of every
+// line; the hits after each slot's last; the counters.  (65,536 positions: sorted 40 us, this 9.)  Lanes
+// with the same slot speak as one, so that the copies of a popular id do not queue at one address.
+template <int MODE, bool LOOKUP>
+__global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const int64_t* __restrict__ ids,
+                                                            int64_t* __restrict__ locs, int64_t n, TouchMarks t,
+                                                            int32_t* __restrict__ line_hits) {
+  __shared__ int64_t s_top[LOOKUP && MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
+  if (LOOKUP && MODE == HB_LOOKUP_SORTED) {
+    stage_top_level(v, s_top);
+    __syncthreads();
   }
-#pragma unroll
-  for (int w = 1; w < kWays; ++w) rb[w] = lower_bound_u32(keys, rb[w - 1], seg_hi, (line << 3) + w);
-  rb[kWays] = seg_hi;
-  const int32_t total = (int32_t)(seg_hi - j);
-#pragma unroll
-  for (int w = 0; w < kWays; ++w) {
-    int32_t* c = lru + (int64_t)line * kWays + w;
-    if (rb[w + 1] == rb[w]) {
-      *c += total;
-    } else {
-      const uint32_t last = vals[rb[w + 1] - 1];
-      int32_t after = 0;
-#pragma unroll
-      for (int x = 0; x < kWays; ++x) {
-        if (x == w || rb[x + 1] == rb[x]) continue;
-        // positions in run x greater than `last`
-        int64_t lo = rb[x], hi = rb[x + 1];
-        while (lo < hi) {
-          const int64_t mid = (lo + hi) >> 1;
-          if (vals[mid] <= last) lo = mid + 1; else hi = mid;
-        }
-        after += (int32_t)(rb[x + 1] - lo);
-      }
-      *c = after;
+  const unsigned long long number = (unsigned long long)batch_number(t.batch) << 32;
+  const int lane = lane_id();
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t base = warp * 32; base < n; base += nwarps * 32) {
+    const int64_t i = base + lane;
+    int64_t slot = -1;
+    if (LOOKUP) {
+      slot = warp_lookup<MODE>(v, s_top, i < n ? __ldg(ids + i) : -1);
+      if (i < n) locs[i] = slot;
+    } else if (i < n) {
+      slot = locs[i];
+      if (slot >= t.capacity) slot = -1;
+    }
+    const unsigned same = __match_any_sync(0xffffffffu, slot);
+    if (slot >= 0 && (same >> lane) == 1u) {  // the last of them
+      atomicMax(t.marks + slot, number | (unsigned long long)(i + 1));
+      atomicAdd(line_hits + (slot >> 3), __popc(same));
     }
   }
 }
 
-// ---- LRU touch from runs -------------------------------------------------------
-// The batch is given as runs of equal ids (each run = the sorted batch positions
-// of one id, ascending), so no sort is needed: a first kernel notes which run hit
-// each slot, a second computes per hit slot the same closed form as above, with
-// "hits on the line after my last hit" counted by binary search in the position
-// lists of the other hit ways of the line.
-struct RunsView {
-  const int64_t* locs;       // slot of every batch position (or of every sorted entry, see below)
-  const uint32_t* perm;      // nullable: position list of the runs (identity when null)
-  const int64_t* run_start;  // nullable: run u = [run_start[u], run_start[u+1]) (run u = {u} when null)
-  const int64_t* num_runs;   // nullable device count
-  const int64_t* n_dev;      // nullable device count of positions
-  int64_t max_runs;
-  int64_t n;
-  int locs_kind;             // locs holds a slot per batch position (0), per sorted entry (1), per run (2)
-  __device__ __forceinline__ int64_t slot_of_run(int64_t u) const {
-    if (locs_kind == 2) return locs[u];
-    const int64_t j = start(u);
-    return locs[locs_kind == 1 ? j : pos(j)];
+// ways of a line that the batch hit: their last positions, 0 = not hit
+__device__ __forceinline__ void line_marks(const unsigned long long* marks, int64_t line, uint32_t number,
+                                           uint32_t (&last)[kWays]) {
+  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(marks + line * kWays);
+#pragma unroll
+  for (int w = 0; w < kWays; w += 2) {
+    const ulonglong2 x = p[w / 2];
+    last[w] = (uint32_t)(x.x >> 32) == number ? (uint32_t)x.x : 0u;
+    last[w + 1] = (uint32_t)(x.y >> 32) == number ? (uint32_t)x.y : 0u;
   }
-  __device__ __forceinline__ int64_t positions() const {
-    if (!n_dev) return n;
-    const int64_t d = *n_dev;
-    return d < n ? (d > 0 ? d : 0) : n;
-  }
-  __device__ __forceinline__ int64_t runs() const {
-    int64_t r = max_runs;
-    if (num_runs && *num_runs < r) r = *num_runs;
-    if (!run_start) { const int64_t p = positions(); if (p < r) r = p; }
-    return r;
-  }
-  __device__ __forceinline__ int64_t start(int64_t u) const { return run_start ? run_start[u] : u; }
-  __device__ __forceinline__ int64_t end(int64_t u, int64_t nruns, int64_t npos) const {
-    return (u + 1 < nruns) ? start(u + 1) : npos;
-  }
-  __device__ __forceinline__ int64_t pos(int64_t j) const { return perm ? (int64_t)perm[j] : j; }
-};
-
-// The batch number lives on the device and is advanced by a kernel, so that a
-// captured CUDA graph that contains the ageing can be replayed.
-__global__ void touch_runs_next_epoch_kernel(int32_t* epoch) { *epoch += 1; }
-
-__global__ void touch_runs_mark_kernel(RunsView v, int64_t capacity, const int32_t* epoch_dev,
-                                       int32_t* __restrict__ slot_run,
-                                       int32_t* __restrict__ slot_epoch) {
-  const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (u >= v.runs()) return;
-  const int32_t epoch = *epoch_dev;
-  const int64_t slot = v.slot_of_run(u);
-  if (slot < 0 || slot >= capacity) return;
-  slot_run[slot] = (int32_t)u;
-  slot_epoch[slot] = epoch;
 }
 
-__global__ void touch_runs_apply_kernel(RunsView v, int64_t capacity, const int32_t* epoch_dev,
-                                        const int32_t* __restrict__ slot_run,
-                                        const int32_t* __restrict__ slot_epoch,
-                                        int32_t* __restrict__ lru) {
-  const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t nruns = v.runs();
-  if (u >= nruns) return;
-  const int32_t epoch = *epoch_dev;
-  const int64_t npos = v.positions();
-  const int64_t slot = v.slot_of_run(u);
-  if (slot < 0 || slot >= capacity) return;
-  const int64_t line = slot >> 3;
-  const int way = (int)(slot & 7);
-  const int64_t last = v.pos(v.end(u, nruns, npos) - 1);
-  int32_t total = 0, after = 0;
-  bool leader = true;
-  bool hit[kWays];
+__global__ void __launch_bounds__(kBlock) touch_after_kernel(const int64_t* __restrict__ locs, int64_t n, TouchMarks t,
+                                                             int32_t* __restrict__ after) {
+  const uint32_t number = batch_number(t.batch);
+  const int lane = lane_id();
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t base = warp * 32; base < n; base += nwarps * 32) {
+    const int64_t i = base + lane;
+    int64_t slot = i < n ? locs[i] : -1;
+    if (slot >= t.capacity) slot = -1;
+    const unsigned same = __match_any_sync(0xffffffffu, slot);
+    if (slot < 0 || (same >> lane) != 1u) continue;
+    uint32_t last[kWays];
+    line_marks(t.marks, slot >> 3, number, last);
 #pragma unroll
-  for (int w = 0; w < kWays; ++w) {
-    hit[w] = slot_epoch[line * kWays + w] == epoch;
-    if (!hit[w]) continue;
-    const int64_t u2 = slot_run[line * kWays + w];
-    const int64_t s2 = v.start(u2), e2 = v.end(u2, nruns, npos);
-    total += (int32_t)(e2 - s2);
-    if (w < way) leader = false;
-    if (w != way) {
+    for (int w = 0; w < kWays; ++w) {
+      if (w == (int)(slot & 7) || !last[w] || last[w] > (uint32_t)(i + 1)) continue;
+      // position p of this slot counts when p + 1 > last[w]: lanes from last[w] - base on
+      const int64_t from = (int64_t)last[w] - base;
+      const unsigned later = from <= 0 ? same : (from >= 32 ? 0u : same & ~((1u << from) - 1u));
+      if (later) atomicAdd(after + (slot & ~(int64_t)7) + w, __popc(later));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) touch_apply_kernel(const int64_t* __restrict__ locs, int64_t n, TouchMarks t,
+                                                             int32_t* __restrict__ after, int32_t* __restrict__ line_hits,
+                                                             int32_t* __restrict__ lru) {
+  const uint32_t number = batch_number(t.batch);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t slot = locs[i];
+    if (slot < 0 || slot >= t.capacity) continue;
+    const int64_t line = slot >> 3;
+    // the line is taken by the last hit of its lowest hit way
+    if (t.marks[slot] != (((unsigned long long)number << 32) | (unsigned long long)(i + 1))) continue;
+    uint32_t last[kWays];
+    line_marks(t.marks, line, number, last);
+    bool first = true;
+#pragma unroll
+    for (int w = 0; w < kWays; ++w)
+      if (w < (int)(slot & 7) && last[w]) first = false;
+    if (!first) continue;
+    const int32_t total = line_hits[line];
+    line_hits[line] = 0;
+#pragma unroll
+    for (int w = 0; w < kWays; ++w) {
+      const int64_t x = line * kWays + w;
+      if (last[w]) {
+        lru[x] = after[x];
+        after[x] = 0;
+      } else {
+        lru[x] += total;
+      }
+    }
+  }
+  batch_done(t.batch, number);
+}
+
+// ---- LRU touch from runs -------------------------------------------------------
+// The batch is given as runs of equal ids (each run = the sorted batch positions
+// of one id, ascending), so "hits on the line after my last hit" is counted by
+// binary search in the position lists of the other hit ways of the line, found through the marks.
+__global__ void touch_runs_mark_kernel(RunsView v, TouchMarks marks) {
+  const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (u < v.runs()) marks.mark(v.slot_of_run(u), u);
+}
+
+__global__ void __launch_bounds__(kBlock) touch_runs_apply_kernel(RunsView v, TouchMarks t, int32_t* __restrict__ lru) {
+  const uint32_t number = batch_number(t.batch);
+  const int64_t nruns = v.runs();
+  const int64_t npos = v.positions();
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nruns; u += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t slot = v.slot_of_run(u);
+    if (slot < 0 || slot >= t.capacity) continue;
+    const int64_t line = slot >> 3;
+    const int way = (int)(slot & 7);
+    uint32_t run[kWays];
+    line_marks(t.marks, line, number, run);
+    const int64_t end = v.end(u, nruns, npos);
+    const int64_t last = v.pos(end - 1);
+    int32_t total = (int32_t)(end - v.start(u)), after = 0;
+    bool leader = true;
+#pragma unroll
+    for (int w = 0; w < kWays; ++w) {
+      if (!run[w] || w == way) continue;
+      const int64_t u2 = (int64_t)run[w] - 1;
+      const int64_t s2 = v.start(u2), e2 = v.end(u2, nruns, npos);
+      total += (int32_t)(e2 - s2);
+      if (w < way) leader = false;
       int64_t lo = s2, hi = e2;  // first position of the run greater than `last`
       while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
@@ -308,13 +467,14 @@ __global__ void touch_runs_apply_kernel(RunsView v, int64_t capacity, const int3
       }
       after += (int32_t)(e2 - lo);
     }
-  }
-  lru[slot] = after;
-  if (leader) {
+    lru[slot] = after;
+    if (leader) {
 #pragma unroll
-    for (int w = 0; w < kWays; ++w)
-      if (!hit[w]) lru[line * kWays + w] += total;
+      for (int w = 0; w < kWays; ++w)
+        if (!run[w] && w != way) lru[line * kWays + w] += total;
+    }
   }
+  batch_done(t.batch, number);
 }
 
 // ---- reset -------------------------------------------------------------------
@@ -395,26 +555,62 @@ int grid_capped(int64_t n, int block = kBlock) {
   return (int)g;
 }
 
-int sort_bits(int64_t max_key_exclusive) {
-  int b = 1;
-  while (b < 32 && ((int64_t)1 << b) < max_key_exclusive) ++b;
-  return b;
-}
-
-size_t pair_sort_temp_bytes(int64_t n) {
-  size_t bytes = 0;
-  cub::DoubleBuffer<uint32_t> k(nullptr, nullptr), v(nullptr, nullptr);
-  cub::DeviceRadixSort::SortPairs(nullptr, bytes, k, v, (int)n, 0, 32, (cudaStream_t)0);
-  return bytes;
-}
-
 }  // namespace
 
-// workspace layout shared by add and touch_lru: 2x keys, 2x vals, cub temp
-static size_t keyval_workspace_bytes(int64_t n) {
+static int alloc_batch_counters(hb_index* h, cudaStream_t st) {
+  if (h->batch) return HB_OK;
+  HB_CUDA(cudaMalloc(&h->batch, 8 * sizeof(int32_t)));
+  HB_CUDA(cudaMemsetAsync(h->batch, 0, 8 * sizeof(int32_t), st));
+  return HB_OK;
+}
+
+// (scratch is allocated on first use: do that outside any stream capture)
+int index_touch_marks(hb_index* h, TouchMarks* out, cudaStream_t st) {
+  if (!h->marks) {
+    const int rc = alloc_batch_counters(h, st);
+    if (rc != HB_OK) return rc;
+    HB_CUDA(cudaMalloc(&h->marks, h->cache_size * sizeof(unsigned long long)));
+    HB_CUDA(cudaMemsetAsync(h->marks, 0, h->cache_size * sizeof(unsigned long long), st));
+  }
+  *out = TouchMarks{h->marks, h->batch, h->cache_size};
+  return HB_OK;
+}
+
+int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st) {
+  TouchMarks marks;
+  const int rc = index_touch_marks(h, &marks, st);
+  if (rc != HB_OK) return rc;
+  HB_LAUNCH(touch_runs_apply_kernel, grid_capped(v.max_runs), kBlock, 0, st, v, marks, h->lru);
+  return HB_OK;
+}
+
+int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st) {
+  if (!h->heads) {
+    const int rc = alloc_batch_counters(h, st);
+    if (rc != HB_OK) return rc;
+    HB_CUDA(cudaMalloc(&h->heads, h->lines * sizeof(unsigned long long)));
+    HB_CUDA(cudaMemsetAsync(h->heads, 0, h->lines * sizeof(unsigned long long), st));
+  }
+  *out = AddLists{h->heads, h->batch + 2, next, h->lines};
+  return HB_OK;
+}
+
+int index_add_walk(hb_index* h, const AddEntries& e, const uint32_t* next, int64_t* locs, uint8_t* last_writer,
+                   cudaStream_t st) {
+  HB_LAUNCH(add_walk_kernel, grid_capped(e.n), kBlock, 0, st, e, h->heads, h->batch, next, h->lines,
+            h->line_ids, h->lru, locs, last_writer);
+  h->sorted_stale = true;
+  return HB_OK;
+}
+
+// One launch of the sort below kAddSortMax ids beats two of the lists; above, the lists, unless sets
+// get so many ids that putting a list in order takes longer than the sort.
+constexpr int64_t kAddSortMax = 16 * (int64_t)kClusterT;
+static bool add_sorts(int64_t n, int64_t lines) { return n <= kAddSortMax || n > 16 * lines; }
+
+static size_t add_workspace_bytes(int64_t n) {
   if (n <= 0) return 256;
-  size_t per = align_up((size_t)n * sizeof(uint32_t), 256);
-  return 4 * per + align_up(pair_sort_temp_bytes(n), 256) + 256;
+  return align_up((size_t)n * 4, 256) + align_up((size_t)n * sizeof(uint2), 256) + sort_grid_bytes(n) + 512;
 }
 
 }  // namespace hb
@@ -532,8 +728,11 @@ int hb_index_destroy(hb_index_t* h) {
   cudaFree(h->pairs);
   cudaFree(h->level_store);
   cudaFree(h->scratch_count);
-  cudaFree(h->slot_run);
-  cudaFree(h->slot_epoch);
+  cudaFree(h->marks);
+  cudaFree(h->after);
+  cudaFree(h->line_hits);
+  cudaFree(h->heads);
+  cudaFree(h->batch);
   delete h;
   return HB_OK;
 }
@@ -555,8 +754,8 @@ int hb_index_valid_entries(hb_index_t* h, int64_t* out_host, hb_stream_t stream)
   return HB_OK;
 }
 
-size_t hb_index_add_workspace_bytes(int64_t n) { return keyval_workspace_bytes(n); }
-size_t hb_index_touch_lru_workspace_bytes(int64_t n) { return keyval_workspace_bytes(n); }
+size_t hb_index_add_workspace_bytes(int64_t n) { return add_workspace_bytes(n); }
+size_t hb_index_touch_lru_workspace_bytes(int64_t) { return 256; }
 
 int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
                  uint8_t* last_writer, void* workspace, size_t workspace_bytes,
@@ -564,56 +763,79 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   HB_CHECK_ARG(h && (n == 0 || (ids && locs)), "hb_index_add: null argument");
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_index_add: n out of range");
   if (n == 0) return HB_OK;
-  if (workspace_bytes < keyval_workspace_bytes(n) || !workspace) {
-    set_error("hb_index_add: workspace of %zu bytes needed, %zu given", keyval_workspace_bytes(n),
-              workspace_bytes);
+  if (workspace_bytes < add_workspace_bytes(n) || !workspace) {
+    set_error("hb_index_add: workspace of %zu bytes needed, %zu given", add_workspace_bytes(n), workspace_bytes);
     return HB_ERR_WORKSPACE;
   }
   cudaStream_t st = (cudaStream_t)stream;
   Carver cv(workspace);
-  uint32_t* k0 = cv.take<uint32_t>(n);
-  uint32_t* k1 = cv.take<uint32_t>(n);
-  uint32_t* v0 = cv.take<uint32_t>(n);
-  uint32_t* v1 = cv.take<uint32_t>(n);
-  size_t temp_bytes = pair_sort_temp_bytes(n);
-  void* temp = cv.take<char>(temp_bytes);
-  HB_LAUNCH(add_keys_kernel, grid_for(n), kBlock, 0, st, ids, n, h->lines, k0, v0);
-  cub::DoubleBuffer<uint32_t> keys(k0, k1), vals(v0, v1);
-  HB_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, vals, (int)n, 0,
-                                          sort_bits(h->lines + 1), st));
-  count_library_launches(3);
-  HB_LAUNCH(add_walk_kernel, grid_for(n), kBlock, 0, st, ids, n, h->lines, keys.Current(),
-            vals.Current(), h->line_ids, h->lru, locs, last_writer);
   h->sorted_stale = true;
+  uint32_t* next = cv.take<uint32_t>(n);
+  uint2* sorted = cv.take<uint2>(n);
+  void* sort_ws = cv.take<char>(0);
+  if (!add_sorts(n, h->lines)) {
+    AddLists lists;
+    int rc = index_add_lists(h, next, &lists, st);
+    if (rc != HB_OK) return rc;
+    HB_LAUNCH(add_push_kernel, grid_for(n), kBlock, 0, st, ids, n, lists, locs, last_writer);
+    AddEntries e;
+    memset(&e, 0, sizeof(e));
+    e.ids = ids;
+    e.n = n;
+    rc = index_add_walk(h, e, next, locs, last_writer, st);
+    if (rc != HB_OK) return rc;
+    return sort_run(SetSource<true>{ids, n, h->lines, h->heads, h->batch},
+                    AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, n, sort_ws, st);
+  }
+  // (a cluster that holds more than one entry per thread leaves the walk to the whole GPU)
+  AddFinish fin{h->line_ids, h->lru, locs, last_writer, sorted, n > kAddSortMax && n <= kSortClusterMax};
+  const int rc = sort_run(SetSource<false>{ids, n, h->lines, nullptr, nullptr}, fin, n, sort_ws, st);
+  if (rc != HB_OK || !fin.walk_later) return rc;
+  HB_LAUNCH(add_sorted_walk_kernel, grid_for(n), kBlock, 0, st, ids, (int)n, fin);
   return HB_OK;
 }
 
-int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n, void* workspace,
-                       size_t workspace_bytes, hb_stream_t stream) {
+// lookup of `ids` into locs first (LOOKUP), or the slots given
+static int touch_positions(hb_index* h, const int64_t* ids, int64_t* locs, int64_t n, int mode, cudaStream_t st) {
+  TouchMarks t;
+  int rc = index_touch_marks(h, &t, st);
+  if (rc != HB_OK) return rc;
+  if (!h->after) {
+    HB_CUDA(cudaMalloc(&h->line_hits, h->lines * sizeof(int32_t)));
+    HB_CUDA(cudaMemsetAsync(h->line_hits, 0, h->lines * sizeof(int32_t), st));
+    HB_CUDA(cudaMalloc(&h->after, h->cache_size * sizeof(int32_t)));
+    HB_CUDA(cudaMemsetAsync(h->after, 0, h->cache_size * sizeof(int32_t), st));
+  }
+  const int grid = grid_capped(n);
+  if (!ids)
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits);
+  else if (mode == HB_LOOKUP_SORTED)
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SORTED, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits);
+  else
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits);
+  HB_LAUNCH(touch_after_kernel, grid, kBlock, 0, st, locs, n, t, h->after);
+  HB_LAUNCH(touch_apply_kernel, grid, kBlock, 0, st, locs, n, t, h->after, h->line_hits, h->lru);
+  return HB_OK;
+}
+
+int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n, void*, size_t, hb_stream_t stream) {
   HB_CHECK_ARG(h && (n == 0 || locs), "hb_index_touch_lru: null argument");
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_index_touch_lru: n out of range");
   if (n == 0) return HB_OK;
-  if (workspace_bytes < keyval_workspace_bytes(n) || !workspace) {
-    set_error("hb_index_touch_lru: workspace of %zu bytes needed, %zu given",
-              keyval_workspace_bytes(n), workspace_bytes);
-    return HB_ERR_WORKSPACE;
+  return touch_positions(h, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, (cudaStream_t)stream);
+}
+
+int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int mode,
+                          hb_stream_t stream) {
+  HB_CHECK_ARG(h && (n == 0 || (ids && locs)), "hb_index_lookup_touch: null argument");
+  HB_CHECK_ARG(mode == HB_LOOKUP_SETASSOC || mode == HB_LOOKUP_SORTED, "hb_index_lookup_touch: unknown mode %d", mode);
+  HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_index_lookup_touch: n out of range");
+  if (n == 0) return HB_OK;
+  if (mode == HB_LOOKUP_SORTED && h->sorted_stale) {
+    const int rc = hb_index_build_sorted(h, stream);
+    if (rc != HB_OK) return rc;
   }
-  cudaStream_t st = (cudaStream_t)stream;
-  Carver cv(workspace);
-  uint32_t* k0 = cv.take<uint32_t>(n);
-  uint32_t* k1 = cv.take<uint32_t>(n);
-  uint32_t* v0 = cv.take<uint32_t>(n);
-  uint32_t* v1 = cv.take<uint32_t>(n);
-  size_t temp_bytes = pair_sort_temp_bytes(n);
-  void* temp = cv.take<char>(temp_bytes);
-  HB_LAUNCH(touch_keys_kernel, grid_for(n), kBlock, 0, st, locs, n, h->cache_size, k0, v0);
-  cub::DoubleBuffer<uint32_t> keys(k0, k1), vals(v0, v1);
-  HB_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, vals, (int)n, 0,
-                                          sort_bits(h->cache_size + 1), st));
-  count_library_launches(3);
-  HB_LAUNCH(touch_apply_kernel, grid_for(n), kBlock, 0, st, keys.Current(), vals.Current(), n,
-            h->cache_size, h->lru);
-  return HB_OK;
+  return touch_positions(h, ids, locs, n, mode, (cudaStream_t)stream);
 }
 
 int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* perm,
@@ -626,21 +848,12 @@ int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* 
   HB_CHECK_ARG(locs_kind >= 0 && locs_kind <= 2, "hb_index_touch_lru_runs: locs_kind is 0, 1 or 2");
   if (n == 0 || max_runs == 0) return HB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int64_t cap = h->cache_size;
-  if (!h->slot_run) {
-    // first use (do it outside any stream capture): marks start at batch 0, the counter at 0
-    HB_CUDA(cudaMalloc(&h->slot_run, cap * sizeof(int32_t)));
-    HB_CUDA(cudaMalloc(&h->slot_epoch, (cap + 1) * sizeof(int32_t)));
-    HB_CUDA(cudaMemsetAsync(h->slot_epoch, 0, (cap + 1) * sizeof(int32_t), st));
-  }
-  int32_t* epoch_dev = h->slot_epoch + cap;  // the batch counter sits after the marks
+  TouchMarks marks;
+  const int rc = index_touch_marks(h, &marks, st);
+  if (rc != HB_OK) return rc;
   RunsView v{locs, perm, run_start, num_runs, n_dev, max_runs, n, locs_kind};
-  HB_LAUNCH(touch_runs_next_epoch_kernel, 1, 1, 0, st, epoch_dev);
-  HB_LAUNCH(touch_runs_mark_kernel, grid_for(max_runs), kBlock, 0, st, v, cap, epoch_dev, h->slot_run,
-            h->slot_epoch);
-  HB_LAUNCH(touch_runs_apply_kernel, grid_for(max_runs), kBlock, 0, st, v, cap, epoch_dev,
-            h->slot_run, h->slot_epoch, h->lru);
-  return HB_OK;
+  HB_LAUNCH(touch_runs_mark_kernel, grid_for(max_runs), kBlock, 0, st, v, marks);
+  return index_touch_apply(h, v, st);
 }
 
 int hb_index_lookup(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, uint8_t* found,

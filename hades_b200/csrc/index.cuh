@@ -15,6 +15,12 @@
 
 #include "common.cuh"
 
+#ifdef __CUDACC__
+#define HB_DEV __device__ __forceinline__
+#else
+#define HB_DEV inline
+#endif
+
 namespace hb {
 
 constexpr int kWays = HB_WAYS;
@@ -48,11 +54,14 @@ struct hb_index {
   int64_t level_off[hb::kMaxLevels];
   int64_t level_cap[hb::kMaxLevels];
   int64_t* scratch_count;      // device int64[4] for small reductions
-  // run-based LRU ageing: which run of the current batch hit a slot (valid when
-  // slot_epoch[slot] == the batch counter kept at slot_epoch[capacity]); allocated
-  // on first use.  The counter is 32 bits: 2^31 batches per index.
-  int32_t* slot_run;
-  int32_t* slot_epoch;
+  // scratch of add and of the LRU ageing, allocated on first use; entries are valid when their
+  // batch number is that of the batch at work, so nothing is cleared between batches (32 bits:
+  // 2^31 batches per index).  The batch numbers live on the device: a captured graph advances them.
+  unsigned long long* marks;    // [capacity] (batch << 32) | 1 + last position / run that hit the slot
+  int32_t* after;               // [capacity] hits on the line after the slot's last; zero between calls
+  int32_t* line_hits;           // [lines] zero between calls
+  unsigned long long* heads;    // [lines] (batch << 32) | 1 + entry: list of the batch's ids of a set
+  int32_t* batch;               // [8] touch: batch, blocks done; add: batch, blocks done, batch with long lists
   hb::IndexView view;
   // An index over another process's lines (hb_index_open): the sorted view is this process's
   // own and is rebuilt before every use, because the owner may have changed the lines since.
@@ -180,3 +189,105 @@ __device__ __forceinline__ int64_t warp_lookup(const IndexView& v, const int64_t
 
 }  // namespace hb
 #endif  // __CUDACC__
+
+namespace hb {
+
+#ifdef __CUDACC__
+// One batch number for all blocks of a kernel, advanced by the block that finishes last (every block
+// has read it by then): counter[0] batches so far, counter[1] blocks done.
+__device__ __forceinline__ uint32_t batch_number(const int32_t* counter) { return (uint32_t)*counter + 1u; }
+__device__ __forceinline__ void batch_done(int32_t* counter, uint32_t number) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(reinterpret_cast<unsigned*>(counter + 1), 1u) == gridDim.x - 1) {
+      counter[1] = 0;
+      counter[0] = (int32_t)number;
+    }
+  }
+}
+#endif
+
+// A batch grouped in runs of equal ids, as the LRU ageing sees it.
+struct RunsView {
+  const int64_t* locs;       // slot of every batch position (or of every sorted entry, see below)
+  const uint32_t* perm;      // nullable: position list of the runs (identity when null)
+  const int64_t* run_start;  // nullable: run u = [run_start[u], run_start[u+1]) (run u = {u} when null)
+  const int64_t* num_runs;   // nullable device count
+  const int64_t* n_dev;      // nullable device count of positions
+  int64_t max_runs;
+  int64_t n;
+  int locs_kind;             // locs holds a slot per batch position (0), per sorted entry (1), per run (2)
+  HB_DEV int64_t slot_of_run(int64_t u) const {
+    if (locs_kind == 2) return locs[u];
+    const int64_t j = start(u);
+    return locs[locs_kind == 1 ? j : pos(j)];
+  }
+  HB_DEV int64_t positions() const {
+    if (!n_dev) return n;
+    const int64_t d = *n_dev;
+    return d < n ? (d > 0 ? d : 0) : n;
+  }
+  HB_DEV int64_t runs() const {
+    int64_t r = max_runs;
+    if (num_runs && *num_runs < r) r = *num_runs;
+    if (!run_start) { const int64_t p = positions(); if (p < r) r = p; }
+    return r;
+  }
+  HB_DEV int64_t start(int64_t u) const { return run_start ? run_start[u] : u; }
+  HB_DEV int64_t end(int64_t u, int64_t nruns, int64_t npos) const {
+    return (u + 1 < nruns) ? start(u + 1) : npos;
+  }
+  HB_DEV int64_t pos(int64_t j) const { return perm ? (int64_t)perm[j] : j; }
+};
+
+// What a kernel that looks ids up leaves for the ageing of their hits (index_touch_apply).
+struct TouchMarks {
+  unsigned long long* marks;
+  int32_t* batch;
+  int64_t capacity;
+#ifdef __CUDACC__
+  __device__ __forceinline__ void mark(int64_t slot, int64_t run) const {
+    if (slot >= 0 && slot < capacity)
+      marks[slot] = ((unsigned long long)batch_number(batch) << 32) | (unsigned long long)(run + 1);
+  }
+#endif
+};
+
+// What a kernel that finds new ids leaves for their insertion (index_add_walk): entry i at the front
+// of the list of its set.
+struct AddLists {
+  unsigned long long* heads;
+  int32_t* batch;
+  uint32_t* next;   // [n] 1 + the entry behind this one, 0 = none
+  int64_t lines;
+#ifdef __CUDACC__
+  __device__ __forceinline__ void push(int64_t id, int64_t i) const {
+    const unsigned long long b = (unsigned long long)batch_number(batch) << 32;
+    const unsigned long long was = atomicExch(heads + mod_nonneg(id, lines), b | (unsigned long long)(i + 1));
+    next[i] = (was >> 32) == (b >> 32) ? (uint32_t)was : 0u;
+  }
+#endif
+};
+
+// Entries that were put on the lists: all n, or (a batch whose lookups missed) those at work[] with
+// at most `cap` of them taken, the first ones.
+struct AddEntries {
+  const int64_t* ids;            // [n] id of an entry
+  int64_t n;
+  const int64_t* n_dev;          // nullable: entries, on the device
+  const uint8_t* listed;         // nullable [n]: entry is on a list (else: non-negative ids are)
+  const int32_t* chunk_listed;   // nullable: listed entries of 32 at a time
+  const unsigned long long* total;  // their number
+  int64_t cap;
+};
+
+int index_touch_marks(hb_index* h, TouchMarks* out, cudaStream_t st);
+int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st);
+int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st);
+// slots into locs and "last writer of its slot" flags, for the listed entries; a listed entry beyond
+// the cap: -1 / 0
+int index_add_walk(hb_index* h, const AddEntries& e, const uint32_t* next, int64_t* locs, uint8_t* last_writer,
+                   cudaStream_t st);
+
+}  // namespace hb

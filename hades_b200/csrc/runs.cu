@@ -30,6 +30,7 @@ constexpr int kBlock = 256;
 // beyond their segment's count sort last.  So does a valid id that is negative or does not fit below
 // `sentinel` (2^id_bits - 1): it raises HB_ERR_INVALID in the device status word.
 struct IdSource {
+  static constexpr bool kSkips = false;
   const int64_t* ids;
   int64_t n;
   const int64_t* n_dev;

@@ -9,6 +9,8 @@
 //   scatter   to base[digit] + rank
 // so that equal keys keep the order of the input.
 //
+// (kSkips: a source that usually has nothing to sort; the launch then ends at once and writes nothing.)
+//
 // What bounds it: latency.  A batch of 65,536 ids is half a megabyte, one of 2,000,000 is 16 MB and
 // stays in L2; with one launch per pass the time goes into launches, cold starts and the chain of
 // look-backs.  So
@@ -327,6 +329,16 @@ struct ClusterCtx {
     sync();
     return true;
   }
+  // the sorted entries of all CTAs, read with __ldcg; buf: [count] in global memory
+  __device__ __forceinline__ const uint2* publish(uint2* buf) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int j = first() + i * 32;
+      if (j < count) __stcg(buf + j, s.kv[j - chunk_begin()]);
+    }
+    barrier();
+    return buf;
+  }
   // before a CTA leaves: no peer reads its shared memory any more
   __device__ __forceinline__ void leave() {
     if (ctas > 1) cg::this_cluster().sync();
@@ -356,6 +368,7 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
   ctx.rank = (int)cluster.block_rank();
   ctx.ctas = (int)cluster.num_blocks();
   const int n = (int)src.count();
+  if (Src::kSkips && n == 0) return;
   ctx.count = n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = ctx.first();
@@ -516,6 +529,7 @@ struct GridCtx {
     }
   }
   __device__ __forceinline__ uint2 get(int j) const { return __ldcg(kv + j); }
+  __device__ __forceinline__ const uint2* publish(uint2*) { return kv; }
   __device__ __forceinline__ bool barrier() {
     ++arrived;
     __syncthreads();
@@ -599,6 +613,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
   ctx.arrived = 0;
   ctx.alive = true;
   const int n = (int)src.count();
+  if (Src::kSkips && n == 0) return;
   ctx.count = n;
   {
     const int per = (n + ctx.ctas - 1) / ctx.ctas;

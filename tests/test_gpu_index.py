@@ -165,3 +165,34 @@ def test_touch_lru_from_runs(cuda_lib, oracle_mod, cache_size, id_range, n):
         ix.cuda_touch_lru_runs(locs, None, torch.tensor([uq.size], device="cuda"))
         assert np.array_equal(locs.cpu().numpy()[: uq.size], want)
         assert np.array_equal(ix.export_state()[1].cpu().numpy(), ora.export()[1]), rnd
+
+
+# one launch of the sort (up to 8,192 ids), the lists of the sets, the sort again for many ids per set
+# (more than 16 per set on average); sets with lists of up to 32 ids, longer ones, copies of one id
+@pytest.mark.parametrize("n,cache_size,kind", [(8192, 4000, "uniform"), (8193, 4000, "uniform"), (8193, 4104, "uniform"),
+                                               (70_000, 100_000, "uniform"), (70_000, 100_000, "copies"),
+                                               (20_000, 80_000, "strided"), (140_000, 800_000, "distinct"),
+                                               (9_000, 160, "uniform"), (66_000, 160, "uniform")])
+def test_add_and_lookup_of_large_batches(cuda_lib, oracle_mod, n, cache_size, kind):
+    rng = np.random.default_rng(n + cache_size)
+    gpu = GpuIndexAdapter(cache_size, 0)
+    ora = oracle_mod.OracleIndex(cache_size)
+    for step in range(3):
+        ids = rng.integers(0, 4 * cache_size, n, dtype=np.int64)
+        if kind == "copies":
+            ids[rng.random(n) < 0.3] = 12345 + step
+        elif kind == "strided":
+            ids[: n // 2] = rng.integers(0, 40, n // 2) * (cache_size // 8) * 3 + rng.integers(0, 50, n // 2)
+        elif kind == "distinct":
+            ids = rng.permutation(4 * cache_size)[:n].astype(np.int64)
+        ids[rng.integers(4, n, 5)] = -1  # padding
+        got, use = gpu.add(ids), ids >= 0
+        _eq(got[use], ora.add(ids[use]), (step, "add"))
+        assert (got[~use] == -1).all()
+        q = rng.integers(0, 4 * cache_size, n, dtype=np.int64)
+        q[rng.random(n) < 0.2] = ids[3]
+        _eq(gpu.lookup(q), ora.lookup(q), (step, "lookup"))
+        got_ids, got_lru = gpu.ix.export_state()
+        want_ids, want_lru = ora.export()
+        _eq(got_ids.cpu().numpy(), want_ids, (step, "ids"))
+        _eq(got_lru.cpu().numpy(), want_lru, (step, "lru"))
