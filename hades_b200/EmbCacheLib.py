@@ -546,23 +546,13 @@ def cudaBinarySearch2(input: torch.Tensor, range: torch.Tensor) -> torch.Tensor:
 def cudaLookupFetch(index: IndexCache, ids, cache_rows, backing_rows, out_rows=None,
                     mode: int | None = None, mover: int = MOVER_AUTO, want_locs: bool = True):
     """Fused IndexCache lookup + cached fetch: returns (out_rows, locs, found)."""
-    _check(ids.is_cuda and ids.dtype == torch.int64, "ids is a CUDA int64 tensor")
-    ids = ids.contiguous()
-    n = ids.numel()
-    if out_rows is None:
-        out_rows = torch.empty((n, cache_rows.size(1)), dtype=cache_rows.dtype, device=ids.device)
-    _check(out_rows.size(1) == cache_rows.size(1), "out_rows.size(1) == cache_rows.size(1)")
+    backing = 0
     if backing_rows is not None:
         _check(backing_rows.size(1) == cache_rows.size(1), "backing_rows.size(1) == cache_rows.size(1)")
-    locs = torch.empty(n, dtype=torch.int64, device=ids.device) if want_locs else None
-    found = torch.empty(n, dtype=torch.bool, device=ids.device)
-    lib = _lib.load()
-    _lib.check(lib.hb_lookup_fetch(index.handle, ids.data_ptr(), n, _dev_ptr(cache_rows, "cache_rows"),
-                                   None if backing_rows is None else _dev_ptr(backing_rows, "backing_rows"),
-                                   _row_bytes(cache_rows), out_rows.data_ptr(), _lib.ptr(locs),
-                                   found.data_ptr(), index.lookup_mode if mode is None else mode,
-                                   mover, _lib.stream_ptr()))
-    return out_rows, locs, found
+        backing = _dev_ptr(backing_rows, "backing_rows")
+    return (_lib._NATIVE or _lib.native()).lookup_fetch(
+        index._h.value, ids, cache_rows, _dev_ptr(cache_rows, "cache_rows"), backing, out_rows,
+        index.lookup_mode if mode is None else mode, mover, want_locs)
 
 
 def cudaAccumulate(src, dst, dst_index, cnt=None) -> None:
@@ -940,6 +930,8 @@ def cudaUniqueSegSum(ids, grads, cnt=None, mean: bool = False, id_bits: int = 64
     _check(grads.dtype == torch.float32 and grads.dim() == 2, "grads is a 2-D fp32 tensor")
     _check(grads.size(0) == ids.numel(), "grads.size(0) == ids.numel()")
     n, dim = ids.numel(), grads.size(1)
+    if sync and n and n_dev is None and seg_counts is None and not want_runs:
+        return (_lib._NATIVE or _lib.native()).unique_segsum(ids, grads, cnt, mean, id_bits)
     dev = ids.device
     uniq = torch.empty(n, dtype=torch.int64, device=dev)
     sums = torch.empty((n, dim), dtype=torch.float32, device=dev)

@@ -1,9 +1,10 @@
 """Build ``libhades_b200.so`` (the C-ABI library) in-tree with nvcc for sm_100a.
 
+(and ``_native``, the CPython extension that calls it on the hot paths.)
 ``python -m hades_b200._build`` or ``hades_b200._build.build()``.  Each ``csrc/*.cu``
 is compiled to an object under ``build/`` (skipped when up to date) and linked into
-``hades_b200/libhades_b200.so``.  No torch headers are involved: the library is plain
-CUDA behind ``include/hades_b200.h``.
+``hades_b200/libhades_b200.so``.  No torch headers are involved there: the library is plain
+CUDA behind ``include/hades_b200.h``; ``csrc/py/native.cpp`` is compiled against torch.
 """
 from __future__ import annotations
 
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -52,6 +54,32 @@ def _compile(src: Path, force: bool) -> tuple[Path, str]:
     return obj, r.stderr
 
 
+def native_path() -> Path:
+    return PKG / ("_native" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def _build_native(force: bool) -> None:
+    """The extension links against libhades_b200.so beside it (the one that ctypes loads too)."""
+    src, out = CSRC / "py" / "native.cpp", native_path()
+    header = ROOT / "include" / "hades_b200.h"
+    if not force and out.exists() and out.stat().st_mtime >= max(src.stat().st_mtime, header.stat().st_mtime):
+        return
+    import torch
+
+    tdir = Path(torch.__file__).parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    gxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else (shutil.which("g++") or "g++")
+    cmd = [gxx, "-O2", "-std=c++17", "-fPIC", "-shared", str(src), "-o", str(out),
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", str(ROOT / "include"), "-I", str(tdir / "include"), "-I", str(tdir / "include/torch/csrc/api/include"),
+           "-I", sysconfig.get_paths()["include"], "-I", str(cuda / "include"),
+           "-L", str(PKG), "-lhades_b200", "-L", str(tdir / "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-lc10", "-lc10_cuda", "-L", str(cuda / "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{gxx} failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+
+
 def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
@@ -75,6 +103,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_native(force)
     return LIB
 
 

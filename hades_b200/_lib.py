@@ -122,6 +122,13 @@ PROTOTYPES: dict[str, tuple] = {
     "hb_peer_table_destroy": (_int, [_p]),
     "hb_peer_table_gather": (_int, [_p, _p, _i64, _p, _p, _p]),
     "hb_lookup_fetch_sharded": (_int, [_p, _p, _i64, _p, _p, _p, _p, _p, _int, _p]),
+    "hb_step_create": (_int, [_p]),
+    "hb_step_destroy": (_int, [_p]),
+    "hb_step_supported": (_int, [_p]),
+    "hb_step_workspace_bytes": (_sz, [_i64, _i64]),
+    "hb_step_forward": (_int, [_p, _p, _p, _i64, _p, _p, _p, _p, _int, _p, _sz, _p]),
+    "hb_step_join": (_int, [_p, _p]),
+    "hb_step_backward": (_int, [_p, _p, _p, _i64, _p, _p, _p, _sz, _p]),
     "hb_fetch_serve": (_int, [_p, _p, _p, _p, _p, _i64, _p]),
 }
 
@@ -151,6 +158,15 @@ class StagingDesc(C.Structure):
     _fields_ = [("grad", _p), ("cnt", _p), ("idx", _p), ("iter_count", _p),
                 ("iter_threshold", _p), ("slots", _i64), ("dim", _i64)]
 
+
+class StepDesc(C.Structure):
+    """hb_step_desc_t"""
+    _fields_ = [("index", _p), ("staging", StagingDesc), ("cache_rows", _p), ("table", _p), ("table_rows", _i64),
+                ("row_bytes", _i64), ("dim", _i64), ("class_table", _p), ("class_len", _i64), ("id_bits", _int),
+                ("lookup_mode", _int), ("touch_lru", _int), ("insert_misses", _int), ("miss_cap", _i64),
+                ("threshold_table", _p), ("default_threshold", C.c_int32), ("dropped", _p), ("opt", OptimDesc)]
+
+
 _LIB: C.CDLL | None = None
 
 
@@ -174,6 +190,25 @@ def load() -> C.CDLL:
         fn.argtypes = args
     _LIB = lib
     return lib
+
+
+_NATIVE = None
+
+
+def native():
+    """The CPython extension over the same library (``csrc/py/native.cpp``); fails loudly when it has
+    not been built."""
+    global _NATIVE
+    if _NATIVE is None:
+        load()
+        try:
+            from . import _native
+        except ImportError as e:
+            raise RuntimeError("hades_b200._native is missing or does not load: build it with "
+                               "`python -m hades_b200._build`. hades_b200 has no CPU fallback.") from e
+        _native.set_error_class(HadesError)
+        _NATIVE = _native
+    return _NATIVE
 
 
 def check(rc: int) -> None:

@@ -195,6 +195,30 @@ __global__ void __launch_bounds__(kBlock) add_push_kernel(const int64_t* __restr
 
 constexpr int kListShort = 32;  // ids of a set that are put in order in a thread's own memory
 
+// Orders a long list (entry numbers + 1, linked through next) ascending: merge sort, bottom up.
+__device__ __noinline__ uint32_t sort_list(uint32_t head, uint32_t* next) {
+  for (uint32_t size = 1;; size *= 2) {
+    uint32_t p = head, tail = 0;
+    head = 0;
+    int merges = 0;
+    while (p) {
+      ++merges;
+      uint32_t q = p, np = 0, nq = size;
+      while (np < size && q) { ++np; q = next[q - 1]; }
+      while (np || (nq && q)) {
+        uint32_t e;
+        if (np && (!nq || !q || p < q)) { e = p; p = next[p - 1]; --np; }
+        else { e = q; q = next[q - 1]; --nq; }
+        if (tail) next[tail - 1] = e; else head = e;
+        tail = e;
+      }
+      p = q;
+    }
+    next[tail - 1] = 0;
+    if (merges <= 1) return head;
+  }
+}
+
 // where the first `cap` listed entries end (a block finds it together); the usual case: nothing to cut
 __device__ __forceinline__ int64_t add_cut(const AddEntries& e, int64_t n) {
   __shared__ long long s_cut[2];
@@ -228,10 +252,9 @@ __device__ __forceinline__ int64_t add_cut(const AddEntries& e, int64_t n) {
       int x = 0;
       while (need >= __ldg(e.chunk_listed + c + x)) { need -= __ldg(e.chunk_listed + c + x); ++x; }
       int64_t i = (c + x) * 32;
-      while (true) {
-        if (e.listed[i]) { if (need == 0) break; --need; }
-        ++i;
-      }
+      const int64_t end = i + 32 < n ? i + 32 : n;
+      for (; i < end; ++i)
+        if (e.listed[i] && need-- == 0) break;
       s_cut[0] = i;
     }
     __syncthreads();
@@ -243,8 +266,30 @@ __device__ __forceinline__ int64_t add_cut(const AddEntries& e, int64_t n) {
   return n;
 }
 
+// the runs of a batch that are on lists, sorted by set instead (many ids per set)
+struct ListedSource {
+  static constexpr bool kSkips = false;
+  const int64_t* ids;
+  int64_t n;
+  const int64_t* n_dev;
+  const uint8_t* listed;
+  const int64_t* cut;
+  int64_t lines;
+  __device__ __forceinline__ int64_t count() const { return *n_dev < n ? *n_dev : n; }
+  __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
+    key = (unsigned long long)mod_nonneg(__ldg(ids + i), lines);
+    return listed[i] && i < *cut;
+  }
+};
+
+__global__ void __launch_bounds__(kBlock) add_cut_kernel(AddEntries e, int64_t* cut) {
+  const int64_t c = add_cut(e, *e.n_dev < e.n ? *e.n_dev : e.n);
+  if (threadIdx.x == 0) *cut = c;
+}
+
+template <bool DISTINCT>
 __global__ void __launch_bounds__(kBlock) add_walk_kernel(AddEntries e, unsigned long long* __restrict__ heads,
-                                                          int32_t* batch, const uint32_t* __restrict__ next, int64_t lines,
+                                                          int32_t* batch, uint32_t* __restrict__ next, int64_t lines,
                                                           int64_t* __restrict__ line_ids, int32_t* __restrict__ lru,
                                                           int64_t* __restrict__ locs, uint8_t* __restrict__ last_writer) {
   const uint32_t number = batch_number(batch + 2);
@@ -276,6 +321,22 @@ __global__ void __launch_bounds__(kBlock) add_walk_kernel(AddEntries e, unsigned
       int k = len++;
       for (; k > 0 && order[k - 1] > at; --k) order[k] = order[k - 1];
       order[k] = at;
+    }
+    if (at && DISTINCT) {
+      // only ids in strides of the number of sets come here: no launch is kept ready for them
+      const uint32_t first = sort_list((uint32_t)i + 1u, next);
+      int k = 0;
+      for (at = first; at; at = next[at - 1], ++k) {
+        const int64_t x = (int64_t)at - 1;
+        const int way = x < cut ? st.place(__ldg(e.ids + x), k) : -1;
+        locs[x] = way >= 0 ? line * kWays + way : -1;
+      }
+      if (last_writer) {
+        k = 0;
+        for (at = first; at; at = next[at - 1], ++k) last_writer[at - 1] = st.is_last(locs[at - 1], k);
+      }
+      st.store(line_ids, lru, line);
+      continue;
     }
     if (at) {
       heads[line] = ((unsigned long long)number << 32) | kLongList;
@@ -595,22 +656,33 @@ int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st)
   return HB_OK;
 }
 
-int index_add_walk(hb_index* h, const AddEntries& e, const uint32_t* next, int64_t* locs, uint8_t* last_writer,
-                   cudaStream_t st) {
-  HB_LAUNCH(add_walk_kernel, grid_capped(e.n), kBlock, 0, st, e, h->heads, h->batch, next, h->lines,
-            h->line_ids, h->lru, locs, last_writer);
-  h->sorted_stale = true;
-  return HB_OK;
-}
-
-// One launch of the sort below kAddSortMax ids beats two of the lists; above, the lists, unless sets
-// get so many ids that putting a list in order takes longer than the sort.
+// Where sets may get more ids than this on average, putting lists in order takes longer than the sort.
+constexpr int64_t kListedPerSet = 16;
+// One launch of the sort beats the launches of the lists up to one id per thread of the largest cluster.
 constexpr int64_t kAddSortMax = 16 * (int64_t)kClusterT;
-static bool add_sorts(int64_t n, int64_t lines) { return n <= kAddSortMax || n > 16 * lines; }
 
 static size_t add_workspace_bytes(int64_t n) {
   if (n <= 0) return 256;
-  return align_up((size_t)n * 4, 256) + align_up((size_t)n * sizeof(uint2), 256) + sort_grid_bytes(n) + 512;
+  return align_up((size_t)n * 4, 256) + align_up((size_t)n * sizeof(uint2), 256) + sort_grid_bytes(n) + 1024;
+}
+
+size_t index_add_runs_bytes(int64_t n) { return add_workspace_bytes(n); }
+bool index_add_runs_lists(const hb_index* h, int64_t n) { return n <= kListedPerSet * h->lines; }
+
+int index_add_runs(hb_index* h, const AddEntries& e, void* ws, int64_t* locs, uint8_t* last_writer, cudaStream_t st) {
+  Carver cv(ws);
+  uint32_t* next = cv.take<uint32_t>(e.n);
+  h->sorted_stale = true;
+  if (index_add_runs_lists(h, e.n)) {
+    HB_LAUNCH(add_walk_kernel<true>, grid_capped(e.n), kBlock, 0, st, e, h->heads, h->batch, next, h->lines,
+              h->line_ids, h->lru, locs, last_writer);
+    return HB_OK;
+  }
+  uint2* sorted = cv.take<uint2>(e.n);
+  int64_t* cut = cv.take<int64_t>(1);
+  HB_LAUNCH(add_cut_kernel, 1, kBlock, 0, st, e, cut);
+  return sort_run(ListedSource{e.ids, e.n, e.n_dev, e.listed, cut, h->lines},
+                  AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, e.n, cv.take<char>(0), st);
 }
 
 }  // namespace hb
@@ -773,7 +845,7 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   uint32_t* next = cv.take<uint32_t>(n);
   uint2* sorted = cv.take<uint2>(n);
   void* sort_ws = cv.take<char>(0);
-  if (!add_sorts(n, h->lines)) {
+  if (n > kAddSortMax && n <= kListedPerSet * h->lines) {
     AddLists lists;
     int rc = index_add_lists(h, next, &lists, st);
     if (rc != HB_OK) return rc;
@@ -782,8 +854,8 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
     memset(&e, 0, sizeof(e));
     e.ids = ids;
     e.n = n;
-    rc = index_add_walk(h, e, next, locs, last_writer, st);
-    if (rc != HB_OK) return rc;
+    HB_LAUNCH(add_walk_kernel<false>, grid_capped(n), kBlock, 0, st, e, h->heads, h->batch, next, h->lines, h->line_ids,
+              h->lru, locs, last_writer);
     return sort_run(SetSource<true>{ids, n, h->lines, h->heads, h->batch},
                     AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, n, sort_ws, st);
   }

@@ -285,9 +285,11 @@ struct AddEntries {
 int index_touch_marks(hb_index* h, TouchMarks* out, cudaStream_t st);
 int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st);
 int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st);
-// slots into locs and "last writer of its slot" flags, for the listed entries; a listed entry beyond
-// the cap: -1 / 0
-int index_add_walk(hb_index* h, const AddEntries& e, const uint32_t* next, int64_t* locs, uint8_t* last_writer,
-                   cudaStream_t st);
+// add() of the distinct ids of a batch that `listed` names: slots into locs and "last writer of its
+// slot" flags for them; beyond the cap -1 / 0.  Where index_add_runs_lists says so the lists have been
+// filled before (AddLists, `next` at the start of the workspace).
+size_t index_add_runs_bytes(int64_t n);
+bool index_add_runs_lists(const hb_index* h, int64_t n);
+int index_add_runs(hb_index* h, const AddEntries& e, void* ws, int64_t* locs, uint8_t* last_writer, cudaStream_t st);
 
 }  // namespace hb

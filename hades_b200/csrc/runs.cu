@@ -76,6 +76,8 @@ struct RunsFinish {
   int64_t* class_counts2;
   int32_t* base8;        // [ceil(n / 8)] runs that start before entry 8k
   int64_t* n_valid;      // number of valid entries of a segmented input
+  unsigned* zero;        // nullable: words that the next launch needs at zero
+  int zero_words;
 
   template <class Ctx>
   __device__ __forceinline__ void run(Ctx& ctx, const IdSource& src) const {
@@ -83,6 +85,7 @@ struct RunsFinish {
     __shared__ int4 s_sum[2 * W + 1];
     __shared__ unsigned long long s_valid;
     const int lane = threadIdx.x & 31;
+    for (int k = ctx.rank * T + threadIdx.x; k < zero_words; k += ctx.ctas * T) zero[k] = 0u;
     int ne = ctx.count;
     if (src.seg_counts) {
       // valid entries are scattered over the segments; their number becomes the device count
@@ -458,25 +461,25 @@ template <bool PEER, int RB>
 __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
     hb_runs_t r, const unsigned long long* __restrict__ run_src, const int64_t* __restrict__ run_slots,
     int64_t row_bytes_arg, int vb, char* __restrict__ out, int64_t* __restrict__ locs,
-    uint8_t* __restrict__ found) {
+    uint8_t* __restrict__ found, int per) {
   constexpr bool V16 = RB != 0;
   const int64_t row_bytes = RB == 512 ? (int64_t)512 : row_bytes_arg;
   const int64_t n = runs_valid_entries(r);
   const int lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * 32;
-  int64_t base = warp * 32;
+  const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * per;
+  int64_t base = warp * per;
   uint32_t pos_next = 0;
   int64_t run_next = -1;
-  if (base + lane < n) {
+  if (lane < per && base + lane < n) {
     pos_next = __ldg(r.perm + base + lane);
     run_next = run_of_entry(r, base + lane);
   }
   for (; base < n; base += stride) {
-    const bool valid = base + lane < n;
+    const bool valid = lane < per && base + lane < n;
     const uint32_t pos = pos_next;
     const int64_t u = valid ? run_next : -1;
-    if (base + stride + lane < n) {
+    if (lane < per && base + stride + lane < n) {
       pos_next = __ldg(r.perm + base + stride + lane);
       run_next = run_of_entry(r, base + stride + lane);
     }
@@ -495,7 +498,7 @@ __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
         const bool on = RB == 512 || lane < vpr;
         uint4 last = make_uint4(0, 0, 0, 0);
         constexpr int kFly = RB == 512 ? 8 : 4;  // rows whose loads are in flight together
-        for (int q0 = 0; q0 < 32; q0 += kFly) {
+        for (int q0 = 0; q0 < per; q0 += kFly) {
           if (((have >> q0) & ((1u << kFly) - 1u)) == 0u) continue;
           uint4 val[kFly];
           uint32_t pq[kFly];
@@ -517,7 +520,7 @@ __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
           }
         }
       } else {
-        for (int q0 = 0; q0 < 32; q0 += 4) {
+        for (int q0 = 0; q0 < per; q0 += 4) {
           if (((have >> q0) & 0xfu) == 0u) continue;
           const uint4* sp[4];
           uint4* dp[4];
@@ -542,7 +545,7 @@ __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
       }
     } else {
       // rows that are not a multiple of 16 bytes (or unaligned buffers): words or bytes
-      for (int q = 0; q < 32; ++q) {
+      for (int q = 0; q < per; ++q) {
         const unsigned long long sb = __shfl_sync(0xffffffffu, src_bits, q);
         const uint32_t pq = __shfl_sync(0xffffffffu, pos, q);
         if (!((have >> q) & 1u)) continue;
@@ -625,6 +628,18 @@ int hb_runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int
                   int64_t* const* class_ids_out, int64_t* class_counts_out, int64_t* uniq_ids_out,
                   int64_t* num_unique_out, void* workspace, size_t workspace_bytes,
                   hb_runs_t* runs_out, hb_stream_t stream) {
+  return runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, class_table, table_len, class_ids_out,
+                    class_counts_out, uniq_ids_out, num_unique_out, nullptr, 0, workspace, workspace_bytes, runs_out,
+                    (cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int64_t* seg_counts, int64_t seg_cap,
+                   int id_bits, const int8_t* class_table, int64_t table_len, int64_t* const* class_ids_out,
+                   int64_t* class_counts_out, int64_t* uniq_ids_out, int64_t* num_unique_out, unsigned* zero,
+                   int64_t zero_words, void* workspace, size_t workspace_bytes, hb_runs_t* runs_out,
+                   cudaStream_t st) {
   HB_CHECK_ARG(runs_out != nullptr, "hb_runs_build: runs_out is null");
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_runs_build: n out of range");
   HB_CHECK_ARG(n == 0 || ids, "hb_runs_build: null ids");
@@ -637,7 +652,6 @@ int hb_runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int
     set_error("hb_runs_build: workspace of %zu bytes needed, %zu given", s.total, workspace_bytes);
     return HB_ERR_WORKSPACE;
   }
-  cudaStream_t st = (cudaStream_t)stream;
   memset(runs_out, 0, sizeof(*runs_out));
   runs_out->n = n;
   runs_out->num_runs = s.num_runs;
@@ -665,9 +679,12 @@ int hb_runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int
                  s.dclass, s.dpos,
                  {class_ids_out ? class_ids_out[0] : nullptr, class_ids_out ? class_ids_out[1] : nullptr,
                   class_ids_out ? class_ids_out[2] : nullptr},
-                 s.num_runs, num_unique_out, s.class_counts, class_counts_out, s.base8, s.n_valid};
+                 s.num_runs, num_unique_out, s.class_counts, class_counts_out, s.base8, s.n_valid, zero,
+                 (int)zero_words};
   return sort_run(src, fin, n, s.sort_ws, st);
 }
+
+extern "C" {
 
 namespace {
 // scratch of hb_lookup_fetch_runs: where every run's row is read from, the slot of every run
@@ -812,12 +829,11 @@ int fetch_runs_impl(hb_index_t* h, const hb_runs_t* runs, const void* cache_rows
     if (rc != HB_OK) return rc;
   }
   if (!expand) return HB_OK;  // per distinct id only: slots in run_slots, remote rows staged or asked for
-  int64_t blocks = ceil_div(ceil_div(runs->n, 32) * 32, kBlock);
-  if (blocks > (int64_t)sm_count() * 32) blocks = (int64_t)sm_count() * 32;
-  const int grid = (int)(blocks < 1 ? 1 : blocks);
+  const int per = items_per_warp(runs->n);
+  const int grid = grid_of_warps(runs->n, per, kBlock, 32);
 #define HB_EXP(PEER, RB)                                                                         \
   HB_LAUNCH((runs_expand_kernel<PEER, RB>), grid, kBlock, 0, st, *runs, f.run_src, slots, row_bytes, \
-            vb, (char*)out_rows, locs, found)
+            vb, (char*)out_rows, locs, found, per)
 #define HB_EXP_V(PEER)                                \
   do {                                                \
     if (v16 && row_bytes == 512) HB_EXP(PEER, 512);   \

@@ -25,6 +25,12 @@ struct RunsPlan {
 
 RunsPlan make_runs_plan(void* ws, int64_t n);
 
+// hb_runs_build; zero: words that the launch after it needs at zero (set by the sort's own launch)
+int runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int64_t* seg_counts, int64_t seg_cap,
+               int id_bits, const int8_t* class_table, int64_t table_len, int64_t* const* class_ids_out,
+               int64_t* class_counts_out, int64_t* uniq_ids_out, int64_t* num_unique_out, unsigned* zero,
+               int64_t zero_words, void* workspace, size_t workspace_bytes, hb_runs_t* runs_out, cudaStream_t st);
+
 #ifdef __CUDACC__
 __device__ __forceinline__ int64_t runs_valid_entries(const hb_runs_t& r) {
   if (!r.n_dev) return r.n;

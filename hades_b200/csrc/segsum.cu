@@ -14,6 +14,15 @@ size_t hb_segsum_runs_workspace_bytes(int64_t n, int64_t dim) { return seg_plan(
 int hb_segsum_runs_f32(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim,
                        int mean, float* sums, int64_t* counts, const hb_class_split_t* split,
                        void* workspace, size_t workspace_bytes, hb_stream_t stream) {
+  return segsum_runs(runs, grads, cnt_in, dim, mean, sums, counts, split, workspace, workspace_bytes, false,
+                     (cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+int hb::segsum_runs(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean,
+                    float* sums, int64_t* counts, const hb_class_split_t* split, void* workspace,
+                    size_t workspace_bytes, bool zeroed, cudaStream_t st) {
   HB_CHECK_ARG(runs != nullptr && dim > 0, "hb_segsum_runs_f32: bad argument");
   const int64_t n = runs->n;
   HB_CHECK_ARG(n == 0 || (grads && runs->perm && runs->head && runs->base8 && runs->run_start && runs->num_runs),
@@ -22,7 +31,6 @@ int hb_segsum_runs_f32(const hb_runs_t* runs, const float* grads, const int64_t*
   HB_CHECK_ARG(!split || n == 0 || (runs->dclass && runs->dpos),
                "hb_segsum_runs_f32: a split needs runs built with the class table");
   if (n == 0) return HB_OK;
-  cudaStream_t st = (cudaStream_t)stream;
   SegPlan s = seg_plan(workspace, n, dim);
   if (!workspace || workspace_bytes < s.total) {
     set_error("hb_segsum_runs_f32: workspace of %zu bytes needed, %zu given", s.total, workspace_bytes);
@@ -42,7 +50,7 @@ int hb_segsum_runs_f32(const hb_runs_t* runs, const float* grads, const int64_t*
     epi.class_rows[c] = split ? split->out_rows[c] : nullptr;
     epi.class_counts[c] = split ? split->out_cnt[c] : nullptr;
   }
-  HB_CUDA(cudaMemsetAsync(s.done, 0, (size_t)s.max_ctas * sizeof(unsigned), st));
+  if (!zeroed) HB_CUDA(cudaMemsetAsync(s.done, 0, (size_t)s.max_ctas * sizeof(unsigned), st));
   const int tile = seg_tile(vec4);
   for (int64_t col0 = 0; col0 < dim; col0 += tile) {
     a.col0 = col0;
@@ -52,6 +60,8 @@ int hb_segsum_runs_f32(const hb_runs_t* runs, const float* grads, const int64_t*
   }
   return HB_OK;
 }
+
+extern "C" {
 
 size_t hb_unique_segsum_workspace_bytes(int64_t n, int64_t dim) {
   return align_up(hb_runs_workspace_bytes(n), 256) + seg_plan(nullptr, n, dim).total;
@@ -79,15 +89,15 @@ int hb_unique_segsum_f32(const int64_t* ids, const float* grads, const int64_t* 
   hb_runs_t runs;
   int64_t* cls_ids[3] = {split ? split->out_ids[0] : nullptr, split ? split->out_ids[1] : nullptr,
                          split ? split->out_ids[2] : nullptr};
-  int rc = hb_runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, split ? split->table : nullptr,
-                         split ? split->table_len : 0, split ? cls_ids : nullptr,
-                         split ? split->class_counts : nullptr, uniq_ids, num_unique, workspace,
-                         runs_bytes, &runs, stream);
+  char* seg_ws = static_cast<char*>(workspace) + runs_bytes;
+  const SegPlan s = seg_plan(seg_ws, n, dim);
+  int rc = runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, split ? split->table : nullptr,
+                      split ? split->table_len : 0, split ? cls_ids : nullptr, split ? split->class_counts : nullptr,
+                      uniq_ids, num_unique, s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream);
   if (rc != HB_OK) return rc;
   if (runs_out) *runs_out = runs;
-  return hb_segsum_runs_f32(&runs, grads, cnt_in, dim, mean, sums, counts, split,
-                            static_cast<char*>(workspace) + runs_bytes, workspace_bytes - runs_bytes,
-                            stream);
+  return segsum_runs(&runs, grads, cnt_in, dim, mean, sums, counts, split, seg_ws, workspace_bytes - runs_bytes, true,
+                     (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -49,9 +49,15 @@ struct SegArgs {
   unsigned* done;             // [CTAs] zero before and after: arrivals of the run that begins in the CTA
 };
 
+// hb_segsum_runs_f32; zeroed: the arrival counters are at zero already
+int segsum_runs(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean, float* sums,
+                int64_t* counts, const hb_class_split_t* split, void* workspace, size_t workspace_bytes, bool zeroed,
+                cudaStream_t st);
+
 // ---- epilogues ---------------------------------------------------------------------------------
 // The sums and counts as they are, or the buffers of the id's class.
 struct StoreRows {
+  static constexpr bool kWeights = true;
   float* sums;                // [U][dim] (null when the rows go to class buffers)
   const int8_t* dclass;       // [U], null = no split
   const int32_t* dpos;        // [U]
@@ -65,6 +71,7 @@ struct StoreRows {
 // 2^30 rows and slots.
 template <bool ADAM, bool STEP>
 struct UpdateRows {
+  static constexpr bool kWeights = !STEP;  // rows with weights come from several senders
   const int64_t* uniq;        // [U] ids
   RowMap map;
   int half;                   // fp16 rows
@@ -78,6 +85,24 @@ struct UpdateRows {
   float* staged;              // [slots][dim]
   const int64_t* slots;       // [U] staging slot of a cold run, -1 = none
 };
+
+template <bool ADAM, bool STEP>
+UpdateRows<ADAM, STEP> update_rows(const hb_runs_t* runs, const hb_optim_t* opt) {
+  UpdateRows<ADAM, STEP> epi;
+  epi.uniq = runs->uniq_ids;
+  epi.map = RowMap{opt->id_offset, opt->id_stride, opt->rows};
+  epi.half = opt->emb_elem_bytes == 2;
+  epi.step = opt->step;
+  epi.s0 = opt->s0;
+  epi.s1 = opt->s1;
+  epi.emb = opt->emb;
+  epi.p = AdamParams{(float)opt->lr, (float)opt->beta1, (float)opt->beta2, (float)opt->eps,
+                     (float)(1.0 - opt->beta1), (float)(1.0 - opt->beta2)};
+  epi.dclass = nullptr;
+  epi.staged = nullptr;
+  epi.slots = nullptr;
+  return epi;
+}
 
 #ifdef __CUDACC__
 
@@ -200,13 +225,15 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
   };
   static __device__ __forceinline__ bool is_staged(int row) { return STEP && row >= kStaged; }
   static __device__ __forceinline__ Lane lane(const Epi& o, int run) {
-    Lane l;
     const int c = STEP ? o.dclass[run] : 1;
+    return lane_of_class(o, c, o.uniq[run], STEP && c == 2 ? o.slots[run] : -1);
+  }
+  static __device__ __forceinline__ Lane lane_of_class(const Epi& o, int c, int64_t id, int64_t slot) {
+    Lane l;
     if (STEP && c == 2) {
-      const int64_t slot = o.slots[run];
       if (slot >= 0) l.row = kStaged + (int)slot;
     } else if (c == 1) {
-      l.row = (int)o.map(o.uniq[run]);
+      l.row = (int)o.map(id);
       if (ADAM && l.row >= 0) {
         // state_step = state_step + 1 (per row), sparse_optim.py:624-626
         l.t = o.step[l.row] + 1.0f;
@@ -244,14 +271,15 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
       }
     }
   }
-  // by all lanes of the warp: the run that ends at the entry of lane `src` of each group
+  // by all lanes of the warp: the run that ends at the entry of lane `src` of each W lanes
+  template <int W = G>
   static __device__ __forceinline__ void fetch(const Epi& o, const SegArgs& a, const Lane& l, int src, bool ends, int sub,
                                                int vpr, Row& r) {
-    r.row = __shfl_sync(0xffffffffu, l.row, src, G);
+    r.row = __shfl_sync(0xffffffffu, l.row, src, W);
     if (ADAM) {
-      r.t = __shfl_sync(0xffffffffu, l.t, src, G);
-      r.ra = __shfl_sync(0xffffffffu, l.ra, src, G);
-      r.rb = __shfl_sync(0xffffffffu, l.rb, src, G);
+      r.t = __shfl_sync(0xffffffffu, l.t, src, W);
+      r.ra = __shfl_sync(0xffffffffu, l.ra, src, W);
+      r.rb = __shfl_sync(0xffffffffu, l.rb, src, W);
     }
     if (ends) load(o, a, sub, vpr, r);
   }
@@ -603,10 +631,13 @@ int seg_launch(SegArgs a, const Epi& epi, cudaStream_t st) {
   const int ng = kSegBlock / G;
   const int grid = (int)ceil_div(a.n, (int64_t)ng * a.piece);
   const size_t smem = (size_t)ng * a.cols * sizeof(float);
-  if (a.cnt_in)
-    HB_LAUNCH((segsum_kernel<VEC, G, VPL, true, Epi>), grid, kSegBlock, smem, st, a, epi);
-  else
-    HB_LAUNCH((segsum_kernel<VEC, G, VPL, false, Epi>), grid, kSegBlock, smem, st, a, epi);
+  if constexpr (Epi::kWeights) {
+    if (a.cnt_in) {
+      HB_LAUNCH((segsum_kernel<VEC, G, VPL, true, Epi>), grid, kSegBlock, smem, st, a, epi);
+      return HB_OK;
+    }
+  }
+  HB_LAUNCH((segsum_kernel<VEC, G, VPL, false, Epi>), grid, kSegBlock, smem, st, a, epi);
   return HB_OK;
 }
 

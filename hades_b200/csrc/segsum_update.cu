@@ -4,36 +4,12 @@
 // the launches and the unique count between the two.
 #include "segsum.cuh"
 
-namespace hb {
-namespace {
-
-template <bool ADAM>
-UpdateRows<ADAM, false> update_rows(const hb_runs_t* runs, const hb_optim_t* opt) {
-  UpdateRows<ADAM, false> epi;
-  epi.uniq = runs->uniq_ids;
-  epi.map = RowMap{opt->id_offset, opt->id_stride, opt->rows};
-  epi.half = opt->emb_elem_bytes == 2;
-  epi.step = opt->step;
-  epi.s0 = opt->s0;
-  epi.s1 = opt->s1;
-  epi.emb = opt->emb;
-  epi.p = AdamParams{(float)opt->lr, (float)opt->beta1, (float)opt->beta2, (float)opt->eps,
-                     (float)(1.0 - opt->beta1), (float)(1.0 - opt->beta2)};
-  epi.dclass = nullptr;
-  epi.staged = nullptr;
-  epi.slots = nullptr;
-  return epi;
-}
-
-}  // namespace
-}  // namespace hb
-
 using namespace hb;
 
-extern "C" {
+namespace {
 
-int hb_segsum_update_f32(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean,
-                         const hb_optim_t* opt, void* workspace, size_t workspace_bytes, hb_stream_t stream) {
+int segsum_update(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean,
+                  const hb_optim_t* opt, void* workspace, size_t workspace_bytes, bool zeroed, cudaStream_t st) {
   HB_CHECK_ARG(runs != nullptr && opt != nullptr && dim > 0, "hb_segsum_update_f32: bad argument");
   const int64_t n = runs->n;
   HB_CHECK_ARG(n == 0 || (grads && runs->perm && runs->head && runs->base8 && runs->run_start && runs->uniq_ids),
@@ -61,12 +37,20 @@ int hb_segsum_update_f32(const hb_runs_t* runs, const float* grads, const int64_
     set_error("hb_segsum_update_f32: workspace of %zu bytes needed, %zu given", s.total, workspace_bytes);
     return HB_ERR_WORKSPACE;
   }
-  cudaStream_t st = (cudaStream_t)stream;
   SegArgs a = seg_args(runs, grads, cnt_in, dim, mean, s);
   a.cols = (int)dim;
-  HB_CUDA(cudaMemsetAsync(s.done, 0, (size_t)s.max_ctas * sizeof(unsigned), st));
-  if (opt->kind == HB_OPT_ADAM) return seg_dispatch(a, update_rows<true>(runs, opt), vec4, st);
-  return seg_dispatch(a, update_rows<false>(runs, opt), vec4, st);
+  if (!zeroed) HB_CUDA(cudaMemsetAsync(s.done, 0, (size_t)s.max_ctas * sizeof(unsigned), st));
+  if (opt->kind == HB_OPT_ADAM) return seg_dispatch(a, update_rows<true, false>(runs, opt), vec4, st);
+  return seg_dispatch(a, update_rows<false, false>(runs, opt), vec4, st);
+}
+
+}  // namespace
+
+extern "C" {
+
+int hb_segsum_update_f32(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean,
+                         const hb_optim_t* opt, void* workspace, size_t workspace_bytes, hb_stream_t stream) {
+  return segsum_update(runs, grads, cnt_in, dim, mean, opt, workspace, workspace_bytes, false, (cudaStream_t)stream);
 }
 
 int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* cnt_in, int64_t n, const int64_t* n_dev,
@@ -79,12 +63,14 @@ int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* 
               runs_bytes + hb_segsum_runs_workspace_bytes(n, dim), workspace_bytes);
     return HB_ERR_WORKSPACE;
   }
+  char* seg_ws = static_cast<char*>(workspace) + runs_bytes;
+  const SegPlan s = seg_plan(seg_ws, n, dim);
   hb_runs_t runs;
-  int rc = hb_runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
-                         workspace, runs_bytes, &runs, stream);
+  int rc = runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
+                      s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream);
   if (rc != HB_OK) return rc;
-  return hb_segsum_update_f32(&runs, grads, cnt_in, dim, mean, opt, static_cast<char*>(workspace) + runs_bytes,
-                              workspace_bytes - runs_bytes, stream);
+  return segsum_update(&runs, grads, cnt_in, dim, mean, opt, seg_ws, workspace_bytes - runs_bytes, true,
+                       (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "partition_core.cuh"
+#include "staging.cuh"
 
 namespace hb {
 namespace {
@@ -72,7 +73,7 @@ template <int MODE, int VEC>
 __global__ void __launch_bounds__(kBlock) staging_accumulate_cached_kernel(
     IndexView v, hb_staging_t s, const int64_t* __restrict__ ids, const float* __restrict__ grads,
     int64_t n, const int64_t* __restrict__ n_dev, const int32_t* __restrict__ thr_table,
-    int32_t default_thr, unsigned long long* __restrict__ dropped, int64_t* __restrict__ locs_out) {
+    int32_t default_thr, unsigned long long* __restrict__ dropped, int64_t* __restrict__ locs_out, int per) {
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -82,8 +83,8 @@ __global__ void __launch_bounds__(kBlock) staging_accumulate_cached_kernel(
   const int lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = warp * 32; base < n; base += nwarps * 32) {
-    const int64_t i = base + lane;
+  for (int64_t base = warp * per; base < n; base += nwarps * per) {
+    const int64_t i = lane < per ? base + lane : n;
     const int64_t id = i < n ? __ldg(ids + i) : -1;
     const int64_t slot = warp_lookup<MODE>(v, s_top, id);
     const bool hit = slot >= 0;
@@ -228,12 +229,13 @@ template <int VEC_BYTES>
 __global__ void __launch_bounds__(kBlock) staging_insert_kernel(
     hb_staging_t s, const int64_t* __restrict__ locs, const uint8_t* __restrict__ last_writer,
     const char* __restrict__ emb_rows, const int64_t* __restrict__ row_index,
-    char* __restrict__ cache_rows, int64_t row_bytes, int64_t n) {
+    char* __restrict__ cache_rows, int64_t row_bytes, int64_t n, const int64_t* __restrict__ n_dev, int per) {
+  n = effective_n(n, n_dev);
   const int lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = warp * 32; base < n; base += nwarps * 32) {
-    const int64_t i = base + lane;
+  for (int64_t base = warp * per; base < n; base += nwarps * per) {
+    const int64_t i = lane < per ? base + lane : n;
     // of several ids that received the same slot, the last of the batch writes it
     const int64_t slot = (i < n && last_writer[i]) ? __ldg(locs + i) : -1;
     const bool ok = slot >= 0;
@@ -300,11 +302,12 @@ int hb_staging_accumulate_cached(hb_index_t* h, const hb_staging_t* s, const int
     if (rc) return rc;
   }
   const bool vec4 = (s->dim % 4 == 0) && (((uintptr_t)grads | (uintptr_t)s->grad) & 15) == 0;
-  const int grid = warp_grid(n);
+  const int per = items_per_warp(n);
+  const int grid = grid_of_warps(n, per, kBlock, 16);
 #define HB_ACC(MODE, VEC)                                                                     \
   HB_LAUNCH((staging_accumulate_cached_kernel<MODE, VEC>), grid, kBlock, 0, st, h->view, *s,  \
             ids, grads, n, n_dev, threshold_table, default_threshold,                         \
-            (unsigned long long*)dropped, locs_out)
+            (unsigned long long*)dropped, locs_out, per)
   if (mode == HB_LOOKUP_SORTED) {
     if (vec4) HB_ACC(HB_LOOKUP_SORTED, 4); else HB_ACC(HB_LOOKUP_SORTED, 1);
   } else {
@@ -404,6 +407,15 @@ int hb_staging_insert_gather(hb_index_t* h, const hb_staging_t* s, const int64_t
 int hb_staging_insert_rows(const hb_staging_t* s, const void* emb_rows, const int64_t* row_index, int64_t n,
                            void* cache_rows, int64_t row_bytes, const int64_t* locs, const uint8_t* last_writer,
                            hb_stream_t stream) {
+  return staging_insert_rows(s, emb_rows, row_index, n, nullptr, cache_rows, row_bytes, locs, last_writer,
+                             (cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+int hb::staging_insert_rows(const hb_staging_t* s, const void* emb_rows, const int64_t* row_index, int64_t n,
+                            const int64_t* n_dev, void* cache_rows, int64_t row_bytes, const int64_t* locs,
+                            const uint8_t* last_writer, cudaStream_t st) {
   HB_CHECK_ARG(n >= 0 && row_bytes > 0, "hb_staging_insert_rows: bad sizes");
   HB_CHECK_ARG(n == 0 || (emb_rows && cache_rows && locs && last_writer), "hb_staging_insert_rows: null argument");
   if (n == 0) return HB_OK;
@@ -411,17 +423,15 @@ int hb_staging_insert_rows(const hb_staging_t* s, const void* emb_rows, const in
   memset(&none, 0, sizeof(none));
   const hb_staging_t st_desc = s ? *s : none;
   const int vb = payload_vec_bytes(row_bytes, emb_rows, cache_rows);
-  cudaStream_t st = (cudaStream_t)stream;
+  const int per = items_per_warp(n);
   if (vb == 16)
-    HB_LAUNCH(staging_insert_kernel<16>, warp_grid(n), kBlock, 0, st, st_desc, locs, last_writer,
-              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n);
+    HB_LAUNCH(staging_insert_kernel<16>, grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, last_writer,
+              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per);
   else if (vb == 4)
-    HB_LAUNCH(staging_insert_kernel<4>, warp_grid(n), kBlock, 0, st, st_desc, locs, last_writer,
-              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n);
+    HB_LAUNCH(staging_insert_kernel<4>, grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, last_writer,
+              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per);
   else
-    HB_LAUNCH(staging_insert_kernel<1>, warp_grid(n), kBlock, 0, st, st_desc, locs, last_writer,
-              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n);
+    HB_LAUNCH(staging_insert_kernel<1>, grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, last_writer,
+              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per);
   return HB_OK;
 }
-
-}  // extern "C"

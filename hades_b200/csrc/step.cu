@@ -1,0 +1,529 @@
+// One trainer's step on one GPU in two calls (hb_step_forward / hb_step_backward).
+//
+//   forward   sort | per distinct id: probe, place its row is read from, mark of a hit for the ageing,
+//             a missed cold id onto the list of its set | rows to the batch positions
+//             beside them: LRU ageing | the listed ids into the index
+//             then: rows of the inserted ids into the cache
+//   backward  per distinct cold id: probe, staging entry, mark | gradients summed, hot rows updated,
+//             cold rows staged | LRU ageing
+//
+// What bounds it: at 2,000 ids nothing but launches (composed from separate calls the same work took
+// 33 launches and 450 us of host time for 160 us of kernels); at 2,000,000 ids HBM.
+#include "index.cuh"
+#include "launch.cuh"
+#include "runs.cuh"
+#include "segsum.cuh"
+#include "staging.cuh"
+
+struct hb_step {
+  int device;
+  cudaStream_t side;
+  cudaEvent_t forked, expanded, maintained;
+  bool side_busy;    // `maintained` has to be waited for
+  hb_runs_t runs;    // of the last batch
+  int64_t runs_n;    // 0: none
+};
+
+namespace hb {
+int* device_error_word();  // runtime.cu
+
+namespace {
+
+constexpr int kBlock = 256;
+constexpr int kCold = 2;
+// Batches below this run everything on the caller's stream: their kernels last a few microseconds each,
+// less than the events that order a second stream.
+constexpr int64_t kSideMin = 32768;
+
+// Small batches update rows as their sums become complete (one launch); large ones write the sums and
+// update in a second pass over the distinct ids: the sums then run at the speed of the copy, and the
+// update has many rows in flight whatever the lengths of the runs.
+// The line lies where the two cost the same (65,536 ids of 128 columns: 149 us the step fused, 154 not;
+// 150,000 of 64: 167 and 162; 2,000,000 of 128: 903 and 846).
+constexpr int64_t kFuseMax = 100000;
+bool fuses_update(int64_t n) { return n <= kFuseMax; }
+
+struct StepPlan {
+  char* runs_ws;
+  size_t runs_bytes;
+  void* fetch_ws;        // hb_lookup_fetch_runs_workspace_bytes: run_src first
+  size_t fetch_bytes;
+  int64_t* run_slots;    // [n] slot of every run at the lookup
+  int64_t* cold_slots;   // [n] slot of every cold run at the accumulate
+  int64_t* new_slots;    // [n] slot a missed cold run was given
+  uint8_t* on_list;      // [n] the run is a cold miss, to be inserted
+  uint8_t* last_writer;  // [n]
+  void* add_ws;          // index_add_runs_bytes: the lists' links first
+  int32_t* chunk_listed; // [n / 32 + 1]
+  unsigned long long* listed;  // [1]
+  char* seg_ws;
+  size_t seg_bytes;
+  float* sums;           // [n][dim], where the update is a launch of its own
+  size_t total;
+};
+
+StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
+  StepPlan p;
+  Carver cv(ws ? ws : (void*)256);
+  const int64_t m = n > 0 ? n : 1;
+  p.runs_bytes = hb_runs_workspace_bytes(m);
+  p.runs_ws = cv.take<char>(p.runs_bytes);
+  p.fetch_bytes = hb_lookup_fetch_runs_workspace_bytes(m, 1, 0);
+  p.fetch_ws = cv.take<char>(p.fetch_bytes);
+  p.run_slots = cv.take<int64_t>(m);
+  p.cold_slots = cv.take<int64_t>(m);
+  p.new_slots = cv.take<int64_t>(m);
+  p.on_list = cv.take<uint8_t>(m);
+  p.last_writer = cv.take<uint8_t>(m);
+  p.add_ws = cv.take<char>(index_add_runs_bytes(m));
+  p.chunk_listed = cv.take<int32_t>(m / 32 + 16);
+  p.listed = cv.take<unsigned long long>(1);
+  p.seg_bytes = seg_plan(nullptr, m, dim).total;
+  p.seg_ws = cv.take<char>(p.seg_bytes);
+  p.sums = cv.take<float>(fuses_update(m) ? 0 : (size_t)m * dim);
+  p.total = cv.used() + 256;
+  return p;
+}
+
+struct ResolveArgs {
+  const char* cache_rows;
+  const char* table;
+  int64_t table_rows;
+  int64_t row_bytes;
+  unsigned long long* run_src;
+  int64_t* run_slots;
+  uint8_t* on_list;       // nullable: misses are not inserted
+  uint8_t* last_writer;
+  int32_t* chunk_listed;
+  unsigned long long* listed;  // zero before
+  int push;               // ... onto the lists of their sets
+  int touch;
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_runs_t r, ResolveArgs a, TouchMarks marks,
+                                                              AddLists lists, int* __restrict__ err) {
+  __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
+  if (MODE == HB_LOOKUP_SORTED) {
+    stage_top_level(v, s_top);
+    __syncthreads();
+  }
+  const int64_t U = *r.num_runs;
+  const int lane = lane_id();
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
+    const int64_t u = u0 + lane;
+    const bool valid = u < U;
+    const int64_t id = valid ? __ldg(r.uniq_ids + u) : -1;
+    const bool cold = valid && a.on_list && r.dclass[u] == kCold;
+    const int64_t slot = warp_lookup<MODE>(v, s_top, id);
+    const bool missed = cold && slot < 0;
+    if (a.on_list) {
+      const unsigned m = __ballot_sync(0xffffffffu, missed);
+      if (lane == 0) {
+        a.chunk_listed[u0 >> 5] = __popc(m);
+        if (m) atomicAdd(a.listed, (unsigned long long)__popc(m));
+      }
+      if (valid) {
+        a.on_list[u] = missed;
+        a.last_writer[u] = 0;
+      }
+      if (missed && a.push) lists.push(id, u);
+    }
+    if (!valid) continue;
+    const char* src = nullptr;
+    if (slot >= 0) src = a.cache_rows + slot * a.row_bytes;
+    else if (id < a.table_rows) src = a.table + id * a.row_bytes;
+    else atomicExch(err, HB_ERR_INVALID);  // no such row: the output rows of the run stay as they were
+    a.run_src[u] = (unsigned long long)src | (slot >= 0 ? 1ull : 0ull);
+    a.run_slots[u] = slot;
+    if (a.touch) marks.mark(slot, u);
+  }
+}
+
+int join_side(hb_step* s, cudaStream_t st) {
+  if (s->side_busy) {
+    HB_CUDA(cudaStreamWaitEvent(st, s->maintained, 0));
+    s->side_busy = false;
+  }
+  return HB_OK;
+}
+
+struct ColdArgs {
+  hb_staging_t s;
+  const int32_t* thr_table;  // nullable
+  int32_t default_thr;
+  unsigned long long* dropped;  // nullable
+  int64_t* slots;            // [runs]
+  TouchMarks marks;
+  int touch;
+};
+
+// The cold ids among 32 distinct ones (a lane each): slot now that this batch's misses are in the
+// cache, staging entry (server.py:546-562 without the row), mark for the ageing.
+template <int MODE>
+__device__ __forceinline__ int64_t cold_entry(const IndexView& v, const int64_t* s_top, const ColdArgs& a, int64_t u,
+                                              bool cold, int64_t id) {
+  const int64_t slot = warp_lookup<MODE>(v, s_top, cold ? id : -1);
+  if (slot >= 0) {
+    a.s.idx[slot] = id;
+    a.s.iter_threshold[slot] = a.thr_table ? __ldg(a.thr_table + id) : a.default_thr;
+    a.s.cnt[slot] += 1;
+    if (a.touch) a.marks.mark(slot, u);
+  }
+  if (a.dropped) {
+    const unsigned miss = __ballot_sync(0xffffffffu, cold && slot < 0);
+    if (lane_id() == 0 && miss) atomicAdd(a.dropped, (unsigned long long)__popc(miss));
+  }
+  return slot;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_t r, ColdArgs a,
+                                                           unsigned* __restrict__ zero, int64_t zero_words) {
+  __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
+  if (MODE == HB_LOOKUP_SORTED) {
+    stage_top_level(v, s_top);
+    __syncthreads();
+  }
+  // the aggregation that follows needs its arrival counters at zero
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < zero_words; k += (int64_t)gridDim.x * blockDim.x)
+    zero[k] = 0u;
+  const int64_t U = *r.num_runs;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
+    const int64_t u = u0 + lane_id();
+    const bool cold = u < U && r.dclass[u] == kCold;
+    const int64_t slot = cold_entry<MODE>(v, s_top, a, u, cold, cold ? __ldg(r.uniq_ids + u) : -1);
+    if (u < U) a.slots[u] = slot;
+  }
+}
+
+// Summed gradients to where they belong: state and table rows of hot ids, staging rows of cold ones.  A
+// warp takes 32 distinct ids, a lane each for what is worked out once per id, then G lanes per row and
+// kFly rows in flight.  Bound by HBM: rows read and written once (175,000 ids of 128 columns: 60 us).
+template <int MODE, bool ADAM, int VEC, int G, int VPL>
+__global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(IndexView v, hb_runs_t r, ColdArgs c,
+                                                                            SegArgs a, UpdateRows<ADAM, true> epi,
+                                                                            const float* __restrict__ sums) {
+  using V = typename VecF<VEC>::T;
+  using Ops = EpiOps<UpdateRows<ADAM, true>, VEC, G, VPL>;
+  constexpr int kFly = VPL > 1 ? 1 : 2;
+  constexpr int RPP = 32 / G;
+  __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
+  if (MODE == HB_LOOKUP_SORTED) {
+    stage_top_level(v, s_top);
+    __syncthreads();
+  }
+  const int64_t U = *r.num_runs;
+  const int lane = lane_id();
+  const int sub = lane & (G - 1), which = lane / G;
+  const int vpr = a.cols / VEC;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
+    const int64_t u = u0 + lane;
+    const bool valid = u < U;
+    const int cls = valid ? r.dclass[u] : -1;
+    const int64_t id = valid ? __ldg(r.uniq_ids + u) : -1;
+    const int64_t slot = cold_entry<MODE>(v, s_top, c, u, cls == kCold, id);
+    if (valid) c.slots[u] = slot;
+    const typename Ops::Lane mine = Ops::lane_of_class(epi, cls, id, slot);
+    int count = 0;
+    if (valid) count = (int)(__ldg(r.run_start + u + 1) - __ldg(r.run_start + u));
+    const int rows = U - u0 < 32 ? (int)(U - u0) : 32;
+    for (int t0 = 0; t0 < rows; t0 += RPP * kFly) {
+      V acc[kFly][VPL];
+      typename Ops::Row with[kFly];
+      int cnt[kFly];
+#pragma unroll
+      for (int x = 0; x < kFly; ++x) {
+        const int q = (t0 + x * RPP + which) & 31;
+        const bool in = t0 + x * RPP + which < rows;
+        cnt[x] = __shfl_sync(0xffffffffu, count, q);
+        Ops::template fetch<32>(epi, a, mine, q, in, sub, vpr, with[x]);
+        if (!in) with[x].row = -1;
+        if (with[x].row >= 0) {
+          const V* src = reinterpret_cast<const V*>(sums + (u0 + q) * a.dim);
+#pragma unroll
+          for (int k = 0; k < VPL; ++k)
+            if (sub + k * G < vpr) acc[x][k] = __ldcs(src + sub + k * G);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < kFly; ++x) Ops::finish(epi, a, 0, acc[x], with[x], sub, vpr, cnt[x]);
+    }
+  }
+}
+
+template <int MODE, bool ADAM, int VEC>
+int launch_apply(const IndexView& v, const hb_runs_t& r, const ColdArgs& c, const SegArgs& a,
+                 const UpdateRows<ADAM, true>& epi, const float* sums, cudaStream_t st) {
+  const int vpr = a.cols / VEC;
+  int64_t blocks = ceil_div(r.n, kBlock);
+  if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
+#define HB_APPLY(G, VPL)                                                                                      \
+  HB_LAUNCH((step_apply_kernel<MODE, ADAM, VEC, G, VPL>), (int)blocks, kBlock, 0, st, v, r, c, a, epi, sums)
+  if (vpr > 64) HB_APPLY(32, 4);
+  else if (vpr > 32) HB_APPLY(32, 2);
+  else if (vpr > 16) HB_APPLY(32, 1);
+  else if (vpr > 8) HB_APPLY(16, 1);
+  else if (vpr > 4) HB_APPLY(8, 1);
+  else HB_APPLY(4, 1);
+#undef HB_APPLY
+  return HB_OK;
+}
+
+template <bool ADAM>
+int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs a, bool vec4, float* sums,
+                const SegPlan& seg, bool fused, cudaStream_t st) {
+  const hb_runs_t& r = s->runs;
+  auto epi = update_rows<ADAM, true>(&r, &d->opt);
+  epi.dclass = r.dclass;
+  epi.staged = d->staging.grad;
+  epi.slots = c.slots;
+  const IndexView& v = d->index->view;
+  const bool sorted = d->lookup_mode == HB_LOOKUP_SORTED;
+  if (fused) {
+    int64_t blocks = ceil_div(r.n, kBlock);
+    if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
+    if (sorted)
+      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SORTED>, (int)blocks, kBlock, 0, st, v, r, c, seg.done, seg.max_ctas);
+    else
+      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SETASSOC>, (int)blocks, kBlock, 0, st, v, r, c, seg.done, seg.max_ctas);
+    return seg_dispatch(a, epi, vec4, st);
+  }
+  HB_CUDA(cudaMemsetAsync(seg.done, 0, (size_t)seg.max_ctas * sizeof(unsigned), st));
+  StoreRows store;
+  memset(&store, 0, sizeof(store));
+  store.sums = sums;
+  int rc = seg_dispatch(a, store, vec4, st);
+  if (rc != HB_OK) return rc;
+  // from here on the fetch of this batch must have read its rows and the cache hold its misses
+  rc = join_side(s, st);
+  if (rc != HB_OK) return rc;
+  if (sorted)
+    return vec4 ? launch_apply<HB_LOOKUP_SORTED, ADAM, 4>(v, r, c, a, epi, sums, st)
+                : launch_apply<HB_LOOKUP_SORTED, ADAM, 1>(v, r, c, a, epi, sums, st);
+  return vec4 ? launch_apply<HB_LOOKUP_SETASSOC, ADAM, 4>(v, r, c, a, epi, sums, st)
+              : launch_apply<HB_LOOKUP_SETASSOC, ADAM, 1>(v, r, c, a, epi, sums, st);
+}
+
+int grid_for_runs(int64_t n) {
+  int64_t blocks = ceil_div(n, kBlock);
+  const int64_t cap = (int64_t)sm_count() * 8;
+  if (blocks > cap) blocks = cap;
+  return blocks < 1 ? 1 : (int)blocks;
+}
+
+int check_desc(const hb_step_desc_t* d, const char* who) {
+  if (!d || !d->index || !d->cache_rows || !d->table || !d->class_table || !d->staging.grad || d->row_bytes <= 0 ||
+      d->dim <= 0 || d->table_rows <= 0 || d->class_len <= 0 || !d->opt.emb || !d->opt.s0) {
+    set_error("%s: incomplete description", who);
+    return HB_ERR_INVALID;
+  }
+  if (d->staging.slots != d->index->cache_size || d->staging.dim != d->dim) {
+    set_error("%s: the staging table must have one slot per cache slot and rows of dim columns", who);
+    return HB_ERR_INVALID;
+  }
+  return HB_OK;
+}
+
+bool vec4_ok(const hb_step_desc_t* d, const float* grads) {
+  const uintptr_t bits = (uintptr_t)grads | (uintptr_t)d->opt.emb | (uintptr_t)d->opt.s0 | (uintptr_t)d->opt.s1 |
+                         (uintptr_t)d->staging.grad;
+  return d->dim % 4 == 0 && (bits & 15) == 0;
+}
+
+int build_runs(hb_step* s, const hb_step_desc_t* d, const StepPlan& p, const int64_t* ids, int64_t n,
+               int64_t* counters, cudaStream_t st) {
+  static_assert(sizeof(unsigned long long) == 2 * sizeof(unsigned), "the list counter is zeroed as two words");
+  const int rc = runs_build(ids, n, nullptr, nullptr, 0, d->id_bits, d->class_table, d->class_len, nullptr,
+                            counters + 1, nullptr, counters, reinterpret_cast<unsigned*>(p.listed), 2, p.runs_ws,
+                            p.runs_bytes, &s->runs, st);
+  s->runs_n = rc == HB_OK ? n : 0;
+  return rc;
+}
+
+}  // namespace
+}  // namespace hb
+
+using namespace hb;
+
+extern "C" {
+
+int hb_step_create(hb_step_t** out) {
+  HB_CHECK_ARG(out, "hb_step_create: out is null");
+  hb_step* s = new hb_step();
+  memset(s, 0, sizeof(*s));
+  HB_CUDA(cudaGetDevice(&s->device));
+  HB_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
+  HB_CUDA(cudaEventCreateWithFlags(&s->forked, cudaEventDisableTiming));
+  HB_CUDA(cudaEventCreateWithFlags(&s->expanded, cudaEventDisableTiming));
+  HB_CUDA(cudaEventCreateWithFlags(&s->maintained, cudaEventDisableTiming));
+  *out = s;
+  return HB_OK;
+}
+
+int hb_step_destroy(hb_step_t* s) {
+  if (!s) return HB_OK;
+  cudaStreamDestroy(s->side);
+  cudaEventDestroy(s->forked);
+  cudaEventDestroy(s->expanded);
+  cudaEventDestroy(s->maintained);
+  delete s;
+  return HB_OK;
+}
+
+size_t hb_step_workspace_bytes(int64_t n, int64_t dim) { return step_plan(nullptr, n, dim > 0 ? dim : 1).total; }
+
+int hb_step_supported(const hb_step_desc_t* d) {
+  if (check_desc(d, "hb_step_supported") != HB_OK) return 0;
+  if (d->opt.kind != HB_OPT_ADAM && d->opt.kind != HB_OPT_ADAGRAD) return 0;
+  if (d->dim > seg_tile(vec4_ok(d, nullptr))) return 0;
+  return d->opt.rows < ((int64_t)1 << 30) && d->staging.slots < ((int64_t)1 << 30);
+}
+
+int hb_step_join(hb_step_t* s, hb_stream_t stream) {
+  HB_CHECK_ARG(s, "hb_step_join: null handle");
+  return join_side(s, (cudaStream_t)stream);
+}
+
+int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, int64_t n, void* out_rows,
+                    int64_t* locs, uint8_t* found, int64_t* counters, int join, void* workspace,
+                    size_t workspace_bytes, hb_stream_t stream) {
+  HB_CHECK_ARG(s, "hb_step_forward: null handle");
+  int rc = check_desc(d, "hb_step_forward");
+  if (rc != HB_OK) return rc;
+  HB_CHECK_ARG(n > 0 && n < ((int64_t)1 << 31), "hb_step_forward: n out of range");
+  HB_CHECK_ARG(ids && out_rows && found && counters, "hb_step_forward: null argument");
+  const StepPlan p = step_plan(workspace, n, d->dim);
+  if (!workspace || workspace_bytes < p.total) {
+    set_error("hb_step_forward: workspace of %zu bytes needed, %zu given", p.total, workspace_bytes);
+    return HB_ERR_WORKSPACE;
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  hb_index* h = d->index;
+  rc = join_side(s, st);
+  if (rc != HB_OK) return rc;
+  if (d->lookup_mode == HB_LOOKUP_SORTED && h->sorted_stale) {
+    rc = hb_index_build_sorted(h, stream);
+    if (rc != HB_OK) return rc;
+  }
+  TouchMarks marks;
+  rc = index_touch_marks(h, &marks, st);
+  if (rc != HB_OK) return rc;
+  AddLists lists;
+  rc = index_add_lists(h, static_cast<uint32_t*>(p.add_ws), &lists, st);
+  if (rc != HB_OK) return rc;
+  rc = build_runs(s, d, p, ids, n, counters, st);
+  if (rc != HB_OK) return rc;
+  // HB_STEP_ASIDE: all of the fetch leaves the caller's stream, which goes on to the aggregation of the
+  // same batch (it needs the sort only); both are bound by HBM, but not all the time
+  const bool aside = join == HB_STEP_ASIDE && !fuses_update(n);
+  if (aside) {
+    HB_CUDA(cudaEventRecord(s->forked, st));
+    HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
+    st = s->side;
+  }
+  const ResolveArgs a{(const char*)d->cache_rows, (const char*)d->table, d->table_rows, d->row_bytes,
+                      static_cast<unsigned long long*>(p.fetch_ws), p.run_slots,
+                      d->insert_misses ? p.on_list : nullptr, p.last_writer, p.chunk_listed, p.listed,
+                      index_add_runs_lists(h, n), d->touch_lru};
+  if (d->lookup_mode == HB_LOOKUP_SORTED)
+    HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SORTED>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a, marks, lists,
+              device_error_word());
+  else
+    HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a, marks,
+              lists, device_error_word());
+  const bool maintain = d->touch_lru || d->insert_misses;
+  const bool beside = !aside && maintain && n >= kSideMin;
+  cudaStream_t side = beside ? s->side : st;
+  if (beside) {
+    HB_CUDA(cudaEventRecord(s->forked, st));
+    HB_CUDA(cudaStreamWaitEvent(side, s->forked, 0));
+  }
+  rc = hb_runs_expand(&s->runs, d->cache_rows, d->table, d->row_bytes, 0, out_rows, locs, found, p.run_slots,
+                      p.fetch_ws, p.fetch_bytes, (hb_stream_t)st);
+  if (rc != HB_OK) return rc;
+  if (d->touch_lru) {
+    const RunsView v{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
+    rc = index_touch_apply(h, v, side);
+    if (rc != HB_OK) return rc;
+  }
+  if (d->insert_misses) {
+    const AddEntries e{s->runs.uniq_ids, n, s->runs.num_runs, p.on_list, p.chunk_listed, p.listed, d->miss_cap};
+    rc = index_add_runs(h, e, p.add_ws, p.new_slots, p.last_writer, side);
+    if (rc != HB_OK) return rc;
+    if (beside) {
+      // a slot that the insertion takes over may hold a row this batch still reads
+      HB_CUDA(cudaEventRecord(s->expanded, st));
+      HB_CUDA(cudaStreamWaitEvent(side, s->expanded, 0));
+    }
+    rc = staging_insert_rows(&d->staging, d->table, s->runs.uniq_ids, n, s->runs.num_runs, d->cache_rows,
+                             d->row_bytes, p.new_slots, p.last_writer, side);
+    if (rc != HB_OK) return rc;
+  }
+  if (beside || aside) {
+    HB_CUDA(cudaEventRecord(s->maintained, side));
+    s->side_busy = true;
+    if (join == HB_STEP_JOIN) return join_side(s, st);
+  }
+  return HB_OK;
+}
+
+int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, int64_t n, const float* grads,
+                     int64_t* counters, void* workspace, size_t workspace_bytes, hb_stream_t stream) {
+  HB_CHECK_ARG(s, "hb_step_backward: null handle");
+  int rc = check_desc(d, "hb_step_backward");
+  if (rc != HB_OK) return rc;
+  HB_CHECK_ARG(n > 0 && n < ((int64_t)1 << 31) && grads, "hb_step_backward: bad argument");
+  HB_CHECK_ARG(ids ? counters != nullptr : s->runs_n == n, "hb_step_backward: not the batch of the last forward call");
+  const StepPlan p = step_plan(workspace, n, d->dim);
+  if (!workspace || workspace_bytes < p.total) {
+    set_error("hb_step_backward: workspace of %zu bytes needed, %zu given", p.total, workspace_bytes);
+    return HB_ERR_WORKSPACE;
+  }
+  const bool vec4 = vec4_ok(d, grads);
+  if (d->dim > seg_tile(vec4)) {
+    set_error("hb_step_backward: rows of %lld columns are not updated in one pass", (long long)d->dim);
+    return HB_ERR_UNSUPPORTED;
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  hb_index* h = d->index;
+  const bool fused = fuses_update(n);
+  if (ids || fused) {
+    rc = join_side(s, st);
+    if (rc != HB_OK) return rc;
+  }
+  if (ids) {
+    rc = build_runs(s, d, p, ids, n, counters, st);
+    s->runs_n = 0;  // the next forward pass is another batch
+    if (rc != HB_OK) return rc;
+  }
+  if (d->lookup_mode == HB_LOOKUP_SORTED && h->sorted_stale) {
+    rc = join_side(s, st);
+    if (rc != HB_OK) return rc;
+    rc = hb_index_build_sorted(h, stream);
+    if (rc != HB_OK) return rc;
+  }
+  TouchMarks marks;
+  rc = index_touch_marks(h, &marks, st);
+  if (rc != HB_OK) return rc;
+  const SegPlan seg = seg_plan(p.seg_ws, n, d->dim);
+  const ColdArgs c{d->staging, d->threshold_table, d->default_threshold, (unsigned long long*)d->dropped,
+                   p.cold_slots, marks, d->touch_lru};
+  SegArgs a = seg_args(&s->runs, grads, nullptr, d->dim, 0, seg);
+  a.cols = (int)d->dim;
+  rc = d->opt.kind == HB_OPT_ADAM ? update_step<true>(s, d, c, a, vec4, p.sums, seg, fused, st)
+                                  : update_step<false>(s, d, c, a, vec4, p.sums, seg, fused, st);
+  if (rc != HB_OK) return rc;
+  if (!d->touch_lru) return HB_OK;
+  // the lookup of the accumulate: every distinct cold id once, in ascending order
+  const RunsView v{p.cold_slots, nullptr, nullptr, s->runs.num_runs, s->runs.num_runs, n, n, 2};
+  return index_touch_apply(h, v, st);
+}
+
+}  // extern "C"

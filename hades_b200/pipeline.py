@@ -26,11 +26,13 @@ carries the exchange.
 from __future__ import annotations
 
 import contextlib
+import ctypes as C
 from dataclasses import dataclass, field
 
 import torch
 
 from . import EmbCacheLib as E
+from .EmbCacheLib import _check
 from .cold_cache import ColdCache, flush_thresholds
 from .sparse_optim import ShardedEmbedding, SparseAdam, SparseAdagrad, exchange_packed
 
@@ -54,6 +56,106 @@ class StepStats:
             return 0
         n = int(self.flushed_dev.sum().item())
         return min(n, self.flush_cap) if self.flush_cap else n
+
+
+class _CounterStats(StepStats):
+    """``StepStats`` over one counter tensor: distinct ids, then those of class 0, 1, 2 (sliced when asked)."""
+
+    def __init__(self, counters: torch.Tensor):
+        self.counters = counters
+        self.flushed_dev, self.flush_cap, self.extra = None, 0, {}
+
+    num_unique = property(lambda self: self.counters[0:1])
+    split_counts = property(lambda self: self.counters[1:4])
+    sent_counts = property(lambda self: self.counters[2:3])
+
+
+class _OneGpuStep:
+    """One trainer's step on one GPU as two library calls (``hb_step_forward`` / ``hb_step_backward``): what
+    ``forward`` and ``backward`` of the path compose from separate operators when other GPUs take part."""
+
+    def __init__(self, path: "EmbeddingPath"):
+        self.path = path
+        self.lib, self.native = E._lib.load(), E._lib.native()
+        h = C.c_void_p()
+        E._lib.check(self.lib.hb_step_create(C.byref(h)))
+        self._h = h
+        self.desc = E._lib.StepDesc()
+        self.addr = C.addressof(self.desc)
+        self.ws, self.kept = None, []
+        self.batch = None  # (ids, version, counters) of the last forward pass
+        self.key = None
+        self.refresh()
+        self.supported = bool(self.lib.hb_step_supported(C.byref(self.desc)))
+
+    def __del__(self):
+        try:
+            self.lib.hb_step_destroy(self._h)
+        except Exception:  # interpreter shutdown
+            pass
+
+    def refresh(self) -> None:
+        """The description follows the path's attributes (they may change between steps)."""
+        p, d = self.path, self.desc
+        cold, opt = p.cold, p.opt
+        key = (p.lookup_mode, p.touch_lru, p.insert_misses, p.miss_cap, p.id_bits, cold.default_threshold, opt._lr,
+               p.table.data_ptr(), p.class_table.data_ptr(), cold.emb.data_ptr(), opt.emb.weight.data_ptr())
+        if key == self.key:
+            return
+        self.key = key
+        d.index, d.staging, d.cache_rows = cold.index._h, cold.remote.desc, cold.emb.data_ptr()
+        d.table, d.table_rows = p.table.data_ptr(), p.table.size(0)
+        d.row_bytes, d.dim = p.dim * cold.emb.element_size(), p.dim
+        d.class_table, d.class_len, d.id_bits = p.class_table.data_ptr(), p.num_nodes, p.id_bits
+        d.lookup_mode, d.touch_lru, d.insert_misses = p.lookup_mode, p.touch_lru, p.insert_misses
+        d.miss_cap, d.default_threshold = p.miss_cap, cold.default_threshold
+        d.threshold_table = None if cold.threshold is None else cold.threshold.data_ptr()
+        d.dropped, d.opt = cold.dropped.data_ptr(), opt._desc()
+
+    def keep(self, ws: torch.Tensor) -> None:
+        """Scratch of the last batch.  What captured graphs hold stays."""
+        if ws is not self.ws:
+            if self.ws is not None and self.path._graphs_hold_scratch():
+                self.kept.append(self.ws)
+            self.ws = ws
+
+    def forward(self, ids: torch.Tensor, out_rows, join: int):
+        """join: HB_STEP_BESIDE / HB_STEP_JOIN / HB_STEP_ASIDE."""
+        p = self.path
+        ids = ids.contiguous()
+        self.refresh()
+        rows, locs, found, counters, ws = self.native.step_forward(
+            self._h.value, self.addr, ids, p.dim, p.cold.emb, out_rows, p.want_locs, join, self.ws)
+        self.keep(ws)
+        self.batch = (ids, ids._version, counters)
+        return rows, locs, found
+
+    def backward(self, ids: torch.Tensor, grads: torch.Tensor) -> StepStats:
+        p, n = self.path, ids.numel()
+        _check(grads.dtype == torch.float32 and grads.shape == (n, p.dim), "grads is fp32 [len(ids), dim]")
+        grads = grads.contiguous()
+        if p.dim > 128 and grads.data_ptr() & 15:
+            grads = grads.clone()  # wide rows are read 16 bytes at a time
+        b = self.batch
+        self.refresh()
+        if b is not None and (ids is b[0] or (ids.data_ptr() == b[0].data_ptr() and n == b[0].numel())) \
+                and ids._version == b[1]:
+            counters, given = b[2], None
+        else:
+            _check(ids.is_cuda and ids.dtype == torch.int64, "ids is a CUDA int64 tensor")
+            given = ids.contiguous()
+            counters = torch.empty(4, dtype=torch.int64, device=ids.device)
+            self.batch = None
+            need = self.lib.hb_step_workspace_bytes(n, p.dim)
+            if self.ws is None or self.ws.numel() < need:
+                # (the call joins the side stream, which may still use the old scratch, before it writes)
+                self.join()
+                self.keep(torch.empty(need, dtype=torch.uint8, device=ids.device))
+        self.native.step_backward(self._h.value, self.addr, given, n, grads, counters, self.ws)
+        return _CounterStats(counters)
+
+    def join(self) -> None:
+        E._lib.check(self.lib.hb_step_join(self._h, E._lib.stream_ptr()))
 
 
 class EmbeddingPath:
@@ -109,6 +211,15 @@ class EmbeddingPath:
         self._side_done, self._side_refs = None, []
         self._runs_ws, self._side_ws, self._fetch_ws = None, None, None
         self._last = None  # (BatchRuns, locs) of the last forward pass
+        # one trainer, its table and its optimiser's state on this GPU: the step as two library calls
+        self._one = None
+        if (world == 1 and self.shared is None and table is not None and table.dtype == cold.emb.dtype
+                and getattr(optimizer, "state_cache", None) is None):
+            one = _OneGpuStep(self)
+            self._one = one if one.supported else None
+
+    def _graphs_hold_scratch(self) -> bool:
+        return bool(self._graphs) or getattr(self, "_split", None) is not None
 
     # ---- streams ---------------------------------------------------------------------------
     def _on_side(self):
@@ -148,8 +259,11 @@ class EmbeddingPath:
         running on the side stream (``backward`` joins it).  on_side=True (``step`` with
         overlap_fetch): everything after the sort runs on the side stream and the rows are
         complete only after the join at the end of the backward pass."""
-        lib = E._lib.load()
         n = ids.numel()
+        if self._one is not None and n > 0:
+            self._last = None
+            return self._one.forward(ids, out_rows, 2 if on_side else int(join))
+        lib = E._lib.load()
         runs = E.cudaRunsBuild(ids, self.id_bits, self.class_table, keep=(False, True, True),
                                caps=(None, self.num_hot_ids, None),
                                ws=self._ws("_runs_ws", lib.hb_runs_workspace_bytes(n)))
@@ -366,6 +480,8 @@ class EmbeddingPath:
         overlap_fetch), the exchange waits until that fetch has read what it needs from the other
         GPUs' shards, and the owner update until it has read what it needs from this GPU's shard:
         a fetch returns the rows as they were before the step's update."""
+        if self._one is not None and ids.numel() > 0:
+            return self._one.backward(ids, grads)
         st, hot_ids, hot_rows, hot_cnt = self._backward_local(ids, grads, join=False)
         n_hot = st.split_counts[HOT:HOT + 1]
         if self.world > 1:

@@ -132,17 +132,16 @@ class _SparseOptimizer:
     def _update_merging(self, idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap) -> bool:
         """unique_grads (sparse_optim.py:611) and the row update of what it returns in one pass over
         the gradients; False: rows too wide or too many for that (``hb_segsum_update_f32``)."""
-        n, dim = idx.numel(), grad.size(1)
+        dim = grad.size(1)
         w = self.emb.weight
         desc = self._desc()
         aligned = (w.data_ptr() | grad.data_ptr() | (desc.s0 or 0) | (desc.s1 or 0)) & 15 == 0
+        if idx.numel() == 0:
+            return True
         if dim > (512 if dim % 4 == 0 and aligned else 128) or self.emb.rows >= 1 << 30:
             return False
-        lib = _lib.load()
-        ws = _lib.workspace(lib.hb_unique_segsum_workspace_bytes(n, dim))
-        _lib.check(lib.hb_unique_update_f32(idx.data_ptr(), grad.data_ptr(), _lib.ptr(cnt), n, _lib.ptr(n_dev),
-                                            _lib.ptr(seg_counts), int(seg_cap), dim, int(id_bits), 1, C.byref(desc),
-                                            ws.data_ptr(), ws.numel(), _lib.stream_ptr()))
+        (_lib._NATIVE or _lib.native()).unique_update(idx, grad, cnt, n_dev, seg_counts, int(seg_cap), int(id_bits),
+                                                      C.addressof(desc), True)
         return True
 
 

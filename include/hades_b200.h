@@ -722,6 +722,54 @@ int hb_lookup_fetch_sharded(hb_index_t* h, const int64_t* ids, int64_t n, const 
                             hb_peer_table_t* table, void* out_rows, int64_t* locs /* nullable */,
                             uint8_t* found /* nullable */, int mode, hb_stream_t stream);
 
+/* ------------------------------------------------------------------------- */
+/* One trainer's step on one GPU as two calls: what EmbeddingPath.forward and     */
+/* .backward compose from the calls above when other GPUs take part              */
+/* (python/EmbCache/dist_emb.py:167-292, sparse_optim.py:212-448 and the server    */
+/* loop, server.py:259-298).  Results as composed.                                */
+/* ------------------------------------------------------------------------- */
+typedef struct hb_step hb_step_t; /* a side stream, its events, the grouping of the last batch */
+typedef struct hb_step_desc {
+  hb_index_t* index;
+  hb_staging_t staging;        /* one slot per cache slot */
+  void* cache_rows;            /* [capacity][row_bytes] */
+  const void* table;           /* [table_rows][row_bytes]: rows of ids that miss */
+  int64_t table_rows;
+  int64_t row_bytes;
+  int64_t dim;                 /* columns of gradients, staging rows and optimiser state */
+  const int8_t* class_table;   /* 1 = HOT, 2 = COLD */
+  int64_t class_len;
+  int id_bits;
+  int lookup_mode;
+  int touch_lru;
+  int insert_misses;
+  int64_t miss_cap;
+  const int32_t* threshold_table; /* nullable */
+  int32_t default_threshold;
+  int64_t* dropped;            /* nullable device int64 */
+  hb_optim_t opt;
+} hb_step_desc_t;
+
+int hb_step_create(hb_step_t** out);
+int hb_step_destroy(hb_step_t* s);
+/* 1 when the rows of this description are updated in one pass (hb_segsum_update_f32's limits). */
+int hb_step_supported(const hb_step_desc_t* d);
+size_t hb_step_workspace_bytes(int64_t n, int64_t dim);
+/* counters: device int64[4] = distinct ids, distinct ids of class 0, 1, 2.  locs nullable.
+ * join: HB_STEP_JOIN; HB_STEP_BESIDE: the maintenance of the cache may still run on the side stream;
+ * HB_STEP_ASIDE: all of the fetch may (out_rows, locs and found too), beside the aggregation of the
+ * hb_step_backward that follows.  The next call of this handle, or hb_step_join, orders it. */
+#define HB_STEP_BESIDE 0
+#define HB_STEP_JOIN 1
+#define HB_STEP_ASIDE 2
+int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, int64_t n, void* out_rows,
+                    int64_t* locs, uint8_t* found, int64_t* counters, int join, void* workspace,
+                    size_t workspace_bytes, hb_stream_t stream);
+int hb_step_join(hb_step_t* s, hb_stream_t stream);
+/* ids NULL: the gradients belong to the batch of the last forward call (same n and workspace). */
+int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, int64_t n, const float* grads,
+                     int64_t* counters, void* workspace, size_t workspace_bytes, hb_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

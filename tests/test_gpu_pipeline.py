@@ -230,3 +230,26 @@ def test_path_with_tiered_optimizer_state_equals_all_hbm(cuda_lib):
         assert torch.equal(x, y)
     hit = pb.opt.state_cache.idx_map != -1
     assert 0 < int(hit.sum().item()) < base.table_rows
+
+
+@pytest.mark.parametrize("cache_entries,batch,stride,miss_cap", [
+    (4096, 2000, 1, 1 << 17), (4096, 40_000, 1, 1 << 17),   # one stream / two streams, few ids per set
+    (512, 40_000, 1, 1 << 17),                               # many ids per set: sorted
+    (16_384, 30_000, 2048, 1 << 17),                         # ids in strides of the number of sets: long lists
+    (4096, 40_000, 1, 700), (512, 40_000, 1, 50)])           # fewer misses taken than there are
+def test_insertion_of_misses_matches_oracle(cuda_lib, oracle_mod, cache_entries, batch, stride, miss_cap):
+    from hades_b200 import pipeline, synth
+
+    cfg = synth.CacheFetchConfig("insert_test", 1, 60_000, 16, cache_entries, batch, 1.05, flush_every=3)
+    path = pipeline.build_path(cfg, hot_fraction=0.002, miss_cap=miss_cap)
+    orc = _oracle_for(path, oracle_mod, cfg)
+    rng = np.random.default_rng(batch + cache_entries)
+    for it in range(1, 5):
+        ids = rng.integers(0, cfg.table_rows, batch, dtype=np.int64)
+        if stride > 1:
+            ids = ids // stride * stride + rng.integers(0, 40, batch) % stride
+        ids[: batch // 5] = ids[0]
+        # Positive values: an id has up to some hundred copies here, and a sum of k terms of one sign is
+        # within k * 6e-8 of the sum (1e-5 is compared); where signs cancel, nothing relative holds.
+        grads = np.abs(synth.normal_rows(rng, batch, cfg.dim, cfg.grad_sigma)) + np.float32(1e-4)
+        _check_step(path, orc, ids, grads, it)
