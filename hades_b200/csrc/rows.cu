@@ -210,11 +210,12 @@ __global__ void __launch_bounds__(kBlock) accumulate_rows_kernel(
 }
 
 // ---- fused lookup + fetch, LSU ---------------------------------------------------
-template <int MODE, int VB>
+template <int MODE, int VB, bool FULL>
 __global__ void __launch_bounds__(kBlock) lookup_fetch_kernel(
     IndexView v, const int64_t* __restrict__ ids, int64_t n, const char* __restrict__ cache_rows,
     const char* __restrict__ backing, int64_t row_bytes, char* __restrict__ out,
-    int64_t* __restrict__ locs, uint8_t* __restrict__ found, int glog2, int per) {
+    int64_t* __restrict__ locs, uint8_t* __restrict__ found, int glog2, int per_arg) {
+  const int per = FULL ? 32 : per_arg;
   using V = typename Vec<VB>::T;
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kBlock) lookup_fetch_kernel(
   const int rows_per_pass = 32 >> glog2;
   const int64_t vpr = row_bytes / VB;
   for (int64_t base = warp * per; base < n; base += nwarps * per) {
-    const int64_t i = lane < per ? base + lane : n;
+    const int64_t i = FULL || lane < per ? base + lane : n;
     const int64_t id = i < n ? __ldg(ids + i) : -1;
     const int64_t slot = warp_lookup<MODE>(v, s_top, id);
     if (i < n) {
@@ -242,7 +243,7 @@ __global__ void __launch_bounds__(kBlock) lookup_fetch_kernel(
     else if (backing && id >= 0) src = backing + id * row_bytes;
     const unsigned long long src_bits = (unsigned long long)src;
     // G lanes per row, 32/G rows per pass, kRows passes in flight
-    for (int p = 0; p * rows_per_pass < per; p += kRows) {
+    for (int p = 0; FULL ? p < G : p * rows_per_pass < per; p += kRows) {
       const V* s[kRows];
       V* d[kRows];
 #pragma unroll
@@ -271,11 +272,12 @@ __global__ void __launch_bounds__(kBlock) lookup_fetch_kernel(
 // The 32 rows of a warp's chunk go in 8 batches of 4; with DEPTH = 2 the loads of
 // batch b+1 are issued before the stores of batch b, which doubles the bytes a warp
 // keeps in flight without waiting.
-template <int MODE, int MINB, int DEPTH>
+template <int MODE, int MINB, int DEPTH, bool FULL>
 __global__ void __launch_bounds__(kBlock, MINB) lookup_fetch512_kernel(
     IndexView v, const int64_t* __restrict__ ids, int64_t n, const char* __restrict__ cache_rows,
     const char* __restrict__ backing, char* __restrict__ out, int64_t* __restrict__ locs,
-    uint8_t* __restrict__ found, int per) {
+    uint8_t* __restrict__ found, int per_arg) {
+  const int per = FULL ? 32 : per_arg;
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(kBlock, MINB) lookup_fetch512_kernel(
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t base = warp * per; base < n; base += nwarps * per) {
-    const int64_t i = lane < per ? base + lane : n;
+    const int64_t i = FULL || lane < per ? base + lane : n;
     const int64_t id = i < n ? __ldg(ids + i) : -1;
     const int64_t slot = warp_lookup<MODE>(v, s_top, id);
     if (i < n) {
@@ -317,7 +319,7 @@ __global__ void __launch_bounds__(kBlock, MINB) lookup_fetch512_kernel(
     if (DEPTH == 1) {
 #pragma unroll
       for (int b = 0; b < 8; ++b) {
-        if (b * 4 >= per) break;
+        if (!FULL && b * 4 >= per) break;
         load(b, buf[0]);
         store(b, buf[0]);
       }
@@ -754,30 +756,33 @@ int hb_lookup_fetch(hb_index_t* h, const int64_t* ids, int64_t n, const void* ca
     // dim 128 fp32: the specialised kernel (measured 2-4 % faster than the generic mover;
     // deeper prefetch or 4 CTAs/SM measured no better: the kernel sits at the random-row
     // bandwidth of the memory system)
-    if (mode == HB_LOOKUP_SORTED)
-      HB_LAUNCH((lookup_fetch512_kernel<HB_LOOKUP_SORTED, 3, 1>), blocks, kBlock, 0, st, h->view,
-                ids, n, (const char*)cache_rows, (const char*)backing_rows, (char*)out_rows, locs, found, per);
-    else
-      HB_LAUNCH((lookup_fetch512_kernel<HB_LOOKUP_SETASSOC, 3, 1>), blocks, kBlock, 0, st, h->view,
-                ids, n, (const char*)cache_rows, (const char*)backing_rows, (char*)out_rows, locs, found, per);
+#define HB_LF512(MODE, FULL)                                                                       \
+  HB_LAUNCH((lookup_fetch512_kernel<MODE, 3, 1, FULL>), blocks, kBlock, 0, st, h->view, ids, n,     \
+            (const char*)cache_rows, (const char*)backing_rows, (char*)out_rows, locs, found, per)
+    if (mode == HB_LOOKUP_SORTED) {
+      if (per == 32) HB_LF512(HB_LOOKUP_SORTED, true); else HB_LF512(HB_LOOKUP_SORTED, false);
+    } else {
+      if (per == 32) HB_LF512(HB_LOOKUP_SETASSOC, true); else HB_LF512(HB_LOOKUP_SETASSOC, false);
+    }
+#undef HB_LF512
     return HB_OK;
   }
-#define HB_LF(MODE, VB)                                                                         \
-  HB_LAUNCH((lookup_fetch_kernel<MODE, VB>), blocks, kBlock, 0, st, h->view, ids, n,       \
+#define HB_LF(MODE, VB, FULL)                                                                         \
+  HB_LAUNCH((lookup_fetch_kernel<MODE, VB, FULL>), blocks, kBlock, 0, st, h->view, ids, n,       \
             (const char*)cache_rows, (const char*)backing_rows, row_bytes, (char*)out_rows, locs, \
             found, glog2, per)
-#define HB_LF_VB(MODE)                 \
-  switch (vb) {                        \
-    case 16: HB_LF(MODE, 16); break;   \
-    case 8: HB_LF(MODE, 8); break;     \
-    case 4: HB_LF(MODE, 4); break;     \
-    case 2: HB_LF(MODE, 2); break;     \
-    default: HB_LF(MODE, 1); break;    \
+#define HB_LF_VB(MODE, FULL)                 \
+  switch (vb) {                              \
+    case 16: HB_LF(MODE, 16, FULL); break;   \
+    case 8: HB_LF(MODE, 8, FULL); break;     \
+    case 4: HB_LF(MODE, 4, FULL); break;     \
+    case 2: HB_LF(MODE, 2, FULL); break;     \
+    default: HB_LF(MODE, 1, FULL); break;    \
   }
   if (mode == HB_LOOKUP_SORTED) {
-    HB_LF_VB(HB_LOOKUP_SORTED)
+    if (per == 32) { HB_LF_VB(HB_LOOKUP_SORTED, true) } else { HB_LF_VB(HB_LOOKUP_SORTED, false) }
   } else {
-    HB_LF_VB(HB_LOOKUP_SETASSOC)
+    if (per == 32) { HB_LF_VB(HB_LOOKUP_SETASSOC, true) } else { HB_LF_VB(HB_LOOKUP_SETASSOC, false) }
   }
 #undef HB_LF_VB
 #undef HB_LF

@@ -40,6 +40,7 @@ constexpr int64_t kSideMin = 32768;
 // update has many rows in flight whatever the lengths of the runs.
 // The line lies where the two cost the same (65,536 ids of 128 columns: 149 us the step fused, 154 not;
 // 150,000 of 64: 167 and 162; 2,000,000 of 128: 903 and 846).
+// In a captured step the fetch runs beside the sums instead.
 constexpr int64_t kFuseMax = 100000;
 bool fuses_update(int64_t n) { return n <= kFuseMax; }
 
@@ -80,7 +81,7 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
   p.listed = cv.take<unsigned long long>(1);
   p.seg_bytes = seg_plan(nullptr, m, dim).total;
   p.seg_ws = cv.take<char>(p.seg_bytes);
-  p.sums = cv.take<float>(fuses_update(m) ? 0 : (size_t)m * dim);
+  p.sums = cv.take<float>((size_t)m * dim);
   p.total = cv.used() + 256;
   return p;
 }
@@ -140,6 +141,12 @@ __global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_ru
     a.run_slots[u] = slot;
     if (a.touch) marks.mark(slot, u);
   }
+}
+
+// in a graph a second stream costs no host time and no events
+bool captured(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
 }
 
 int join_side(hb_step* s, cudaStream_t st) {
@@ -422,7 +429,8 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
   if (rc != HB_OK) return rc;
   // HB_STEP_ASIDE: all of the fetch leaves the caller's stream, which goes on to the aggregation of the
   // same batch (it needs the sort only); both are bound by HBM, but not all the time
-  const bool aside = join == HB_STEP_ASIDE && !fuses_update(n);
+  const bool in_graph = captured(st);
+  const bool aside = join == HB_STEP_ASIDE && (in_graph || !fuses_update(n));
   if (aside) {
     HB_CUDA(cudaEventRecord(s->forked, st));
     HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
@@ -439,7 +447,7 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
     HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a, marks,
               lists, device_error_word());
   const bool maintain = d->touch_lru || d->insert_misses;
-  const bool beside = !aside && maintain && n >= kSideMin;
+  const bool beside = !aside && maintain && (in_graph || n >= kSideMin);
   cudaStream_t side = beside ? s->side : st;
   if (beside) {
     HB_CUDA(cudaEventRecord(s->forked, st));
@@ -493,7 +501,7 @@ int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, 
   }
   cudaStream_t st = (cudaStream_t)stream;
   hb_index* h = d->index;
-  const bool fused = fuses_update(n);
+  const bool fused = fuses_update(n) && !captured(st);
   if (ids || fused) {
     rc = join_side(s, st);
     if (rc != HB_OK) return rc;

@@ -75,7 +75,8 @@ class _OneGpuStep:
     ``forward`` and ``backward`` of the path compose from separate operators when other GPUs take part."""
 
     def __init__(self, path: "EmbeddingPath"):
-        self.path = path
+        # (no reference to the path: a cycle would keep the table and the optimiser's state until a
+        # garbage collection)
         self.lib, self.native = E._lib.load(), E._lib.native()
         h = C.c_void_p()
         E._lib.check(self.lib.hb_step_create(C.byref(h)))
@@ -85,7 +86,7 @@ class _OneGpuStep:
         self.ws, self.kept = None, []
         self.batch = None  # (ids, version, counters) of the last forward pass
         self.key = None
-        self.refresh()
+        self.refresh(path)
         self.supported = bool(self.lib.hb_step_supported(C.byref(self.desc)))
 
     def __del__(self):
@@ -94,9 +95,9 @@ class _OneGpuStep:
         except Exception:  # interpreter shutdown
             pass
 
-    def refresh(self) -> None:
+    def refresh(self, p: "EmbeddingPath") -> None:
         """The description follows the path's attributes (they may change between steps)."""
-        p, d = self.path, self.desc
+        d = self.desc
         cold, opt = p.cold, p.opt
         key = (p.lookup_mode, p.touch_lru, p.insert_misses, p.miss_cap, p.id_bits, cold.default_threshold, opt._lr,
                p.table.data_ptr(), p.class_table.data_ptr(), cold.emb.data_ptr(), opt.emb.weight.data_ptr())
@@ -112,32 +113,31 @@ class _OneGpuStep:
         d.threshold_table = None if cold.threshold is None else cold.threshold.data_ptr()
         d.dropped, d.opt = cold.dropped.data_ptr(), opt._desc()
 
-    def keep(self, ws: torch.Tensor) -> None:
+    def keep(self, p: "EmbeddingPath", ws: torch.Tensor) -> None:
         """Scratch of the last batch.  What captured graphs hold stays."""
         if ws is not self.ws:
-            if self.ws is not None and self.path._graphs_hold_scratch():
+            if self.ws is not None and p._graphs_hold_scratch():
                 self.kept.append(self.ws)
             self.ws = ws
 
-    def forward(self, ids: torch.Tensor, out_rows, join: int):
+    def forward(self, p: "EmbeddingPath", ids: torch.Tensor, out_rows, join: int):
         """join: HB_STEP_BESIDE / HB_STEP_JOIN / HB_STEP_ASIDE."""
-        p = self.path
         ids = ids.contiguous()
-        self.refresh()
+        self.refresh(p)
         rows, locs, found, counters, ws = self.native.step_forward(
             self._h.value, self.addr, ids, p.dim, p.cold.emb, out_rows, p.want_locs, join, self.ws)
-        self.keep(ws)
+        self.keep(p, ws)
         self.batch = (ids, ids._version, counters)
         return rows, locs, found
 
-    def backward(self, ids: torch.Tensor, grads: torch.Tensor) -> StepStats:
-        p, n = self.path, ids.numel()
+    def backward(self, p: "EmbeddingPath", ids: torch.Tensor, grads: torch.Tensor) -> StepStats:
+        n = ids.numel()
         _check(grads.dtype == torch.float32 and grads.shape == (n, p.dim), "grads is fp32 [len(ids), dim]")
         grads = grads.contiguous()
         if p.dim > 128 and grads.data_ptr() & 15:
             grads = grads.clone()  # wide rows are read 16 bytes at a time
         b = self.batch
-        self.refresh()
+        self.refresh(p)
         if b is not None and (ids is b[0] or (ids.data_ptr() == b[0].data_ptr() and n == b[0].numel())) \
                 and ids._version == b[1]:
             counters, given = b[2], None
@@ -150,7 +150,7 @@ class _OneGpuStep:
             if self.ws is None or self.ws.numel() < need:
                 # (the call joins the side stream, which may still use the old scratch, before it writes)
                 self.join()
-                self.keep(torch.empty(need, dtype=torch.uint8, device=ids.device))
+                self.keep(p, torch.empty(need, dtype=torch.uint8, device=ids.device))
         self.native.step_backward(self._h.value, self.addr, given, n, grads, counters, self.ws)
         return _CounterStats(counters)
 
@@ -262,7 +262,7 @@ class EmbeddingPath:
         n = ids.numel()
         if self._one is not None and n > 0:
             self._last = None
-            return self._one.forward(ids, out_rows, 2 if on_side else int(join))
+            return self._one.forward(self, ids, out_rows, 2 if on_side else int(join))
         lib = E._lib.load()
         runs = E.cudaRunsBuild(ids, self.id_bits, self.class_table, keep=(False, True, True),
                                caps=(None, self.num_hot_ids, None),
@@ -481,7 +481,7 @@ class EmbeddingPath:
         GPUs' shards, and the owner update until it has read what it needs from this GPU's shard:
         a fetch returns the rows as they were before the step's update."""
         if self._one is not None and ids.numel() > 0:
-            return self._one.backward(ids, grads)
+            return self._one.backward(self, ids, grads)
         st, hot_ids, hot_rows, hot_cnt = self._backward_local(ids, grads, join=False)
         n_hot = st.split_counts[HOT:HOT + 1]
         if self.world > 1:
