@@ -8,6 +8,7 @@
 
 #include "index.cuh"
 #include "launch.cuh"
+#include "maintain.cuh"
 #include "sortcore.cuh"
 
 namespace hb {
@@ -28,85 +29,11 @@ __global__ void fill_i32_kernel(int32_t* p, int64_t n, int32_t v) {
 }
 
 // ---- add ---------------------------------------------------------------------
-// The line of one set in registers.  Placement policy: src/cache/cache.h:51-88 with
-// find_or_empty_entry (cache_line.h:67-78) and find_lru (cache_line.h:92-103).
-struct LineState {
-  int64_t lid[kWays];
-  int32_t cnt[kWays];
-  int last[kWays];  // which id of the batch was placed in each way last, -1 = none
-
-  __device__ __forceinline__ void load(const int64_t* line_ids, const int32_t* lru, int64_t line) {
-    const longlong2* p = reinterpret_cast<const longlong2*>(line_ids + line * kWays);
-    const int4* q = reinterpret_cast<const int4*>(lru + line * kWays);
-#pragma unroll
-    for (int w = 0; w < kWays; w += 2) {
-      const longlong2 v = p[w / 2];
-      lid[w] = v.x;
-      lid[w + 1] = v.y;
-    }
-#pragma unroll
-    for (int w = 0; w < kWays; w += 4) {
-      const int4 v = q[w / 4];
-      cnt[w] = v.x; cnt[w + 1] = v.y; cnt[w + 2] = v.z; cnt[w + 3] = v.w;
-    }
-#pragma unroll
-    for (int w = 0; w < kWays; ++w) last[w] = -1;
-  }
-  __device__ __forceinline__ void store(int64_t* line_ids, int32_t* lru, int64_t line) const {
-    longlong2* p = reinterpret_cast<longlong2*>(line_ids + line * kWays);
-    int4* q = reinterpret_cast<int4*>(lru + line * kWays);
-#pragma unroll
-    for (int w = 0; w < kWays; w += 2) p[w / 2] = make_longlong2(lid[w], lid[w + 1]);
-#pragma unroll
-    for (int w = 0; w < kWays; w += 4) q[w / 4] = make_int4(cnt[w], cnt[w + 1], cnt[w + 2], cnt[w + 3]);
-  }
-  // places the k-th id of the batch for this set; the way, -1 = refused
-  __device__ __forceinline__ int place(int64_t id, int k) {
-    int way = -1;
-    bool exists = false;
-#pragma unroll
-    for (int w = 0; w < kWays; ++w) {
-      if (!exists) {
-        if (lid[w] == id) { way = w; exists = true; }
-        else if (lid[w] == -1) way = w;  // keeps the LAST empty way
-      }
-    }
-    if (way < 0) {
-      // no empty way: least recently used = largest non-zero counter, first on ties
-      int best = 0;
-      int32_t tmp = cnt[0];
-#pragma unroll
-      for (int w = 0; w < kWays; ++w) {
-        if (cnt[w] > tmp && cnt[w] != 0) { best = w; tmp = cnt[w]; }
-      }
-      way = tmp == 0 ? -1 : best;
-    }
-#pragma unroll
-    for (int w = 0; w < kWays; ++w)
-      if (w == way) {
-        if (!exists) { lid[w] = id; cnt[w] = 0; }  // set_id zeroes the counter
-        last[w] = k;
-      }
-    return way;
-  }
-  __device__ __forceinline__ bool is_last(int64_t loc, int k) const {
-    if (loc < 0) return false;
-    const int way = (int)(loc & (kWays - 1));
-    bool yes = false;
-#pragma unroll
-    for (int w = 0; w < kWays; ++w)
-      if (w == way) yes = last[w] == k;
-    return yes;
-  }
-};
-
 // Two ways to the ids of a set in input order.
 //
 // (1) Sorted by set (sortcore.cuh), input order kept inside a set; one thread per set walks them.  For
 //     small batches (one launch), for batches of many ids per set, and (LONG_LISTS) for the sets that
 //     (2) leaves behind, usually none.
-constexpr uint32_t kLongList = 0xffffffffu;  // in place of the entry: the set's list is long
-
 template <bool LONG_LISTS>
 struct SetSource {
   static constexpr bool kSkips = LONG_LISTS;
@@ -115,12 +42,13 @@ struct SetSource {
   int64_t lines;
   const unsigned long long* heads;
   const int32_t* batch;
-  __device__ __forceinline__ int64_t count() const { return !LONG_LISTS || batch[4] == batch[2] ? n : 0; }
+  __device__ __forceinline__ int known_bits() const { return 0; }
+  __device__ __forceinline__ int64_t count() const { return !LONG_LISTS || batch[2] == batch[0] ? n : 0; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
     const int64_t x = __ldg(ids + i);
     if (x < 0) return false;  // unusable (padding)
     key = (unsigned long long)mod_nonneg(x, lines);
-    return !LONG_LISTS || heads[key] == (((unsigned long long)(uint32_t)batch[2] << 32) | kLongList);
+    return !LONG_LISTS || heads[key] == (((unsigned long long)(uint32_t)batch[0] << 32) | kLongList);
   }
 };
 
@@ -193,79 +121,6 @@ __global__ void __launch_bounds__(kBlock) add_push_kernel(const int64_t* __restr
   }
 }
 
-constexpr int kListShort = 32;  // ids of a set that are put in order in a thread's own memory
-
-// Orders a long list (entry numbers + 1, linked through next) ascending: merge sort, bottom up.
-__device__ __noinline__ uint32_t sort_list(uint32_t head, uint32_t* next) {
-  for (uint32_t size = 1;; size *= 2) {
-    uint32_t p = head, tail = 0;
-    head = 0;
-    int merges = 0;
-    while (p) {
-      ++merges;
-      uint32_t q = p, np = 0, nq = size;
-      while (np < size && q) { ++np; q = next[q - 1]; }
-      while (np || (nq && q)) {
-        uint32_t e;
-        if (np && (!nq || !q || p < q)) { e = p; p = next[p - 1]; --np; }
-        else { e = q; q = next[q - 1]; --nq; }
-        if (tail) next[tail - 1] = e; else head = e;
-        tail = e;
-      }
-      p = q;
-    }
-    next[tail - 1] = 0;
-    if (merges <= 1) return head;
-  }
-}
-
-// where the first `cap` listed entries end (a block finds it together); the usual case: nothing to cut
-__device__ __forceinline__ int64_t add_cut(const AddEntries& e, int64_t n) {
-  __shared__ long long s_cut[2];
-  if (!e.total || (int64_t)*e.total <= e.cap) return n;
-  __shared__ int s_warp[kBlock / 32];
-  const int64_t chunks = (n + 31) / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int64_t left = e.cap;  // listed entries still allowed
-  for (int64_t c0 = 0; c0 < chunks; c0 += kBlock * 16) {
-    const int64_t c = c0 + threadIdx.x * 16;
-    int mine = 0;
-    for (int x = 0; x < 16; ++x)
-      if (c + x < chunks) mine += __ldg(e.chunk_listed + c + x);
-    int inc = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += t;
-    }
-    if (lane == 31) s_warp[warp] = inc;
-    if (threadIdx.x == 0) s_cut[0] = -1;
-    __syncthreads();
-    int before = 0, all = 0;
-    for (int w = 0; w < kBlock / 32; ++w) {
-      if (w < warp) before += s_warp[w];
-      all += s_warp[w];
-    }
-    const int64_t first = before + inc - mine;  // listed entries of this round ahead of this thread's
-    if (left >= first && left < first + mine) {
-      int64_t need = left - first;
-      int x = 0;
-      while (need >= __ldg(e.chunk_listed + c + x)) { need -= __ldg(e.chunk_listed + c + x); ++x; }
-      int64_t i = (c + x) * 32;
-      const int64_t end = i + 32 < n ? i + 32 : n;
-      for (; i < end; ++i)
-        if (e.listed[i] && need-- == 0) break;
-      s_cut[0] = i;
-    }
-    __syncthreads();
-    const int64_t cut = s_cut[0];
-    if (cut >= 0) return cut;
-    left -= all;
-    __syncthreads();
-  }
-  return n;
-}
-
 // the runs of a batch that are on lists, sorted by set instead (many ids per set)
 struct ListedSource {
   static constexpr bool kSkips = false;
@@ -275,6 +130,7 @@ struct ListedSource {
   const uint8_t* listed;
   const int64_t* cut;
   int64_t lines;
+  __device__ __forceinline__ int known_bits() const { return 0; }
   __device__ __forceinline__ int64_t count() const { return *n_dev < n ? *n_dev : n; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
     key = (unsigned long long)mod_nonneg(__ldg(ids + i), lines);
@@ -283,79 +139,22 @@ struct ListedSource {
 };
 
 __global__ void __launch_bounds__(kBlock) add_cut_kernel(AddEntries e, int64_t* cut) {
-  const int64_t c = add_cut(e, *e.n_dev < e.n ? *e.n_dev : e.n);
+  const int64_t c = add_cut<kBlock>(e, *e.n_dev < e.n ? *e.n_dev : e.n);
   if (threadIdx.x == 0) *cut = c;
 }
 
-template <bool DISTINCT>
-__global__ void __launch_bounds__(kBlock) add_walk_kernel(AddEntries e, unsigned long long* __restrict__ heads,
-                                                          int32_t* batch, uint32_t* __restrict__ next, int64_t lines,
-                                                          int64_t* __restrict__ line_ids, int32_t* __restrict__ lru,
-                                                          int64_t* __restrict__ locs, uint8_t* __restrict__ last_writer) {
-  const uint32_t number = batch_number(batch + 2);
-  int64_t n = e.n;
-  if (e.n_dev && *e.n_dev < n) n = *e.n_dev;
-  const int64_t cut = add_cut(e, n);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const bool listed = e.listed ? e.listed[i] != 0 : true;
-    if (!listed) continue;
+__global__ void __launch_bounds__(kBlock) add_walk_kernel(AddEntries e, AddState a) {
+  const uint32_t number = batch_number(a.batch);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < e.n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t id = __ldg(e.ids + i);
     if (id < 0) continue;
-    const int64_t line = mod_nonneg(id, lines);
-    if (heads[line] != (((unsigned long long)number << 32) | (unsigned long long)(i + 1))) continue;
+    const int64_t line = mod_nonneg(id, a.lines);
+    if (a.heads[line] != (((unsigned long long)number << 32) | (unsigned long long)(i + 1))) continue;
     LineState st;
-    st.load(line_ids, lru, line);
-    uint32_t behind = next[i];
-    if (!behind) {  // the usual case: one id for the set
-      const bool taken = i < cut;
-      const int way = taken ? st.place(id, 0) : -1;
-      locs[i] = way >= 0 ? line * kWays + way : -1;
-      if (last_writer) last_writer[i] = way >= 0;
-      if (way >= 0) st.store(line_ids, lru, line);
-      continue;
-    }
-    uint32_t order[kListShort];
-    int len = 0;
-    uint32_t at = (uint32_t)i + 1u;
-    for (; at && len < kListShort; at = next[at - 1]) {
-      int k = len++;
-      for (; k > 0 && order[k - 1] > at; --k) order[k] = order[k - 1];
-      order[k] = at;
-    }
-    if (at && DISTINCT) {
-      // only ids in strides of the number of sets come here: no launch is kept ready for them
-      const uint32_t first = sort_list((uint32_t)i + 1u, next);
-      int k = 0;
-      for (at = first; at; at = next[at - 1], ++k) {
-        const int64_t x = (int64_t)at - 1;
-        const int way = x < cut ? st.place(__ldg(e.ids + x), k) : -1;
-        locs[x] = way >= 0 ? line * kWays + way : -1;
-      }
-      if (last_writer) {
-        k = 0;
-        for (at = first; at; at = next[at - 1], ++k) last_writer[at - 1] = st.is_last(locs[at - 1], k);
-      }
-      st.store(line_ids, lru, line);
-      continue;
-    }
-    if (at) {
-      heads[line] = ((unsigned long long)number << 32) | kLongList;
-      batch[4] = (int32_t)number;
-      continue;
-    }
-    for (int k = 0; k < len; ++k) {
-      const int64_t x = (int64_t)order[k] - 1;
-      const int way = x < cut ? st.place(__ldg(e.ids + x), k) : -1;
-      locs[x] = way >= 0 ? line * kWays + way : -1;
-    }
-    if (last_writer)
-      for (int k = 0; k < len; ++k) {
-        const int64_t x = (int64_t)order[k] - 1;
-        last_writer[x] = st.is_last(locs[x], k);
-      }
-    st.store(line_ids, lru, line);
+    st.load(a.line_ids, a.lru, line);
+    walk_list<false>(e, a, i, e.n, number, line, id, st);
   }
-  batch_done(batch + 2, number);
+  batch_done(a.batch, number, gridDim.x);
 }
 
 // ---- lookup ------------------------------------------------------------------
@@ -420,18 +219,6 @@ __global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const i
   }
 }
 
-// ways of a line that the batch hit: their last positions, 0 = not hit
-__device__ __forceinline__ void line_marks(const unsigned long long* marks, int64_t line, uint32_t number,
-                                           uint32_t (&last)[kWays]) {
-  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(marks + line * kWays);
-#pragma unroll
-  for (int w = 0; w < kWays; w += 2) {
-    const ulonglong2 x = p[w / 2];
-    last[w] = (uint32_t)(x.x >> 32) == number ? (uint32_t)x.x : 0u;
-    last[w + 1] = (uint32_t)(x.y >> 32) == number ? (uint32_t)x.y : 0u;
-  }
-}
-
 __global__ void __launch_bounds__(kBlock) touch_after_kernel(const int64_t* __restrict__ locs, int64_t n, TouchMarks t,
                                                              int32_t* __restrict__ after) {
   const uint32_t number = batch_number(t.batch);
@@ -487,7 +274,7 @@ __global__ void __launch_bounds__(kBlock) touch_apply_kernel(const int64_t* __re
       }
     }
   }
-  batch_done(t.batch, number);
+  batch_done(t.batch, number, gridDim.x);
 }
 
 // ---- LRU touch from runs -------------------------------------------------------
@@ -500,42 +287,7 @@ __global__ void touch_runs_mark_kernel(RunsView v, TouchMarks marks) {
 }
 
 __global__ void __launch_bounds__(kBlock) touch_runs_apply_kernel(RunsView v, TouchMarks t, int32_t* __restrict__ lru) {
-  const uint32_t number = batch_number(t.batch);
-  const int64_t nruns = v.runs();
-  const int64_t npos = v.positions();
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nruns; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t slot = v.slot_of_run(u);
-    if (slot < 0 || slot >= t.capacity) continue;
-    const int64_t line = slot >> 3;
-    const int way = (int)(slot & 7);
-    uint32_t run[kWays];
-    line_marks(t.marks, line, number, run);
-    const int64_t end = v.end(u, nruns, npos);
-    const int64_t last = v.pos(end - 1);
-    int32_t total = (int32_t)(end - v.start(u)), after = 0;
-    bool leader = true;
-#pragma unroll
-    for (int w = 0; w < kWays; ++w) {
-      if (!run[w] || w == way) continue;
-      const int64_t u2 = (int64_t)run[w] - 1;
-      const int64_t s2 = v.start(u2), e2 = v.end(u2, nruns, npos);
-      total += (int32_t)(e2 - s2);
-      if (w < way) leader = false;
-      int64_t lo = s2, hi = e2;  // first position of the run greater than `last`
-      while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (v.pos(mid) <= last) lo = mid + 1; else hi = mid;
-      }
-      after += (int32_t)(e2 - lo);
-    }
-    lru[slot] = after;
-    if (leader) {
-#pragma unroll
-      for (int w = 0; w < kWays; ++w)
-        if (!run[w] && w != way) lru[line * kWays + w] += total;
-    }
-  }
-  batch_done(t.batch, number);
+  touch_runs(v, t, lru, blockIdx.x, gridDim.x);
 }
 
 // ---- reset -------------------------------------------------------------------
@@ -669,20 +421,20 @@ static size_t add_workspace_bytes(int64_t n) {
 size_t index_add_runs_bytes(int64_t n) { return add_workspace_bytes(n); }
 bool index_add_runs_lists(const hb_index* h, int64_t n) { return n <= kListedPerSet * h->lines; }
 
-int index_add_runs(hb_index* h, const AddEntries& e, void* ws, int64_t* locs, uint8_t* last_writer, cudaStream_t st) {
+int index_add_runs_sorted(hb_index* h, const AddEntries& e, void* ws, int64_t* locs, uint8_t* last_writer,
+                          cudaStream_t st) {
   Carver cv(ws);
-  uint32_t* next = cv.take<uint32_t>(e.n);
-  h->sorted_stale = true;
-  if (index_add_runs_lists(h, e.n)) {
-    HB_LAUNCH(add_walk_kernel<true>, grid_capped(e.n), kBlock, 0, st, e, h->heads, h->batch, next, h->lines,
-              h->line_ids, h->lru, locs, last_writer);
-    return HB_OK;
-  }
   uint2* sorted = cv.take<uint2>(e.n);
   int64_t* cut = cv.take<int64_t>(1);
   HB_LAUNCH(add_cut_kernel, 1, kBlock, 0, st, e, cut);
   return sort_run(ListedSource{e.ids, e.n, e.n_dev, e.listed, cut, h->lines},
                   AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, e.n, cv.take<char>(0), st);
+}
+
+int index_add_state(hb_index* h, uint32_t* next, int64_t* locs, uint8_t* last_writer, AddState* out) {
+  *out = AddState{h->heads, h->batch + 2, next, h->lines, h->line_ids, h->lru, locs, last_writer};
+  h->sorted_stale = true;
+  return HB_OK;
 }
 
 }  // namespace hb
@@ -854,9 +606,11 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
     memset(&e, 0, sizeof(e));
     e.ids = ids;
     e.n = n;
-    HB_LAUNCH(add_walk_kernel<false>, grid_capped(n), kBlock, 0, st, e, h->heads, h->batch, next, h->lines, h->line_ids,
-              h->lru, locs, last_writer);
-    return sort_run(SetSource<true>{ids, n, h->lines, h->heads, h->batch},
+    AddState state;
+    rc = index_add_state(h, next, locs, last_writer, &state);
+    if (rc != HB_OK) return rc;
+    HB_LAUNCH(add_walk_kernel, grid_capped(n), kBlock, 0, st, e, state);
+    return sort_run(SetSource<true>{ids, n, h->lines, h->heads, h->batch + 2},
                     AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, n, sort_ws, st);
   }
   // (a cluster that holds more than one entry per thread leaves the walk to the whole GPU)

@@ -196,11 +196,11 @@ namespace hb {
 // One batch number for all blocks of a kernel, advanced by the block that finishes last (every block
 // has read it by then): counter[0] batches so far, counter[1] blocks done.
 __device__ __forceinline__ uint32_t batch_number(const int32_t* counter) { return (uint32_t)*counter + 1u; }
-__device__ __forceinline__ void batch_done(int32_t* counter, uint32_t number) {
+__device__ __forceinline__ void batch_done(int32_t* counter, uint32_t number, int blocks) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    if (atomicAdd(reinterpret_cast<unsigned*>(counter + 1), 1u) == gridDim.x - 1) {
+    if (atomicAdd(reinterpret_cast<unsigned*>(counter + 1), 1u) == (unsigned)blocks - 1u) {
       counter[1] = 0;
       counter[0] = (int32_t)number;
     }
@@ -285,11 +285,12 @@ struct AddEntries {
 int index_touch_marks(hb_index* h, TouchMarks* out, cudaStream_t st);
 int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st);
 int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st);
-// add() of the distinct ids of a batch that `listed` names: slots into locs and "last writer of its
-// slot" flags for them; beyond the cap -1 / 0.  Where index_add_runs_lists says so the lists have been
-// filled before (AddLists, `next` at the start of the workspace).
+// add() of the distinct ids of a batch that `listed` names: slots and "last writer of its slot" flags
+// for them; beyond the cap -1 / 0.  Where index_add_runs_lists says so through the lists of their sets
+// (AddLists, Maintain), else sorted by set.
 size_t index_add_runs_bytes(int64_t n);
 bool index_add_runs_lists(const hb_index* h, int64_t n);
-int index_add_runs(hb_index* h, const AddEntries& e, void* ws, int64_t* locs, uint8_t* last_writer, cudaStream_t st);
+int index_add_runs_sorted(hb_index* h, const AddEntries& e, void* ws, int64_t* locs, uint8_t* last_writer,
+                          cudaStream_t st);
 
 }  // namespace hb

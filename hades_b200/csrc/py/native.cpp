@@ -207,7 +207,7 @@ PyObject* unique_update(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   });
 }
 
-// step_forward(step, desc, ids, dim, row dtype tensor, out_rows | None, want_locs, join, ws | None)
+// step_forward(step, desc, ids, dim, row dtype tensor, out_rows | None, want_locs, aside, ws | None)
 // -> (rows, locs | None, found, counters, ws)
 PyObject* step_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
@@ -229,7 +229,7 @@ PyObject* step_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!ws.defined() || ws.numel() < (int64_t)need) ws = cuda_empty({(int64_t)(need + need / 4)}, at::kByte, dev);
     check(hb_step_forward(static_cast<hb_step_t*>(pointer(a[0])), static_cast<const hb_step_desc_t*>(pointer(a[1])),
                           ids.data_ptr<int64_t>(), n, out.data_ptr(), locs.defined() ? locs.data_ptr<int64_t>() : nullptr,
-                          static_cast<uint8_t*>(found.data_ptr()), counters.data_ptr<int64_t>(), (int)integer(a[7]),
+                          static_cast<uint8_t*>(found.data_ptr()), counters.data_ptr<int64_t>(), PyObject_IsTrue(a[7]),
                           ws.data_ptr(), (size_t)ws.numel(), stream_of(dev)));
     return pack({THPVariable_Wrap(out), wrap_or_none(locs), THPVariable_Wrap(found), THPVariable_Wrap(counters),
                  THPVariable_Wrap(ws)});

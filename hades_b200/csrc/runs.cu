@@ -15,6 +15,7 @@
 #include "a2a.cuh"
 #include "compact.cuh"
 #include "index.cuh"
+#include "maintain.cuh"
 #include "runs.cuh"
 #include "shard.cuh"
 #include "sortcore.cuh"
@@ -38,6 +39,8 @@ struct IdSource {
   uint32_t seg_cap;
   int64_t sentinel;
   int* err;
+  int bits;  // stated by the caller
+  __device__ __forceinline__ int known_bits() const { return bits; }
   __device__ __forceinline__ int64_t count() const {
     if (!n_dev) return n;
     const int64_t d = *n_dev;
@@ -457,17 +460,28 @@ __device__ __forceinline__ int64_t run_of_entry(const hb_runs_t& r, int64_t j) {
 // RB: 512 = rows of exactly 512 bytes (128 fp32: the address arithmetic folds, no lane is idle);
 // 16 = any multiple of 16 bytes; 0 = words or bytes.  PEER: a source may be another GPU's memory
 // (runs that found no room in the stage), so rows are read with plain loads.
-template <bool PEER, int RB>
+// MAINTAIN: the first blocks of the launch bring the index up to date meanwhile (a chain of dependent
+// reads beside a stream of rows: a second launch of it costs more than it takes).
+template <bool PEER, int RB, bool MAINTAIN>
 __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
     hb_runs_t r, const unsigned long long* __restrict__ run_src, const int64_t* __restrict__ run_slots,
     int64_t row_bytes_arg, int vb, char* __restrict__ out, int64_t* __restrict__ locs,
-    uint8_t* __restrict__ found, int per) {
+    uint8_t* __restrict__ found, int per, Maintain duty) {
+  int block = blockIdx.x, blocks = gridDim.x;
+  if (MAINTAIN) {
+    if (block < duty.blocks) {
+      duty.template run<kBlock>(block);
+      return;
+    }
+    block -= duty.blocks;
+    blocks -= duty.blocks;
+  }
   constexpr bool V16 = RB != 0;
   const int64_t row_bytes = RB == 512 ? (int64_t)512 : row_bytes_arg;
   const int64_t n = runs_valid_entries(r);
   const int lane = lane_id();
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * per;
+  const int64_t warp = (block * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t stride = (((int64_t)blocks * blockDim.x) >> 5) * per;
   int64_t base = warp * per;
   uint32_t pos_next = 0;
   int64_t run_next = -1;
@@ -674,7 +688,7 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
   const int64_t sentinel = id_bits >= 63 ? INT64_MAX : (((int64_t)1 << id_bits) - 1);
   runs_out->perm = s.perm;
   IdSource src{ids, n, seg_counts ? nullptr : n_dev, seg_counts, (uint32_t)(seg_counts ? seg_cap : 1), sentinel,
-               device_error_word()};
+               device_error_word(), id_bits};
   RunsFinish fin{class_table, table_len, s.perm, s.head, s.uniq, uniq_ids_out, s.run_start,
                  s.dclass, s.dpos,
                  {class_ids_out ? class_ids_out[0] : nullptr, class_ids_out ? class_ids_out[1] : nullptr,
@@ -831,9 +845,11 @@ int fetch_runs_impl(hb_index_t* h, const hb_runs_t* runs, const void* cache_rows
   if (!expand) return HB_OK;  // per distinct id only: slots in run_slots, remote rows staged or asked for
   const int per = items_per_warp(runs->n);
   const int grid = grid_of_warps(runs->n, per, kBlock, 32);
-#define HB_EXP(PEER, RB)                                                                         \
-  HB_LAUNCH((runs_expand_kernel<PEER, RB>), grid, kBlock, 0, st, *runs, f.run_src, slots, row_bytes, \
-            vb, (char*)out_rows, locs, found, per)
+  Maintain none;
+  memset(&none, 0, sizeof(none));
+#define HB_EXP(PEER, RB)                                                                                \
+  HB_LAUNCH((runs_expand_kernel<PEER, RB, false>), grid, kBlock, 0, st, *runs, f.run_src, slots, row_bytes, \
+            vb, (char*)out_rows, locs, found, per, none)
 #define HB_EXP_V(PEER)                                \
   do {                                                \
     if (v16 && row_bytes == 512) HB_EXP(PEER, 512);   \
@@ -846,6 +862,29 @@ int fetch_runs_impl(hb_index_t* h, const hb_runs_t* runs, const void* cache_rows
   return HB_OK;
 }
 }  // namespace
+
+}  // extern "C"
+
+int hb::runs_expand_maintain(const hb_runs_t* runs, const unsigned long long* run_src, const int64_t* run_slots,
+                             const void* cache_rows, const void* table, int64_t row_bytes, void* out_rows,
+                             int64_t* locs, uint8_t* found, const Maintain& duty, cudaStream_t st) {
+  const uintptr_t bits = (uintptr_t)row_bytes | (uintptr_t)cache_rows | (uintptr_t)out_rows | (uintptr_t)table;
+  HB_CHECK_ARG((bits & 1) == 0, "hb_step_forward: rows must start at even addresses");
+  const bool v16 = (bits & 15) == 0;
+  const int vb = v16 ? 16 : ((bits & 3) == 0 ? 4 : 1);
+  const int per = items_per_warp(runs->n);
+  const int grid = grid_of_warps(runs->n, per, kBlock, 32) + duty.blocks;
+#define HB_EXP(RB)                                                                                        \
+  HB_LAUNCH((runs_expand_kernel<false, RB, true>), grid, kBlock, 0, st, *runs, run_src, run_slots, row_bytes, \
+            vb, (char*)out_rows, locs, found, per, duty)
+  if (v16 && row_bytes == 512) HB_EXP(512);
+  else if (v16) HB_EXP(16);
+  else HB_EXP(0);
+#undef HB_EXP
+  return HB_OK;
+}
+
+extern "C" {
 
 size_t hb_lookup_fetch_runs_workspace_bytes(int64_t n, int64_t row_bytes, int sharded) {
   return make_fetch_plan(nullptr, n, row_bytes > 0 ? row_bytes : 1, sharded != 0).total;

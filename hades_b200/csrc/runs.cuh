@@ -31,6 +31,13 @@ int runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int64_
                int64_t* class_counts_out, int64_t* uniq_ids_out, int64_t* num_unique_out, unsigned* zero,
                int64_t zero_words, void* workspace, size_t workspace_bytes, hb_runs_t* runs_out, cudaStream_t st);
 
+struct Maintain;
+// The rows of a batch to its positions (run_src: where every run's row lies, bit 0 = a cache row), the
+// index brought up to date in the same launch.
+int runs_expand_maintain(const hb_runs_t* runs, const unsigned long long* run_src, const int64_t* run_slots,
+                         const void* cache_rows, const void* table, int64_t row_bytes, void* out_rows, int64_t* locs,
+                         uint8_t* found, const Maintain& duty, cudaStream_t st);
+
 #ifdef __CUDACC__
 __device__ __forceinline__ int64_t runs_valid_entries(const hb_runs_t& r) {
   if (!r.n_dev) return r.n;

@@ -19,6 +19,7 @@
 #pragma once
 
 #include "launch.cuh"
+#include "maintain.cuh"
 #include "optim.cuh"
 #include "runs.cuh"
 
@@ -58,6 +59,7 @@ int segsum_runs(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in
 // The sums and counts as they are, or the buffers of the id's class.
 struct StoreRows {
   static constexpr bool kWeights = true;
+  static constexpr bool kStep = false;
   float* sums;                // [U][dim] (null when the rows go to class buffers)
   const int8_t* dclass;       // [U], null = no split
   const int32_t* dpos;        // [U]
@@ -71,6 +73,7 @@ struct StoreRows {
 // 2^30 rows and slots.
 template <bool ADAM, bool STEP>
 struct UpdateRows {
+  static constexpr bool kStep = STEP;
   static constexpr bool kWeights = !STEP;  // rows with weights come from several senders
   const int64_t* uniq;        // [U] ids
   RowMap map;
@@ -84,6 +87,11 @@ struct UpdateRows {
   const int8_t* dclass;       // [U]
   float* staged;              // [slots][dim]
   const int64_t* slots;       // [U] staging slot of a cold run, -1 = none
+  // the first blocks of the launch age the LRU counters by the lookup that found the slots
+  int touch_blocks;
+  RunsView touched;
+  TouchMarks marks;
+  int32_t* lru;
 };
 
 template <bool ADAM, bool STEP>
@@ -101,6 +109,7 @@ UpdateRows<ADAM, STEP> update_rows(const hb_runs_t* runs, const hb_optim_t* opt)
   epi.dclass = nullptr;
   epi.staged = nullptr;
   epi.slots = nullptr;
+  epi.touch_blocks = 0;
   return epi;
 }
 
@@ -356,7 +365,15 @@ __global__ void __launch_bounds__(kSegBlock, EpiOps<Epi, VEC, G, VPL>::kMinBlock
   }
   const int R = a.piece;
   const int span = NG * R;
-  const int64_t b0 = (int64_t)blockIdx.x * span;
+  int block = blockIdx.x;
+  if constexpr (Epi::kStep) {
+    if (block < epi.touch_blocks) {
+      touch_runs(epi.touched, epi.marks, epi.lru, block, epi.touch_blocks);
+      return;
+    }
+    block -= epi.touch_blocks;
+  }
+  const int64_t b0 = (int64_t)block * span;
   if (b0 >= n_eff) return;
   if (threadIdx.x == 0) s_nfin = 0;
   const int64_t at = b0 + (int64_t)grp * R;
@@ -525,8 +542,8 @@ __global__ void __launch_bounds__(kSegBlock, EpiOps<Epi, VEC, G, VPL>::kMinBlock
       if (HAS_CNT) w += s_cnt[g];
       if (!(s_flag[g] & kSegWhole)) break;
     }
-    put(a.head_part + (int64_t)blockIdx.x * a.cols, row);
-    if (HAS_CNT && sub == 0) a.head_cnt[blockIdx.x] = w;
+    put(a.head_part + (int64_t)block * a.cols, row);
+    if (HAS_CNT && sub == 0) a.head_cnt[block] = w;
     arrive(u_first);
   }
   if (flag & kSegTail) {
@@ -540,8 +557,8 @@ __global__ void __launch_bounds__(kSegBlock, EpiOps<Epi, VEC, G, VPL>::kMinBlock
       typename Ops::Row with = Ops::fetch_alone(epi, a, u, sub, vpr);
       complete(u, acc, with, HAS_CNT ? cacc : (unsigned long long)(__ldg(a.run_start + u + 1) - __ldg(a.run_start + u)));
     } else {
-      put(a.tail_part + (int64_t)blockIdx.x * a.cols, acc);
-      if (HAS_CNT && sub == 0) a.tail_cnt[blockIdx.x] = cacc;
+      put(a.tail_part + (int64_t)block * a.cols, acc);
+      if (HAS_CNT && sub == 0) a.tail_cnt[block] = cacc;
       arrive(u);
     }
   }
@@ -629,7 +646,8 @@ template <int VEC, int G, int VPL, class Epi>
 int seg_launch(SegArgs a, const Epi& epi, cudaStream_t st) {
   a.piece = seg_piece(a.n, G);  // the same for every epilogue: the sums have the same bits
   const int ng = kSegBlock / G;
-  const int grid = (int)ceil_div(a.n, (int64_t)ng * a.piece);
+  int grid = (int)ceil_div(a.n, (int64_t)ng * a.piece);
+  if constexpr (Epi::kStep) grid += epi.touch_blocks;
   const size_t smem = (size_t)ng * a.cols * sizeof(float);
   if constexpr (Epi::kWeights) {
     if (a.cnt_in) {

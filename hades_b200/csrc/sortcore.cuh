@@ -105,6 +105,17 @@ __device__ __forceinline__ SortDigits sort_digits(unsigned lo, unsigned hi, bool
   return d;
 }
 
+// Digits from what the caller says of its keys (valid ones below 2^bits - 1), where that is as good as
+// looking: not when one bit less would save a pass.  Spares an exchange between all CTAs.
+__device__ __forceinline__ bool sort_known_digits(int bits, int max_width, SortDigits& d) {
+  if (bits <= 1 || bits > 30 || (bits + max_width - 1) / max_width != (bits - 1 + max_width - 1) / max_width) return false;
+  d.wide = false;
+  d.bits = bits;
+  d.passes = (bits + max_width - 1) / max_width;
+  d.width = (bits + d.passes - 1) / d.passes;
+  return true;
+}
+
 // exclusive scan over the first `bins` threads of the CTA (bins <= 1024, a multiple of 32 or below
 // 32); s_warp: [32].  All threads call it.
 __device__ __forceinline__ uint32_t sort_block_exscan(uint32_t v, int bins, uint32_t* s_warp) {
@@ -392,35 +403,40 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
         }
       }
     }
-    lo = __reduce_or_sync(0xffffffffu, lo);
-    hi = __reduce_or_sync(0xffffffffu, hi);
-    none = __reduce_or_sync(0xffffffffu, none);
-    uint4* per_warp = reinterpret_cast<uint4*>(s.sums);
-    if (lane == 0) per_warp[warp] = make_uint4(lo, hi, none, 0u);
-    __syncthreads();
-    if (warp == 0) {
-      const uint4 x = lane < W ? per_warp[lane] : make_uint4(0u, 0u, 0u, 0u);
-      lo = __reduce_or_sync(0xffffffffu, x.x);
-      hi = __reduce_or_sync(0xffffffffu, x.y);
-      none = __reduce_or_sync(0xffffffffu, x.z);
-      if (lane == 0) s.seen[0] = make_uint4(lo, hi, none, 0u);
-    }
-    ctx.sync();
-    if (ctx.ctas > 1) {
+    const bool known = sort_known_digits(src.known_bits(), kClusterDigit, dig);
+    ctx.wide = false;
+    ctx.none = true;
+    if (!known) {
+      lo = __reduce_or_sync(0xffffffffu, lo);
+      hi = __reduce_or_sync(0xffffffffu, hi);
+      none = __reduce_or_sync(0xffffffffu, none);
+      uint4* per_warp = reinterpret_cast<uint4*>(s.sums);
+      if (lane == 0) per_warp[warp] = make_uint4(lo, hi, none, 0u);
+      __syncthreads();
       if (warp == 0) {
-        uint4 x = make_uint4(0u, 0u, 0u, 0u);
-        if (lane < ctx.ctas) x = *cluster.map_shared_rank(s.seen, lane);
+        const uint4 x = lane < W ? per_warp[lane] : make_uint4(0u, 0u, 0u, 0u);
         lo = __reduce_or_sync(0xffffffffu, x.x);
         hi = __reduce_or_sync(0xffffffffu, x.y);
         none = __reduce_or_sync(0xffffffffu, x.z);
-        if (lane == 0) s.seen[1] = make_uint4(lo, hi, none, 0u);
+        if (lane == 0) s.seen[0] = make_uint4(lo, hi, none, 0u);
       }
-      __syncthreads();
+      ctx.sync();
+      if (ctx.ctas > 1) {
+        if (warp == 0) {
+          uint4 x = make_uint4(0u, 0u, 0u, 0u);
+          if (lane < ctx.ctas) x = *cluster.map_shared_rank(s.seen, lane);
+          lo = __reduce_or_sync(0xffffffffu, x.x);
+          hi = __reduce_or_sync(0xffffffffu, x.y);
+          none = __reduce_or_sync(0xffffffffu, x.z);
+          if (lane == 0) s.seen[1] = make_uint4(lo, hi, none, 0u);
+        }
+        __syncthreads();
+      }
+      const uint4 x = s.seen[ctx.ctas > 1 ? 1 : 0];
+      dig = sort_digits(x.x, x.y, x.z != 0u, kClusterDigit);
+      ctx.wide = dig.wide;
+      ctx.none = x.z != 0u;
     }
-    const uint4 x = s.seen[ctx.ctas > 1 ? 1 : 0];
-    dig = sort_digits(x.x, x.y, x.z != 0u, kClusterDigit);
-    ctx.wide = dig.wide;
-    ctx.none = x.z != 0u;
   }
   for (int pass = 0; pass < dig.passes; ++pass) {
     const int bit = pass * dig.width;
@@ -630,7 +646,12 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
   {
     unsigned lo = 0, hi = 0;
     bool none = false;
+    const bool known = sort_known_digits(src.known_bits(), max_digit, dig);
+    ctx.wide = false;
+    ctx.none = true;
+    // (a chunk of several tiles is read again by the first pass: needed here only to find the width)
     for (int t = 0; t < nt; ++t) {
+      if (nt > 1 && known) break;
       const int first = ctx.first(t);
 #pragma unroll
       for (int i = 0; i < I; ++i) {
@@ -648,31 +669,33 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
         }
       }
     }
-    lo = __reduce_or_sync(0xffffffffu, lo);
-    hi = __reduce_or_sync(0xffffffffu, hi);
-    none = __any_sync(0xffffffffu, none);
-    if (threadIdx.x < 4) s_seen[threadIdx.x] = 0u;
-    __syncthreads();
-    if (lane == 0) {
-      if (lo) atomicOr(s_seen, lo);
-      if (hi) atomicOr(s_seen + 1, hi);
-      if (none) atomicOr(s_seen + 2, 1u);
+    if (!known) {
+      lo = __reduce_or_sync(0xffffffffu, lo);
+      hi = __reduce_or_sync(0xffffffffu, hi);
+      none = __any_sync(0xffffffffu, none);
+      if (threadIdx.x < 4) s_seen[threadIdx.x] = 0u;
+      __syncthreads();
+      if (lane == 0) {
+        if (lo) atomicOr(s_seen, lo);
+        if (hi) atomicOr(s_seen + 1, hi);
+        if (none) atomicOr(s_seen + 2, 1u);
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) __stcg(reinterpret_cast<uint4*>(b.partial) + ctx.rank, make_uint4(s_seen[0], s_seen[1], s_seen[2], 0u));
+      if (!ctx.barrier()) return;
+      lo = hi = 0;
+      unsigned nn = 0;
+      for (int c = lane; c < ctx.ctas; c += 32) {
+        const uint4 p = __ldcg(reinterpret_cast<const uint4*>(b.partial) + c);
+        lo |= p.x; hi |= p.y; nn |= p.z;
+      }
+      lo = __reduce_or_sync(0xffffffffu, lo);
+      hi = __reduce_or_sync(0xffffffffu, hi);
+      nn = __reduce_or_sync(0xffffffffu, nn);
+      dig = sort_digits(lo, hi, nn != 0, max_digit);
+      ctx.wide = dig.wide;
+      ctx.none = nn != 0;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) __stcg(reinterpret_cast<uint4*>(b.partial) + ctx.rank, make_uint4(s_seen[0], s_seen[1], s_seen[2], 0u));
-    if (!ctx.barrier()) return;
-    lo = hi = 0;
-    unsigned nn = 0;
-    for (int c = lane; c < ctx.ctas; c += 32) {
-      const uint4 p = __ldcg(reinterpret_cast<const uint4*>(b.partial) + c);
-      lo |= p.x; hi |= p.y; nn |= p.z;
-    }
-    lo = __reduce_or_sync(0xffffffffu, lo);
-    hi = __reduce_or_sync(0xffffffffu, hi);
-    nn = __reduce_or_sync(0xffffffffu, nn);
-    dig = sort_digits(lo, hi, nn != 0, max_digit);
-    ctx.wide = dig.wide;
-    ctx.none = nn != 0;
   }
   const uint2* in = nullptr;
   uint2* out = b.kv0;

@@ -1,16 +1,16 @@
 // One trainer's step on one GPU in two calls (hb_step_forward / hb_step_backward).
 //
 //   forward   sort | per distinct id: probe, place its row is read from, mark of a hit for the ageing,
-//             a missed cold id onto the list of its set | rows to the batch positions
-//             beside them: LRU ageing | the listed ids into the index
-//             then: rows of the inserted ids into the cache
+//             a missed cold id onto the list of its set | rows to the batch positions, meanwhile LRU
+//             ageing and the listed ids into the index | rows of the inserted ids into the cache
 //   backward  per distinct cold id: probe, staging entry, mark | gradients summed, hot rows updated,
-//             cold rows staged | LRU ageing
+//             cold rows staged, meanwhile LRU ageing
 //
 // What bounds it: at 2,000 ids nothing but launches (composed from separate calls the same work took
 // 33 launches and 450 us of host time for 160 us of kernels); at 2,000,000 ids HBM.
 #include "index.cuh"
 #include "launch.cuh"
+#include "maintain.cuh"
 #include "runs.cuh"
 #include "segsum.cuh"
 #include "staging.cuh"
@@ -18,8 +18,8 @@
 struct hb_step {
   int device;
   cudaStream_t side;
-  cudaEvent_t forked, expanded, maintained;
-  bool side_busy;    // `maintained` has to be waited for
+  cudaEvent_t forked, fetched;
+  bool side_busy;    // `fetched` has to be waited for
   hb_runs_t runs;    // of the last batch
   int64_t runs_n;    // 0: none
 };
@@ -31,10 +31,6 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr int kCold = 2;
-// Batches below this run everything on the caller's stream: their kernels last a few microseconds each,
-// less than the events that order a second stream.
-constexpr int64_t kSideMin = 32768;
-
 // Small batches update rows as their sums become complete (one launch); large ones write the sums and
 // update in a second pass over the distinct ids: the sums then run at the speed of the copy, and the
 // update has many rows in flight whatever the lengths of the runs.
@@ -151,7 +147,7 @@ bool captured(cudaStream_t st) {
 
 int join_side(hb_step* s, cudaStream_t st) {
   if (s->side_busy) {
-    HB_CUDA(cudaStreamWaitEvent(st, s->maintained, 0));
+    HB_CUDA(cudaStreamWaitEvent(st, s->fetched, 0));
     s->side_busy = false;
   }
   return HB_OK;
@@ -291,6 +287,8 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
   epi.dclass = r.dclass;
   epi.staged = d->staging.grad;
   epi.slots = c.slots;
+  // the lookup of the accumulate: every distinct cold id once, in ascending order
+  const RunsView touched{c.slots, nullptr, nullptr, r.num_runs, r.num_runs, r.n, r.n, 2};
   const IndexView& v = d->index->view;
   const bool sorted = d->lookup_mode == HB_LOOKUP_SORTED;
   if (fused) {
@@ -300,6 +298,12 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
       HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SORTED>, (int)blocks, kBlock, 0, st, v, r, c, seg.done, seg.max_ctas);
     else
       HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SETASSOC>, (int)blocks, kBlock, 0, st, v, r, c, seg.done, seg.max_ctas);
+    if (d->touch_lru) {
+      epi.touch_blocks = (int)blocks;
+      epi.touched = touched;
+      epi.marks = c.marks;
+      epi.lru = d->index->lru;
+    }
     return seg_dispatch(a, epi, vec4, st);
   }
   HB_CUDA(cudaMemsetAsync(seg.done, 0, (size_t)seg.max_ctas * sizeof(unsigned), st));
@@ -312,10 +316,13 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
   rc = join_side(s, st);
   if (rc != HB_OK) return rc;
   if (sorted)
-    return vec4 ? launch_apply<HB_LOOKUP_SORTED, ADAM, 4>(v, r, c, a, epi, sums, st)
-                : launch_apply<HB_LOOKUP_SORTED, ADAM, 1>(v, r, c, a, epi, sums, st);
-  return vec4 ? launch_apply<HB_LOOKUP_SETASSOC, ADAM, 4>(v, r, c, a, epi, sums, st)
+    rc = vec4 ? launch_apply<HB_LOOKUP_SORTED, ADAM, 4>(v, r, c, a, epi, sums, st)
+              : launch_apply<HB_LOOKUP_SORTED, ADAM, 1>(v, r, c, a, epi, sums, st);
+  else
+    rc = vec4 ? launch_apply<HB_LOOKUP_SETASSOC, ADAM, 4>(v, r, c, a, epi, sums, st)
               : launch_apply<HB_LOOKUP_SETASSOC, ADAM, 1>(v, r, c, a, epi, sums, st);
+  if (rc != HB_OK || !d->touch_lru) return rc;
+  return index_touch_apply(d->index, touched, st);
 }
 
 int grid_for_runs(int64_t n) {
@@ -368,8 +375,7 @@ int hb_step_create(hb_step_t** out) {
   HB_CUDA(cudaGetDevice(&s->device));
   HB_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
   HB_CUDA(cudaEventCreateWithFlags(&s->forked, cudaEventDisableTiming));
-  HB_CUDA(cudaEventCreateWithFlags(&s->expanded, cudaEventDisableTiming));
-  HB_CUDA(cudaEventCreateWithFlags(&s->maintained, cudaEventDisableTiming));
+  HB_CUDA(cudaEventCreateWithFlags(&s->fetched, cudaEventDisableTiming));
   *out = s;
   return HB_OK;
 }
@@ -378,8 +384,7 @@ int hb_step_destroy(hb_step_t* s) {
   if (!s) return HB_OK;
   cudaStreamDestroy(s->side);
   cudaEventDestroy(s->forked);
-  cudaEventDestroy(s->expanded);
-  cudaEventDestroy(s->maintained);
+  cudaEventDestroy(s->fetched);
   delete s;
   return HB_OK;
 }
@@ -399,7 +404,7 @@ int hb_step_join(hb_step_t* s, hb_stream_t stream) {
 }
 
 int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, int64_t n, void* out_rows,
-                    int64_t* locs, uint8_t* found, int64_t* counters, int join, void* workspace,
+                    int64_t* locs, uint8_t* found, int64_t* counters, int aside_allowed, void* workspace,
                     size_t workspace_bytes, hb_stream_t stream) {
   HB_CHECK_ARG(s, "hb_step_forward: null handle");
   int rc = check_desc(d, "hb_step_forward");
@@ -427,10 +432,9 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
   if (rc != HB_OK) return rc;
   rc = build_runs(s, d, p, ids, n, counters, st);
   if (rc != HB_OK) return rc;
-  // HB_STEP_ASIDE: all of the fetch leaves the caller's stream, which goes on to the aggregation of the
+  // aside: all of the fetch leaves the caller's stream, which goes on to the aggregation of the
   // same batch (it needs the sort only); both are bound by HBM, but not all the time
-  const bool in_graph = captured(st);
-  const bool aside = join == HB_STEP_ASIDE && (in_graph || !fuses_update(n));
+  const bool aside = aside_allowed && (captured(st) || !fuses_update(n));
   if (aside) {
     HB_CUDA(cudaEventRecord(s->forked, st));
     HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
@@ -446,38 +450,35 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
   else
     HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a, marks,
               lists, device_error_word());
-  const bool maintain = d->touch_lru || d->insert_misses;
-  const bool beside = !aside && maintain && (in_graph || n >= kSideMin);
-  cudaStream_t side = beside ? s->side : st;
-  if (beside) {
-    HB_CUDA(cudaEventRecord(s->forked, st));
-    HB_CUDA(cudaStreamWaitEvent(side, s->forked, 0));
+  Maintain m;
+  memset(&m, 0, sizeof(m));
+  const bool lists_used = d->insert_misses && index_add_runs_lists(h, n);
+  if (d->touch_lru || lists_used) {
+    m.v = RunsView{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
+    m.marks = marks;
+    m.e = AddEntries{s->runs.uniq_ids, n, s->runs.num_runs, p.on_list, p.chunk_listed, p.listed, d->miss_cap};
+    rc = index_add_state(h, static_cast<uint32_t*>(p.add_ws), p.new_slots, p.last_writer, &m.add);
+    if (rc != HB_OK) return rc;
+    m.touch = d->touch_lru;
+    m.insert = lists_used;
+    m.blocks = grid_for_runs(n);
   }
-  rc = hb_runs_expand(&s->runs, d->cache_rows, d->table, d->row_bytes, 0, out_rows, locs, found, p.run_slots,
-                      p.fetch_ws, p.fetch_bytes, (hb_stream_t)st);
+  rc = runs_expand_maintain(&s->runs, a.run_src, p.run_slots, d->cache_rows, d->table, d->row_bytes, out_rows, locs,
+                            found, m, st);
   if (rc != HB_OK) return rc;
-  if (d->touch_lru) {
-    const RunsView v{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
-    rc = index_touch_apply(h, v, side);
-    if (rc != HB_OK) return rc;
-  }
   if (d->insert_misses) {
-    const AddEntries e{s->runs.uniq_ids, n, s->runs.num_runs, p.on_list, p.chunk_listed, p.listed, d->miss_cap};
-    rc = index_add_runs(h, e, p.add_ws, p.new_slots, p.last_writer, side);
-    if (rc != HB_OK) return rc;
-    if (beside) {
-      // a slot that the insertion takes over may hold a row this batch still reads
-      HB_CUDA(cudaEventRecord(s->expanded, st));
-      HB_CUDA(cudaStreamWaitEvent(side, s->expanded, 0));
+    if (!lists_used) {
+      const AddEntries e{s->runs.uniq_ids, n, s->runs.num_runs, p.on_list, p.chunk_listed, p.listed, d->miss_cap};
+      rc = index_add_runs_sorted(h, e, p.add_ws, p.new_slots, p.last_writer, st);
+      if (rc != HB_OK) return rc;
     }
     rc = staging_insert_rows(&d->staging, d->table, s->runs.uniq_ids, n, s->runs.num_runs, d->cache_rows,
-                             d->row_bytes, p.new_slots, p.last_writer, side);
+                             d->row_bytes, p.new_slots, p.last_writer, st);
     if (rc != HB_OK) return rc;
   }
-  if (beside || aside) {
-    HB_CUDA(cudaEventRecord(s->maintained, side));
+  if (aside) {
+    HB_CUDA(cudaEventRecord(s->fetched, st));
     s->side_busy = true;
-    if (join == HB_STEP_JOIN) return join_side(s, st);
   }
   return HB_OK;
 }
@@ -525,13 +526,8 @@ int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, 
                    p.cold_slots, marks, d->touch_lru};
   SegArgs a = seg_args(&s->runs, grads, nullptr, d->dim, 0, seg);
   a.cols = (int)d->dim;
-  rc = d->opt.kind == HB_OPT_ADAM ? update_step<true>(s, d, c, a, vec4, p.sums, seg, fused, st)
-                                  : update_step<false>(s, d, c, a, vec4, p.sums, seg, fused, st);
-  if (rc != HB_OK) return rc;
-  if (!d->touch_lru) return HB_OK;
-  // the lookup of the accumulate: every distinct cold id once, in ascending order
-  const RunsView v{p.cold_slots, nullptr, nullptr, s->runs.num_runs, s->runs.num_runs, n, n, 2};
-  return index_touch_apply(h, v, st);
+  return d->opt.kind == HB_OPT_ADAM ? update_step<true>(s, d, c, a, vec4, p.sums, seg, fused, st)
+                                    : update_step<false>(s, d, c, a, vec4, p.sums, seg, fused, st);
 }
 
 }  // extern "C"

@@ -120,12 +120,11 @@ class _OneGpuStep:
                 self.kept.append(self.ws)
             self.ws = ws
 
-    def forward(self, p: "EmbeddingPath", ids: torch.Tensor, out_rows, join: int):
-        """join: HB_STEP_BESIDE / HB_STEP_JOIN / HB_STEP_ASIDE."""
+    def forward(self, p: "EmbeddingPath", ids: torch.Tensor, out_rows, aside: bool):
         ids = ids.contiguous()
         self.refresh(p)
         rows, locs, found, counters, ws = self.native.step_forward(
-            self._h.value, self.addr, ids, p.dim, p.cold.emb, out_rows, p.want_locs, join, self.ws)
+            self._h.value, self.addr, ids, p.dim, p.cold.emb, out_rows, p.want_locs, aside, self.ws)
         self.keep(p, ws)
         self.batch = (ids, ids._version, counters)
         return rows, locs, found
@@ -262,7 +261,7 @@ class EmbeddingPath:
         n = ids.numel()
         if self._one is not None and n > 0:
             self._last = None
-            return self._one.forward(self, ids, out_rows, 2 if on_side else int(join))
+            return self._one.forward(self, ids, out_rows, on_side)
         lib = E._lib.load()
         runs = E.cudaRunsBuild(ids, self.id_bits, self.class_table, keep=(False, True, True),
                                caps=(None, self.num_hot_ids, None),

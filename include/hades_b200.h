@@ -756,14 +756,11 @@ int hb_step_destroy(hb_step_t* s);
 int hb_step_supported(const hb_step_desc_t* d);
 size_t hb_step_workspace_bytes(int64_t n, int64_t dim);
 /* counters: device int64[4] = distinct ids, distinct ids of class 0, 1, 2.  locs nullable.
- * join: HB_STEP_JOIN; HB_STEP_BESIDE: the maintenance of the cache may still run on the side stream;
- * HB_STEP_ASIDE: all of the fetch may (out_rows, locs and found too), beside the aggregation of the
- * hb_step_backward that follows.  The next call of this handle, or hb_step_join, orders it. */
-#define HB_STEP_BESIDE 0
-#define HB_STEP_JOIN 1
-#define HB_STEP_ASIDE 2
+ * aside: the fetch (out_rows, locs and found too) may still run on the side stream, beside the
+ * aggregation of the hb_step_backward that follows; that call, the next one of this handle, or
+ * hb_step_join, orders it. */
 int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, int64_t n, void* out_rows,
-                    int64_t* locs, uint8_t* found, int64_t* counters, int join, void* workspace,
+                    int64_t* locs, uint8_t* found, int64_t* counters, int aside, void* workspace,
                     size_t workspace_bytes, hb_stream_t stream);
 int hb_step_join(hb_step_t* s, hb_stream_t stream);
 /* ids NULL: the gradients belong to the batch of the last forward call (same n and workspace). */
