@@ -48,6 +48,8 @@ PROTOTYPES: dict[str, tuple] = {
     "hb_index_touch_lru_workspace_bytes": (_sz, [_i64]),
     "hb_index_touch_lru": (_int, [_p, _p, _i64, _p, _sz, _p]),
     "hb_index_lookup_touch": (_int, [_p, _p, _i64, _p, _int, _p]),
+    "hb_index_lookup_touch_part": (_int, [_p, _p, _i64, _p, _i64, _p, _p, _int, _p]),
+    "hb_index_lookup_touch_end": (_int, [_p, _p, _i64, _p]),
     "hb_index_touch_lru_runs": (_int, [_p, _p, _p, _p, _i64, _p, _i64, _p, _int, _p]),
     "hb_index_reset": (_int, [_p, _p, _i64, _p]),
     "hb_index_getall": (_int, [_p, _p, _p, _i64, _p, _p]),

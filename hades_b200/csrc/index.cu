@@ -188,10 +188,19 @@ __global__ void __launch_bounds__(kBlock) lookup_kernel(IndexView v, const int64
 // Three passes over the batch positions, no sort: the last hit of every slot and the hits of every
 // line; the hits after each slot's last; the counters.  (65,536 positions: sorted 40 us, this 9.)  Lanes
 // with the same slot speak as one, so that the copies of a popular id do not queue at one address.
+// A caller that works on ids in host memory has them and wants the slots in pinned buffers, a part of the
+// batch at a time: positions first .. first + n of it, slots to host_locs too, and then a word that says
+// that they have arrived.
+struct HostPart {
+  int64_t first;
+  int64_t* locs;    // nullable
+  int64_t* arrived; // nullable
+};
+
 template <int MODE, bool LOOKUP>
 __global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const int64_t* __restrict__ ids,
                                                             int64_t* __restrict__ locs, int64_t n, TouchMarks t,
-                                                            int32_t* __restrict__ line_hits) {
+                                                            int32_t* __restrict__ line_hits, HostPart part) {
   __shared__ int64_t s_top[LOOKUP && MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (LOOKUP && MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -206,15 +215,30 @@ __global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const i
     int64_t slot = -1;
     if (LOOKUP) {
       slot = warp_lookup<MODE>(v, s_top, i < n ? __ldg(ids + i) : -1);
-      if (i < n) locs[i] = slot;
+      if (i < n) {
+        locs[i] = slot;
+        if (part.locs) part.locs[i] = slot;
+      }
     } else if (i < n) {
       slot = locs[i];
       if (slot >= t.capacity) slot = -1;
     }
     const unsigned same = __match_any_sync(0xffffffffu, slot);
     if (slot >= 0 && (same >> lane) == 1u) {  // the last of them
-      atomicMax(t.marks + slot, number | (unsigned long long)(i + 1));
+      atomicMax(t.marks + slot, number | (unsigned long long)(part.first + i + 1));
       atomicAdd(line_hits + (slot >> 3), __popc(same));
+    }
+  }
+  if (part.arrived) {
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned* done = reinterpret_cast<unsigned*>(t.batch + 6);
+      if (atomicAdd(done, 1u) == gridDim.x - 1u) {
+        *done = 0u;
+        __threadfence_system();
+        *reinterpret_cast<volatile int64_t*>(part.arrived) = 1;
+      }
     }
   }
 }
@@ -621,10 +645,8 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   return HB_OK;
 }
 
-// lookup of `ids` into locs first (LOOKUP), or the slots given
-static int touch_positions(hb_index* h, const int64_t* ids, int64_t* locs, int64_t n, int mode, cudaStream_t st) {
-  TouchMarks t;
-  int rc = index_touch_marks(h, &t, st);
+static int touch_buffers(hb_index* h, TouchMarks* t, cudaStream_t st) {
+  const int rc = index_touch_marks(h, t, st);
   if (rc != HB_OK) return rc;
   if (!h->after) {
     HB_CUDA(cudaMalloc(&h->line_hits, h->lines * sizeof(int32_t)));
@@ -632,13 +654,27 @@ static int touch_positions(hb_index* h, const int64_t* ids, int64_t* locs, int64
     HB_CUDA(cudaMalloc(&h->after, h->cache_size * sizeof(int32_t)));
     HB_CUDA(cudaMemsetAsync(h->after, 0, h->cache_size * sizeof(int32_t), st));
   }
+  return HB_OK;
+}
+
+// lookup of `ids` into locs (or the slots there, ids null), first pass of the ageing
+static int touch_mark(hb_index* h, const TouchMarks& t, const int64_t* ids, int64_t* locs, int64_t n, int mode,
+                      const HostPart& part, cudaStream_t st) {
   const int grid = grid_capped(n);
   if (!ids)
-    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits);
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
+              part);
   else if (mode == HB_LOOKUP_SORTED)
-    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SORTED, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits);
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SORTED, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
+              part);
   else
-    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits);
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
+              part);
+  return HB_OK;
+}
+
+static int touch_finish(hb_index* h, const TouchMarks& t, const int64_t* locs, int64_t n, cudaStream_t st) {
+  const int grid = grid_capped(n);
   HB_LAUNCH(touch_after_kernel, grid, kBlock, 0, st, locs, n, t, h->after);
   HB_LAUNCH(touch_apply_kernel, grid, kBlock, 0, st, locs, n, t, h->after, h->line_hits, h->lru);
   return HB_OK;
@@ -648,20 +684,41 @@ int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n, void*, siz
   HB_CHECK_ARG(h && (n == 0 || locs), "hb_index_touch_lru: null argument");
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_index_touch_lru: n out of range");
   if (n == 0) return HB_OK;
-  return touch_positions(h, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  TouchMarks t;
+  int rc = touch_buffers(h, &t, st);
+  if (rc != HB_OK) return rc;
+  rc = touch_mark(h, t, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, HostPart{0, nullptr, nullptr}, st);
+  return rc != HB_OK ? rc : touch_finish(h, t, locs, n, st);
 }
 
 int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int mode,
                           hb_stream_t stream) {
-  HB_CHECK_ARG(h && (n == 0 || (ids && locs)), "hb_index_lookup_touch: null argument");
+  int rc = hb_index_lookup_touch_part(h, ids, n, locs, 0, nullptr, nullptr, mode, stream);
+  return rc != HB_OK || n == 0 ? rc : hb_index_lookup_touch_end(h, locs, n, stream);
+}
+
+int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
+                               int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream) {
+  HB_CHECK_ARG(h && first >= 0 && (n == 0 || (ids && locs)), "hb_index_lookup_touch: null argument");
   HB_CHECK_ARG(mode == HB_LOOKUP_SETASSOC || mode == HB_LOOKUP_SORTED, "hb_index_lookup_touch: unknown mode %d", mode);
-  HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_index_lookup_touch: n out of range");
+  HB_CHECK_ARG(n >= 0 && first + n < ((int64_t)1 << 31), "hb_index_lookup_touch: n out of range");
   if (n == 0) return HB_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  int rc;
   if (mode == HB_LOOKUP_SORTED && h->sorted_stale) {
-    const int rc = hb_index_build_sorted(h, stream);
+    rc = hb_index_build_sorted(h, stream);
     if (rc != HB_OK) return rc;
   }
-  return touch_positions(h, ids, locs, n, mode, (cudaStream_t)stream);
+  TouchMarks t;
+  rc = touch_buffers(h, &t, st);
+  if (rc != HB_OK) return rc;
+  return touch_mark(h, t, ids, locs + first, n, mode, HostPart{first, host_locs, arrived}, st);
+}
+
+int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream) {
+  HB_CHECK_ARG(h && h->after && locs && n > 0, "hb_index_lookup_touch: no part of the batch was looked up");
+  return touch_finish(h, TouchMarks{h->marks, h->batch, h->cache_size}, locs, n, (cudaStream_t)stream);
 }
 
 int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* perm,

@@ -118,6 +118,14 @@ int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n,
  * index on first use; the workspace of the latter is not used any more.) */
 int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int mode,
                           hb_stream_t stream);
+/* The same in parts, so that a caller with ids in host memory can copy one part while another is looked
+ * up: positions first .. first + n of the batch (ids of the part: device or pinned; locs of the whole
+ * batch: device), slots also to host_locs (nullable, pinned, of the part), then *arrived (nullable,
+ * pinned) = 1.  After the last part hb_index_lookup_touch_end ages the counters by the whole batch; no
+ * other call on the index may come between. */
+int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
+                               int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream);
+int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream);
 
 /* The same LRU effect for a batch that is already grouped: run u holds the batch
  * positions perm[run_start[u] .. run_start[u+1]) (ascending) of ONE id, so all of

@@ -196,3 +196,25 @@ def test_add_and_lookup_of_large_batches(cuda_lib, oracle_mod, n, cache_size, ki
         want_ids, want_lru = ora.export()
         _eq(got_ids.cpu().numpy(), want_ids, (step, "ids"))
         _eq(got_lru.cpu().numpy(), want_lru, (step, "lru"))
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [1, 16_383, 16_384, 16_385, 32_769, 70_001])
+def test_host_lookups_in_parts(cuda_lib, oracle_mod, n, mode):
+    """Host ids are looked up in parts of 16,384: slots, line ids and LRU counters at the edges of the
+    parts, with a hot id that ages in every part, ids that are strided in memory, and adds between."""
+    from hades_b200 import EmbCacheLib as E
+
+    rng = np.random.default_rng(n)
+    ix = E.IndexCache(6000, f"parts{n}_{mode}", True, False, lookup_mode=mode)
+    ora = oracle_mod.OracleIndex(6000)
+    for rnd in range(3):
+        new = rng.integers(0, 20_000, n, dtype=np.int64)
+        _eq(ix.add(torch.from_numpy(new)).numpy(), ora.add(new), ("add", rnd))
+        q = rng.integers(0, 20_000, 2 * n, dtype=np.int64)[::2]
+        q[:: 5] = new[-1]
+        _eq(ix.lookup(torch.from_numpy(q)).numpy(), ora.lookup(np.ascontiguousarray(q), touch=True), ("lookup", rnd))
+        ids, lru = ix.export_state()
+        oi, ol = ora.export()
+        _eq(ids.cpu().numpy(), oi, ("line ids", rnd))
+        _eq(lru.cpu().numpy(), ol, ("lru", rnd))
