@@ -91,6 +91,7 @@ PROTOTYPES: dict[str, tuple] = {
     "hb_staging_accumulate_cached": (_int, [_p, _p, _p, _p, _i64, _p, _p, C.c_int32, _int, _p, _p, _p]),
     "hb_staging_accumulate_direct": (_int, [_p, _p, _p, _i64, _p, _i64, _i64, _p]),
     "hb_staging_flush_workspace_bytes": (_sz, [_i64, _int]),
+    "hb_staging_flush_counted": (_int, [_p, _p, C.c_int32, _int, _i64, _p, _p, _p, _p, _p, _p, _sz, _p]),
     "hb_staging_flush": (_int, [_p, _p, C.c_int32, _int, _i64, _p, _p, _p, _p, _p, _sz, _p]),
     "hb_staging_insert_workspace_bytes": (_sz, [_i64]),
     "hb_staging_insert_rows": (_int, [_p, _p, _p, _i64, _p, _i64, _p, _p, _p]),

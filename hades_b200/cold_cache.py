@@ -52,9 +52,14 @@ class StagingTable:
         sync=False: no host read; the outputs hold out_cap entries (0: one per slot) of which
         the first min(counts.sum(), out_cap) are valid.  out_cap < slots needs num_clients == 1:
         stale rows beyond it stay staged until the next flush."""
-        lib = _lib.load()
         dev = self.grad.device
         cap = self.slots if out_cap <= 0 else min(int(out_cap), self.slots)
+        if sync and num_clients == 1 and dev.type == "cuda":
+            *out, stale = (_lib._NATIVE or _lib.native()).staging_flush(
+                None if index is None else index.handle.value, C.addressof(self.desc), int(cnt_threshold), cap, dev.index)
+            self.last_counts_host = [stale]
+            return tuple(out)
+        lib = _lib.load()
         out_ids = torch.empty(cap, dtype=torch.int64, device=dev)
         out_rows = torch.empty((cap, self.dim), dtype=torch.float32, device=dev)
         out_cnt = torch.empty(cap, dtype=torch.int64, device=dev)

@@ -288,6 +288,30 @@ PyObject* index_add(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   });
 }
 
+// staging_flush(index | None, address of the hb_staging_t, cnt_threshold, rows the output holds, device) for
+// one client -> (ids, rows, cnt, counts, number of stale rows); the number is read while the rows move
+PyObject* staging_flush(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  return guarded([&]() -> PyObject* {
+    arity(n_args, 5, "staging_flush");
+    hb_index_t* h = none(a[0]) ? nullptr : static_cast<hb_index_t*>(pointer(a[0]));
+    const hb_staging_t* s = static_cast<const hb_staging_t*>(pointer(a[1]));
+    const int64_t cap = integer(a[3]);
+    const at::Device dev(at::kCUDA, (c10::DeviceIndex)integer(a[4]));
+    c10::cuda::CUDAGuard guard(dev);
+    at::Tensor ids = cuda_empty({cap}, at::kLong, dev), rows = cuda_empty({cap, s->dim}, at::kFloat, dev);
+    at::Tensor cnt = cuda_empty({cap}, at::kLong, dev), counts = cuda_empty({1}, at::kLong, dev);
+    const size_t need = hb_staging_flush_workspace_bytes(s->slots, 1);
+    const at::Tensor ws = cuda_empty({(int64_t)need}, at::kByte, dev);
+    void* st = stream_of(dev);
+    int64_t* num = t_word.arm();
+    check(hb_staging_flush_counted(h, s, (int32_t)integer(a[2]), 1, cap, ids.data_ptr<int64_t>(), rows.data_ptr<float>(),
+                                   cnt.data_ptr<int64_t>(), counts.data_ptr<int64_t>(), num, ws.data_ptr(), need, st));
+    const int64_t stale = t_word.wait(static_cast<cudaStream_t>(st)), u = stale < cap ? stale : cap;
+    return pack({THPVariable_Wrap(ids.narrow(0, 0, u)), THPVariable_Wrap(rows.narrow(0, 0, u)),
+                 THPVariable_Wrap(cnt.narrow(0, 0, u)), THPVariable_Wrap(counts), PyLong_FromLongLong(stale)});
+  });
+}
+
 // step_forward(step, desc, ids, dim, row dtype tensor, out_rows | None, want_locs, aside, ws | None)
 // -> (rows, locs | None, found, counters, ws)
 PyObject* step_forward(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
@@ -347,6 +371,7 @@ PyMethodDef g_methods[] = {
     {"unique_update", HB_FAST(unique_update), nullptr},
     {"index_lookup", HB_FAST(index_lookup), nullptr},
     {"index_add", HB_FAST(index_add), nullptr},
+    {"staging_flush", HB_FAST(staging_flush), nullptr},
     {"step_forward", HB_FAST(step_forward), nullptr},
     {"step_backward", HB_FAST(step_backward), nullptr},
     {"set_error_class", set_error_class, METH_O, nullptr},

@@ -559,6 +559,11 @@ int hb_staging_flush(hb_index_t* h /* nullable */, const hb_staging_t* s, int32_
                      int num_clients, int64_t out_cap, int64_t* out_ids, float* out_rows,
                      int64_t* out_cnt, int64_t* counts, void* workspace, size_t workspace_bytes,
                      hb_stream_t stream);
+/* The same; host_count (nullable, pinned, num_clients == 1): counts[0], written before the rows move. */
+int hb_staging_flush_counted(hb_index_t* h /* nullable */, const hb_staging_t* s, int32_t cnt_threshold,
+                             int num_clients, int64_t out_cap, int64_t* out_ids, float* out_rows,
+                             int64_t* out_cnt, int64_t* counts, int64_t* host_count, void* workspace,
+                             size_t workspace_bytes, hb_stream_t stream);
 
 /* _update_cache, server.py:499-544: locs = add(ids); cache_rows[locs[i]] =
  * emb_rows[i] where locs[i] >= 0; the staging state of those slots is cleared

@@ -202,3 +202,47 @@ def test_sparse_adam_state_through_the_tiered_cache(cuda_lib, unique):
     idx_map = b.state_cache.idx_map.cpu()
     uncached = torch.nonzero(idx_map == -1).flatten()
     assert torch.equal(b.state_mem[uncached], a.state_mem.cpu()[uncached])
+
+
+@pytest.mark.parametrize("slots,dim,cap", [(1, 4, 0), (31, 3, 0), (1023, 128, 0), (1024, 128, 100), (1025, 1, 0),
+                                           (40_000, 130, 0), (40_000, 260, 7_000), (4_194_304 + 1_500, 2, 0)])
+@pytest.mark.parametrize("share", [0.0, 0.03, 1.0])
+@pytest.mark.parametrize("sync", [True, False])
+def test_flush_to_one_client(cuda_lib, slots, dim, cap, share, sync):
+    """The whole table after a flush and what left, bit for bit, at the edges of the 1,024 slots a block
+    takes at a time, with several rounds a block (over 4,194,304 slots), an output smaller than the
+    stale rows, none or all slots stale, and rows of vectors and of single floats."""
+    from hades_b200.cold_cache import StagingTable
+
+    rng = np.random.default_rng(slots + dim)
+    t = StagingTable(slots, dim, "cuda")
+    grad = rng.standard_normal((slots, dim)).astype(np.float32)
+    cnt = rng.integers(-1, 4, slots).astype(np.int32)
+    age = rng.integers(0, 5, slots).astype(np.int32)
+    stale = rng.random(slots) < share
+    cnt[stale] = np.maximum(cnt[stale], 1)
+    limit = np.where(stale, age, age + 1).astype(np.int32)
+    often = stale & (rng.random(slots) < 0.3)
+    limit[often] += 5
+    cnt[often] = 16
+    ids = rng.permutation(slots).astype(np.int64)
+    ids[rng.random(slots) < 0.01] = -1
+    for dst, src in ((t.grad, grad), (t.cnt, cnt), (t.idx, ids), (t.iter_count, age), (t.iter_threshold, limit)):
+        dst.copy_(_t(src))
+    found = np.nonzero(stale & (ids >= 0))[0]
+    left = found[:cap] if cap else found
+    got_ids, got_rows, got_cnt, counts = t.flush(None, 16, 1, sync, cap)
+    if sync:
+        assert t.last_counts_host == [found.size]
+    else:
+        got_ids, got_rows, got_cnt = got_ids[:left.size], got_rows[:left.size], got_cnt[:left.size]
+    assert counts.tolist() == [found.size]
+    assert np.array_equal(got_ids.cpu().numpy(), ids[left])
+    assert np.array_equal(got_cnt.cpu().numpy(), cnt[left])
+    assert np.array_equal(got_rows.cpu().numpy(), grad[left])
+    stays = cnt > 0
+    stays[left] = False
+    age[stays] += 1
+    age[left], cnt[left], grad[left] = 0, 0, 0
+    for dst, want in ((t.grad, grad), (t.cnt, cnt), (t.idx, ids), (t.iter_count, age), (t.iter_threshold, limit)):
+        assert np.array_equal(dst.cpu().numpy(), want)
