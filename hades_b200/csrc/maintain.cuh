@@ -195,13 +195,26 @@ __device__ __forceinline__ void walk_list(const AddEntries& e, const AddState& a
     st.store(a.line_ids, a.lru, line);
     return;
   }
+  // A step along the list is one trip to L2, with the id of the entry in its shadow; what the walk needs
+  // again stays in the thread (reading ids in order and slots back took two more trips per entry:
+  // 100,000 ids on 62,500 lists 22.9 -> 20.3 us).
   uint32_t order[kListShort];
-  int len = 0;
-  uint32_t at = (uint32_t)i + 1u;
-  for (; at && len < kListShort; at = a.next[at - 1]) {
+  int64_t held[kListShort];  // the id of an entry, later its way
+  order[0] = (uint32_t)i + 1u;
+  held[0] = id;
+  int len = 1;
+  uint32_t at = behind;
+  while (at && len < kListShort) {
+    const uint32_t after = a.next[at - 1];
+    const int64_t its = __ldg(e.ids + (int64_t)at - 1);
     int k = len++;
-    for (; k > 0 && order[k - 1] > at; --k) order[k] = order[k - 1];
+    for (; k > 0 && order[k - 1] > at; --k) {
+      order[k] = order[k - 1];
+      held[k] = held[k - 1];
+    }
     order[k] = at;
+    held[k] = its;
+    at = after;
   }
   if (at && DISTINCT) {
     // only ids in strides of the number of sets come here: no launch is kept ready for them
@@ -223,14 +236,12 @@ __device__ __forceinline__ void walk_list(const AddEntries& e, const AddState& a
   } else {
     for (int k = 0; k < len; ++k) {
       const int64_t x = (int64_t)order[k] - 1;
-      const int way = x < cut ? st.place(__ldg(e.ids + x), k) : -1;
+      const int way = x < cut ? st.place(held[k], k) : -1;
       a.locs[x] = way >= 0 ? line * kWays + way : -1;
+      held[k] = way;
     }
     if (a.last_writer)
-      for (int k = 0; k < len; ++k) {
-        const int64_t x = (int64_t)order[k] - 1;
-        a.last_writer[x] = st.is_last(a.locs[x], k);
-      }
+      for (int k = 0; k < len; ++k) a.last_writer[(int64_t)order[k] - 1] = st.is_last(held[k], k);
   }
   st.store(a.line_ids, a.lru, line);
 }
