@@ -80,7 +80,7 @@ PROTOTYPES: dict[str, tuple] = {
     "hb_runs_build": (_int, [_p, _i64, _p, _p, _i64, _int, _p, _i64, _p, _p, _p, _p, _p, _sz, _p, _p]),
     "hb_segsum_runs_workspace_bytes": (_sz, [_i64, _i64]),
     "hb_segsum_runs_f32": (_int, [_p, _p, _p, _i64, _int, _p, _p, _p, _p, _sz, _p]),
-    "hb_segsum_update_f32": (_int, [_p, _p, _p, _i64, _int, _p, _p, _sz, _p]),
+    "hb_unique_update_workspace_bytes": (_sz, [_i64, _i64, _p, _p]),
     "hb_unique_update_f32": (_int, [_p, _p, _p, _i64, _p, _p, _i64, _i64, _int, _int, _p, _p, _sz, _p]),
     "hb_lookup_fetch_runs_workspace_bytes": (_sz, [_i64, _i64, _int]),
     "hb_lookup_fetch_runs": (_int, [_p, _p, _p, _p, _i64, _p, _i64, _p, _p, _p, _p, _int, _p, _sz, _p]),

@@ -199,12 +199,13 @@ PyObject* unique_update(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const at::Device dev = ids.device();
     c10::cuda::CUDAGuard guard(dev);
     const int64_t n = ids.numel(), dim = grads.size(1);
+    const hb_optim_t* opt = static_cast<const hb_optim_t*>(pointer(a[7]));
     auto i64 = [&](PyObject* o) -> const int64_t* { return none(o) ? nullptr : tensor(o, "count").data_ptr<int64_t>(); };
-    const size_t need = hb_unique_segsum_workspace_bytes(n, dim);
+    const size_t need = hb_unique_update_workspace_bytes(n, dim, grads.data_ptr<float>(), opt);
     const at::Tensor ws = cuda_empty({(int64_t)need}, at::kByte, dev);
     check(hb_unique_update_f32(ids.data_ptr<int64_t>(), grads.data_ptr<float>(), i64(a[2]), n, i64(a[3]), i64(a[4]),
                                integer(a[5]), dim, (int)integer(a[6]), PyObject_IsTrue(a[8]),
-                               static_cast<const hb_optim_t*>(pointer(a[7])), ws.data_ptr(), need, stream_of(dev)));
+                               opt, ws.data_ptr(), need, stream_of(dev)));
     Py_RETURN_NONE;
   });
 }

@@ -25,8 +25,7 @@
 
 namespace hb {
 
-constexpr int kSegBlock = 256;
-
+constexpr int kSegBlockMin = 128;  // threads of the smallest CTA of any epilogue
 
 struct SegArgs {
   const uint8_t* head;        // [n] 1 where a run of equal ids starts in the sorted order
@@ -157,7 +156,9 @@ template <int VEC, int G, int VPL>
 struct EpiOps<StoreRows, VEC, G, VPL> {
   using V = typename VecF<VEC>::T;
   static constexpr int kFly = (8 / VPL) < G ? (8 / VPL) : G;
+  static constexpr int kBlock = 256;
   static constexpr int kMinBlocks = 4;
+  static constexpr int kPieceMax = 32;
   static constexpr bool kPrefetch = false;
   struct Lane {};
   struct Row {};
@@ -221,7 +222,10 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
   using Epi = UpdateRows<ADAM, STEP>;
   static constexpr int kStaged = 1 << 30;  // added to a row number: a staging slot
   static constexpr int kFly = VPL == 1 ? 2 : 1;
-  static constexpr int kMinBlocks = VPL > 2 ? 2 : 3;
+  // (a step's sums have the bits of StoreRows: a captured step and an eager one may differ in which they use)
+  static constexpr int kBlock = STEP ? 256 : 128;
+  static constexpr int kMinBlocks = (VPL > 2 ? 512 : 768) / kBlock;
+  static constexpr int kPieceMax = STEP ? 32 : 16;
   static constexpr bool kPrefetch = true;
   struct Lane {
     int row = -1;   // table row, or kStaged + staging slot
@@ -342,10 +346,11 @@ constexpr unsigned char kSegWhole = 2;   // ... which goes on behind the piece
 constexpr unsigned char kSegTail = 4;    // the piece's last run begins in it and goes on behind it
 
 template <int VEC, int G, int VPL, bool HAS_CNT, class Epi>
-__global__ void __launch_bounds__(kSegBlock, EpiOps<Epi, VEC, G, VPL>::kMinBlocks) segsum_kernel(SegArgs a, Epi epi) {
+__global__ void __launch_bounds__(EpiOps<Epi, VEC, G, VPL>::kBlock, EpiOps<Epi, VEC, G, VPL>::kMinBlocks)
+segsum_kernel(SegArgs a, Epi epi) {
   using V = typename VecF<VEC>::T;
   using Ops = EpiOps<Epi, VEC, G, VPL>;
-  constexpr int NG = kSegBlock / G;
+  constexpr int NG = Ops::kBlock / G;
   constexpr int U = Ops::kFly;  // rows whose loads are in flight together
   extern __shared__ __align__(16) float s_rows[];   // [NG][cols] pieces' parts of a run that began earlier
   __shared__ unsigned char s_flag[NG];
@@ -610,11 +615,13 @@ __global__ void __launch_bounds__(kSegBlock, EpiOps<Epi, VEC, G, VPL>::kMinBlock
 
 // ---- host side ------------------------------------------------------------------------------------
 // Rows per lane group: short pieces while the GPU has room for more groups (a piece is a chain of
-// loads), up to 32 once every SM has its 32 warps.  Measured on 2,000,000 x 128 (us, sums): 8: 224,
-// 16: 198, 32: 197, 64: 205; on 1,048,576 x 64 with the update fused: 235, 222, 239, 279.
-static inline int seg_piece(int64_t n, int lanes_per_row) {
+// loads), up to kPieceMax once every SM has its 32 warps.  Measured on 2,000,000 x 128 (us, sums): 8: 224,
+// 16: 198, 32: 197, 64: 205; on 1,048,576 x 64 with the update fused: 235, 222, 239, 279 (16 in CTAs of 128
+// threads instead of 32 in CTAs of 256: the whole call 314 -> 291, with 3 to 5 % on other widths; CTAs of 128
+// cost the plain sums of 2,000 x 64 2 us).
+static inline int seg_piece(int64_t n, int lanes_per_row, int most) {
   int r = 8;
-  while (r < 32 && ceil_div(n, r) * lanes_per_row / 32 > (int64_t)sm_count() * 32) r *= 2;
+  while (r < most && ceil_div(n, r) * lanes_per_row / 32 > (int64_t)sm_count() * 32) r *= 2;
   return r;
 }
 
@@ -630,8 +637,8 @@ static inline SegPlan seg_plan(void* ws, int64_t n, int64_t dim) {
   SegPlan s;
   Carver cv(ws ? ws : (void*)256);  // a null workspace still yields the sizes
   const int64_t m = n > 0 ? n : 1;
-  // CTAs: pieces of at least 8 rows, 8 groups (32 lanes per row) or more per CTA
-  s.max_ctas = ceil_div(m, 8 * (kSegBlock / 32)) + 1;
+  // CTAs: pieces of at least 8 rows, 4 groups (32 lanes per row) or more per CTA
+  s.max_ctas = ceil_div(m, 8 * (kSegBlockMin / 32)) + 1;
   const size_t cols = (size_t)(dim < 512 ? dim : 512);
   s.head_part = cv.take<float>((size_t)s.max_ctas * cols);
   s.tail_part = cv.take<float>((size_t)s.max_ctas * cols);
@@ -644,18 +651,19 @@ static inline SegPlan seg_plan(void* ws, int64_t n, int64_t dim) {
 
 template <int VEC, int G, int VPL, class Epi>
 int seg_launch(SegArgs a, const Epi& epi, cudaStream_t st) {
-  a.piece = seg_piece(a.n, G);  // the same for every epilogue: the sums have the same bits
-  const int ng = kSegBlock / G;
+  using Ops = EpiOps<Epi, VEC, G, VPL>;
+  a.piece = seg_piece(a.n, G, Ops::kPieceMax);
+  const int ng = Ops::kBlock / G;
   int grid = (int)ceil_div(a.n, (int64_t)ng * a.piece);
   if constexpr (Epi::kStep) grid += epi.touch_blocks;
   const size_t smem = (size_t)ng * a.cols * sizeof(float);
   if constexpr (Epi::kWeights) {
     if (a.cnt_in) {
-      HB_LAUNCH((segsum_kernel<VEC, G, VPL, true, Epi>), grid, kSegBlock, smem, st, a, epi);
+      HB_LAUNCH((segsum_kernel<VEC, G, VPL, true, Epi>), grid, Ops::kBlock, smem, st, a, epi);
       return HB_OK;
     }
   }
-  HB_LAUNCH((segsum_kernel<VEC, G, VPL, false, Epi>), grid, kSegBlock, smem, st, a, epi);
+  HB_LAUNCH((segsum_kernel<VEC, G, VPL, false, Epi>), grid, Ops::kBlock, smem, st, a, epi);
   return HB_OK;
 }
 

@@ -1,76 +1,76 @@
-// Aggregation of duplicate gradients and the sparse optimiser's row update in one pass: what
+// Aggregation of duplicate gradients and the sparse optimiser's row update in one call: what
 // SparseAdam.update does with ids that repeat (python/EmbCache/sparse_optim.py:608-681: unique_grads,
-// then state and table rows) without writing the merged rows and reading them back, and without
-// the launches and the unique count between the two.
+// then state and table rows), without the host reading the unique count between the two.
 #include "segsum.cuh"
 
 using namespace hb;
 
 namespace {
 
-int segsum_update(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean,
-                  const hb_optim_t* opt, void* workspace, size_t workspace_bytes, bool zeroed, cudaStream_t st) {
-  HB_CHECK_ARG(runs != nullptr && opt != nullptr && dim > 0, "hb_segsum_update_f32: bad argument");
-  const int64_t n = runs->n;
-  HB_CHECK_ARG(n == 0 || (grads && runs->perm && runs->head && runs->base8 && runs->run_start && runs->uniq_ids),
-               "hb_segsum_update_f32: null argument");
-  HB_CHECK_ARG(opt->kind == HB_OPT_ADAM || opt->kind == HB_OPT_ADAGRAD, "hb_segsum_update_f32: unknown optimiser");
-  HB_CHECK_ARG(opt->emb && opt->s0 && (opt->kind != HB_OPT_ADAM || (opt->s1 && opt->step)),
-               "hb_segsum_update_f32: incomplete optimiser description");
-  HB_CHECK_ARG(opt->emb_elem_bytes == 4 || opt->emb_elem_bytes == 2,
-               "hb_segsum_update_f32: embedding must be fp32 (4) or fp16 (2)");
-  HB_CHECK_ARG(opt->rows > 0 && opt->id_stride > 0, "hb_segsum_update_f32: bad sizes");
-  if (opt->rows >= ((int64_t)1 << 30)) {
-    set_error("hb_segsum_update_f32: shards of 2^30 rows and more are not updated in one pass");
-    return HB_ERR_UNSUPPORTED;
-  }
-  if (n == 0) return HB_OK;
-  const uintptr_t bits = (uintptr_t)grads | (uintptr_t)opt->emb | (uintptr_t)opt->s0 | (uintptr_t)opt->s1;
-  const bool vec4 = dim % 4 == 0 && (bits & 15) == 0;
-  if (dim > seg_tile(vec4)) {
-    // a row's step counter would be advanced once per pass over its columns
-    set_error("hb_segsum_update_f32: rows of %lld columns are not updated in one pass", (long long)dim);
-    return HB_ERR_UNSUPPORTED;
-  }
-  SegPlan s = seg_plan(workspace, n, dim);
-  if (!workspace || workspace_bytes < s.total) {
-    set_error("hb_segsum_update_f32: workspace of %zu bytes needed, %zu given", s.total, workspace_bytes);
-    return HB_ERR_WORKSPACE;
-  }
-  SegArgs a = seg_args(runs, grads, cnt_in, dim, mean, s);
-  a.cols = (int)dim;
-  if (!zeroed) HB_CUDA(cudaMemsetAsync(s.done, 0, (size_t)s.max_ctas * sizeof(unsigned), st));
-  if (opt->kind == HB_OPT_ADAM) return seg_dispatch(a, update_rows<true, false>(runs, opt), vec4, st);
-  return seg_dispatch(a, update_rows<false, false>(runs, opt), vec4, st);
+// Whether the sum of a run updates its rows at once instead of going through memory (write, read, one
+// launch).  That saves traffic, but rows are updated where their run ends, a few here and there in a warp,
+// while the update kernel takes 32 rows per warp.  Adagrad (us, at once / through memory): 20,000 x 32
+// 45 / 43, 60,000 x 128 71 / 75, 262,144 x 64 139 / 133, 524,288 x 64 194 / 204, 1,048,576 x 64 of fp16 291 / 329.
+// Adam, with two state rows and two powers per row: 5,000 x 100 47 / 37, 60,000 x 128 84 / 85, 200,000 x 128
+// 164 / 144, 700,000 x 128 278 / 268, 1,048,576 x 64 378 / 378: never.
+bool at_once(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt) {
+  if (opt->kind == HB_OPT_ADAM || n <= 32768 || opt->rows >= ((int64_t)1 << 30)) return false;
+  const uintptr_t bits = (uintptr_t)grads | (uintptr_t)opt->emb | (uintptr_t)opt->s0;
+  return dim <= seg_tile(dim % 4 == 0 && (bits & 15) == 0);
 }
+
+size_t sums_bytes(int64_t n, int64_t dim) { return align_up((size_t)(n * dim) * sizeof(float), 256); }
 
 }  // namespace
 
 extern "C" {
 
-int hb_segsum_update_f32(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean,
-                         const hb_optim_t* opt, void* workspace, size_t workspace_bytes, hb_stream_t stream) {
-  return segsum_update(runs, grads, cnt_in, dim, mean, opt, workspace, workspace_bytes, false, (cudaStream_t)stream);
+size_t hb_unique_update_workspace_bytes(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt) {
+  return hb_unique_segsum_workspace_bytes(n, dim) + (at_once(n, dim, grads, opt) ? 0 : sums_bytes(n, dim));
 }
 
 int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* cnt_in, int64_t n, const int64_t* n_dev,
                          const int64_t* seg_counts, int64_t seg_cap, int64_t dim, int id_bits, int mean,
                          const hb_optim_t* opt, void* workspace, size_t workspace_bytes, hb_stream_t stream) {
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31) && dim > 0, "hb_unique_update_f32: bad sizes");
-  const size_t runs_bytes = align_up(hb_runs_workspace_bytes(n), 256);
-  if (!workspace || workspace_bytes < runs_bytes + hb_segsum_runs_workspace_bytes(n, dim)) {
-    set_error("hb_unique_update_f32: workspace of %zu bytes needed, %zu given",
-              runs_bytes + hb_segsum_runs_workspace_bytes(n, dim), workspace_bytes);
+  HB_CHECK_ARG(opt != nullptr && (n == 0 || (ids && grads)), "hb_unique_update_f32: null argument");
+  HB_CHECK_ARG(opt->kind == HB_OPT_ADAM || opt->kind == HB_OPT_ADAGRAD, "hb_unique_update_f32: unknown optimiser");
+  HB_CHECK_ARG(opt->emb && opt->s0 && (opt->kind != HB_OPT_ADAM || (opt->s1 && opt->step)),
+               "hb_unique_update_f32: incomplete optimiser description");
+  HB_CHECK_ARG(opt->emb_elem_bytes == 4 || opt->emb_elem_bytes == 2,
+               "hb_unique_update_f32: embedding must be fp32 (4) or fp16 (2)");
+  HB_CHECK_ARG(opt->rows > 0 && opt->id_stride > 0, "hb_unique_update_f32: bad sizes");
+  if (n == 0) return HB_OK;
+  const size_t need = hb_unique_update_workspace_bytes(n, dim, grads, opt);
+  if (!workspace || workspace_bytes < need) {
+    set_error("hb_unique_update_f32: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
     return HB_ERR_WORKSPACE;
   }
-  char* seg_ws = static_cast<char*>(workspace) + runs_bytes;
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool once = at_once(n, dim, grads, opt);
+  float* sums = static_cast<float*>(workspace);  // first: on a 256-byte boundary
+  char* runs_ws = static_cast<char*>(workspace) + (once ? 0 : sums_bytes(n, dim));
+  const size_t runs_bytes = align_up(hb_runs_workspace_bytes(n), 256);
+  char* seg_ws = runs_ws + runs_bytes;
   const SegPlan s = seg_plan(seg_ws, n, dim);
   hb_runs_t runs;
   int rc = runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
-                      s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream);
+                      s.done, s.max_ctas, runs_ws, runs_bytes, &runs, st);
   if (rc != HB_OK) return rc;
-  return segsum_update(&runs, grads, cnt_in, dim, mean, opt, seg_ws, workspace_bytes - runs_bytes, true,
-                       (cudaStream_t)stream);
+  if (once) {
+    SegArgs a = seg_args(&runs, grads, cnt_in, dim, mean, s);
+    a.cols = (int)dim;
+    const uintptr_t bits = (uintptr_t)grads | (uintptr_t)opt->emb | (uintptr_t)opt->s0;
+    return seg_dispatch(a, update_rows<false, false>(&runs, opt), dim % 4 == 0 && (bits & 15) == 0, st);
+  }
+  rc = segsum_runs(&runs, grads, cnt_in, dim, mean, sums, nullptr, nullptr, seg_ws, s.total, true, st);
+  if (rc != HB_OK) return rc;
+  if (opt->kind == HB_OPT_ADAM)
+    return hb_sparse_adam(runs.uniq_ids, sums, nullptr, n, runs.num_runs, dim, opt->id_offset, opt->id_stride, opt->rows,
+                          opt->step, opt->s0, opt->s1, opt->emb, opt->emb_elem_bytes, opt->lr, opt->beta1, opt->beta2,
+                          opt->eps, stream);
+  return hb_sparse_adagrad(runs.uniq_ids, sums, nullptr, n, runs.num_runs, dim, opt->id_offset, opt->id_stride, opt->rows,
+                           opt->s0, opt->emb, opt->emb_elem_bytes, opt->lr, opt->eps, stream);
 }
 
 }  // extern "C"

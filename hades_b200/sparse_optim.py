@@ -129,20 +129,12 @@ class _SparseOptimizer:
         return idx.contiguous(), grad.contiguous(), None if cnt is None else cnt.contiguous()
 
 
-    def _update_merging(self, idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap) -> bool:
-        """unique_grads (sparse_optim.py:611) and the row update of what it returns in one pass over
-        the gradients; False: rows too wide or too many for that (``hb_segsum_update_f32``)."""
-        dim = grad.size(1)
-        w = self.emb.weight
-        desc = self._desc()
-        aligned = (w.data_ptr() | grad.data_ptr() | (desc.s0 or 0) | (desc.s1 or 0)) & 15 == 0
-        if idx.numel() == 0:
-            return True
-        if dim > (512 if dim % 4 == 0 and aligned else 128) or self.emb.rows >= 1 << 30:
-            return False
-        (_lib._NATIVE or _lib.native()).unique_update(idx, grad, cnt, n_dev, seg_counts, int(seg_cap), int(id_bits),
-                                                      C.addressof(desc), True)
-        return True
+    def _update_merging(self, idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap) -> None:
+        """unique_grads (sparse_optim.py:611) and the row update of what it returns."""
+        if idx.numel():
+            desc = self._desc()
+            (_lib._NATIVE or _lib.native()).unique_update(idx, grad, cnt, n_dev, seg_counts, int(seg_cap), int(id_bits),
+                                                          C.addressof(desc), True)
 
 
 class SparseAdam(_SparseOptimizer):
@@ -240,8 +232,8 @@ class SparseAdam(_SparseOptimizer):
         every segment holds strictly ascending ids (merge instead of sort)."""
         idx, grad, cnt = self._args(idx, grad, cnt)
         if not is_unique:
-            if self.state_cache is None and self._update_merging(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap):
-                return
+            if self.state_cache is None:
+                return self._update_merging(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap)
             idx, grad, n_dev = _merge_duplicates(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap, sorted_segments)
             cnt = None
         if self.state_cache is not None:
@@ -279,10 +271,7 @@ class SparseAdagrad(_SparseOptimizer):
         every segment holds strictly ascending ids (merge instead of sort)."""
         idx, grad, cnt = self._args(idx, grad, cnt)
         if not is_unique:
-            if self._update_merging(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap):
-                return
-            idx, grad, n_dev = _merge_duplicates(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap, sorted_segments)
-            cnt = None
+            return self._update_merging(idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap)
         lib = _lib.load()
         w = self.emb.weight
         _lib.check(lib.hb_sparse_adagrad(idx.data_ptr(), grad.data_ptr(), _lib.ptr(cnt), idx.numel(),

@@ -420,17 +420,10 @@ typedef struct hb_optim {
   double lr, beta1, beta2, eps;
 } hb_optim_t;
 
-/* hb_segsum_runs_f32 with the optimiser's update as its output: the merged row of every distinct id
- * updates the state and the table row directly (SparseAdam.update on ids that repeat,
- * python/EmbCache/sparse_optim.py:608-681), no merged rows in memory.  Rows of up to 512 columns (128
- * when dim is not a multiple of 4 or a buffer not 16-byte aligned), else HB_ERR_UNSUPPORTED.
- * Workspace: hb_segsum_runs_workspace_bytes. */
-int hb_segsum_update_f32(const hb_runs_t* runs /* host */, const float* grads,
-                         const int64_t* cnt_in /* nullable */, int64_t dim, int mean,
-                         const hb_optim_t* opt /* host */, void* workspace, size_t workspace_bytes,
-                         hb_stream_t stream);
-/* hb_runs_build + hb_segsum_update_f32; ids, n_dev, seg_counts, seg_cap, id_bits as for
- * hb_unique_segsum_f32.  Workspace: hb_unique_segsum_workspace_bytes. */
+/* hb_unique_segsum_f32 and the row update of the merged rows (SparseAdam.update on ids that repeat,
+ * python/EmbCache/sparse_optim.py:608-681), through memory or, where that is faster, as soon as a row's
+ * sum is complete; ids, n_dev, seg_counts, seg_cap, id_bits as for hb_unique_segsum_f32. */
+size_t hb_unique_update_workspace_bytes(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt /* host */);
 int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* cnt_in /* nullable */, int64_t n,
                          const int64_t* n_dev /* nullable */, const int64_t* seg_counts /* nullable */,
                          int64_t seg_cap, int64_t dim, int id_bits, int mean, const hb_optim_t* opt /* host */,
@@ -765,7 +758,8 @@ typedef struct hb_step_desc {
 
 int hb_step_create(hb_step_t** out);
 int hb_step_destroy(hb_step_t* s);
-/* 1 when the rows of this description are updated in one pass (hb_segsum_update_f32's limits). */
+/* 1 when the rows of this description can be updated as their sums are complete: rows of up to 512 columns
+ * (128 when dim is not a multiple of 4 or a buffer not 16-byte aligned). */
 int hb_step_supported(const hb_step_desc_t* d);
 size_t hb_step_workspace_bytes(int64_t n, int64_t dim);
 /* counters: device int64[4] = distinct ids, distinct ids of class 0, 1, 2.  locs nullable.

@@ -71,3 +71,11 @@ def test_update_of_repeated_ids(cuda_lib, kind, dtype, n, dim):
             assert torch.equal(opt.state_step.double(), step)
             assert float((opt.state_power.double() - s1).abs().max() / s1.abs().max()) < tol
         w = emb.weight.double()  # from here on the same table
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("n,dim", [(32_768, 64), (32_769, 3), (32_769, 64), (33_001, 8), (33_001, 16), (33_001, 47),
+                                   (33_001, 130), (33_001, 256), (33_001, 512), (33_001, 520)])
+def test_adagrad_at_the_edge_of_updating_at_once(cuda_lib, dtype, n, dim):
+    """More than 32,768 ids and rows of one pass: the row is updated when its sum is complete."""
+    test_update_of_repeated_ids(cuda_lib, "adagrad", dtype, n, dim)
