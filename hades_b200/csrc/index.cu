@@ -230,9 +230,9 @@ __global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const i
     }
   }
   if (part.arrived) {
-    __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) {
+      __threadfence_system();  // after the barrier: for the stores of the whole block
       unsigned* done = reinterpret_cast<unsigned*>(t.batch + 6);
       if (atomicAdd(done, 1u) == gridDim.x - 1u) {
         *done = 0u;

@@ -199,9 +199,9 @@ def test_add_and_lookup_of_large_batches(cuda_lib, oracle_mod, n, cache_size, ki
 
 
 @pytest.mark.parametrize("mode", [0, 1])
-@pytest.mark.parametrize("n", [1, 16_383, 16_384, 16_385, 32_769, 70_001])
+@pytest.mark.parametrize("n", [1, 16_383, 32_768, 32_769, 65_537, 98_306])
 def test_host_lookups_in_parts(cuda_lib, oracle_mod, n, mode):
-    """Host ids are looked up in parts of 16,384: slots, line ids and LRU counters at the edges of the
+    """Host ids are looked up in parts of up to 32,768: slots, line ids and LRU counters at the edges of the
     parts, with a hot id that ages in every part, ids that are strided in memory, and adds between."""
     from hades_b200 import EmbCacheLib as E
 
