@@ -434,8 +434,9 @@ int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st)
 
 // Where sets may get more ids than this on average, putting lists in order takes longer than the sort.
 constexpr int64_t kListedPerSet = 16;
-// One launch of the sort beats the launches of the lists up to one id per thread of the largest cluster.
-constexpr int64_t kAddSortMax = 16 * (int64_t)kClusterT;
+// One launch of the sort beats the launches of the lists up to here (add() of host ids: 2,000 33 us against
+// 32, 4,000 39 against 40, 6,000 49 against 42, 8,000 57 against 45).
+constexpr int64_t kAddSortMax = 8 * (int64_t)kClusterT;
 
 static size_t add_workspace_bytes(int64_t n) {
   if (n <= 0) return 256;

@@ -169,7 +169,8 @@ def test_touch_lru_from_runs(cuda_lib, oracle_mod, cache_size, id_range, n):
 
 # one launch of the sort (up to 8,192 ids), the lists of the sets, the sort again for many ids per set
 # (more than 16 per set on average); sets with lists of up to 32 ids, longer ones, copies of one id
-@pytest.mark.parametrize("n,cache_size,kind", [(8192, 4000, "uniform"), (8193, 4000, "uniform"), (8193, 4104, "uniform"),
+@pytest.mark.parametrize("n,cache_size,kind", [(4096, 4000, "uniform"), (4097, 4000, "uniform"), (4097, 1000, "uniform"),
+                                               (8192, 4000, "uniform"), (8193, 4000, "uniform"), (8193, 4104, "uniform"),
                                                (70_000, 100_000, "uniform"), (70_000, 100_000, "copies"),
                                                (20_000, 80_000, "strided"), (140_000, 800_000, "distinct"),
                                                (9_000, 160, "uniform"), (66_000, 160, "uniform")])
