@@ -42,7 +42,7 @@ struct SetSource {
   int64_t lines;
   const unsigned long long* heads;
   const int32_t* batch;
-  __device__ __forceinline__ int known_bits() const { return 0; }
+  __host__ __device__ int known_bits() const { return 0; }
   __device__ __forceinline__ int64_t count() const { return !LONG_LISTS || batch[2] == batch[0] ? n : 0; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
     const int64_t x = __ldg(ids + i);
@@ -130,7 +130,7 @@ struct ListedSource {
   const uint8_t* listed;
   const int64_t* cut;
   int64_t lines;
-  __device__ __forceinline__ int known_bits() const { return 0; }
+  __host__ __device__ int known_bits() const { return 0; }
   __device__ __forceinline__ int64_t count() const { return *n_dev < n ? *n_dev : n; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
     key = (unsigned long long)mod_nonneg(__ldg(ids + i), lines);

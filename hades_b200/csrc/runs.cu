@@ -40,7 +40,7 @@ struct IdSource {
   int64_t sentinel;
   int* err;
   int bits;  // stated by the caller
-  __device__ __forceinline__ int known_bits() const { return bits; }
+  __host__ __device__ int known_bits() const { return bits; }
   __device__ __forceinline__ int64_t count() const {
     if (!n_dev) return n;
     const int64_t d = *n_dev;

@@ -107,7 +107,7 @@ __device__ __forceinline__ SortDigits sort_digits(unsigned lo, unsigned hi, bool
 
 // Digits from what the caller says of its keys (valid ones below 2^bits - 1), where that is as good as
 // looking: not when one bit less would save a pass.  Spares an exchange between all CTAs.
-__device__ __forceinline__ bool sort_known_digits(int bits, int max_width, SortDigits& d) {
+__host__ __device__ inline bool sort_known_digits(int bits, int max_width, SortDigits& d) {
   if (bits <= 1 || bits > 30 || (bits + max_width - 1) / max_width != (bits - 1 + max_width - 1) / max_width) return false;
   d.wide = false;
   d.bits = bits;
@@ -602,18 +602,19 @@ struct GridCtx {
   }
 };
 
-static inline size_t sort_grid_smem_bytes() {
-  return (size_t)(kGridT / 32) * kGridBins * 6 + 2 * (size_t)kGridBins * 4 + (kGridT / 32) * 4 + 2 * sizeof(int4) + 32;
+static inline size_t sort_grid_smem_bytes(int digit) {
+  const size_t bins = (size_t)1 << digit;
+  return (size_t)(kGridT / 32) * bins * 6 + 2 * bins * 4 + (kGridT / 32) * 4 + 2 * sizeof(int4) + 32;
 }
 
 template <class Src, class Fin, int I>
 __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, SortGridBufs b, int max_digit, int* err) {
   extern __shared__ __align__(16) char smem[];
   uint16_t* wcnt = reinterpret_cast<uint16_t*>(smem);
-  uint32_t* wmask = reinterpret_cast<uint32_t*>(smem + (size_t)(kGridT / 32) * kGridBins * 2);
-  uint32_t* s_base = wmask + (kGridT / 32) * kGridBins;
-  uint32_t* s_tot = s_base + kGridBins;
-  int4* s_pref = reinterpret_cast<int4*>(s_tot + kGridBins);
+  uint32_t* wmask = reinterpret_cast<uint32_t*>(smem + ((size_t)(kGridT / 32) << max_digit) * 2);
+  uint32_t* s_base = wmask + ((kGridT / 32) << max_digit);
+  uint32_t* s_tot = s_base + (1 << max_digit);
+  int4* s_pref = reinterpret_cast<int4*>(s_tot + (1 << max_digit));
   uint32_t* s_warp = reinterpret_cast<uint32_t*>(s_pref + 2);
   unsigned* s_seen = s_warp + (kGridT / 32);
   int* s_flag = reinterpret_cast<int*>(s_seen + 4);
@@ -836,13 +837,22 @@ int sort_launch_cluster(const Src& src, const Fin& fin, int ctas, cudaStream_t s
 template <class Src, class Fin, int I>
 int sort_launch_grid(const Src& src, const Fin& fin, int64_t n, int max_digit, void* ws, cudaStream_t st) {
   SortGridBufs b = sort_grid_bufs(ws, n);
-  const size_t smem = sort_grid_smem_bytes();
+  // Ids of a stated width that needs no digit of 10 bits leave half of the 205 KB to the L1 cache (25 bits,
+  // three digits of 9: 282,624 ids 49.3 -> 47.3 us, 2,000,000 106.6 -> 102.6).  Not below 8 bits: the
+  // finish works in the words of the masks.
+  SortDigits stated;
+  if (sort_known_digits(src.known_bits(), max_digit, stated) && stated.width < max_digit) {
+    const int digit = stated.width < 8 ? 8 : stated.width;
+    if (sort_known_digits(src.known_bits(), digit, stated)) max_digit = digit;
+  }
+  const size_t smem = sort_grid_smem_bytes(max_digit);
   auto kernel = sort_grid_kernel<Src, Fin, I>;
   static thread_local int ready_dev = -1;
   int dev = 0;
   HB_CUDA(cudaGetDevice(&dev));
   if (ready_dev != dev) {
-    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sort_grid_smem_bytes(kGridDigit)));
     ready_dev = dev;
   }
   HB_CUDA(cudaMemsetAsync(b.barrier, 0, sizeof(unsigned), st));

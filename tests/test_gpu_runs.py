@@ -253,3 +253,21 @@ def test_miss_list_and_gathered_insert(cuda_lib, oracle_mod):
         gi, gl = cc.index.export_state()
         oi, ol = ox.export()
         assert np.array_equal(gi.cpu().numpy(), oi) and np.array_equal(gl.cpu().numpy(), ol)
+
+
+@pytest.mark.parametrize("bits", [2, 9, 16, 17, 18, 20, 21, 24, 25, 27, 28, 30, 31])
+def test_sort_of_ids_of_stated_width(cuda_lib, bits):
+    """Digits come from the stated width, and the shared memory of the grid version from the digits: the
+    largest ids of every width, the first one that does not fit, and the widths where it looks instead."""
+    from hades_b200 import EmbCacheLib as E
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(bits)
+    for n in (3_001, 65_537, 300_001):
+        top = (1 << bits) - 2  # 2^bits - 1 sorts last: it marks entries that take no part
+        ids = torch.randint(0, top + 1, (n,), device="cuda", generator=g)
+        ids[:5] = top
+        rows = torch.ones((n, 1), device="cuda")
+        u, _, cnt = E.cudaUniqueSegSum(ids, rows, id_bits=bits)
+        want, counts = torch.unique(ids, return_counts=True)
+        assert torch.equal(u, want) and torch.equal(cnt, counts), n
