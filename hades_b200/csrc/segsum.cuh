@@ -39,7 +39,7 @@ struct SegArgs {
   int64_t dim;
   int64_t col0;               // first column of this pass
   int cols;                   // columns of this pass (<= G * VEC * VPL)
-  int piece;                  // R: rows per lane group, a multiple of 8
+  int piece;                  // R: rows per lane group, a power of two
   int mean;                   // divide by the count
   // per CTA: what its part of a run that began earlier / of its last run adds up to
   float* head_part;           // [CTAs][cols]
@@ -618,9 +618,11 @@ segsum_kernel(SegArgs a, Epi epi) {
 // loads), up to kPieceMax once every SM has its 32 warps.  Measured on 2,000,000 x 128 (us, sums): 8: 224,
 // 16: 198, 32: 197, 64: 205; on 1,048,576 x 64 with the update fused: 235, 222, 239, 279 (16 in CTAs of 128
 // threads instead of 32 in CTAs of 256: the whole call 314 -> 291, with 3 to 5 % on other widths; CTAs of 128
-// cost the plain sums of 2,000 x 64 2 us).
+// cost the plain sums of 2,000 x 64 2 us).  The shortest, 4: with 8 a step of 2,000 x 64 takes 66 us instead of
+// 62, of 20,000 x 128 91 instead of 87, sums of 30,000 x 128 14.4 instead of 11.2.
+constexpr int kPieceMin = 4;
 static inline int seg_piece(int64_t n, int lanes_per_row, int most) {
-  int r = 8;
+  int r = kPieceMin;
   while (r < most && ceil_div(n, r) * lanes_per_row / 32 > (int64_t)sm_count() * 32) r *= 2;
   return r;
 }
@@ -637,8 +639,12 @@ static inline SegPlan seg_plan(void* ws, int64_t n, int64_t dim) {
   SegPlan s;
   Carver cv(ws ? ws : (void*)256);  // a null workspace still yields the sizes
   const int64_t m = n > 0 ? n : 1;
-  // CTAs: pieces of at least 8 rows, 4 groups (32 lanes per row) or more per CTA
-  s.max_ctas = ceil_div(m, 8 * (kSegBlockMin / 32)) + 1;
+  // CTAs of 4 groups (32 lanes per row) or more; pieces of 8 rows or longer, shorter ones only while the
+  // groups do not fill the GPU (a bound that does not fall with n: a workspace serves smaller batches)
+  s.max_ctas = ceil_div(m, 8 * (kSegBlockMin / 32));
+  const int64_t few = ceil_div(m, kPieceMin * (kSegBlockMin / 32)), filled = (int64_t)sm_count() * 64;
+  if (s.max_ctas < few) s.max_ctas = s.max_ctas > filled ? s.max_ctas : (few < filled ? few : filled);
+  s.max_ctas += 1;
   const size_t cols = (size_t)(dim < 512 ? dim : 512);
   s.head_part = cv.take<float>((size_t)s.max_ctas * cols);
   s.tail_part = cv.take<float>((size_t)s.max_ctas * cols);
