@@ -338,6 +338,19 @@ int check_desc(const hb_step_desc_t* d, const char* who) {
     set_error("%s: incomplete description", who);
     return HB_ERR_INVALID;
   }
+  // (as the stand-alone updates refuse them: hb_sparse_adam, hb_sparse_adagrad)
+  if (d->opt.kind != HB_OPT_ADAM && d->opt.kind != HB_OPT_ADAGRAD) {
+    set_error("%s: unknown optimiser", who);
+    return HB_ERR_INVALID;
+  }
+  if (d->opt.emb_elem_bytes != 4 && d->opt.emb_elem_bytes != 2) {
+    set_error("%s: embedding must be fp32 (4) or fp16 (2)", who);
+    return HB_ERR_INVALID;
+  }
+  if (d->opt.rows <= 0 || d->opt.id_stride <= 0 || (d->opt.kind == HB_OPT_ADAM && (!d->opt.s1 || !d->opt.step))) {
+    set_error("%s: incomplete optimiser description", who);
+    return HB_ERR_INVALID;
+  }
   if (d->staging.slots != d->index->cache_size || d->staging.dim != d->dim) {
     set_error("%s: the staging table must have one slot per cache slot and rows of dim columns", who);
     return HB_ERR_INVALID;
@@ -393,7 +406,6 @@ size_t hb_step_workspace_bytes(int64_t n, int64_t dim) { return step_plan(nullpt
 
 int hb_step_supported(const hb_step_desc_t* d) {
   if (check_desc(d, "hb_step_supported") != HB_OK) return 0;
-  if (d->opt.kind != HB_OPT_ADAM && d->opt.kind != HB_OPT_ADAGRAD) return 0;
   if (d->dim > seg_tile(vec4_ok(d, nullptr))) return 0;
   return d->opt.rows < ((int64_t)1 << 30) && d->staging.slots < ((int64_t)1 << 30);
 }

@@ -52,6 +52,26 @@ def test_no_gpu_calls_return_status_not_crash(built_lib):
     assert lib.hb_index_size(None) == -1
 
 
+@pytest.mark.parametrize("kind,change,why", [
+    (0, {"emb_elem_bytes": 8}, b"fp32 (4) or fp16 (2)"), (1, {"emb_elem_bytes": 8}, b"fp32 (4) or fp16 (2)"),
+    (0, {"s1": None}, b"optimiser description"), (0, {"step": None}, b"optimiser description"),
+    (1, {"id_stride": 0}, b"optimiser description"), (1, {"rows": 0}, b"optimiser description"),
+    (2, {}, b"unknown optimiser")])
+def test_step_refuses_what_the_updates_refuse(built_lib, kind, change, why):
+    """The description is checked before anything that it points to is looked at (addresses here are made up)."""
+    from hades_b200 import _lib
+
+    lib = _lib.load()
+    d = _lib.StepDesc()
+    d.index = d.cache_rows = d.table = d.class_table = 256
+    d.staging = _lib.StagingDesc(256, 256, 256, 256, 256, 8, 4)
+    d.row_bytes, d.dim, d.table_rows, d.class_len = 16, 4, 100, 100
+    d.opt = _lib.OptimDesc(kind, 4, 256, 256, 256, 256, 0, 1, 100, 0.01, 0.9, 0.999, 1e-8)
+    for k, v in change.items():
+        setattr(d.opt, k, v)
+    assert lib.hb_step_supported(ctypes.byref(d)) == 0 and why in lib.hb_last_error()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from hades_b200 import _lib
 

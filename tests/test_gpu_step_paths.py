@@ -1,0 +1,63 @@
+"""The one-trainer step as two library calls (``hb_step_forward`` / ``hb_step_backward``) against the same step
+composed of separate operators, and what it has to follow, refuse or leave to the composed form."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _small(name, dim=32, batch=4096, flush_every=3):
+    from hades_b200 import synth
+
+    return synth.CacheFetchConfig(name, 1, 30_000, dim, 3000, batch, 1.1, flush_every=flush_every)
+
+
+def _steps(cfg, n, seed=3):
+    from hades_b200 import synth
+
+    rng = synth.rng_for(1, 0, seed)
+    sampler = synth.ZipfSampler(cfg.table_rows, cfg.zipf_s)
+    return [(torch.from_numpy(sampler.ids(rng, cfg.batch)).cuda(),
+             torch.from_numpy(synth.normal_rows(rng, cfg.batch, cfg.dim, cfg.grad_sigma)).cuda()) for _ in range(n)]
+
+
+def _state(path):
+    r = path.cold.remote
+    out = {"table": path.table, "cache": path.cold.emb, "staged": r.grad, "cnt": r.cnt, "iter": r.iter_count,
+           "thr": r.iter_threshold, "dropped": path.cold.dropped}
+    out.update({k: v for k, v in vars(path.opt).items() if isinstance(v, torch.Tensor)})
+    out["line_ids"], out["lru"] = path.cold.index.export_state()
+    return out
+
+
+def _pair(name, **kw):
+    """The step as two library calls, and composed of separate operators."""
+    from hades_b200 import pipeline
+
+    dim = kw.pop("dim", 32)
+    a = pipeline.build_path(_small(name + "_a", dim), **kw)
+    b = pipeline.build_path(_small(name + "_b", dim), **kw)
+    assert a._one is not None
+    b._one = None
+    return a, b
+
+
+def _run_pair(a, b, batches):
+    for ids, g in batches:
+        ra, rb = a.step(ids, g), b.step(ids, g)
+        assert torch.equal(ra[0], rb[0]) and torch.equal(ra[2], rb[2])
+    sa, sb = _state(a), _state(b)
+    for k in sb:
+        assert torch.equal(sa[k], sb[k]), k
+
+
+def test_table_of_an_unsupported_type_is_refused(cuda_lib):
+    from hades_b200 import pipeline
+
+    cfg = _small("fp64_shard")
+    path = pipeline.build_path(cfg, table_dtype=torch.float64)
+    weight = path.opt.emb.weight.clone()
+    (ids, g), = _steps(cfg, 1)
+    with pytest.raises(RuntimeError, match=r"fp32 \(4\) or fp16 \(2\)"):
+        path.step(ids, g)
+    assert torch.equal(path.opt.emb.weight, weight)
