@@ -74,7 +74,7 @@ class _OneGpuStep:
     """One trainer's step on one GPU as two library calls (``hb_step_forward`` / ``hb_step_backward``): what
     ``forward`` and ``backward`` of the path compose from separate operators when other GPUs take part."""
 
-    def __init__(self, path: "EmbeddingPath"):
+    def __init__(self):
         # (no reference to the path: a cycle would keep the table and the optimiser's state until a
         # garbage collection)
         self.lib, self.native = E._lib.load(), E._lib.native()
@@ -85,9 +85,7 @@ class _OneGpuStep:
         self.addr = C.addressof(self.desc)
         self.ws, self.kept = None, []
         self.batch = None  # (ids, version, counters) of the last forward pass
-        self.key = None
-        self.refresh(path)
-        self.supported = bool(self.lib.hb_step_supported(C.byref(self.desc)))
+        self.key, self.supported = None, False
 
     def __del__(self):
         try:
@@ -95,23 +93,30 @@ class _OneGpuStep:
         except Exception:  # interpreter shutdown
             pass
 
-    def refresh(self, p: "EmbeddingPath") -> None:
-        """The description follows the path's attributes (they may change between steps)."""
-        d = self.desc
-        cold, opt = p.cold, p.opt
-        key = (p.lookup_mode, p.touch_lru, p.insert_misses, p.miss_cap, p.id_bits, cold.default_threshold, opt._lr,
-               p.table.data_ptr(), p.class_table.data_ptr(), cold.emb.data_ptr(), opt.emb.weight.data_ptr())
-        if key == self.key:
-            return
-        self.key = key
-        d.index, d.staging, d.cache_rows = cold.index._h, cold.remote.desc, cold.emb.data_ptr()
-        d.table, d.table_rows = p.table.data_ptr(), p.table.size(0)
-        d.row_bytes, d.dim = p.dim * cold.emb.element_size(), p.dim
-        d.class_table, d.class_len, d.id_bits = p.class_table.data_ptr(), p.num_nodes, p.id_bits
-        d.lookup_mode, d.touch_lru, d.insert_misses = p.lookup_mode, p.touch_lru, p.insert_misses
-        d.miss_cap, d.default_threshold = p.miss_cap, cold.default_threshold
-        d.threshold_table = None if cold.threshold is None else cold.threshold.data_ptr()
-        d.dropped, d.opt = cold.dropped.data_ptr(), opt._desc()
+    def takes(self, p: "EmbeddingPath") -> bool:
+        """Brings the description up to date with the path, whose attributes may change between steps;
+        False where the step has to be composed.  The key holds everything that the description does:
+        addresses as they are now, and the staging table itself."""
+        cold, opt, table = p.cold, p.opt, p.table
+        if p.world != 1 or p.shared is not None or table is None or getattr(opt, "state_cache", None) is not None:
+            return False
+        fields, cls, emb, thr = opt._fields(), p.class_table, cold.emb, cold.threshold
+        key = (p.lookup_mode, p.touch_lru, p.insert_misses, p.miss_cap, p.id_bits, p.dim, table.data_ptr(), table.size(0),
+               table.dtype, cls.data_ptr(), cls.numel(), emb.data_ptr(), emb.dtype, cold.index._h.value, cold.remote,
+               cold.default_threshold, None if thr is None else thr.data_ptr(), cold.dropped.data_ptr(), fields)
+        if key != self.key:
+            d = self.desc
+            d.index, d.staging, d.cache_rows = cold.index._h, cold.remote.desc, emb.data_ptr()
+            d.table, d.table_rows = table.data_ptr(), table.size(0)
+            d.row_bytes, d.dim = p.dim * emb.element_size(), p.dim
+            d.class_table, d.class_len, d.id_bits = cls.data_ptr(), cls.numel(), p.id_bits
+            d.lookup_mode, d.touch_lru, d.insert_misses = p.lookup_mode, p.touch_lru, p.insert_misses
+            d.miss_cap, d.default_threshold = p.miss_cap, cold.default_threshold
+            d.threshold_table = None if thr is None else thr.data_ptr()
+            d.dropped, d.opt = cold.dropped.data_ptr(), E._lib.OptimDesc(*fields)
+            self.supported = table.dtype == emb.dtype and bool(self.lib.hb_step_supported(C.byref(d)))
+            self.key = key
+        return self.supported
 
     def keep(self, p: "EmbeddingPath", ws: torch.Tensor) -> None:
         """Scratch of the last batch.  What captured graphs hold stays."""
@@ -122,7 +127,6 @@ class _OneGpuStep:
 
     def forward(self, p: "EmbeddingPath", ids: torch.Tensor, out_rows, aside: bool):
         ids = ids.contiguous()
-        self.refresh(p)
         rows, locs, found, counters, ws = self.native.step_forward(
             self._h.value, self.addr, ids, p.dim, p.cold.emb, out_rows, p.want_locs, aside, self.ws)
         self.keep(p, ws)
@@ -136,7 +140,6 @@ class _OneGpuStep:
         if p.dim > 128 and grads.data_ptr() & 15:
             grads = grads.clone()  # wide rows are read 16 bytes at a time
         b = self.batch
-        self.refresh(p)
         if b is not None and (ids is b[0] or (ids.data_ptr() == b[0].data_ptr() and n == b[0].numel())) \
                 and ids._version == b[1]:
             counters, given = b[2], None
@@ -211,11 +214,15 @@ class EmbeddingPath:
         self._runs_ws, self._side_ws, self._fetch_ws = None, None, None
         self._last = None  # (BatchRuns, locs) of the last forward pass
         # one trainer, its table and its optimiser's state on this GPU: the step as two library calls
-        self._one = None
-        if (world == 1 and self.shared is None and table is not None and table.dtype == cold.emb.dtype
-                and getattr(optimizer, "state_cache", None) is None):
-            one = _OneGpuStep(self)
-            self._one = one if one.supported else None
+        self._one = _OneGpuStep() if world == 1 and self.shared is None and table is not None else None
+
+    def _in_two_calls(self) -> bool:
+        """Whether the step takes the form of two library calls; work of its side stream is joined where not."""
+        one = self._one
+        if one is None or one.takes(self):
+            return one is not None
+        one.join()
+        return False
 
     def _graphs_hold_scratch(self) -> bool:
         return bool(self._graphs) or getattr(self, "_split", None) is not None
@@ -259,7 +266,7 @@ class EmbeddingPath:
         overlap_fetch): everything after the sort runs on the side stream and the rows are
         complete only after the join at the end of the backward pass."""
         n = ids.numel()
-        if self._one is not None and n > 0:
+        if n > 0 and self._in_two_calls():
             self._last = None
             return self._one.forward(self, ids, out_rows, on_side)
         lib = E._lib.load()
@@ -479,7 +486,8 @@ class EmbeddingPath:
         overlap_fetch), the exchange waits until that fetch has read what it needs from the other
         GPUs' shards, and the owner update until it has read what it needs from this GPU's shard:
         a fetch returns the rows as they were before the step's update."""
-        if self._one is not None and ids.numel() > 0:
+        if ids.numel() > 0 and self._in_two_calls():
+            self._join_side()  # of a forward pass that was composed
             return self._one.backward(self, ids, grads)
         st, hot_ids, hot_rows, hot_cnt = self._backward_local(ids, grads, join=False)
         n_hot = st.split_counts[HOT:HOT + 1]

@@ -132,7 +132,7 @@ class _SparseOptimizer:
     def _update_merging(self, idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap) -> None:
         """unique_grads (sparse_optim.py:611) and the row update of what it returns."""
         if idx.numel():
-            desc = self._desc()
+            desc = _lib.OptimDesc(*self._fields())
             (_lib._NATIVE or _lib.native()).unique_update(idx, grad, cnt, n_dev, seg_counts, int(seg_cap), int(id_bits),
                                                           C.addressof(desc), True)
 
@@ -176,12 +176,11 @@ class SparseAdam(_SparseOptimizer):
         self.state_mem = torch.zeros((emb.rows, dim), dtype=torch.float32, device=dev)
         self.state_power = torch.zeros((emb.rows, dim), dtype=torch.float32, device=dev)
 
-    def _desc(self):
-        """hb_optim_t of the state in HBM (its tensors keep their addresses; lr may change)."""
+    def _fields(self) -> tuple:
+        """The members of hb_optim_t as they are now (state in HBM)."""
         w, e = self.emb.weight, self.emb
-        return _lib.OptimDesc(0, w.element_size(), w.data_ptr(), self.state_mem.data_ptr(), self.state_power.data_ptr(),
-                              self.state_step.data_ptr(), e.rank, e.world, e.rows, self._lr, self._beta1, self._beta2,
-                              self._eps)
+        return (0, w.element_size(), w.data_ptr(), self.state_mem.data_ptr(), self.state_power.data_ptr(),
+                self.state_step.data_ptr(), e.rank, e.world, e.rows, self._lr, self._beta1, self._beta2, self._eps)
 
     def full_state(self):
         """(step, mem, power) of the whole shard as CUDA tensors, whichever tier the rows are in."""
@@ -257,11 +256,11 @@ class SparseAdagrad(_SparseOptimizer):
         self.state_sum = torch.zeros((emb.rows, emb.embedding_dim), dtype=torch.float32,
                                      device=emb.weight.device)
 
-    def _desc(self):
-        """hb_optim_t of the state (its tensors keep their addresses; lr may change)."""
+    def _fields(self) -> tuple:
+        """The members of hb_optim_t as they are now."""
         w, e = self.emb.weight, self.emb
-        return _lib.OptimDesc(1, w.element_size(), w.data_ptr(), self.state_sum.data_ptr(), None, None, e.rank, e.world,
-                              e.rows, self._lr, 0.0, 0.0, self._eps)
+        return (1, w.element_size(), w.data_ptr(), self.state_sum.data_ptr(), None, None, e.rank, e.world, e.rows, self._lr,
+                0.0, 0.0, self._eps)
 
     def update(self, idx, grad, cnt=None, is_unique: bool = False, n_dev: torch.Tensor | None = None,
                id_bits: int = 64, seg_counts: torch.Tensor | None = None, seg_cap: int = 0,

@@ -61,3 +61,35 @@ def test_table_of_an_unsupported_type_is_refused(cuda_lib):
     with pytest.raises(RuntimeError, match=r"fp32 \(4\) or fp16 \(2\)"):
         path.step(ids, g)
     assert torch.equal(path.opt.emb.weight, weight)
+
+
+@pytest.mark.parametrize("what", ["adagrad", "fresh_adam", "eps", "threshold", "dropped", "staging", "class_table"])
+def test_attributes_of_the_path_may_change_between_steps(cuda_lib, what):
+    from hades_b200.cold_cache import StagingTable
+    from hades_b200.sparse_optim import SparseAdagrad, SparseAdam
+
+    a, b = _pair("attr_" + what)
+    batches = _steps(_small("attr"), 8)
+    _run_pair(a, b, batches[:4])
+    old = []  # what was in use stays allocated
+    for p in (a, b):
+        old.append(dict(vars(p)))
+        if what == "adagrad":
+            p.opt = SparseAdagrad(p.opt.emb, lr=0.01)
+        elif what == "fresh_adam":
+            old.append(p.opt)
+            p.opt = SparseAdam(p.opt.emb, lr=0.01)
+        elif what == "eps":
+            p.opt._eps = 1e-2
+        elif what == "threshold":
+            old.append(p.cold.threshold)
+            p.cold.threshold = torch.full((p.num_nodes,), 2, dtype=torch.int32, device="cuda")
+        elif what == "dropped":
+            old.append(p.cold.dropped)
+            p.cold.dropped = torch.zeros(1, dtype=torch.int64, device="cuda")
+        elif what == "staging":
+            old.append(p.cold.remote)
+            p.cold.remote = StagingTable(p.cold.remote.slots, p.dim, p.cold.emb.device)
+        elif what == "class_table":
+            p.class_table = torch.full_like(p.class_table, 2)
+    _run_pair(a, b, batches[4:])
