@@ -70,6 +70,18 @@ class _CounterStats(StepStats):
     sent_counts = property(lambda self: self.counters[2:3])
 
 
+def _own_arithmetic(cold, opt) -> bool:
+    """The update and the staging are this package's, with the state in HBM (an optimiser of the user's own is called)."""
+    return (type(cold) is ColdCache and type(opt) in (SparseAdam, SparseAdagrad) and "update" not in opt.__dict__
+            and getattr(opt, "state_cache", None) is None)
+
+
+def _rows_of(t: torch.Tensor, dtype, dim: int) -> bool:
+    """Rows of dim columns that kernels can read."""
+    return (t.dtype == dtype and t.dim() == 2 and t.size(1) == dim and t.is_contiguous()
+            and (t.is_cuda or t.is_pinned() or t.data_ptr() in E._PINNED))
+
+
 class _OneGpuStep:
     """One trainer's step on one GPU as two library calls (``hb_step_forward`` / ``hb_step_backward``): what
     ``forward`` and ``backward`` of the path compose from separate operators when other GPUs take part."""
@@ -98,12 +110,13 @@ class _OneGpuStep:
         False where the step has to be composed.  The key holds everything that the description does:
         addresses as they are now, and the staging table itself."""
         cold, opt, table = p.cold, p.opt, p.table
-        if p.world != 1 or p.shared is not None or table is None or getattr(opt, "state_cache", None) is not None:
+        if p.world != 1 or p.shared is not None or table is None or not _own_arithmetic(cold, opt):
             return False
         fields, cls, emb, thr = opt._fields(), p.class_table, cold.emb, cold.threshold
-        key = (p.lookup_mode, p.touch_lru, p.insert_misses, p.miss_cap, p.id_bits, p.dim, table.data_ptr(), table.size(0),
-               table.dtype, cls.data_ptr(), cls.numel(), emb.data_ptr(), emb.dtype, cold.index._h.value, cold.remote,
-               cold.default_threshold, None if thr is None else thr.data_ptr(), cold.dropped.data_ptr(), fields)
+        key = (p.lookup_mode, p.touch_lru, p.insert_misses, p.miss_cap, p.id_bits, p.dim, table.data_ptr(), table.shape,
+               table.stride(), table.dtype, cls.data_ptr(), cls.shape, cls.stride(), cls.dtype, emb.data_ptr(), emb.shape,
+               emb.stride(), emb.dtype, cold.index._h.value, cold.remote, cold.default_threshold,
+               None if thr is None else thr.data_ptr(), cold.dropped.data_ptr(), fields)
         if key != self.key:
             d = self.desc
             d.index, d.staging, d.cache_rows = cold.index._h, cold.remote.desc, emb.data_ptr()
@@ -114,7 +127,10 @@ class _OneGpuStep:
             d.miss_cap, d.default_threshold = p.miss_cap, cold.default_threshold
             d.threshold_table = None if thr is None else thr.data_ptr()
             d.dropped, d.opt = cold.dropped.data_ptr(), E._lib.OptimDesc(*fields)
-            self.supported = table.dtype == emb.dtype and bool(self.lib.hb_step_supported(C.byref(d)))
+            # (what the operators of the composed step check: there it raises)
+            self.supported = (cls.dtype == torch.int8 and cls.is_cuda and cls.is_contiguous()
+                              and _rows_of(table, emb.dtype, p.dim) and _rows_of(emb, emb.dtype, p.dim)
+                              and bool(self.lib.hb_step_supported(C.byref(d))))
             self.key = key
         return self.supported
 

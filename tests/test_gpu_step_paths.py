@@ -93,3 +93,46 @@ def test_attributes_of_the_path_may_change_between_steps(cuda_lib, what):
         elif what == "class_table":
             p.class_table = torch.full_like(p.class_table, 2)
     _run_pair(a, b, batches[4:])
+
+
+def test_optimizer_of_the_users_own_is_called(cuda_lib):
+    from hades_b200.sparse_optim import SparseAdam
+
+    class Clipped(SparseAdam):
+        calls = 0
+
+        def update(self, idx, grad, *args, **kw):
+            Clipped.calls += 1
+            return super().update(idx, grad.clamp(-1e-4, 1e-4), *args, **kw)
+
+    from hades_b200 import pipeline
+
+    cfg = _small("own_opt")
+    p = pipeline.build_path(cfg)
+    q = pipeline.EmbeddingPath(p.table, p.class_table, p.cold, Clipped(p.opt.emb, lr=0.01), flush_every=3, id_bits=p.id_bits)
+    (ids, g), = _steps(cfg, 1)
+    q.step(ids, g)
+    assert Clipped.calls == 1
+
+
+@pytest.mark.parametrize("what,why", [("wide_classes", "int8"), ("host_table", "pinned host memory"),
+                                      ("strided_table", "contiguous"), ("narrow_table", r"size\(1\)")])
+def test_tensors_that_do_not_fit_are_refused(cuda_lib, what, why):
+    from hades_b200 import pipeline
+
+    cfg = _small("misfit_" + what)
+    path = pipeline.build_path(cfg)
+    (ids, g), = _steps(cfg, 1)
+    if what == "wide_classes":
+        path.class_table = path.class_table.long()
+    elif what == "host_table":
+        path.table = path.table.cpu()
+    elif what == "strided_table":
+        path.table = torch.cat([path.table, path.table], 1)[:, :cfg.dim]
+    else:
+        path.table = path.table[:, : cfg.dim // 2].contiguous()
+    before = _state(path)
+    with pytest.raises(RuntimeError, match=why):
+        path.forward(ids)
+    after = _state(path)
+    assert all(torch.equal(before[k], after[k]) for k in before)
