@@ -124,11 +124,14 @@ __device__ __forceinline__ void vadd(float4& a, const float4& b) {
 __device__ __forceinline__ void vadd(float& a, const float& b) { a += b; }
 __device__ __forceinline__ void vzero(float4& a) { a = make_float4(0.f, 0.f, 0.f, 0.f); }
 __device__ __forceinline__ void vzero(float& a) { a = 0.f; }
-// a / d with r = 1 / d given: one correction of the product by its exact remainder (Markstein: the
-// quotient is then correctly rounded), three instructions instead of a division per value
+// a / d for a whole number d with r = 1 / d given: one correction of the product by its remainder, which is
+// exact as d is whole (Markstein: the quotient is then correctly rounded; a subnormal one that lies halfway
+// between two floats goes to either), instead of a division per value.  The remainder of an infinite sum is NaN, of
+// which the minimum makes a number that leaves the infinity as it is.  (60,000 rows for Adam, sums and update: 84.2
+// us without, 84.7 so, with a select 2 % more, with a branch to a division 5 %: registers.)
 __device__ __forceinline__ void vdiv(float& a, float d, float r) {
   const float q = a * r;
-  a = fmaf(fmaf(-q, d, a), r, q);
+  a = fmaf(fminf(fmaf(-q, d, a), 3.402823466e38f), r, q);
 }
 __device__ __forceinline__ void vdiv(float4& a, float d, float r) {
   vdiv(a.x, d, r);

@@ -146,3 +146,47 @@ def test_merge_sorted_slabs_equals_sorting_path(cuda_lib, oracle_mod, num_seg, c
                                             cnt.reshape(-1)[valid] if with_cnt else None)
         assert np.array_equal(u[:k].cpu().numpy(), wu)
         np.testing.assert_allclose(r[:k].cpu().numpy(), wm, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("dim", [4, 5])
+def test_means_of_infinite_and_tiny_sums(cuda_lib, dim):
+    from hades_b200 import EmbCacheLib as E
+
+    inf, nan = float("inf"), float("nan")
+    vals = [inf, -inf, nan, 3e38, -3e38, 0.0, -0.0, 1e-45, -1e-45, 3e-39, 1.1754944e-38, 5e-38, 1e-37, 7e-33, -3e-31, 1.0, 1 / 3]
+    copies = [1, 2, 3, 5, 7, 10]
+    ids, rows, want = [], [], []
+    for k, c in enumerate(copies):
+        for j, v in enumerate(vals):
+            ids += [k * len(vals) + j] * c
+            # one copy holds the value, the others nothing: the sum is the value
+            rows += [[v] * dim] + [[-0.0] * dim] * (c - 1)
+            want.append(torch.tensor(0.0 + v) / torch.tensor(float(c)))
+    ids = torch.tensor(ids, device="cuda")
+    grads = torch.tensor(rows, dtype=torch.float32, device="cuda")
+    _, got, _ = E.cudaUniqueSegSum(ids, grads, mean=True, id_bits=32)
+    want = torch.stack(want).float()[:, None].expand(-1, dim)
+    got = got.cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    ok = ~torch.isnan(want)
+    assert torch.equal(got[ok], want[ok]) and torch.equal(torch.signbit(got[ok]), torch.signbit(want[ok]))
+
+
+def test_means_are_divisions(cuda_lib):
+    from hades_b200 import EmbCacheLib as E
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    bits = torch.randint(-2**31, 2**31, (1 << 20,), device="cuda", generator=g).to(torch.int32)
+    v = bits.view(torch.float32)
+    v = torch.where(torch.isfinite(v), v, torch.zeros_like(v)).view(-1, 16)
+    n = v.size(0)
+    ids = torch.arange(n, device="cuda")
+    for c in (2, 3, 7, 10, 49, 1000, 65_537, 16_777_213, 16_777_215):
+        cnt = torch.full((n,), c - 1, device="cuda")
+        _, got, _ = E.cudaUniqueSegSum(ids, v, cnt, mean=True, id_bits=32)
+        got, want = got.cpu(), v.cpu() / torch.tensor(float(c))
+        # a quotient halfway between two subnormal numbers may go to either
+        halves = (want.abs() < 2.0**-126) & ((2 * v.cpu().double() / c / 2.0**-149) % 2 == 1)
+        assert torch.equal(got[~halves], want[~halves]), c
+        assert bool(((got - want)[halves].abs() <= 2.0**-149).all()), c
