@@ -131,6 +131,7 @@ class _SparseOptimizer:
 
     def _update_merging(self, idx, grad, cnt, n_dev, id_bits, seg_counts, seg_cap) -> None:
         """unique_grads (sparse_optim.py:611) and the row update of what it returns."""
+        _check(grad.dim() == 2 and grad.size(0) == idx.numel(), "grads.size(0) == ids.numel()")
         if idx.numel():
             desc = _lib.OptimDesc(*self._fields())
             (_lib._NATIVE or _lib.native()).unique_update(idx, grad, cnt, n_dev, seg_counts, int(seg_cap), int(id_bits),

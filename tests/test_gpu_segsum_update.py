@@ -79,3 +79,15 @@ def test_update_of_repeated_ids(cuda_lib, kind, dtype, n, dim):
 def test_adagrad_at_the_edge_of_updating_at_once(cuda_lib, dtype, n, dim):
     """More than 32,768 ids and rows of one pass: the row is updated when its sum is complete."""
     test_update_of_repeated_ids(cuda_lib, "adagrad", dtype, n, dim)
+
+
+@pytest.mark.parametrize("kind", ["adam", "adagrad"])
+def test_fewer_rows_than_ids_are_refused(cuda_lib, kind):
+    from hades_b200.sparse_optim import ShardedEmbedding, SparseAdagrad, SparseAdam
+
+    emb = ShardedEmbedding(100, 8, init_sigma=0.01)
+    opt = (SparseAdam if kind == "adam" else SparseAdagrad)(emb, lr=LR)
+    before = emb.weight.clone()
+    with pytest.raises(RuntimeError, match="Check failed"):
+        opt.update(torch.arange(20, device="cuda"), torch.ones((19, 8), device="cuda"))
+    assert torch.equal(emb.weight, before)
