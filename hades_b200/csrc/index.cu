@@ -452,13 +452,13 @@ int index_add_runs_sorted(hb_index* h, const AddEntries& e, void* ws, int64_t* l
   uint2* sorted = cv.take<uint2>(e.n);
   int64_t* cut = cv.take<int64_t>(1);
   HB_LAUNCH(add_cut_kernel, 1, kBlock, 0, st, e, cut);
+  h->sorted_stale = true;
   return sort_run(ListedSource{e.ids, e.n, e.n_dev, e.listed, cut, h->lines},
                   AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, e.n, cv.take<char>(0), st);
 }
 
 int index_add_state(hb_index* h, uint32_t* next, int64_t* locs, uint8_t* last_writer, AddState* out) {
   *out = AddState{h->heads, h->batch + 2, next, h->lines, h->line_ids, h->lru, locs, last_writer};
-  h->sorted_stale = true;
   return HB_OK;
 }
 

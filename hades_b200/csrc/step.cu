@@ -465,6 +465,7 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
   Maintain m;
   memset(&m, 0, sizeof(m));
   const bool lists_used = d->insert_misses && index_add_runs_lists(h, n);
+  if (lists_used) h->sorted_stale = true;  // (ageing leaves the ids where they are)
   if (d->touch_lru || lists_used) {
     m.v = RunsView{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
     m.marks = marks;

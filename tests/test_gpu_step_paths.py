@@ -136,3 +136,31 @@ def test_tensors_that_do_not_fit_are_refused(cuda_lib, what, why):
         path.forward(ids)
     after = _state(path)
     assert all(torch.equal(before[k], after[k]) for k in before)
+
+
+def test_sorted_view_stays_fresh_where_nothing_is_inserted(cuda_lib):
+    from hades_b200 import EmbCacheLib as E
+    from hades_b200 import pipeline
+
+    cfg = _small("sorted_noinsert", flush_every=0)
+    paths = [pipeline.build_path(_small(f"sorted_noinsert_{k}", flush_every=0), lookup_mode=E.LOOKUP_SORTED, insert_misses=False)
+             for k in range(2)]
+    batches = _steps(cfg, 6)
+    outs = [torch.empty((cfg.batch, cfg.dim), device="cuda") for _ in paths]
+    for ids, _ in batches[:2]:
+        for p, o in zip(paths, outs):
+            p.step(ids, batches[0][1], o)
+    buf = torch.empty_like(batches[0][0])
+    paths[1].capture(buf, batches[0][1], outs[1])
+    for ids, _ in batches[2:]:
+        r = [p.step(ids, batches[0][1], o) for p, o in zip(paths, outs)]
+        assert torch.equal(r[0][0], r[1][0]) and torch.equal(r[0][2], r[1][2])
+    sa, sb = _state(paths[0]), _state(paths[1])
+    for k in sa:
+        assert torch.equal(sa[k], sb[k]), k
+
+
+def test_sorted_view_follows_insertions(cuda_lib):
+    from hades_b200 import EmbCacheLib as E
+
+    _run_pair(*_pair("sorted_insert", lookup_mode=E.LOOKUP_SORTED), _steps(_small("sorted_insert"), 7))
