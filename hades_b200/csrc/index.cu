@@ -394,41 +394,8 @@ int grid_capped(int64_t n, int block = kBlock) {
 
 }  // namespace
 
-static int alloc_batch_counters(hb_index* h, cudaStream_t st) {
-  if (h->batch) return HB_OK;
-  HB_CUDA(cudaMalloc(&h->batch, 8 * sizeof(int32_t)));
-  HB_CUDA(cudaMemsetAsync(h->batch, 0, 8 * sizeof(int32_t), st));
-  return HB_OK;
-}
-
-// (scratch is allocated on first use: do that outside any stream capture)
-int index_touch_marks(hb_index* h, TouchMarks* out, cudaStream_t st) {
-  if (!h->marks) {
-    const int rc = alloc_batch_counters(h, st);
-    if (rc != HB_OK) return rc;
-    HB_CUDA(cudaMalloc(&h->marks, h->cache_size * sizeof(unsigned long long)));
-    HB_CUDA(cudaMemsetAsync(h->marks, 0, h->cache_size * sizeof(unsigned long long), st));
-  }
-  *out = TouchMarks{h->marks, h->batch, h->cache_size};
-  return HB_OK;
-}
-
 int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st) {
-  TouchMarks marks;
-  const int rc = index_touch_marks(h, &marks, st);
-  if (rc != HB_OK) return rc;
-  HB_LAUNCH(touch_runs_apply_kernel, grid_capped(v.max_runs), kBlock, 0, st, v, marks, h->lru);
-  return HB_OK;
-}
-
-int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st) {
-  if (!h->heads) {
-    const int rc = alloc_batch_counters(h, st);
-    if (rc != HB_OK) return rc;
-    HB_CUDA(cudaMalloc(&h->heads, h->lines * sizeof(unsigned long long)));
-    HB_CUDA(cudaMemsetAsync(h->heads, 0, h->lines * sizeof(unsigned long long), st));
-  }
-  *out = AddLists{h->heads, h->batch + 2, next, h->lines};
+  HB_LAUNCH(touch_runs_apply_kernel, grid_capped(v.max_runs), kBlock, 0, st, v, index_touch_marks(h), h->lru);
   return HB_OK;
 }
 
@@ -457,11 +424,6 @@ int index_add_runs_sorted(hb_index* h, const AddEntries& e, void* ws, int64_t* l
                   AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, e.n, cv.take<char>(0), st);
 }
 
-int index_add_state(hb_index* h, uint32_t* next, int64_t* locs, uint8_t* last_writer, AddState* out) {
-  *out = AddState{h->heads, h->batch + 2, next, h->lines, h->line_ids, h->lru, locs, last_writer};
-  return HB_OK;
-}
-
 }  // namespace hb
 
 using namespace hb;
@@ -469,9 +431,19 @@ using namespace hb;
 extern "C" {
 
 namespace {
-// everything of an index except its lines: the sorted view's storage and the scratch word
+// everything of an index except its lines: the sorted view's storage, the scratch word and what add and the
+// ageing keep between kernels (13.5 bytes a slot; with the index, so that every call may be captured)
 int alloc_derived(hb_index_t* h) {
   const int64_t cap = h->cache_size;
+  const size_t bytes = (size_t)cap * 12 + (size_t)h->lines * 12 + 8 * sizeof(int32_t);
+  HB_CUDA(cudaMalloc(&h->batch_scratch, bytes));
+  HB_CUDA(cudaMemsetAsync(h->batch_scratch, 0, bytes, 0));
+  h->marks = static_cast<unsigned long long*>(h->batch_scratch);
+  h->heads = h->marks + cap;
+  h->after = reinterpret_cast<int32_t*>(h->heads + h->lines);
+  h->line_hits = h->after + cap;
+  h->batch = h->line_hits + h->lines;
+  device_error_word();  // (allocated on first use)
   HB_CUDA(cudaMalloc(&h->pairs, (cap + kLeafFan) * sizeof(longlong2)));
   HB_CUDA(cudaMalloc(&h->scratch_count, 4 * sizeof(int64_t)));
   // level capacities for a full index
@@ -561,6 +533,7 @@ int hb_index_open(const void* handle, hb_index_t** out) {
   h->lru = static_cast<int32_t*>(p);
   int rc = alloc_derived(h);
   if (rc != HB_OK) return rc;
+  HB_CUDA(cudaStreamSynchronize(0));
   *out = h;
   return HB_OK;
 }
@@ -577,11 +550,7 @@ int hb_index_destroy(hb_index_t* h) {
   cudaFree(h->pairs);
   cudaFree(h->level_store);
   cudaFree(h->scratch_count);
-  cudaFree(h->marks);
-  cudaFree(h->after);
-  cudaFree(h->line_hits);
-  cudaFree(h->heads);
-  cudaFree(h->batch);
+  cudaFree(h->batch_scratch);
   delete h;
   return HB_OK;
 }
@@ -623,18 +592,12 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   uint2* sorted = cv.take<uint2>(n);
   void* sort_ws = cv.take<char>(0);
   if (n > kAddSortMax && n <= kListedPerSet * h->lines) {
-    AddLists lists;
-    int rc = index_add_lists(h, next, &lists, st);
-    if (rc != HB_OK) return rc;
-    HB_LAUNCH(add_push_kernel, grid_for(n), kBlock, 0, st, ids, n, lists, locs, last_writer);
+    HB_LAUNCH(add_push_kernel, grid_for(n), kBlock, 0, st, ids, n, index_add_lists(h, next), locs, last_writer);
     AddEntries e;
     memset(&e, 0, sizeof(e));
     e.ids = ids;
     e.n = n;
-    AddState state;
-    rc = index_add_state(h, next, locs, last_writer, &state);
-    if (rc != HB_OK) return rc;
-    HB_LAUNCH(add_walk_kernel, grid_capped(n), kBlock, 0, st, e, state);
+    HB_LAUNCH(add_walk_kernel, grid_capped(n), kBlock, 0, st, e, index_add_state(h, next, locs, last_writer));
     return sort_run(SetSource<true>{ids, n, h->lines, h->heads, h->batch + 2},
                     AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, n, sort_ws, st);
   }
@@ -643,18 +606,6 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   const int rc = sort_run(SetSource<false>{ids, n, h->lines, nullptr, nullptr}, fin, n, sort_ws, st);
   if (rc != HB_OK || !fin.walk_later) return rc;
   HB_LAUNCH(add_sorted_walk_kernel, grid_for(n), kBlock, 0, st, ids, (int)n, fin);
-  return HB_OK;
-}
-
-static int touch_buffers(hb_index* h, TouchMarks* t, cudaStream_t st) {
-  const int rc = index_touch_marks(h, t, st);
-  if (rc != HB_OK) return rc;
-  if (!h->after) {
-    HB_CUDA(cudaMalloc(&h->line_hits, h->lines * sizeof(int32_t)));
-    HB_CUDA(cudaMemsetAsync(h->line_hits, 0, h->lines * sizeof(int32_t), st));
-    HB_CUDA(cudaMalloc(&h->after, h->cache_size * sizeof(int32_t)));
-    HB_CUDA(cudaMemsetAsync(h->after, 0, h->cache_size * sizeof(int32_t), st));
-  }
   return HB_OK;
 }
 
@@ -686,10 +637,8 @@ int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n, void*, siz
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_index_touch_lru: n out of range");
   if (n == 0) return HB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  TouchMarks t;
-  int rc = touch_buffers(h, &t, st);
-  if (rc != HB_OK) return rc;
-  rc = touch_mark(h, t, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, HostPart{0, nullptr, nullptr}, st);
+  const TouchMarks t = index_touch_marks(h);
+  const int rc = touch_mark(h, t, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, HostPart{0, nullptr, nullptr}, st);
   return rc != HB_OK ? rc : touch_finish(h, t, locs, n, st);
 }
 
@@ -706,20 +655,16 @@ int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int
   HB_CHECK_ARG(n >= 0 && first + n < ((int64_t)1 << 31), "hb_index_lookup_touch: n out of range");
   if (n == 0) return HB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc;
   if (mode == HB_LOOKUP_SORTED && h->sorted_stale) {
-    rc = hb_index_build_sorted(h, stream);
+    const int rc = hb_index_build_sorted(h, stream);
     if (rc != HB_OK) return rc;
   }
-  TouchMarks t;
-  rc = touch_buffers(h, &t, st);
-  if (rc != HB_OK) return rc;
-  return touch_mark(h, t, ids, locs + first, n, mode, HostPart{first, host_locs, arrived}, st);
+  return touch_mark(h, index_touch_marks(h), ids, locs + first, n, mode, HostPart{first, host_locs, arrived}, st);
 }
 
 int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream) {
-  HB_CHECK_ARG(h && h->after && locs && n > 0, "hb_index_lookup_touch: no part of the batch was looked up");
-  return touch_finish(h, TouchMarks{h->marks, h->batch, h->cache_size}, locs, n, (cudaStream_t)stream);
+  HB_CHECK_ARG(h && locs && n > 0, "hb_index_lookup_touch: no part of the batch was looked up");
+  return touch_finish(h, index_touch_marks(h), locs, n, (cudaStream_t)stream);
 }
 
 int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* perm,
@@ -732,11 +677,8 @@ int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* 
   HB_CHECK_ARG(locs_kind >= 0 && locs_kind <= 2, "hb_index_touch_lru_runs: locs_kind is 0, 1 or 2");
   if (n == 0 || max_runs == 0) return HB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  TouchMarks marks;
-  const int rc = index_touch_marks(h, &marks, st);
-  if (rc != HB_OK) return rc;
   RunsView v{locs, perm, run_start, num_runs, n_dev, max_runs, n, locs_kind};
-  HB_LAUNCH(touch_runs_mark_kernel, grid_for(max_runs), kBlock, 0, st, v, marks);
+  HB_LAUNCH(touch_runs_mark_kernel, grid_for(max_runs), kBlock, 0, st, v, index_touch_marks(h));
   return index_touch_apply(h, v, st);
 }
 

@@ -54,9 +54,10 @@ struct hb_index {
   int64_t level_off[hb::kMaxLevels];
   int64_t level_cap[hb::kMaxLevels];
   int64_t* scratch_count;      // device int64[4] for small reductions
-  // scratch of add and of the LRU ageing, allocated on first use; entries are valid when their
+  // scratch of add and of the LRU ageing, one allocation made with the index; entries are valid when their
   // batch number is that of the batch at work, so nothing is cleared between batches (32 bits:
   // 2^31 batches per index).  The batch numbers live on the device: a captured graph advances them.
+  void* batch_scratch;
   unsigned long long* marks;    // [capacity] (batch << 32) | 1 + last position / run that hit the slot
   int32_t* after;               // [capacity] hits on the line after the slot's last; zero between calls
   int32_t* line_hits;           // [lines] zero between calls
@@ -282,9 +283,9 @@ struct AddEntries {
   int64_t cap;
 };
 
-int index_touch_marks(hb_index* h, TouchMarks* out, cudaStream_t st);
+inline TouchMarks index_touch_marks(const hb_index* h) { return TouchMarks{h->marks, h->batch, h->cache_size}; }
 int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st);
-int index_add_lists(hb_index* h, uint32_t* next, AddLists* out, cudaStream_t st);
+inline AddLists index_add_lists(const hb_index* h, uint32_t* next) { return AddLists{h->heads, h->batch + 2, next, h->lines}; }
 // add() of the distinct ids of a batch that `listed` names: slots and "last writer of its slot" flags
 // for them; beyond the cap -1 / 0.  Where index_add_runs_lists says so through the lists of their sets
 // (AddLists, Maintain), else sorted by set.

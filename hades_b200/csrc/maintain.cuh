@@ -19,7 +19,9 @@ struct AddState {
   uint8_t* last_writer; // nullable [n]
 };
 
-int index_add_state(hb_index* h, uint32_t* next, int64_t* locs, uint8_t* last_writer, AddState* out);
+inline AddState index_add_state(const hb_index* h, uint32_t* next, int64_t* locs, uint8_t* last_writer) {
+  return AddState{h->heads, h->batch + 2, next, h->lines, h->line_ids, h->lru, locs, last_writer};
+}
 
 #ifdef __CUDACC__
 

@@ -436,12 +436,8 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
     rc = hb_index_build_sorted(h, stream);
     if (rc != HB_OK) return rc;
   }
-  TouchMarks marks;
-  rc = index_touch_marks(h, &marks, st);
-  if (rc != HB_OK) return rc;
-  AddLists lists;
-  rc = index_add_lists(h, static_cast<uint32_t*>(p.add_ws), &lists, st);
-  if (rc != HB_OK) return rc;
+  const TouchMarks marks = index_touch_marks(h);
+  const AddLists lists = index_add_lists(h, static_cast<uint32_t*>(p.add_ws));
   rc = build_runs(s, d, p, ids, n, counters, st);
   if (rc != HB_OK) return rc;
   // aside: all of the fetch leaves the caller's stream, which goes on to the aggregation of the
@@ -470,8 +466,7 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
     m.v = RunsView{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
     m.marks = marks;
     m.e = AddEntries{s->runs.uniq_ids, n, s->runs.num_runs, p.on_list, p.chunk_listed, p.listed, d->miss_cap};
-    rc = index_add_state(h, static_cast<uint32_t*>(p.add_ws), p.new_slots, p.last_writer, &m.add);
-    if (rc != HB_OK) return rc;
+    m.add = index_add_state(h, static_cast<uint32_t*>(p.add_ws), p.new_slots, p.last_writer);
     m.touch = d->touch_lru;
     m.insert = lists_used;
     m.blocks = grid_for_runs(n);
@@ -531,9 +526,7 @@ int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, 
     rc = hb_index_build_sorted(h, stream);
     if (rc != HB_OK) return rc;
   }
-  TouchMarks marks;
-  rc = index_touch_marks(h, &marks, st);
-  if (rc != HB_OK) return rc;
+  const TouchMarks marks = index_touch_marks(h);
   const SegPlan seg = seg_plan(p.seg_ws, n, d->dim);
   const ColdArgs c{d->staging, d->threshold_table, d->default_threshold, (unsigned long long*)d->dropped,
                    p.cold_slots, marks, d->touch_lru};

@@ -114,8 +114,8 @@ int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n,
                        void* workspace, size_t workspace_bytes, hb_stream_t stream);
 
 /* lookup(ids) with that side effect: what the reference's CPU lookup does
- * (src/cache/cache.h:213-222).  (This and hb_index_touch_lru allocate 20 bytes per slot inside the
- * index on first use; the workspace of the latter is not used any more.) */
+ * (src/cache/cache.h:213-222).  (The workspace of hb_index_touch_lru is not used any more: what the
+ * ageing keeps between its kernels, 13.5 bytes per slot with that of add, belongs to the index.) */
 int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int mode,
                           hb_stream_t stream);
 /* The same in parts, so that a caller with ids in host memory can copy one part while another is looked
@@ -135,7 +135,7 @@ int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_
  * needs no second sort for the ageing.  perm NULL = identity; run_start NULL =
  * every position is its own run (a batch of unique ids); num_runs / n_dev:
  * nullable device counts capping max_runs / n.  locs_kind: locs holds a slot per batch
- * position (0), per sorted entry (1) or per run (2: the run_slots of hb_lookup_fetch_runs).  The first call allocates 8 bytes per slot inside the index. */
+ * position (0), per sorted entry (1) or per run (2: the run_slots of hb_lookup_fetch_runs). */
 int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* perm,
                             const int64_t* run_start, int64_t max_runs,
                             const int64_t* num_runs, int64_t n, const int64_t* n_dev,

@@ -219,3 +219,41 @@ def test_host_lookups_in_parts(cuda_lib, oracle_mod, n, mode):
         oi, ol = ora.export()
         _eq(ids.cpu().numpy(), oi, ("line ids", rnd))
         _eq(lru.cpu().numpy(), ol, ("lru", rnd))
+
+
+@pytest.mark.parametrize("what,n", [("add", 20_000), ("add", 70_000), ("touch", 20_000), ("lookup", 20_000)])
+def test_first_call_may_be_captured(cuda_lib, oracle_mod, what, n):
+    """A call on a fresh index inside a stream capture: nothing is allocated on first use."""
+    from hades_b200 import EmbCacheLib as E
+    from hades_b200 import _lib
+
+    rng = np.random.default_rng(2)
+    ids = rng.integers(0, 30_000, n, dtype=np.int64)
+    ix = E.IndexCache(10_000, f"first_{what}{n}", True, False)
+    ora = oracle_mod.OracleIndex(10_000)
+    d = torch.from_numpy(ids).cuda()
+    if what != "add":
+        ora.add(ids[:5000])  # filled without a call that ages or adds
+        ix.import_state(*(torch.from_numpy(x) for x in ora.export()))
+    lib, st = _lib.load(), torch.cuda.Stream()
+    locs = torch.empty_like(d)
+    ws = torch.empty(lib.hb_index_add_workspace_bytes(n), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        s = _lib.stream_ptr()
+        if what == "add":
+            _lib.check(lib.hb_index_add(ix.handle, d.data_ptr(), n, locs.data_ptr(), None, ws.data_ptr(), ws.numel(), s))
+        elif what == "touch":
+            _lib.check(lib.hb_index_lookup(ix.handle, d.data_ptr(), n, locs.data_ptr(), None, 0, s))
+            _lib.check(lib.hb_index_touch_lru(ix.handle, locs.data_ptr(), n, ws.data_ptr(), ws.numel(), s))
+        else:
+            _lib.check(lib.hb_index_lookup_touch(ix.handle, d.data_ptr(), n, locs.data_ptr(), 0, s))
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        want = ora.add(ids) if what == "add" else ora.lookup(ids, touch=True)
+        assert np.array_equal(locs.cpu().numpy(), want)
+    gi, gl = ix.export_state()
+    oi, ol = ora.export()
+    assert np.array_equal(gi.cpu().numpy(), oi) and np.array_equal(gl.cpu().numpy(), ol)
