@@ -101,6 +101,7 @@ class IndexCache:
         self._name = name
         self.lookup_mode = lookup_mode
         self._shm_file = None
+        self._opened_flag = None  # a byte that another process sets when it opens this index
         if create:
             h = C.c_void_p()
             _lib.check(self._lib.hb_index_create(int(cache_size), C.byref(h)))
@@ -116,32 +117,40 @@ class IndexCache:
             self._owner = False
             self._device = other._device
             self._changing = other._changing
+            self._opened_flag = other._opened_flag
         else:
             # another process of this box created it: map its lines (src/cache/cache.h:155-158)
             path = _index_handle_path(name)
             try:
-                with open(path, "rb") as f:
+                with open(path, "r+b") as f:
                     blob = f.read()
+                    _check(len(blob) == self._lib.hb_index_handle_bytes() + 1, "index handle file has the expected size")
+                    # before the open: it waits for the calls that have not seen the flag
+                    f.seek(len(blob) - 1)
+                    f.write(b"\1")
             except OSError as e:
                 raise RuntimeError(f"fail to open {name}: no such index on this box ({e.strerror})") from e
-            _check(len(blob) == self._lib.hb_index_handle_bytes(), "index handle file has the expected size")
             h = C.c_void_p()
-            _lib.check(self._lib.hb_index_open(blob, C.byref(h)))
+            _lib.check(self._lib.hb_index_open(blob[:-1], C.byref(h)))
+            self._opened_flag = C.c_char(b"\1")
             self._h = h
             self._owner = True  # of the mapping: destroyed (closed) with this object
             self._device = torch.cuda.current_device()
             self._changing = threading.Lock()
 
     def _publish(self) -> None:
-        """Leave the IPC handle where other processes of the box find it by name."""
+        """Leave the IPC handle, and behind it the flag of an opener, where other processes of the box find it by name."""
+        import mmap
         import os
 
         buf = C.create_string_buffer(self._lib.hb_index_handle_bytes())
         try:
             _lib.check(self._lib.hb_index_export_handle(self._h, buf))
             path = _index_handle_path(self._name)
-            with open(path + ".tmp", "wb") as f:
-                f.write(buf.raw)
+            with open(path + ".tmp", "w+b") as f:
+                f.write(buf.raw + b"\0")
+                f.flush()
+                self._opened_flag = C.c_char.from_buffer(mmap.mmap(f.fileno(), len(buf.raw) + 1), len(buf.raw))
             os.replace(path + ".tmp", path)
             self._shm_file = path
             _PUBLISHED.add(path)
@@ -206,8 +215,9 @@ class IndexCache:
         if not ids.is_cuda and 0 < ids.numel() <= _STAGED:
             _check(ids.dtype == torch.int64, "ids.dtype == int64")
             with self._changing:  # the batch goes to the index in parts
+                flag = self._opened_flag
                 return (_lib._NATIVE or _lib.native()).index_lookup(getattr(self._h, "value", 0), ids, self._device,
-                                                                     self.lookup_mode)
+                                                                     self.lookup_mode, 0 if flag is None else C.addressof(flag))
         dev = self._to_dev(ids)
         locs = torch.empty_like(dev)
         with self._changing:

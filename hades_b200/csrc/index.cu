@@ -243,13 +243,14 @@ __global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const i
   }
 }
 
-__global__ void __launch_bounds__(kBlock) touch_after_kernel(const int64_t* __restrict__ locs, int64_t n, TouchMarks t,
-                                                             int32_t* __restrict__ after) {
+// (positions first .. n of the batch)
+__global__ void __launch_bounds__(kBlock) touch_after_kernel(const int64_t* __restrict__ locs, int64_t first, int64_t n,
+                                                             TouchMarks t, int32_t* __restrict__ after) {
   const uint32_t number = batch_number(t.batch);
   const int lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = warp * 32; base < n; base += nwarps * 32) {
+  for (int64_t base = first + warp * 32; base < n; base += nwarps * 32) {
     const int64_t i = base + lane;
     int64_t slot = i < n ? locs[i] : -1;
     if (slot >= t.capacity) slot = -1;
@@ -268,11 +269,11 @@ __global__ void __launch_bounds__(kBlock) touch_after_kernel(const int64_t* __re
   }
 }
 
-__global__ void __launch_bounds__(kBlock) touch_apply_kernel(const int64_t* __restrict__ locs, int64_t n, TouchMarks t,
-                                                             int32_t* __restrict__ after, int32_t* __restrict__ line_hits,
-                                                             int32_t* __restrict__ lru) {
+__global__ void __launch_bounds__(kBlock) touch_apply_kernel(const int64_t* __restrict__ locs, int64_t first, int64_t n,
+                                                             TouchMarks t, int32_t* __restrict__ after,
+                                                             int32_t* __restrict__ line_hits, int32_t* __restrict__ lru) {
   const uint32_t number = batch_number(t.batch);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = first + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t slot = locs[i];
     if (slot < 0 || slot >= t.capacity) continue;
     const int64_t line = slot >> 3;
@@ -394,6 +395,59 @@ int grid_capped(int64_t n, int block = kBlock) {
 
 }  // namespace
 
+// the rest of the ageing by the marked positions first .. n
+static int age_marked(hb_index* h, const int64_t* locs, int64_t first, int64_t n, cudaStream_t st) {
+  const int grid = grid_capped(n - first);
+  const TouchMarks t = index_touch_marks(h);
+  HB_LAUNCH(touch_after_kernel, grid, kBlock, 0, st, locs, first, n, t, h->after);
+  HB_LAUNCH(touch_apply_kernel, grid, kBlock, 0, st, locs, first, n, t, h->after, h->line_hits, h->lru);
+  return HB_OK;
+}
+
+// (a number of its own for every stream there ever was: handles come back)
+static bool eager_stream(cudaStream_t st, unsigned long long* id) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone &&
+      cudaStreamGetId(st, id) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
+}
+
+int IndexTurn::on(cudaStream_t st, bool goes_on) {
+  st_ = st;
+  used_ = eager_stream(st, &id_);
+  if (!used_) return HB_OK;
+  if (h_->was_changed && id_ != h_->changed_on) {
+    if (h_->unrecorded) {
+      int dev = h_->device;
+      HB_CUDA(cudaGetDevice(&dev));
+      if (dev != h_->device) HB_CUDA(cudaSetDevice(h_->device));
+      const cudaError_t e = cudaEventRecord(h_->changed, cudaStreamLegacy);
+      if (dev != h_->device) HB_CUDA(cudaSetDevice(dev));
+      HB_CUDA(e);
+      h_->unrecorded = false;
+    }
+    HB_CUDA(cudaStreamWaitEvent(st, h_->changed, 0));
+  }
+  if (goes_on || h_->open_first == h_->open_end) return HB_OK;
+  const int64_t first = h_->open_first;
+  h_->open_first = h_->open_end;
+  return age_marked(h_, h_->open_locs, first, h_->open_end, st);
+}
+
+IndexTurn::~IndexTurn() {
+  if (!used_) return;
+  // (an event costs the call a microsecond or two)
+  h_->unrecorded = st_ == nullptr || st_ == cudaStreamLegacy;
+  if (!h_->unrecorded && cudaEventRecord(h_->changed, st_) != cudaSuccess) {
+    cudaGetLastError();  // (the launches of the call have failed too)
+    return;
+  }
+  h_->changed_on = id_;
+  h_->was_changed = true;
+}
+
 int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st) {
   HB_LAUNCH(touch_runs_apply_kernel, grid_capped(v.max_runs), kBlock, 0, st, v, index_touch_marks(h), h->lru);
   return HB_OK;
@@ -444,6 +498,9 @@ int alloc_derived(hb_index_t* h) {
   h->line_hits = h->after + cap;
   h->batch = h->line_hits + h->lines;
   device_error_word();  // (allocated on first use)
+  HB_CUDA(cudaEventCreateWithFlags(&h->changed, cudaEventDisableTiming));
+  // (exported with the lines: a process that opens them begins behind the lookups before)
+  if (!h->opened) HB_CUDA(cudaEventCreateWithFlags(&h->aged, cudaEventDisableTiming | cudaEventInterprocess));
   HB_CUDA(cudaMalloc(&h->pairs, (cap + kLeafFan) * sizeof(longlong2)));
   HB_CUDA(cudaMalloc(&h->scratch_count, 4 * sizeof(int64_t)));
   // level capacities for a full index
@@ -469,6 +526,7 @@ struct IndexIpcHandle {
   int64_t lines;
   cudaIpcMemHandle_t line_ids;
   cudaIpcMemHandle_t lru;
+  cudaIpcEventHandle_t aged;
 };
 }  // namespace
 
@@ -477,8 +535,7 @@ int hb_index_create(int64_t cache_size, hb_index_t** out) {
   HB_CHECK_ARG(cache_size > 0, "hb_index_create: cache_size must be positive");
   const int64_t lines = ceil_div(cache_size, kWays);
   HB_CHECK_ARG(lines <= ((int64_t)1 << 28), "hb_index_create: at most 2^31 slots are supported");
-  hb_index_t* h = new hb_index_t();
-  memset(h, 0, sizeof(*h));
+  hb_index_t* h = new hb_index_t();  // (all members zero)
   HB_CUDA(cudaGetDevice(&h->device));
   h->lines = lines;
   h->cache_size = lines * kWays;
@@ -510,6 +567,7 @@ int hb_index_export_handle(hb_index_t* h, void* handle_out) {
   x.lines = h->lines;
   HB_CUDA(cudaIpcGetMemHandle(&x.line_ids, h->line_ids));
   HB_CUDA(cudaIpcGetMemHandle(&x.lru, h->lru));
+  HB_CUDA(cudaIpcGetEventHandle(&x.aged, h->aged));
   memcpy(handle_out, &x, sizeof(x));
   return HB_OK;
 }
@@ -519,8 +577,7 @@ int hb_index_open(const void* handle, hb_index_t** out) {
   IndexIpcHandle x;
   memcpy(&x, handle, sizeof(x));
   HB_CHECK_ARG(x.lines > 0 && x.cache_size == x.lines * kWays, "hb_index_open: not an index handle");
-  hb_index_t* h = new hb_index_t();
-  memset(h, 0, sizeof(*h));
+  hb_index_t* h = new hb_index_t();  // (all members zero)
   HB_CUDA(cudaGetDevice(&h->device));
   h->lines = x.lines;
   h->cache_size = x.cache_size;
@@ -534,6 +591,10 @@ int hb_index_open(const void* handle, hb_index_t** out) {
   int rc = alloc_derived(h);
   if (rc != HB_OK) return rc;
   HB_CUDA(cudaStreamSynchronize(0));
+  cudaEvent_t creators;
+  HB_CUDA(cudaIpcOpenEventHandle(&creators, x.aged));
+  HB_CUDA(cudaEventSynchronize(creators));
+  HB_CUDA(cudaEventDestroy(creators));
   *out = h;
   return HB_OK;
 }
@@ -551,6 +612,8 @@ int hb_index_destroy(hb_index_t* h) {
   cudaFree(h->level_store);
   cudaFree(h->scratch_count);
   cudaFree(h->batch_scratch);
+  if (h->changed) cudaEventDestroy(h->changed);
+  if (h->aged) cudaEventDestroy(h->aged);
   delete h;
   return HB_OK;
 }
@@ -586,6 +649,9 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
     return HB_ERR_WORKSPACE;
   }
   cudaStream_t st = (cudaStream_t)stream;
+  IndexTurn turn(h);
+  int rc = turn.on(st);
+  if (rc != HB_OK) return rc;
   Carver cv(workspace);
   h->sorted_stale = true;
   uint32_t* next = cv.take<uint32_t>(n);
@@ -603,16 +669,21 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   }
   // (a cluster that holds more than one entry per thread leaves the walk to the whole GPU)
   AddFinish fin{h->line_ids, h->lru, locs, last_writer, sorted, n > kAddSortMax && n <= kSortClusterMax};
-  const int rc = sort_run(SetSource<false>{ids, n, h->lines, nullptr, nullptr}, fin, n, sort_ws, st);
+  rc = sort_run(SetSource<false>{ids, n, h->lines, nullptr, nullptr}, fin, n, sort_ws, st);
   if (rc != HB_OK || !fin.walk_later) return rc;
   HB_LAUNCH(add_sorted_walk_kernel, grid_for(n), kBlock, 0, st, ids, (int)n, fin);
   return HB_OK;
 }
 
 // lookup of `ids` into locs (or the slots there, ids null), first pass of the ageing
-static int touch_mark(hb_index* h, const TouchMarks& t, const int64_t* ids, int64_t* locs, int64_t n, int mode,
-                      const HostPart& part, cudaStream_t st) {
+static int touch_mark(hb_index* h, const int64_t* ids, int64_t* locs, int64_t n, int mode, const HostPart& part,
+                      cudaStream_t st) {
+  if (ids && mode == HB_LOOKUP_SORTED && h->sorted_stale) {
+    const int rc = hb_index_build_sorted(h, st);
+    if (rc != HB_OK) return rc;
+  }
   const int grid = grid_capped(n);
+  const TouchMarks t = index_touch_marks(h);
   if (!ids)
     HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
               part);
@@ -625,46 +696,66 @@ static int touch_mark(hb_index* h, const TouchMarks& t, const int64_t* ids, int6
   return HB_OK;
 }
 
-static int touch_finish(hb_index* h, const TouchMarks& t, const int64_t* locs, int64_t n, cudaStream_t st) {
-  const int grid = grid_capped(n);
-  HB_LAUNCH(touch_after_kernel, grid, kBlock, 0, st, locs, n, t, h->after);
-  HB_LAUNCH(touch_apply_kernel, grid, kBlock, 0, st, locs, n, t, h->after, h->line_hits, h->lru);
-  return HB_OK;
-}
-
 int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n, void*, size_t, hb_stream_t stream) {
   HB_CHECK_ARG(h && (n == 0 || locs), "hb_index_touch_lru: null argument");
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_index_touch_lru: n out of range");
   if (n == 0) return HB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const TouchMarks t = index_touch_marks(h);
-  const int rc = touch_mark(h, t, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, HostPart{0, nullptr, nullptr}, st);
-  return rc != HB_OK ? rc : touch_finish(h, t, locs, n, st);
+  IndexTurn turn(h);
+  int rc = turn.on(st);
+  if (rc == HB_OK)
+    rc = touch_mark(h, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, HostPart{0, nullptr, nullptr}, st);
+  return rc != HB_OK ? rc : age_marked(h, locs, 0, n, st);
+}
+
+static int check_lookup(hb_index_t* h, const int64_t* ids, int64_t n, const int64_t* locs, int64_t first, int mode) {
+  HB_CHECK_ARG(h && first >= 0 && (n == 0 || (ids && locs)), "hb_index_lookup_touch: null argument");
+  HB_CHECK_ARG(mode == HB_LOOKUP_SETASSOC || mode == HB_LOOKUP_SORTED, "hb_index_lookup_touch: unknown mode %d", mode);
+  HB_CHECK_ARG(n >= 0 && first + n < ((int64_t)1 << 31), "hb_index_lookup_touch: n out of range");
+  return HB_OK;
 }
 
 int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int mode,
                           hb_stream_t stream) {
-  int rc = hb_index_lookup_touch_part(h, ids, n, locs, 0, nullptr, nullptr, mode, stream);
-  return rc != HB_OK || n == 0 ? rc : hb_index_lookup_touch_end(h, locs, n, stream);
+  int rc = check_lookup(h, ids, n, locs, 0, mode);
+  if (rc != HB_OK || n == 0) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  IndexTurn turn(h);
+  rc = turn.on(st);
+  if (rc == HB_OK) rc = touch_mark(h, ids, locs, n, mode, HostPart{0, nullptr, nullptr}, st);
+  return rc != HB_OK ? rc : age_marked(h, locs, 0, n, st);
 }
 
 int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
                                int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream) {
-  HB_CHECK_ARG(h && first >= 0 && (n == 0 || (ids && locs)), "hb_index_lookup_touch: null argument");
-  HB_CHECK_ARG(mode == HB_LOOKUP_SETASSOC || mode == HB_LOOKUP_SORTED, "hb_index_lookup_touch: unknown mode %d", mode);
-  HB_CHECK_ARG(n >= 0 && first + n < ((int64_t)1 << 31), "hb_index_lookup_touch: n out of range");
-  if (n == 0) return HB_OK;
+  int rc = check_lookup(h, ids, n, locs, first, mode);
+  if (rc != HB_OK || n == 0) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  if (mode == HB_LOOKUP_SORTED && h->sorted_stale) {
-    const int rc = hb_index_build_sorted(h, stream);
-    if (rc != HB_OK) return rc;
-  }
-  return touch_mark(h, index_touch_marks(h), ids, locs + first, n, mode, HostPart{first, host_locs, arrived}, st);
+  IndexTurn turn(h);
+  const bool next = h->open_locs == locs && h->open_end == first && h->open_first < first;
+  rc = turn.on(st, next);
+  if (rc == HB_OK) rc = touch_mark(h, ids, locs + first, n, mode, HostPart{first, host_locs, arrived}, st);
+  if (rc != HB_OK) return rc;
+  h->open_locs = locs;
+  if (!next) h->open_first = first;
+  h->open_end = first + n;
+  return HB_OK;
 }
 
 int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream) {
   HB_CHECK_ARG(h && locs && n > 0, "hb_index_lookup_touch: no part of the batch was looked up");
-  return touch_finish(h, index_touch_marks(h), locs, n, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  IndexTurn turn(h);
+  int rc = turn.on(st, true);  // (also behind a call that has found the parts and aged by them: locs may be freed)
+  if (rc != HB_OK) return rc;
+  const int64_t first = h->open_first;
+  if (h->open_locs == locs && h->open_end == n && first < n) {
+    h->open_first = n;
+    rc = age_marked(h, locs, first, n, st);
+    if (rc != HB_OK) return rc;
+  }
+  if (h->aged) HB_CUDA(cudaEventRecord(h->aged, st));
+  return HB_OK;
 }
 
 int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* perm,
@@ -677,6 +768,9 @@ int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* 
   HB_CHECK_ARG(locs_kind >= 0 && locs_kind <= 2, "hb_index_touch_lru_runs: locs_kind is 0, 1 or 2");
   if (n == 0 || max_runs == 0) return HB_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  IndexTurn turn(h);
+  const int rc = turn.on(st);
+  if (rc != HB_OK) return rc;
   RunsView v{locs, perm, run_start, num_runs, n_dev, max_runs, n, locs_kind};
   HB_LAUNCH(touch_runs_mark_kernel, grid_for(max_runs), kBlock, 0, st, v, index_touch_marks(h));
   return index_touch_apply(h, v, st);
@@ -706,8 +800,11 @@ int hb_index_lookup(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
 int hb_index_reset(hb_index_t* h, const int64_t* ids, int64_t n, hb_stream_t stream) {
   HB_CHECK_ARG(h && (n == 0 || ids), "hb_index_reset: null argument");
   if (n <= 0) return HB_OK;
-  HB_LAUNCH(reset_kernel, grid_for(n), kBlock, 0, (cudaStream_t)stream, ids, n, h->lines,
-            h->line_ids, h->lru);
+  cudaStream_t st = (cudaStream_t)stream;
+  IndexTurn turn(h);
+  const int rc = turn.on(st);
+  if (rc != HB_OK) return rc;
+  HB_LAUNCH(reset_kernel, grid_for(n), kBlock, 0, st, ids, n, h->lines, h->line_ids, h->lru);
   h->sorted_stale = true;
   return HB_OK;
 }
@@ -840,6 +937,9 @@ int hb_index_build_sorted(hb_index_t* h, hb_stream_t stream) {
 int hb_index_export(hb_index_t* h, int64_t* line_ids, int32_t* lru, hb_stream_t stream) {
   HB_CHECK_ARG(h, "hb_index_export: null index");
   cudaStream_t st = (cudaStream_t)stream;
+  IndexTurn turn(h);
+  const int rc = turn.on(st);
+  if (rc != HB_OK) return rc;
   if (line_ids)
     HB_CUDA(cudaMemcpyAsync(line_ids, h->line_ids, h->cache_size * sizeof(int64_t),
                             cudaMemcpyDefault, st));
@@ -853,6 +953,9 @@ int hb_index_import(hb_index_t* h, const int64_t* line_ids, const int32_t* lru,
                     hb_stream_t stream) {
   HB_CHECK_ARG(h, "hb_index_import: null index");
   cudaStream_t st = (cudaStream_t)stream;
+  IndexTurn turn(h);
+  const int rc = turn.on(st);
+  if (rc != HB_OK) return rc;
   if (line_ids)
     HB_CUDA(cudaMemcpyAsync(h->line_ids, line_ids, h->cache_size * sizeof(int64_t),
                             cudaMemcpyDefault, st));

@@ -13,6 +13,8 @@
 //                      (<= kTopMax ids) is staged in shared memory by each CTA.
 #pragma once
 
+#include <mutex>
+
 #include "common.cuh"
 
 #ifdef __CUDACC__
@@ -70,6 +72,16 @@ struct hb_index {
   // calls hb_index_build_sorted.)
   bool shared;
   bool opened;  // line_ids / lru are mappings of another process's memory
+  // Calls that change lines or counters take turns (IndexTurn): they share the scratch above.
+  std::mutex turn;
+  cudaEvent_t changed;            // behind the last such call
+  unsigned long long changed_on;  // the id of its stream
+  bool was_changed;
+  bool unrecorded;                // ... on the default stream, which stays: recorded when another one has to wait
+  cudaEvent_t aged;               // interprocess: behind the last lookup of host ids
+  // a batch of host ids of which some parts are looked up: positions that wait for their ageing
+  const int64_t* open_locs;
+  int64_t open_first, open_end;
 };
 
 #ifdef __CUDACC__
@@ -281,6 +293,26 @@ struct AddEntries {
   const int32_t* chunk_listed;   // nullable: listed entries of 32 at a time
   const unsigned long long* total;  // their number
   int64_t cap;
+};
+
+// The turn of a call that changes an index: from one thread at a time (the kernels of a call are enqueued
+// together), and behind the last such call where that one went to another stream.  Streams inside a capture are
+// ordered by whoever replays the graph.
+class IndexTurn {
+ public:
+  explicit IndexTurn(hb_index* h) : h_(h), lock_(h->turn) {}
+  ~IndexTurn();
+  // The stream of the launches to come, before the first of them.  A batch that another thread looks up in
+  // parts is aged by its parts so far (one hit after the other: cut in two it ages the same), unless this call
+  // is its next.
+  int on(cudaStream_t st, bool goes_on = false);
+
+ private:
+  hb_index* h_;
+  std::lock_guard<std::mutex> lock_;
+  cudaStream_t st_ = nullptr;
+  unsigned long long id_ = 0;
+  bool used_ = false;
 };
 
 inline TouchMarks index_touch_marks(const hb_index* h) { return TouchMarks{h->marks, h->batch, h->cache_size}; }

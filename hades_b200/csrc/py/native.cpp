@@ -210,17 +210,34 @@ PyObject* unique_update(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   });
 }
 
+// Kernels of a call read and write pinned buffers of that call: one that fails half way waits for them, and
+// leaves no batch open.
+struct InFlight {
+  cudaStream_t stream;
+  hb_index_t* index = nullptr;
+  const int64_t* locs = nullptr;
+  int64_t looked_up = 0;
+  bool ended = false;
+  ~InFlight() {
+    if (ended) return;
+    if (looked_up) hb_index_lookup_touch_end(index, locs, looked_up, stream);
+    cudaStreamSynchronize(stream);
+  }
+};
+
 at::Tensor pinned_empty(int64_t n) {
   return at::empty({n}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
 }
 
-// index_lookup(index, ids in host memory, device, mode) -> slots in host memory.  Ids and slots pass
-// through two pinned buffers each, a part of the batch at a time: while the GPU looks one part up the host
-// copies the next in and the one before out, and the ageing runs under the last copies.  500 ids: 26 us (two
-// pageable copies: 70), 65,536: 99 (183).
+// index_lookup(index, ids in host memory, device, mode, address of the flag of other processes | 0) -> slots in
+// host memory.  Ids and slots pass through two pinned buffers each, a part of the batch at a time: while the GPU
+// looks one part up the host copies the next in and the one before out, and the ageing runs under the last copies
+// and after.  Calls on the index from other streams wait for it; where another process has the lines too, which
+// can only be ordered by the host, the call does.  (The flag is read last: a process that sets it later waits for
+// the event of the lookups.)  500 ids: 26 us (two pageable copies: 70), 65,536: 99 (183).
 PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
-    arity(n_args, 4, "index_lookup");
+    arity(n_args, 5, "index_lookup");
     hb_index_t* h = static_cast<hb_index_t*>(pointer(a[0]));
     const at::Tensor ids = tensor(a[1], "ids").contiguous();
     const at::Device dev(at::kCUDA, (c10::DeviceIndex)integer(a[2]));
@@ -238,6 +255,7 @@ PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const int64_t* src = ids.data_ptr<int64_t>();
     int64_t *to = out.data_ptr<int64_t>(), *pin = in.data_ptr<int64_t>(), *pback = back.data_ptr<int64_t>();
     volatile int64_t* words = t_word.arm();
+    InFlight in_flight{st, h, locs.data_ptr<int64_t>()};
     auto length = [&](int64_t k) { return (k + 1) * part < n ? part : n - k * part; };
     auto collect = [&](int64_t k) {
       t_word.wait(st, (int)(k & 1));
@@ -249,9 +267,20 @@ PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       memcpy(pin + (k & 1) * part, src + k * part, length(k) * sizeof(int64_t));
       check(hb_index_lookup_touch_part(h, pin + (k & 1) * part, length(k), locs.data_ptr<int64_t>(), k * part,
                                        pback + (k & 1) * part, const_cast<int64_t*>(words + (k & 1)), mode, st));
+      in_flight.looked_up = k * part + length(k);
     }
     check(hb_index_lookup_touch_end(h, locs.data_ptr<int64_t>(), n, st));
+    in_flight.looked_up = 0;
     for (int64_t k = parts < 2 ? 0 : parts - 2; k < parts; ++k) collect(k);
+    const volatile char* opened = static_cast<const volatile char*>(pointer(a[4]));
+    if (opened && *opened) {
+      cudaError_t e;
+      Py_BEGIN_ALLOW_THREADS;
+      e = cudaStreamSynchronize(st);
+      Py_END_ALLOW_THREADS;
+      if (e != cudaSuccess) throw std::runtime_error(cudaGetErrorString(e));
+    }
+    in_flight.ended = true;  // (what still runs uses device memory only)
     return THPVariable_Wrap(out);
   });
 }
@@ -276,6 +305,7 @@ PyObject* index_add(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const size_t need = hb_index_add_workspace_bytes(n);
     const at::Tensor ws = cuda_empty({(int64_t)need}, at::kByte, dev);
     memcpy(in.data_ptr(), ids.data_ptr(), bytes);
+    InFlight in_flight{st};
     if (cudaMemcpyAsync(dids.data_ptr(), in.data_ptr(), bytes, cudaMemcpyHostToDevice, st) != cudaSuccess)
       throw std::runtime_error("copy of the ids to the device failed");
     check(hb_index_add(h, dids.data_ptr<int64_t>(), n, locs.data_ptr<int64_t>(), nullptr, ws.data_ptr(), need, st));
@@ -285,6 +315,7 @@ PyObject* index_add(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     Py_END_ALLOW_THREADS;
     if (e != cudaSuccess) throw std::runtime_error(cudaGetErrorString(e));
+    in_flight.ended = true;
     memcpy(out.data_ptr(), back.data_ptr(), bytes);
     return THPVariable_Wrap(out);
   });

@@ -291,7 +291,10 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
   const RunsView touched{c.slots, nullptr, nullptr, r.num_runs, r.num_runs, r.n, r.n, 2};
   const IndexView& v = d->index->view;
   const bool sorted = d->lookup_mode == HB_LOOKUP_SORTED;
+  IndexTurn turn(d->index);
   if (fused) {
+    int rc = turn.on(st);
+    if (rc != HB_OK) return rc;
     int64_t blocks = ceil_div(r.n, kBlock);
     if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
     if (sorted)
@@ -314,6 +317,7 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
   if (rc != HB_OK) return rc;
   // from here on the fetch of this batch must have read its rows and the cache hold its misses
   rc = join_side(s, st);
+  if (rc == HB_OK) rc = turn.on(st);
   if (rc != HB_OK) return rc;
   if (sorted)
     rc = vec4 ? launch_apply<HB_LOOKUP_SORTED, ADAM, 4>(v, r, c, a, epi, sums, st)
@@ -448,6 +452,9 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
     HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
     st = s->side;
   }
+  IndexTurn turn(h);
+  rc = turn.on(st);
+  if (rc != HB_OK) return rc;
   const ResolveArgs a{(const char*)d->cache_rows, (const char*)d->table, d->table_rows, d->row_bytes,
                       static_cast<unsigned long long*>(p.fetch_ws), p.run_slots,
                       d->insert_misses ? p.on_list : nullptr, p.last_writer, p.chunk_listed, p.listed,

@@ -50,6 +50,8 @@ int hb_device_status(int* status_host, hb_stream_t stream);
 /* Replaces SACacheIndex / IndexCache (src/cache/cache.h:11-257,               */
 /* src/cache/cache_line.h:7-103, bound in src/pybind.cc:17-33).                */
 /* slot = (id % lines) * 8 + way; -1 = absent.  ids must be >= 0.              */
+/* Calls that change an index (add, reset, the ageing, the steps) may come from several threads and on several
+ * streams: each waits for the one before it, except inside a stream capture.  Two processes order theirs. */
 /* ------------------------------------------------------------------------- */
 typedef struct hb_index hb_index_t;
 typedef struct hb_peer_table hb_peer_table_t; /* a table sharded over the GPUs of a box, see the end of this file */
@@ -120,9 +122,9 @@ int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t*
                           hb_stream_t stream);
 /* The same in parts, so that a caller with ids in host memory can copy one part while another is looked
  * up: positions first .. first + n of the batch (ids of the part: device or pinned; locs of the whole
- * batch: device), slots also to host_locs (nullable, pinned, of the part), then *arrived (nullable,
- * pinned) = 1.  After the last part hb_index_lookup_touch_end ages the counters by the whole batch; no
- * other call on the index may come between. */
+ * batch: device, allocated until the end), slots also to host_locs (nullable, pinned, of the part), then *arrived
+ * (nullable, pinned) = 1.  After the last part hb_index_lookup_touch_end ages the counters by the whole
+ * batch; the ageing may still run when the slots have arrived. */
 int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
                                int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream);
 int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream);

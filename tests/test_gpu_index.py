@@ -1,6 +1,8 @@
 """Cache index on the GPU (through the C ABI) against the oracle and the golden vectors:
 slots, found masks, valid counts, enumeration order and the complete state including the
 LRU counters must be bit-exact."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -257,3 +259,129 @@ def test_first_call_may_be_captured(cuda_lib, oracle_mod, what, n):
     gi, gl = ix.export_state()
     oi, ol = ora.export()
     assert np.array_equal(gi.cpu().numpy(), oi) and np.array_equal(gl.cpu().numpy(), ol)
+
+
+def _split_ids(rng, lines, n, low, ids_per_set=6):
+    """ids whose sets are [0, lines / 2) (low) or the rest"""
+    half = lines // 2
+    s = rng.integers(0, half, n) + (0 if low else half)
+    return (s + lines * rng.integers(0, ids_per_set, n)).astype(np.int64)
+
+
+def _load(stream, times=40):
+    """Kernels of many blocks, some 50 us each."""
+    x = torch.zeros(1 << 26, device="cuda")
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        for _ in range(times):
+            x += 1.0
+    x.record_stream(stream)
+
+
+def _same_state(ix, ora, where=None):
+    for got, want in zip(ix.export_state(), ora.export()):
+        assert np.array_equal(got.cpu().numpy(), want), where
+
+
+@pytest.mark.parametrize("n", [500, 60_000, 130_000])
+def test_what_follows_a_host_lookup_on_another_stream_finds_the_counters_aged(cuda_lib, oracle_mod, n):
+    from hades_b200 import EmbCacheLib as E
+
+    rng = np.random.default_rng(n)
+    ix = E.IndexCache(40_000, f"complete{n}", True, False)
+    ora = oracle_mod.OracleIndex(40_000)
+    # what is read goes ahead of the kernels that keep the GPU busy, the lookup's own wait behind them
+    streams, busy = [torch.cuda.Stream(), torch.cuda.Stream(priority=-1)], torch.cuda.Stream()
+    for rnd in range(12):
+        new = rng.integers(0, 120_000, 9_000, dtype=np.int64)
+        q = rng.integers(0, 120_000, n, dtype=np.int64)
+        dnew = torch.from_numpy(new).cuda()
+        torch.cuda.synchronize()
+        want = ora.lookup(q, touch=True)
+        _load(busy)
+        with torch.cuda.stream(streams[0]):
+            got = ix.lookup(torch.from_numpy(q))
+        with torch.cuda.stream(streams[1]):
+            _, lru = ix.export_state()
+            lru = lru.cpu()
+        assert np.array_equal(got.numpy(), want) and np.array_equal(lru.numpy(), ora.export()[1]), rnd
+        with torch.cuda.stream(streams[1]):
+            got = ix.cuda_add(dnew).cpu().numpy()
+        assert np.array_equal(got, ora.add(new)), rnd
+
+
+@pytest.mark.parametrize("first", ["default", "own"])
+@pytest.mark.parametrize("kind", ["touch", "lookup", "add"])
+def test_calls_from_two_streams(cuda_lib, oracle_mod, kind, first):
+    """Two streams, each with the ids of sets of its own: whichever runs first, the lines are the same."""
+    from hades_b200 import EmbCacheLib as E
+
+    rng = np.random.default_rng(7)
+    lines = 5000
+    ix = E.IndexCache(lines * 8, f"streams_{kind}_{first}", True, False)
+    ora = oracle_mod.OracleIndex(lines * 8)
+    start = np.concatenate([_split_ids(rng, lines, 30_000, low) for low in (True, False)])
+    assert np.array_equal(ix.add(torch.from_numpy(start)).numpy(), ora.add(start))
+    streams = [torch.cuda.default_stream() if first == "default" else torch.cuda.Stream(), torch.cuda.Stream()]
+    rounds = [[_split_ids(rng, lines, 6000 + 3000 * int(rng.integers(0, 40)), low, 12) for low in (True, False)] for _ in range(20)]
+    dev = [[torch.from_numpy(x).cuda() for x in r] for r in rounds]
+    locs = [[ix.cudalookup(x) for x in r] for r in dev]
+    torch.cuda.synchronize()
+    keep = []
+    _load(torch.cuda.Stream(), 200)
+    for r, l in zip(dev, locs):
+        for k in range(2):
+            with torch.cuda.stream(streams[k]):
+                if kind == "touch":
+                    ix.cuda_touch_lru(l[k])
+                elif kind == "lookup":
+                    keep.append(ix.lookup(r[k]))
+                else:
+                    keep.append(ix.cuda_add(r[k]))
+    torch.cuda.synchronize()
+    for r in rounds:
+        for x in r:
+            ora.add(x) if kind == "add" else ora.lookup(x, touch=True)
+    _same_state(ix, ora)
+
+
+@pytest.mark.parametrize("own", [False, True])
+def test_ageing_from_two_threads(cuda_lib, oracle_mod, own):
+    """Host lookups of several parts in one thread, ageing of slots in another, each of sets of its own, on one
+    stream or (own) two."""
+    from hades_b200 import EmbCacheLib as E
+
+    rng = np.random.default_rng(8)
+    lines = 5000
+    ix = E.IndexCache(lines * 8, f"two_threads_{own}", True, False)
+    ora = oracle_mod.OracleIndex(lines * 8)
+    first = np.concatenate([_split_ids(rng, lines, 30_000, low) for low in (True, False)])
+    ix.add(torch.from_numpy(first))
+    ora.add(first)
+    host = [_split_ids(rng, lines, 120_000, True, 12) for _ in range(10)]
+    uniq = [np.unique(_split_ids(rng, lines, 5000, False, 12)) for _ in range(200)]
+    slots = [ix.cudalookup(torch.from_numpy(u).cuda()) for u in uniq]
+    torch.cuda.synchronize()
+    failed, done, enough = [], [], threading.Event()
+    _load(torch.cuda.Stream(), 400)
+
+    def touches():
+        try:
+            with torch.cuda.stream(torch.cuda.Stream() if own else torch.cuda.default_stream()):
+                while not enough.is_set():
+                    ix.cuda_touch_lru_runs(slots[len(done) % len(slots)], None)
+                    done.append(1)
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    t = threading.Thread(target=touches)
+    t.start()
+    for q in host:
+        ix.lookup(torch.from_numpy(q))
+    enough.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    for q in host + [uniq[k % len(uniq)] for k in range(len(done))]:
+        ora.lookup(q, touch=True)
+    _same_state(ix, ora)

@@ -82,3 +82,57 @@ def test_open_without_creator_raises(cuda_lib):
 
     with pytest.raises(RuntimeError, match="fail to open"):
         E.IndexCache(100, "no_such_index_anywhere", False, False)
+
+
+def _complete_worker(rank, port, name):
+    """The creator looks up under load; the other process, ordered by barriers alone, reads the counters."""
+    sys.path.insert(0, str(ROOT))
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
+    import torch.distributed as dist
+
+    dist.init_process_group("gloo", rank=rank, world_size=2)
+    torch.cuda.set_device(0)
+    from hades_b200 import EmbCacheLib as E
+    from oracle import oracle as om
+
+    rng = np.random.default_rng(6)
+    ora = om.OracleIndex(10_000)
+    first = rng.integers(0, 50_000, 20_000, dtype=np.int64)
+    ora.add(first)
+    x = torch.zeros(1 << 26, device="cuda")
+    busy = torch.cuda.Stream()
+    if rank == 0:
+        ix = E.IndexCache(10_000, name, True, False)
+        ix.add(torch.from_numpy(first))
+    for rnd in range(6):
+        q = rng.integers(0, 50_000, 3000, dtype=np.int64)
+        want = ora.lookup(q, touch=True)
+        torch.cuda.synchronize()
+        if rank == 0:
+            with torch.cuda.stream(busy):
+                for _ in range(100):
+                    x += 1.0
+            assert np.array_equal(ix.lookup(torch.from_numpy(q)).numpy(), want)
+        dist.barrier()
+        if rank == 1:
+            if rnd == 0:
+                ix = E.IndexCache(10_000, name, False, False)
+            assert np.array_equal(ix.export_state()[1].cpu().numpy(), ora.export()[1]), rnd
+        dist.barrier()
+    if rank == 1:
+        ix.close()
+    dist.barrier()
+    if rank == 0:
+        ix.close()
+    dist.destroy_process_group()
+
+
+def test_lookup_of_a_shared_index_is_complete_when_it_returns():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import torch.multiprocessing as mp
+
+    from oracle import build_oracle
+
+    build_oracle.build_oracle()
+    mp.spawn(_complete_worker, args=(_free_port(), f"complete_ix_{os.getpid()}"), nprocs=2, join=True)
