@@ -51,6 +51,7 @@ def _compile(src: Path, force: bool) -> tuple[Path, str]:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"nvcc failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+    obj.with_suffix(".ptxas").write_text(r.stderr)  # registers and spills of every kernel
     return obj, r.stderr
 
 

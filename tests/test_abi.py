@@ -72,6 +72,23 @@ def test_step_refuses_what_the_updates_refuse(built_lib, kind, change, why):
     assert lib.hb_step_supported(ctypes.byref(d)) == 0 and why in lib.hb_last_error()
 
 
+@pytest.mark.parametrize("peer", [0, 1])
+@pytest.mark.parametrize("maintain", [0, 1])
+def test_expansion_of_full_lists_holds_its_rows_in_registers(built_lib, peer, maintain):
+    """runs_expand_kernel for rows of 512 bytes, 32 entries a warp: eight rows in flight and no spills."""
+    from hades_b200 import _build
+
+    log = _build.OBJ / "runs.ptxas"
+    if not log.exists():
+        pytest.skip("the objects were built elsewhere")
+    name = f"runs_expand_kernelILb{peer}ELi512ELb{maintain}ELb1E"
+    if peer and maintain:
+        assert name not in log.read_text()  # several GPUs: maintenance has launches of its own
+        return
+    entry = log.read_text().split(name, 1)[1].split("Compiling entry function", 1)[0]
+    assert " 0 bytes spill stores, 0 bytes spill loads" in entry, entry[:600]
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from hades_b200 import _lib
 
