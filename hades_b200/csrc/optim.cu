@@ -18,16 +18,6 @@ __device__ __forceinline__ int64_t effective_n(int64_t n, const int64_t* n_dev) 
   return d < n ? d : n;
 }
 
-__device__ __forceinline__ float adam_elem(float g, float& m, float& v, float bias1, float bias2,
-                                           const AdamParams& p) {
-  // update_mem = beta1*mem + (1-beta1)*grad; update_power = beta2*power + (1-beta2)*grad^2
-  m = p.beta1 * m + p.one_minus_beta1 * g;
-  v = p.beta2 * v + p.one_minus_beta2 * (g * g);
-  const float mc = m / bias1;
-  const float vc = v / bias2;
-  return p.lr * mc / (sqrtf(vc) + p.eps);  // std_values, sparse_optim.py:654-655
-}
-
 // A group of G lanes per row, kOptRows rows in flight per group (their loads are
 // issued together, then the arithmetic and the stores follow).
 constexpr int kOptRows = 2;

@@ -55,10 +55,22 @@ template <> struct EmbIO<__half> {
   static __device__ __forceinline__ void store(__half* p, float v) { *p = __float2half_rn(v); }
 };
 
-// One element.  Divisions by per-row scalars are multiplications by their reciprocals (ra, rb: 1 /
+// One element of rows that are not a multiple of four columns (bias1, bias2: the bias corrections), as the
+// reference divides; what the row loses.
+__device__ __forceinline__ float adam_elem(float g, float& m, float& v, float bias1, float bias2,
+                                           const AdamParams& p) {
+  // update_mem = beta1*mem + (1-beta1)*grad; update_power = beta2*power + (1-beta2)*grad^2
+  // (fused explicitly, here and below: every kernel that updates rows gives the same bits)
+  m = fmaf(p.beta1, m, p.one_minus_beta1 * g);
+  v = fmaf(p.beta2, v, p.one_minus_beta2 * (g * g));
+  const float mc = m / bias1;
+  const float vc = v / bias2;
+  return p.lr * mc / (sqrtf(vc) + p.eps);  // std_values, sparse_optim.py:654-655
+}
+
+// One element of vectors.  Divisions by per-row scalars are multiplications by their reciprocals (ra, rb: 1 /
 // bias correction); the element-wise division and the square root are IEEE.
 __device__ __forceinline__ void adam_value(float g, float& m, float& v, float& e, float ra, float rb, const AdamParams& p) {
-  // (fused explicitly: every kernel that updates rows gives the same bits)
   m = fmaf(p.beta1, m, p.one_minus_beta1 * g);
   v = fmaf(p.beta2, v, p.one_minus_beta2 * (g * g));
   e -= p.lr * (m * ra) / (sqrtf(v * rb) + p.eps);  // sparse_optim.py:654-655

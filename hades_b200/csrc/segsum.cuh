@@ -230,9 +230,11 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
   static constexpr int kMinBlocks = (VPL > 2 ? 512 : 768) / kBlock;
   static constexpr int kPieceMax = STEP ? 32 : 16;
   static constexpr bool kPrefetch = true;
+  // per-row scalars divide where the stand-alone kernels do (columns one by one), else their reciprocals multiply
+  static constexpr bool kDivide = VEC == 1;
   struct Lane {
     int row = -1;   // table row, or kStaged + staging slot
-    float t = 0.0f, ra = 1.0f, rb = 1.0f;
+    float t = 0.0f, ra = 1.0f, rb = 1.0f;  // the bias corrections or their reciprocals
   };
   struct Row {
     int row;
@@ -253,8 +255,12 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
       if (ADAM && l.row >= 0) {
         // state_step = state_step + 1 (per row), sparse_optim.py:624-626
         l.t = o.step[l.row] + 1.0f;
-        l.ra = 1.0f / (1.0f - powf(o.p.beta1, l.t));
-        l.rb = 1.0f / (1.0f - powf(o.p.beta2, l.t));
+        l.ra = 1.0f - powf(o.p.beta1, l.t);
+        l.rb = 1.0f - powf(o.p.beta2, l.t);
+        if (!kDivide) {
+          l.ra = 1.0f / l.ra;
+          l.rb = 1.0f / l.rb;
+        }
       }
     }
     return l;
@@ -324,15 +330,18 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
       return;
     }
     // one trainer: unique_grads of its own rows divides by 1 + their count
-    const float rc = STEP ? 1.0f / (float)(count + 1) : 1.0f;
+    const float c = STEP ? (float)(count + 1) : 1.0f, rc = kDivide ? 1.0f : 1.0f / c;
     if (ADAM && sub == 0) o.step[r.row] = r.t;
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
       if (sub + v * G >= vpr) continue;
 #pragma unroll
       for (int j = 0; j < VEC; ++j) {
-        const float g = STEP ? lane_of(acc[v], j) * rc : lane_of(acc[v], j);
-        if constexpr (ADAM) adam_value(g, lane_of(r.s0[v], j), lane_of(r.s1[v], j), lane_of(r.e[v], j), r.ra, r.rb, o.p);
+        const float sum = lane_of(acc[v], j);
+        const float g = !STEP ? sum : kDivide ? sum / c : sum * rc;
+        if constexpr (ADAM && kDivide)
+          lane_of(r.e[v], j) -= adam_elem(g, lane_of(r.s0[v], j), lane_of(r.s1[v], j), r.ra, r.rb, o.p);
+        else if constexpr (ADAM) adam_value(g, lane_of(r.s0[v], j), lane_of(r.s1[v], j), lane_of(r.e[v], j), r.ra, r.rb, o.p);
         else adagrad_value(g, lane_of(r.s0[v], j), lane_of(r.e[v], j), o.p);
       }
       const int64_t k = at + v * G * VEC;

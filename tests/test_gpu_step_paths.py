@@ -164,3 +164,11 @@ def test_sorted_view_follows_insertions(cuda_lib):
     from hades_b200 import EmbCacheLib as E
 
     _run_pair(*_pair("sorted_insert", lookup_mode=E.LOOKUP_SORTED), _steps(_small("sorted_insert"), 7))
+
+
+@pytest.mark.parametrize("optimizer", ["adam", "adagrad"])
+@pytest.mark.parametrize("dim", [3, 47, 127])
+def test_rows_of_odd_width_as_composed(cuda_lib, dim, optimizer):
+    """Columns one by one: counts and bias corrections divide in both forms."""
+    a, b = _pair(f"odd_{dim}_{optimizer}", dim=dim, optimizer=optimizer)
+    _run_pair(a, b, _steps(_small("odd", dim), 7))
