@@ -95,8 +95,8 @@ struct AddFinish {
   __device__ __forceinline__ void run(Ctx& ctx, const Src& src) const {
     const uint2* kv = ctx.publish(sorted);
     if (walk_later) return;
-    for (int j = ctx.chunk_begin() + threadIdx.x; j < ctx.chunk_end(); j += Ctx::kThreads)
-      add_sorted_set<Src::kSkips>(j, ctx.count, kv, src.ids, line_ids, lru, locs, last_writer);
+    for (uint32_t j = ctx.chunk_begin() + threadIdx.x; j < ctx.chunk_end(); j += Ctx::kThreads)
+      add_sorted_set<Src::kSkips>((int)j, ctx.count, kv, src.ids, line_ids, lru, locs, last_writer);
   }
 };
 

@@ -104,7 +104,7 @@ struct RunsFinish {
       ne = (int)s_valid;
       if (ctx.rank == 0 && threadIdx.x == 0) *n_valid = ne;
     }
-    const int begin = ctx.chunk_begin(), end = ctx.chunk_end();
+    const uint32_t begin = ctx.chunk_begin(), end = ctx.chunk_end();
     // id of an entry of the narrow kind (entries that sort last: the sentinel)
     auto narrow_id = [&](uint32_t key) -> int64_t {
       return key == kSortNone && ctx.none ? src.sentinel : (int64_t)key;
@@ -116,7 +116,7 @@ struct RunsFinish {
     // A thread takes 8 consecutive entries (whole vectors of positions and head flags to
     // write, one entry of base8, no votes), the CTA 8 * T in a strip.
     uint32_t code = 0u;  // per entry 3 bits: 4 | class (3: none) where a run starts, else 0
-    auto classify = [&](int j0, bool write) -> int4 {
+    auto classify = [&](uint32_t j0, bool write) -> int4 {
       int4 c = make_int4(0, 0, 0, 0);
       code = 0u;
       uint2 e[8];
@@ -129,7 +129,7 @@ struct RunsFinish {
       if (!ctx.wide) {
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
-          heads |= (unsigned)(j0 + x < ne && (j0 + x == 0 || e[x].x != before)) << x;
+          heads |= (unsigned)(j0 + x < (uint32_t)ne && (j0 + x == 0 || e[x].x != before)) << x;
           before = e[x].x;
         }
       } else {
@@ -137,7 +137,7 @@ struct RunsFinish {
 #pragma unroll 1
         for (int x = 0; x < 8 && j0 + x < end; ++x) {
           const int64_t id = wide_id(ctx.get(j0 + x).y);
-          heads |= (unsigned)(j0 + x < ne && id != was) << x;
+          heads |= (unsigned)(j0 + x < (uint32_t)ne && id != was) << x;
           was = id;
         }
       }
@@ -199,7 +199,7 @@ struct RunsFinish {
       return make_int4((int)(inc & 0xffff), (int)((inc >> 16) & 0xffff), (int)((inc >> 32) & 0xffff), (int)(inc >> 48));
     };
     uint32_t kept = 0u;  // the codes of the first of two strips
-    const int strips = (end - begin + 8 * T - 1) / (8 * T);
+    const int strips = (int)((end - begin + 8 * T - 1) / (8 * T));
     int4 mine = make_int4(0, 0, 0, 0), lanes = mine, warps, cta, ahead, all;
 #pragma unroll 1
     for (int q = 0; q < strips; ++q) {
@@ -213,8 +213,8 @@ struct RunsFinish {
     if (!ctx.prefix(cta, ahead, all)) return;
 #pragma unroll 1
     for (int q = 0; q < strips; ++q) {
-      const int strip = begin + q * (8 * T);
-      const int j0 = strip + threadIdx.x * 8;
+      const uint32_t strip = begin + q * (8 * T);
+      const uint32_t j0 = strip + threadIdx.x * 8;
       if (strips > 1) {
         int4 total, c = make_int4(0, 0, 0, 0);
         if (strips > 2) {
@@ -261,7 +261,7 @@ struct RunsFinish {
 #pragma unroll 2
       for (int r = threadIdx.x; r < runs; r += T) {
         const uint32_t w = ctx.scratch[r];
-        const int j = strip + (int)(w & 8191u);
+        const uint32_t j = strip + (w & 8191u);
         const uint2 e = ctx.get(j);
         const int64_t id = ctx.wide ? wide_id(e.y) : narrow_id(e.x);
         const int u = before + r;

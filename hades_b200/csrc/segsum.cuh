@@ -396,7 +396,7 @@ segsum_kernel(SegArgs a, Epi epi) {
   const int64_t at = b0 + (int64_t)grp * R;
   const bool live = at < n_eff;
   const int j0 = live ? (int)at : n_eff;
-  const int j1 = n_eff - j0 < R ? n_eff : j0 + R;
+  const int len = n_eff - j0 < R ? n_eff - j0 : R;  // (j0 + R may not be a number: entries are counted from j0)
   const int vpr = a.cols / VEC;  // vectors per row in this pass
 
   int u = -1;              // the open run; before the first head of a piece that begins with one: the run before
@@ -451,10 +451,10 @@ segsum_kernel(SegArgs a, Epi epi) {
     head_next = __ldg(a.head + j) != 0;
     end_next = j + 1 >= n_eff || __ldg(a.head + j + 1) != 0;
   };
-  if (sub < eg && j0 + sub < j1) look(j0 + sub);
+  if (sub < eg && sub < len) look(j0 + sub);
   for (int s = 0; s < steps; ++s) {
-    const int j = j0 + s * eg + sub;
-    const bool valid = sub < eg && j < j1;
+    const int at = s * eg + sub;
+    const bool valid = sub < eg && at < len;
     const uint32_t p = p_next;
     const unsigned heads = (__ballot_sync(0xffffffffu, valid && head_next) >> shift) & gbits;
     const unsigned ends = (__ballot_sync(0xffffffffu, valid && end_next) >> shift) & gbits;
@@ -471,7 +471,7 @@ segsum_kernel(SegArgs a, Epi epi) {
       l2_prefetch_row(a.grads + (int64_t)p * a.dim + a.col0, a.cols * 4);
       Ops::prefetch(epi, a, mine);
     }
-    if (s + 1 < steps && sub < eg && j + eg < j1) look(j + eg);
+    if (s + 1 < steps && sub < eg && at + eg < len) look(j0 + at + eg);
 #pragma unroll 1
     for (int t0 = 0; t0 < eg; t0 += U) {
       V val[U][VPL];

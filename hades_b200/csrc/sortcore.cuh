@@ -28,6 +28,7 @@
 
 #include <cooperative_groups.h>
 
+#include "chunks.cuh"
 #include "launch.cuh"
 
 namespace hb {
@@ -276,14 +277,14 @@ struct ClusterCtx {
   __device__ __forceinline__ int first() const {
     return rank * kChunk + (threadIdx.x >> 5) * (32 * ITEMS) + (threadIdx.x & 31);
   }
-  __device__ __forceinline__ int chunk_begin() const { return rank * kChunk; }
-  __device__ __forceinline__ int chunk_end() const {
-    const int e = chunk_begin() + kChunk;
+  __device__ __forceinline__ uint32_t chunk_begin() const { return rank * kChunk; }
+  __device__ __forceinline__ uint32_t chunk_end() const {
+    const int e = rank * kChunk + kChunk;
     return e < count ? e : count;
   }
   // a sorted entry of this chunk, or the last one of the chunk before
   __device__ __forceinline__ uint2 get(int j) const {
-    const int at = j - chunk_begin();
+    const int at = j - (int)chunk_begin();
     if (at >= 0) return s.kv[at];
     return *cg::this_cluster().map_shared_rank(s.kv + (kChunk + at), rank - 1);
   }
@@ -518,22 +519,18 @@ struct GridCtx {
   int4* s_pref;        // shared memory [2]
   int* s_flag;         // shared memory [1]
   int* err;
+  SortChunks chunks;
   int count;
-  int chunk;       // entries per CTA
   int rank, ctas, ntiles;
   unsigned arrived;    // barriers passed so far
   bool wide, none, alive;
-  __device__ __forceinline__ int chunk_begin() const {
-    const int b = rank * chunk;
-    return b < count ? b : count;
-  }
-  __device__ __forceinline__ int chunk_end() const {
-    const int e = rank * chunk + chunk;
-    return e < count ? e : count;
-  }
+  __device__ __forceinline__ explicit GridCtx(int n)
+      : chunks((uint32_t)n, gridDim.x, kGridT), count(n), rank(blockIdx.x), ctas(gridDim.x), arrived(0), alive(true) {}
+  __device__ __forceinline__ uint32_t chunk_begin() const { return chunks.begin(rank); }
+  __device__ __forceinline__ uint32_t chunk_end() const { return chunks.end(rank); }
   // a tile is kGridT * kItems entries (the last one fewer), a warp takes 32 * kItems consecutive ones
-  __device__ __forceinline__ int first(int t) const {
-    return rank * chunk + t * (kGridT * kItems) + (threadIdx.x >> 5) * (32 * kItems) + (threadIdx.x & 31);
+  __device__ __forceinline__ uint32_t first(int t) const {
+    return chunks.entry(rank, t, kGridT * kItems, (threadIdx.x >> 5) * (32 * kItems) + (threadIdx.x & 31));
   }
   __device__ __forceinline__ void get8(int j, uint2 (&e)[8]) const {
     const uint4* p = reinterpret_cast<const uint4*>(kv + j);
@@ -618,29 +615,20 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
   uint32_t* s_warp = reinterpret_cast<uint32_t*>(s_pref + 2);
   unsigned* s_seen = s_warp + (kGridT / 32);
   int* s_flag = reinterpret_cast<int*>(s_seen + 4);
-  GridCtx<I> ctx;
+  const int n = (int)src.count();
+  if (Src::kSkips && n == 0) return;
+  GridCtx<I> ctx(n);
   ctx.scratch = wmask;
   ctx.exchange = b.exchange;
   ctx.bar = b.barrier;
   ctx.s_pref = s_pref;
   ctx.s_flag = s_flag;
   ctx.err = err;
-  ctx.rank = blockIdx.x;
-  ctx.ctas = gridDim.x;
-  ctx.arrived = 0;
-  ctx.alive = true;
-  const int n = (int)src.count();
-  if (Src::kSkips && n == 0) return;
-  ctx.count = n;
-  {
-    const int per = (n + ctx.ctas - 1) / ctx.ctas;
-    ctx.chunk = (per + kGridT - 1) / kGridT * kGridT;  // whole rounds of the CTA
-  }
-  ctx.ntiles = ((ctx.chunk + kGridT * I - 1) / (kGridT * I));
+  ctx.ntiles = (int)((ctx.chunks.chunk + kGridT * I - 1) / (kGridT * I));
   if (ctx.ntiles < 1) ctx.ntiles = 1;
   const int nt = ctx.ntiles;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int end = ctx.chunk_end();
+  const uint32_t end = ctx.chunk_end();
   uint32_t k[I];
   uint32_t rank[(I + 1) / 2];
   SortDigits dig;
@@ -653,10 +641,10 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
     // (a chunk of several tiles is read again by the first pass: needed here only to find the width)
     for (int t = 0; t < nt; ++t) {
       if (nt > 1 && known) break;
-      const int first = ctx.first(t);
+      const uint32_t first = ctx.first(t);
 #pragma unroll
       for (int i = 0; i < I; ++i) {
-        const int j = first + i * 32;
+        const uint32_t j = first + i * 32;
         k[i] = kSortNone;
         if (j < end) {
           unsigned long long key;
@@ -709,14 +697,14 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
     uint16_t* wc = wcnt + warp * bins;
     // keys of a tile into k[] (already there for the first pass of a chunk of one tile)
     auto load_tile = [&](int t) {
-      const int first = ctx.first(t);
+      const uint32_t first = ctx.first(t);
 #pragma unroll
       for (int i = 0; i < I; ++i) {
-        const int j = first + i * 32;
+        const uint32_t j = first + i * 32;
         if (j >= end) continue;
         unsigned long long key;
         if (dig.wide)
-          k[i] = src.load(in ? (int)__ldcg(&in[j].y) : j, key) ? (uint32_t)(key >> bit) : kSortNone;
+          k[i] = src.load(in ? __ldcg(&in[j].y) : j, key) ? (uint32_t)(key >> bit) : kSortNone;
         else if (in)
           k[i] = __ldcg(&in[j].x);
         else if (nt > 1)
@@ -728,7 +716,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
       sort_zero_counts<kGridT>(wcnt, wmask, bins, pass == 0 && t == 0 ? (kGridT / 32) * bins : 0);
       load_tile(t);
       __syncthreads();
-      sort_rank_warp<I>(k, end - ctx.first(t), shift, width, wc, wmask + warp * bins, rank);
+      sort_rank_warp<I>(k, (int)(end - ctx.first(t)), shift, width, wc, wmask + warp * bins, rank);
       __syncthreads();
       sort_scan_warps<kGridT>(wcnt, bins, s_tot);
       __syncthreads();
@@ -781,14 +769,14 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
     for (int t = 0; t < nt; ++t) {
       if (nt > 1) last = rank_tile(t);
       __syncthreads();
-      const int first = ctx.first(t);
+      const uint32_t first = ctx.first(t);
 #pragma unroll
       for (int i = 0; i < I; ++i) {
-        const int j = first + i * 32;
+        const uint32_t j = first + i * 32;
         if (j < end) {
           const uint32_t d = (k[i] >> shift) & mask;
           const uint32_t to = s_base[d] + wc[d] + ((rank[i >> 1] >> (16 * (i & 1))) & 0xffffu);
-          __stcg(out + to, make_uint2(k[i], in ? __ldcg(&in[j].y) : (uint32_t)j));
+          __stcg(out + to, make_uint2(k[i], in ? __ldcg(&in[j].y) : j));
         }
       }
       if (nt > 1) {
