@@ -1,0 +1,31 @@
+// The barrier between the CTAs of a cooperative grid: one word counts the arrivals of all barriers so far.  Waits
+// are bounded; a CTA that gives up marks the word for good, unless the barrier completes first, so that all CTAs
+// of a launch see the same end of its last barrier: either every one passes it or none does.
+#pragma once
+
+#include "chunks.cuh"
+
+namespace hb {
+
+constexpr unsigned kGaveUp = 0x80000000u;
+
+// Word: add(1), load() and swap(was, to) on the word, pause(turn).  want: arrivals when this barrier is complete.
+template <class Word>
+HB_BOTH bool grid_barrier(Word& w, unsigned want, int turns) {
+  if (w.add(1u) & kGaveUp) return false;
+  for (int it = 0; it < turns; ++it) {
+    const unsigned seen = w.load();
+    if (seen & kGaveUp) return false;
+    if (seen >= want) return true;
+    w.pause(it);
+  }
+  for (int it = 0; it < 65536; ++it) {  // (a swap fails once per arrival at most)
+    const unsigned seen = w.load();
+    if (seen & kGaveUp) return false;
+    if (seen >= want) return true;
+    if (w.swap(seen, seen | kGaveUp)) return false;
+  }
+  return false;
+}
+
+}  // namespace hb

@@ -91,6 +91,16 @@ struct AddFinish {
   uint8_t* last_writer;    // nullable [n]: of several ids that received one slot, the last
   uint2* sorted;           // [n] scratch
   bool walk_later;         // by a launch of its own
+  // nothing was placed: no slots (of the sets that the lists left behind, where only those are sorted)
+  template <class Ctx, class Src>
+  __device__ __forceinline__ void give_up(Ctx& ctx, const Src& src) const {
+    for (uint32_t j = ctx.chunk_begin() + threadIdx.x; j < ctx.chunk_end(); j += Ctx::kThreads) {
+      unsigned long long key;
+      if (Src::kSkips && !src.load(j, key)) continue;
+      locs[j] = -1;
+      if (last_writer) last_writer[j] = 0;
+    }
+  }
   template <class Ctx, class Src>
   __device__ __forceinline__ void run(Ctx& ctx, const Src& src) const {
     const uint2* kv = ctx.publish(sorted);

@@ -185,6 +185,7 @@ PyObject* unique_segsum(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
                                uniq.data_ptr<int64_t>(), sums.data_ptr<float>(), counts.data_ptr<int64_t>(), num, nullptr,
                                nullptr, ws.data_ptr(), need, st));
     const int64_t u = t_word.wait(static_cast<cudaStream_t>(st));
+    if (u == 0) throw std::runtime_error("the sort of the ids gave up waiting (hb_device_status)");
     return pack({THPVariable_Wrap(uniq.narrow(0, 0, u)), THPVariable_Wrap(sums.narrow(0, 0, u)),
                  THPVariable_Wrap(counts.narrow(0, 0, u))});
   });

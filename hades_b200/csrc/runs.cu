@@ -78,9 +78,20 @@ struct RunsFinish {
   int64_t* class_counts;
   int64_t* class_counts2;
   int32_t* base8;        // [ceil(n / 8)] runs that start before entry 8k
-  int64_t* n_valid;      // number of valid entries of a segmented input
+  int64_t* n_valid;      // number of valid entries (read where the input is segmented or large)
   unsigned* zero;        // nullable: words that the next launch needs at zero
   int zero_words;
+
+  // no runs and no entries: what works on the runs has nothing to do
+  template <class Ctx>
+  __device__ __forceinline__ void give_up(Ctx& ctx, const IdSource&) const {
+    for (int k = threadIdx.x; k < zero_words; k += Ctx::kThreads) zero[k] = 0u;
+    if (threadIdx.x != 0) return;  // (every CTA writes the same)
+    *num_runs = *n_valid = run_start[0] = 0;
+    if (num_runs2) *num_runs2 = 0;
+    for (int c = 0; c < 4; ++c) class_counts[c] = 0;
+    for (int c = 0; class_counts2 && c < 3; ++c) class_counts2[c] = 0;
+  }
 
   template <class Ctx>
   __device__ __forceinline__ void run(Ctx& ctx, const IdSource& src) const {
@@ -102,7 +113,6 @@ struct RunsFinish {
       if (t) atomicAdd(&s_valid, t);
       __syncthreads();
       ne = (int)s_valid;
-      if (ctx.rank == 0 && threadIdx.x == 0) *n_valid = ne;
     }
     const uint32_t begin = ctx.chunk_begin(), end = ctx.chunk_end();
     // id of an entry of the narrow kind (entries that sort last: the sentinel)
@@ -210,7 +220,7 @@ struct RunsFinish {
       if (q == 0) kept = code;
     }
     sort_warp_sums<W>(mine, s_sum, warps, cta);
-    if (!ctx.prefix(cta, ahead, all)) return;
+    if (!ctx.prefix(cta, ahead, all)) return give_up(ctx, src);
 #pragma unroll 1
     for (int q = 0; q < strips; ++q) {
       const uint32_t strip = begin + q * (8 * T);
@@ -286,6 +296,7 @@ struct RunsFinish {
       *num_runs = u;
       if (num_runs2) *num_runs2 = u;
       run_start[u] = ne;
+      *n_valid = ne;
       class_counts[0] = all.x; class_counts[1] = all.y; class_counts[2] = all.z; class_counts[3] = all.w;
       if (class_counts2) { class_counts2[0] = all.x; class_counts2[1] = all.y; class_counts2[2] = all.z; }
     }
@@ -688,7 +699,8 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
     if (class_counts_out) HB_CUDA(cudaMemsetAsync(class_counts_out, 0, 3 * sizeof(int64_t), st));
     return HB_OK;
   }
-  runs_out->n_dev = seg_counts ? s.n_valid : n_dev;
+  // (a grid whose barrier runs out leaves no entries)
+  runs_out->n_dev = seg_counts || n > kSortClusterMax ? s.n_valid : n_dev;
   const int64_t sentinel = id_bits >= 63 ? INT64_MAX : (((int64_t)1 << id_bits) - 1);
   runs_out->perm = s.perm;
   IdSource src{ids, n, seg_counts ? nullptr : n_dev, seg_counts, (uint32_t)(seg_counts ? seg_cap : 1), sentinel,

@@ -23,12 +23,13 @@
 //    memory directly;
 //  * above that a cooperative grid, one CTA per SM, keeps its keys and ranks in registers between
 //    the counting and the scatter of a pass and goes through L2; barriers are counters in the
-//    workspace with bounded waits.
+//    workspace with bounded waits (gridbar.cuh).  A launch whose barrier runs out leaves an empty result
+//    (give_up of its finish) for the launches behind it.
 #pragma once
 
 #include <cooperative_groups.h>
 
-#include "chunks.cuh"
+#include "gridbar.cuh"
 #include "launch.cuh"
 
 namespace hb {
@@ -523,9 +524,9 @@ struct GridCtx {
   int count;
   int rank, ctas, ntiles;
   unsigned arrived;    // barriers passed so far
-  bool wide, none, alive;
+  bool wide, none;
   __device__ __forceinline__ explicit GridCtx(int n)
-      : chunks((uint32_t)n, gridDim.x, kGridT), count(n), rank(blockIdx.x), ctas(gridDim.x), arrived(0), alive(true) {}
+      : chunks((uint32_t)n, gridDim.x, kGridT), count(n), rank(blockIdx.x), ctas(gridDim.x), arrived(0) {}
   __device__ __forceinline__ uint32_t chunk_begin() const { return chunks.begin(rank); }
   __device__ __forceinline__ uint32_t chunk_end() const { return chunks.end(rank); }
   // a tile is kGridT * kItems entries (the last one fewer), a warp takes 32 * kItems consecutive ones
@@ -543,30 +544,33 @@ struct GridCtx {
   }
   __device__ __forceinline__ uint2 get(int j) const { return __ldcg(kv + j); }
   __device__ __forceinline__ const uint2* publish(uint2*) { return kv; }
+  struct Word {
+    unsigned* at;
+    __device__ __forceinline__ unsigned add(unsigned v) const { return atomicAdd(at, v); }
+    __device__ __forceinline__ unsigned load() const {
+      unsigned seen;
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(at) : "memory");
+      return seen;
+    }
+    __device__ __forceinline__ bool swap(unsigned was, unsigned to) const { return atomicCAS(at, was, to) == was; }
+    __device__ __forceinline__ void pause(int turn) const {
+      if (turn > 4096) __nanosleep(64);
+    }
+  };
+  // false: some CTA did not arrive within a second or two; the launch ends, its status word says so
   __device__ __forceinline__ bool barrier() {
     ++arrived;
     __syncthreads();
     if (threadIdx.x == 0) {
-      bool ok = alive;
-      if (ok) {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        const unsigned want = arrived * (unsigned)ctas;
-        ok = false;
-        for (int it = 0; it < (1 << 21); ++it) {  // bounded: a second or two, then the call reports a time-out
-          unsigned seen;
-          asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-          if (seen >= want) { ok = true; break; }
-          if (it > 4096) __nanosleep(64);
-        }
-        __threadfence();
-        if (!ok && err) atomicExch(err, HB_ERR_TIMEOUT);
-      }
+      __threadfence();
+      Word w{bar};
+      const bool ok = grid_barrier(w, arrived * (unsigned)ctas, 1 << 21);
+      __threadfence();
+      if (!ok && err) atomicExch(err, HB_ERR_TIMEOUT);
       *s_flag = ok;
     }
     __syncthreads();
-    alive = *s_flag != 0;
-    return alive;
+    return *s_flag != 0;
   }
   __device__ __forceinline__ bool prefix(const int4& mine, int4& before, int4& all) {
     if (threadIdx.x == 0) __stcg(exchange + rank, mine);
@@ -671,7 +675,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
       }
       __syncthreads();
       if (threadIdx.x == 0) __stcg(reinterpret_cast<uint4*>(b.partial) + ctx.rank, make_uint4(s_seen[0], s_seen[1], s_seen[2], 0u));
-      if (!ctx.barrier()) return;
+      if (!ctx.barrier()) return fin.give_up(ctx, src);
       lo = hi = 0;
       unsigned nn = 0;
       for (int c = lane; c < ctx.ctas; c += 32) {
@@ -728,7 +732,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
       mine += last;
     }
     if ((int)threadIdx.x < bins) __stcg(b.hist + ctx.rank * bins + threadIdx.x, mine);
-    if (!ctx.barrier()) return;
+    if (!ctx.barrier()) return fin.give_up(ctx, src);
     // every CTA turns the counts of its share of the digits into offsets, a warp per digit
     {
       const int per = (bins + ctx.ctas - 1) / ctx.ctas;
@@ -759,7 +763,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
         if (lane == 0) __stcg(b.total + d, run);
       }
     }
-    if (!ctx.barrier()) return;
+    if (!ctx.barrier()) return fin.give_up(ctx, src);
     {
       const uint32_t all = (int)threadIdx.x < bins ? __ldcg(b.total + threadIdx.x) : 0u;
       const uint32_t pre = (int)threadIdx.x < bins ? __ldcg(b.hist + ctx.rank * bins + threadIdx.x) : 0u;
@@ -784,7 +788,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
         if ((int)threadIdx.x < bins) s_base[threadIdx.x] += last;
       }
     }
-    if (!ctx.barrier()) return;
+    if (!ctx.barrier()) return fin.give_up(ctx, src);
     in = out;
     out = out == b.kv0 ? b.kv1 : b.kv0;
   }
