@@ -468,6 +468,18 @@ __device__ __forceinline__ int64_t run_of_entry(const hb_runs_t& r, int64_t j) {
   return (int64_t)__ldg(r.base8 + (j >> 3)) + __popcll(flags & mask) - 1;
 }
 
+// The id of every sorted entry; entries that take no part hold the sentinel.  perm (nullable): positions
+// at and beyond the device count follow in order.
+template <typename K>
+__global__ void __launch_bounds__(kBlock) runs_keys_kernel(hb_runs_t r, int64_t sentinel, K* __restrict__ keys,
+                                                           uint32_t* __restrict__ perm) {
+  const int64_t n = runs_valid_entries(r);
+  for (int64_t j = blockIdx.x * (int64_t)kBlock + threadIdx.x; j < r.n; j += (int64_t)gridDim.x * kBlock) {
+    keys[j] = (K)(j < n ? __ldg(r.uniq_ids + run_of_entry(r, j)) : sentinel);
+    if (perm && j >= n) perm[j] = (uint32_t)j;
+  }
+}
+
 // RB: 512 = rows of exactly 512 bytes (128 fp32: the address arithmetic folds, no lane is idle);
 // 16 = any multiple of 16 bytes; 0 = words or bytes.  PEER: a source may be another GPU's memory
 // (runs that found no room in the stage), so rows are read with plain loads.
@@ -625,7 +637,7 @@ __global__ void fill_i64_kernel(int64_t* p, int64_t n, int64_t v) {
 
 }  // namespace
 
-RunsPlan make_runs_plan(void* ws, int64_t n) {
+RunsPlan make_runs_plan(void* ws, int64_t n, bool keys) {
   RunsPlan s;
   Carver cv(ws ? ws : (void*)256);  // a null workspace still yields the sizes
   const int64_t m = n > 0 ? n : 1;
@@ -640,6 +652,7 @@ RunsPlan make_runs_plan(void* ws, int64_t n) {
   s.dpos = cv.take<int32_t>(m + 1);
   s.uniq = cv.take<int64_t>(m + 1);
   s.base8 = cv.take<int32_t>(m / 8 + 2);
+  s.keys = keys ? cv.take<int64_t>(m) : nullptr;
   s.total = cv.used() + 256;
   return s;
 }
@@ -650,19 +663,41 @@ using namespace hb;
 
 extern "C" {
 
-size_t hb_runs_workspace_bytes(int64_t n) { return make_runs_plan(nullptr, n).total; }
+size_t hb_runs_workspace_bytes(int64_t n) { return make_runs_plan(nullptr, n, true).total; }
 
 int hb_runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int64_t* seg_counts,
                   int64_t seg_cap, int id_bits, const int8_t* class_table, int64_t table_len,
                   int64_t* const* class_ids_out, int64_t* class_counts_out, int64_t* uniq_ids_out,
                   int64_t* num_unique_out, void* workspace, size_t workspace_bytes,
                   hb_runs_t* runs_out, hb_stream_t stream) {
-  return runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, class_table, table_len, class_ids_out,
-                    class_counts_out, uniq_ids_out, num_unique_out, nullptr, 0, workspace, workspace_bytes, runs_out,
-                    (cudaStream_t)stream);
+  if (workspace && workspace_bytes < hb_runs_workspace_bytes(n)) workspace = nullptr;  // (runs_build says what is missing)
+  const int rc = runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, class_table, table_len, class_ids_out,
+                            class_counts_out, uniq_ids_out, num_unique_out, nullptr, 0, workspace, workspace_bytes,
+                            runs_out, (cudaStream_t)stream);
+  return rc != HB_OK ? rc : runs_keys(seg_counts, id_bits, workspace, runs_out, (cudaStream_t)stream);
 }
 
 }  // extern "C"
+
+// what stands for an entry without a valid id: above every other
+static int64_t runs_sentinel(int id_bits) { return id_bits >= 63 ? INT64_MAX : (((int64_t)1 << id_bits) - 1); }
+
+int hb::runs_keys(const int64_t* seg_counts, int id_bits, void* workspace, hb_runs_t* runs, cudaStream_t st) {
+  runs->keys = nullptr;
+  runs->key_bytes = 0;
+  if (runs->n == 0) return HB_OK;
+  const RunsPlan s = make_runs_plan(workspace, runs->n, true);
+  int64_t blocks = ceil_div(runs->n, kBlock);
+  if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
+  uint32_t* rest = seg_counts ? nullptr : s.perm;
+  if (id_bits <= 32)
+    HB_LAUNCH(runs_keys_kernel<uint32_t>, (int)blocks, kBlock, 0, st, *runs, runs_sentinel(id_bits), (uint32_t*)s.keys, rest);
+  else
+    HB_LAUNCH(runs_keys_kernel<int64_t>, (int)blocks, kBlock, 0, st, *runs, runs_sentinel(id_bits), (int64_t*)s.keys, rest);
+  runs->keys = s.keys;
+  runs->key_bytes = id_bits <= 32 ? 4 : 8;
+  return HB_OK;
+}
 
 int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int64_t* seg_counts, int64_t seg_cap,
                    int id_bits, const int8_t* class_table, int64_t table_len, int64_t* const* class_ids_out,
@@ -676,9 +711,9 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
   HB_CHECK_ARG(!seg_counts || (seg_cap > 0 && n % seg_cap == 0),
                "hb_runs_build: a segmented input holds whole segments of seg_cap entries");
   HB_CHECK_ARG(!class_table || table_len > 0, "hb_runs_build: a class table needs its length");
-  RunsPlan s = make_runs_plan(workspace, n);
+  RunsPlan s = make_runs_plan(workspace, n, false);
   if (!workspace || workspace_bytes < s.total) {
-    set_error("hb_runs_build: workspace of %zu bytes needed, %zu given", s.total, workspace_bytes);
+    set_error("hb_runs_build: workspace of %zu bytes needed, %zu given", hb_runs_workspace_bytes(n), workspace_bytes);
     return HB_ERR_WORKSPACE;
   }
   memset(runs_out, 0, sizeof(*runs_out));
@@ -701,7 +736,7 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
   }
   // (a grid whose barrier runs out leaves no entries)
   runs_out->n_dev = seg_counts || n > kSortClusterMax ? s.n_valid : n_dev;
-  const int64_t sentinel = id_bits >= 63 ? INT64_MAX : (((int64_t)1 << id_bits) - 1);
+  const int64_t sentinel = runs_sentinel(id_bits);
   runs_out->perm = s.perm;
   IdSource src{ids, n, seg_counts ? nullptr : n_dev, seg_counts, (uint32_t)(seg_counts ? seg_cap : 1), sentinel,
                device_error_word(), id_bits};

@@ -95,7 +95,11 @@ int hb_unique_segsum_f32(const int64_t* ids, const float* grads, const int64_t* 
                       split ? split->table_len : 0, split ? cls_ids : nullptr, split ? split->class_counts : nullptr,
                       uniq_ids, num_unique, s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream);
   if (rc != HB_OK) return rc;
-  if (runs_out) *runs_out = runs;
+  if (runs_out) {
+    rc = runs_keys(seg_counts, id_bits, workspace, &runs, (cudaStream_t)stream);
+    if (rc != HB_OK) return rc;
+    *runs_out = runs;
+  }
   return segsum_runs(&runs, grads, cnt_in, dim, mean, sums, counts, split, seg_ws, workspace_bytes - runs_bytes, true,
                      (cudaStream_t)stream);
 }

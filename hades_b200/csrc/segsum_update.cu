@@ -19,6 +19,7 @@ bool at_once(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt) 
   return dim <= seg_tile(dim % 4 == 0 && (bits & 15) == 0);
 }
 
+size_t runs_bytes_of(int64_t n) { return align_up(make_runs_plan(nullptr, n, false).total, 256); }
 size_t sums_bytes(int64_t n, int64_t dim) { return align_up((size_t)(n * dim) * sizeof(float), 256); }
 
 }  // namespace
@@ -26,7 +27,7 @@ size_t sums_bytes(int64_t n, int64_t dim) { return align_up((size_t)(n * dim) * 
 extern "C" {
 
 size_t hb_unique_update_workspace_bytes(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt) {
-  return hb_unique_segsum_workspace_bytes(n, dim) + (at_once(n, dim, grads, opt) ? 0 : sums_bytes(n, dim));
+  return runs_bytes_of(n) + seg_plan(nullptr, n, dim).total + (at_once(n, dim, grads, opt) ? 0 : sums_bytes(n, dim));
 }
 
 int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* cnt_in, int64_t n, const int64_t* n_dev,
@@ -50,7 +51,7 @@ int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* 
   const bool once = at_once(n, dim, grads, opt);
   float* sums = static_cast<float*>(workspace);  // first: on a 256-byte boundary
   char* runs_ws = static_cast<char*>(workspace) + (once ? 0 : sums_bytes(n, dim));
-  const size_t runs_bytes = align_up(hb_runs_workspace_bytes(n), 256);
+  const size_t runs_bytes = runs_bytes_of(n);
   char* seg_ws = runs_ws + runs_bytes;
   const SegPlan s = seg_plan(seg_ws, n, dim);
   hb_runs_t runs;

@@ -63,7 +63,7 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
   StepPlan p;
   Carver cv(ws ? ws : (void*)256);
   const int64_t m = n > 0 ? n : 1;
-  p.runs_bytes = hb_runs_workspace_bytes(m);
+  p.runs_bytes = make_runs_plan(nullptr, m, false).total;
   p.runs_ws = cv.take<char>(p.runs_bytes);
   p.fetch_bytes = hb_lookup_fetch_runs_workspace_bytes(m, 1, 0);
   p.fetch_ws = cv.take<char>(p.fetch_bytes);

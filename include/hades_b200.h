@@ -338,7 +338,7 @@ typedef struct hb_runs {
   const int64_t* run_start;   /* [num_runs + 1]; run_start[num_runs] = valid entries */
   const int64_t* num_runs;    /* device int64 (= number of distinct ids) */
   int64_t n;
-  const void* keys;           /* NULL: the id of a sorted entry is uniq_ids of its run */
+  const void* keys;           /* [n] sorted ids: uint32 (key_bytes 4) or int64 (key_bytes 8) */
   int key_bytes;
   const uint8_t* head;        /* [n] 1 where a run starts */
   const int64_t* uniq_ids;    /* [num_runs] ascending */

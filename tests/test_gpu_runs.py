@@ -271,3 +271,32 @@ def test_sort_of_ids_of_stated_width(cuda_lib, bits):
         u, _, cnt = E.cudaUniqueSegSum(ids, rows, id_bits=bits)
         want, counts = torch.unique(ids, return_counts=True)
         assert torch.equal(u, want) and torch.equal(cnt, counts), n
+
+
+@pytest.mark.parametrize("n", [1, 1000, 65_536, 70_000])
+@pytest.mark.parametrize("bits,low,space", [(21, 0, 1_000_000), (32, 2**32 - 60_000, 59_999), (64, 0, 900), (64, 2**40, 10**6)])
+def test_sorted_ids_of_the_entries(cuda_lib, n, bits, low, space):
+    """hb_runs_t.keys, and perm where a device count or segments leave entries out."""
+    from hades_b200 import EmbCacheLib as E
+    from hades_b200.exchange import _as_tensor
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + bits)
+    ids = low + torch.randint(0, space, (n,), device="cuda", generator=g)
+    last = 2**63 - 1 if bits == 64 else 2**bits - 1
+    cap = max(n // 2, 1)
+    seg = torch.tensor([cap // 3, cap][: n // cap], device="cuda")
+    for kw in ({}, {"n_dev": torch.tensor([n // 3], device="cuda")}, {"seg_counts": seg, "seg_cap": cap}):
+        runs = E.cudaRunsBuild(ids, bits, **kw)
+        assert runs.desc.key_bytes == (4 if bits <= 32 else 8)
+        keys = _as_tensor(runs.desc.keys, (n,), "<i4" if bits <= 32 else "<i8", ids.device).long()
+        keys = keys & 0xFFFFFFFF if bits <= 32 else keys
+        at = torch.arange(n, device="cuda")
+        out = torch.zeros(n, dtype=torch.bool, device="cuda")
+        if "n_dev" in kw:
+            out = at >= n // 3
+        elif kw:
+            out = at % cap >= seg[at // cap]
+        want, order = torch.where(out, last, ids).sort(stable=True)
+        assert torch.equal(keys, want)
+        assert torch.equal(_as_tensor(runs.desc.perm, (n,), "<i4", ids.device).long(), order)
