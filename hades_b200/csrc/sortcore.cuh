@@ -278,20 +278,17 @@ struct ClusterCtx {
   __device__ __forceinline__ int first() const {
     return rank * kChunk + (threadIdx.x >> 5) * (32 * ITEMS) + (threadIdx.x & 31);
   }
-  __device__ __forceinline__ uint32_t chunk_begin() const { return rank * kChunk; }
-  __device__ __forceinline__ uint32_t chunk_end() const {
-    const int e = rank * kChunk + kChunk;
-    return e < count ? e : count;
-  }
+  __device__ __forceinline__ uint32_t chunk_begin() const { return SortChunks(count, kChunk).begin(rank); }
+  __device__ __forceinline__ uint32_t chunk_end() const { return SortChunks(count, kChunk).end(rank); }
   // a sorted entry of this chunk, or the last one of the chunk before
   __device__ __forceinline__ uint2 get(int j) const {
-    const int at = j - (int)chunk_begin();
+    const int at = j - rank * kChunk;
     if (at >= 0) return s.kv[at];
     return *cg::this_cluster().map_shared_rank(s.kv + (kChunk + at), rank - 1);
   }
   // 8 consecutive ones of this chunk from a multiple of 8 on (those at and beyond `count` are undefined)
   __device__ __forceinline__ void get8(int j, uint2 (&e)[8]) const {
-    const uint4* p = reinterpret_cast<const uint4*>(s.kv + j - chunk_begin());
+    const uint4* p = reinterpret_cast<const uint4*>(s.kv + (j - rank * kChunk));
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint4 x = p[q];
@@ -347,7 +344,7 @@ struct ClusterCtx {
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
       const int j = first() + i * 32;
-      if (j < count) __stcg(buf + j, s.kv[j - chunk_begin()]);
+      if (j < count) __stcg(buf + j, s.kv[j - rank * kChunk]);
     }
     barrier();
     return buf;

@@ -1,5 +1,5 @@
-"""How the grid version of the sort cuts its input (csrc/chunks.cuh), compiled for the host: every entry is in
-one place, up to the largest number of entries that the library takes (2^31 - 1)."""
+"""How the sort cuts its input (csrc/chunks.cuh), compiled for the host: every entry is in one place, up to the
+largest number of entries that the library takes (2^31 - 1); the chunk of a CTA that gets nothing is empty."""
 import subprocess
 from pathlib import Path
 
@@ -39,6 +39,19 @@ int main() {
             }
         }
         if (next != n) return std::printf("end n=%u ctas=%d\n", n, ctas), 1;
+      }
+  // a cluster: chunks of one size, of which the last CTAs may get nothing
+  for (uint32_t chunk = 512; chunk <= 4096; chunk *= 2)
+    for (int ctas = 1; ctas <= 16; ++ctas)
+      for (uint32_t n = 0; n <= chunk * ctas; n += (n % 512 < 3 || n % 512 > 509) ? 1 : 101) {
+        const hb::SortChunks c(n, chunk);
+        uint32_t next = 0;
+        for (int r = 0; r < ctas; ++r) {
+          if (c.begin(r) != next || c.end(r) < next || c.end(r) - c.begin(r) > chunk)
+            return std::printf("cluster n=%u chunk=%u ctas=%d r=%d\n", n, chunk, ctas, r), 1;
+          next = c.end(r);
+        }
+        if (next != n) return std::printf("cluster end n=%u chunk=%u ctas=%d\n", n, chunk, ctas), 1;
       }
   return 0;
 }
