@@ -82,12 +82,24 @@ struct RunsFinish {
   unsigned* zero;        // nullable: words that the next launch needs at zero
   int zero_words;
 
-  // no runs and no entries: what works on the runs has nothing to do
+  // No runs and no entries: what works on the runs has nothing to do.  The sums go by the entries and do not
+  // wait for a device count where the caller has none: they find one run of all entries and no id.
   template <class Ctx>
-  __device__ __forceinline__ void give_up(Ctx& ctx, const IdSource&) const {
+  __device__ __forceinline__ void give_up(Ctx& ctx, const IdSource& src) const {
     for (int k = threadIdx.x; k < zero_words; k += Ctx::kThreads) zero[k] = 0u;
+    for (uint32_t j = ctx.chunk_begin() + threadIdx.x; j < ctx.chunk_end(); j += Ctx::kThreads) {
+      perm[j] = j;
+      head[j] = j == 0;
+      if ((j & 7u) == 0u) base8[j >> 3] = j != 0;
+    }
     if (threadIdx.x != 0) return;  // (every CTA writes the same)
     *num_runs = *n_valid = run_start[0] = 0;
+    run_start[1] = ctx.count;
+    uniq[0] = src.sentinel;
+    if (table) {
+      dclass[0] = -1;
+      dpos[0] = 0;
+    }
     if (num_runs2) *num_runs2 = 0;
     for (int c = 0; c < 4; ++c) class_counts[c] = 0;
     for (int c = 0; class_counts2 && c < 3; ++c) class_counts2[c] = 0;

@@ -100,6 +100,7 @@ int hb_unique_segsum_f32(const int64_t* ids, const float* grads, const int64_t* 
     if (rc != HB_OK) return rc;
     *runs_out = runs;
   }
+  if (!n_dev && !seg_counts) runs.n_dev = nullptr;  // all entries: nothing to wait for
   return segsum_runs(&runs, grads, cnt_in, dim, mean, sums, counts, split, seg_ws, workspace_bytes - runs_bytes, true,
                      (cudaStream_t)stream);
 }

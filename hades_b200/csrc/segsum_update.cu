@@ -58,6 +58,7 @@ int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* 
   int rc = runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
                       s.done, s.max_ctas, runs_ws, runs_bytes, &runs, st);
   if (rc != HB_OK) return rc;
+  if (!n_dev && !seg_counts) runs.n_dev = nullptr;  // all entries: nothing to wait for
   if (once) {
     SegArgs a = seg_args(&runs, grads, cnt_in, dim, mean, s);
     a.cols = (int)dim;

@@ -538,6 +538,7 @@ int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, 
   const ColdArgs c{d->staging, d->threshold_table, d->default_threshold, (unsigned long long*)d->dropped,
                    p.cold_slots, marks, d->touch_lru};
   SegArgs a = seg_args(&s->runs, grads, nullptr, d->dim, 0, seg);
+  a.n_dev = nullptr;  // all entries: nothing to wait for
   a.cols = (int)d->dim;
   return d->opt.kind == HB_OPT_ADAM ? update_step<true>(s, d, c, a, vec4, p.sums, seg, fused, st)
                                     : update_step<false>(s, d, c, a, vec4, p.sums, seg, fused, st);
