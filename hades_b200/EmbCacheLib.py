@@ -42,6 +42,11 @@ def _index_handle_path(name: str) -> str:
     return "/dev/shm/hades_b200_index_" + name.replace("/", "_")
 
 
+def _words_at(handle_bytes: int) -> int:
+    """Where the two 8-byte words behind an index's handle begin."""
+    return -(-handle_bytes // 8) * 8
+
+
 _PUBLISHED: set = set()  # handle files this process left in /dev/shm
 
 
@@ -101,7 +106,7 @@ class IndexCache:
         self._name = name
         self.lookup_mode = lookup_mode
         self._shm_file = None
-        self._opened_flag = None  # a byte that another process sets when it opens this index
+        self._shared_words = None  # [another process has opened this index, its lookups of host ids so far]
         if create:
             h = C.c_void_p()
             _lib.check(self._lib.hb_index_create(int(cache_size), C.byref(h)))
@@ -117,29 +122,31 @@ class IndexCache:
             self._owner = False
             self._device = other._device
             self._changing = other._changing
-            self._opened_flag = other._opened_flag
+            self._shared_words = other._shared_words
         else:
             # another process of this box created it: map its lines (src/cache/cache.h:155-158)
             path = _index_handle_path(name)
             try:
-                with open(path, "r+b") as f:
+                size = self._lib.hb_index_handle_bytes()
+                with open(path, "r+b", buffering=0) as f:
                     blob = f.read()
-                    _check(len(blob) == self._lib.hb_index_handle_bytes() + 1, "index handle file has the expected size")
-                    # before the open: it waits for the calls that have not seen the flag
-                    f.seek(len(blob) - 1)
-                    f.write(b"\1")
+                    _check(len(blob) == _words_at(size) + 16, "index handle file has the expected size")
+                    f.seek(_words_at(size))
+                    f.write((1).to_bytes(8, "little"))
+                    lookups = int.from_bytes(f.read(8), "little")
             except OSError as e:
                 raise RuntimeError(f"fail to open {name}: no such index on this box ({e.strerror})") from e
             h = C.c_void_p()
-            _lib.check(self._lib.hb_index_open(blob[:-1], C.byref(h)))
-            self._opened_flag = C.c_char(b"\1")
+            _lib.check(self._lib.hb_index_open(blob[:size], C.byref(h)))
+            _lib.check(self._lib.hb_index_wait_lookups(h, lookups, _lib.stream_ptr()))
+            self._shared_words = (C.c_uint64 * 2)(1, 0)
             self._h = h
             self._owner = True  # of the mapping: destroyed (closed) with this object
             self._device = torch.cuda.current_device()
             self._changing = threading.Lock()
 
     def _publish(self) -> None:
-        """Leave the IPC handle, and behind it the flag of an opener, where other processes of the box find it by name."""
+        """Leave the IPC handle, and the words shared with openers behind it, where other processes of the box find it."""
         import mmap
         import os
 
@@ -148,9 +155,10 @@ class IndexCache:
             _lib.check(self._lib.hb_index_export_handle(self._h, buf))
             path = _index_handle_path(self._name)
             with open(path + ".tmp", "w+b") as f:
-                f.write(buf.raw + b"\0")
+                at = _words_at(len(buf.raw))
+                f.write(buf.raw.ljust(at + 16, b"\0"))
                 f.flush()
-                self._opened_flag = C.c_char.from_buffer(mmap.mmap(f.fileno(), len(buf.raw) + 1), len(buf.raw))
+                self._shared_words = (C.c_uint64 * 2).from_buffer(mmap.mmap(f.fileno(), at + 16), at)
             os.replace(path + ".tmp", path)
             self._shm_file = path
             _PUBLISHED.add(path)
@@ -215,9 +223,9 @@ class IndexCache:
         if not ids.is_cuda and 0 < ids.numel() <= _STAGED:
             _check(ids.dtype == torch.int64, "ids.dtype == int64")
             with self._changing:  # the batch goes to the index in parts
-                flag = self._opened_flag
+                words = self._shared_words
                 return (_lib._NATIVE or _lib.native()).index_lookup(getattr(self._h, "value", 0), ids, self._device,
-                                                                     self.lookup_mode, 0 if flag is None else C.addressof(flag))
+                                                                     self.lookup_mode, 0 if words is None else C.addressof(words))
         dev = self._to_dev(ids)
         locs = torch.empty_like(dev)
         with self._changing:

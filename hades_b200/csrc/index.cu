@@ -6,6 +6,9 @@
 #include <cub/device/device_select.cuh>
 #include <cub/iterator/counting_input_iterator.cuh>
 
+#include <chrono>
+#include <thread>
+
 #include "index.cuh"
 #include "launch.cuh"
 #include "maintain.cuh"
@@ -281,7 +284,8 @@ __global__ void __launch_bounds__(kBlock) touch_after_kernel(const int64_t* __re
 
 __global__ void __launch_bounds__(kBlock) touch_apply_kernel(const int64_t* __restrict__ locs, int64_t first, int64_t n,
                                                              TouchMarks t, int32_t* __restrict__ after,
-                                                             int32_t* __restrict__ line_hits, int32_t* __restrict__ lru) {
+                                                             int32_t* __restrict__ line_hits, int32_t* __restrict__ lru,
+                                                             unsigned long long* aged, unsigned long long lookup) {
   const uint32_t number = batch_number(t.batch);
   for (int64_t i = first + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t slot = locs[i];
@@ -309,8 +313,13 @@ __global__ void __launch_bounds__(kBlock) touch_apply_kernel(const int64_t* __re
       }
     }
   }
-  batch_done(t.batch, number, gridDim.x);
+  if (batch_done(t.batch, number, gridDim.x) && aged) {  // (nullable: which batch of host ids this was)
+    __threadfence();
+    *reinterpret_cast<volatile unsigned long long*>(aged) = lookup;
+  }
 }
+
+__global__ void aged_kernel(unsigned long long* aged, unsigned long long lookup) { *aged = lookup; }
 
 // ---- LRU touch from runs -------------------------------------------------------
 // The batch is given as runs of equal ids (each run = the sorted batch positions
@@ -405,12 +414,14 @@ int grid_capped(int64_t n, int block = kBlock) {
 
 }  // namespace
 
-// the rest of the ageing by the marked positions first .. n
-static int age_marked(hb_index* h, const int64_t* locs, int64_t first, int64_t n, cudaStream_t st) {
+// the rest of the ageing by the marked positions first .. n; lookup: the batch of host ids that is complete then
+static int age_marked(hb_index* h, const int64_t* locs, int64_t first, int64_t n, cudaStream_t st,
+                      unsigned long long lookup = 0) {
   const int grid = grid_capped(n - first);
   const TouchMarks t = index_touch_marks(h);
   HB_LAUNCH(touch_after_kernel, grid, kBlock, 0, st, locs, first, n, t, h->after);
-  HB_LAUNCH(touch_apply_kernel, grid, kBlock, 0, st, locs, first, n, t, h->after, h->line_hits, h->lru);
+  HB_LAUNCH(touch_apply_kernel, grid, kBlock, 0, st, locs, first, n, t, h->after, h->line_hits, h->lru,
+            lookup ? h->aged : nullptr, lookup);
   return HB_OK;
 }
 
@@ -509,8 +520,7 @@ int alloc_derived(hb_index_t* h) {
   h->batch = h->line_hits + h->lines;
   device_error_word();  // (allocated on first use)
   HB_CUDA(cudaEventCreateWithFlags(&h->changed, cudaEventDisableTiming));
-  // (exported with the lines: a process that opens them begins behind the lookups before)
-  if (!h->opened) HB_CUDA(cudaEventCreateWithFlags(&h->aged, cudaEventDisableTiming | cudaEventInterprocess));
+  h->aged = reinterpret_cast<unsigned long long*>(h->lru + cap);
   HB_CUDA(cudaMalloc(&h->pairs, (cap + kLeafFan) * sizeof(longlong2)));
   HB_CUDA(cudaMalloc(&h->scratch_count, 4 * sizeof(int64_t)));
   // level capacities for a full index
@@ -536,7 +546,6 @@ struct IndexIpcHandle {
   int64_t lines;
   cudaIpcMemHandle_t line_ids;
   cudaIpcMemHandle_t lru;
-  cudaIpcEventHandle_t aged;
 };
 }  // namespace
 
@@ -551,7 +560,9 @@ int hb_index_create(int64_t cache_size, hb_index_t** out) {
   h->cache_size = lines * kWays;
   const int64_t cap = h->cache_size;
   HB_CUDA(cudaMalloc(&h->line_ids, cap * sizeof(int64_t)));
-  HB_CUDA(cudaMalloc(&h->lru, cap * sizeof(int32_t)));
+  // (and the word of the lookups, which an opener reads)
+  HB_CUDA(cudaMalloc(&h->lru, cap * sizeof(int32_t) + sizeof(unsigned long long)));
+  HB_CUDA(cudaMemsetAsync(h->lru + cap, 0, sizeof(unsigned long long), 0));
   int rc = alloc_derived(h);
   if (rc != HB_OK) return rc;
   HB_LAUNCH(fill_i64_kernel, grid_capped(cap), kBlock, 0, 0, h->line_ids, cap, (int64_t)-1);
@@ -577,7 +588,6 @@ int hb_index_export_handle(hb_index_t* h, void* handle_out) {
   x.lines = h->lines;
   HB_CUDA(cudaIpcGetMemHandle(&x.line_ids, h->line_ids));
   HB_CUDA(cudaIpcGetMemHandle(&x.lru, h->lru));
-  HB_CUDA(cudaIpcGetEventHandle(&x.aged, h->aged));
   memcpy(handle_out, &x, sizeof(x));
   return HB_OK;
 }
@@ -601,10 +611,6 @@ int hb_index_open(const void* handle, hb_index_t** out) {
   int rc = alloc_derived(h);
   if (rc != HB_OK) return rc;
   HB_CUDA(cudaStreamSynchronize(0));
-  cudaEvent_t creators;
-  HB_CUDA(cudaIpcOpenEventHandle(&creators, x.aged));
-  HB_CUDA(cudaEventSynchronize(creators));
-  HB_CUDA(cudaEventDestroy(creators));
   *out = h;
   return HB_OK;
 }
@@ -623,7 +629,6 @@ int hb_index_destroy(hb_index_t* h) {
   cudaFree(h->scratch_count);
   cudaFree(h->batch_scratch);
   if (h->changed) cudaEventDestroy(h->changed);
-  if (h->aged) cudaEventDestroy(h->aged);
   delete h;
   return HB_OK;
 }
@@ -759,13 +764,31 @@ int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_
   int rc = turn.on(st, true);  // (also behind a call that has found the parts and aged by them: locs may be freed)
   if (rc != HB_OK) return rc;
   const int64_t first = h->open_first;
+  const unsigned long long lookup = h->opened ? 0 : ++h->lookups;  // (the word is the creator's)
   if (h->open_locs == locs && h->open_end == n && first < n) {
     h->open_first = n;
-    rc = age_marked(h, locs, first, n, st);
-    if (rc != HB_OK) return rc;
+    return age_marked(h, locs, first, n, st, lookup);
   }
-  if (h->aged) HB_CUDA(cudaEventRecord(h->aged, st));
+  if (lookup) HB_LAUNCH(aged_kernel, 1, 1, 0, st, h->aged, lookup);
   return HB_OK;
+}
+
+uint64_t hb_index_lookups(const hb_index_t* h) { return h ? h->lookups : 0; }
+
+int hb_index_wait_lookups(hb_index_t* h, uint64_t lookups, hb_stream_t stream) {
+  HB_CHECK_ARG(h, "hb_index_wait_lookups: null index");
+  cudaStream_t st = (cudaStream_t)stream;
+  const auto until = std::chrono::steady_clock::now() + std::chrono::seconds(30);
+  for (;;) {
+    unsigned long long done = 0;
+    HB_CUDA(cudaMemcpyAsync(&done, h->aged, sizeof(done), cudaMemcpyDeviceToHost, st));
+    HB_CUDA(cudaStreamSynchronize(st));
+    if (done >= lookups) return HB_OK;
+    if (std::chrono::steady_clock::now() > until) break;
+    std::this_thread::sleep_for(std::chrono::microseconds(50));
+  }
+  set_error("hb_index_wait_lookups: the creator's lookups do not end");
+  return HB_ERR_TIMEOUT;
 }
 
 int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* perm,

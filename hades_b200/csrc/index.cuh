@@ -78,7 +78,8 @@ struct hb_index {
   unsigned long long changed_on;  // the id of its stream
   bool was_changed;
   bool unrecorded;                // ... on the default stream, which stays: recorded when another one has to wait
-  cudaEvent_t aged;               // interprocess: behind the last lookup of host ids
+  unsigned long long lookups;     // batches of host ids so far
+  unsigned long long* aged;       // behind lru on the device: the last of them whose ageing is done
   // a batch of host ids of which some parts are looked up: positions that wait for their ageing
   const int64_t* open_locs;
   int64_t open_first, open_end;
@@ -209,15 +210,18 @@ namespace hb {
 // One batch number for all blocks of a kernel, advanced by the block that finishes last (every block
 // has read it by then): counter[0] batches so far, counter[1] blocks done.
 __device__ __forceinline__ uint32_t batch_number(const int32_t* counter) { return (uint32_t)*counter + 1u; }
-__device__ __forceinline__ void batch_done(int32_t* counter, uint32_t number, int blocks) {
+// True in one thread of that block.
+__device__ __forceinline__ bool batch_done(int32_t* counter, uint32_t number, int blocks) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicAdd(reinterpret_cast<unsigned*>(counter + 1), 1u) == (unsigned)blocks - 1u) {
       counter[1] = 0;
       counter[0] = (int32_t)number;
+      return true;
     }
   }
+  return false;
 }
 #endif
 

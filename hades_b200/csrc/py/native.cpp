@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <atomic>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -230,12 +231,13 @@ at::Tensor pinned_empty(int64_t n) {
   return at::empty({n}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
 }
 
-// index_lookup(index, ids in host memory, device, mode, address of the flag of other processes | 0) -> slots in
-// host memory.  Ids and slots pass through two pinned buffers each, a part of the batch at a time: while the GPU
-// looks one part up the host copies the next in and the one before out, and the ageing runs under the last copies
-// and after.  Calls on the index from other streams wait for it; where another process has the lines too, which
-// can only be ordered by the host, the call does.  (The flag is read last: a process that sets it later waits for
-// the event of the lookups.)  500 ids: 26 us (two pageable copies: 70), 65,536: 99 (183).
+// index_lookup(index, ids in host memory, device, mode, address of two words shared with other processes | 0) ->
+// slots in host memory.  Ids and slots pass through two pinned buffers each, a part of the batch at a time: while
+// the GPU looks one part up the host copies the next in and the one before out, and the ageing runs under the last
+// copies and after.  Calls on the index from other streams wait for it; where another process has opened the index
+// (words[0]), which can only be ordered by the host, the call does.  A process that opens it later finds in words[1]
+// how many lookups to wait for: that is written before words[0] is read, so that one of the two waits.
+// 500 ids: 25 us (two pageable copies: 70), 65,536: 85 (183).
 PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
     arity(n_args, 5, "index_lookup");
@@ -273,8 +275,12 @@ PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     check(hb_index_lookup_touch_end(h, locs.data_ptr<int64_t>(), n, st));
     in_flight.looked_up = 0;
     for (int64_t k = parts < 2 ? 0 : parts - 2; k < parts; ++k) collect(k);
-    const volatile char* opened = static_cast<const volatile char*>(pointer(a[4]));
-    if (opened && *opened) {
+    volatile uint64_t* shared = static_cast<volatile uint64_t*>(pointer(a[4]));
+    if (shared) {
+      shared[1] = hb_index_lookups(h);
+      std::atomic_thread_fence(std::memory_order_seq_cst);
+    }
+    if (shared && shared[0]) {
       cudaError_t e;
       Py_BEGIN_ALLOW_THREADS;
       e = cudaStreamSynchronize(st);

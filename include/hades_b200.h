@@ -128,6 +128,10 @@ int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t*
 int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
                                int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream);
 int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream);
+/* Batches that hb_index_lookup_touch_end has ended in the creating process, and the wait of a process that has
+ * opened the index for the ageing by the first `lookups` of them (status HB_ERR_TIMEOUT after half a minute). */
+uint64_t hb_index_lookups(const hb_index_t* h);
+int hb_index_wait_lookups(hb_index_t* h, uint64_t lookups, hb_stream_t stream);
 
 /* The same LRU effect for a batch that is already grouped: run u holds the batch
  * positions perm[run_start[u] .. run_start[u+1]) (ascending) of ONE id, so all of
