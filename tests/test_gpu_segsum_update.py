@@ -91,3 +91,36 @@ def test_fewer_rows_than_ids_are_refused(cuda_lib, kind):
     with pytest.raises(RuntimeError, match="Check failed"):
         opt.update(torch.arange(20, device="cuda"), torch.ones((19, 8), device="cuda"))
     assert torch.equal(emb.weight, before)
+
+
+@pytest.mark.parametrize("kind", ["adam", "adagrad"])
+@pytest.mark.parametrize("senders,cap,merged", [(1, 40, True), (4, 700, True), (4, 1 << 17, True), (4, (1 << 17) + 1, False),
+                                                (5, 700, False)])
+def test_ascending_slabs_of_few_senders_are_merged(cuda_lib, monkeypatch, kind, senders, cap, merged):
+    """Merged or sorted, the update is that of the slabs as an unsorted list; slabs are empty, part full and full."""
+    from hades_b200 import sparse_optim
+    from hades_b200.sparse_optim import ShardedEmbedding, SparseAdagrad, SparseAdam
+
+    calls = []
+    merge = sparse_optim._merge_duplicates
+    monkeypatch.setattr(sparse_optim, "_merge_duplicates", lambda *a: (calls.append(1), merge(*a))[1])
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(cap)
+    dim, rows = 12, 2 * cap
+    opts = []
+    for _ in range(2):
+        emb = ShardedEmbedding(rows * senders, dim, 0, senders, init_sigma=0.01, seed=3)
+        opts.append((SparseAdam if kind == "adam" else SparseAdagrad)(emb, lr=LR))
+    ids = torch.zeros((senders, cap), dtype=torch.int64, device="cuda")
+    seg = torch.tensor([[cap, 0, cap // 3, 1, cap // 2][s] for s in range(senders)], device="cuda")
+    for s in range(senders):
+        ids[s] = (torch.randperm(rows, device="cuda", generator=gen)[:cap] * senders).sort().values
+    # values whose sums do not nearly cancel: the first updates of a row are lr * g / |g|
+    grads = (1 + torch.rand((senders * cap, dim), device="cuda", generator=gen)) * 1e-3
+    cnt = torch.randint(1, 5, (senders * cap,), device="cuda", generator=gen)
+    for opt, in_order in zip(opts, (True, False)):
+        opt.update(ids.flatten(), grads, cnt, seg_counts=seg, seg_cap=cap, sorted_segments=in_order, id_bits=32)
+    assert len(calls) == merged
+    # sums of up to five rows in another order: a unit or two of fp32
+    a, b = (o.emb.weight for o in opts)
+    assert float((a - b).abs().max()) < 1e-6 * LR + 2.0**-22 * float(b.abs().max())
