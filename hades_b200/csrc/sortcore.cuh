@@ -38,7 +38,9 @@ int* device_error_word();  // runtime.cu
 constexpr int kClusterT = 512;         // threads per CTA of the cluster version
 constexpr int kClusterDigit = 8;       // its bits per pass: counts are exchanged between all CTAs
 constexpr int kClusterMaxItems = 8;
-constexpr int64_t kSortClusterMax = 16 * (int64_t)kClusterT * kClusterMaxItems;  // its largest input
+// The cluster's largest input, and its line: it is ahead of the grid as far as its shared memory reaches (us,
+// cluster / grid, ids of 21 to 26 bits: 16,384 18-20 / 43-50, 32,768 22-25 / 44-47, 65,536 30-36 / 43-47).
+constexpr int64_t kSortClusterMax = 16 * (int64_t)kClusterT * kClusterMaxItems;
 constexpr int kGridT = 1024;           // threads per CTA of the grid version
 constexpr int kGridDigit = 10;
 constexpr int kGridBins = 1 << kGridDigit;

@@ -34,8 +34,10 @@ constexpr int kCold = 2;
 // Small batches update rows as their sums become complete (one launch); large ones write the sums and
 // update in a second pass over the distinct ids: the sums then run at the speed of the copy, and the
 // update has many rows in flight whatever the lengths of the runs.
-// The line lies where the two cost the same (65,536 ids of 128 columns: 149 us the step fused, 154 not;
-// 150,000 of 64: 167 and 162; 2,000,000 of 128: 903 and 846).
+// The line lies where the two cost the same, at much the same number of ids for all widths (us a step, Adam, at
+// once / in a second pass: 50,000 ids of 16 columns 88 / 92, of 64 96 / 107, of 128 109 / 125, of 256 136 / 159;
+// 100,000: 114 / 114, 131 / 140, 156 / 163, 208 / 217; 200,000: 143 / 137, 174 / 176, 207 / 205, 293 / 292;
+// 2,000,000 of 128: 903 / 846).
 // In a captured step the fetch runs beside the sums instead.
 constexpr int64_t kFuseMax = 100000;
 bool fuses_update(int64_t n) { return n <= kFuseMax; }
