@@ -35,6 +35,9 @@ from ._lib import LOOKUP_SETASSOC, LOOKUP_SORTED, MOVER_AUTO, MOVER_BULK, MOVER_
 # add 317 against 319) and beyond that faster.
 _STAGED = 1 << 17
 
+# Ids of one lookup() whose ageing goes with the lookup (hb_index_lookup_touch); more are sorted for it.
+_MARKED = 3 << 18
+
 _REGISTRY: dict[str, "IndexCache"] = {}
 
 
@@ -227,6 +230,10 @@ class IndexCache:
                 return (_lib._NATIVE or _lib.native()).index_lookup(getattr(self._h, "value", 0), ids, self._device,
                                                                      self.lookup_mode, 0 if words is None else C.addressof(words))
         dev = self._to_dev(ids)
+        if dev.numel() > _MARKED:
+            locs = self.cudalookup(dev)
+            self.cuda_touch_lru(locs)
+            return locs if ids.is_cuda else locs.cpu()
         locs = torch.empty_like(dev)
         with self._changing:
             _lib.check(self._lib.hb_index_lookup_touch(self._h, dev.data_ptr(), dev.numel(), locs.data_ptr(),

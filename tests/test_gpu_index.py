@@ -385,3 +385,29 @@ def test_ageing_from_two_threads(cuda_lib, oracle_mod, own):
     for q in host + [uniq[k % len(uniq)] for k in range(len(done))]:
         ora.lookup(q, touch=True)
     _same_state(ix, ora)
+
+
+@pytest.mark.parametrize("n", [786_432, 786_433, 1_000_003])
+def test_ageing_of_large_batches(cuda_lib, oracle_mod, n):
+    """Marks up to 786,432 positions, sorted by slot beyond; with a hot id and misses.  Without a workspace: marks."""
+    from hades_b200 import EmbCacheLib as E
+
+    rng = np.random.default_rng(n)
+    ix = E.IndexCache(50_000, f"large{n}", True, False)
+    ora = oracle_mod.OracleIndex(50_000)
+    first = rng.integers(0, 150_000, 60_000, dtype=np.int64)
+    assert np.array_equal(ix.add(torch.from_numpy(first)).numpy(), ora.add(first))
+    lib = E._lib.load()
+    assert (lib.hb_index_touch_lru_workspace_bytes(n) > 256) == (n > 786_432)
+    for rnd in range(3):
+        q = rng.integers(0, 150_000, n, dtype=np.int64)
+        q[rng.random(n) < 0.2] = first[-1]
+        want = ora.lookup(q, touch=True)
+        if rnd < 2:
+            got = ix.lookup(torch.from_numpy(q) if rnd else torch.from_numpy(q).cuda()).cpu().numpy()
+        else:
+            locs = ix.cudalookup(torch.from_numpy(q).cuda())
+            E._lib.check(lib.hb_index_touch_lru(ix.handle, locs.data_ptr(), n, None, 0, E._lib.stream_ptr()))
+            got = locs.cpu().numpy()
+        assert np.array_equal(got, want), rnd
+        _same_state(ix, ora, rnd)
