@@ -23,6 +23,7 @@ from __future__ import annotations
 
 import atexit
 import ctypes as C
+import mmap
 import threading
 
 import torch
@@ -150,7 +151,6 @@ class IndexCache:
 
     def _publish(self) -> None:
         """Leave the IPC handle, and the words shared with openers behind it, where other processes of the box find it."""
-        import mmap
         import os
 
         buf = C.create_string_buffer(self._lib.hb_index_handle_bytes())

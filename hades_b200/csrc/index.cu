@@ -596,19 +596,6 @@ namespace {
 // ageing keep between kernels (13.5 bytes a slot; with the index, so that every call may be captured)
 int alloc_derived(hb_index_t* h) {
   const int64_t cap = h->cache_size;
-  const size_t bytes = (size_t)cap * 12 + (size_t)h->lines * 12 + 8 * sizeof(int32_t);
-  HB_CUDA(cudaMalloc(&h->batch_scratch, bytes));
-  HB_CUDA(cudaMemsetAsync(h->batch_scratch, 0, bytes, 0));
-  h->marks = static_cast<unsigned long long*>(h->batch_scratch);
-  h->heads = h->marks + cap;
-  h->after = reinterpret_cast<int32_t*>(h->heads + h->lines);
-  h->line_hits = h->after + cap;
-  h->batch = h->line_hits + h->lines;
-  device_error_word();  // (allocated on first use)
-  HB_CUDA(cudaEventCreateWithFlags(&h->changed, cudaEventDisableTiming));
-  h->aged = reinterpret_cast<unsigned long long*>(h->lru + cap);
-  HB_CUDA(cudaMalloc(&h->pairs, (cap + kLeafFan) * sizeof(longlong2)));
-  HB_CUDA(cudaMalloc(&h->scratch_count, 4 * sizeof(int64_t)));
   // level capacities for a full index
   int64_t len = h->lines;  // level 1: one id per leaf block
   int64_t total = 0;
@@ -618,7 +605,24 @@ int alloc_derived(hb_index_t* h) {
     total += align_up(h->level_cap[l], 32);
     len = ceil_div(len, kNodeFan);
   }
-  HB_CUDA(cudaMalloc(&h->level_store, total * sizeof(int64_t)));
+  // one allocation for all of it: each costs an index some 0.1 to 1 ms, and again when it goes
+  const size_t pairs_bytes = align_up((cap + kLeafFan) * sizeof(longlong2), 256);
+  const size_t level_bytes = align_up(total * sizeof(int64_t), 256);
+  const size_t batch_bytes = align_up((size_t)cap * 12 + (size_t)h->lines * 12 + 8 * sizeof(int32_t), 256);
+  HB_CUDA(cudaMalloc(&h->batch_scratch, batch_bytes + pairs_bytes + level_bytes + 4 * sizeof(int64_t)));
+  HB_CUDA(cudaMemsetAsync(h->batch_scratch, 0, batch_bytes, 0));
+  h->marks = static_cast<unsigned long long*>(h->batch_scratch);
+  h->heads = h->marks + cap;
+  h->after = reinterpret_cast<int32_t*>(h->heads + h->lines);
+  h->line_hits = h->after + cap;
+  h->batch = h->line_hits + h->lines;
+  char* rest = static_cast<char*>(h->batch_scratch) + batch_bytes;
+  h->pairs = reinterpret_cast<longlong2*>(rest);
+  h->level_store = reinterpret_cast<int64_t*>(rest + pairs_bytes);
+  h->scratch_count = reinterpret_cast<int64_t*>(rest + pairs_bytes + level_bytes);
+  device_error_word();  // (allocated on first use)
+  HB_CUDA(cudaEventCreateWithFlags(&h->changed, cudaEventDisableTiming));
+  h->aged = reinterpret_cast<unsigned long long*>(h->lru + cap);
   h->sorted_stale = true;
   h->view.line_ids = h->line_ids;
   h->view.lines = h->lines;
@@ -710,10 +714,7 @@ int hb_index_destroy(hb_index_t* h) {
     cudaFree(h->line_ids);
     cudaFree(h->lru);
   }
-  cudaFree(h->pairs);
-  cudaFree(h->level_store);
-  cudaFree(h->scratch_count);
-  cudaFree(h->batch_scratch);
+  cudaFree(h->batch_scratch);  // (the sorted view's storage too)
   if (h->changed) cudaEventDestroy(h->changed);
   delete h;
   return HB_OK;
