@@ -1341,7 +1341,7 @@ def run_micro(update_only: bool) -> None:
         print(f"unique+segment-sum {qn:9s}               {ms * 1e3:8.1f} us")
         locs = ix.cudalookup(q)
         ms = _time(lambda: ix.cuda_touch_lru(locs))
-        print(f"LRU ageing by sort {qn:9s}               {ms * 1e3:8.1f} us")
+        print(f"LRU ageing of slots {qn:8s}               {ms * 1e3:8.1f} us")
         ms = _time(lambda: ix.cuda_touch_lru_runs(locs, runs))
         print(f"LRU ageing from runs {qn:9s}             {ms * 1e3:8.1f} us  (grouping taken from the step's sort)")
     print("device status", _lib.device_status())
