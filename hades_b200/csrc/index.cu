@@ -88,6 +88,7 @@ __device__ __forceinline__ void add_sorted_set(int j, int n, const uint2* kv, co
 }
 
 struct AddFinish {
+  static constexpr bool kOneEach = false;
   int64_t* line_ids;
   int32_t* lru;
   int64_t* locs;           // [n]

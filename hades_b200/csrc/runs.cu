@@ -12,6 +12,8 @@
 //                           the batch position whose output row holds their embedding
 //                           (the uncached cold ids sent to the server, dist_emb.py:218-259)
 // The backward aggregation (segsum.cu) and the LRU ageing (index.cu) take the same runs.
+#include <type_traits>
+
 #include "a2a.cuh"
 #include "compact.cuh"
 #include "index.cuh"
@@ -61,8 +63,11 @@ struct IdSource {
   }
 };
 
-// Runs of equal ids in the sorted order, numbered over all runs and inside the class of their id.
+// Runs of equal ids in the sorted order, numbered over all runs and inside the class of their id.  RESOLVE: each
+// is looked up where it is written.
+template <bool RESOLVE>
 struct RunsFinish {
+  static constexpr bool kOneEach = RESOLVE;
   const int8_t* table;   // nullable: no classes
   int64_t table_len;
   uint32_t* perm;        // [n]
@@ -79,8 +84,10 @@ struct RunsFinish {
   int64_t* class_counts2;
   int32_t* base8;        // [ceil(n / 8)] runs that start before entry 8k
   int64_t* n_valid;      // number of valid entries (read where the input is segmented or large)
-  unsigned* zero;        // nullable: words that the next launch needs at zero
+  unsigned* zero;        // nullable: words that `resolve` or the next launch needs at zero
   int zero_words;
+  struct Nothing {};
+  std::conditional_t<RESOLVE, RunsResolve, Nothing> resolve;
 
   // No runs and no entries: what works on the runs has nothing to do.  The sums go by the entries and do not
   // wait for a device count where the caller has none: they find one run of all entries and no id.
@@ -280,12 +287,11 @@ struct RunsFinish {
       }
       __syncthreads();
       const int runs = cta.x + cta.y + cta.z + cta.w;
-#pragma unroll 2
-      for (int r = threadIdx.x; r < runs; r += T) {
+      auto put = [&](int r, int64_t& id, bool& cold) {
         const uint32_t w = ctx.scratch[r];
         const uint32_t j = strip + (w & 8191u);
         const uint2 e = ctx.get(j);
-        const int64_t id = ctx.wide ? wide_id(e.y) : narrow_id(e.x);
+        id = ctx.wide ? wide_id(e.y) : narrow_id(e.x);
         const int u = before + r;
         uniq[u] = id;
         if (uniq2) uniq2[u] = id;
@@ -297,6 +303,23 @@ struct RunsFinish {
           dpos[u] = pos;
           int64_t* to = k == 0 ? out_ids[0] : (k == 1 ? out_ids[1] : (k == 2 ? out_ids[2] : nullptr));
           if (to) to[pos] = id;
+          cold = k == 2;
+        }
+      };
+      if constexpr (RESOLVE) {
+#pragma unroll 1
+        for (int r = threadIdx.x; r - lane < runs; r += T) {  // whole warps
+          int64_t id = -1;
+          bool cold = false;
+          if (r < runs) put(r, id, cold);
+          resolve_run(resolve, before + r, r < runs, id, cold);
+        }
+      } else {
+#pragma unroll 2
+        for (int r = threadIdx.x; r < runs; r += T) {
+          int64_t id;
+          bool cold;
+          put(r, id, cold);
         }
       }
       if (strips > 1) __syncthreads();
@@ -715,7 +738,7 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
                    int id_bits, const int8_t* class_table, int64_t table_len, int64_t* const* class_ids_out,
                    int64_t* class_counts_out, int64_t* uniq_ids_out, int64_t* num_unique_out, unsigned* zero,
                    int64_t zero_words, void* workspace, size_t workspace_bytes, hb_runs_t* runs_out,
-                   cudaStream_t st) {
+                   cudaStream_t st, const RunsResolve* resolve) {
   HB_CHECK_ARG(runs_out != nullptr, "hb_runs_build: runs_out is null");
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_runs_build: n out of range");
   HB_CHECK_ARG(n == 0 || ids, "hb_runs_build: null ids");
@@ -752,13 +775,30 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
   runs_out->perm = s.perm;
   IdSource src{ids, n, seg_counts ? nullptr : n_dev, seg_counts, (uint32_t)(seg_counts ? seg_cap : 1), sentinel,
                device_error_word(), id_bits};
-  RunsFinish fin{class_table, table_len, s.perm, s.head, s.uniq, uniq_ids_out, s.run_start,
-                 s.dclass, s.dpos,
-                 {class_ids_out ? class_ids_out[0] : nullptr, class_ids_out ? class_ids_out[1] : nullptr,
-                  class_ids_out ? class_ids_out[2] : nullptr},
-                 s.num_runs, num_unique_out, s.class_counts, class_counts_out, s.base8, s.n_valid, zero,
-                 (int)zero_words};
-  return sort_run(src, fin, n, s.sort_ws, st);
+  static_assert(kResolvedMax <= kSortOneEach, "one run per thread");
+  auto run = [&](auto fin) -> int {
+    fin.table = class_table;
+    fin.table_len = table_len;
+    fin.perm = s.perm;
+    fin.head = s.head;
+    fin.uniq = s.uniq;
+    fin.uniq2 = uniq_ids_out;
+    fin.run_start = s.run_start;
+    fin.dclass = s.dclass;
+    fin.dpos = s.dpos;
+    for (int c = 0; c < 3; ++c) fin.out_ids[c] = class_ids_out ? class_ids_out[c] : nullptr;
+    fin.num_runs = s.num_runs;
+    fin.num_runs2 = num_unique_out;
+    fin.class_counts = s.class_counts;
+    fin.class_counts2 = class_counts_out;
+    fin.base8 = s.base8;
+    fin.n_valid = s.n_valid;
+    fin.zero = zero;
+    fin.zero_words = (int)zero_words;
+    if constexpr (decltype(fin)::kOneEach) fin.resolve = *resolve;
+    return sort_run(src, fin, n, s.sort_ws, st);
+  };
+  return resolve ? run(RunsFinish<true>{}) : run(RunsFinish<false>{});
 }
 
 extern "C" {

@@ -38,6 +38,7 @@ int* device_error_word();  // runtime.cu
 constexpr int kClusterT = 512;         // threads per CTA of the cluster version
 constexpr int kClusterDigit = 8;       // its bits per pass: counts are exchanged between all CTAs
 constexpr int kClusterMaxItems = 8;
+constexpr int64_t kSortOneEach = 16 * (int64_t)kClusterT;  // ... with one entry per thread
 // The cluster's largest input, and its line: it is ahead of the grid as far as its shared memory reaches (us,
 // cluster / grid, ids of 21 to 26 bits: 16,384 18-20 / 43-50, 32,768 22-25 / 44-47, 65,536 30-36 / 43-47).
 constexpr int64_t kSortClusterMax = 16 * (int64_t)kClusterT * kClusterMaxItems;
@@ -873,14 +874,19 @@ int sort_run(const Src& src, const Fin& fin, int64_t n, void* ws, cudaStream_t s
   if (n <= 4 * kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 4, st);
   if (n <= 8 * kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 8, st);
   if (n <= 16 * kClusterT) return sort_launch_cluster<Src, Fin, 1>(src, fin, 16, st);
-  if (n <= 32 * kClusterT) return sort_launch_cluster<Src, Fin, 2>(src, fin, 16, st);
-  if (n <= 64 * kClusterT) return sort_launch_cluster<Src, Fin, 4>(src, fin, 16, st);
-  if (n <= kSortClusterMax) return sort_launch_cluster<Src, Fin, 8>(src, fin, 16, st);
-  const int64_t per = ceil_div(n, sort_grid_ctas(n));
-  if (per <= 2 * kGridT) return sort_launch_grid<Src, Fin, 2>(src, fin, n, kGridDigit, ws, st);
-  if (per <= 4 * kGridT) return sort_launch_grid<Src, Fin, 4>(src, fin, n, kGridDigit, ws, st);
-  if (per <= 8 * kGridT) return sort_launch_grid<Src, Fin, 8>(src, fin, n, kGridDigit, ws, st);
-  return sort_launch_grid<Src, Fin, 16>(src, fin, n, kGridDigit, ws, st);
+  if constexpr (Fin::kOneEach) {
+    set_error("a sort of %lld entries with one per thread", (long long)n);
+    return HB_ERR_INVALID;
+  } else {
+    if (n <= 32 * kClusterT) return sort_launch_cluster<Src, Fin, 2>(src, fin, 16, st);
+    if (n <= 64 * kClusterT) return sort_launch_cluster<Src, Fin, 4>(src, fin, 16, st);
+    if (n <= kSortClusterMax) return sort_launch_cluster<Src, Fin, 8>(src, fin, 16, st);
+    const int64_t per = ceil_div(n, sort_grid_ctas(n));
+    if (per <= 2 * kGridT) return sort_launch_grid<Src, Fin, 2>(src, fin, n, kGridDigit, ws, st);
+    if (per <= 4 * kGridT) return sort_launch_grid<Src, Fin, 4>(src, fin, n, kGridDigit, ws, st);
+    if (per <= 8 * kGridT) return sort_launch_grid<Src, Fin, 8>(src, fin, n, kGridDigit, ws, st);
+    return sort_launch_grid<Src, Fin, 16>(src, fin, n, kGridDigit, ws, st);
+  }
 }
 
 #endif  // __CUDACC__

@@ -42,6 +42,8 @@ constexpr int kCold = 2;
 constexpr int64_t kFuseMax = 100000;
 bool fuses_update(int64_t n) { return n <= kFuseMax; }
 
+constexpr int kListedWords = 64;  // of the counter, which all warps add to: a line of its own
+
 struct StepPlan {
   char* runs_ws;
   size_t runs_bytes;
@@ -53,8 +55,8 @@ struct StepPlan {
   uint8_t* on_list;      // [n] the run is a cold miss, to be inserted
   uint8_t* last_writer;  // [n]
   void* add_ws;          // index_add_runs_bytes: the lists' links first
+  unsigned long long* listed;  // [1], and behind it
   int32_t* chunk_listed; // [n / 32 + 1]
-  unsigned long long* listed;  // [1]
   char* seg_ws;
   size_t seg_bytes;
   float* sums;           // [n][dim], where the update is a launch of its own
@@ -75,8 +77,8 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
   p.on_list = cv.take<uint8_t>(m);
   p.last_writer = cv.take<uint8_t>(m);
   p.add_ws = cv.take<char>(index_add_runs_bytes(m));
-  p.chunk_listed = cv.take<int32_t>(m / 32 + 16);
-  p.listed = cv.take<unsigned long long>(1);
+  p.listed = cv.take<unsigned long long>(kListedWords / 2 + m / 64 + 8);
+  p.chunk_listed = reinterpret_cast<int32_t*>(p.listed) + kListedWords;
   p.seg_bytes = seg_plan(nullptr, m, dim).total;
   p.seg_ws = cv.take<char>(p.seg_bytes);
   p.sums = cv.take<float>((size_t)m * dim);
@@ -84,24 +86,9 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
   return p;
 }
 
-struct ResolveArgs {
-  const char* cache_rows;
-  const char* table;
-  int64_t table_rows;
-  int64_t row_bytes;
-  unsigned long long* run_src;
-  int64_t* run_slots;
-  uint8_t* on_list;       // nullable: misses are not inserted
-  uint8_t* last_writer;
-  int32_t* chunk_listed;
-  unsigned long long* listed;  // zero before
-  int push;               // ... onto the lists of their sets
-  int touch;
-};
-
+// The lookup of the runs in a launch of its own (resolve_run: as part of the sort's).
 template <int MODE>
-__global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_runs_t r, ResolveArgs a, TouchMarks marks,
-                                                              AddLists lists, int* __restrict__ err) {
+__global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_runs_t r, RunsResolve a) {
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -113,31 +100,9 @@ __global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_ru
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
     const int64_t u = u0 + lane;
-    const bool valid = u < U;
-    const int64_t id = valid ? __ldg(r.uniq_ids + u) : -1;
-    const bool cold = valid && a.on_list && r.dclass[u] == kCold;
-    const int64_t slot = warp_lookup<MODE>(v, s_top, id);
-    const bool missed = cold && slot < 0;
-    if (a.on_list) {
-      const unsigned m = __ballot_sync(0xffffffffu, missed);
-      if (lane == 0) {
-        a.chunk_listed[u0 >> 5] = __popc(m);
-        if (m) atomicAdd(a.listed, (unsigned long long)__popc(m));
-      }
-      if (valid) {
-        a.on_list[u] = missed;
-        a.last_writer[u] = 0;
-      }
-      if (missed && a.push) lists.push(id, u);
-    }
-    if (!valid) continue;
-    const char* src = nullptr;
-    if (slot >= 0) src = a.cache_rows + slot * a.row_bytes;
-    else if (id < a.table_rows) src = a.table + id * a.row_bytes;
-    else atomicExch(err, HB_ERR_INVALID);  // no such row: the output rows of the run stay as they were
-    a.run_src[u] = (unsigned long long)src | (slot >= 0 ? 1ull : 0ull);
-    a.run_slots[u] = slot;
-    if (a.touch) marks.mark(slot, u);
+    const int64_t id = u < U ? __ldg(r.uniq_ids + u) : -1;
+    const bool cold = u < U && r.dclass[u] == kCold;
+    resolved_run<true>(a, u, u < U, id, cold, warp_lookup<MODE>(v, s_top, id));
   }
 }
 
@@ -371,11 +336,11 @@ bool vec4_ok(const hb_step_desc_t* d, const float* grads) {
 }
 
 int build_runs(hb_step* s, const hb_step_desc_t* d, const StepPlan& p, const int64_t* ids, int64_t n,
-               int64_t* counters, cudaStream_t st) {
+               int64_t* counters, cudaStream_t st, const RunsResolve* resolve = nullptr) {
   static_assert(sizeof(unsigned long long) == 2 * sizeof(unsigned), "the list counter is zeroed as two words");
   const int rc = runs_build(ids, n, nullptr, nullptr, 0, d->id_bits, d->class_table, d->class_len, nullptr,
-                            counters + 1, nullptr, counters, reinterpret_cast<unsigned*>(p.listed), 2, p.runs_ws,
-                            p.runs_bytes, &s->runs, st);
+                            counters + 1, nullptr, counters, reinterpret_cast<unsigned*>(p.listed),
+                            resolve ? kListedWords + n / 32 + 1 : 2, p.runs_ws, p.runs_bytes, &s->runs, st, resolve);
   s->runs_n = rc == HB_OK ? n : 0;
   return rc;
 }
@@ -442,38 +407,38 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
     rc = hb_index_build_sorted(h, stream);
     if (rc != HB_OK) return rc;
   }
-  const TouchMarks marks = index_touch_marks(h);
-  const AddLists lists = index_add_lists(h, static_cast<uint32_t*>(p.add_ws));
-  rc = build_runs(s, d, p, ids, n, counters, st);
-  if (rc != HB_OK) return rc;
+  const bool lists_used = d->insert_misses && index_add_runs_lists(h, n);
+  const RunsResolve a{h->line_ids, h->lines, (const char*)d->cache_rows, (const char*)d->table, d->table_rows, d->row_bytes,
+                      static_cast<unsigned long long*>(p.fetch_ws), p.run_slots, d->insert_misses ? p.on_list : nullptr,
+                      p.last_writer, p.chunk_listed, p.listed, lists_used, d->touch_lru, index_touch_marks(h),
+                      index_add_lists(h, static_cast<uint32_t*>(p.add_ws)), device_error_word()};
   // aside: all of the fetch leaves the caller's stream, which goes on to the aggregation of the
   // same batch (it needs the sort only); both are bound by HBM, but not all the time
   const bool aside = aside_allowed && (captured(st) || !fuses_update(n));
+  const bool in_sort = !aside && n <= kResolvedMax && d->lookup_mode == HB_LOOKUP_SETASSOC;
+  IndexTurn turn(h);
+  if (in_sort) rc = turn.on(st);
+  if (rc == HB_OK) rc = build_runs(s, d, p, ids, n, counters, st, in_sort ? &a : nullptr);
+  if (rc != HB_OK) return rc;
   if (aside) {
     HB_CUDA(cudaEventRecord(s->forked, st));
     HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
     st = s->side;
   }
-  IndexTurn turn(h);
-  rc = turn.on(st);
-  if (rc != HB_OK) return rc;
-  const ResolveArgs a{(const char*)d->cache_rows, (const char*)d->table, d->table_rows, d->row_bytes,
-                      static_cast<unsigned long long*>(p.fetch_ws), p.run_slots,
-                      d->insert_misses ? p.on_list : nullptr, p.last_writer, p.chunk_listed, p.listed,
-                      index_add_runs_lists(h, n), d->touch_lru};
-  if (d->lookup_mode == HB_LOOKUP_SORTED)
-    HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SORTED>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a, marks, lists,
-              device_error_word());
-  else
-    HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a, marks,
-              lists, device_error_word());
+  if (!in_sort) {
+    rc = turn.on(st);
+    if (rc != HB_OK) return rc;
+    if (d->lookup_mode == HB_LOOKUP_SORTED)
+      HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SORTED>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a);
+    else
+      HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a);
+  }
   Maintain m;
   memset(&m, 0, sizeof(m));
-  const bool lists_used = d->insert_misses && index_add_runs_lists(h, n);
   if (lists_used) h->sorted_stale = true;  // (ageing leaves the ids where they are)
   if (d->touch_lru || lists_used) {
     m.v = RunsView{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
-    m.marks = marks;
+    m.marks = a.marks;
     m.e = AddEntries{s->runs.uniq_ids, n, s->runs.num_runs, p.on_list, p.chunk_listed, p.listed, d->miss_cap};
     m.add = index_add_state(h, static_cast<uint32_t*>(p.add_ws), p.new_slots, p.last_writer);
     m.touch = d->touch_lru;

@@ -172,3 +172,12 @@ def test_rows_of_odd_width_as_composed(cuda_lib, dim, optimizer):
     """Columns one by one: counts and bias corrections divide in both forms."""
     a, b = _pair(f"odd_{dim}_{optimizer}", dim=dim, optimizer=optimizer)
     _run_pair(a, b, _steps(_small("odd", dim), 7))
+
+
+@pytest.mark.parametrize("n", [1, 33, 513, 8191, 8192, 8193])
+def test_runs_looked_up_in_the_launch_of_the_sort(cuda_lib, n):
+    """Up to 8,192 ids a run is looked up where the sort writes it, above in a launch of its own; the runs of a warp
+    lie in two chunks of 32, whose counts cut the list of misses (miss_cap)."""
+    a, b = _pair(f"resolve_{n}")
+    a.miss_cap = b.miss_cap = max(n // 8, 1)
+    _run_pair(a, b, [(ids[:n], g[:n]) for ids, g in _steps(_small("resolve", batch=8193), 4, seed=n)])
