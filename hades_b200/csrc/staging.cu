@@ -403,34 +403,88 @@ __global__ void __launch_bounds__(kBlock) staging_flush_move_kernel(
 }
 
 // ---- insert (server.py:499-544): rows into the cache buffer at the slots add() gave ----------
-template <int VEC_BYTES>
-__global__ void __launch_bounds__(kBlock) staging_insert_kernel(
+// Bound by row traffic: a row read, a cache row and a staging row written, all at random places.  Of a warp's 32
+// entries a part has a row to move (of the distinct ids of a batch some 30 to 45 per cent); moved where they stand,
+// four of 32 at a time, one or two rows of a warp were on their way together.  So the warp closes the gaps first.
+// (512-byte rows, us: 700 of 2,000 entries 4.9 -> 3.0, 20,000 8.0 -> 6.2, 76,000 of 227,000 33.3 -> 28.9, 4.0 TB/s;
+// 100,000 of 100,000 36.3 -> 33.2, 4.6 TB/s.)
+
+// `rows` rows of vpr 16-byte vectors, lane r holds those of row r: copied (or zeroed where SRC is false)
+template <bool SRC>
+__device__ __forceinline__ void warp_put_rows(unsigned long long src, unsigned long long dst, int rows, int vpr) {
+  constexpr int kFly = 8;
+  const int lane = lane_id();
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  int glog2 = 5;
+  while (glog2 > 0 && (1 << (glog2 - 1)) >= vpr) --glog2;
+  const int rpp = 32 >> glog2, sub = lane & ((1 << glog2) - 1), which = lane >> glog2;
+  for (int q0 = 0; q0 < rows; q0 += kFly * rpp) {
+    for (int k0 = 0; k0 < vpr; k0 += 32) {
+      const int k = k0 + sub;
+      uint4 v[kFly];
+      if (SRC) {
+#pragma unroll
+        for (int x = 0; x < kFly; ++x) {
+          const int q = q0 + x * rpp + which;
+          const unsigned long long from = __shfl_sync(0xffffffffu, src, q & 31);
+          if (q < rows && k < vpr) v[x] = __ldg(reinterpret_cast<const uint4*>(from) + k);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < kFly; ++x) {
+        const int q = q0 + x * rpp + which;
+        const unsigned long long to = __shfl_sync(0xffffffffu, dst, q & 31);
+        if (q < rows && k < vpr) reinterpret_cast<uint4*>(to)[k] = SRC ? v[x] : zero;
+      }
+    }
+  }
+}
+
+// VEC_BYTES of a cached row; ZERO16: staging rows are zeroed in vectors of 16 bytes
+template <int VEC_BYTES, bool ZERO16>
+__global__ void __launch_bounds__(kBlock, 4) staging_insert_kernel(
     hb_staging_t s, const int64_t* __restrict__ locs, const uint8_t* __restrict__ last_writer,
     const char* __restrict__ emb_rows, const int64_t* __restrict__ row_index,
     char* __restrict__ cache_rows, int64_t row_bytes, int64_t n, const int64_t* __restrict__ n_dev, int per) {
+  __shared__ uint8_t s_at[kBlock / 32][32];
   n = effective_n(n, n_dev);
   const int lane = lane_id();
+  uint8_t* const mine = s_at[threadIdx.x >> 5];
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t base = warp * per; base < n; base += nwarps * per) {
     const int64_t i = lane < per ? base + lane : n;
+    const int64_t loc = i < n ? __ldg(locs + i) : -1;
+    const int64_t row = i < n && row_index ? __ldg(row_index + i) : i;  // row of entry i in emb_rows
     // of several ids that received the same slot, the last of the batch writes it
-    const int64_t slot = (i < n && last_writer[i]) ? __ldg(locs + i) : -1;
-    const bool ok = slot >= 0;
-    if (ok && s.cnt) {
-      s.cnt[slot] = 0;   // server.py:539-541
-      s.idx[slot] = -1;
+    const bool ok = i < n && last_writer[i] && loc >= 0;
+    const unsigned act = __ballot_sync(0xffffffffu, ok);
+    if (act == 0u) continue;
+    const int rows = __popc(act);
+    if (ok) {
+      if (s.cnt) {
+        s.cnt[loc] = 0;   // server.py:539-541
+        s.idx[loc] = -1;
+      }
+      mine[__popc(act & ((1u << lane) - 1u))] = (uint8_t)lane;
     }
-    const int64_t from = (ok && row_index) ? __ldg(row_index + i) : i;  // row of entry i in emb_rows
-    warp_move_rows(emb_rows + from * row_bytes, cache_rows + (ok ? slot : 0) * row_bytes, ok, row_bytes,
-                   VEC_BYTES);
-    if (s.grad) {
-      const unsigned act = __ballot_sync(0xffffffffu, ok);
-      for (int q = 0; q < 32; ++q) {
-        if (!((act >> q) & 1u)) continue;
-        const int64_t sq = __shfl_sync(0xffffffffu, slot, q);
-        float* row = s.grad + sq * s.dim;
-        for (int64_t k = lane; k < s.dim; k += 32) row[k] = 0.f;
+    __syncwarp();
+    const int at = lane < rows ? mine[lane] : 0;  // the lane whose row this one holds from here on
+    __syncwarp();
+    const int64_t slot = __shfl_sync(0xffffffffu, loc, at);
+    const char* src = emb_rows + __shfl_sync(0xffffffffu, row, at) * row_bytes;
+    char* dst = cache_rows + slot * row_bytes;
+    if (VEC_BYTES == 16)
+      warp_put_rows<true>((unsigned long long)src, (unsigned long long)dst, rows, (int)(row_bytes >> 4));
+    else
+      warp_move_rows(src, dst, lane < rows, row_bytes, VEC_BYTES);
+    if (!s.grad) continue;
+    if (ZERO16) {
+      warp_put_rows<false>(0ull, (unsigned long long)(s.grad + slot * s.dim), rows, (int)(s.dim >> 2));
+    } else {
+      for (int q = 0; q < rows; ++q) {
+        float* to = s.grad + __shfl_sync(0xffffffffu, slot, q) * s.dim;
+        for (int64_t k = lane; k < s.dim; k += 32) to[k] = 0.f;
       }
     }
   }
@@ -630,15 +684,18 @@ int hb::staging_insert_rows(const hb_staging_t* s, const void* emb_rows, const i
   memset(&none, 0, sizeof(none));
   const hb_staging_t st_desc = s ? *s : none;
   const int vb = payload_vec_bytes(row_bytes, emb_rows, cache_rows);
+  const bool zero16 = st_desc.dim % 4 == 0 && ((uintptr_t)st_desc.grad & 15) == 0;
   const int per = items_per_warp(n);
-  if (vb == 16)
-    HB_LAUNCH(staging_insert_kernel<16>, grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, last_writer,
-              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per);
-  else if (vb == 4)
-    HB_LAUNCH(staging_insert_kernel<4>, grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, last_writer,
-              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per);
-  else
-    HB_LAUNCH(staging_insert_kernel<1>, grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, last_writer,
-              (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per);
+#define HB_INSERT(VB, Z16)                                                                                     \
+  HB_LAUNCH((staging_insert_kernel<VB, Z16>), grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, \
+            last_writer, (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per)
+  if (vb == 16) {
+    if (zero16) HB_INSERT(16, true); else HB_INSERT(16, false);
+  } else if (vb == 4) {
+    if (zero16) HB_INSERT(4, true); else HB_INSERT(4, false);
+  } else {
+    if (zero16) HB_INSERT(1, true); else HB_INSERT(1, false);
+  }
+#undef HB_INSERT
   return HB_OK;
 }
