@@ -55,10 +55,12 @@ struct StepPlan {
   uint8_t* on_list;      // [n] the run is a cold miss, to be inserted
   uint8_t* last_writer;  // [n]
   void* add_ws;          // index_add_runs_bytes: the lists' links first
-  unsigned long long* listed;  // [1], and behind it
+  // what the sort's launch sets to zero
+  unsigned* zero;
+  int64_t zero_words;
+  unsigned long long* listed;  // [1]
   int32_t* chunk_listed; // [n / 32 + 1]
-  char* seg_ws;
-  size_t seg_bytes;
+  SegPlan seg;           // its arrival counters among the zeroed words
   float* sums;           // [n][dim], where the update is a launch of its own
   size_t total;
 };
@@ -77,10 +79,14 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
   p.on_list = cv.take<uint8_t>(m);
   p.last_writer = cv.take<uint8_t>(m);
   p.add_ws = cv.take<char>(index_add_runs_bytes(m));
-  p.listed = cv.take<unsigned long long>(kListedWords / 2 + m / 64 + 8);
-  p.chunk_listed = reinterpret_cast<int32_t*>(p.listed) + kListedWords;
-  p.seg_bytes = seg_plan(nullptr, m, dim).total;
-  p.seg_ws = cv.take<char>(p.seg_bytes);
+  const SegPlan sizes = seg_plan(nullptr, m, dim);
+  const int64_t chunks = m / 32 + 1;
+  p.zero_words = kListedWords + chunks + sizes.max_ctas;
+  p.zero = cv.take<unsigned>(p.zero_words);
+  p.listed = reinterpret_cast<unsigned long long*>(p.zero);
+  p.chunk_listed = reinterpret_cast<int32_t*>(p.zero + kListedWords);
+  p.seg = seg_plan(cv.take<char>(sizes.total), m, dim);
+  p.seg.done = p.zero + kListedWords + chunks;
   p.sums = cv.take<float>((size_t)m * dim);
   p.total = cv.used() + 256;
   return p;
@@ -130,79 +136,71 @@ struct ColdArgs {
   int touch;
 };
 
-// The cold ids among 32 distinct ones (a lane each): slot now that this batch's misses are in the
-// cache, staging entry (server.py:546-562 without the row), mark for the ageing.
+// The cold ids: slot now that this batch's misses are in the cache, staging entry (server.py:546-562 without the
+// row), mark for the ageing.
 template <int MODE>
-__device__ __forceinline__ int64_t cold_entry(const IndexView& v, const int64_t* s_top, const ColdArgs& a, int64_t u,
-                                              bool cold, int64_t id) {
-  const int64_t slot = warp_lookup<MODE>(v, s_top, cold ? id : -1);
-  if (slot >= 0) {
-    a.s.idx[slot] = id;
-    a.s.iter_threshold[slot] = a.thr_table ? __ldg(a.thr_table + id) : a.default_thr;
-    a.s.cnt[slot] += 1;
-    if (a.touch) a.marks.mark(slot, u);
-  }
-  if (a.dropped) {
-    const unsigned miss = __ballot_sync(0xffffffffu, cold && slot < 0);
-    if (lane_id() == 0 && miss) atomicAdd(a.dropped, (unsigned long long)__popc(miss));
-  }
-  return slot;
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_t r, ColdArgs a,
-                                                           unsigned* __restrict__ zero, int64_t zero_words) {
+__global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_t r, ColdArgs a) {
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
     __syncthreads();
   }
-  // the aggregation that follows needs its arrival counters at zero
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < zero_words; k += (int64_t)gridDim.x * blockDim.x)
-    zero[k] = 0u;
   const int64_t U = *r.num_runs;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
     const int64_t u = u0 + lane_id();
     const bool cold = u < U && r.dclass[u] == kCold;
-    const int64_t slot = cold_entry<MODE>(v, s_top, a, u, cold, cold ? __ldg(r.uniq_ids + u) : -1);
+    const int64_t id = cold ? __ldg(r.uniq_ids + u) : -1;
+    const int64_t slot = warp_lookup<MODE>(v, s_top, id);
+    if (slot >= 0) {
+      a.s.idx[slot] = id;
+      a.s.iter_threshold[slot] = a.thr_table ? __ldg(a.thr_table + id) : a.default_thr;
+      a.s.cnt[slot] += 1;
+      if (a.touch) a.marks.mark(slot, u);
+    }
+    if (a.dropped) {
+      const unsigned miss = __ballot_sync(0xffffffffu, cold && slot < 0);
+      if (lane_id() == 0 && miss) atomicAdd(a.dropped, (unsigned long long)__popc(miss));
+    }
     if (u < U) a.slots[u] = slot;
   }
 }
 
-// Summed gradients to where they belong: state and table rows of hot ids, staging rows of cold ones.  A
-// warp takes 32 distinct ids, a lane each for what is worked out once per id, then G lanes per row and
-// kFly rows in flight.  Bound by HBM: rows read and written once (175,000 ids of 128 columns: 60 us).
-template <int MODE, bool ADAM, int VEC, int G, int VPL>
-__global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(IndexView v, hb_runs_t r, ColdArgs c,
-                                                                            SegArgs a, UpdateRows<ADAM, true> epi,
+// Summed gradients to where they belong: state and table rows of hot ids, staging rows of cold ones; meanwhile LRU
+// ageing by the lookup that found the staging rows.  A warp takes 32 distinct ids, a lane each for what is worked
+// out once per id, then G lanes per row and kFly rows in flight.  Bound by HBM: rows read and written once.  (With the
+// lookup of the cold ids in it and the ageing behind it: 85,000 hot and 76,000 cold ids of 128 columns for Adam 99 + 12
+// us, now 95; 88,000 and 80,000 118 + 14, now 103.)
+template <bool ADAM, int VEC, int G, int VPL>
+__global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(hb_runs_t r, SegArgs a,
+                                                                            UpdateRows<ADAM, true> epi,
                                                                             const float* __restrict__ sums) {
   using V = typename VecF<VEC>::T;
   using Ops = EpiOps<UpdateRows<ADAM, true>, VEC, G, VPL>;
   constexpr int kFly = VPL > 1 ? 1 : 2;
   constexpr int RPP = 32 / G;
-  __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
-  if (MODE == HB_LOOKUP_SORTED) {
-    stage_top_level(v, s_top);
-    __syncthreads();
+  int block = blockIdx.x;
+  if (block < epi.touch_blocks) {
+    touch_runs(epi.touched, epi.marks, epi.lru, block, epi.touch_blocks);
+    return;
   }
+  block -= epi.touch_blocks;
   const int64_t U = *r.num_runs;
   const int lane = lane_id();
   const int sub = lane & (G - 1), which = lane / G;
   const int vpr = a.cols / VEC;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t warp = (block * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)(gridDim.x - epi.touch_blocks) * blockDim.x) >> 5;
   for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
     const int64_t u = u0 + lane;
-    const bool valid = u < U;
-    const int cls = valid ? r.dclass[u] : -1;
-    const int64_t id = valid ? __ldg(r.uniq_ids + u) : -1;
-    const int64_t slot = cold_entry<MODE>(v, s_top, c, u, cls == kCold, id);
-    if (valid) c.slots[u] = slot;
-    const typename Ops::Lane mine = Ops::lane_of_class(epi, cls, id, slot);
+    typename Ops::Lane mine;
     int count = 0;
-    if (valid) count = (int)(__ldg(r.run_start + u + 1) - __ldg(r.run_start + u));
+    if (u < U) {
+      const int64_t begin = __ldg(r.run_start + u), end = __ldg(r.run_start + u + 1);
+      mine = Ops::lane_of_class(epi, r.dclass[u], __ldg(r.uniq_ids + u), __ldg(epi.slots + u));
+      count = (int)(end - begin);
+    }
     const int rows = U - u0 < 32 ? (int)(U - u0) : 32;
     for (int t0 = 0; t0 < rows; t0 += RPP * kFly) {
       V acc[kFly][VPL];
@@ -228,14 +226,14 @@ __global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(Ind
   }
 }
 
-template <int MODE, bool ADAM, int VEC>
-int launch_apply(const IndexView& v, const hb_runs_t& r, const ColdArgs& c, const SegArgs& a,
-                 const UpdateRows<ADAM, true>& epi, const float* sums, cudaStream_t st) {
+template <bool ADAM, int VEC>
+int launch_apply(const hb_runs_t& r, const SegArgs& a, const UpdateRows<ADAM, true>& epi, const float* sums,
+                 cudaStream_t st) {
   const int vpr = a.cols / VEC;
   int64_t blocks = ceil_div(r.n, kBlock);
   if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
-#define HB_APPLY(G, VPL)                                                                                      \
-  HB_LAUNCH((step_apply_kernel<MODE, ADAM, VEC, G, VPL>), (int)blocks, kBlock, 0, st, v, r, c, a, epi, sums)
+  blocks += epi.touch_blocks;
+#define HB_APPLY(G, VPL) HB_LAUNCH((step_apply_kernel<ADAM, VEC, G, VPL>), (int)blocks, kBlock, 0, st, r, a, epi, sums)
   if (vpr > 64) HB_APPLY(32, 4);
   else if (vpr > 32) HB_APPLY(32, 2);
   else if (vpr > 16) HB_APPLY(32, 1);
@@ -246,61 +244,61 @@ int launch_apply(const IndexView& v, const hb_runs_t& r, const ColdArgs& c, cons
   return HB_OK;
 }
 
-template <bool ADAM>
-int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs a, bool vec4, float* sums,
-                const SegPlan& seg, bool fused, cudaStream_t st) {
-  const hb_runs_t& r = s->runs;
-  auto epi = update_rows<ADAM, true>(&r, &d->opt);
-  epi.dclass = r.dclass;
-  epi.staged = d->staging.grad;
-  epi.slots = c.slots;
-  // the lookup of the accumulate: every distinct cold id once, in ascending order
-  const RunsView touched{c.slots, nullptr, nullptr, r.num_runs, r.num_runs, r.n, r.n, 2};
-  const IndexView& v = d->index->view;
-  const bool sorted = d->lookup_mode == HB_LOOKUP_SORTED;
-  IndexTurn turn(d->index);
-  if (fused) {
-    int rc = turn.on(st);
-    if (rc != HB_OK) return rc;
-    int64_t blocks = ceil_div(r.n, kBlock);
-    if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-    if (sorted)
-      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SORTED>, (int)blocks, kBlock, 0, st, v, r, c, seg.done, seg.max_ctas);
-    else
-      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SETASSOC>, (int)blocks, kBlock, 0, st, v, r, c, seg.done, seg.max_ctas);
-    if (d->touch_lru) {
-      epi.touch_blocks = (int)blocks;
-      epi.touched = touched;
-      epi.marks = c.marks;
-      epi.lru = d->index->lru;
-    }
-    return seg_dispatch(a, epi, vec4, st);
-  }
-  HB_CUDA(cudaMemsetAsync(seg.done, 0, (size_t)seg.max_ctas * sizeof(unsigned), st));
-  StoreRows store;
-  memset(&store, 0, sizeof(store));
-  store.sums = sums;
-  int rc = seg_dispatch(a, store, vec4, st);
-  if (rc != HB_OK) return rc;
-  // from here on the fetch of this batch must have read its rows and the cache hold its misses
-  rc = join_side(s, st);
-  if (rc == HB_OK) rc = turn.on(st);
-  if (rc != HB_OK) return rc;
-  if (sorted)
-    rc = vec4 ? launch_apply<HB_LOOKUP_SORTED, ADAM, 4>(v, r, c, a, epi, sums, st)
-              : launch_apply<HB_LOOKUP_SORTED, ADAM, 1>(v, r, c, a, epi, sums, st);
-  else
-    rc = vec4 ? launch_apply<HB_LOOKUP_SETASSOC, ADAM, 4>(v, r, c, a, epi, sums, st)
-              : launch_apply<HB_LOOKUP_SETASSOC, ADAM, 1>(v, r, c, a, epi, sums, st);
-  if (rc != HB_OK || !d->touch_lru) return rc;
-  return index_touch_apply(d->index, touched, st);
-}
-
 int grid_for_runs(int64_t n) {
   int64_t blocks = ceil_div(n, kBlock);
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   return blocks < 1 ? 1 : (int)blocks;
+}
+
+template <bool ADAM>
+int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs a, bool vec4, float* sums, bool fused,
+                cudaStream_t st) {
+  const hb_runs_t& r = s->runs;
+  auto epi = update_rows<ADAM, true>(&r, &d->opt);
+  epi.dclass = r.dclass;
+  epi.staged = d->staging.grad;
+  epi.slots = c.slots;
+  if (d->touch_lru) {
+    epi.touch_blocks = grid_for_runs(r.n);
+    // the lookup of the accumulate: every distinct cold id once, in ascending order
+    epi.touched = RunsView{c.slots, nullptr, nullptr, r.num_runs, r.num_runs, r.n, r.n, 2};
+    epi.marks = c.marks;
+    epi.lru = d->index->lru;
+  }
+  IndexTurn turn(d->index);
+  auto look_up = [&](cudaStream_t on) -> int {
+    const int rc = turn.on(on);
+    if (rc != HB_OK) return rc;
+    const IndexView& v = d->index->view;
+    if (d->lookup_mode == HB_LOOKUP_SORTED)
+      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SORTED>, grid_for_runs(r.n), kBlock, 0, on, v, r, c);
+    else
+      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(r.n), kBlock, 0, on, v, r, c);
+    return HB_OK;
+  };
+  if (fused) {
+    const int rc = look_up(st);
+    return rc != HB_OK ? rc : seg_dispatch(a, epi, vec4, st);
+  }
+  // The sums need the sort only.  Beside them, once the cache holds the misses of this batch: where the cold ids are.
+  if (!s->side_busy) {
+    HB_CUDA(cudaEventRecord(s->forked, st));
+    HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
+  }
+  int rc = look_up(s->side);
+  if (rc != HB_OK) return rc;
+  HB_CUDA(cudaEventRecord(s->fetched, s->side));
+  s->side_busy = true;
+  StoreRows store;
+  memset(&store, 0, sizeof(store));
+  store.sums = sums;
+  rc = seg_dispatch(a, store, vec4, st);
+  // from here on the fetch of this batch must have read its rows
+  if (rc == HB_OK) rc = join_side(s, st);
+  if (rc == HB_OK) rc = turn.on(st);
+  if (rc != HB_OK) return rc;
+  return vec4 ? launch_apply<ADAM, 4>(r, a, epi, sums, st) : launch_apply<ADAM, 1>(r, a, epi, sums, st);
 }
 
 int check_desc(const hb_step_desc_t* d, const char* who) {
@@ -337,10 +335,8 @@ bool vec4_ok(const hb_step_desc_t* d, const float* grads) {
 
 int build_runs(hb_step* s, const hb_step_desc_t* d, const StepPlan& p, const int64_t* ids, int64_t n,
                int64_t* counters, cudaStream_t st, const RunsResolve* resolve = nullptr) {
-  static_assert(sizeof(unsigned long long) == 2 * sizeof(unsigned), "the list counter is zeroed as two words");
   const int rc = runs_build(ids, n, nullptr, nullptr, 0, d->id_bits, d->class_table, d->class_len, nullptr,
-                            counters + 1, nullptr, counters, reinterpret_cast<unsigned*>(p.listed),
-                            resolve ? kListedWords + n / 32 + 1 : 2, p.runs_ws, p.runs_bytes, &s->runs, st, resolve);
+                            counters + 1, nullptr, counters, p.zero, p.zero_words, p.runs_ws, p.runs_bytes, &s->runs, st, resolve);
   s->runs_n = rc == HB_OK ? n : 0;
   return rc;
 }
@@ -501,14 +497,13 @@ int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, 
     if (rc != HB_OK) return rc;
   }
   const TouchMarks marks = index_touch_marks(h);
-  const SegPlan seg = seg_plan(p.seg_ws, n, d->dim);
   const ColdArgs c{d->staging, d->threshold_table, d->default_threshold, (unsigned long long*)d->dropped,
                    p.cold_slots, marks, d->touch_lru};
-  SegArgs a = seg_args(&s->runs, grads, nullptr, d->dim, 0, seg);
+  SegArgs a = seg_args(&s->runs, grads, nullptr, d->dim, 0, p.seg);
   a.n_dev = nullptr;  // all entries: nothing to wait for
   a.cols = (int)d->dim;
-  return d->opt.kind == HB_OPT_ADAM ? update_step<true>(s, d, c, a, vec4, p.sums, seg, fused, st)
-                                    : update_step<false>(s, d, c, a, vec4, p.sums, seg, fused, st);
+  return d->opt.kind == HB_OPT_ADAM ? update_step<true>(s, d, c, a, vec4, p.sums, fused, st)
+                                    : update_step<false>(s, d, c, a, vec4, p.sums, fused, st);
 }
 
 }  // extern "C"
