@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(kBlock) add_sorted_walk_kernel(const int64_t* 
 //     than 32 ids (copies of one id, ids in strides of the number of sets) go to (1).
 __global__ void __launch_bounds__(kBlock) add_push_kernel(const int64_t* __restrict__ ids, int64_t n, AddLists lists,
                                                           int64_t* __restrict__ locs, uint8_t* __restrict__ last_writer) {
+  begin_after_previous();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t id = __ldg(ids + i);
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(kBlock) add_cut_kernel(AddEntries e, int64_t* 
 }
 
 __global__ void __launch_bounds__(kBlock) add_walk_kernel(AddEntries e, AddState a) {
+  begin_after_previous();
   const uint32_t number = batch_number(a.batch);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < e.n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t id = __ldg(e.ids + i);
@@ -398,11 +400,13 @@ __global__ void touch_sorted_kernel(const uint32_t* __restrict__ keys,
 // of one id, ascending), so "hits on the line after my last hit" is counted by
 // binary search in the position lists of the other hit ways of the line, found through the marks.
 __global__ void touch_runs_mark_kernel(RunsView v, TouchMarks marks) {
+  begin_after_previous();
   const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (u < v.runs()) marks.mark(v.slot_of_run(u), u);
 }
 
 __global__ void __launch_bounds__(kBlock) touch_runs_apply_kernel(RunsView v, TouchMarks t, int32_t* __restrict__ lru) {
+  begin_after_previous();
   touch_runs(v, t, lru, blockIdx.x, gridDim.x);
 }
 
@@ -542,7 +546,7 @@ IndexTurn::~IndexTurn() {
 }
 
 int index_touch_apply(hb_index* h, const RunsView& v, cudaStream_t st) {
-  HB_LAUNCH(touch_runs_apply_kernel, grid_capped(v.max_runs), kBlock, 0, st, v, index_touch_marks(h), h->lru);
+  HB_LAUNCH_NEXT(touch_runs_apply_kernel, grid_capped(v.max_runs), kBlock, 0, st, v, index_touch_marks(h), h->lru);
   return HB_OK;
 }
 
@@ -761,12 +765,12 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   uint2* sorted = cv.take<uint2>(n);
   void* sort_ws = cv.take<char>(0);
   if (n > kAddSortMax && n <= kListedPerSet * h->lines) {
-    HB_LAUNCH(add_push_kernel, grid_for(n), kBlock, 0, st, ids, n, index_add_lists(h, next), locs, last_writer);
+    HB_LAUNCH_NEXT(add_push_kernel, grid_for(n), kBlock, 0, st, ids, n, index_add_lists(h, next), locs, last_writer);
     AddEntries e;
     memset(&e, 0, sizeof(e));
     e.ids = ids;
     e.n = n;
-    HB_LAUNCH(add_walk_kernel, grid_capped(n), kBlock, 0, st, e, index_add_state(h, next, locs, last_writer));
+    HB_LAUNCH_NEXT(add_walk_kernel, grid_capped(n), kBlock, 0, st, e, index_add_state(h, next, locs, last_writer));
     return sort_run(SetSource<true>{ids, n, h->lines, h->heads, h->batch + 2},
                     AddFinish{h->line_ids, h->lru, locs, last_writer, sorted, false}, n, sort_ws, st);
   }
@@ -915,7 +919,7 @@ int hb_index_touch_lru_runs(hb_index_t* h, const int64_t* locs, const uint32_t* 
   const int rc = turn.on(st);
   if (rc != HB_OK) return rc;
   RunsView v{locs, perm, run_start, num_runs, n_dev, max_runs, n, locs_kind};
-  HB_LAUNCH(touch_runs_mark_kernel, grid_for(max_runs), kBlock, 0, st, v, index_touch_marks(h));
+  HB_LAUNCH_NEXT(touch_runs_mark_kernel, grid_for(max_runs), kBlock, 0, st, v, index_touch_marks(h));
   return index_touch_apply(h, v, st);
 }
 

@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
     const int64_t* __restrict__ cnt, int64_t n, const int64_t* __restrict__ n_dev, int64_t dim,
     RowMap map, float* __restrict__ step, float* __restrict__ s0, float* __restrict__ s1,
     E* __restrict__ emb, AdamParams p, int glog2, int rpw) {
+  begin_after_previous();
   // rpw: rows a warp takes per round (32, or fewer so that a short list still fills the GPU)
   n = effective_n(n, n_dev);
   const int lane = threadIdx.x & 31;
@@ -283,7 +284,7 @@ int hb_sparse_adam(const int64_t* ids, const float* grads, const int64_t* cnt, i
   HB_LAUNCH((sparse_adam_kernel<E, V>), grid, kBlock, 0, st, ids, grads, cnt, n, n_dev, dim, map, \
             step, mem, power, (E*)emb, p, glog2)
 #define HB_ADAM_VEC(E)                                                                         \
-  HB_LAUNCH((sparse_update_vec_kernel<E, true>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
+  HB_LAUNCH_NEXT((sparse_update_vec_kernel<E, true>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
             n_dev, dim, map, step, mem, power, (E*)emb, p, glog2, rpw)
   if (emb_elem_bytes == 4) {
     if (vec4) HB_ADAM_VEC(float); else HB_ADAM(float, false);
@@ -317,7 +318,7 @@ int hb_sparse_adagrad(const int64_t* ids, const float* grads, const int64_t* cnt
             map, state_sum, (E*)emb, (float)lr, (float)eps, glog2)
   const AdamParams p{(float)lr, 0.f, 0.f, (float)eps, 0.f, 0.f};
 #define HB_ADAGRAD_VEC(E)                                                                       \
-  HB_LAUNCH((sparse_update_vec_kernel<E, false>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
+  HB_LAUNCH_NEXT((sparse_update_vec_kernel<E, false>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
             n_dev, dim, map, nullptr, state_sum, nullptr, (E*)emb, p, glog2, rpw)
   if (emb_elem_bytes == 4) {
     if (vec4) HB_ADAGRAD_VEC(float); else HB_ADAGRAD(float, false);

@@ -528,6 +528,7 @@ __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
     hb_runs_t r, const unsigned long long* __restrict__ run_src, const int64_t* __restrict__ run_slots,
     int64_t row_bytes_arg, int vb, char* __restrict__ out, int64_t* __restrict__ locs,
     uint8_t* __restrict__ found, int per_arg, Maintain duty) {
+  begin_after_previous();
   const int per = FULL ? 32 : per_arg;
   int block = blockIdx.x, blocks = gridDim.x;
   if (MAINTAIN) {
@@ -951,7 +952,7 @@ int fetch_runs_impl(hb_index_t* h, const hb_runs_t* runs, const void* cache_rows
   Maintain none;
   memset(&none, 0, sizeof(none));
 #define HB_EXP_F(PEER, RB, FULL)                                                                              \
-  HB_LAUNCH((runs_expand_kernel<PEER, RB, false, FULL>), grid, kBlock, 0, st, *runs, f.run_src, slots, row_bytes, \
+  HB_LAUNCH_NEXT((runs_expand_kernel<PEER, RB, false, FULL>), grid, kBlock, 0, st, *runs, f.run_src, slots, row_bytes, \
             vb, (char*)out_rows, locs, found, per, none)
 #define HB_EXP(PEER, RB)                                               \
   do {                                                                       \
@@ -983,7 +984,7 @@ int hb::runs_expand_maintain(const hb_runs_t* runs, const unsigned long long* ru
   const int per = items_per_warp(runs->n);
   const int grid = grid_of_warps(runs->n, per, kBlock, 32) + duty.blocks;
 #define HB_EXP_F(RB, FULL)                                                                                       \
-  HB_LAUNCH((runs_expand_kernel<false, RB, true, FULL>), grid, kBlock, 0, st, *runs, run_src, run_slots, row_bytes, \
+  HB_LAUNCH_NEXT((runs_expand_kernel<false, RB, true, FULL>), grid, kBlock, 0, st, *runs, run_src, run_slots, row_bytes, \
             vb, (char*)out_rows, locs, found, per, duty)
 #define HB_EXP(RB)                                         \
   do {                                                           \

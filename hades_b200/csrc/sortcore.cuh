@@ -42,6 +42,7 @@ constexpr int64_t kSortOneEach = 16 * (int64_t)kClusterT;  // ... with one entry
 // The cluster's largest input, and its line: it is ahead of the grid as far as its shared memory reaches (us,
 // cluster / grid, ids of 21 to 26 bits: 16,384 18-20 / 43-50, 32,768 22-25 / 44-47, 65,536 30-36 / 43-47).
 constexpr int64_t kSortClusterMax = 16 * (int64_t)kClusterT * kClusterMaxItems;
+static_assert(kSortClusterMax == kSortClusterEntries, "the line that launches behind a sort go by");
 constexpr int kGridT = 1024;           // threads per CTA of the grid version
 constexpr int kGridDigit = 10;
 constexpr int kGridBins = 1 << kGridDigit;
@@ -360,6 +361,7 @@ struct ClusterCtx {
 
 template <class Src, class Fin, int I>
 __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin fin) {
+  begin_after_previous();
   constexpr int T = kClusterT, W = T / 32, B = 1 << kClusterDigit;
   extern __shared__ __align__(16) char smem[];
   ClusterCtx<I> ctx;
@@ -610,6 +612,7 @@ static inline size_t sort_grid_smem_bytes(int digit) {
 
 template <class Src, class Fin, int I>
 __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, SortGridBufs b, int max_digit, int* err) {
+  begin_after_previous();
   extern __shared__ __align__(16) char smem[];
   uint16_t* wcnt = reinterpret_cast<uint16_t*>(smem);
   uint32_t* wmask = reinterpret_cast<uint32_t*>(smem + ((size_t)(kGridT / 32) << max_digit) * 2);
@@ -814,13 +817,15 @@ int sort_launch_cluster(const Src& src, const Fin& fin, int ctas, cudaStream_t s
   cfg.blockDim = dim3(kClusterT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = ctas;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (HB_LAUNCH_NEXT)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = stream_captures(st) ? 1 : 2;
   HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, src, fin));
   count_launch();
   return HB_OK;

@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(kBlock, MODE == HB_LOOKUP_SETASSOC ? 3 : 2) st
     IndexView v, hb_staging_t s, const int64_t* __restrict__ ids, const float* __restrict__ grads,
     int64_t n, const int64_t* __restrict__ n_dev, const int32_t* __restrict__ thr_table,
     int32_t default_thr, unsigned long long* __restrict__ dropped, int64_t* __restrict__ locs_out, int per) {
+  begin_after_previous();
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -167,6 +168,7 @@ FlushPlan flush_plan(void* ws, int64_t slots) {
 }
 
 __global__ void __launch_bounds__(kBlock) flush_select_kernel(hb_staging_t s, int32_t cnt_threshold, FlushPlan p) {
+  begin_after_previous();
   __shared__ int s_found[kBlock / 32];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
   const int64_t begin = blockIdx.x * p.per_block;
@@ -214,6 +216,7 @@ __global__ void __launch_bounds__(kBlock) flush_leave_kernel(
     hb_staging_t s, FlushPlan p, int64_t out_cap, int64_t* __restrict__ line_ids, int32_t* __restrict__ lru,
     int64_t* __restrict__ out_ids, float* __restrict__ out_rows, int64_t* __restrict__ out_cnt,
     int64_t* __restrict__ counts, int64_t* host_count) {
+  begin_after_previous();
   using V = typename std::conditional<VB == 16, uint4, uint32_t>::type;
   __shared__ int s_sum[kBlock / 32];
   __shared__ uint16_t s_list[kFlushRound];
@@ -446,6 +449,7 @@ __global__ void __launch_bounds__(kBlock, 4) staging_insert_kernel(
     hb_staging_t s, const int64_t* __restrict__ locs, const uint8_t* __restrict__ last_writer,
     const char* __restrict__ emb_rows, const int64_t* __restrict__ row_index,
     char* __restrict__ cache_rows, int64_t row_bytes, int64_t n, const int64_t* __restrict__ n_dev, int per) {
+  begin_after_previous();
   __shared__ uint8_t s_at[kBlock / 32][32];
   n = effective_n(n, n_dev);
   const int lane = lane_id();
@@ -537,7 +541,7 @@ int hb_staging_accumulate_cached(hb_index_t* h, const hb_staging_t* s, const int
   const int per = items_per_warp(n);
   const int grid = grid_of_warps(n, per, kBlock, 16);
 #define HB_ACC(MODE, VEC)                                                                     \
-  HB_LAUNCH((staging_accumulate_cached_kernel<MODE, VEC>), grid, kBlock, 0, st, h->view, *s,  \
+  HB_LAUNCH_NEXT((staging_accumulate_cached_kernel<MODE, VEC>), grid, kBlock, 0, st, h->view, *s,  \
             ids, grads, n, n_dev, threshold_table, default_threshold,                         \
             (unsigned long long*)dropped, locs_out, per)
   if (mode == HB_LOOKUP_SORTED) {
@@ -603,13 +607,13 @@ int hb_staging_flush_counted(hb_index_t* h, const hb_staging_t* s, int32_t cnt_t
     const FlushPlan p = flush_plan(workspace, s->slots);
     int64_t* line_ids = h ? h->line_ids : nullptr;
     int32_t* lru = h ? h->lru : nullptr;
-    HB_LAUNCH(flush_select_kernel, p.blocks, kBlock, 0, (cudaStream_t)stream, *s, cnt_threshold, p);
+    HB_LAUNCH_NEXT(flush_select_kernel, p.blocks, kBlock, 0, (cudaStream_t)stream, *s, cnt_threshold, p);
     if (h) h->sorted_stale = true;
     if (vec16)
-      HB_LAUNCH(flush_leave_kernel<16>, p.blocks, kBlock, 0, (cudaStream_t)stream, *s, p, out_cap, line_ids, lru, out_ids,
+      HB_LAUNCH_NEXT(flush_leave_kernel<16>, p.blocks, kBlock, 0, (cudaStream_t)stream, *s, p, out_cap, line_ids, lru, out_ids,
                 out_rows, out_cnt, counts, host_count);
     else
-      HB_LAUNCH(flush_leave_kernel<4>, p.blocks, kBlock, 0, (cudaStream_t)stream, *s, p, out_cap, line_ids, lru, out_ids,
+      HB_LAUNCH_NEXT(flush_leave_kernel<4>, p.blocks, kBlock, 0, (cudaStream_t)stream, *s, p, out_cap, line_ids, lru, out_ids,
                 out_rows, out_cnt, counts, host_count);
     return HB_OK;
   }
@@ -687,7 +691,7 @@ int hb::staging_insert_rows(const hb_staging_t* s, const void* emb_rows, const i
   const bool zero16 = st_desc.dim % 4 == 0 && ((uintptr_t)st_desc.grad & 15) == 0;
   const int per = items_per_warp(n);
 #define HB_INSERT(VB, Z16)                                                                                     \
-  HB_LAUNCH((staging_insert_kernel<VB, Z16>), grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, \
+  HB_LAUNCH_NEXT((staging_insert_kernel<VB, Z16>), grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, locs, \
             last_writer, (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per)
   if (vb == 16) {
     if (zero16) HB_INSERT(16, true); else HB_INSERT(16, false);

@@ -95,6 +95,7 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
 // The lookup of the runs in a launch of its own (resolve_run: as part of the sort's).
 template <int MODE>
 __global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_runs_t r, RunsResolve a) {
+  begin_after_previous();
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -110,12 +111,6 @@ __global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_ru
     const bool cold = u < U && r.dclass[u] == kCold;
     resolved_run<true>(a, u, u < U, id, cold, warp_lookup<MODE>(v, s_top, id));
   }
-}
-
-// in a graph a second stream costs no host time and no events
-bool captured(cudaStream_t st) {
-  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
 }
 
 int join_side(hb_step* s, cudaStream_t st) {
@@ -140,6 +135,7 @@ struct ColdArgs {
 // row), mark for the ageing.
 template <int MODE>
 __global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_t r, ColdArgs a) {
+  begin_after_previous();
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -176,6 +172,7 @@ template <bool ADAM, int VEC, int G, int VPL>
 __global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(hb_runs_t r, SegArgs a,
                                                                             UpdateRows<ADAM, true> epi,
                                                                             const float* __restrict__ sums) {
+  begin_after_previous();
   using V = typename VecF<VEC>::T;
   using Ops = EpiOps<UpdateRows<ADAM, true>, VEC, G, VPL>;
   constexpr int kFly = VPL > 1 ? 1 : 2;
@@ -233,7 +230,7 @@ int launch_apply(const hb_runs_t& r, const SegArgs& a, const UpdateRows<ADAM, tr
   int64_t blocks = ceil_div(r.n, kBlock);
   if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
   blocks += epi.touch_blocks;
-#define HB_APPLY(G, VPL) HB_LAUNCH((step_apply_kernel<ADAM, VEC, G, VPL>), (int)blocks, kBlock, 0, st, r, a, epi, sums)
+#define HB_APPLY(G, VPL) HB_LAUNCH_NEXT((step_apply_kernel<ADAM, VEC, G, VPL>), (int)blocks, kBlock, 0, st, r, a, epi, sums)
   if (vpr > 64) HB_APPLY(32, 4);
   else if (vpr > 32) HB_APPLY(32, 2);
   else if (vpr > 16) HB_APPLY(32, 1);
@@ -272,9 +269,9 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
     if (rc != HB_OK) return rc;
     const IndexView& v = d->index->view;
     if (d->lookup_mode == HB_LOOKUP_SORTED)
-      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SORTED>, grid_for_runs(r.n), kBlock, 0, on, v, r, c);
+      HB_LAUNCH_NEXT(step_cold_kernel<HB_LOOKUP_SORTED>, grid_for_runs(r.n), kBlock, 0, on, v, r, c);
     else
-      HB_LAUNCH(step_cold_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(r.n), kBlock, 0, on, v, r, c);
+      HB_LAUNCH_NEXT(step_cold_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(r.n), kBlock, 0, on, v, r, c);
     return HB_OK;
   };
   if (fused) {
@@ -410,7 +407,7 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
                       index_add_lists(h, static_cast<uint32_t*>(p.add_ws)), device_error_word()};
   // aside: all of the fetch leaves the caller's stream, which goes on to the aggregation of the
   // same batch (it needs the sort only); both are bound by HBM, but not all the time
-  const bool aside = aside_allowed && (captured(st) || !fuses_update(n));
+  const bool aside = aside_allowed && (stream_captures(st) || !fuses_update(n));
   const bool in_sort = !aside && n <= kResolvedMax && d->lookup_mode == HB_LOOKUP_SETASSOC;
   IndexTurn turn(h);
   if (in_sort) rc = turn.on(st);
@@ -425,9 +422,9 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
     rc = turn.on(st);
     if (rc != HB_OK) return rc;
     if (d->lookup_mode == HB_LOOKUP_SORTED)
-      HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SORTED>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a);
+      HB_LAUNCH_NEXT(step_resolve_kernel<HB_LOOKUP_SORTED>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a);
     else
-      HB_LAUNCH(step_resolve_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a);
+      HB_LAUNCH_NEXT(step_resolve_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(n), kBlock, 0, st, h->view, s->runs, a);
   }
   Maintain m;
   memset(&m, 0, sizeof(m));
@@ -480,7 +477,7 @@ int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, 
   }
   cudaStream_t st = (cudaStream_t)stream;
   hb_index* h = d->index;
-  const bool fused = fuses_update(n) && !captured(st);
+  const bool fused = fuses_update(n) && !stream_captures(st);
   if (ids || fused) {
     rc = join_side(s, st);
     if (rc != HB_OK) return rc;
