@@ -49,6 +49,7 @@ PROTOTYPES: dict[str, tuple] = {
     "hb_index_touch_lru": (_int, [_p, _p, _i64, _p, _sz, _p]),
     "hb_index_lookup_touch": (_int, [_p, _p, _i64, _p, _int, _p]),
     "hb_index_lookup_touch_part": (_int, [_p, _p, _i64, _p, _i64, _p, _p, _int, _p]),
+    "hb_index_lookup_touch_part32": (_int, [_p, _p, _i64, _p, _i64, _p, _p, _int, _p]),
     "hb_index_lookup_touch_end": (_int, [_p, _p, _i64, _p]),
     "hb_index_lookups": (C.c_uint64, [_p]),
     "hb_index_wait_lookups": (_int, [_p, C.c_uint64, _p]),

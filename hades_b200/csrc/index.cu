@@ -206,17 +206,19 @@ __global__ void __launch_bounds__(kBlock) lookup_kernel(IndexView v, const int64
 // with the same slot speak as one, so that the copies of a popular id do not queue at one address.
 // A caller that works on ids in host memory has them and wants the slots in pinned buffers, a part of the
 // batch at a time: positions first .. first + n of it, slots to host_locs too, and then a word that says
-// that they have arrived.
+// that they have arrived.  Ids (as WORD, signed) and slots cross PCIe in half the bytes where the ids fit 32 bits: a
+// part of 32,768 is bound by that.
+template <typename WORD>
 struct HostPart {
   int64_t first;
-  int64_t* locs;    // nullable
+  WORD* locs;       // nullable
   int64_t* arrived; // nullable
 };
 
-template <int MODE, bool LOOKUP>
-__global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const int64_t* __restrict__ ids,
+template <int MODE, bool LOOKUP, typename WORD>
+__global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const WORD* __restrict__ ids,
                                                             int64_t* __restrict__ locs, int64_t n, TouchMarks t,
-                                                            int32_t* __restrict__ line_hits, HostPart part) {
+                                                            int32_t* __restrict__ line_hits, HostPart<WORD> part) {
   __shared__ int64_t s_top[LOOKUP && MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (LOOKUP && MODE == HB_LOOKUP_SORTED) {
     stage_top_level(v, s_top);
@@ -230,10 +232,10 @@ __global__ void __launch_bounds__(kBlock) touch_mark_kernel(IndexView v, const i
     const int64_t i = base + lane;
     int64_t slot = -1;
     if (LOOKUP) {
-      slot = warp_lookup<MODE>(v, s_top, i < n ? __ldg(ids + i) : -1);
+      slot = warp_lookup<MODE>(v, s_top, i < n ? (int64_t)__ldg(ids + i) : -1);
       if (i < n) {
         locs[i] = slot;
-        if (part.locs) part.locs[i] = slot;
+        if (part.locs) part.locs[i] = (WORD)slot;
       }
     } else if (i < n) {
       slot = locs[i];
@@ -782,8 +784,11 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
   return HB_OK;
 }
 
+}  // extern "C"
+
 // lookup of `ids` into locs (or the slots there, ids null), first pass of the ageing
-static int touch_mark(hb_index* h, const int64_t* ids, int64_t* locs, int64_t n, int mode, const HostPart& part,
+template <typename WORD>
+static int touch_mark(hb_index* h, const WORD* ids, int64_t* locs, int64_t n, int mode, const HostPart<WORD>& part,
                       cudaStream_t st) {
   if (ids && mode == HB_LOOKUP_SORTED && h->sorted_stale) {
     const int rc = hb_index_build_sorted(h, st);
@@ -792,16 +797,18 @@ static int touch_mark(hb_index* h, const int64_t* ids, int64_t* locs, int64_t n,
   const int grid = grid_capped(n);
   const TouchMarks t = index_touch_marks(h);
   if (!ids)
-    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false, WORD>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
               part);
   else if (mode == HB_LOOKUP_SORTED)
-    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SORTED, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SORTED, true, WORD>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
               part);
   else
-    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, true>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
+    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, true, WORD>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
               part);
   return HB_OK;
 }
+
+extern "C" {
 
 // (workspace large enough for it)
 static int touch_sorted(hb_index* h, const int64_t* locs, int64_t n, void* workspace, cudaStream_t st) {
@@ -833,11 +840,11 @@ int hb_index_touch_lru(hb_index_t* h, const int64_t* locs, int64_t n, void* work
   if (rc == HB_OK && n > kTouchMarksMax && workspace && workspace_bytes >= touch_sort_bytes(n))
     return touch_sorted(h, locs, n, workspace, st);
   if (rc == HB_OK)
-    rc = touch_mark(h, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, HostPart{0, nullptr, nullptr}, st);
+    rc = touch_mark<int64_t>(h, nullptr, const_cast<int64_t*>(locs), n, HB_LOOKUP_SETASSOC, {0, nullptr, nullptr}, st);
   return rc != HB_OK ? rc : age_marked(h, locs, 0, n, st);
 }
 
-static int check_lookup(hb_index_t* h, const int64_t* ids, int64_t n, const int64_t* locs, int64_t first, int mode) {
+static int check_lookup(hb_index_t* h, const void* ids, int64_t n, const int64_t* locs, int64_t first, int mode) {
   HB_CHECK_ARG(h && first >= 0 && (n == 0 || (ids && locs)), "hb_index_lookup_touch: null argument");
   HB_CHECK_ARG(mode == HB_LOOKUP_SETASSOC || mode == HB_LOOKUP_SORTED, "hb_index_lookup_touch: unknown mode %d", mode);
   HB_CHECK_ARG(n >= 0 && first + n < ((int64_t)1 << 31), "hb_index_lookup_touch: n out of range");
@@ -851,24 +858,39 @@ int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t*
   cudaStream_t st = (cudaStream_t)stream;
   IndexTurn turn(h);
   rc = turn.on(st);
-  if (rc == HB_OK) rc = touch_mark(h, ids, locs, n, mode, HostPart{0, nullptr, nullptr}, st);
+  if (rc == HB_OK) rc = touch_mark<int64_t>(h, ids, locs, n, mode, {0, nullptr, nullptr}, st);
   return rc != HB_OK ? rc : age_marked(h, locs, 0, n, st);
 }
 
-int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
-                               int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream) {
+}  // extern "C"
+
+template <typename WORD>
+static int lookup_touch_part(hb_index_t* h, const WORD* ids, int64_t n, int64_t* locs, int64_t first, WORD* host_locs,
+                             int64_t* arrived, int mode, cudaStream_t st) {
   int rc = check_lookup(h, ids, n, locs, first, mode);
   if (rc != HB_OK || n == 0) return rc;
-  cudaStream_t st = (cudaStream_t)stream;
   IndexTurn turn(h);
   const bool next = h->open_locs == locs && h->open_end == first && h->open_first < first;
   rc = turn.on(st, next);
-  if (rc == HB_OK) rc = touch_mark(h, ids, locs + first, n, mode, HostPart{first, host_locs, arrived}, st);
+  if (rc == HB_OK) rc = touch_mark<WORD>(h, ids, locs + first, n, mode, {first, host_locs, arrived}, st);
   if (rc != HB_OK) return rc;
   h->open_locs = locs;
   if (!next) h->open_first = first;
   h->open_end = first + n;
   return HB_OK;
+}
+
+extern "C" {
+
+int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
+                               int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream) {
+  return lookup_touch_part<int64_t>(h, ids, n, locs, first, host_locs, arrived, mode, (cudaStream_t)stream);
+}
+
+int hb_index_lookup_touch_part32(hb_index_t* h, const int32_t* ids, int64_t n, int64_t* locs, int64_t first,
+                                 int32_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream) {
+  static_assert(sizeof(int) == sizeof(int32_t), "slots of 32 bits");
+  return lookup_touch_part<int>(h, ids, n, locs, first, host_locs, arrived, mode, (cudaStream_t)stream);
 }
 
 int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream) {

@@ -227,6 +227,19 @@ struct InFlight {
   }
 };
 
+// n ids as signed 32-bit numbers; false: some do not fit.
+__attribute__((optimize("O3"))) bool narrow(const int64_t* __restrict__ from, int32_t* __restrict__ to, int64_t n) {
+  uint64_t off = 0;  // (an id that fits lies in [0, 2^32) from -2^31 on)
+  for (int64_t i = 0; i < n; ++i) {
+    off |= ((uint64_t)from[i] + 0x80000000ull) >> 32;
+    to[i] = (int32_t)from[i];
+  }
+  return off == 0;
+}
+__attribute__((optimize("O3"))) void widen(const int32_t* __restrict__ from, int64_t* __restrict__ to, int64_t n) {
+  for (int64_t i = 0; i < n; ++i) to[i] = from[i];
+}
+
 at::Tensor pinned_empty(int64_t n) {
   return at::empty({n}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
 }
@@ -237,7 +250,7 @@ at::Tensor pinned_empty(int64_t n) {
 // copies and after.  Calls on the index from other streams wait for it; where another process has opened the index
 // (words[0]), which can only be ordered by the host, the call does.  A process that opens it later finds in words[1]
 // how many lookups to wait for: that is written before words[0] is read, so that one of the two waits.
-// 500 ids: 25 us (two pageable copies: 70), 65,536: 85 (183).
+// 500 ids: 25 us (two pageable copies: 70), 65,536: 65 (183; 85 with ids and slots in 64 bits on their way).
 PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
     arity(n_args, 5, "index_lookup");
@@ -249,8 +262,8 @@ PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     cudaStream_t st = static_cast<cudaStream_t>(stream_of(dev));
     const int64_t n = ids.numel();
     at::Tensor out = at::empty_like(ids);
-    // as few parts as 32,768 ids each allow, all of one size: a part costs the GPU some 15 us of trips over
-    // PCIe whatever its size (65,000 ids in parts of 8,192: 134 us, 16,384: 87, 32,768: 81, 65,536: 89)
+    // as few parts as 32,768 ids each allow, all of one size: a part costs the GPU some 10 us of trips over
+    // PCIe whatever its size (65,536 ids in parts of 11,000: 109 us, 16,384: 87, 22,000: 74, 32,768: 65, 65,536: 70)
     constexpr int64_t kPart = 32768;
     const int64_t parts = (n + kPart - 1) / kPart, part = (n + parts - 1) / parts;
     const at::Tensor in = pinned_empty(2 * part), back = pinned_empty(2 * part);
@@ -260,16 +273,27 @@ PyObject* index_lookup(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     volatile int64_t* words = t_word.arm();
     InFlight in_flight{st, h, locs.data_ptr<int64_t>()};
     auto length = [&](int64_t k) { return (k + 1) * part < n ? part : n - k * part; };
+    bool narrowed[2] = {false, false};
     auto collect = [&](int64_t k) {
       t_word.wait(st, (int)(k & 1));
       words[k & 1] = -1;
-      memcpy(to + k * part, pback + (k & 1) * part, length(k) * sizeof(int64_t));
+      const int64_t* slots = pback + (k & 1) * part;
+      if (narrowed[k & 1]) widen(reinterpret_cast<const int32_t*>(slots), to + k * part, length(k));
+      else memcpy(to + k * part, slots, length(k) * sizeof(int64_t));
     };
     for (int64_t k = 0; k < parts; ++k) {
       if (k >= 2) collect(k - 2);
-      memcpy(pin + (k & 1) * part, src + k * part, length(k) * sizeof(int64_t));
-      check(hb_index_lookup_touch_part(h, pin + (k & 1) * part, length(k), locs.data_ptr<int64_t>(), k * part,
-                                       pback + (k & 1) * part, const_cast<int64_t*>(words + (k & 1)), mode, st));
+      int64_t *ids_in = pin + (k & 1) * part, *slots = pback + (k & 1) * part;
+      int64_t* word = const_cast<int64_t*>(words + (k & 1));
+      int32_t* ids32 = reinterpret_cast<int32_t*>(ids_in);
+      narrowed[k & 1] = narrow(src + k * part, ids32, length(k));
+      if (narrowed[k & 1]) {
+        check(hb_index_lookup_touch_part32(h, ids32, length(k), locs.data_ptr<int64_t>(), k * part,
+                                           reinterpret_cast<int32_t*>(slots), word, mode, st));
+      } else {
+        memcpy(ids_in, src + k * part, length(k) * sizeof(int64_t));
+        check(hb_index_lookup_touch_part(h, ids_in, length(k), locs.data_ptr<int64_t>(), k * part, slots, word, mode, st));
+      }
       in_flight.looked_up = k * part + length(k);
     }
     check(hb_index_lookup_touch_end(h, locs.data_ptr<int64_t>(), n, st));

@@ -128,6 +128,9 @@ int hb_index_lookup_touch(hb_index_t* h, const int64_t* ids, int64_t n, int64_t*
  * batch; the ageing may still run when the slots have arrived. */
 int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs, int64_t first,
                                int64_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream);
+/* Ids and host_locs as signed 32-bit numbers (half the bytes over PCIe): what fits keeps its value. */
+int hb_index_lookup_touch_part32(hb_index_t* h, const int32_t* ids, int64_t n, int64_t* locs, int64_t first,
+                                 int32_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream);
 int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream);
 /* Batches that hb_index_lookup_touch_end has ended in the creating process, and the wait of a process that has
  * opened the index for the ageing by the first `lookups` of them (status HB_ERR_TIMEOUT after half a minute). */

@@ -411,3 +411,20 @@ def test_ageing_of_large_batches(cuda_lib, oracle_mod, n):
             got = locs.cpu().numpy()
         assert np.array_equal(got, want), rnd
         _same_state(ix, ora, rnd)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32_768, 70_001])
+@pytest.mark.parametrize("top", [2**31 - 1, 2**31, 2**40])
+def test_host_lookups_of_ids_at_the_edge_of_32_bits(cuda_lib, n, top):
+    """A part whose ids fit 32 signed bits crosses PCIe in half the bytes; one with a larger id does not."""
+    from hades_b200 import EmbCacheLib as E
+
+    rng = np.random.default_rng(n)
+    ix = E.IndexCache(4000, f"edge{n}_{top}", True, False)
+    ids = np.concatenate([rng.integers(0, 3000, n, dtype=np.int64), [-1, -2**31, top, top - 1]])[-n:]
+    held = torch.from_numpy(np.unique(np.concatenate([np.arange(3000), [2**31 - 2, 2**31 - 1, 2**31, top - 1, top]])))
+    ix.cuda_add(held.cuda())
+    other = np.where(np.arange(n) % 2 == 0, ids, ids % (1 << 32) if top > 2**31 else ids)  # a low half that is another id
+    for q in (ids, other):
+        want, _ = ix.cuda_lookup_found(torch.from_numpy(np.ascontiguousarray(q)).cuda())
+        _eq(ix.lookup(torch.from_numpy(np.ascontiguousarray(q))).numpy(), want.cpu().numpy(), "slots")
