@@ -7,6 +7,8 @@
 
 using namespace hb;
 
+static constexpr int64_t kHostBoundMax = 16384;
+
 extern "C" {
 
 size_t hb_segsum_runs_workspace_bytes(int64_t n, int64_t dim) { return seg_plan(nullptr, n, dim).total; }
@@ -14,7 +16,7 @@ size_t hb_segsum_runs_workspace_bytes(int64_t n, int64_t dim) { return seg_plan(
 int hb_segsum_runs_f32(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim,
                        int mean, float* sums, int64_t* counts, const hb_class_split_t* split,
                        void* workspace, size_t workspace_bytes, hb_stream_t stream) {
-  return segsum_runs(runs, grads, cnt_in, dim, mean, sums, counts, split, workspace, workspace_bytes, false,
+  return segsum_runs(runs, grads, cnt_in, dim, mean, sums, counts, split, workspace, workspace_bytes, false, true,
                      (cudaStream_t)stream);
 }
 
@@ -22,7 +24,7 @@ int hb_segsum_runs_f32(const hb_runs_t* runs, const float* grads, const int64_t*
 
 int hb::segsum_runs(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean,
                     float* sums, int64_t* counts, const hb_class_split_t* split, void* workspace,
-                    size_t workspace_bytes, bool zeroed, cudaStream_t st) {
+                    size_t workspace_bytes, bool zeroed, bool early, cudaStream_t st) {
   HB_CHECK_ARG(runs != nullptr && dim > 0, "hb_segsum_runs_f32: bad argument");
   const int64_t n = runs->n;
   HB_CHECK_ARG(n == 0 || (grads && runs->perm && runs->head && runs->base8 && runs->run_start && runs->num_runs),
@@ -41,6 +43,7 @@ int hb::segsum_runs(const hb_runs_t* runs, const float* grads, const int64_t* cn
     for (int c = 0; c < 3; ++c) align_bits |= (uintptr_t)split->out_rows[c];
   const bool vec4 = (dim % 4 == 0) && (align_bits & 15) == 0;
   SegArgs a = seg_args(runs, grads, cnt_in, dim, mean, s);
+  a.early = early;
   StoreRows epi;
   epi.sums = sums;
   epi.dclass = split ? runs->dclass : nullptr;
@@ -91,9 +94,13 @@ int hb_unique_segsum_f32(const int64_t* ids, const float* grads, const int64_t* 
                          split ? split->out_ids[2] : nullptr};
   char* seg_ws = static_cast<char*>(workspace) + runs_bytes;
   const SegPlan s = seg_plan(seg_ws, n, dim);
+  // A caller that reads the count is ready for the next call about when the sums of a short list end: what counts is
+  // then the host's time, of which launches that do not start early take less (12,345 x 47: 28.4 us, with 29.3).
+  const bool early = n > kHostBoundMax;
   int rc = runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, split ? split->table : nullptr,
                       split ? split->table_len : 0, split ? cls_ids : nullptr, split ? split->class_counts : nullptr,
-                      uniq_ids, num_unique, s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream);
+                      uniq_ids, num_unique, s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream, nullptr,
+                      early);
   if (rc != HB_OK) return rc;
   if (runs_out) {
     rc = runs_keys(seg_counts, id_bits, workspace, &runs, (cudaStream_t)stream);
@@ -102,7 +109,7 @@ int hb_unique_segsum_f32(const int64_t* ids, const float* grads, const int64_t* 
   }
   if (!n_dev && !seg_counts) runs.n_dev = nullptr;  // all entries: nothing to wait for
   return segsum_runs(&runs, grads, cnt_in, dim, mean, sums, counts, split, seg_ws, workspace_bytes - runs_bytes, true,
-                     (cudaStream_t)stream);
+                     early, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -41,6 +41,7 @@ struct SegArgs {
   int cols;                   // columns of this pass (<= G * VEC * VPL)
   int piece;                  // R: rows per lane group, a power of two
   int mean;                   // divide by the count
+  int early;                  // blocks may take their places under the kernel before (HB_LAUNCH_NEXT)
   // per CTA: what its part of a run that began earlier / of its last run adds up to
   float* head_part;           // [CTAs][cols]
   float* tail_part;           // [CTAs][cols]
@@ -49,10 +50,10 @@ struct SegArgs {
   unsigned* done;             // [CTAs] zero before and after: arrivals of the run that begins in the CTA
 };
 
-// hb_segsum_runs_f32; zeroed: the arrival counters are at zero already
+// hb_segsum_runs_f32; zeroed: the arrival counters are at zero already; early: SegArgs
 int segsum_runs(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim, int mean, float* sums,
                 int64_t* counts, const hb_class_split_t* split, void* workspace, size_t workspace_bytes, bool zeroed,
-                cudaStream_t st);
+                bool early, cudaStream_t st);
 
 // ---- epilogues ---------------------------------------------------------------------------------
 // The sums and counts as they are, or the buffers of the id's class.
@@ -678,7 +679,7 @@ int seg_launch(SegArgs a, const Epi& epi, cudaStream_t st) {
   const size_t smem = (size_t)ng * a.cols * sizeof(float);
   // Behind a sort of the whole GPU blocks that take their places early find the SMs set up for its 200 KB of shared
   // memory, and next to no L1 for their rows (524,288 x 128: 64 -> 78 us).
-  const bool early = a.n <= kSortClusterEntries;
+  const bool early = a.early && a.n <= kSortClusterEntries;
 #define HB_SEG(CNT)                                                                                     \
   do {                                                                                                  \
     if (early) HB_LAUNCH_NEXT((segsum_kernel<VEC, G, VPL, CNT, Epi>), grid, Ops::kBlock, smem, st, a, epi); \
@@ -735,6 +736,7 @@ static inline SegArgs seg_args(const hb_runs_t* runs, const float* grads, const 
   a.cols = 0;
   a.piece = 0;
   a.mean = mean;
+  a.early = 1;
   a.head_part = s.head_part;
   a.tail_part = s.tail_part;
   a.head_cnt = s.head_cnt;

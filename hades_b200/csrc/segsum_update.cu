@@ -65,7 +65,7 @@ int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* 
     const uintptr_t bits = (uintptr_t)grads | (uintptr_t)opt->emb | (uintptr_t)opt->s0;
     return seg_dispatch(a, update_rows<false, false>(&runs, opt), dim % 4 == 0 && (bits & 15) == 0, st);
   }
-  rc = segsum_runs(&runs, grads, cnt_in, dim, mean, sums, nullptr, nullptr, seg_ws, s.total, true, st);
+  rc = segsum_runs(&runs, grads, cnt_in, dim, mean, sums, nullptr, nullptr, seg_ws, s.total, true, true, st);
   if (rc != HB_OK) return rc;
   if (opt->kind == HB_OPT_ADAM)
     return hb_sparse_adam(runs.uniq_ids, sums, nullptr, n, runs.num_runs, dim, opt->id_offset, opt->id_stride, opt->rows,
