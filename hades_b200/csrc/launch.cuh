@@ -53,7 +53,9 @@ cudaError_t launch_next(void (*kernel)(P...), int grid, int block, size_t smem, 
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = stream_captures(st) ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // (reported here, not by the next launch of somebody else)
+  return e;
 }
 #endif
 }  // namespace hb
@@ -67,7 +69,8 @@ cudaError_t launch_next(void (*kernel)(P...), int grid, int block, size_t smem, 
   } while (0)
 
 // A launch whose blocks may take their places while the kernel before it in the stream still runs: they wait in
-// begin_after_previous.  Steps of 2,000 to 65,536 ids are chains of five or six kernels of 3 to 35 us that had 1.7 us
+// begin_after_previous.  (What the stream waits for in between, as an event of another stream, comes first as ever.)
+// Steps of 2,000 to 65,536 ids are chains of five or six kernels of 3 to 35 us that had 1.7 us
 // from the end of one to the start of the next (a step of 2,000 x 64 57.0 -> 49.4 us, of 65,536 x 128 130 -> 118, the
 // update of 60,000 rows for Adam 87 -> 81, a round of the cold cache 171 -> 164).
 #define HB_LAUNCH_NEXT(kernel, grid, block, smem, stream, ...)                          \

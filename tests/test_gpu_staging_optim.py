@@ -246,3 +246,36 @@ def test_flush_to_one_client(cuda_lib, slots, dim, cap, share, sync):
     age[left], cnt[left], grad[left] = 0, 0, 0
     for dst, want in ((t.grad, grad), (t.cnt, cnt), (t.idx, ids), (t.iter_count, age), (t.iter_threshold, limit)):
         assert np.array_equal(dst.cpu().numpy(), want)
+
+
+def test_early_launches_come_behind_events_and_copies(cuda_lib):
+    """Kernels whose blocks take their places under the kernel before them still see what the stream waited for in
+    between: another stream's writes behind an event, a copy, a kernel that is not this library's."""
+    from hades_b200.cold_cache import ColdCache
+
+    dev, n, dim = torch.device("cuda"), 4096, 128
+    cold = ColdCache("early_launch", 8 * n, dim)
+    ids = torch.arange(n, device=dev)
+    cold.insert(ids, torch.zeros((n, dim), device=dev))
+    torch.cuda.synchronize()
+    host = torch.full((n, dim), 2.0).pin_memory()
+    grads, other, main = torch.zeros((n, dim), device=dev), torch.cuda.Stream(), torch.cuda.Stream()
+    for rnd in range(3):
+        grads.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(20_000_000)
+            grads.fill_(1.0)
+            written = other.record_event()
+        with torch.cuda.stream(main):
+            cold.accumulate_remote(ids, grads * 0)
+            main.wait_event(written)
+            cold.accumulate_remote(ids, grads)        # 1
+            torch.cuda._sleep(5_000_000)
+            grads.copy_(host, non_blocking=True)
+            cold.accumulate_remote(ids, grads)        # 2
+            grads.mul_(2.0)
+            cold.accumulate_remote(ids, grads)        # 4
+        torch.cuda.synchronize()
+        slots = cold.index.cuda_lookup_found(ids)[0]
+        assert torch.equal(cold.remote.grad[slots], torch.full((n, dim), 7.0 * (rnd + 1), device=dev)), rnd
