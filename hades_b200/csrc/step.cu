@@ -35,9 +35,9 @@ constexpr int kCold = 2;
 // update in a second pass over the distinct ids: the sums then run at the speed of the copy, and the
 // update has many rows in flight whatever the lengths of the runs.
 // The line lies where the two cost the same, at much the same number of ids for all widths (us a step, Adam, at
-// once / in a second pass: 50,000 ids of 16 columns 88 / 92, of 64 96 / 107, of 128 109 / 125, of 256 136 / 159;
-// 100,000: 114 / 114, 131 / 140, 156 / 163, 208 / 217; 200,000: 143 / 137, 174 / 176, 207 / 205, 293 / 292;
-// 2,000,000 of 128: 903 / 846).
+// once / in a second pass: 50,000 ids of 16 columns 80 / 75, of 64 91 / 91, of 128 105 / 110, of 256 138 / 151;
+// 100,000: 109 / 102, 131 / 129, 160 / 157, 222 / 225; 200,000: 135 / 123, 170 / 160, 209 / 200, 312 / 300;
+// 2,000,000 of 128 a tenth apart).
 // In a captured step the fetch runs beside the sums instead.
 constexpr int64_t kFuseMax = 100000;
 bool fuses_update(int64_t n) { return n <= kFuseMax; }
