@@ -278,11 +278,10 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
     const int rc = look_up(st);
     return rc != HB_OK ? rc : seg_dispatch(a, epi, vec4, st);
   }
-  // The sums need the sort only.  Beside them, once the cache holds the misses of this batch: where the cold ids are.
-  if (!s->side_busy) {
-    HB_CUDA(cudaEventRecord(s->forked, st));
-    HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
-  }
+  // The sums need the sort only.  Beside them, once the cache holds the misses of this batch: where the cold ids are,
+  // behind all that the caller has enqueued up to here (a fetch aside waits for less: for the forward call).
+  HB_CUDA(cudaEventRecord(s->forked, st));
+  HB_CUDA(cudaStreamWaitEvent(s->side, s->forked, 0));
   int rc = look_up(s->side);
   if (rc != HB_OK) return rc;
   HB_CUDA(cudaEventRecord(s->fetched, s->side));
@@ -478,7 +477,10 @@ int hb_step_backward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, 
   cudaStream_t st = (cudaStream_t)stream;
   hb_index* h = d->index;
   const bool fused = fuses_update(n) && !stream_captures(st);
-  if (ids || fused) {
+  // A fetch that is still aside outside of the capture that this call belongs to (or inside one that it does not):
+  // the join is refused, before the second stream takes work of this call.
+  const bool apart = s->side_busy && stream_captures(st) != stream_captures(s->side);
+  if (ids || fused || apart) {
     rc = join_side(s, st);
     if (rc != HB_OK) return rc;
   }

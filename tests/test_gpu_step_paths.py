@@ -181,3 +181,54 @@ def test_runs_looked_up_in_the_launch_of_the_sort(cuda_lib, n):
     a, b = _pair(f"resolve_{n}")
     a.miss_cap = b.miss_cap = max(n // 8, 1)
     _run_pair(a, b, [(ids[:n], g[:n]) for ids, g in _steps(_small("resolve", batch=8193), 4, seed=n)])
+
+
+@pytest.mark.parametrize("optimizer", ["adam", "adagrad"])
+def test_backward_comes_behind_the_callers_stream(cuda_lib, optimizer):
+    """What the caller enqueues between a fetch aside and its backward pass is seen by the lookup of the cold ids, which
+    runs on the step's second stream in steps of more than 100,000 ids."""
+    n = 100_001
+    a, b = _pair("behind_" + optimizer, optimizer=optimizer)
+    for p in (a, b):
+        p.cold.threshold = torch.full((p.num_nodes,), 1, dtype=torch.int32, device="cuda")
+        p.miss_cap = 500  # the cold ids beyond it are dropped
+    for rnd, (ids, g) in enumerate(_steps(_small("behind", batch=n), 4)):
+        rows = []
+        for p, aside in ((a, True), (b, False)):
+            rows.append(p.forward(ids, on_side=aside))
+            torch.cuda._sleep(20_000_000)
+            p.cold.threshold.fill_(rnd + 2)
+            p.cold.dropped.zero_()
+            p.backward(ids, g)
+        assert torch.equal(rows[0][0], rows[1][0]) and torch.equal(rows[0][2], rows[1][2])
+        assert a.cold.dropped.item() > 0
+        sa, sb = _state(a), _state(b)
+        for k in sb:
+            assert torch.equal(sa[k], sb[k]), (rnd, k)
+
+
+def test_capture_behind_a_fetch_aside_is_refused(cuda_lib):
+    """A fetch enqueued outside of a capture cannot be waited for inside it; nothing of the call runs."""
+    import ctypes
+
+    cu, n = ctypes.CDLL("libcuda.so.1"), 100_001
+    a, b = _pair("aside_capture")
+    (ids, g), (ids2, g2) = _steps(_small("aside_capture", batch=n), 2)
+    other = torch.cuda.Stream()
+    a.forward(ids, on_side=True)
+    b.forward(ids)
+    torch.cuda.synchronize()
+    before = _state(a)
+    graph = ctypes.c_void_p()
+    with torch.cuda.stream(other):
+        assert cu.cuStreamBeginCapture_v2(ctypes.c_void_p(other.cuda_stream), 1) == 0
+        with pytest.raises(RuntimeError):
+            a._backward_core(ids, g)
+        assert cu.cuStreamEndCapture(ctypes.c_void_p(other.cuda_stream), ctypes.byref(graph)) != 0
+    ctypes.CDLL("libcudart.so.12").cudaGetLastError()
+    torch.cuda.synchronize()
+    after = _state(a)
+    assert all(torch.equal(before[k], after[k]) for k in before)
+    a.backward(ids, g)
+    b.backward(ids, g)
+    _run_pair(a, b, [(ids2, g2)])
