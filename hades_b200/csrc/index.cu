@@ -49,7 +49,7 @@ struct SetSource {
   static constexpr bool starts_early() { return true; }
   __device__ __forceinline__ int64_t count() const { return !LONG_LISTS || batch[2] == batch[0] ? n : 0; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
-    const int64_t x = __ldg(ids + i);
+    const int64_t x = ids[i];
     if (x < 0) return false;  // unusable (padding)
     key = (unsigned long long)mod_nonneg(x, lines);
     return !LONG_LISTS || heads[key] == (((unsigned long long)(uint32_t)batch[0] << 32) | kLongList);
@@ -73,7 +73,7 @@ __device__ __forceinline__ void add_sorted_set(int j, int n, const uint2* kv, co
   int k = j;
   uint2 x = e;
   while (true) {
-    const int way = st.place(__ldg(ids + x.y), k);
+    const int way = st.place(ids[x.y], k);
     locs[x.y] = way >= 0 ? line * kWays + way : -1;
     ++k;
     if (k >= n) break;
@@ -123,12 +123,12 @@ __global__ void __launch_bounds__(kBlock) add_sorted_walk_kernel(const int64_t* 
 // (2) Every id puts itself on the list of its set (one atomic exchange); the thread whose id ended up
 //     in front owns the set, brings the list into input order and walks it.  No sort.  Lists of more
 //     than 32 ids (copies of one id, ids in strides of the number of sets) go to (1).
-__global__ void __launch_bounds__(kBlock) add_push_kernel(const int64_t* __restrict__ ids, int64_t n, AddLists lists,
-                                                          int64_t* __restrict__ locs, uint8_t* __restrict__ last_writer) {
+__global__ void __launch_bounds__(kBlock) add_push_kernel(const int64_t* ids, int64_t n, AddLists lists, int64_t* locs,
+                                                          uint8_t* last_writer) {
   begin_after_previous();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int64_t id = __ldg(ids + i);
+  const int64_t id = ids[i];
   if (id >= 0) {
     lists.push(id, i);
   } else {
@@ -150,7 +150,7 @@ struct ListedSource {
   static constexpr bool starts_early() { return true; }
   __device__ __forceinline__ int64_t count() const { return *n_dev < n ? *n_dev : n; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
-    key = (unsigned long long)mod_nonneg(__ldg(ids + i), lines);
+    key = (unsigned long long)mod_nonneg(ids[i], lines);
     return listed[i] && i < *cut;
   }
 };
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kBlock) add_walk_kernel(AddEntries e, AddState
   begin_after_previous();
   const uint32_t number = batch_number(a.batch);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < e.n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t id = __ldg(e.ids + i);
+    const int64_t id = e.ids[i];
     if (id < 0) continue;
     const int64_t line = mod_nonneg(id, a.lines);
     if (a.heads[line] != (((unsigned long long)number << 32) | (unsigned long long)(i + 1))) continue;
@@ -409,7 +409,7 @@ __global__ void touch_runs_mark_kernel(RunsView v, TouchMarks marks) {
   if (u < v.runs()) marks.mark(v.slot_of_run(u), u);
 }
 
-__global__ void __launch_bounds__(kBlock) touch_runs_apply_kernel(RunsView v, TouchMarks t, int32_t* __restrict__ lru) {
+__global__ void __launch_bounds__(kBlock) touch_runs_apply_kernel(RunsView v, TouchMarks t, int32_t* lru) {
   begin_after_previous();
   touch_runs(v, t, lru, blockIdx.x, gridDim.x);
 }

@@ -105,7 +105,7 @@ __device__ __forceinline__ int64_t warp_lookup_setassoc(const IndexView& v, int6
     const int q = r * 4 + grp;
     const int64_t lq = __shfl_sync(0xffffffffu, line, q);
     qid[r] = __shfl_sync(0xffffffffu, id, q);
-    keys[r] = lq >= 0 ? __ldg(v.line_ids + lq * kWays + sub) : (int64_t)-1;
+    keys[r] = lq >= 0 ? v.line_ids[lq * kWays + sub] : (int64_t)-1;
   }
   int64_t slot = -1;
 #pragma unroll
@@ -125,7 +125,7 @@ __device__ __forceinline__ int64_t warp_lookup_setassoc(const IndexView& v, int6
 __device__ __forceinline__ void stage_top_level(const IndexView& v, int64_t* smem_top) {
   if (v.top == 0) return;
   const int n = v.level_len[v.top];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) smem_top[i] = __ldg(v.level[v.top] + i);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) smem_top[i] = v.level[v.top][i];
 }
 
 __device__ __forceinline__ int64_t warp_lookup_sorted(const IndexView& v, const int64_t* smem_top,
@@ -154,7 +154,7 @@ __device__ __forceinline__ int64_t warp_lookup_sorted(const IndexView& v, const 
       const int q = r * 4 + grp;
       const int64_t tq = __shfl_sync(0xffffffffu, t, q);
       qid[r] = __shfl_sync(0xffffffffu, id, q);
-      k[r] = tq >= 0 ? __ldg(lv + tq * (kNodeFan / 2) + sub) : make_longlong2(INT64_MAX, INT64_MAX);
+      k[r] = tq >= 0 ? lv[tq * (kNodeFan / 2) + sub] : make_longlong2(INT64_MAX, INT64_MAX);
     }
     int64_t nt = t;
 #pragma unroll
@@ -177,7 +177,7 @@ __device__ __forceinline__ int64_t warp_lookup_sorted(const IndexView& v, const 
     const int q = r * 4 + grp;
     const int64_t tq = __shfl_sync(0xffffffffu, t, q);
     qid[r] = __shfl_sync(0xffffffffu, id, q);
-    p[r] = tq >= 0 ? __ldg(v.pairs + tq * kLeafFan + sub) : make_longlong2(INT64_MAX, -1);
+    p[r] = tq >= 0 ? v.pairs[tq * kLeafFan + sub] : make_longlong2(INT64_MAX, -1);
   }
   int64_t slot = -1;
 #pragma unroll

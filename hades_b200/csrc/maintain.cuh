@@ -4,6 +4,7 @@
 #pragma once
 
 #include "index.cuh"
+#include "launch.cuh"
 
 namespace hb {
 
@@ -136,7 +137,7 @@ __device__ __forceinline__ int64_t add_cut(const AddEntries& e, int64_t n) {
     const int64_t c = c0 + threadIdx.x * 16;
     int mine = 0;
     for (int x = 0; x < 16; ++x)
-      if (c + x < chunks) mine += __ldg(e.chunk_listed + c + x);
+      if (c + x < chunks) mine += e.chunk_listed[c + x];
     int inc = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -155,7 +156,7 @@ __device__ __forceinline__ int64_t add_cut(const AddEntries& e, int64_t n) {
     if (left >= first && left < first + mine) {
       int64_t need = left - first;
       int x = 0;
-      while (need >= __ldg(e.chunk_listed + c + x)) { need -= __ldg(e.chunk_listed + c + x); ++x; }
+      while (need >= e.chunk_listed[c + x]) { need -= e.chunk_listed[c + x]; ++x; }
       int64_t i = (c + x) * 32;
       const int64_t end = i + 32 < n ? i + 32 : n;
       for (; i < end; ++i)
@@ -208,7 +209,7 @@ __device__ __forceinline__ void walk_list(const AddEntries& e, const AddState& a
   uint32_t at = behind;
   while (at && len < kListShort) {
     const uint32_t after = a.next[at - 1];
-    const int64_t its = __ldg(e.ids + (int64_t)at - 1);
+    const int64_t its = DISTINCT ? e.ids[(int64_t)at - 1] : load_settled(e.ids + (int64_t)at - 1);
     int k = len++;
     for (; k > 0 && order[k - 1] > at; --k) {
       order[k] = order[k - 1];
@@ -224,7 +225,7 @@ __device__ __forceinline__ void walk_list(const AddEntries& e, const AddState& a
     int k = 0;
     for (at = first; at; at = a.next[at - 1], ++k) {
       const int64_t x = (int64_t)at - 1;
-      const int way = x < cut ? st.place(__ldg(e.ids + x), k) : -1;
+      const int way = x < cut ? st.place(e.ids[x], k) : -1;
       a.locs[x] = way >= 0 ? line * kWays + way : -1;
     }
     if (a.last_writer) {
@@ -353,7 +354,7 @@ struct Maintain {
         if (insert && (uint32_t)(add.heads[slot >> 3] >> 32) == add_number) continue;
         touch_run(v, marks, add.lru, u, slot, nruns, npos, hit_number);
       } else if (insert && e.listed[u]) {
-        const int64_t id = __ldg(e.ids + u);
+        const int64_t id = e.ids[u];
         const int64_t line = mod_nonneg(id, add.lines);
         if (add.heads[line] != (((unsigned long long)add_number << 32) | (unsigned long long)(u + 1))) continue;
         LineState st;

@@ -108,10 +108,8 @@ __global__ void __launch_bounds__(kBlock, 4) sparse_adam_kernel(
 // shuffle.
 template <typename E, bool ADAM>
 __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
-    const int64_t* __restrict__ ids, const float* __restrict__ grads,
-    const int64_t* __restrict__ cnt, int64_t n, const int64_t* __restrict__ n_dev, int64_t dim,
-    RowMap map, float* __restrict__ step, float* __restrict__ s0, float* __restrict__ s1,
-    E* __restrict__ emb, AdamParams p, int glog2, int rpw) {
+    const int64_t* ids, const float* grads, const int64_t* cnt, int64_t n, const int64_t* n_dev, int64_t dim,
+    RowMap map, float* step, float* s0, float* s1, E* emb, AdamParams p, int glog2, int rpw) {
   begin_after_previous();
   // rpw: rows a warp takes per round (32, or fewer so that a short list still fills the GPU)
   n = effective_n(n, n_dev);
@@ -123,7 +121,7 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
   const int64_t vpr = dim >> 2;
   for (int64_t base = warp * rpw; base < n; base += nwarps * rpw) {
     const int64_t i = base + lane;
-    const int64_t row = (lane < rpw && i < n) ? map(__ldg(ids + i)) : -1;
+    const int64_t row = (lane < rpw && i < n) ? map(ids[i]) : -1;
     float ra = 1.0f, rb = 1.0f, rc = 1.0f;
     if (row >= 0) {
       if (ADAM) {
@@ -133,7 +131,7 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
         ra = 1.0f / (1.0f - powf(p.beta1, t));
         rb = 1.0f / (1.0f - powf(p.beta2, t));
       }
-      if (cnt) rc = 1.0f / (float)__ldg(cnt + i);  // grad / cnt, sparse_optim.py:608-611
+      if (cnt) rc = 1.0f / (float)cnt[i];  // grad / cnt, sparse_optim.py:608-611
     }
     for (int pass = 0; pass * rpp < rpw; pass += kOptRows) {
       int64_t rw[kOptRows];
@@ -154,7 +152,7 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
 #pragma unroll
         for (int u = 0; u < kOptRows; ++u)
           if (rw[u] >= 0) {
-            gg[u] = __ldg(gp[u] + k);
+            gg[u] = __ldcg(gp[u] + k);
             mm[u] = reinterpret_cast<const float4*>(s0 + rw[u] * dim)[k];
             if (ADAM) vv[u] = reinterpret_cast<const float4*>(s1 + rw[u] * dim)[k];
             ee[u] = EmbIO<E>::load4(emb + rw[u] * dim + 4 * k);

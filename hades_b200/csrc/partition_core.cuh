@@ -271,7 +271,7 @@ __device__ __forceinline__ void warp_move_rows(const char* src_row, char* dst_ro
       uint4 v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (s[u]) v[u] = __ldg(s[u] + sub);
+        if (s[u]) v[u] = s[u][sub];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (s[u]) d[u][sub] = v[u];
@@ -294,7 +294,7 @@ __device__ __forceinline__ void warp_move_rows(const char* src_row, char* dst_ro
         uint4 v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          if (s[u]) v[u] = __ldg(s[u] + k);
+          if (s[u]) v[u] = s[u][k];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           if (s[u]) d[u][k] = v[u];
@@ -308,8 +308,16 @@ __device__ __forceinline__ void warp_move_rows(const char* src_row, char* dst_ro
       const char* s = reinterpret_cast<const char*>(a);
       char* d = reinterpret_cast<char*>(b);
       if (vb == 4) {
-        for (int64_t k = lane; k < (row_bytes >> 2); k += 32)
-          reinterpret_cast<uint32_t*>(d)[k] = __ldg(reinterpret_cast<const uint32_t*>(s) + k);
+        const int64_t words = row_bytes >> 2;
+        for (int64_t k = lane; k < words; k += 128) {  // four on their way at once
+          uint32_t v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (k + 32 * u < words) v[u] = reinterpret_cast<const uint32_t*>(s)[k + 32 * u];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (k + 32 * u < words) reinterpret_cast<uint32_t*>(d)[k + 32 * u] = v[u];
+        }
       } else {
         for (int64_t k = lane; k < row_bytes; k += 32) d[k] = s[k];
       }

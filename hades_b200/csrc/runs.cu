@@ -55,7 +55,7 @@ struct IdSource {
       const uint32_t seg = (uint32_t)i / seg_cap;
       if ((int64_t)((uint32_t)i - seg * seg_cap) >= seg_counts[seg]) return false;
     }
-    const int64_t id = __ldg(ids + i);
+    const int64_t id = __ldcg(ids + i);  // (as a plain load: 56 bytes of spills in the sort of 65,537 to 303,104 ids)
     if (id < 0 || id >= sentinel) {
       atomicExch(err, HB_ERR_INVALID);
       return false;
@@ -200,7 +200,7 @@ struct RunsFinish {
         cls[x] = 3;
         if ((heads >> x) & 1u) {
           const int64_t id = ctx.wide ? wide_id(e[x].y) : narrow_id(e[x].x);
-          if (id < table_len) cls[x] = __ldg(table + id);
+          if (id < table_len) cls[x] = Ctx::kBehindAll ? load_settled(table + id) : table[id];
         }
       }
 #pragma unroll
@@ -369,7 +369,7 @@ struct RowSource {
 template <bool PEER>
 __device__ __forceinline__ uint4 load_row16(const uint4* p) {
   if (PEER) return *p;  // may be a peer GPU's memory that its owner rewrites between steps
-  return __ldg(p);
+  return load_settled(p);  // (the launch before it looks the rows up)
 }
 
 // run_src[u]: address of the run's row (16-byte aligned, 0 = none) | 1 when it is a cache row
@@ -502,7 +502,7 @@ __device__ __forceinline__ int64_t run_of_entry(const hb_runs_t& r, int64_t j) {
   const unsigned long long flags = *reinterpret_cast<const unsigned long long*>(r.head + (j & ~(int64_t)7));
   const int k = (int)(j & 7);
   const unsigned long long mask = k == 7 ? ~0ull : ((1ull << (8 * (k + 1))) - 1ull);
-  return (int64_t)__ldg(r.base8 + (j >> 3)) + __popcll(flags & mask) - 1;
+  return (int64_t)r.base8[j >> 3] + __popcll(flags & mask) - 1;
 }
 
 // The id of every sorted entry; entries that take no part hold the sentinel.  perm (nullable): positions
@@ -527,9 +527,8 @@ __global__ void __launch_bounds__(kBlock) runs_keys_kernel(hb_runs_t r, int64_t 
 // distinct ids 0.376 -> 0.441 ms).  The other form is for lists that do not fill the GPU.
 template <bool PEER, int RB, bool MAINTAIN, bool FULL>
 __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
-    hb_runs_t r, const unsigned long long* __restrict__ run_src, const int64_t* __restrict__ run_slots,
-    int64_t row_bytes_arg, int vb, char* __restrict__ out, int64_t* __restrict__ locs,
-    uint8_t* __restrict__ found, int per_arg, Maintain duty) {
+    hb_runs_t r, const unsigned long long* run_src, const int64_t* run_slots, int64_t row_bytes_arg, int vb, char* out,
+    int64_t* locs, uint8_t* found, int per_arg, Maintain duty) {
   begin_after_previous();
   const int per = FULL ? 32 : per_arg;
   int block = blockIdx.x, blocks = gridDim.x;
@@ -551,7 +550,7 @@ __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
   uint32_t pos_next = 0;
   int64_t run_next = -1;
   if (lane < per && base + lane < n) {
-    pos_next = __ldg(r.perm + base + lane);
+    pos_next = r.perm[base + lane];
     run_next = run_of_entry(r, base + lane);
   }
   for (; base < n; base += stride) {
@@ -559,7 +558,7 @@ __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
     const uint32_t pos = pos_next;
     const int64_t u = valid ? run_next : -1;
     if (lane < per && base + stride + lane < n) {
-      pos_next = __ldg(r.perm + base + stride + lane);
+      pos_next = r.perm[base + stride + lane];
       run_next = run_of_entry(r, base + stride + lane);
     }
     const int64_t prev = __shfl_up_sync(0xffffffffu, u, 1);
@@ -953,9 +952,10 @@ int fetch_runs_impl(hb_index_t* h, const hb_runs_t* runs, const void* cache_rows
   const int grid = grid_of_warps(runs->n, per, kBlock, 32);
   Maintain none;
   memset(&none, 0, sizeof(none));
+  // (a call that only expands does not know what wrote the rows, nor whether it still runs)
 #define HB_EXP_F(PEER, RB, FULL)                                                                              \
-  HB_LAUNCH_NEXT((runs_expand_kernel<PEER, RB, false, FULL>), grid, kBlock, 0, st, *runs, f.run_src, slots, row_bytes, \
-            vb, (char*)out_rows, locs, found, per, none)
+  HB_LAUNCH_NEXT_IF(resolve, (runs_expand_kernel<PEER, RB, false, FULL>), grid, kBlock, 0, st, *runs, f.run_src, slots, \
+                    row_bytes, vb, (char*)out_rows, locs, found, per, none)
 #define HB_EXP(PEER, RB)                                               \
   do {                                                                       \
     if (RB != 0 && per == 32) HB_EXP_F(PEER, RB, RB != 0); else HB_EXP_F(PEER, RB, false); \

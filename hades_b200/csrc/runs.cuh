@@ -119,7 +119,7 @@ __device__ __forceinline__ void resolve_run(const RunsResolve& a, int64_t u, boo
     const longlong2* p = reinterpret_cast<const longlong2*>(a.line_ids + line * kWays);
     longlong2 k[kWays / 2];
 #pragma unroll
-    for (int w = 0; w < kWays / 2; ++w) k[w] = __ldg(p + w);
+    for (int w = 0; w < kWays / 2; ++w) k[w] = p[w];
 #pragma unroll
     for (int w = kWays / 2 - 1; w >= 0; --w) {  // the FIRST way that matches (cache_line.h:49-55)
       if (k[w].y == id) slot = line * kWays + 2 * w + 1;

@@ -16,7 +16,7 @@ size_t hb_segsum_runs_workspace_bytes(int64_t n, int64_t dim) { return seg_plan(
 int hb_segsum_runs_f32(const hb_runs_t* runs, const float* grads, const int64_t* cnt_in, int64_t dim,
                        int mean, float* sums, int64_t* counts, const hb_class_split_t* split,
                        void* workspace, size_t workspace_bytes, hb_stream_t stream) {
-  return segsum_runs(runs, grads, cnt_in, dim, mean, sums, counts, split, workspace, workspace_bytes, false, true,
+  return segsum_runs(runs, grads, cnt_in, dim, mean, sums, counts, split, workspace, workspace_bytes, false, false,
                      (cudaStream_t)stream);
 }
 

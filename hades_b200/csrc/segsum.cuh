@@ -41,7 +41,7 @@ struct SegArgs {
   int cols;                   // columns of this pass (<= G * VEC * VPL)
   int piece;                  // R: rows per lane group, a power of two
   int mean;                   // divide by the count
-  int early;                  // blocks may take their places under the kernel before (HB_LAUNCH_NEXT)
+  int early;                  // the launch before is one of this call's: blocks may take their places under it (HB_LAUNCH_NEXT)
   // per CTA: what its part of a run that began earlier / of its last run adds up to
   float* head_part;           // [CTAs][cols]
   float* tail_part;           // [CTAs][cols]
@@ -407,7 +407,7 @@ segsum_kernel(SegArgs a, Epi epi) {
     // head flags of the 8 entries around j0 (pieces of a narrow row may begin inside them)
     const unsigned long long f = *reinterpret_cast<const unsigned long long*>(a.head + (j0 & ~7));
     first_partial = ((f >> (8 * (j0 & 7))) & 1ull) == 0ull;
-    u = __ldg(a.base8 + (j0 >> 3)) - 1 + __popcll(f & ((1ull << (8 * (j0 & 7))) - 1ull));
+    u = a.base8[j0 >> 3] - 1 + __popcll(f & ((1ull << (8 * (j0 & 7))) - 1ull));
   }
   const int u_first = u;
   bool open = first_partial;  // a run is open
@@ -449,9 +449,9 @@ segsum_kernel(SegArgs a, Epi epi) {
   uint32_t p_next = 0;
   bool head_next = false, end_next = false;
   auto look = [&](int j) {  // entry j of the sorted order
-    p_next = __ldg(a.perm + j);
-    head_next = __ldg(a.head + j) != 0;
-    end_next = j + 1 >= n_eff || __ldg(a.head + j + 1) != 0;
+    p_next = a.perm[j];
+    head_next = a.head[j] != 0;
+    end_next = j + 1 >= n_eff || a.head[j + 1] != 0;
   };
   if (sub < eg && sub < len) look(j0 + sub);
   for (int s = 0; s < steps; ++s) {
@@ -468,7 +468,7 @@ segsum_kernel(SegArgs a, Epi epi) {
       if (begun || !first_partial) mine = Ops::lane(epi, u + begun);
     }
     int cv = 1;
-    if (HAS_CNT && valid) cv = (int)__ldg(a.cnt_in + p);
+    if (HAS_CNT && valid) cv = (int)a.cnt_in[p];
     if (Ops::kPrefetch && valid) {
       l2_prefetch_row(a.grads + (int64_t)p * a.dim + a.col0, a.cols * 4);
       Ops::prefetch(epi, a, mine);
@@ -488,7 +488,7 @@ segsum_kernel(SegArgs a, Epi epi) {
 #pragma unroll
           for (int v = 0; v < VPL; ++v) {
             const int k = sub + v * G;
-            if (k < vpr) val[x][v] = __ldg(src + k);
+            if (k < vpr) val[x][v] = load_settled(src + k);
           }
         }
         Ops::fetch(epi, a, mine, t0 + x, (ends >> (t0 + x)) & 1u, sub, vpr, with[x]);
@@ -537,8 +537,8 @@ segsum_kernel(SegArgs a, Epi epi) {
 
   // this CTA's part of a run that crosses CTAs is in the workspace: has every other part arrived?
   auto arrive = [&](int run) {
-    const int first = (int)(__ldg(a.run_start + run) / span);
-    const int last = (int)((__ldg(a.run_start + run + 1) - 1) / span);
+    const int first = (int)(a.run_start[run] / span);
+    const int last = (int)((a.run_start[run + 1] - 1) / span);
     __threadfence();
     __syncwarp(gmask);
     if (sub == 0) {
@@ -574,7 +574,7 @@ segsum_kernel(SegArgs a, Epi epi) {
     }
     if (ended) {
       typename Ops::Row with = Ops::fetch_alone(epi, a, u, sub, vpr);
-      complete(u, acc, with, HAS_CNT ? cacc : (unsigned long long)(__ldg(a.run_start + u + 1) - __ldg(a.run_start + u)));
+      complete(u, acc, with, HAS_CNT ? cacc : (unsigned long long)(a.run_start[u + 1] - a.run_start[u]));
     } else {
       put(a.tail_part + (int64_t)block * a.cols, acc);
       if (HAS_CNT && sub == 0) a.tail_cnt[block] = cacc;
@@ -620,7 +620,7 @@ segsum_kernel(SegArgs a, Epi epi) {
         if (HAS_CNT) w += s_cnt[g];
       }
       typename Ops::Row with = Ops::fetch_alone(epi, a, run, sub, vpr);
-      complete(run, row, with, HAS_CNT ? w : (unsigned long long)(__ldg(a.run_start + run + 1) - __ldg(a.run_start + run)));
+      complete(run, row, with, HAS_CNT ? w : (unsigned long long)(a.run_start[run + 1] - a.run_start[run]));
       if (sub == 0) a.done[first] = 0u;
     }
     __syncthreads();

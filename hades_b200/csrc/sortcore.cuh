@@ -271,6 +271,7 @@ struct ClusterCtx {
   static constexpr int kThreads = kClusterT;
   static constexpr int kItems = ITEMS;
   static constexpr int kChunk = kClusterT * ITEMS;
+  static constexpr bool kBehindAll = false;
   SortClusterSmem s;
   int count;   // entries that were sorted
   uint32_t* scratch;  // shared memory, 8 * kThreads words, free after the sort
@@ -515,6 +516,7 @@ template <int ITEMS>
 struct GridCtx {
   static constexpr int kThreads = kGridT;
   static constexpr int kItems = ITEMS;
+  static constexpr bool kBehindAll = true;  // ids are: the launch does not start early (sort_launch_grid)
   const uint2* kv;     // the sorted entries
   uint32_t* scratch;   // shared memory, 8 * kThreads words, free after the sort
   int4* exchange;

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_ru
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
     const int64_t u = u0 + lane;
-    const int64_t id = u < U ? __ldg(r.uniq_ids + u) : -1;
+    const int64_t id = u < U ? r.uniq_ids[u] : -1;
     const bool cold = u < U && r.dclass[u] == kCold;
     resolved_run<true>(a, u, u < U, id, cold, warp_lookup<MODE>(v, s_top, id));
   }
@@ -147,11 +147,11 @@ __global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_
   for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
     const int64_t u = u0 + lane_id();
     const bool cold = u < U && r.dclass[u] == kCold;
-    const int64_t id = cold ? __ldg(r.uniq_ids + u) : -1;
+    const int64_t id = cold ? r.uniq_ids[u] : -1;
     const int64_t slot = warp_lookup<MODE>(v, s_top, id);
     if (slot >= 0) {
       a.s.idx[slot] = id;
-      a.s.iter_threshold[slot] = a.thr_table ? __ldg(a.thr_table + id) : a.default_thr;
+      a.s.iter_threshold[slot] = a.thr_table ? a.thr_table[id] : a.default_thr;
       a.s.cnt[slot] += 1;
       if (a.touch) a.marks.mark(slot, u);
     }
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_
 template <bool ADAM, int VEC, int G, int VPL>
 __global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(hb_runs_t r, SegArgs a,
                                                                             UpdateRows<ADAM, true> epi,
-                                                                            const float* __restrict__ sums) {
+                                                                            const float* sums) {
   begin_after_previous();
   using V = typename VecF<VEC>::T;
   using Ops = EpiOps<UpdateRows<ADAM, true>, VEC, G, VPL>;
@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(hb_
     typename Ops::Lane mine;
     int count = 0;
     if (u < U) {
-      const int64_t begin = __ldg(r.run_start + u), end = __ldg(r.run_start + u + 1);
-      mine = Ops::lane_of_class(epi, r.dclass[u], __ldg(r.uniq_ids + u), __ldg(epi.slots + u));
+      const int64_t begin = r.run_start[u], end = r.run_start[u + 1];
+      mine = Ops::lane_of_class(epi, r.dclass[u], r.uniq_ids[u], epi.slots[u]);
       count = (int)(end - begin);
     }
     const int rows = U - u0 < 32 ? (int)(U - u0) : 32;
@@ -447,7 +447,7 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
       if (rc != HB_OK) return rc;
     }
     rc = staging_insert_rows(&d->staging, d->table, s->runs.uniq_ids, n, s->runs.num_runs, d->cache_rows,
-                             d->row_bytes, p.new_slots, p.last_writer, st);
+                             d->row_bytes, p.new_slots, p.last_writer, true, st);
     if (rc != HB_OK) return rc;
   }
   if (aside) {
