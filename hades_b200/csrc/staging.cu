@@ -74,9 +74,9 @@ __device__ __forceinline__ void warp_add_rows(const float* src_row, float* dst_r
 
 // ---- accumulate through the cache index (cold remote, server.py:546-562) --------------
 // Bound by row traffic (read, read, write of 512 bytes at random places).  Three blocks on an SM: 100,000
-// rows, 391 blocks, took a wave and a third with the two that 112 registers allow (37.5 -> 31.0 us), and no store
-that waits for a load stands ahead of the rows (31.4 -> 28.4).  The
-// sorted lookup keeps its top level in shared memory and stays at two.
+// rows, 391 blocks, took a wave and a third with the two that 112 registers allow (37.5 -> 31.0 us), and no
+// store that waits for a load stands ahead of the rows (31.4 -> 28.4).  The sorted lookup keeps its top level in
+// shared memory and stays at two.
 template <int MODE, int VEC>
 __global__ void __launch_bounds__(kBlock, MODE == HB_LOOKUP_SETASSOC ? 3 : 2) staging_accumulate_cached_kernel(
     IndexView v, hb_staging_t s, const int64_t* ids, const float* grads, int64_t n, const int64_t* n_dev,
