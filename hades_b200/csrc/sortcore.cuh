@@ -362,7 +362,7 @@ struct ClusterCtx {
 
 template <class Src, class Fin, int I>
 __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin fin) {
-  begin_after_previous();
+  wait_for_previous();
   constexpr int T = kClusterT, W = T / 32, B = 1 << kClusterDigit;
   extern __shared__ __align__(16) char smem[];
   ClusterCtx<I> ctx;
@@ -505,6 +505,7 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
     }
     ctx.sync();
   }
+  start_next();  // (from here on its start is hidden as well)
   fin.run(ctx, src);
   ctx.leave();
 }
@@ -619,7 +620,7 @@ static __global__ void sort_grid_begin_kernel(unsigned* barrier) {
 
 template <class Src, class Fin, int I>
 __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, SortGridBufs b, int max_digit, int* err) {
-  begin_after_previous();
+  wait_for_previous();
   extern __shared__ __align__(16) char smem[];
   uint16_t* wcnt = reinterpret_cast<uint16_t*>(smem);
   uint32_t* wmask = reinterpret_cast<uint32_t*>(smem + ((size_t)(kGridT / 32) << max_digit) * 2);
@@ -803,6 +804,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
     out = out == b.kv0 ? b.kv1 : b.kv0;
   }
   ctx.kv = in;
+  start_next();
   fin.run(ctx, src);
 }
 

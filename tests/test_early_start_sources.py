@@ -7,7 +7,7 @@ import re
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent.parent / "hades_b200" / "csrc"
-WAIT = "begin_after_previous"
+WAITS = ("begin_after_previous", "wait_for_previous")
 SETTLED = "load_settled"
 NOT_FUNCTIONS = {"if", "for", "while", "switch", "return", "sizeof", "catch", "alignof", "decltype", "__launch_bounds__"}
 
@@ -53,7 +53,7 @@ def _reached(path):
     names = {}
     for f in functions:
         names.setdefault(f[0], []).append(f)
-    early = [f for f in functions if WAIT + "()" in f[2] and f[0] != WAIT]
+    early = [f for f in functions if f[0] not in WAITS and any(w + "()" in f[2] for w in WAITS)]
     seen, todo = [], list(early)
     while todo:
         f = todo.pop()
@@ -78,7 +78,8 @@ def test_the_wait_is_the_first_statement():
     early, _ = _all()
     assert len({f[0] for f in early}) >= 17
     for name, _, body in early:
-        assert re.match(r"\{\s*" + WAIT + r"\(\);", body), name
+        assert re.match(r"\{\s*(" + "|".join(WAITS) + r")\(\);", body), name
+        assert ("wait_for_previous()" in body) == ("start_next()" in body), name
 
 
 def test_what_starts_early_waits():
