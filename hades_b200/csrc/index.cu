@@ -46,7 +46,6 @@ struct SetSource {
   const unsigned long long* heads;
   const int32_t* batch;
   __host__ __device__ int known_bits() const { return 0; }
-  static constexpr bool starts_early() { return true; }
   __device__ __forceinline__ int64_t count() const { return !LONG_LISTS || batch[2] == batch[0] ? n : 0; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
     const int64_t x = ids[i];
@@ -147,7 +146,6 @@ struct ListedSource {
   const int64_t* cut;
   int64_t lines;
   __host__ __device__ int known_bits() const { return 0; }
-  static constexpr bool starts_early() { return true; }
   __device__ __forceinline__ int64_t count() const { return *n_dev < n ? *n_dev : n; }
   __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
     key = (unsigned long long)mod_nonneg(ids[i], lines);

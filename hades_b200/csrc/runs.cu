@@ -42,9 +42,7 @@ struct IdSource {
   int64_t sentinel;
   int* err;
   int bits;  // stated by the caller
-  bool early;  // the launch may start under the kernel before it
   __host__ __device__ int known_bits() const { return bits; }
-  bool starts_early() const { return early; }
   __device__ __forceinline__ int64_t count() const {
     if (!n_dev) return n;
     const int64_t d = *n_dev;
@@ -740,7 +738,7 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
                    int id_bits, const int8_t* class_table, int64_t table_len, int64_t* const* class_ids_out,
                    int64_t* class_counts_out, int64_t* uniq_ids_out, int64_t* num_unique_out, unsigned* zero,
                    int64_t zero_words, void* workspace, size_t workspace_bytes, hb_runs_t* runs_out,
-                   cudaStream_t st, const RunsResolve* resolve, bool early) {
+                   cudaStream_t st, const RunsResolve* resolve) {
   HB_CHECK_ARG(runs_out != nullptr, "hb_runs_build: runs_out is null");
   HB_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "hb_runs_build: n out of range");
   HB_CHECK_ARG(n == 0 || ids, "hb_runs_build: null ids");
@@ -776,7 +774,7 @@ int hb::runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const in
   const int64_t sentinel = runs_sentinel(id_bits);
   runs_out->perm = s.perm;
   IdSource src{ids, n, seg_counts ? nullptr : n_dev, seg_counts, (uint32_t)(seg_counts ? seg_cap : 1), sentinel,
-               device_error_word(), id_bits, early};
+               device_error_word(), id_bits};
   static_assert(kResolvedMax <= kSortOneEach, "one run per thread");
   auto run = [&](auto fin) -> int {
     fin.table = class_table;

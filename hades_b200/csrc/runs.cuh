@@ -54,12 +54,12 @@ constexpr int64_t kResolvedMax = 8192;
 
 // hb_runs_build (without the sorted ids of the entries, which nothing here reads: runs_keys).  zero: words that the
 // sort's own launch sets to zero, for `resolve` or the launches after it.  resolve (up to kResolvedMax ids): done with
-// every run, through the lines of the sets.  early: the launch may start under the kernel before it.
+// every run, through the lines of the sets.
 int runs_build(const int64_t* ids, int64_t n, const int64_t* n_dev, const int64_t* seg_counts, int64_t seg_cap,
                int id_bits, const int8_t* class_table, int64_t table_len, int64_t* const* class_ids_out,
                int64_t* class_counts_out, int64_t* uniq_ids_out, int64_t* num_unique_out, unsigned* zero,
                int64_t zero_words, void* workspace, size_t workspace_bytes, hb_runs_t* runs_out, cudaStream_t st,
-               const RunsResolve* resolve = nullptr, bool early = true);
+               const RunsResolve* resolve = nullptr);
 
 // The sorted id of every entry (hb_runs_t.keys) of runs built in a plan that has room for them.
 int runs_keys(const int64_t* seg_counts, int id_bits, void* workspace, hb_runs_t* runs, cudaStream_t st);

@@ -7,8 +7,6 @@
 
 using namespace hb;
 
-static constexpr int64_t kHostBoundMax = 16384;
-
 extern "C" {
 
 size_t hb_segsum_runs_workspace_bytes(int64_t n, int64_t dim) { return seg_plan(nullptr, n, dim).total; }
@@ -94,13 +92,9 @@ int hb_unique_segsum_f32(const int64_t* ids, const float* grads, const int64_t* 
                          split ? split->out_ids[2] : nullptr};
   char* seg_ws = static_cast<char*>(workspace) + runs_bytes;
   const SegPlan s = seg_plan(seg_ws, n, dim);
-  // A caller that reads the count is ready for the next call about when the sums of a short list end: what counts is
-  // then the host's time, of which launches that do not start early take less (12,345 x 47: 28.4 us, with 29.3).
-  const bool early = n > kHostBoundMax;
   int rc = runs_build(ids, n, n_dev, seg_counts, seg_cap, id_bits, split ? split->table : nullptr,
                       split ? split->table_len : 0, split ? cls_ids : nullptr, split ? split->class_counts : nullptr,
-                      uniq_ids, num_unique, s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream, nullptr,
-                      early);
+                      uniq_ids, num_unique, s.done, s.max_ctas, workspace, runs_bytes, &runs, (cudaStream_t)stream);
   if (rc != HB_OK) return rc;
   if (runs_out) {
     rc = runs_keys(seg_counts, id_bits, workspace, &runs, (cudaStream_t)stream);
@@ -109,7 +103,7 @@ int hb_unique_segsum_f32(const int64_t* ids, const float* grads, const int64_t* 
   }
   if (!n_dev && !seg_counts) runs.n_dev = nullptr;  // all entries: nothing to wait for
   return segsum_runs(&runs, grads, cnt_in, dim, mean, sums, counts, split, seg_ws, workspace_bytes - runs_bytes, true,
-                     early, (cudaStream_t)stream);
+                     true, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -834,7 +834,7 @@ int sort_launch_cluster(const Src& src, const Fin& fin, int ctas, cudaStream_t s
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (HB_LAUNCH_NEXT)
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = src.starts_early() && !stream_captures(st) ? 2 : 1;
+  cfg.numAttrs = stream_captures(st) ? 1 : 2;
   HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, src, fin));
   count_launch();
   return HB_OK;
