@@ -227,14 +227,21 @@ struct InFlight {
   }
 };
 
-// n ids as signed 32-bit numbers; false: some do not fit.
+// n ids as signed 32-bit numbers; false: some do not fit, found out within 512 ids of the first that does not, or at
+// once from the last (sorted ids).  (Ids beyond 32 bits, 32,768 / 65,536: 47 / 78 us as in 64 bits, 54 / 87 where all of a part was
+// narrowed first; one such id amid others near the end of a part still 54 / 71.)
 __attribute__((optimize("O3"))) bool narrow(const int64_t* __restrict__ from, int32_t* __restrict__ to, int64_t n) {
-  uint64_t off = 0;  // (an id that fits lies in [0, 2^32) from -2^31 on)
-  for (int64_t i = 0; i < n; ++i) {
-    off |= ((uint64_t)from[i] + 0x80000000ull) >> 32;
-    to[i] = (int32_t)from[i];
+  if (from[n - 1] != (int32_t)from[n - 1]) return false;
+  for (int64_t at = 0; at < n; at += 512) {
+    const int64_t end = n - at < 512 ? n : at + 512;
+    uint64_t off = 0;  // (an id that fits lies in [0, 2^32) from -2^31 on)
+    for (int64_t i = at; i < end; ++i) {
+      off |= ((uint64_t)from[i] + 0x80000000ull) >> 32;
+      to[i] = (int32_t)from[i];
+    }
+    if (off) return false;
   }
-  return off == 0;
+  return true;
 }
 __attribute__((optimize("O3"))) void widen(const int32_t* __restrict__ from, int64_t* __restrict__ to, int64_t n) {
   for (int64_t i = 0; i < n; ++i) to[i] = from[i];

@@ -428,3 +428,18 @@ def test_host_lookups_of_ids_at_the_edge_of_32_bits(cuda_lib, n, top):
     for q in (ids, other):
         want, _ = ix.cuda_lookup_found(torch.from_numpy(np.ascontiguousarray(q)).cuda())
         _eq(ix.lookup(torch.from_numpy(np.ascontiguousarray(q))).numpy(), want.cpu().numpy(), "slots")
+
+
+@pytest.mark.parametrize("n,at", [(1, 0), (512, 511), (513, 0), (1025, 511), (1025, 512), (1025, 1023), (40_000, 19_999),
+                                  (40_000, 20_000), (40_000, 39_998), (70_001, 30_000)])
+def test_host_lookups_with_one_id_beyond_32_bits(cuda_lib, n, at):
+    """Parts are narrowed 512 ids at a time until one does not fit; then the part crosses in 64 bits."""
+    from hades_b200 import EmbCacheLib as E
+
+    rng = np.random.default_rng(n + at)
+    ix = E.IndexCache(4000, f"one_wide{n}_{at}", True, False)
+    ids = rng.integers(0, 3000, n, dtype=np.int64)
+    ids[at] += 1 << 32  # its low half is an id of the cache
+    ix.cuda_add(torch.arange(3000).cuda())
+    want, _ = ix.cuda_lookup_found(torch.from_numpy(ids).cuda())
+    _eq(ix.lookup(torch.from_numpy(ids)).numpy(), want.cpu().numpy(), "slots")
