@@ -174,13 +174,63 @@ def test_rows_of_odd_width_as_composed(cuda_lib, dim, optimizer):
     _run_pair(a, b, _steps(_small("odd", dim), 7))
 
 
+@pytest.mark.parametrize("flags", [{}, {"insert_misses": False}, {"touch_lru": False},
+                                   {"insert_misses": False, "touch_lru": False}], ids=lambda f: "_".join(f) or "default")
 @pytest.mark.parametrize("n", [1, 33, 513, 8191, 8192, 8193])
-def test_runs_looked_up_in_the_launch_of_the_sort(cuda_lib, n):
+def test_runs_looked_up_in_the_launch_of_the_sort(cuda_lib, n, flags):
     """Up to 8,192 ids a run is looked up where the sort writes it, above in a launch of its own; the runs of a warp
     lie in two chunks of 32, whose counts cut the list of misses (miss_cap)."""
-    a, b = _pair(f"resolve_{n}")
+    a, b = _pair(f"resolve_{n}_" + "_".join(flags), **flags)
     a.miss_cap = b.miss_cap = max(n // 8, 1)
     _run_pair(a, b, [(ids[:n], g[:n]) for ids, g in _steps(_small("resolve", batch=8193), 4, seed=n)])
+
+
+@pytest.mark.parametrize("n", [40, 8192, 8193])
+def test_ids_outside_of_the_table_as_composed(cuda_lib, n):
+    """Negative ids are a run of their own, which sorts last; ids behind the table have no class and no row.  Their
+    output rows stay as they were, the status word tells."""
+    from hades_b200 import _lib
+
+    a, b = _pair(f"outside_{n}")
+    for ids, g in _steps(_small("outside", batch=n), 3, seed=n):
+        ids[::7], ids[3::11] = -1, 30_000 + n % 2000
+        outs = [torch.full_like(g, 7.0) for _ in range(2)]
+        ra, rb = a.step(ids, g, outs[0]), b.step(ids, g, outs[1])
+        assert _lib.device_status() != 0
+        assert torch.equal(outs[0], outs[1]) and torch.equal(ra[2], rb[2])
+        assert (outs[0][ids < 0] == 7.0).all() and (outs[0][ids >= 30_000] == 7.0).all()
+    sa, sb = _state(a), _state(b)
+    for k in sb:
+        assert torch.equal(sa[k], sb[k]), k
+
+
+@pytest.mark.parametrize("n,aside,optimizer,mode,miss_cap,dim", [
+    (100_000, False, "adam", 0, 1 << 17, 32), (100_000, True, "adagrad", 0, 700, 32),
+    (100_001, False, "adam", 0, 700, 32), (100_001, True, "adam", 0, 1 << 17, 32), (100_001, True, "adagrad", 1, 700, 32),
+    (150_001, False, "adagrad", 1, 1 << 17, 3), (150_001, True, "adam", 0, 700, 47), (282_624, True, "adam", 1, 1 << 17, 16),
+    (303_105, False, "adam", 0, 1 << 17, 128)])
+def test_steps_with_a_second_pass_as_composed(cuda_lib, n, aside, optimizer, mode, miss_cap, dim):
+    """Above 100,000 ids sums, the lookup of the cold ids on the second stream and the update with the ageing in it;
+    with and without a fetch aside, through step() and through its two halves, over several flushes, and with
+    gradients of another batch than the last one fetched."""
+    a, b = _pair(f"second_{n}_{aside}_{optimizer}_{mode}", dim=dim, optimizer=optimizer, lookup_mode=mode)
+    for p in (a, b):
+        p.overlap_fetch, p.miss_cap = aside, miss_cap
+    batches = _steps(_small("second", dim, batch=n), 5)
+    for k, (ids, g) in enumerate(batches):
+        rows = []
+        for p in (a, b):
+            if k % 2 == 0:
+                rows.append(p.step(ids, g))
+            else:
+                rows.append(p.forward(ids, join=False, on_side=aside))
+                p.backward(*((ids, g) if k == 1 else batches[0]))
+                if k == 3:
+                    torch.cuda.synchronize()
+        assert torch.equal(rows[0][0], rows[1][0]) and torch.equal(rows[0][2], rows[1][2]), k
+    sa, sb = _state(a), _state(b)
+    for k in sb:
+        assert torch.equal(sa[k], sb[k]), k
 
 
 @pytest.mark.parametrize("optimizer", ["adam", "adagrad"])
