@@ -786,7 +786,7 @@ int hb_index_add(hb_index_t* h, const int64_t* ids, int64_t n, int64_t* locs,
 
 }  // extern "C"
 
-// lookup of `ids` into locs (or the slots there, ids null), first pass of the ageing
+// lookup of `ids` into locs (or the slots there, ids null: 64 bits only), first pass of the ageing
 template <typename WORD>
 static int touch_mark(hb_index* h, const WORD* ids, int64_t* locs, int64_t n, int mode, const HostPart<WORD>& part,
                       cudaStream_t st) {
@@ -796,10 +796,14 @@ static int touch_mark(hb_index* h, const WORD* ids, int64_t* locs, int64_t n, in
   }
   const int grid = grid_capped(n);
   const TouchMarks t = index_touch_marks(h);
-  if (!ids)
-    HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false, WORD>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
-              part);
-  else if (mode == HB_LOOKUP_SORTED)
+  if constexpr (sizeof(WORD) == sizeof(int64_t)) {
+    if (!ids) {
+      HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SETASSOC, false, WORD>), grid, kBlock, 0, st, h->view, ids, locs, n, t,
+                h->line_hits, part);
+      return HB_OK;
+    }
+  }
+  if (mode == HB_LOOKUP_SORTED)
     HB_LAUNCH((touch_mark_kernel<HB_LOOKUP_SORTED, true, WORD>), grid, kBlock, 0, st, h->view, ids, locs, n, t, h->line_hits,
               part);
   else
@@ -889,8 +893,8 @@ int hb_index_lookup_touch_part(hb_index_t* h, const int64_t* ids, int64_t n, int
 
 int hb_index_lookup_touch_part32(hb_index_t* h, const int32_t* ids, int64_t n, int64_t* locs, int64_t first,
                                  int32_t* host_locs, int64_t* arrived, int mode, hb_stream_t stream) {
-  static_assert(sizeof(int) == sizeof(int32_t), "slots of 32 bits");
-  return lookup_touch_part<int>(h, ids, n, locs, first, host_locs, arrived, mode, (cudaStream_t)stream);
+  // (slots fit: hb_index_create makes no more than 2^31)
+  return lookup_touch_part<int32_t>(h, ids, n, locs, first, host_locs, arrived, mode, (cudaStream_t)stream);
 }
 
 int hb_index_lookup_touch_end(hb_index_t* h, const int64_t* locs, int64_t n, hb_stream_t stream) {

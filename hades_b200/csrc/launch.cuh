@@ -27,7 +27,7 @@ static inline int grid_of_warps(int64_t n, int per, int block, int blocks_per_sm
 // Entries that one cluster of CTAs sorts; more take the whole GPU (sortcore.cuh).
 constexpr int64_t kSortClusterEntries = 65536;
 
-// In a graph kernels are ordered by its edges.
+// Captured launches do not start early: what they would give as programmatic edges of a graph was not measured.
 static inline bool stream_captures(cudaStream_t st) {
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(st, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
