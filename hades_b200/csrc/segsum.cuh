@@ -394,6 +394,11 @@ segsum_kernel(SegArgs a, Epi epi) {
   }
   const int64_t b0 = (int64_t)block * span;
   if (b0 >= n_eff) return;
+  // what the sort found (in a step the lookup of the cold ids comes between)
+  auto found = [](const auto* p) {
+    if constexpr (Epi::kStep) return load_settled(p);
+    else return *p;
+  };
   if (threadIdx.x == 0) s_nfin = 0;
   const int64_t at = b0 + (int64_t)grp * R;
   const bool live = at < n_eff;
@@ -407,7 +412,7 @@ segsum_kernel(SegArgs a, Epi epi) {
     // head flags of the 8 entries around j0 (pieces of a narrow row may begin inside them)
     const unsigned long long f = *reinterpret_cast<const unsigned long long*>(a.head + (j0 & ~7));
     first_partial = ((f >> (8 * (j0 & 7))) & 1ull) == 0ull;
-    u = a.base8[j0 >> 3] - 1 + __popcll(f & ((1ull << (8 * (j0 & 7))) - 1ull));
+    u = found(a.base8 + (j0 >> 3)) - 1 + __popcll(f & ((1ull << (8 * (j0 & 7))) - 1ull));
   }
   const int u_first = u;
   bool open = first_partial;  // a run is open
@@ -449,9 +454,9 @@ segsum_kernel(SegArgs a, Epi epi) {
   uint32_t p_next = 0;
   bool head_next = false, end_next = false;
   auto look = [&](int j) {  // entry j of the sorted order
-    p_next = a.perm[j];
-    head_next = a.head[j] != 0;
-    end_next = j + 1 >= n_eff || a.head[j + 1] != 0;
+    p_next = found(a.perm + j);
+    head_next = found(a.head + j) != 0;
+    end_next = j + 1 >= n_eff || found(a.head + j + 1) != 0;
   };
   if (sub < eg && sub < len) look(j0 + sub);
   for (int s = 0; s < steps; ++s) {
@@ -537,8 +542,8 @@ segsum_kernel(SegArgs a, Epi epi) {
 
   // this CTA's part of a run that crosses CTAs is in the workspace: has every other part arrived?
   auto arrive = [&](int run) {
-    const int first = (int)(a.run_start[run] / span);
-    const int last = (int)((a.run_start[run + 1] - 1) / span);
+    const int first = (int)(found(a.run_start + run) / span);
+    const int last = (int)((found(a.run_start + run + 1) - 1) / span);
     __threadfence();
     __syncwarp(gmask);
     if (sub == 0) {
@@ -574,7 +579,7 @@ segsum_kernel(SegArgs a, Epi epi) {
     }
     if (ended) {
       typename Ops::Row with = Ops::fetch_alone(epi, a, u, sub, vpr);
-      complete(u, acc, with, HAS_CNT ? cacc : (unsigned long long)(a.run_start[u + 1] - a.run_start[u]));
+      complete(u, acc, with, HAS_CNT ? cacc : (unsigned long long)(found(a.run_start + u + 1) - found(a.run_start + u)));
     } else {
       put(a.tail_part + (int64_t)block * a.cols, acc);
       if (HAS_CNT && sub == 0) a.tail_cnt[block] = cacc;
@@ -620,7 +625,7 @@ segsum_kernel(SegArgs a, Epi epi) {
         if (HAS_CNT) w += s_cnt[g];
       }
       typename Ops::Row with = Ops::fetch_alone(epi, a, run, sub, vpr);
-      complete(run, row, with, HAS_CNT ? w : (unsigned long long)(a.run_start[run + 1] - a.run_start[run]));
+      complete(run, row, with, HAS_CNT ? w : (unsigned long long)(found(a.run_start + run + 1) - found(a.run_start + run)));
       if (sub == 0) a.done[first] = 0u;
     }
     __syncthreads();
