@@ -228,8 +228,8 @@ struct InFlight {
 };
 
 // n ids as signed 32-bit numbers; false: some do not fit, found out within 512 ids of the first that does not, or at
-// once from the last (sorted ids).  (Ids beyond 32 bits, 32,768 / 65,536: 47 / 78 us as in 64 bits, 54 / 87 where all of a part was
-// narrowed first; one such id amid others near the end of a part still 54 / 71.)
+// once from the last (sorted ids).  (Ids beyond 32 bits, 32,768 / 65,536: 48 / 79 us, 54 / 87 where all of a part was
+// narrowed first, 47 / 78 without narrowing; one such id amid others near the end of a part still 54 / 71.)
 __attribute__((optimize("O3"))) bool narrow(const int64_t* __restrict__ from, int32_t* __restrict__ to, int64_t n) {
   if (from[n - 1] != (int32_t)from[n - 1]) return false;
   for (int64_t at = 0; at < n; at += 512) {

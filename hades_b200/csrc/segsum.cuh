@@ -161,7 +161,7 @@ struct EpiOps<StoreRows, VEC, G, VPL> {
   using V = typename VecF<VEC>::T;
   static constexpr int kFly = (8 / VPL) < G ? (8 / VPL) : G;
   static constexpr int kBlock = 256;
-  static constexpr int kMinBlocks = 4;
+  static constexpr int kMinBlocks = 4;  // (rows of 128 columns: 64 registers and 30 bytes of spills; with weights 68)
   static constexpr int kPieceMax = 32;
   static constexpr bool kPrefetch = false;
   struct Lane {};
@@ -228,7 +228,7 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
   static constexpr int kFly = VPL == 1 ? 2 : 1;
   // (a step's sums have the bits of StoreRows: a captured step and an eager one may differ in which they use)
   static constexpr int kBlock = STEP ? 256 : 128;
-  static constexpr int kMinBlocks = (VPL > 2 ? 512 : 768) / kBlock;
+  static constexpr int kMinBlocks = (VPL > 2 ? 512 : 768) / kBlock;  // (Adam of a step, VPL 2: 80 and 44 bytes)
   static constexpr int kPieceMax = STEP ? 32 : 16;
   static constexpr bool kPrefetch = true;
   // per-row scalars divide where the stand-alone kernels do (columns one by one), else their reciprocals multiply

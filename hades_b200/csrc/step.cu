@@ -34,10 +34,11 @@ constexpr int kCold = 2;
 // Small batches update rows as their sums become complete (one launch); large ones write the sums and
 // update in a second pass over the distinct ids: the sums then run at the speed of the copy, and the
 // update has many rows in flight whatever the lengths of the runs.
-// The line lies where the two cost the same, at much the same number of ids for all widths (us a step, Adam, at
-// once / in a second pass: 50,000 ids of 16 columns 80 / 75, of 64 91 / 91, of 128 105 / 110, of 256 138 / 151;
-// 100,000: 109 / 102, 131 / 129, 160 / 157, 222 / 225; 200,000: 135 / 123, 170 / 160, 209 / 200, 312 / 300;
-// 2,000,000 of 128 a tenth apart).
+// Where the two cost the same depends on the width: below 25,000 ids of 16 columns, at 25,000 of 64, between 50,000 and
+// 100,000 of 128, at 100,000 of 256.  One line for all of them stands at the last: up to it narrow rows pay 7 % for updates
+// at once (us a step without flushes, Adam, at once / in a second pass: 25,000 ids of 16 columns 62 / 59, of 64
+// 66 / 66, of 128 67 / 76, of 256 78 / 101; 50,000: 73 / 67, 80 / 78, 93 / 100, 114 / 124; 100,000: 97 / 91, 117 / 114,
+// 136 / 132, 176 / 176; 200,000: 126 / 115, 158 / 143, 184 / 169, 256 / 238; 2,000,000 of 128 914 / 883).
 // In a captured step the fetch runs beside the sums instead.
 constexpr int64_t kFuseMax = 100000;
 bool fuses_update(int64_t n) { return n <= kFuseMax; }

@@ -775,7 +775,8 @@ size_t hb_step_workspace_bytes(int64_t n, int64_t dim);
 /* counters: device int64[4] = distinct ids, distinct ids of class 0, 1, 2.  locs nullable.
  * aside: the fetch (out_rows, locs and found too) may still run on the side stream, beside the
  * aggregation of the hb_step_backward that follows; that call, the next one of this handle, or
- * hb_step_join, orders it. */
+ * hb_step_join, orders it.  What the caller enqueues on `stream` between the two calls (thresholds, staging counters,
+ * `dropped`) comes before the backward call. */
 int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, int64_t n, void* out_rows,
                     int64_t* locs, uint8_t* found, int64_t* counters, int aside, void* workspace,
                     size_t workspace_bytes, hb_stream_t stream);
