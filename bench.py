@@ -43,8 +43,8 @@ NVLINK_MEASURED_GBS = 770.0   # peer copy measured on this pool (cudaMemcpyPeer,
 # that source changes the figure is withheld (traffic = null) until it is captured again.
 TRAFFIC_CAPTURE = {
     "kernel_sources": ["hades_b200/csrc/runs.cu", "hades_b200/csrc/index.cuh"],
-    "sha256": "1e5194350bf8200a802c73a7ef4b55a28d60525a650b66497d2ac2f78f8a7213",
-    "bytes_per_launch": 1_093_170_000,
+    "sha256": "c2b1130d29f2935f50a59b419aff5db2baf6def27d99644278332800b200357b",
+    "bytes_per_launch": 1_093_190_000,
     "source": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none (1 pass) over "
               "bench.py --steps 8 --warmup 3 --no-graph at full configuration 2 on one B200: runs_resolve_kernel "
               "17.8 MB read + runs_expand_kernel 106.0 MB read, 969.4 MB written, mean of 6 calls",
