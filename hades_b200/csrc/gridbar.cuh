@@ -9,10 +9,11 @@ namespace hb {
 
 constexpr unsigned kGaveUp = 0x80000000u;
 
-// Word: add(1), load() and swap(was, to) on the word, pause(turn).  want: arrivals when this barrier is complete.
+// Word: add(1) that releases what was written before it, load() that acquires, swap(was, to), pause(turn).  want:
+// arrivals when this barrier is complete.  (An arrival does not wait for the word's value: the first load says all.)
 template <class Word>
 HB_BOTH bool grid_barrier(Word& w, unsigned want, int turns) {
-  if (w.add(1u) & kGaveUp) return false;
+  w.add(1u);
   for (int it = 0; it < turns; ++it) {
     const unsigned seen = w.load();
     if (seen & kGaveUp) return false;
