@@ -47,10 +47,13 @@ struct SetSource {
   const int32_t* batch;
   __host__ __device__ int known_bits() const { return 0; }
   __device__ __forceinline__ int64_t count() const { return !LONG_LISTS || batch[2] == batch[0] ? n : 0; }
-  __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
-    const int64_t x = ids[i];
-    if (x < 0) return false;  // unusable (padding)
-    key = (unsigned long long)mod_nonneg(x, lines);
+  __device__ __forceinline__ bool fetch(int64_t i, int64_t& id) const {
+    id = ids[i];
+    return true;
+  }
+  __device__ __forceinline__ bool accept(int64_t id, unsigned long long& key) const {
+    if (id < 0) return false;  // unusable (padding)
+    key = (unsigned long long)mod_nonneg(id, lines);
     return !LONG_LISTS || heads[key] == (((unsigned long long)(uint32_t)batch[0] << 32) | kLongList);
   }
 };
@@ -100,7 +103,7 @@ struct AddFinish {
   __device__ __forceinline__ void give_up(Ctx& ctx, const Src& src) const {
     for (uint32_t j = ctx.chunk_begin() + threadIdx.x; j < ctx.chunk_end(); j += Ctx::kThreads) {
       unsigned long long key;
-      if (Src::kSkips && !src.load(j, key)) continue;
+      if (Src::kSkips && !sort_load(src, j, key)) continue;
       locs[j] = -1;
       if (last_writer) last_writer[j] = 0;
     }
@@ -147,9 +150,13 @@ struct ListedSource {
   int64_t lines;
   __host__ __device__ int known_bits() const { return 0; }
   __device__ __forceinline__ int64_t count() const { return *n_dev < n ? *n_dev : n; }
-  __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
-    key = (unsigned long long)mod_nonneg(ids[i], lines);
+  __device__ __forceinline__ bool fetch(int64_t i, int64_t& id) const {
+    id = ids[i];
     return listed[i] && i < *cut;
+  }
+  __device__ __forceinline__ bool accept(int64_t id, unsigned long long& key) const {
+    key = (unsigned long long)mod_nonneg(id, lines);
+    return true;
   }
 };
 

@@ -48,12 +48,15 @@ struct IdSource {
     const int64_t d = *n_dev;
     return d < n ? (d > 0 ? d : 0) : n;
   }
-  __device__ __forceinline__ bool load(int64_t i, unsigned long long& key) const {
+  __device__ __forceinline__ bool fetch(int64_t i, int64_t& id) const {
     if (seg_counts) {
       const uint32_t seg = (uint32_t)i / seg_cap;
       if ((int64_t)((uint32_t)i - seg * seg_cap) >= seg_counts[seg]) return false;
     }
-    const int64_t id = __ldcg(ids + i);  // (as a plain load: 56 bytes of spills in the sort of 65,537 to 303,104 ids)
+    id = __ldcg(ids + i);  // (as a plain load: 56 bytes of spills in the sort of 65,537 to 303,104 ids)
+    return true;
+  }
+  __device__ __forceinline__ bool accept(int64_t id, unsigned long long& key) const {
     if (id < 0 || id >= sentinel) {
       atomicExch(err, HB_ERR_INVALID);
       return false;
@@ -140,12 +143,13 @@ struct RunsFinish {
     };
     auto wide_id = [&](uint32_t pos) -> int64_t {
       unsigned long long key;
-      return src.load(pos, key) ? (int64_t)key : src.sentinel;
+      return sort_load(src, pos, key) ? (int64_t)key : src.sentinel;
     };
     // A thread takes 8 consecutive entries (whole vectors of positions and head flags to
     // write, one entry of base8, no votes), the CTA 8 * T in a strip.
+    uint32_t at[8];      // their positions
     uint32_t code = 0u;  // per entry 3 bits: 4 | class (3: none) where a run starts, else 0
-    auto classify = [&](uint32_t j0, bool write) -> int4 {
+    auto classify = [&](uint32_t j0) -> int4 {
       int4 c = make_int4(0, 0, 0, 0);
       code = 0u;
       uint2 e[8];
@@ -170,22 +174,8 @@ struct RunsFinish {
           was = id;
         }
       }
-      if (write) {
-        if (j0 + 8 <= end) {
-          uint4* p = reinterpret_cast<uint4*>(perm + j0);
-          p[0] = make_uint4(e[0].y, e[1].y, e[2].y, e[3].y);
-          p[1] = make_uint4(e[4].y, e[5].y, e[6].y, e[7].y);
-        } else {
 #pragma unroll
-          for (int x = 0; x < 8; ++x)
-            if (j0 + x < end) perm[j0 + x] = e[x].y;
-        }
-        // one byte per entry (the allocation holds whole groups of 8)
-        const uint32_t lo = (heads & 1u) | ((heads & 2u) << 7) | ((heads & 4u) << 14) | ((heads & 8u) << 21);
-        const uint32_t h4 = heads >> 4;
-        const uint32_t hi = (h4 & 1u) | ((h4 & 2u) << 7) | ((h4 & 4u) << 14) | ((h4 & 8u) << 21);
-        *reinterpret_cast<uint2*>(head + j0) = make_uint2(lo, hi);
-      }
+      for (int x = 0; x < 8; ++x) at[x] = e[x].y;
       if (!table) {
 #pragma unroll
         for (int x = 0; x < 8; ++x) code |= ((heads >> x) & 1u) << (3 * x + 2);
@@ -213,6 +203,23 @@ struct RunsFinish {
       }
       return c;
     };
+    auto put_entries = [&](uint32_t j0) {
+      if (j0 >= end) return;
+      if (j0 + 8 <= end) {
+        uint4* p = reinterpret_cast<uint4*>(perm + j0);
+        p[0] = make_uint4(at[0], at[1], at[2], at[3]);
+        p[1] = make_uint4(at[4], at[5], at[6], at[7]);
+      } else {
+#pragma unroll
+        for (int x = 0; x < 8; ++x)
+          if (j0 + x < end) perm[j0 + x] = at[x];
+      }
+      // one byte per entry (the allocation holds whole groups of 8)
+      auto flag = [&](int x) -> uint32_t { return (code >> (3 * x + 2)) & 1u; };
+      const uint32_t lo = flag(0) | (flag(1) << 8) | (flag(2) << 16) | (flag(3) << 24);
+      const uint32_t hi = flag(4) | (flag(5) << 8) | (flag(6) << 16) | (flag(7) << 24);
+      *reinterpret_cast<uint2*>(head + j0) = make_uint2(lo, hi);
+    };
     // a thread's counts -> those of the threads ahead in its warp and of the whole warp
     auto scan_warp = [&](const int4& c, int4& total) -> int4 {
       const unsigned long long v = (unsigned long long)(uint32_t)(c.x | (c.y << 16)) | ((unsigned long long)(uint32_t)(c.z | (c.w << 16)) << 32);
@@ -229,10 +236,14 @@ struct RunsFinish {
     };
     uint32_t kept = 0u;  // the codes of the first of two strips
     const int strips = (int)((end - begin + 8 * T - 1) / (8 * T));
+    // (stores ahead of the barrier are what it waits for)
+    const bool late = Ctx::kStoresLate && strips <= 1 && ctx.ctas > 1;
     int4 mine = make_int4(0, 0, 0, 0), lanes = mine, warps, cta, ahead, all;
 #pragma unroll 1
     for (int q = 0; q < strips; ++q) {
-      const int4 c = classify(begin + q * (8 * T) + threadIdx.x * 8, true);
+      const uint32_t j0 = begin + q * (8 * T) + threadIdx.x * 8;
+      const int4 c = classify(j0);
+      if (!late) put_entries(j0);
       int4 total;
       lanes = scan_warp(c, total);
       mine.x += total.x; mine.y += total.y; mine.z += total.z; mine.w += total.w;
@@ -240,6 +251,7 @@ struct RunsFinish {
     }
     sort_warp_sums<W>(mine, s_sum, warps, cta);
     if (!ctx.prefix(cta, ahead, all)) return give_up(ctx, src);
+    if (late && strips == 1) put_entries(begin + threadIdx.x * 8);
 #pragma unroll 1
     for (int q = 0; q < strips; ++q) {
       const uint32_t strip = begin + q * (8 * T);
@@ -247,7 +259,7 @@ struct RunsFinish {
       if (strips > 1) {
         int4 total, c = make_int4(0, 0, 0, 0);
         if (strips > 2) {
-          c = classify(j0, false);
+          c = classify(j0);
         } else {
           const uint32_t last = code;  // strip 1 was classified last: its codes stay for the next turn
           if (q == 0) code = kept;

@@ -102,6 +102,15 @@ namespace cg = cooperative_groups;
 // key of an entry that takes no part: larger than any other at every width (all ones)
 constexpr uint32_t kSortNone = 0xffffffffu;
 
+// A source's entry i: fetch() brings its id, false where it takes no part; accept() makes the key of an id, false for
+// one that is left out.  (Apart, so that the ids of a thread are on their way at once: what accept() does
+// with a bad id kept the next load behind it.)
+template <class Src>
+__device__ __forceinline__ bool sort_load(const Src& src, int64_t i, unsigned long long& key) {
+  int64_t id;
+  return src.fetch(i, id) && src.accept(id, key);
+}
+
 struct SortDigits {
   int passes, width, bits;
   bool wide;  // keys of more than 32 bits: digits come from the source, by position
@@ -264,14 +273,14 @@ struct SortClusterSmem {
   uint32_t* base;    // [bins]
   uint32_t* warp;    // [32]
   int4* sums;        // [2 * warps + 1]
-  int4* cta4;        // [3]: [0] read by the peers, [1..2] sums of the peers
-  uint4* seen;       // [2]: [0] read by the peers
+  int4* cta4;        // [16 + 2]: stored by the peers; what lies ahead, all
+  uint4* seen;       // [16]: stored by the peers
 };
 
 static inline size_t sort_cluster_smem_bytes(int items) {
   constexpr int W = kClusterT / 32, B = 1 << kClusterDigit;
   return (size_t)kClusterT * items * sizeof(uint2) + (size_t)W * B * 6 + 2 * B * 4 + 32 * 4 + (2 * W + 1) * sizeof(int4) +
-         3 * sizeof(int4) + 2 * sizeof(uint4);
+         18 * sizeof(int4) + 16 * sizeof(uint4);
 }
 
 // what a finish sees: the sorted entries chunk by chunk, barriers and exchanges between the CTAs
@@ -281,6 +290,9 @@ struct ClusterCtx {
   static constexpr int kItems = ITEMS;
   static constexpr int kChunk = kClusterT * ITEMS;
   static constexpr bool kBehindAll = false;
+  // Stores of a finish behind its barrier, which would wait for them; its entries are kept in registers till then (the
+  // grid has none to spare: 1,048,576 ids 62.5 -> 63.2 us, 2,000,000 103.6 -> 105.6).
+  static constexpr bool kStoresLate = true;
   SortClusterSmem s;
   int count;   // entries that were sorted
   uint32_t* scratch;  // shared memory, 8 * kThreads words, free after the sort
@@ -294,7 +306,8 @@ struct ClusterCtx {
   }
   __device__ __forceinline__ uint32_t chunk_begin() const { return SortChunks(count, kChunk).begin(rank); }
   __device__ __forceinline__ uint32_t chunk_end() const { return SortChunks(count, kChunk).end(rank); }
-  // a sorted entry of this chunk, or the last one of the chunk before
+  // a sorted entry of this chunk, or the last one of the chunk before: that one ahead of prefix() only (nobody's
+  // shared memory is read after it, so that CTAs leave without waiting for each other)
   __device__ __forceinline__ uint2 get(int j) const {
     const int at = j - rank * kChunk;
     if (at >= 0) return s.kv[at];
@@ -317,30 +330,22 @@ struct ClusterCtx {
       all = mine;
       return true;
     }
-    if (threadIdx.x == 0) s.cta4[0] = mine;
+    // stored at every peer: behind the barrier nobody waits for somebody else's shared memory
+    if ((int)threadIdx.x < ctas) *cg::this_cluster().map_shared_rank(s.cta4 + rank, threadIdx.x) = mine;
     sync();
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-      int4 v = make_int4(0, 0, 0, 0);
-      if (lane < ctas) v = *cg::this_cluster().map_shared_rank(s.cta4, lane);
-      int4 a, b;
-      a.x = __reduce_add_sync(0xffffffffu, v.x);
-      a.y = __reduce_add_sync(0xffffffffu, v.y);
-      a.z = __reduce_add_sync(0xffffffffu, v.z);
-      a.w = __reduce_add_sync(0xffffffffu, v.w);
-      if (lane >= rank) v = make_int4(0, 0, 0, 0);
-      b.x = __reduce_add_sync(0xffffffffu, v.x);
-      b.y = __reduce_add_sync(0xffffffffu, v.y);
-      b.z = __reduce_add_sync(0xffffffffu, v.z);
-      b.w = __reduce_add_sync(0xffffffffu, v.w);
+    if (threadIdx.x < 128) {  // a warp per component
+      const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+      const int v = lane < ctas ? reinterpret_cast<const int*>(s.cta4 + lane)[c] : 0;
+      const int b = __reduce_add_sync(0xffffffffu, lane < rank ? v : 0);
+      const int a = __reduce_add_sync(0xffffffffu, v);
       if (lane == 0) {
-        s.cta4[1] = b;
-        s.cta4[2] = a;
+        reinterpret_cast<int*>(s.cta4 + 16)[c] = b;
+        reinterpret_cast<int*>(s.cta4 + 17)[c] = a;
       }
     }
     __syncthreads();
-    before = s.cta4[1];
-    all = s.cta4[2];
+    before = s.cta4[16];
+    all = s.cta4[17];
     return true;
   }
   // shared memory written before it, the peers' too, is seen after it
@@ -363,10 +368,6 @@ struct ClusterCtx {
     barrier();
     return buf;
   }
-  // before a CTA leaves: no peer reads its shared memory any more
-  __device__ __forceinline__ void leave() {
-    if (ctas > 1) cg::this_cluster().sync();
-  }
 };
 
 template <class Src, class Fin, int I>
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
     s.base = reinterpret_cast<uint32_t*>(p); p += B * 4;
     s.warp = reinterpret_cast<uint32_t*>(p); p += 32 * 4;
     s.sums = reinterpret_cast<int4*>(p); p += (2 * W + 1) * sizeof(int4);
-    s.cta4 = reinterpret_cast<int4*>(p); p += 3 * sizeof(int4);
+    s.cta4 = reinterpret_cast<int4*>(p); p += 18 * sizeof(int4);
     s.seen = reinterpret_cast<uint4*>(p);
   }
   auto cluster = cg::this_cluster();
@@ -401,6 +402,14 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
   SortDigits dig;
   {
     unsigned lo = 0, hi = 0, none = 0;
+    const bool known = sort_known_digits(src.known_bits(), kClusterDigit, dig);
+    // (the peers have to run before something is stored at them)
+    if (!known && ctx.ctas > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    int64_t id[I];
+    unsigned part = 0u;
+#pragma unroll
+    for (int i = 0; i < I; ++i)
+      if (first + i * 32 < n && src.fetch(first + i * 32, id[i])) part |= 1u << i;
 #pragma unroll
     for (int i = 0; i < I; ++i) {
       const int j = first + i * 32;
@@ -408,7 +417,7 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
       v[i] = (uint32_t)j;
       if (j < n) {
         unsigned long long key;
-        if (src.load(j, key)) {
+        if (((part >> i) & 1u) && src.accept(id[i], key)) {
           k[i] = (uint32_t)key;
           lo |= (unsigned)key;
           hi |= (unsigned)(key >> 32);
@@ -417,7 +426,6 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
         }
       }
     }
-    const bool known = sort_known_digits(src.known_bits(), kClusterDigit, dig);
     ctx.wide = false;
     ctx.none = true;
     if (!known) {
@@ -427,26 +435,21 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
       uint4* per_warp = reinterpret_cast<uint4*>(s.sums);
       if (lane == 0) per_warp[warp] = make_uint4(lo, hi, none, 0u);
       __syncthreads();
-      if (warp == 0) {
-        const uint4 x = lane < W ? per_warp[lane] : make_uint4(0u, 0u, 0u, 0u);
-        lo = __reduce_or_sync(0xffffffffu, x.x);
-        hi = __reduce_or_sync(0xffffffffu, x.y);
-        none = __reduce_or_sync(0xffffffffu, x.z);
-        if (lane == 0) s.seen[0] = make_uint4(lo, hi, none, 0u);
-      }
-      ctx.sync();
+      uint4 x = lane < W ? per_warp[lane] : make_uint4(0u, 0u, 0u, 0u);
       if (ctx.ctas > 1) {
         if (warp == 0) {
-          uint4 x = make_uint4(0u, 0u, 0u, 0u);
-          if (lane < ctx.ctas) x = *cluster.map_shared_rank(s.seen, lane);
-          lo = __reduce_or_sync(0xffffffffu, x.x);
-          hi = __reduce_or_sync(0xffffffffu, x.y);
-          none = __reduce_or_sync(0xffffffffu, x.z);
-          if (lane == 0) s.seen[1] = make_uint4(lo, hi, none, 0u);
+          x.x = __reduce_or_sync(0xffffffffu, x.x);
+          x.y = __reduce_or_sync(0xffffffffu, x.y);
+          x.z = __reduce_or_sync(0xffffffffu, x.z);
         }
-        __syncthreads();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        if ((int)threadIdx.x < ctx.ctas) *cluster.map_shared_rank(s.seen + ctx.rank, threadIdx.x) = x;
+        ctx.sync();
+        x = lane < ctx.ctas ? s.seen[lane] : make_uint4(0u, 0u, 0u, 0u);
       }
-      const uint4 x = s.seen[ctx.ctas > 1 ? 1 : 0];
+      x.x = __reduce_or_sync(0xffffffffu, x.x);
+      x.y = __reduce_or_sync(0xffffffffu, x.y);
+      x.z = __reduce_or_sync(0xffffffffu, x.z);
       dig = sort_digits(x.x, x.y, x.z != 0u, kClusterDigit);
       ctx.wide = dig.wide;
       ctx.none = x.z != 0u;
@@ -472,7 +475,7 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
       for (int i = 0; i < I; ++i)
         if (first + i * 32 < n) {
           unsigned long long key;
-          k[i] = src.load(v[i], key) ? (uint32_t)(key >> bit) : kSortNone;
+          k[i] = sort_load(src, v[i], key) ? (uint32_t)(key >> bit) : kSortNone;
         }
     }
     const int shift = dig.wide ? 0 : bit;
@@ -516,7 +519,6 @@ __global__ void __launch_bounds__(kClusterT, 1) sort_cluster_kernel(Src src, Fin
   }
   start_next();  // (from here on its start is hidden as well)
   fin.run(ctx, src);
-  ctx.leave();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -526,6 +528,7 @@ template <int ITEMS>
 struct GridCtx {
   static constexpr int kThreads = kGridT;
   static constexpr int kItems = ITEMS;
+  static constexpr bool kStoresLate = false;
   static constexpr bool kBehindAll = true;  // ids are: the launch does not start early (sort_launch_grid)
   const uint2* kv;     // the sorted entries
   uint32_t* scratch;   // shared memory, 8 * kThreads words, free after the sort
@@ -673,7 +676,7 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
         k[i] = kSortNone;
         if (j < end) {
           unsigned long long key;
-          if (src.load(j, key)) {
+          if (sort_load(src, j, key)) {
             k[i] = (uint32_t)key;
             lo |= (unsigned)key;
             hi |= (unsigned)(key >> 32);
@@ -725,17 +728,19 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
     // keys of a tile into k[] (already there for the first pass of a chunk of one tile)
     auto load_tile = [&](int t) {
       const uint32_t first = ctx.first(t);
+      // (the keys of a pass in a loop of their own, all on their way at once: 2,000,000 ids 111.0 -> 103.6 us, 1,048,576
+      // 64.5 -> 62.5; the ids four at a time 113, 68.6)
+      if (dig.wide || (!in && nt > 1)) {
 #pragma unroll
-      for (int i = 0; i < I; ++i) {
-        const uint32_t j = first + i * 32;
-        if (j >= end) continue;
-        unsigned long long key;
-        if (dig.wide)
-          k[i] = src.load(in ? __ldcg(&in[j].y) : j, key) ? (uint32_t)(key >> bit) : kSortNone;
-        else if (in)
-          k[i] = __ldcg(&in[j].x);
-        else if (nt > 1)
-          k[i] = src.load(j, key) ? (uint32_t)key : kSortNone;
+        for (int i = 0; i < I; ++i) {
+          const uint32_t j = first + i * 32;
+          unsigned long long key;
+          if (j < end) k[i] = sort_load(src, in ? __ldcg(&in[j].y) : j, key) ? (uint32_t)(dig.wide ? key >> bit : key) : kSortNone;
+        }
+      } else if (in) {
+#pragma unroll
+        for (int i = 0; i < I; ++i)
+          if (first + i * 32 < end) k[i] = __ldcg(&in[first + i * 32].x);
       }
     };
     auto rank_tile = [&](int t) -> uint32_t {  // the tile's count of digit threadIdx.x
