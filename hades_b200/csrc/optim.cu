@@ -104,13 +104,18 @@ __global__ void __launch_bounds__(kBlock, 4) sparse_adam_kernel(
 // The vector path of both update rules (dim % 4 == 0, 16-byte aligned rows).  A warp takes 32
 // rows per round: lane l works out the per-row scalars of row l once (for Adam the two bias
 // corrections, whose powf would otherwise be issued for every 16 bytes of the row), then the
-// warp walks the rows, G lanes per row and kOptRows rows in flight, taking the scalars by
-// shuffle.
-template <typename E, bool ADAM>
+// warp walks the rows, G lanes per row with W values each, taking the scalars by shuffle.
+// Bound by HBM as long as the warps of an SM hide each other's arithmetic (two roots or divisions a value).  Rows of 32
+// bytes a lane (rows_of_8), one in flight per lane group, against two of 16 bytes (us): Adagrad 600,000 x 64 fp16
+// 128.9 -> 116.5, 524,288 x 128 228 -> 222, 40,000 x 128 23.4 -> 21.8, Adam 300,000 x 64 fp16 107.6 -> 99.4, 200,000 x 256
+// 249 -> 236, 524,288 x 128 331.6 -> 330.7 (5.7 TB/s; without the arithmetic 313).  One row of 16 bytes a lane and more
+// warps: 200,000 x 100 for Adam 140 -> 147.
+template <typename E, bool ADAM, int W>
 __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
     const int64_t* ids, const float* grads, const int64_t* cnt, int64_t n, const int64_t* n_dev, int64_t dim,
     RowMap map, float* step, float* s0, float* s1, E* emb, AdamParams p, int glog2, int rpw) {
   begin_after_previous();
+  constexpr int kFly = W == 8 ? 1 : 2;  // rows in flight per lane group
   // rpw: rows a warp takes per round (32, or fewer so that a short list still fills the GPU)
   n = effective_n(n, n_dev);
   const int lane = threadIdx.x & 31;
@@ -118,7 +123,6 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int G = 1 << glog2, rpp = 32 >> glog2;
   const int sub = lane & (G - 1), which = lane >> glog2;
-  const int64_t vpr = dim >> 2;
   for (int64_t base = warp * rpw; base < n; base += nwarps * rpw) {
     const int64_t i = base + lane;
     const int64_t row = (lane < rpw && i < n) ? map(ids[i]) : -1;
@@ -133,46 +137,44 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
       }
       if (cnt) rc = 1.0f / (float)cnt[i];  // grad / cnt, sparse_optim.py:608-611
     }
-    for (int pass = 0; pass * rpp < rpw; pass += kOptRows) {
-      int64_t rw[kOptRows];
-      float a[kOptRows], b[kOptRows], c[kOptRows];
-      const float4* gp[kOptRows];
+    for (int q0 = 0; q0 < rpw; q0 += rpp * kFly) {
+      int64_t rw[kFly];
+      float a[kFly], b[kFly], c[kFly];
+      const float* gp[kFly];
 #pragma unroll
-      for (int u = 0; u < kOptRows; ++u) {
-        const int q = ((pass + u) * rpp + which) & 31;
-        rw[u] = __shfl_sync(0xffffffffu, row, q);
-        a[u] = __shfl_sync(0xffffffffu, ra, q);
-        b[u] = __shfl_sync(0xffffffffu, rb, q);
-        c[u] = __shfl_sync(0xffffffffu, rc, q);
-        if ((pass + u) * rpp + which >= rpw) rw[u] = -1;
-        gp[u] = reinterpret_cast<const float4*>(grads + (base + q) * dim);
+      for (int u = 0; u < kFly; ++u) {
+        const int q = q0 + u * rpp + which;
+        rw[u] = __shfl_sync(0xffffffffu, row, q & 31);
+        a[u] = __shfl_sync(0xffffffffu, ra, q & 31);
+        b[u] = __shfl_sync(0xffffffffu, rb, q & 31);
+        c[u] = __shfl_sync(0xffffffffu, rc, q & 31);
+        if (q >= rpw) rw[u] = -1;
+        gp[u] = grads + (base + q) * dim;
       }
-      for (int64_t k = sub; k < vpr; k += G) {
-        float4 gg[kOptRows], mm[kOptRows], vv[kOptRows], ee[kOptRows];
+      for (int k = sub * W; k < (int)dim; k += G * W) {
+        Floats<W> gg[kFly], mm[kFly], vv[kFly], ee[kFly];
 #pragma unroll
-        for (int u = 0; u < kOptRows; ++u)
+        for (int u = 0; u < kFly; ++u)
           if (rw[u] >= 0) {
-            gg[u] = __ldcg(gp[u] + k);
-            mm[u] = reinterpret_cast<const float4*>(s0 + rw[u] * dim)[k];
-            if (ADAM) vv[u] = reinterpret_cast<const float4*>(s1 + rw[u] * dim)[k];
-            ee[u] = EmbIO<E>::load4(emb + rw[u] * dim + 4 * k);
+            const int64_t at = rw[u] * dim + k;
+            load_row(gp[u] + k, gg[u]);
+            load_row(s0 + at, mm[u]);
+            if (ADAM) load_row(s1 + at, vv[u]);
+            load_row(emb + at, ee[u]);
           }
 #pragma unroll
-        for (int u = 0; u < kOptRows; ++u)
+        for (int u = 0; u < kFly; ++u)
           if (rw[u] >= 0) {
-            float* g4 = reinterpret_cast<float*>(&gg[u]);
-            float* m4 = reinterpret_cast<float*>(&mm[u]);
-            float* v4 = reinterpret_cast<float*>(&vv[u]);
-            float* e4 = reinterpret_cast<float*>(&ee[u]);
+            const int64_t at = rw[u] * dim + k;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float g = cnt ? g4[j] * c[u] : g4[j];
-              if (ADAM) adam_value(g, m4[j], v4[j], e4[j], a[u], b[u], p);
-              else adagrad_value(g, m4[j], e4[j], p);
+            for (int j = 0; j < W; ++j) {
+              const float g = gg[u].x[j] * c[u];
+              if (ADAM) adam_value(g, mm[u].x[j], vv[u].x[j], ee[u].x[j], a[u], b[u], p);
+              else adagrad_value(g, mm[u].x[j], ee[u].x[j], p);
             }
-            reinterpret_cast<float4*>(s0 + rw[u] * dim)[k] = mm[u];
-            if (ADAM) reinterpret_cast<float4*>(s1 + rw[u] * dim)[k] = vv[u];
-            EmbIO<E>::store4(emb + rw[u] * dim + 4 * k, ee[u]);
+            store_row(s0 + at, mm[u]);
+            if (ADAM) store_row(s1 + at, vv[u]);
+            store_row(emb + at, ee[u]);
           }
       }
     }
@@ -186,6 +188,11 @@ int rows_per_warp_for(int64_t n, int glog2) {
   int rpw = 32;
   while (rpw > min_rows && ceil_div(n, rpw) < (int64_t)sm_count() * 48) rpw >>= 1;
   return rpw;
+}
+
+// 32 bytes a lane (of fp16 rows 16)
+bool rows_of_8(int64_t dim, uintptr_t state_bits, const void* emb, int emb_elem_bytes) {
+  return dim % 8 == 0 && (state_bits & 31) == 0 && ((uintptr_t)emb & (8 * emb_elem_bytes - 1)) == 0;
 }
 
 int grid_for_warps(int64_t n, int rpw) {
@@ -272,22 +279,23 @@ int hb_sparse_adam(const int64_t* ids, const float* grads, const int64_t* cnt, i
   const AdamParams p{(float)lr, (float)beta1, (float)beta2, (float)eps, (float)(1.0 - beta1),
                      (float)(1.0 - beta2)};
   const RowMap map{id_offset, id_stride, rows};
-  const uintptr_t bits = (uintptr_t)grads | (uintptr_t)mem | (uintptr_t)power | (uintptr_t)emb;
-  const bool vec4 = dim % 4 == 0 && (bits & 15) == 0;
-  const int glog2 = group_log2_for(vec4 ? dim / 4 : dim);
+  const uintptr_t bits = (uintptr_t)grads | (uintptr_t)mem | (uintptr_t)power;
+  const bool vec4 = dim % 4 == 0 && dim < (1 << 30) && ((bits | (uintptr_t)emb) & 15) == 0;
+  const bool vec8 = vec4 && rows_of_8(dim, bits, emb, emb_elem_bytes);
+  const int glog2 = group_log2_for(vec8 ? dim / 8 : (vec4 ? dim / 4 : dim));
   const int grid = grid_for_groups(n, glog2);
   const int rpw = rows_per_warp_for(n, glog2);
   cudaStream_t st = (cudaStream_t)stream;
 #define HB_ADAM(E, V)                                                                          \
   HB_LAUNCH((sparse_adam_kernel<E, V>), grid, kBlock, 0, st, ids, grads, cnt, n, n_dev, dim, map, \
             step, mem, power, (E*)emb, p, glog2)
-#define HB_ADAM_VEC(E)                                                                         \
-  HB_LAUNCH_NEXT((sparse_update_vec_kernel<E, true>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
+#define HB_ADAM_VEC(E, W)                                                                      \
+  HB_LAUNCH_NEXT((sparse_update_vec_kernel<E, true, W>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
             n_dev, dim, map, step, mem, power, (E*)emb, p, glog2, rpw)
   if (emb_elem_bytes == 4) {
-    if (vec4) HB_ADAM_VEC(float); else HB_ADAM(float, false);
+    if (vec8) HB_ADAM_VEC(float, 8); else if (vec4) HB_ADAM_VEC(float, 4); else HB_ADAM(float, false);
   } else {
-    if (vec4) HB_ADAM_VEC(__half); else HB_ADAM(__half, false);
+    if (vec8) HB_ADAM_VEC(__half, 8); else if (vec4) HB_ADAM_VEC(__half, 4); else HB_ADAM(__half, false);
   }
 #undef HB_ADAM_VEC
 #undef HB_ADAM
@@ -304,10 +312,11 @@ int hb_sparse_adagrad(const int64_t* ids, const float* grads, const int64_t* cnt
   HB_CHECK_ARG(n == 0 || (ids && grads && state_sum && emb), "hb_sparse_adagrad: null argument");
   if (n == 0) return HB_OK;
   const RowMap map{id_offset, id_stride, rows};
-  const uintptr_t bits = (uintptr_t)grads | (uintptr_t)state_sum | (uintptr_t)emb;
+  const uintptr_t bits = (uintptr_t)grads | (uintptr_t)state_sum;
   // fp16 rows are read 8 bytes at a time on the vector path
-  const bool vec4 = dim % 4 == 0 && (bits & 15) == 0;
-  const int glog2 = group_log2_for(vec4 ? dim / 4 : dim);
+  const bool vec4 = dim % 4 == 0 && dim < (1 << 30) && ((bits | (uintptr_t)emb) & 15) == 0;
+  const bool vec8 = vec4 && rows_of_8(dim, bits, emb, emb_elem_bytes);
+  const int glog2 = group_log2_for(vec8 ? dim / 8 : (vec4 ? dim / 4 : dim));
   const int grid = grid_for_groups(n, glog2);
   const int rpw = rows_per_warp_for(n, glog2);
   cudaStream_t st = (cudaStream_t)stream;
@@ -315,13 +324,13 @@ int hb_sparse_adagrad(const int64_t* ids, const float* grads, const int64_t* cnt
   HB_LAUNCH((sparse_adagrad_kernel<E, V>), grid, kBlock, 0, st, ids, grads, cnt, n, n_dev, dim, \
             map, state_sum, (E*)emb, (float)lr, (float)eps, glog2)
   const AdamParams p{(float)lr, 0.f, 0.f, (float)eps, 0.f, 0.f};
-#define HB_ADAGRAD_VEC(E)                                                                       \
-  HB_LAUNCH_NEXT((sparse_update_vec_kernel<E, false>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
+#define HB_ADAGRAD_VEC(E, W)                                                                    \
+  HB_LAUNCH_NEXT((sparse_update_vec_kernel<E, false, W>), grid_for_warps(n, rpw), kBlock, 0, st, ids, grads, cnt, n, \
             n_dev, dim, map, nullptr, state_sum, nullptr, (E*)emb, p, glog2, rpw)
   if (emb_elem_bytes == 4) {
-    if (vec4) HB_ADAGRAD_VEC(float); else HB_ADAGRAD(float, false);
+    if (vec8) HB_ADAGRAD_VEC(float, 8); else if (vec4) HB_ADAGRAD_VEC(float, 4); else HB_ADAGRAD(float, false);
   } else {
-    if (vec4) HB_ADAGRAD_VEC(__half); else HB_ADAGRAD(__half, false);
+    if (vec8) HB_ADAGRAD_VEC(__half, 8); else if (vec4) HB_ADAGRAD_VEC(__half, 4); else HB_ADAGRAD(__half, false);
   }
 #undef HB_ADAGRAD_VEC
 #undef HB_ADAGRAD

@@ -55,6 +55,53 @@ template <> struct EmbIO<__half> {
   static __device__ __forceinline__ void store(__half* p, float v) { *p = __float2half_rn(v); }
 };
 
+// W values of a row at once: 4, or 8 from rows that begin at 32 bytes (fp16: 16).  (Plain loads: what the kernel before
+// has written may be read.)
+template <int W> struct Floats { float x[W]; };
+__device__ __forceinline__ void load_row(const float* p, Floats<4>& v) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v.x[0] = t.x; v.x[1] = t.y; v.x[2] = t.z; v.x[3] = t.w;
+}
+__device__ __forceinline__ void load_row(const float* p, Floats<8>& v) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v.x[0]), "=f"(v.x[1]), "=f"(v.x[2]), "=f"(v.x[3]), "=f"(v.x[4]), "=f"(v.x[5]), "=f"(v.x[6]), "=f"(v.x[7])
+               : "l"(p));
+}
+__device__ __forceinline__ void load_row(const __half* p, Floats<4>& v) {
+  const float4 t = EmbIO<__half>::load4(p);
+  v.x[0] = t.x; v.x[1] = t.y; v.x[2] = t.z; v.x[3] = t.w;
+}
+__device__ __forceinline__ void load_row(const __half* p, Floats<8>& v) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const unsigned w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+    v.x[2 * k] = f.x;
+    v.x[2 * k + 1] = f.y;
+  }
+}
+__device__ __forceinline__ void store_row(float* p, const Floats<4>& v) {
+  *reinterpret_cast<float4*>(p) = make_float4(v.x[0], v.x[1], v.x[2], v.x[3]);
+}
+__device__ __forceinline__ void store_row(float* p, const Floats<8>& v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v.x[0]), "f"(v.x[1]), "f"(v.x[2]),
+               "f"(v.x[3]), "f"(v.x[4]), "f"(v.x[5]), "f"(v.x[6]), "f"(v.x[7])
+               : "memory");
+}
+__device__ __forceinline__ void store_row(__half* p, const Floats<4>& v) {
+  EmbIO<__half>::store4(p, make_float4(v.x[0], v.x[1], v.x[2], v.x[3]));
+}
+__device__ __forceinline__ void store_row(__half* p, const Floats<8>& v) {
+  unsigned w[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const __half2 h = __floats2half2_rn(v.x[2 * k], v.x[2 * k + 1]);
+    w[k] = *reinterpret_cast<const unsigned*>(&h);
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // One element of rows that are not a multiple of four columns (bias1, bias2: the bias corrections), as the
 // reference divides; what the row loses.
 __device__ __forceinline__ float adam_elem(float g, float& m, float& v, float bias1, float bias2,

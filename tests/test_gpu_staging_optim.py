@@ -279,3 +279,33 @@ def test_early_launches_come_behind_events_and_copies(cuda_lib):
         torch.cuda.synchronize()
         slots = cold.index.cuda_lookup_found(ids)[0]
         assert torch.equal(cold.remote.grad[slots], torch.full((n, dim), 7.0 * (rnd + 1), device=dev)), rnd
+
+
+@pytest.mark.parametrize("emb_dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("kind", ["adam", "adagrad"])
+@pytest.mark.parametrize("n,dim", [(1, 8), (33, 24), (257, 16), (1000, 128), (700, 256), (90, 264), (40, 1032)])
+def test_updates_of_8_values_a_lane_have_the_bits_of_4(cuda_lib, emb_dtype, kind, n, dim):
+    """Rows of a multiple of 8 columns move 32 bytes a lane where their buffers begin at 32 bytes; gradients that
+    begin 16 bytes further take the form of 16 bytes a lane.  The values are worked out alike: the same bits."""
+    from hades_b200.sparse_optim import ShardedEmbedding, SparseAdagrad, SparseAdam
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n * dim)
+    results = []
+    w0 = torch.randn((2 * n + 5, dim), device="cuda", generator=g) * 0.01
+    ids = torch.randperm(2 * n + 5, device="cuda", generator=g)[:n]
+    flat = torch.randn(n * dim + 4, device="cuda", generator=g) * 1e-3
+    cnt = torch.randint(1, 5, (n,), device="cuda", generator=g)
+    for offset in (0, 4):
+        grads = torch.empty(n * dim + 8, device="cuda")[offset:offset + n * dim].view(n, dim)
+        grads.copy_(flat[:n * dim].view(n, dim))
+        assert grads.data_ptr() % 32 == 4 * offset
+        emb = ShardedEmbedding(2 * n + 5, dim, dtype=emb_dtype)
+        emb.weight.copy_(w0)
+        opt = (SparseAdam if kind == "adam" else SparseAdagrad)(emb, lr=0.01)
+        for c in (None, cnt):
+            opt.update(ids, grads, c, is_unique=True)
+        results.append([emb.weight.clone()] + [v.clone() for v in vars(opt).values() if isinstance(v, torch.Tensor)])
+    assert not torch.equal(results[0][0].float(), w0)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
