@@ -340,20 +340,24 @@ struct Maintain {
   AddEntries e;
   AddState add;
   int touch, insert;
-  int blocks;          // that do this, the first ones of the launch
+  int apart;           // of the blocks every other one ages and the ones between insert
+  int blocks;          // that do this (an even number where they are apart)
+  int spread;          // they are spread over the launch; else the first ones of it
 
   template <int BLOCK>
   __device__ __forceinline__ void run(int block) const {
     const uint32_t hit_number = batch_number(marks.batch), add_number = batch_number(add.batch);
     const int64_t nruns = v.runs(), npos = v.positions();
-    const int64_t cut = insert ? add_cut<BLOCK>(e, nruns) : 0;
-    for (int64_t u = block * (int64_t)BLOCK + threadIdx.x; u < nruns; u += (int64_t)blocks * BLOCK) {
+    const bool ages = touch && !(apart && (block & 1)), inserts = insert && !(apart && !(block & 1));
+    const int64_t cut = inserts ? add_cut<BLOCK>(e, nruns) : 0;
+    const int64_t stride = (apart ? blocks >> 1 : blocks) * (int64_t)BLOCK;
+    for (int64_t u = (apart ? block >> 1 : block) * (int64_t)BLOCK + threadIdx.x; u < nruns; u += stride) {
       const int64_t slot = v.locs[u];
       if (slot >= 0) {
-        if (!touch) continue;
+        if (!ages) continue;
         if (insert && (uint32_t)(add.heads[slot >> 3] >> 32) == add_number) continue;
         touch_run(v, marks, add.lru, u, slot, nruns, npos, hit_number);
-      } else if (insert && e.listed[u]) {
+      } else if (inserts && e.listed[u]) {
         const int64_t id = e.ids[u];
         const int64_t line = mod_nonneg(id, add.lines);
         if (add.heads[line] != (((unsigned long long)add_number << 32) | (unsigned long long)(u + 1))) continue;

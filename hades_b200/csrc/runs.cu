@@ -543,11 +543,16 @@ __global__ void __launch_bounds__(kBlock, RB == 512 ? 4 : 3) runs_expand_kernel(
   const int per = FULL ? 32 : per_arg;
   int block = blockIdx.x, blocks = gridDim.x;
   if (MAINTAIN) {
-    if (block < duty.blocks) {
-      duty.template run<kBlock>(block);
+    int before = block < duty.blocks ? block : duty.blocks, upto = block < duty.blocks ? block + 1 : duty.blocks;
+    if (duty.spread) {
+      before = (int)((unsigned)block * (unsigned)duty.blocks / (unsigned)blocks);
+      upto = (int)((unsigned)(block + 1) * (unsigned)duty.blocks / (unsigned)blocks);
+    }
+    if (upto != before) {
+      duty.template run<kBlock>(before);
       return;
     }
-    block -= duty.blocks;
+    block -= before;
     blocks -= duty.blocks;
   }
   constexpr bool V16 = RB != 0;

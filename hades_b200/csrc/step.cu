@@ -428,6 +428,11 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
   }
   Maintain m;
   memset(&m, 0, sizeof(m));
+  // Few rows: their blocks and those that bring the index up to date run at once, and what counts is the latter's chain
+  // of reads: hits and misses to different blocks (2,000 ids 48.4 -> 48.0 us a step, 65,536 113.3 -> 112.6; 282,624 415.8 ->
+  // 418.8).  Many: those blocks are spread among the rows', not ahead of them (282,624 415.8 -> 413, 2,000,000 750.4 ->
+  // 745.4; 65,536 113.3 -> 114.2).
+  const bool few_rows = n <= kFuseMax;
   if (lists_used) h->sorted_stale = true;  // (ageing leaves the ids where they are)
   if (d->touch_lru || lists_used) {
     m.v = RunsView{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
@@ -436,7 +441,9 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
     m.add = index_add_state(h, static_cast<uint32_t*>(p.add_ws), p.new_slots, p.last_writer);
     m.touch = d->touch_lru;
     m.insert = lists_used;
-    m.blocks = grid_for_runs(n);
+    m.apart = m.touch && m.insert && few_rows;
+    m.blocks = grid_for_runs(n) * (m.apart ? 2 : 1);
+    m.spread = !few_rows;
   }
   rc = runs_expand_maintain(&s->runs, a.run_src, p.run_slots, d->cache_rows, d->table, d->row_bytes, out_rows, locs,
                             found, m, st);
