@@ -455,7 +455,7 @@ __device__ __forceinline__ void warp_put_rows(unsigned long long src, unsigned l
 template <int VEC_BYTES, bool ZERO16>
 __global__ void __launch_bounds__(kBlock, 4) staging_insert_kernel(
     hb_staging_t s, const int64_t* locs, const uint8_t* last_writer, const char* emb_rows, const int64_t* row_index,
-    char* cache_rows, int64_t row_bytes, int64_t n, const int64_t* n_dev, int per) {
+    char* cache_rows, int64_t row_bytes, int64_t n, const int64_t* n_dev) {
   begin_after_previous();
   __shared__ uint8_t s_at[kBlock / 32][32];
   n = effective_n(n, n_dev);
@@ -463,12 +463,15 @@ __global__ void __launch_bounds__(kBlock, 4) staging_insert_kernel(
   uint8_t* const mine = s_at[threadIdx.x >> 5];
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = warp * per; base < n; base += nwarps * per) {
-    const int64_t i = lane < per ? base + lane : n;
-    const int64_t loc = i < n ? locs[i] : -1;
-    const int64_t row = i < n && row_index ? row_index[i] : i;  // row of entry i in emb_rows
+  // Every warp has its share, of the warps that run at once (a round of 32 a warp: five warps' work on four warps' places
+  // for 76,000 new ids among 175,000; a step of 65,536 ids 113.3 -> 111.7 us, others the same).
+  const int64_t end = n * (warp + 1) / nwarps;
+  for (int64_t base = n * warp / nwarps; base < end; base += 32) {
+    const int64_t i = base + lane;
+    const int64_t loc = i < end ? locs[i] : -1;
+    const int64_t row = i < end && row_index ? row_index[i] : i;  // row of entry i in emb_rows
     // of several ids that received the same slot, the last of the batch writes it
-    const bool ok = i < n && last_writer[i] && loc >= 0;
+    const bool ok = i < end && last_writer[i] && loc >= 0;
     const unsigned act = __ballot_sync(0xffffffffu, ok);
     if (act == 0u) continue;
     const int rows = __popc(act);
@@ -697,10 +700,9 @@ int hb::staging_insert_rows(const hb_staging_t* s, const void* emb_rows, const i
   const hb_staging_t st_desc = s ? *s : none;
   const int vb = payload_vec_bytes(row_bytes, emb_rows, cache_rows);
   const bool zero16 = st_desc.dim % 4 == 0 && ((uintptr_t)st_desc.grad & 15) == 0;
-  const int per = items_per_warp(n);
 #define HB_INSERT(VB, Z16)                                                                                     \
-  HB_LAUNCH_NEXT_IF(early, (staging_insert_kernel<VB, Z16>), grid_of_warps(n, per, kBlock, 16), kBlock, 0, st, st_desc, \
-                    locs, last_writer, (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev, per)
+  HB_LAUNCH_NEXT_IF(early, (staging_insert_kernel<VB, Z16>), grid_of_warps(n, 4, kBlock, 4), kBlock, 0, st, st_desc, \
+                    locs, last_writer, (const char*)emb_rows, row_index, (char*)cache_rows, row_bytes, n, n_dev)
   if (vb == 16) {
     if (zero16) HB_INSERT(16, true); else HB_INSERT(16, false);
   } else if (vb == 4) {
