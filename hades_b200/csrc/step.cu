@@ -164,62 +164,54 @@ __global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_
   }
 }
 
-// Summed gradients to where they belong: state and table rows of hot ids, staging rows of cold ones; meanwhile LRU
-// ageing by the lookup that found the staging rows.  A warp takes 32 distinct ids, a lane each for what is worked
-// out once per id, then G lanes per row and kFly rows in flight.  Bound by HBM: rows read and written once.  (With the
-// lookup of the cold ids in it and the ageing behind it: 85,000 hot and 76,000 cold ids of 128 columns for Adam 99 + 12
-// us, now 95; 88,000 and 80,000 118 + 14, now 103.)
+// Summed gradients to where they belong: state and table rows of hot ids, staging rows of cold ones; then LRU
+// ageing by the lookup that found the staging rows.  A warp takes 32 distinct ids a round, a lane each for what is worked
+// out once per id, then G lanes per row.  Bound by HBM: rows read and written once.  As many warps as run at once, 32 an
+// SM with one row in flight per lane group, walk the ids side by side in chunks of eight: no second, partly filled wave,
+// and neighbouring rows of the table at one time (a stretch of its own for every warp: 10 us more).  A step of 282,624
+// ids of 128 columns for Adam (85,000 hot, 76,000 cold) 411 -> 403 us, of 2,000,000 (88,000, 80,000) 751 -> 748; with 24
+// warps and two rows in flight 427, with the ageing ahead of the rows 405.
 template <bool ADAM, int VEC, int G, int VPL>
-__global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 3) step_apply_kernel(hb_runs_t r, SegArgs a,
+__global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 4) step_apply_kernel(hb_runs_t r, SegArgs a,
                                                                             UpdateRows<ADAM, true> epi,
                                                                             const float* sums) {
   begin_after_previous();
   using V = typename VecF<VEC>::T;
   using Ops = EpiOps<UpdateRows<ADAM, true>, VEC, G, VPL>;
-  constexpr int kFly = VPL > 1 ? 1 : 2;
-  constexpr int RPP = 32 / G;
-  int block = blockIdx.x;
-  if (block < epi.touch_blocks) {
-    touch_runs(epi.touched, epi.marks, epi.lru, block, epi.touch_blocks);
+  constexpr int RPP = 32 / G, kChunk = 8;
+  const int row_blocks = (int)gridDim.x - epi.touch_blocks;
+  if ((int)blockIdx.x >= row_blocks) {
+    touch_runs(epi.touched, epi.marks, epi.lru, (int)blockIdx.x - row_blocks, epi.touch_blocks);
     return;
   }
-  block -= epi.touch_blocks;
   const int64_t U = *r.num_runs;
   const int lane = lane_id();
   const int sub = lane & (G - 1), which = lane / G;
   const int vpr = a.cols / VEC;
-  const int64_t warp = (block * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)(gridDim.x - epi.touch_blocks) * blockDim.x) >> 5;
-  for (int64_t u0 = warp * 32; u0 < U; u0 += nwarps * 32) {
-    const int64_t u = u0 + lane;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)row_blocks * blockDim.x) >> 5;
+  auto run_of = [&](int64_t chunk, int q) { return ((chunk + q / kChunk) * nwarps + warp) * kChunk + q % kChunk; };
+  for (int64_t chunk = 0; run_of(chunk, 0) < U; chunk += 32 / kChunk) {
+    const int64_t u = run_of(chunk, lane);
     typename Ops::Lane mine;
     int count = 0;
     if (u < U) {
-      const int64_t begin = r.run_start[u], end = r.run_start[u + 1];
+      count = (int)(r.run_start[u + 1] - r.run_start[u]);
       mine = Ops::lane_of_class(epi, r.dclass[u], r.uniq_ids[u], epi.slots[u]);
-      count = (int)(end - begin);
     }
-    const int rows = U - u0 < 32 ? (int)(U - u0) : 32;
-    for (int t0 = 0; t0 < rows; t0 += RPP * kFly) {
-      V acc[kFly][VPL];
-      typename Ops::Row with[kFly];
-      int cnt[kFly];
+    const unsigned some = __ballot_sync(0xffffffffu, mine.row >= 0);
+    for (int t0 = 0; t0 < 32 && (some >> t0) != 0u; t0 += RPP) {
+      const int q = t0 + which;
+      V acc[VPL];
+      typename Ops::Row with;
+      const int cnt = __shfl_sync(0xffffffffu, count, q);
+      Ops::template fetch<32>(epi, a, mine, q, true, sub, vpr, with);
+      if (with.row < 0) continue;
+      const V* src = reinterpret_cast<const V*>(sums + run_of(chunk, q) * a.dim);
 #pragma unroll
-      for (int x = 0; x < kFly; ++x) {
-        const int q = (t0 + x * RPP + which) & 31;
-        const bool in = t0 + x * RPP + which < rows;
-        cnt[x] = __shfl_sync(0xffffffffu, count, q);
-        Ops::template fetch<32>(epi, a, mine, q, in, sub, vpr, with[x]);
-        if (!in) with[x].row = -1;
-        if (with[x].row >= 0) {
-          const V* src = reinterpret_cast<const V*>(sums + (u0 + q) * a.dim);
-#pragma unroll
-          for (int k = 0; k < VPL; ++k)
-            if (sub + k * G < vpr) acc[x][k] = __ldcs(src + sub + k * G);
-        }
-      }
-#pragma unroll
-      for (int x = 0; x < kFly; ++x) Ops::finish(epi, a, 0, acc[x], with[x], sub, vpr, cnt[x]);
+      for (int k = 0; k < VPL; ++k)
+        if (sub + k * G < vpr) acc[k] = __ldcs(src + sub + k * G);
+      Ops::finish(epi, a, 0, acc, with, sub, vpr, cnt);
     }
   }
 }
@@ -228,10 +220,13 @@ template <bool ADAM, int VEC>
 int launch_apply(const hb_runs_t& r, const SegArgs& a, const UpdateRows<ADAM, true>& epi, const float* sums,
                  cudaStream_t st) {
   const int vpr = a.cols / VEC;
-  int64_t blocks = ceil_div(r.n, kBlock);
-  if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
-  blocks += epi.touch_blocks;
-#define HB_APPLY(G, VPL) HB_LAUNCH_NEXT((step_apply_kernel<ADAM, VEC, G, VPL>), (int)blocks, kBlock, 0, st, r, a, epi, sums)
+#define HB_APPLY(G, VPL)                                                                                              \
+  do {                                                                                                                \
+    int64_t blocks = ceil_div(r.n, kBlock);                                                                           \
+    const int64_t most = (int64_t)sm_count() * (VPL > 1 ? 2 : 4); /* what runs at once */                              \
+    if (blocks > most) blocks = most;                                                                                 \
+    HB_LAUNCH_NEXT((step_apply_kernel<ADAM, VEC, G, VPL>), (int)(blocks + epi.touch_blocks), kBlock, 0, st, r, a, epi, sums); \
+  } while (0)
   if (vpr > 64) HB_APPLY(32, 4);
   else if (vpr > 32) HB_APPLY(32, 2);
   else if (vpr > 16) HB_APPLY(32, 1);
