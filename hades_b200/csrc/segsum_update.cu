@@ -9,12 +9,15 @@ namespace {
 
 // Whether the sum of a run updates its rows at once instead of going through memory (write, read, one
 // launch).  That saves traffic, but rows are updated where their run ends, a few here and there in a warp,
-// while the update kernel takes 32 rows per warp.  Adagrad (us, at once / through memory): 20,000 x 32
-// 45 / 43, 60,000 x 128 71 / 75, 262,144 x 64 139 / 133, 524,288 x 64 194 / 204, 1,048,576 x 64 of fp16 291 / 329.
+// while the update kernel takes 32 rows per warp.  For Adagrad it pays where the sums do not fit in L2 (us, at
+// once / through memory, ids of Zipf 1.1): 60,000 x 128 77 / 74, 262,144 x 64 of fp16 133 / 119, 120,000 x 128 124 / 114,
+// 200,000 x 128 149 / 146, 400,000 x 64 of fp16 154 / 151; 120,000 x 256 158 / 171, 700,000 x 64 231 / 248, 400,000 x 128
+// 249 / 263, 1,048,576 x 64 of fp16 284 / 306.
 // Adam, with two state rows and two powers per row: 5,000 x 100 47 / 37, 60,000 x 128 84 / 85, 200,000 x 128
 // 164 / 144, 700,000 x 128 278 / 268, 1,048,576 x 64 378 / 378: never.
+constexpr int64_t kSumsInL2 = 28000000;  // values
 bool at_once(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt) {
-  if (opt->kind == HB_OPT_ADAM || n <= 32768 || opt->rows >= ((int64_t)1 << 30)) return false;
+  if (opt->kind == HB_OPT_ADAM || n * dim <= kSumsInL2 || opt->rows >= ((int64_t)1 << 30)) return false;
   const uintptr_t bits = (uintptr_t)grads | (uintptr_t)opt->emb | (uintptr_t)opt->s0;
   return dim <= seg_tile(dim % 4 == 0 && (bits & 15) == 0);
 }
