@@ -73,6 +73,7 @@ struct StoreRows {
 // 2^30 rows and slots.
 template <bool ADAM, bool STEP>
 struct UpdateRows {
+  static constexpr bool kAdam = ADAM;
   static constexpr bool kStep = STEP;
   static constexpr bool kWeights = !STEP;  // rows with weights come from several senders
   const int64_t* uniq;        // [U] ids
@@ -84,6 +85,7 @@ struct UpdateRows {
   void* emb;
   AdamParams p;
   // STEP only
+  float* sums;                // [U][dim], where updates come behind the sums (SegWalk)
   const int8_t* dclass;       // [U]
   float* staged;              // [slots][dim]
   const int64_t* slots;       // [U] staging slot of a cold run, -1 = none
@@ -106,6 +108,7 @@ UpdateRows<ADAM, STEP> update_rows(const hb_runs_t* runs, const hb_optim_t* opt)
   epi.emb = opt->emb;
   epi.p = AdamParams{(float)opt->lr, (float)opt->beta1, (float)opt->beta2, (float)opt->eps,
                      (float)(1.0 - opt->beta1), (float)(1.0 - opt->beta2)};
+  epi.sums = nullptr;
   epi.dclass = nullptr;
   epi.staged = nullptr;
   epi.slots = nullptr;
@@ -228,7 +231,7 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
   static constexpr int kFly = VPL == 1 ? 2 : 1;
   // (a step's sums have the bits of StoreRows: a captured step and an eager one may differ in which they use)
   static constexpr int kBlock = STEP ? 256 : 128;
-  static constexpr int kMinBlocks = (VPL > 2 ? 512 : 768) / kBlock;  // (Adam of a step, VPL 2: 80 and 44 bytes)
+  static constexpr int kMinBlocks = (VPL > 2 ? 512 : 768) / kBlock;
   static constexpr int kPieceMax = STEP ? 32 : 16;
   static constexpr bool kPrefetch = true;
   // per-row scalars divide where the stand-alone kernels do (columns one by one), else their reciprocals multiply
@@ -243,36 +246,36 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
     V e[VPL], s0[VPL], s1[ADAM ? VPL : 1];
   };
   static __device__ __forceinline__ bool is_staged(int row) { return STEP && row >= kStaged; }
-  static __device__ __forceinline__ Lane lane(const Epi& o, int run) {
+  static __device__ __forceinline__ int row_of(const Epi& o, int64_t run) {
+    // (all on their way before one of them decides)
+    const int64_t id = o.uniq[run], slot = STEP ? o.slots[run] : -1;
     const int c = STEP ? o.dclass[run] : 1;
-    return lane_of_class(o, c, o.uniq[run], STEP && c == 2 ? o.slots[run] : -1);
+    if (STEP && c == 2) return slot >= 0 ? kStaged + (int)slot : -1;
+    return c == 1 ? (int)o.map(id) : -1;
   }
-  static __device__ __forceinline__ Lane lane_of_class(const Epi& o, int c, int64_t id, int64_t slot) {
+  static __device__ __forceinline__ Lane lane(const Epi& o, int64_t run) {
     Lane l;
-    if (STEP && c == 2) {
-      if (slot >= 0) l.row = kStaged + (int)slot;
-    } else if (c == 1) {
-      l.row = (int)o.map(id);
-      if (ADAM && l.row >= 0) {
-        // state_step = state_step + 1 (per row), sparse_optim.py:624-626
-        l.t = o.step[l.row] + 1.0f;
-        l.ra = 1.0f - powf(o.p.beta1, l.t);
-        l.rb = 1.0f - powf(o.p.beta2, l.t);
-        if (!kDivide) {
-          l.ra = 1.0f / l.ra;
-          l.rb = 1.0f / l.rb;
-        }
+    l.row = row_of(o, run);
+    if (ADAM && l.row >= 0 && !is_staged(l.row)) {
+      // state_step = state_step + 1 (per row), sparse_optim.py:624-626
+      l.t = o.step[l.row] + 1.0f;
+      l.ra = 1.0f - powf(o.p.beta1, l.t);
+      l.rb = 1.0f - powf(o.p.beta2, l.t);
+      if (!kDivide) {
+        l.ra = 1.0f / l.ra;
+        l.rb = 1.0f / l.rb;
       }
     }
     return l;
   }
-  static __device__ __forceinline__ void prefetch(const Epi& o, const SegArgs& a, const Lane& l) {
-    if (l.row < 0) return;
-    if (is_staged(l.row)) {
-      l2_prefetch_row(o.staged + (int64_t)(l.row - kStaged) * a.dim, (int)a.dim * 4);
+  static __device__ __forceinline__ void prefetch(const Epi& o, const SegArgs& a, const Lane& l) { prefetch(o, a, l.row); }
+  static __device__ __forceinline__ void prefetch(const Epi& o, const SegArgs& a, int row) {
+    if (row < 0) return;
+    if (is_staged(row)) {
+      l2_prefetch_row(o.staged + (int64_t)(row - kStaged) * a.dim, (int)a.dim * 4);
       return;
     }
-    const int64_t at = (int64_t)l.row * a.dim;
+    const int64_t at = (int64_t)row * a.dim;
     l2_prefetch_row(o.s0 + at, (int)a.dim * 4);
     if (ADAM) l2_prefetch_row(o.s1 + at, (int)a.dim * 4);
     l2_prefetch_row(reinterpret_cast<const char*>(o.emb) + at * (o.half ? 2 : 4), (int)a.dim * (o.half ? 2 : 4));
@@ -353,17 +356,81 @@ struct EpiOps<UpdateRows<ADAM, STEP>, VEC, G, VPL> {
   }
 };
 
+// Runs first .. first + runs, whose sums are in sums[run], by `nwarps` warps side by side in chunks of eight: a lane
+// each for what is worked out once per id, then G lanes per row.
+template <bool ADAM, int VEC, int G, int VPL>
+__device__ __forceinline__ void apply_runs(const UpdateRows<ADAM, true>& o, const SegArgs& a, const float* sums, int64_t first,
+                                           int64_t runs, int64_t warp, int64_t nwarps) {
+  using V = typename VecF<VEC>::T;
+  using Ops = EpiOps<UpdateRows<ADAM, true>, VEC, G, VPL>;
+  constexpr int RPP = 32 / G, kChunk = 8;
+  const int lane = threadIdx.x & 31;
+  const int sub = lane & (G - 1), which = lane / G;
+  const int vpr = a.cols / VEC;
+  auto run_of = [&](int64_t chunk, int q) { return ((chunk + q / kChunk) * nwarps + warp) * kChunk + q % kChunk; };
+  for (int64_t chunk = 0; run_of(chunk, 0) < runs; chunk += 32 / kChunk) {
+    const int64_t u = run_of(chunk, lane);
+    typename Ops::Lane mine;
+    int count = 0;
+    if (u < runs) {
+      count = (int)(a.run_start[first + u + 1] - a.run_start[first + u]);
+      mine = Ops::lane(o, first + u);
+    }
+    const unsigned some = __ballot_sync(0xffffffffu, mine.row >= 0);
+    for (int t0 = 0; t0 < 32 && (some >> t0) != 0u; t0 += RPP) {
+      const int q = t0 + which;
+      V acc[VPL];
+      typename Ops::Row with;
+      const int cnt = __shfl_sync(0xffffffffu, count, q);
+      Ops::template fetch<32>(o, a, mine, q, true, sub, vpr, with);
+      if (with.row < 0) continue;
+      const V* src = reinterpret_cast<const V*>(sums + (first + run_of(chunk, q)) * a.dim);
+#pragma unroll
+      for (int k = 0; k < VPL; ++k)
+        if (sub + k * G < vpr) acc[k] = __ldcg(src + sub + k * G);
+      Ops::finish(o, a, 0, acc, with, sub, vpr, cnt);
+    }
+  }
+}
+
+// What the walk over the entries does with complete rows: the epilogue at once, or, for Adam in a step, they are stored
+// in the shape of StoreRows (a captured step and an eager one may differ in which they use), and the CTA updates their rows
+// when it has them all.  An update where a run ends holds up the lane groups whose runs go on, and where runs are of
+// very different lengths most warps wait for a few; behind the sums every warp has its share (us a step without flushes,
+// in the walk / behind it: 10,000 x 64 63.1 / 58.9, 50,000 x 32 83.1 / 76.4, 65,536 x 128 111.0 / 107.5, 100,000 x 128
+// 148.2 / 144.6, 100,000 x 256 184 / 179.5; Adagrad, with half the values and half the arithmetic, 65,536 x 128 102.9 /
+// 103.7, 100,000 x 64 114.5 / 115.3.  With all lanes of a warp on one row and 32 warps an SM: 50,000 x 128 of next to no
+// duplicates 106.4 / 108.4, now 104.5).
+template <class Epi, int VEC, int G, int VPL> struct SegWalk {
+  using Ops = EpiOps<Epi, VEC, G, VPL>;
+  static constexpr bool kBehind = false;
+  static constexpr int kMinBlocks = Ops::kMinBlocks;
+  static __device__ __forceinline__ const Epi& out(const Epi& epi) { return epi; }
+};
+template <int VEC, int G, int VPL> struct SegWalk<UpdateRows<true, true>, VEC, G, VPL> {
+  using Ops = EpiOps<StoreRows, VEC, G, VPL>;
+  static constexpr int kMinBlocks = VPL > 2 ? 2 : 3;
+  static constexpr bool kBehind = true;
+  static __device__ __forceinline__ StoreRows out(const UpdateRows<true, true>& epi) {
+    StoreRows o = {};
+    o.sums = epi.sums;
+    return o;
+  }
+};
+
 // ---- the kernel ----------------------------------------------------------------------------------
 constexpr unsigned char kSegHead = 1;    // the piece begins inside a run: a row in s_head
 constexpr unsigned char kSegWhole = 2;   // ... which goes on behind the piece
 constexpr unsigned char kSegTail = 4;    // the piece's last run begins in it and goes on behind it
 
 template <int VEC, int G, int VPL, bool HAS_CNT, class Epi>
-__global__ void __launch_bounds__(EpiOps<Epi, VEC, G, VPL>::kBlock, EpiOps<Epi, VEC, G, VPL>::kMinBlocks)
+__global__ void __launch_bounds__(SegWalk<Epi, VEC, G, VPL>::Ops::kBlock, SegWalk<Epi, VEC, G, VPL>::kMinBlocks)
 segsum_kernel(SegArgs a, Epi epi) {
   begin_after_previous();
   using V = typename VecF<VEC>::T;
-  using Ops = EpiOps<Epi, VEC, G, VPL>;
+  using Walk = SegWalk<Epi, VEC, G, VPL>;
+  using Ops = typename Walk::Ops;
+  const auto& out = Walk::out(epi);
   constexpr int NG = Ops::kBlock / G;
   constexpr int U = Ops::kFly;  // rows whose loads are in flight together
   extern __shared__ __align__(16) float s_rows[];   // [NG][cols] pieces' parts of a run that began earlier
@@ -406,6 +473,21 @@ segsum_kernel(SegArgs a, Epi epi) {
   const int len = n_eff - j0 < R ? n_eff - j0 : R;  // (j0 + R may not be a number: entries are counted from j0)
   const int vpr = a.cols / VEC;  // vectors per row in this pass
 
+  // The runs that begin and end in this CTA, which it updates once they are summed up: their state and table rows are on
+  // their way to L2 meanwhile.
+  int run0 = 0, runs = 0;
+  if constexpr (Walk::kBehind) {
+    auto begun = [&](int j) {  // runs that begin at entry j or before it
+      const unsigned long long f = *reinterpret_cast<const unsigned long long*>(a.head + (j & ~7));
+      return found(a.base8 + (j >> 3)) + __popcll(f & (~0ull >> (8 * (7 - (j & 7)))));
+    };
+    const int e = n_eff - (int)b0 < span ? n_eff : (int)b0 + span;  // (b0 + span may not be a number)
+    run0 = begun((int)b0) - (found(a.head + b0) != 0);
+    runs = begun(e - 1) - 1 + (e == n_eff || found(a.head + e) != 0) - run0;
+    using Rows = EpiOps<Epi, VEC, G, VPL>;
+    for (int r = threadIdx.x; r < runs; r += Ops::kBlock) Rows::prefetch(epi, a, Rows::row_of(epi, run0 + r));
+  }
+
   int u = -1;              // the open run; before the first head of a piece that begins with one: the run before
   bool first_partial = false;
   if (live) {
@@ -432,7 +514,7 @@ segsum_kernel(SegArgs a, Epi epi) {
 #pragma unroll
       for (int v = 0; v < VPL; ++v) vdiv(row[v], d, r);
     }
-    Ops::finish(epi, a, run, row, with, sub, vpr, count);
+    Ops::finish(out, a, run, row, with, sub, vpr, count);
   };
   auto put = [&](float* dst, const V (&row)[VPL]) {
 #pragma unroll
@@ -470,13 +552,13 @@ segsum_kernel(SegArgs a, Epi epi) {
     // (a run that began before the piece is not finished by this group)
     if ((ends >> sub) & 1u) {
       const int begun = __popc(heads & ((2u << sub) - 1u));
-      if (begun || !first_partial) mine = Ops::lane(epi, u + begun);
+      if (begun || !first_partial) mine = Ops::lane(out, u + begun);
     }
     int cv = 1;
     if (HAS_CNT && valid) cv = (int)a.cnt_in[p];
     if (Ops::kPrefetch && valid) {
       l2_prefetch_row(a.grads + (int64_t)p * a.dim + a.col0, a.cols * 4);
-      Ops::prefetch(epi, a, mine);
+      Ops::prefetch(out, a, mine);
     }
     if (s + 1 < steps && sub < eg && at + eg < len) look(j0 + at + eg);
 #pragma unroll 1
@@ -496,7 +578,7 @@ segsum_kernel(SegArgs a, Epi epi) {
             if (k < vpr) val[x][v] = load_settled(src + k);
           }
         }
-        Ops::fetch(epi, a, mine, t0 + x, (ends >> (t0 + x)) & 1u, sub, vpr, with[x]);
+        Ops::fetch(out, a, mine, t0 + x, (ends >> (t0 + x)) & 1u, sub, vpr, with[x]);
       }
 #pragma unroll
       for (int x = 0; x < U; ++x) {
@@ -578,7 +660,7 @@ segsum_kernel(SegArgs a, Epi epi) {
       if (!(s_flag[g] & kSegWhole)) { ended = true; break; }
     }
     if (ended) {
-      typename Ops::Row with = Ops::fetch_alone(epi, a, u, sub, vpr);
+      typename Ops::Row with = Ops::fetch_alone(out, a, u, sub, vpr);
       complete(u, acc, with, HAS_CNT ? cacc : (unsigned long long)(found(a.run_start + u + 1) - found(a.run_start + u)));
     } else {
       put(a.tail_part + (int64_t)block * a.cols, acc);
@@ -624,11 +706,18 @@ segsum_kernel(SegArgs a, Epi epi) {
         add(row, s_rows + g * a.cols);
         if (HAS_CNT) w += s_cnt[g];
       }
-      typename Ops::Row with = Ops::fetch_alone(epi, a, run, sub, vpr);
+      typename Ops::Row with = Ops::fetch_alone(out, a, run, sub, vpr);
       complete(run, row, with, HAS_CNT ? w : (unsigned long long)(found(a.run_start + run + 1) - found(a.run_start + run)));
       if (sub == 0) a.done[first] = 0u;
     }
     __syncthreads();
+  }
+  if constexpr (Walk::kBehind) {
+    constexpr int W = Ops::kBlock / 32;
+    const int warp = threadIdx.x >> 5;
+    for (int f = 0; f < nfin; ++f)  // runs that crossed CTAs: a warp each, of those that may have fewer of the others
+      if (warp == W - 1 - f) apply_runs<Epi::kAdam, VEC, G, VPL>(epi, a, epi.sums, s_fin_run[f], 1, 0, 1);
+    apply_runs<Epi::kAdam, VEC, G, VPL>(epi, a, epi.sums, run0, runs, warp, W);
   }
 }
 
@@ -676,7 +765,7 @@ static inline SegPlan seg_plan(void* ws, int64_t n, int64_t dim) {
 
 template <int VEC, int G, int VPL, class Epi>
 int seg_launch(SegArgs a, const Epi& epi, cudaStream_t st) {
-  using Ops = EpiOps<Epi, VEC, G, VPL>;
+  using Ops = typename SegWalk<Epi, VEC, G, VPL>::Ops;
   a.piece = seg_piece(a.n, G, Ops::kPieceMax);
   const int ng = Ops::kBlock / G;
   int grid = (int)ceil_div(a.n, (int64_t)ng * a.piece);

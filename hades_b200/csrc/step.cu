@@ -176,44 +176,13 @@ __global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 4) step_apply_kernel(hb_
                                                                             UpdateRows<ADAM, true> epi,
                                                                             const float* sums) {
   begin_after_previous();
-  using V = typename VecF<VEC>::T;
-  using Ops = EpiOps<UpdateRows<ADAM, true>, VEC, G, VPL>;
-  constexpr int RPP = 32 / G, kChunk = 8;
   const int row_blocks = (int)gridDim.x - epi.touch_blocks;
   if ((int)blockIdx.x >= row_blocks) {
     touch_runs(epi.touched, epi.marks, epi.lru, (int)blockIdx.x - row_blocks, epi.touch_blocks);
     return;
   }
-  const int64_t U = *r.num_runs;
-  const int lane = lane_id();
-  const int sub = lane & (G - 1), which = lane / G;
-  const int vpr = a.cols / VEC;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)row_blocks * blockDim.x) >> 5;
-  auto run_of = [&](int64_t chunk, int q) { return ((chunk + q / kChunk) * nwarps + warp) * kChunk + q % kChunk; };
-  for (int64_t chunk = 0; run_of(chunk, 0) < U; chunk += 32 / kChunk) {
-    const int64_t u = run_of(chunk, lane);
-    typename Ops::Lane mine;
-    int count = 0;
-    if (u < U) {
-      count = (int)(r.run_start[u + 1] - r.run_start[u]);
-      mine = Ops::lane_of_class(epi, r.dclass[u], r.uniq_ids[u], epi.slots[u]);
-    }
-    const unsigned some = __ballot_sync(0xffffffffu, mine.row >= 0);
-    for (int t0 = 0; t0 < 32 && (some >> t0) != 0u; t0 += RPP) {
-      const int q = t0 + which;
-      V acc[VPL];
-      typename Ops::Row with;
-      const int cnt = __shfl_sync(0xffffffffu, count, q);
-      Ops::template fetch<32>(epi, a, mine, q, true, sub, vpr, with);
-      if (with.row < 0) continue;
-      const V* src = reinterpret_cast<const V*>(sums + run_of(chunk, q) * a.dim);
-#pragma unroll
-      for (int k = 0; k < VPL; ++k)
-        if (sub + k * G < vpr) acc[k] = __ldcs(src + sub + k * G);
-      Ops::finish(epi, a, 0, acc, with, sub, vpr, cnt);
-    }
-  }
+  apply_runs<ADAM, VEC, G, VPL>(epi, a, sums, 0, *r.num_runs, warp, ((int64_t)row_blocks * blockDim.x) >> 5);
 }
 
 template <bool ADAM, int VEC>
@@ -270,6 +239,7 @@ int update_step(hb_step* s, const hb_step_desc_t* d, const ColdArgs& c, SegArgs 
       HB_LAUNCH_NEXT(step_cold_kernel<HB_LOOKUP_SETASSOC>, grid_for_runs(r.n), kBlock, 0, on, v, r, c);
     return HB_OK;
   };
+  epi.sums = sums;
   if (fused) {
     const int rc = look_up(st);
     return rc != HB_OK ? rc : seg_dispatch(a, epi, vec4, st);

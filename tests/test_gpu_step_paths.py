@@ -316,3 +316,20 @@ def test_other_streams_run_beside_the_sort(cuda_lib):
         step.append(at[0].elapsed_time(at[1]))
         beside.append(at[2].elapsed_time(at[3]))
     assert sorted(beside)[20] < 0.2 * sorted(step)[20], (sorted(beside)[20], sorted(step)[20])
+
+
+@pytest.mark.parametrize("dim", [16, 100, 128, 256, 512])
+@pytest.mark.parametrize("n,length", [(1, 1), (63, 1), (64, 64), (65, 7), (130, 129), (1000, 1000), (5000, 37), (5000, 1),
+                                      (40_000, 3), (40_000, 900)])
+def test_runs_of_every_length_updated_by_the_ctas_that_sum_them(cuda_lib, n, length, dim):
+    """Runs inside a piece, across pieces, across CTAs and across many of them, and batches that end inside a CTA's
+    share: the same bits as sums and update one after the other."""
+    a, b = _pair(f"runs_{n}_{length}_{dim}", dim=dim, optimizer="adam")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + length + dim)
+    batches = []
+    for _ in range(2):
+        distinct = torch.randperm(30_000, device="cuda", generator=g)[:max(min(n // length, 30_000), 1)]
+        ids = distinct[torch.arange(n, device="cuda") % distinct.numel()]
+        batches.append((ids[torch.randperm(n, device="cuda", generator=g)], torch.randn((n, dim), device="cuda", generator=g) * 1e-3))
+    _run_pair(a, b, batches)
