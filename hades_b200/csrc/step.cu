@@ -93,9 +93,17 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
   return p;
 }
 
+// slot of a lane's own id (-1: none)
+template <int MODE>
+__device__ __forceinline__ int64_t step_lookup(const IndexView& v, const int64_t* s_top, int64_t id) {
+  if constexpr (MODE == HB_LOOKUP_SORTED) return warp_lookup<MODE>(v, s_top, id);
+  else return lane_lookup(v.line_ids, v.lines, id >= 0, id);
+}
+constexpr int step_lookup_blocks(int mode) { return mode == HB_LOOKUP_SORTED ? 2 : 6; }  // (an SM)
+
 // The lookup of the runs in a launch of its own (resolve_run: as part of the sort's).
 template <int MODE>
-__global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_runs_t r, RunsResolve a) {
+__global__ void __launch_bounds__(kBlock, step_lookup_blocks(MODE)) step_resolve_kernel(IndexView v, hb_runs_t r, RunsResolve a) {
   begin_after_previous();
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
@@ -110,7 +118,7 @@ __global__ void __launch_bounds__(kBlock) step_resolve_kernel(IndexView v, hb_ru
     const int64_t u = u0 + lane;
     const int64_t id = u < U ? r.uniq_ids[u] : -1;
     const bool cold = u < U && r.dclass[u] == kCold;
-    resolved_run<true>(a, u, u < U, id, cold, warp_lookup<MODE>(v, s_top, id));
+    resolved_run<true>(a, u, u < U, id, cold, step_lookup<MODE>(v, s_top, id));
   }
 }
 
@@ -135,7 +143,7 @@ struct ColdArgs {
 // The cold ids: slot now that this batch's misses are in the cache, staging entry (server.py:546-562 without the
 // row), mark for the ageing.
 template <int MODE>
-__global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_t r, ColdArgs a) {
+__global__ void __launch_bounds__(kBlock, step_lookup_blocks(MODE)) step_cold_kernel(IndexView v, hb_runs_t r, ColdArgs a) {
   begin_after_previous();
   __shared__ int64_t s_top[MODE == HB_LOOKUP_SORTED ? kTopMax : 1];
   if (MODE == HB_LOOKUP_SORTED) {
@@ -149,7 +157,7 @@ __global__ void __launch_bounds__(kBlock) step_cold_kernel(IndexView v, hb_runs_
     const int64_t u = u0 + lane_id();
     const bool cold = u < U && r.dclass[u] == kCold;
     const int64_t id = cold ? r.uniq_ids[u] : -1;
-    const int64_t slot = warp_lookup<MODE>(v, s_top, id);
+    const int64_t slot = step_lookup<MODE>(v, s_top, id);
     if (slot >= 0) {
       a.s.idx[slot] = id;
       a.s.iter_threshold[slot] = a.thr_table ? a.thr_table[id] : a.default_thr;
