@@ -529,7 +529,7 @@ struct GridCtx {
   static constexpr int kThreads = kGridT;
   static constexpr int kItems = ITEMS;
   static constexpr bool kStoresLate = false;
-  static constexpr bool kBehindAll = true;  // ids are: the launch does not start early (sort_launch_grid)
+  static constexpr bool kBehindAll = true;  // it starts early under a kernel of its own only (sort_launch_grid)
   const uint2* kv;     // the sorted entries
   uint32_t* scratch;   // shared memory, 8 * kThreads words, free after the sort
   int4* exchange;
@@ -869,11 +869,11 @@ int sort_launch_grid(const Src& src, const Fin& fin, int64_t n, int max_digit, v
                                  (int)sort_grid_smem_bytes(kGridDigit)));
     ready_dev = dev;
   }
-  // Where the sort usually ends at once, what counts is its start behind a kernel that runs: the barrier's word is set
-  // by a kernel whose start, and whose successor's, overlap with that one's end (HB_LAUNCH_NEXT).  A round of the
-  // cold cache 161.0 -> 154.7 us; a step of 282,624 ids, whose sort follows a copy of
-  // the ids, 421.9 -> 425.7, so that the others take a fill.
-  const bool early = Src::kSkips && !stream_captures(st);
+  // The words that have to be zero are set by a kernel whose start, and whose successor's, overlap with the end of the
+  // one before it (HB_LAUNCH_NEXT): a round of the cold cache, whose sort usually ends at once, 161.0 -> 154.7 us, sums of
+  // 524,288 rows 116 -> 113.7, an update of 1,048,576 286 -> 283.5.  The sort itself lives from the end of that kernel's
+  // wait on, behind all that came before (GridCtx::kBehindAll).
+  const bool early = !stream_captures(st);
   const int words = (int)sort_zero_words(max_digit);
   if (early) HB_LAUNCH_NEXT(sort_grid_begin_kernel, (words + 1023) / 1024, 1024, 0, st, b.barrier, words);
   else HB_CUDA(cudaMemsetAsync(b.barrier, 0, words * sizeof(unsigned), st));
