@@ -210,7 +210,15 @@ __global__ void __launch_bounds__(kBlock) accumulate_rows_kernel(
 }
 
 // ---- fused lookup + fetch, LSU ---------------------------------------------------
-template <int MODE, int VB, bool FULL>
+// LANE: a lane probes the line of its own id (rows of up to 512 bytes; with wider ones, which keep a warp busy with few,
+// the fewer warps of the other form are ahead: 500,000 rows of 1,024 bytes 130.7 us, 135 so)
+template <int MODE, bool LANE>
+__device__ __forceinline__ int64_t fetch_lookup(const IndexView& v, const int64_t* s_top, int64_t id) {
+  if constexpr (LANE && MODE == HB_LOOKUP_SETASSOC) return lane_lookup(v.line_ids, v.lines, id);
+  else return warp_lookup<MODE>(v, s_top, id);
+}
+
+template <int MODE, int VB, bool FULL, bool LANE>
 __global__ void __launch_bounds__(kBlock) lookup_fetch_kernel(
     IndexView v, const int64_t* __restrict__ ids, int64_t n, const char* __restrict__ cache_rows,
     const char* __restrict__ backing, int64_t row_bytes, char* __restrict__ out,
@@ -233,7 +241,7 @@ __global__ void __launch_bounds__(kBlock) lookup_fetch_kernel(
   for (int64_t base = warp * per; base < n; base += nwarps * per) {
     const int64_t i = FULL || lane < per ? base + lane : n;
     const int64_t id = i < n ? __ldg(ids + i) : -1;
-    const int64_t slot = warp_lookup<MODE>(v, s_top, id);
+    const int64_t slot = fetch_lookup<MODE, LANE>(v, s_top, id);
     if (i < n) {
       if (locs) locs[i] = slot;
       if (found) found[i] = slot >= 0;
@@ -289,7 +297,7 @@ __global__ void __launch_bounds__(kBlock, MINB) lookup_fetch512_kernel(
   for (int64_t base = warp * per; base < n; base += nwarps * per) {
     const int64_t i = FULL || lane < per ? base + lane : n;
     const int64_t id = i < n ? __ldg(ids + i) : -1;
-    const int64_t slot = warp_lookup<MODE>(v, s_top, id);
+    const int64_t slot = fetch_lookup<MODE, true>(v, s_top, id);
     if (i < n) {
       if (locs) locs[i] = slot;
       if (found) found[i] = slot >= 0;
@@ -749,15 +757,18 @@ int hb_lookup_fetch(hb_index_t* h, const int64_t* ids, int64_t n, const void* ca
   }
   const int vb = vec_bytes_for(row_bytes, {cache_rows, backing_rows, out_rows});
   const int glog2 = group_log2_for(row_bytes / vb);
-  // 1,000 rows of 400 bytes: 6.2 us with 32 rows per warp
-  const int per = items_per_warp(n);
+  // 1,000 rows of 400 bytes: 6.2 us with 32 rows per warp.  Where all warps of 32 rows would run at once, they look up at
+  // one time and move rows at one time: 16 rows a warp and two waves (200,000 rows of 512 bytes 31.1 -> 27.5 us).
+  const bool lane = row_bytes <= 512;
+  int per = items_per_warp(n);
+  if (lane && per == 32 && ceil_div(n, 32) < (int64_t)sm_count() * 48) per = 16;
   const int blocks = grid_of_warps(n, per, kBlock, 16);
   if (vb == 16 && row_bytes == 512) {
-    // dim 128 fp32: the specialised kernel (measured 2-4 % faster than the generic mover;
-    // deeper prefetch or 4 CTAs/SM measured no better: the kernel sits at the random-row
-    // bandwidth of the memory system)
+    // dim 128 fp32: the specialised kernel (measured 2-4 % faster than the generic mover; deeper prefetch measured no
+    // better).  Five CTAs an SM (2,000,000 ids of Zipf 1.05 258 -> 246 us, 400,000 53.8 -> 51.1; three 249, six 244 but
+    // 17 for 100,000 instead of 15); the sorted search has no registers for them.
 #define HB_LF512(MODE, FULL)                                                                       \
-  HB_LAUNCH((lookup_fetch512_kernel<MODE, 3, 1, FULL>), blocks, kBlock, 0, st, h->view, ids, n,     \
+  HB_LAUNCH((lookup_fetch512_kernel<MODE, MODE == HB_LOOKUP_SORTED ? 3 : 5, 1, FULL>), blocks, kBlock, 0, st, h->view, ids, n,     \
             (const char*)cache_rows, (const char*)backing_rows, (char*)out_rows, locs, found, per)
     if (mode == HB_LOOKUP_SORTED) {
       if (per == 32) HB_LF512(HB_LOOKUP_SORTED, true); else HB_LF512(HB_LOOKUP_SORTED, false);
@@ -767,22 +778,24 @@ int hb_lookup_fetch(hb_index_t* h, const int64_t* ids, int64_t n, const void* ca
 #undef HB_LF512
     return HB_OK;
   }
-#define HB_LF(MODE, VB, FULL)                                                                         \
-  HB_LAUNCH((lookup_fetch_kernel<MODE, VB, FULL>), blocks, kBlock, 0, st, h->view, ids, n,       \
+#define HB_LF(MODE, VB, FULL, LANE)                                                                   \
+  HB_LAUNCH((lookup_fetch_kernel<MODE, VB, FULL, LANE>), blocks, kBlock, 0, st, h->view, ids, n, \
             (const char*)cache_rows, (const char*)backing_rows, row_bytes, (char*)out_rows, locs, \
             found, glog2, per)
-#define HB_LF_VB(MODE, FULL)                 \
-  switch (vb) {                              \
-    case 16: HB_LF(MODE, 16, FULL); break;   \
-    case 8: HB_LF(MODE, 8, FULL); break;     \
-    case 4: HB_LF(MODE, 4, FULL); break;     \
-    case 2: HB_LF(MODE, 2, FULL); break;     \
-    default: HB_LF(MODE, 1, FULL); break;    \
+#define HB_LF_VB(MODE, FULL, LANE)                 \
+  switch (vb) {                                    \
+    case 16: HB_LF(MODE, 16, FULL, LANE); break;   \
+    case 8: HB_LF(MODE, 8, FULL, LANE); break;     \
+    case 4: HB_LF(MODE, 4, FULL, LANE); break;     \
+    case 2: HB_LF(MODE, 2, FULL, LANE); break;     \
+    default: HB_LF(MODE, 1, FULL, LANE); break;    \
   }
   if (mode == HB_LOOKUP_SORTED) {
-    if (per == 32) { HB_LF_VB(HB_LOOKUP_SORTED, true) } else { HB_LF_VB(HB_LOOKUP_SORTED, false) }
+    if (per == 32) { HB_LF_VB(HB_LOOKUP_SORTED, true, false) } else { HB_LF_VB(HB_LOOKUP_SORTED, false, false) }
+  } else if (lane) {
+    if (per == 32) { HB_LF_VB(HB_LOOKUP_SETASSOC, true, true) } else { HB_LF_VB(HB_LOOKUP_SETASSOC, false, true) }
   } else {
-    if (per == 32) { HB_LF_VB(HB_LOOKUP_SETASSOC, true) } else { HB_LF_VB(HB_LOOKUP_SETASSOC, false) }
+    if (per == 32) { HB_LF_VB(HB_LOOKUP_SETASSOC, true, false) } else { HB_LF_VB(HB_LOOKUP_SETASSOC, false, false) }
   }
 #undef HB_LF_VB
 #undef HB_LF

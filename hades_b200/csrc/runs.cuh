@@ -111,27 +111,8 @@ __device__ __forceinline__ void resolved_run(const RunsResolve& a, int64_t u, bo
   if (a.touch) a.marks.mark(slot, u);
 }
 
-// A lane probes the line of its own id: all lines are on their way at once, in 36 registers with what the step does about
-// them, so that 48 warps of an SM wait for theirs (eight lanes a line, 32 warps: a step of 282,624 ids 403 -> 397.5 us, of
-// 2,000,000 742.5 -> 740, of 65,536 107.8 -> 106.8).
-__device__ __forceinline__ int64_t lane_lookup(const int64_t* line_ids, int64_t lines, bool valid, int64_t id) {
-  int64_t slot = -1;
-  if (valid) {
-    const int64_t line = mod_nonneg(id, lines);
-    const longlong2* p = reinterpret_cast<const longlong2*>(line_ids + line * kWays);
-    longlong2 k[kWays / 2];
-#pragma unroll
-    for (int w = 0; w < kWays / 2; ++w) k[w] = p[w];
-#pragma unroll
-    for (int w = kWays / 2 - 1; w >= 0; --w) {  // the FIRST way that matches (cache_line.h:49-55)
-      if (k[w].y == id) slot = line * kWays + 2 * w + 1;
-      if (k[w].x == id) slot = line * kWays + 2 * w;
-    }
-  }
-  return slot;
-}
 __device__ __forceinline__ void resolve_run(const RunsResolve& a, int64_t u, bool valid, int64_t id, bool cold) {
-  resolved_run<false>(a, u, valid, id, cold, lane_lookup(a.line_ids, a.lines, valid, id));
+  resolved_run<false>(a, u, valid, id, cold, lane_lookup(a.line_ids, a.lines, valid ? id : -1));
 }
 
 __device__ __forceinline__ int64_t runs_valid_entries(const hb_runs_t& r) {

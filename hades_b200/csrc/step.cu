@@ -97,7 +97,7 @@ StepPlan step_plan(void* ws, int64_t n, int64_t dim) {
 template <int MODE>
 __device__ __forceinline__ int64_t step_lookup(const IndexView& v, const int64_t* s_top, int64_t id) {
   if constexpr (MODE == HB_LOOKUP_SORTED) return warp_lookup<MODE>(v, s_top, id);
-  else return lane_lookup(v.line_ids, v.lines, id >= 0, id);
+  else return lane_lookup(v.line_ids, v.lines, id);
 }
 constexpr int step_lookup_blocks(int mode) { return mode == HB_LOOKUP_SORTED ? 2 : 6; }  // (an SM)
 

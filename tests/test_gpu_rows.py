@@ -220,3 +220,26 @@ def test_shape_errors_raise_like_check():
         E.cudaSet(a, b, i)
     with pytest.raises(RuntimeError, match="float or double"):
         E.cudaFetch2(a.int(), i, a.int())
+
+
+@pytest.mark.parametrize("dim", [4, 33, 128, 129, 256])
+@pytest.mark.parametrize("n", [1, 255, 2_400, 75_775, 75_777, 227_327, 227_329])
+def test_lookup_fetch_at_the_lines_of_its_launch(cuda_lib, n, dim):
+    """Sizes at which the rows a warp takes change, widths on both sides of 512 bytes."""
+    from hades_b200 import EmbCacheLib as E
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + dim)
+    nodes = 50_000
+    index = E.IndexCache(4_000, "lines_of_the_launch", True, False)
+    held = torch.randperm(nodes, device="cuda", generator=g)[:4_000]
+    slots = index.cuda_add(held)
+    where = torch.full((nodes,), -1, dtype=torch.int64, device="cuda")
+    where[held[slots >= 0]] = slots[slots >= 0]
+    table = torch.randn((nodes, dim), device="cuda", generator=g)
+    rows = torch.randn((index.get_capacity(), dim), device="cuda", generator=g)
+    ids = torch.randint(0, nodes, (n,), device="cuda", generator=g)
+    out, locs, found = E.cudaLookupFetch(index, ids, rows, table)
+    want = where[ids]
+    assert torch.equal(locs, want) and torch.equal(found.bool(), want >= 0)
+    assert torch.equal(out, torch.where((want >= 0)[:, None], rows[want.clamp(min=0)], table[ids]))
