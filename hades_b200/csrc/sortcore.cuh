@@ -68,8 +68,10 @@ __host__ __device__ inline int sort_group_ctas(int ctas) { return (ctas + kSortG
 static inline size_t sort_zero_words(int digit) { return kSortBarrierWords + ((size_t)kSortGroups << digit); }
 
 static inline int sort_grid_ctas(int64_t n) {
-  // fewer CTAs where the chunks would get short: a barrier over few CTAs is quicker
-  int64_t g = ceil_div(n, 2048);
+  // Fewer CTAs where the chunks would get short: a barrier over few CTAs is quicker, and a CTA takes all registers of its SM,
+  // so that what runs on other streams meanwhile needs an SM without one.  Up to 128 CTAs an entry a thread (70,000 ids
+  // 32.8 us, with two 33.7), then two.
+  int64_t g = ceil_div(n, n <= 128 * (int64_t)kGridT ? kGridT : 2 * kGridT);
   const int64_t cap = sm_count();
   return (int)(g > cap ? cap : (g < 1 ? 1 : g));
 }
