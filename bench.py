@@ -43,7 +43,7 @@ NVLINK_MEASURED_GBS = 770.0   # peer copy measured on this pool (cudaMemcpyPeer,
 # that source changes the figure is withheld (traffic = null) until it is captured again.
 TRAFFIC_CAPTURE = {
     "kernel_sources": ["hades_b200/csrc/runs.cu", "hades_b200/csrc/index.cuh"],
-    "sha256": "c2b1130d29f2935f50a59b419aff5db2baf6def27d99644278332800b200357b",
+    "sha256": "13326e16062e6367a993969a73874d0900c591db05f8bf16c097de40e49f31f6",
     "bytes_per_launch": 1_093_190_000,
     "source": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none (1 pass) over "
               "bench.py --steps 8 --warmup 3 --no-graph at full configuration 2 on one B200: runs_resolve_kernel "
