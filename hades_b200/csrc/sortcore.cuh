@@ -40,7 +40,7 @@ constexpr int kClusterDigit = 8;       // its bits per pass: counts are exchange
 constexpr int kClusterMaxItems = 8;
 constexpr int64_t kSortOneEach = 16 * (int64_t)kClusterT;  // ... with one entry per thread
 // The cluster's largest input, and its line: it is ahead of the grid as far as its shared memory reaches (us,
-// cluster / grid, ids of 21 to 26 bits: 16,384 18-20 / 43-50, 32,768 22-25 / 44-47, 65,536 30-36 / 43-47).
+// cluster / grid, ids of 21 bits: 24,000 21.4 / 30.8, 32,000 22.4 / 30.6, 45,000 28.2 / 31.5, 65,536 29.5 / 32.4).
 constexpr int64_t kSortClusterMax = 16 * (int64_t)kClusterT * kClusterMaxItems;
 static_assert(kSortClusterMax == kSortClusterEntries, "the line that launches behind a sort go by");
 constexpr int kGridT = 1024;           // threads per CTA of the grid version

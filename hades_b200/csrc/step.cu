@@ -34,13 +34,13 @@ constexpr int kCold = 2;
 // Small batches update rows as their sums become complete (one launch); large ones write the sums and
 // update in a second pass over the distinct ids: the sums then run at the speed of the copy, and the
 // update has many rows in flight whatever the lengths of the runs.
-// Where the two cost the same depends on the width: below 25,000 ids of 16 columns, at 25,000 of 64, between 50,000 and
-// 100,000 of 128, at 100,000 of 256.  One line for all of them stands at the last: up to it narrow rows pay 7 % for updates
-// at once (us a step without flushes, Adam, at once / in a second pass: 25,000 ids of 16 columns 62 / 59, of 64
-// 66 / 66, of 128 67 / 76, of 256 78 / 101; 50,000: 73 / 67, 80 / 78, 93 / 100, 114 / 124; 100,000: 97 / 91, 117 / 114,
-// 136 / 132, 176 / 176; 200,000: 126 / 115, 158 / 143, 184 / 169, 256 / 238; 2,000,000 of 128 914 / 883).
-// In a captured step the fetch runs beside the sums instead.
-constexpr int64_t kFuseMax = 100000;
+// The line lies where the two cost the same (us a step with flushes, Adam, forward and backward called apart, at once / in
+// a second pass: 50,000 ids of 16 columns 72.4 / 72.0, of 64 80.2 / 81.6, of 128 96.6 / 98.6, of 256 128.8 / 127.4; 75,000: 85.9 /
+// 83.9, 100.8 / 97.8, 123.5 / 122.2, 165.0 / 160.9; 100,000: 96.3 / 93.9, 116.7 / 113.3, 139.0 / 133.2, 203.8 / 188.9; Adagrad 50,000
+// of 128 90.5 / 93.6, 75,000 116.5 / 116.4, 100,000 130.1 / 126.9).  In a captured step, and in one call above the line,
+// the fetch runs beside the sums.
+constexpr int64_t kFuseMax = 70000;
+constexpr int64_t kFewRows = 100000;
 bool fuses_update(int64_t n) { return n <= kFuseMax; }
 
 constexpr int kListedWords = 64;  // of the counter, which all warps add to: a line of its own
@@ -405,7 +405,7 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
   // of reads: hits and misses to different blocks (2,000 ids 48.4 -> 48.0 us a step, 65,536 113.3 -> 112.6; 282,624 415.8 ->
   // 418.8).  Many: those blocks are spread among the rows', not ahead of them (282,624 415.8 -> 413, 2,000,000 750.4 ->
   // 745.4; 65,536 113.3 -> 114.2).
-  const bool few_rows = n <= kFuseMax;
+  const bool few_rows = n <= kFewRows;
   if (lists_used) h->sorted_stale = true;  // (ageing leaves the ids where they are)
   if (d->touch_lru || lists_used) {
     m.v = RunsView{p.run_slots, s->runs.perm, s->runs.run_start, s->runs.num_runs, nullptr, n, n, 2};
