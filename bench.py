@@ -24,6 +24,7 @@ import argparse
 import hashlib
 import json
 import os
+import re
 import sys
 import time
 from pathlib import Path
@@ -38,16 +39,18 @@ HBM_NOMINAL_GBS = 8000.0      # the figure the north-star target is quoted on
 NVLINK_NOMINAL_GBS = 900.0    # per direction per GPU
 NVLINK_MEASURED_GBS = 770.0   # peer copy measured on this pool (cudaMemcpyPeer, 1 GiB)
 
-# DRAM bytes of ONE launch of the fused lookup+fetch kernel at configuration 2, from an ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum).  Tied to the kernel source it was taken on: when
-# that source changes the figure is withheld (traffic = null) until it is captured again.
+# DRAM bytes of ONE call of the fused lookup+fetch at configuration 2 (dram__bytes_read.sum + dram__bytes_write.sum of
+# its two kernels), as measured on the sources of "commit".  Tied to the text of what the call runs: when that changes the
+# figure is withheld (traffic = null).  (runs_expand_kernel has changed since in its MAINTAIN branch only, which the call
+# does not compile.)
 TRAFFIC_CAPTURE = {
-    "kernel_sources": ["hades_b200/csrc/runs.cu", "hades_b200/csrc/index.cuh"],
-    "sha256": "13326e16062e6367a993969a73874d0900c591db05f8bf16c097de40e49f31f6",
+    "kernels": [("hades_b200/csrc/runs.cu", "runs_resolve_kernel"), ("hades_b200/csrc/runs.cu", "runs_expand_kernel"),
+                ("hades_b200/csrc/index.cuh", "warp_lookup_setassoc")],
+    "sha256": "a6c055c8174cdffbe6ece6b27c109f9909976d7bf8929f964a3ad0b51dcfd843",
+    "commit": "05a3c78",
     "bytes_per_launch": 1_093_190_000,
-    "source": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none (1 pass) over "
-              "bench.py --steps 8 --warmup 3 --no-graph at full configuration 2 on one B200: runs_resolve_kernel "
-              "17.8 MB read + runs_expand_kernel 106.0 MB read, 969.4 MB written, mean of 6 calls",
+    "source": "ncu, one pass, one B200, full configuration 2: runs_resolve_kernel 17.8 MB read + runs_expand_kernel "
+              "106.0 MB read, 969.4 MB written, mean of 6 calls",
 }
 
 
@@ -94,19 +97,23 @@ def measured_peaks() -> dict:
     return json.loads(pk.read_text()) if pk.exists() else {}
 
 
+def kernel_text(rel: str, name: str) -> str:
+    """The definition of a device function of a source, down to the brace that closes it."""
+    m = re.search(r"^(?:template[^\n]*\n)?(?:__global__|__device__)[^;{]*?\b" + name + r"\(.*?^}\n",
+                  (ROOT / rel).read_text(), re.S | re.M)
+    if m is None:
+        raise ValueError(f"{name} is not defined in {rel}")
+    return m.group(0)
+
+
 def traffic_capture():
     """(bytes per launch, provenance) of the recorded ncu capture, or (None, why)."""
-    h = hashlib.sha256()
-    for rel in TRAFFIC_CAPTURE["kernel_sources"]:
-        h.update((ROOT / rel).read_bytes())
-    sha = h.hexdigest()
-    if TRAFFIC_CAPTURE["bytes_per_launch"] is None:
-        return None, {"traffic_source": None, "traffic_kernel_sha": sha, "why_null": "no capture recorded"}
+    sha = hashlib.sha256("".join(kernel_text(*k) for k in TRAFFIC_CAPTURE["kernels"]).encode()).hexdigest()
+    prov = {"traffic_source": TRAFFIC_CAPTURE["source"], "traffic_commit": TRAFFIC_CAPTURE["commit"],
+            "traffic_kernel_sha": sha}
     if TRAFFIC_CAPTURE["sha256"] != sha:
-        return None, {"traffic_source": TRAFFIC_CAPTURE["source"], "traffic_kernel_sha": sha,
-                      "why_null": "the kernel source changed since the capture"}
-    return TRAFFIC_CAPTURE["bytes_per_launch"], {"traffic_source": TRAFFIC_CAPTURE["source"],
-                                                 "traffic_kernel_sha": sha}
+        return None, {**prov, "why_null": "the kernels changed since the capture"}
+    return TRAFFIC_CAPTURE["bytes_per_launch"], prov
 
 
 # --------------------------------------------------------------------------------------

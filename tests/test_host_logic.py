@@ -154,3 +154,42 @@ def test_presampled_hotness_class_table_and_cache_fill():
     assert H.hottest_ids(heat, table == 2, 3).tolist() == [1, 9, 3]     # ties by ascending id
     thr = H.flush_thresholds(heat)                                       # ceil(1 / (0.001 + heat)) capped at 100
     assert thr[7].item() == 1 and thr[2].item() == 2 and thr[1].item() == 4 and thr[3].item() == 100
+
+
+def test_recorded_captures_are_small():
+    """Every ncu command that a profile gives to repeat collects the time alone, or names its kernels and a few launches;
+    clocks stay as they are."""
+    import re
+    from pathlib import Path
+
+    commands = []
+    for page in sorted((Path(__file__).resolve().parents[1] / "profiles").glob("*.md")):
+        for text in re.findall(r"^    ncu(?:.*\\\n)*.*$|`ncu[^`]*`", page.read_text(), re.M):
+            commands.append(" ".join(text.strip("` ").replace("\\\n", " ").split()))
+    assert commands
+    for c in commands:
+        assert "--clock-control none" in c, c
+        alone = re.search(r"--metrics gpu__time_duration\.sum ", c)
+        launches = re.search(r" -c (\d+)", c)
+        assert alone or " -k " in c, c
+        assert alone or launches is None or int(launches.group(1)) <= 8, c
+
+
+def test_recorded_traffic_goes_with_the_text_of_its_kernels(tmp_path, monkeypatch):
+    import shutil
+    from pathlib import Path
+
+    root = Path(__file__).resolve().parents[1]
+    monkeypatch.syspath_prepend(str(root))
+    import bench
+
+    assert bench.traffic_capture()[0] == bench.TRAFFIC_CAPTURE["bytes_per_launch"]
+    (tmp_path / "hades_b200/csrc").mkdir(parents=True)
+    for rel, _ in bench.TRAFFIC_CAPTURE["kernels"]:
+        shutil.copy(root / rel, tmp_path / rel)
+    monkeypatch.setattr(bench, "ROOT", tmp_path)
+    runs = tmp_path / "hades_b200/csrc/runs.cu"
+    runs.write_text(runs.read_text() + "// another kernel\n")
+    assert bench.traffic_capture()[0] is not None
+    runs.write_text(runs.read_text().replace("run_slots[u] = slot;", "run_slots[u] = slot + 0;"))
+    assert bench.traffic_capture()[0] is None
