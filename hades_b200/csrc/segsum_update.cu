@@ -16,10 +16,13 @@ namespace {
 // Adam, with two state rows and two powers per row: 5,000 x 100 47 / 37, 60,000 x 128 84 / 85, 200,000 x 128
 // 164 / 144, 700,000 x 128 278 / 268, 1,048,576 x 64 378 / 378: never.
 constexpr int64_t kSumsInL2 = 28000000;  // values
-bool at_once(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt) {
-  if (opt->kind == HB_OPT_ADAM || n * dim <= kSumsInL2 || opt->rows >= ((int64_t)1 << 30)) return false;
+bool can_at_once(int64_t dim, const float* grads, const hb_optim_t* opt) {
+  if (opt->kind == HB_OPT_ADAM || opt->rows >= ((int64_t)1 << 30)) return false;
   const uintptr_t bits = (uintptr_t)grads | (uintptr_t)opt->emb | (uintptr_t)opt->s0;
   return dim <= seg_tile(dim % 4 == 0 && (bits & 15) == 0);
+}
+bool at_once(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt) {
+  return n * dim > kSumsInL2 && can_at_once(dim, grads, opt);
 }
 
 size_t runs_bytes_of(int64_t n) { return align_up(make_runs_plan(nullptr, n, false).total, 256); }
@@ -45,13 +48,16 @@ int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* 
                "hb_unique_update_f32: embedding must be fp32 (4) or fp16 (2)");
   HB_CHECK_ARG(opt->rows > 0 && opt->id_stride > 0, "hb_unique_update_f32: bad sizes");
   if (n == 0) return HB_OK;
-  const size_t need = hb_unique_update_workspace_bytes(n, dim, grads, opt);
+  // A workspace of a larger batch that is updated at once has no room for the sums: this one is updated at once too.
+  const bool can = can_at_once(dim, grads, opt);
+  const size_t least = runs_bytes_of(n) + seg_plan(nullptr, n, dim).total;
+  const size_t need = least + (can ? 0 : sums_bytes(n, dim));
   if (!workspace || workspace_bytes < need) {
     set_error("hb_unique_update_f32: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
     return HB_ERR_WORKSPACE;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  const bool once = at_once(n, dim, grads, opt);
+  const bool once = at_once(n, dim, grads, opt) || (can && workspace_bytes < least + sums_bytes(n, dim));
   float* sums = static_cast<float*>(workspace);  // first: on a 256-byte boundary
   char* runs_ws = static_cast<char*>(workspace) + (once ? 0 : sums_bytes(n, dim));
   const size_t runs_bytes = runs_bytes_of(n);

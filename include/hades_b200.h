@@ -432,7 +432,9 @@ typedef struct hb_optim {
 
 /* hb_unique_segsum_f32 and the row update of the merged rows (SparseAdam.update on ids that repeat,
  * python/EmbCache/sparse_optim.py:608-681), through memory or, where that is faster, as soon as a row's
- * sum is complete; ids, n_dev, seg_counts, seg_cap, id_bits as for hb_unique_segsum_f32. */
+ * sum is complete; ids, n_dev, seg_counts, seg_cap, id_bits as for hb_unique_segsum_f32.
+ * A workspace for n ids serves fewer.  Through memory takes n * dim floats more than at once, so that the bytes for
+ * Adagrad fall where the latter begins; fewer ids in a workspace without that room are updated at once. */
 size_t hb_unique_update_workspace_bytes(int64_t n, int64_t dim, const float* grads, const hb_optim_t* opt /* host */);
 int hb_unique_update_f32(const int64_t* ids, const float* grads, const int64_t* cnt_in /* nullable */, int64_t n,
                          const int64_t* n_dev /* nullable */, const int64_t* seg_counts /* nullable */,

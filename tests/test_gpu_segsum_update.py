@@ -81,6 +81,62 @@ def test_adagrad_at_the_edge_of_updating_at_once(cuda_lib, dtype, n, dim):
     test_update_of_repeated_ids(cuda_lib, "adagrad", dtype, n, dim)
 
 
+def _update_in(opt, ids, grads, cnt, id_bits, workspace_bytes):
+    """hb_unique_update_f32 with a workspace of that size; its return code."""
+    import ctypes as C
+
+    from hades_b200 import _lib
+
+    ws = torch.empty(workspace_bytes, dtype=torch.uint8, device="cuda")
+    desc = _lib.OptimDesc(*opt._fields())
+    rc = _lib.load().hb_unique_update_f32(ids.data_ptr(), grads.data_ptr(), _lib.ptr(cnt), ids.numel(), None, None, 0,
+                                          grads.size(1), id_bits, 1, C.addressof(desc), ws.data_ptr(), workspace_bytes,
+                                          _lib.stream_ptr())
+    torch.cuda.synchronize()
+    return rc
+
+
+def _workspace_bytes(opt, n, dim, grads):
+    import ctypes as C
+
+    from hades_b200 import _lib
+
+    desc = _lib.OptimDesc(*opt._fields())
+    return _lib.load().hb_unique_update_workspace_bytes(n, dim, grads.data_ptr(), C.addressof(desc))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("largest,n,dim", [(1_048_576, 437_500, 64), (437_501, 437_500, 64), (2_000_000, 32_768, 16),
+                                           (300_000, 4_097, 100), (700_000, 33_001, 47), (300_000, 129, 130),
+                                           (200_000, 9_001, 256), (100_000, 33_001, 512), (4_000_000, 1, 8)])
+def test_adagrad_in_the_workspace_of_a_larger_batch(cuda_lib, dtype, largest, n, dim):
+    """A buffer for the largest batch, which is updated at once, serves smaller ones; one byte below what both need is
+    refused and nothing happens."""
+    from hades_b200.sparse_optim import ShardedEmbedding, SparseAdagrad
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n + dim)
+    rank, world, num = 1, 3, 30_000
+    emb = ShardedEmbedding(num, dim, rank, world, dtype=dtype, init_sigma=0.01, seed=n)
+    opt = SparseAdagrad(emb, lr=LR)
+    ids = torch.randint(0, emb.rows, (n,), device="cuda", generator=gen) * world + rank
+    grads = (1 + torch.rand((n, dim), device="cuda", generator=gen)) * 1e-3
+    cnt = torch.randint(1, 5, (n,), device="cuda", generator=gen)
+    given = _workspace_bytes(opt, largest, dim, grads)
+    for weights in (None, cnt):
+        w, s0 = emb.weight.double(), opt.state_sum.double()
+        assert _update_in(opt, ids, grads, weights, 20, given) == 0
+        _reference("adagrad", ids, grads, weights, w, s0, None, None, rank, world)
+        # (the bounds of test_update_of_repeated_ids)
+        assert float((opt.state_sum.double() - s0).abs().max() / s0.abs().max()) < 1e-5
+        err = (emb.weight.double() - w).abs() / w.abs().clamp(min=1e-3)
+        assert float(err.max()) < (2e-3 if dtype == torch.float16 else 1e-4), float(err.max())
+    least = _workspace_bytes(opt, n, dim, grads) - (n * dim * 4 + 255) // 256 * 256
+    before = emb.weight.clone()
+    assert _update_in(opt, ids, grads, cnt, 20, least - 1) != 0
+    assert torch.equal(emb.weight, before)
+
+
 @pytest.mark.parametrize("kind", ["adam", "adagrad"])
 def test_fewer_rows_than_ids_are_refused(cuda_lib, kind):
     from hades_b200.sparse_optim import ShardedEmbedding, SparseAdagrad, SparseAdam
