@@ -178,11 +178,17 @@ __global__ void __launch_bounds__(kBlock, step_lookup_blocks(MODE)) step_cold_ke
 // SM with one row in flight per lane group, walk the ids side by side in chunks of eight: no second, partly filled wave,
 // and neighbouring rows of the table at one time (a stretch of its own for every warp: 10 us more).  A step of 282,624
 // ids of 128 columns for Adam (85,000 hot, 76,000 cold) 411 -> 403 us, of 2,000,000 (88,000, 80,000) 751 -> 748; with 24
-// warps and two rows in flight 427, with the ageing ahead of the rows 405.
+// warps and two rows in flight 427, with the ageing ahead of the rows 405.  (Two CTAs an SM where four fit, at other widths:
+// 1,000,000 x 47 for Adam 559 us, with four 538, for Adagrad 513 and 492, 282,624 x 256 for Adagrad 310 and 301.)
+// CTAs that run on an SM at once: 4 by 64 registers a thread, fewer where a lane holds more of a row.
+constexpr int step_apply_ctas(bool adam, int vec, int vpl) {
+  return vec * vpl <= (adam ? 4 : 8) ? 4 : 2;
+}
+
 template <bool ADAM, int VEC, int G, int VPL>
-__global__ void __launch_bounds__(kBlock, VPL > 1 ? 2 : 4) step_apply_kernel(hb_runs_t r, SegArgs a,
-                                                                            UpdateRows<ADAM, true> epi,
-                                                                            const float* sums) {
+__global__ void __launch_bounds__(kBlock, step_apply_ctas(ADAM, VEC, VPL)) step_apply_kernel(hb_runs_t r, SegArgs a,
+                                                                                           UpdateRows<ADAM, true> epi,
+                                                                                           const float* sums) {
   begin_after_previous();
   const int row_blocks = (int)gridDim.x - epi.touch_blocks;
   if ((int)blockIdx.x >= row_blocks) {
@@ -200,7 +206,7 @@ int launch_apply(const hb_runs_t& r, const SegArgs& a, const UpdateRows<ADAM, tr
 #define HB_APPLY(G, VPL)                                                                                              \
   do {                                                                                                                \
     int64_t blocks = ceil_div(r.n, kBlock);                                                                           \
-    const int64_t most = (int64_t)sm_count() * (VPL > 1 ? 2 : 4); /* what runs at once */                              \
+    const int64_t most = (int64_t)sm_count() * step_apply_ctas(ADAM, VEC, VPL); /* what runs at once */                \
     if (blocks > most) blocks = most;                                                                                 \
     HB_LAUNCH_NEXT((step_apply_kernel<ADAM, VEC, G, VPL>), (int)(blocks + epi.touch_blocks), kBlock, 0, st, r, a, epi, sums); \
   } while (0)

@@ -39,3 +39,30 @@ def cuda_lib():
 
 
 GOLDEN = ROOT / "tests" / "golden"
+
+
+@pytest.fixture
+def kernels_of(tmp_path):
+    """kernels_of(call): the kernels that the call launches, as the profiler names them: dicts of name, grid, block,
+    registers per thread, in the order of their start."""
+    import json
+
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    def run(call):
+        call()
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        prof.export_chrome_trace(str(tmp_path / "trace.json"))
+        events = [e for e in json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+                  if e.get("cat") == "kernel" and "grid" in e.get("args", {})]
+        if not events:
+            pytest.skip("the profiler reports no kernels here")
+        return [{"name": e["name"].replace("(anonymous namespace)::", ""), "grid": e["args"]["grid"][0],
+                 "block": e["args"]["block"][0], "registers": e["args"]["registers per thread"]}
+                for e in sorted(events, key=lambda e: e["ts"])]
+
+    return run

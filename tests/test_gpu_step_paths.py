@@ -233,6 +233,21 @@ def test_steps_with_a_second_pass_as_composed(cuda_lib, n, aside, optimizer, mod
         assert torch.equal(sa[k], sb[k]), k
 
 
+@pytest.mark.parametrize("optimizer,dim", [("adam", 47), ("adam", 127), ("adam", 128), ("adam", 256), ("adagrad", 47),
+                                           ("adagrad", 127), ("adagrad", 256), ("adagrad", 320)])
+def test_the_second_pass_has_the_blocks_that_run_at_once(cuda_lib, kernels_of, optimizer, dim):
+    """As many as the registers of its form leave room for, whatever its rows, and one per 256 ids below that."""
+    n = 160_001
+    a, _ = _pair(f"blocks_{optimizer}_{dim}", dim=dim, optimizer=optimizer, touch_lru=False)
+    (ids, g), = _steps(_small("blocks", dim, batch=n), 1)
+    second = [k for k in kernels_of(lambda: a.step(ids, g)) if "step_apply_kernel" in k["name"]]
+    assert len(second) == 1
+    for k in second:
+        warps = 65_536 // (32 * (-(-k["registers"] // 8) * 8))
+        fit = warps // (k["block"] // 32) * torch.cuda.get_device_properties(0).multi_processor_count
+        assert k["grid"] == min(fit, -(-n // 256)), k
+
+
 @pytest.mark.parametrize("optimizer", ["adam", "adagrad"])
 def test_backward_comes_behind_the_callers_stream(cuda_lib, optimizer):
     """What the caller enqueues between a fetch aside and its backward pass is seen by the lookup of the cold ids, which
