@@ -759,7 +759,8 @@ int hb_lookup_fetch(hb_index_t* h, const int64_t* ids, int64_t n, const void* ca
   const int glog2 = group_log2_for(row_bytes / vb);
   // 1,000 rows of 400 bytes: 6.2 us with 32 rows per warp.  Where all warps of 32 rows would run at once, they look up at
   // one time and move rows at one time: 16 rows a warp and two waves (200,000 rows of 512 bytes 31.1 -> 27.5 us).
-  const bool lane = row_bytes <= 512;
+  // The sorted search takes as long for 16 ids as for 32 (200,000 rows of 64 bytes, 16 a warp / 32, 36.3 / 22.1).
+  const bool lane = mode == HB_LOOKUP_SETASSOC && row_bytes <= 512;
   int per = items_per_warp(n);
   if (lane && per == 32 && ceil_div(n, 32) < (int64_t)sm_count() * 48) per = 16;
   const int blocks = grid_of_warps(n, per, kBlock, 16);

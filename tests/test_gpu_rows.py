@@ -243,3 +243,23 @@ def test_lookup_fetch_at_the_lines_of_its_launch(cuda_lib, n, dim):
     want = where[ids]
     assert torch.equal(locs, want) and torch.equal(found.bool(), want >= 0)
     assert torch.equal(out, torch.where((want >= 0)[:, None], rows[want.clamp(min=0)], table[ids]))
+
+
+@pytest.mark.parametrize("mode,dim,n,per,lane", [
+    ("sorted", 16, 200_000, 32, False), ("sorted", 128, 100_000, 32, False), ("sorted", 100, 80_000, 32, False)])
+def test_lookup_fetch_rows_a_warp(cuda_lib, kernels_of, mode, dim, n, per, lane):
+    """The launch that lists between the lines take: rows a warp, and whether a lane probes a line."""
+    from hades_b200 import EmbCacheLib as E
+
+    index = E.IndexCache(4_000, "rows_a_warp", True, False)
+    index.cuda_add(torch.randperm(50_000, device="cuda")[:4_000])
+    if mode == "sorted":
+        index.build_sorted()
+    table, rows = torch.zeros((50_000, dim), device="cuda"), torch.zeros((index.get_capacity(), dim), device="cuda")
+    ids = torch.randint(0, 50_000, (n,), device="cuda")
+    how = E.LOOKUP_SORTED if mode == "sorted" else E.LOOKUP_SETASSOC
+    k, = [k for k in kernels_of(lambda: E.cudaLookupFetch(index, ids, rows, table, mode=how)) if "lookup_fetch" in k["name"]]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert k["grid"] == min(-(-(-(-n // per) * 32) // k["block"]), 16 * sms), k
+    if "lookup_fetch_kernel" in k["name"]:
+        assert k["name"].split("lookup_fetch_kernel<")[1].split(">")[0].split(", ")[3] in (("true", "1") if lane else ("false", "0")), k
