@@ -218,6 +218,11 @@ __device__ __forceinline__ int64_t fetch_lookup(const IndexView& v, const int64_
   else return warp_lookup<MODE>(v, s_top, id);
 }
 
+// CTAs of the set-associative forms that run on an SM at once: 16-byte words 62 registers with a lane a line, else 78,
+// smaller ones 48 and 64.  (Stated as launch bounds, they cost the byte forms spills and the sorted ones a CTA.)
+constexpr int fetch_ctas(int vb, bool lane) { return (vb == 16 ? 3 : 4) + lane; }
+constexpr int kFetch512Ctas = 5;
+
 template <int MODE, int VB, bool FULL, bool LANE>
 __global__ void __launch_bounds__(kBlock) lookup_fetch_kernel(
     IndexView v, const int64_t* __restrict__ ids, int64_t n, const char* __restrict__ cache_rows,
@@ -757,19 +762,33 @@ int hb_lookup_fetch(hb_index_t* h, const int64_t* ids, int64_t n, const void* ca
   }
   const int vb = vec_bytes_for(row_bytes, {cache_rows, backing_rows, out_rows});
   const int glog2 = group_log2_for(row_bytes / vb);
-  // 1,000 rows of 400 bytes: 6.2 us with 32 rows per warp.  Where all warps of 32 rows would run at once, they look up at
-  // one time and move rows at one time: 16 rows a warp and two waves (200,000 rows of 512 bytes 31.1 -> 27.5 us).
+  // 1,000 rows of 400 bytes: 6.2 us with 32 rows per warp.  A lane a line takes fewer registers, so that more warps run
+  // at once; but these look up at one time and move rows at one time, and of few rounds of warps each counts.
+  // (1) 16 rows a warp where twice as many warps all run at once (80,000 rows of 200 bytes 8.6 -> 7.9 us), and for rows of
+  // 512 bytes, which have a kernel of their own, or of words of 4 bytes and less, up to 225,000 (200,000 of 512 bytes 31.1 ->
+  // 27.5), but for the few that would make a second round (110,000 16.2, 16.5 with 16).
+  // (2) Wide rows in words of 8 or 16 bytes: the other form unless it takes more rounds (us, a lane a line / the other:
+  // 100,000 of 400 bytes, a round each, 17.8 / 14.8; 150,000, one and two, 21.3 / 23.8; 200,000, two each, 31.0 / 27.5;
+  // 230,000, two and three, 32.8 / 33.7; 260,000 of 40 bytes 10.1 / 9.2; of 32 bytes 100,000 4.2 / 4.4, 200,000 6.7 / 7.4).
+  // More than 32 words of 8 bytes: but for short lists (504 bytes 10,000 4.2 / 4.6, 40,000 9.0 / 8.7, 800,000 125 / 116).
   // The sorted search takes as long for 16 ids as for 32 (200,000 rows of 64 bytes, 16 a warp / 32, 36.3 / 22.1).
-  const bool lane = mode == HB_LOOKUP_SETASSOC && row_bytes <= 512;
+  const bool row512 = vb == 16 && row_bytes == 512;
   int per = items_per_warp(n);
-  if (lane && per == 32 && ceil_div(n, 32) < (int64_t)sm_count() * 48) per = 16;
+  bool lane = mode == HB_LOOKUP_SETASSOC && row_bytes <= 512 && !(vb == 8 && row_bytes > 256 && per > 8);
+  if (lane && per == 32) {
+    const int64_t sm_warps = (int64_t)sm_count() * (kBlock / 32);
+    const int64_t round = sm_warps * (row512 ? kFetch512Ctas : fetch_ctas(vb, true));
+    if (n <= 16 * round || ((row512 || vb < 8) && n > 19 * round && n <= 38 * round)) per = 16;
+    else if (!row512 && vb >= 8 && row_bytes > (vb == 16 ? 64 : 16))
+      lane = ceil_div(n, 32 * round) < ceil_div(n, 32 * sm_warps * fetch_ctas(vb, false));
+  }
   const int blocks = grid_of_warps(n, per, kBlock, 16);
-  if (vb == 16 && row_bytes == 512) {
+  if (row512) {
     // dim 128 fp32: the specialised kernel (measured 2-4 % faster than the generic mover; deeper prefetch measured no
     // better).  Five CTAs an SM (2,000,000 ids of Zipf 1.05 258 -> 246 us, 400,000 53.8 -> 51.1; three 249, six 244 but
     // 17 for 100,000 instead of 15); the sorted search has no registers for them.
 #define HB_LF512(MODE, FULL)                                                                       \
-  HB_LAUNCH((lookup_fetch512_kernel<MODE, MODE == HB_LOOKUP_SORTED ? 3 : 5, 1, FULL>), blocks, kBlock, 0, st, h->view, ids, n,     \
+  HB_LAUNCH((lookup_fetch512_kernel<MODE, MODE == HB_LOOKUP_SORTED ? 3 : kFetch512Ctas, 1, FULL>), blocks, kBlock, 0, st, h->view, ids, n,     \
             (const char*)cache_rows, (const char*)backing_rows, (char*)out_rows, locs, found, per)
     if (mode == HB_LOOKUP_SORTED) {
       if (per == 32) HB_LF512(HB_LOOKUP_SORTED, true); else HB_LF512(HB_LOOKUP_SORTED, false);

@@ -245,8 +245,42 @@ def test_lookup_fetch_at_the_lines_of_its_launch(cuda_lib, n, dim):
     assert torch.equal(out, torch.where((want >= 0)[:, None], rows[want.clamp(min=0)], table[ids]))
 
 
+@pytest.mark.parametrize("mode", ["set", "sorted"])
+@pytest.mark.parametrize("dim", [2, 10, 16, 33, 50, 100, 126, 128])
+@pytest.mark.parametrize("n", [40_000, 94_720, 94_721, 112_481, 113_665, 151_552, 151_553, 189_441, 224_961, 227_329])
+def test_lookup_fetch_at_the_lines_of_its_forms(cuda_lib, n, dim, mode):
+    """Sizes on both sides of what runs at once, rows in words of 4, 8 and 16 bytes, both lookups."""
+    from hades_b200 import EmbCacheLib as E
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + dim)
+    nodes = 50_000
+    index = E.IndexCache(4_000, "lines_of_the_forms", True, False)
+    held = torch.randperm(nodes, device="cuda", generator=g)[:4_000]
+    slots = index.cuda_add(held)
+    if mode == "sorted":
+        index.build_sorted()
+    where = torch.full((nodes,), -1, dtype=torch.int64, device="cuda")
+    where[held[slots >= 0]] = slots[slots >= 0]
+    table = torch.randn((nodes, dim), device="cuda", generator=g)
+    rows = torch.randn((index.get_capacity(), dim), device="cuda", generator=g)
+    ids = torch.randint(0, nodes, (n,), device="cuda", generator=g)
+    out, locs, found = E.cudaLookupFetch(index, ids, rows, table, mode=E.LOOKUP_SORTED if mode == "sorted" else E.LOOKUP_SETASSOC)
+    want = where[ids]
+    assert torch.equal(locs, want) and torch.equal(found.bool(), want >= 0)
+    assert torch.equal(out, torch.where((want >= 0)[:, None], rows[want.clamp(min=0)], table[ids]))
+
+
 @pytest.mark.parametrize("mode,dim,n,per,lane", [
-    ("sorted", 16, 200_000, 32, False), ("sorted", 128, 100_000, 32, False), ("sorted", 100, 80_000, 32, False)])
+    ("sorted", 16, 200_000, 32, False), ("sorted", 128, 100_000, 32, False), ("sorted", 100, 80_000, 32, False),
+    # one round of warps of 16 rows; rows of 512 bytes and of words of 4 bytes up to 225,000
+    ("set", 50, 80_000, 16, True), ("set", 50, 94_720, 16, True), ("set", 50, 94_721, 32, False), ("set", 128, 94_720, 16, True),
+    ("set", 128, 94_721, 32, True), ("set", 128, 112_481, 16, True), ("set", 33, 224_960, 16, True), ("set", 33, 224_961, 32, True),
+    # rounds of 113,664 and 151,552 ids; 151,552 and 189,440 in words of 8 bytes
+    ("set", 100, 113_664, 32, False), ("set", 100, 113_665, 32, True), ("set", 100, 151_552, 32, True),
+    ("set", 100, 151_553, 32, False), ("set", 100, 227_328, 32, False), ("set", 100, 227_329, 32, True),
+    ("set", 50, 151_553, 32, True), ("set", 50, 189_441, 32, False), ("set", 16, 200_000, 32, True), ("set", 2, 200_000, 32, True),
+    ("set", 10, 200_000, 32, False), ("set", 126, 40_000, 16, False), ("set", 126, 10_000, 4, True)])
 def test_lookup_fetch_rows_a_warp(cuda_lib, kernels_of, mode, dim, n, per, lane):
     """The launch that lists between the lines take: rows a warp, and whether a lane probes a line."""
     from hades_b200 import EmbCacheLib as E
@@ -260,6 +294,8 @@ def test_lookup_fetch_rows_a_warp(cuda_lib, kernels_of, mode, dim, n, per, lane)
     how = E.LOOKUP_SORTED if mode == "sorted" else E.LOOKUP_SETASSOC
     k, = [k for k in kernels_of(lambda: E.cudaLookupFetch(index, ids, rows, table, mode=how)) if "lookup_fetch" in k["name"]]
     sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms != 148:
+        pytest.skip("the lines are those of 148 SMs")
     assert k["grid"] == min(-(-(-(-n // per) * 32) // k["block"]), 16 * sms), k
     if "lookup_fetch_kernel" in k["name"]:
         assert k["name"].split("lookup_fetch_kernel<")[1].split(">")[0].split(", ")[3] in (("true", "1") if lane else ("false", "0")), k
