@@ -181,6 +181,12 @@ __global__ void __launch_bounds__(kBlock, 3) sparse_update_vec_kernel(
   }
 }
 
+int group_log2_for(int64_t units) {
+  int g = 0;
+  while ((1 << g) < units && g < 5) ++g;
+  return g;
+}
+
 // rows per warp and round: 32 unless that leaves the GPU short of warps (a list of 84k rows is
 // only 2.6k rounds of 32)
 int rows_per_warp_for(int64_t n, int glog2) {
@@ -190,9 +196,14 @@ int rows_per_warp_for(int64_t n, int glog2) {
   return rpw;
 }
 
-// 32 bytes a lane (of fp16 rows 16)
-bool rows_of_8(int64_t dim, uintptr_t state_bits, const void* emb, int emb_elem_bytes) {
-  return dim % 8 == 0 && (state_bits & 31) == 0 && ((uintptr_t)emb & (8 * emb_elem_bytes - 1)) == 0;
+// 32 bytes a lane (of fp16 rows 16).  Not for rows of up to 32 columns, of which a pass of a warp takes 8 or more, while
+// all warps of the other form run at once (us, 32 / 16 bytes a lane: 2,000 x 32 Adam 3.82 / 3.30, 8,000 3.85 / 3.59,
+// 15,000 4.35 / 5.67; 30,000 x 8 4.13 / 3.88, 60,000 4.89 / 6.82), nor for the two wide rows in flight of a short list
+// for Adagrad (2,000 x 256 6.13 / 5.90, 4,000 6.41 / 6.46; 1,000 x 512 9.89 / 9.72, 2,000 10.0 / 10.2).
+bool rows_of_8(int64_t n, int64_t dim, bool adam, uintptr_t state_bits, const void* emb, int emb_elem_bytes) {
+  if (dim % 8 != 0 || (state_bits & 31) != 0 || ((uintptr_t)emb & (8 * emb_elem_bytes - 1)) != 0) return false;
+  if (dim <= 32) return n << group_log2_for(dim / 4) > (int64_t)sm_count() * 3 * kBlock;
+  return adam || dim < 256 || n * dim > (int64_t)sm_count() * 4096;
 }
 
 int grid_for_warps(int64_t n, int rpw) {
@@ -246,12 +257,6 @@ __global__ void __launch_bounds__(kBlock) sparse_adagrad_kernel(
   }
 }
 
-int group_log2_for(int64_t units) {
-  int g = 0;
-  while ((1 << g) < units && g < 5) ++g;
-  return g;
-}
-
 int grid_for_groups(int64_t n, int glog2) {
   int64_t blocks = ceil_div(ceil_div(n, kOptRows) << glog2, kBlock);
   const int64_t cap = (int64_t)sm_count() * 16;
@@ -281,7 +286,7 @@ int hb_sparse_adam(const int64_t* ids, const float* grads, const int64_t* cnt, i
   const RowMap map{id_offset, id_stride, rows};
   const uintptr_t bits = (uintptr_t)grads | (uintptr_t)mem | (uintptr_t)power;
   const bool vec4 = dim % 4 == 0 && dim < (1 << 30) && ((bits | (uintptr_t)emb) & 15) == 0;
-  const bool vec8 = vec4 && rows_of_8(dim, bits, emb, emb_elem_bytes);
+  const bool vec8 = vec4 && rows_of_8(n, dim, true, bits, emb, emb_elem_bytes);
   const int glog2 = group_log2_for(vec8 ? dim / 8 : (vec4 ? dim / 4 : dim));
   const int grid = grid_for_groups(n, glog2);
   const int rpw = rows_per_warp_for(n, glog2);
@@ -315,7 +320,7 @@ int hb_sparse_adagrad(const int64_t* ids, const float* grads, const int64_t* cnt
   const uintptr_t bits = (uintptr_t)grads | (uintptr_t)state_sum;
   // fp16 rows are read 8 bytes at a time on the vector path
   const bool vec4 = dim % 4 == 0 && dim < (1 << 30) && ((bits | (uintptr_t)emb) & 15) == 0;
-  const bool vec8 = vec4 && rows_of_8(dim, bits, emb, emb_elem_bytes);
+  const bool vec8 = vec4 && rows_of_8(n, dim, false, bits, emb, emb_elem_bytes);
   const int glog2 = group_log2_for(vec8 ? dim / 8 : (vec4 ? dim / 4 : dim));
   const int grid = grid_for_groups(n, glog2);
   const int rpw = rows_per_warp_for(n, glog2);

@@ -309,3 +309,26 @@ def test_updates_of_8_values_a_lane_have_the_bits_of_4(cuda_lib, emb_dtype, kind
     assert not torch.equal(results[0][0].float(), w0)
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("emb_dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("kind,n,dim", [("adam", 56_833, 8), ("adagrad", 60_001, 8), ("adam", 28_417, 16), ("adagrad", 14_209, 24),
+                                        ("adam", 14_209, 32), ("adam", 33, 40), ("adagrad", 2_369, 256), ("adagrad", 1_149, 528)])
+def test_larger_updates_of_8_values_a_lane_have_the_bits_of_4(cuda_lib, emb_dtype, kind, n, dim):
+    test_updates_of_8_values_a_lane_have_the_bits_of_4(cuda_lib, emb_dtype, kind, n, dim)
+
+
+@pytest.mark.parametrize("kind,n,dim,values", [
+    ("adam", 2_000, 32, 4), ("adagrad", 2_000, 8, 4), ("adam", 56_832, 8, 4), ("adam", 56_833, 8, 8), ("adagrad", 28_416, 16, 4),
+    ("adagrad", 28_417, 16, 8), ("adam", 14_208, 24, 4), ("adam", 14_209, 32, 8), ("adam", 100, 40, 8), ("adagrad", 100, 64, 8),
+    ("adam", 100, 256, 8), ("adagrad", 2_368, 256, 4), ("adagrad", 2_369, 256, 8), ("adagrad", 100, 248, 8), ("adam", 60_000, 100, 4)])
+def test_values_a_lane_of_updates(cuda_lib, kernels_of, kind, n, dim, values):
+    """Narrow rows move 32 bytes a lane where the warps of 16 bytes a lane would not all run at once."""
+    from hades_b200.sparse_optim import ShardedEmbedding, SparseAdagrad, SparseAdam
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines are those of 148 SMs")
+    opt = (SparseAdam if kind == "adam" else SparseAdagrad)(ShardedEmbedding(n, dim), lr=0.01)
+    ids, grads = torch.arange(n, device="cuda"), torch.zeros((n, dim), device="cuda")
+    k, = [k for k in kernels_of(lambda: opt.update(ids, grads, None, is_unique=True)) if "sparse_update" in k["name"]]
+    assert k["name"].split("sparse_update_vec_kernel<")[1].split(">")[0].split(", ")[2] == str(values), k
