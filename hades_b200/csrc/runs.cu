@@ -235,9 +235,10 @@ struct RunsFinish {
       return make_int4((int)(inc & 0xffff), (int)((inc >> 16) & 0xffff), (int)((inc >> 32) & 0xffff), (int)(inc >> 48));
     };
     uint32_t kept = 0u;  // the codes of the first of two strips
-    const int strips = (int)((end - begin + 8 * T - 1) / (8 * T));
-    // (stores ahead of the barrier are what it waits for)
-    const bool late = Ctx::kStoresLate && strips <= 1 && ctx.ctas > 1;
+    // (stores ahead of the barrier are what it waits for; that a kernel has them behind it, and then one strip, is known
+    // when it is compiled: 512 ids with their classes 10.8 -> 10.3 us, 8,192 17.3 -> 16.8)
+    constexpr bool late = Ctx::kStoresLate;
+    const int strips = late ? (int)(end > begin) : (int)((end - begin + 8 * T - 1) / (8 * T));
     int4 mine = make_int4(0, 0, 0, 0), lanes = mine, warps, cta, ahead, all;
 #pragma unroll 1
     for (int q = 0; q < strips; ++q) {
@@ -251,7 +252,7 @@ struct RunsFinish {
     }
     sort_warp_sums<W>(mine, s_sum, warps, cta);
     if (!ctx.prefix(cta, ahead, all)) return give_up(ctx, src);
-    if (late && strips == 1) put_entries(begin + threadIdx.x * 8);
+    if (late) put_entries(begin + threadIdx.x * 8);
 #pragma unroll 1
     for (int q = 0; q < strips; ++q) {
       const uint32_t strip = begin + q * (8 * T);

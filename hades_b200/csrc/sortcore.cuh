@@ -295,6 +295,7 @@ struct ClusterCtx {
   // Stores of a finish behind its barrier, which would wait for them; its entries are kept in registers till then (the
   // grid has none to spare: 1,048,576 ids 62.5 -> 63.2 us, 2,000,000 103.6 -> 105.6).
   static constexpr bool kStoresLate = true;
+  static_assert(ITEMS <= 8, "a chunk is a strip of eight entries a thread");
   SortClusterSmem s;
   int count;   // entries that were sorted
   uint32_t* scratch;  // shared memory, 8 * kThreads words, free after the sort
