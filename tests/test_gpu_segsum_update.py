@@ -77,7 +77,7 @@ def test_update_of_repeated_ids(cuda_lib, kind, dtype, n, dim):
 @pytest.mark.parametrize("n,dim", [(32_768, 64), (32_769, 3), (32_769, 64), (33_001, 8), (33_001, 16), (33_001, 47),
                                    (33_001, 130), (33_001, 256), (33_001, 512), (33_001, 520)])
 def test_adagrad_at_the_edge_of_updating_at_once(cuda_lib, dtype, n, dim):
-    """More than 32,768 ids and rows of one pass: the row is updated when its sum is complete."""
+    """A third of the ids are one id, whose run crosses many CTAs; rows of one pass of the sums, and wider."""
     test_update_of_repeated_ids(cuda_lib, "adagrad", dtype, n, dim)
 
 
@@ -135,6 +135,14 @@ def test_adagrad_in_the_workspace_of_a_larger_batch(cuda_lib, dtype, largest, n,
     before = emb.weight.clone()
     assert _update_in(opt, ids, grads, cnt, 20, least - 1) != 0
     assert torch.equal(emb.weight, before)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("n,dim", [(437_500, 64), (437_501, 64), (218_750, 128), (218_751, 128), (224_001, 125),
+                                   (54_687, 512), (54_688, 512), (110_001, 256), (280_001, 100), (3_500_001, 8), (600_001, 47)])
+def test_adagrad_where_sums_no_longer_fit_in_l2(cuda_lib, dtype, n, dim):
+    """Both sides of 28,000,000 values: up to there through memory, beyond it the row is updated when its sum is complete."""
+    test_update_of_repeated_ids(cuda_lib, "adagrad", dtype, n, dim)
 
 
 @pytest.mark.parametrize("kind", ["adam", "adagrad"])

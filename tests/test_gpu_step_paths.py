@@ -210,7 +210,7 @@ def test_ids_outside_of_the_table_as_composed(cuda_lib, n):
     (150_001, False, "adagrad", 1, 1 << 17, 3), (150_001, True, "adam", 0, 700, 47), (282_624, True, "adam", 1, 1 << 17, 16),
     (303_105, False, "adam", 0, 1 << 17, 128)])
 def test_steps_with_a_second_pass_as_composed(cuda_lib, n, aside, optimizer, mode, miss_cap, dim):
-    """Above 100,000 ids sums, the lookup of the cold ids on the second stream and the update with the ageing in it;
+    """Above 70,000 ids sums, the lookup of the cold ids on the second stream and the update with the ageing in it;
     with and without a fetch aside, through step() and through its two halves, over several flushes, and with
     gradients of another batch than the last one fetched."""
     a, b = _pair(f"second_{n}_{aside}_{optimizer}_{mode}", dim=dim, optimizer=optimizer, lookup_mode=mode)
@@ -233,6 +233,23 @@ def test_steps_with_a_second_pass_as_composed(cuda_lib, n, aside, optimizer, mod
         assert torch.equal(sa[k], sb[k]), k
 
 
+@pytest.mark.parametrize("optimizer", ["adam", "adagrad"])
+@pytest.mark.parametrize("dim", [3, 16, 47, 100, 127, 128, 256, 512])
+def test_steps_at_the_line_of_updates_at_once(cuda_lib, optimizer, dim):
+    """70,000 ids are updated as their sums become complete, one more in a launch of its own: the state is that of the
+    composed step, and the launches say which it was."""
+    launches = []
+    for n in (70_000, 70_001):
+        a, b = _pair(f"line_{n}_{optimizer}_{dim}", dim=dim, optimizer=optimizer)
+        batches = _steps(_small("line", dim, batch=n), 3)
+        _run_pair(a, b, batches)
+        a.forward(batches[0][0], join=False)
+        before = cuda_lib.hb_launch_count()
+        a.backward(*batches[0])
+        launches.append(cuda_lib.hb_launch_count() - before)
+    assert launches[1] == launches[0] + 1
+
+
 @pytest.mark.parametrize("optimizer,dim", [("adam", 47), ("adam", 127), ("adam", 128), ("adam", 256), ("adagrad", 47),
                                            ("adagrad", 127), ("adagrad", 256), ("adagrad", 320)])
 def test_the_second_pass_has_the_blocks_that_run_at_once(cuda_lib, kernels_of, optimizer, dim):
@@ -251,7 +268,7 @@ def test_the_second_pass_has_the_blocks_that_run_at_once(cuda_lib, kernels_of, o
 @pytest.mark.parametrize("optimizer", ["adam", "adagrad"])
 def test_backward_comes_behind_the_callers_stream(cuda_lib, optimizer):
     """What the caller enqueues between a fetch aside and its backward pass is seen by the lookup of the cold ids, which
-    runs on the step's second stream in steps of more than 100,000 ids."""
+    runs on the step's second stream in steps of more than 70,000 ids."""
     n = 100_001
     a, b = _pair("behind_" + optimizer, optimizer=optimizer)
     for p in (a, b):
