@@ -765,8 +765,8 @@ int hb_lookup_fetch(hb_index_t* h, const int64_t* ids, int64_t n, const void* ca
   // 1,000 rows of 400 bytes: 6.2 us with 32 rows per warp.  A lane a line takes fewer registers, so that more warps run
   // at once; but these look up at one time and move rows at one time, and of few rounds of warps each counts.
   // (1) 16 rows a warp where twice as many warps all run at once (80,000 rows of 200 bytes 8.6 -> 7.9 us), and for rows of
-  // 512 bytes, which have a kernel of their own, or of words of 4 bytes and less, up to 225,000 (200,000 of 512 bytes 31.1 ->
-  // 27.5), but for the few that would make a second round (110,000 16.2, 16.5 with 16).
+  // 512 bytes, which have a kernel of their own, or of words of 4 bytes and less, up to 227,000 (200,000 of 512 bytes 31.1 ->
+  // 27.5, 225,000 30.3 -> 27.5), but for the few that would make a second round (110,000 16.2, 16.5 with 16).
   // (2) Wide rows in words of 8 or 16 bytes: the other form unless it takes more rounds (us, a lane a line / the other:
   // 100,000 of 400 bytes, a round each, 17.8 / 14.8; 150,000, one and two, 21.3 / 23.8; 200,000, two each, 31.0 / 27.5;
   // 230,000, two and three, 32.8 / 33.7; 260,000 of 40 bytes 10.1 / 9.2; of 32 bytes 100,000 4.2 / 4.4, 200,000 6.7 / 7.4).
@@ -778,7 +778,7 @@ int hb_lookup_fetch(hb_index_t* h, const int64_t* ids, int64_t n, const void* ca
   if (lane && per == 32) {
     const int64_t sm_warps = (int64_t)sm_count() * (kBlock / 32);
     const int64_t round = sm_warps * (row512 ? kFetch512Ctas : fetch_ctas(vb, true));
-    if (n <= 16 * round || ((row512 || vb < 8) && n > 19 * round && n <= 38 * round)) per = 16;
+    if (n <= 16 * round || ((row512 || vb < 8) && n > 19 * round && n <= 32 * 6 * sm_warps)) per = 16;
     else if (!row512 && vb >= 8 && row_bytes > (vb == 16 ? 64 : 16))
       lane = ceil_div(n, 32 * round) < ceil_div(n, 32 * sm_warps * fetch_ctas(vb, false));
   }

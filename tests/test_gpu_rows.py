@@ -247,7 +247,7 @@ def test_lookup_fetch_at_the_lines_of_its_launch(cuda_lib, n, dim):
 
 @pytest.mark.parametrize("mode", ["set", "sorted"])
 @pytest.mark.parametrize("dim", [2, 10, 16, 33, 50, 100, 126, 128])
-@pytest.mark.parametrize("n", [40_000, 94_720, 94_721, 112_481, 113_665, 151_552, 151_553, 189_441, 224_961, 227_329])
+@pytest.mark.parametrize("n", [40_000, 94_720, 94_721, 112_481, 113_665, 151_552, 151_553, 189_441, 227_328, 227_329])
 def test_lookup_fetch_at_the_lines_of_its_forms(cuda_lib, n, dim, mode):
     """Sizes on both sides of what runs at once, rows in words of 4, 8 and 16 bytes, both lookups."""
     from hades_b200 import EmbCacheLib as E
@@ -273,9 +273,9 @@ def test_lookup_fetch_at_the_lines_of_its_forms(cuda_lib, n, dim, mode):
 
 @pytest.mark.parametrize("mode,dim,n,per,lane", [
     ("sorted", 16, 200_000, 32, False), ("sorted", 128, 100_000, 32, False), ("sorted", 100, 80_000, 32, False),
-    # one round of warps of 16 rows; rows of 512 bytes and of words of 4 bytes up to 225,000
+    # one round of warps of 16 rows; rows of 512 bytes and of words of 4 bytes up to 227,328
     ("set", 50, 80_000, 16, True), ("set", 50, 94_720, 16, True), ("set", 50, 94_721, 32, False), ("set", 128, 94_720, 16, True),
-    ("set", 128, 94_721, 32, True), ("set", 128, 112_481, 16, True), ("set", 33, 224_960, 16, True), ("set", 33, 224_961, 32, True),
+    ("set", 128, 94_721, 32, True), ("set", 128, 112_481, 16, True), ("set", 33, 227_328, 16, True), ("set", 128, 227_329, 32, True),
     # rounds of 113,664 and 151,552 ids; 151,552 and 189,440 in words of 8 bytes
     ("set", 100, 113_664, 32, False), ("set", 100, 113_665, 32, True), ("set", 100, 151_552, 32, True),
     ("set", 100, 151_553, 32, False), ("set", 100, 227_328, 32, False), ("set", 100, 227_329, 32, True),
