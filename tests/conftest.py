@@ -42,27 +42,49 @@ GOLDEN = ROOT / "tests" / "golden"
 
 
 @pytest.fixture
-def kernels_of(tmp_path):
-    """kernels_of(call): the kernels that the call launches, as the profiler names them: dicts of name, grid, block,
-    registers per thread, in the order of their start."""
-    import json
+def kernels_of():
+    """kernels_of(call): the kernels that the call launches, by capturing it: dicts of name (as linked), the numbers among
+    its template arguments, grid, block, registers per thread."""
+    import ctypes as C
+    import re
 
     import torch
-    from torch.profiler import ProfilerActivity, profile
+
+    class Params(C.Structure):  # CUDA_KERNEL_NODE_PARAMS_v2
+        _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("smem", C.c_uint),
+                    ("args", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
 
     def run(call):
+        driver = C.CDLL("libcuda.so.1")
+
+        def check(rc):
+            assert rc == 0, f"CUDA driver error {rc}"
+
         call()
         torch.cuda.synchronize()
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            call()
-            torch.cuda.synchronize()
-        prof.export_chrome_trace(str(tmp_path / "trace.json"))
-        events = [e for e in json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
-                  if e.get("cat") == "kernel" and "grid" in e.get("args", {})]
-        if not events:
-            pytest.skip("the profiler reports no kernels here")
-        return [{"name": e["name"].replace("(anonymous namespace)::", ""), "grid": e["args"]["grid"][0],
-                 "block": e["args"]["block"][0], "registers": e["args"]["registers per thread"]}
-                for e in sorted(events, key=lambda e: e["ts"])]
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            kept = call()  # noqa: F841
+        handle, count = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t()
+        check(driver.cuGraphGetNodes(handle, None, C.byref(count)))
+        nodes = (C.c_void_p * count.value)()
+        check(driver.cuGraphGetNodes(handle, nodes, C.byref(count)))
+        out = []
+        for node in nodes:
+            kind = C.c_int()
+            check(driver.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)))
+            if kind.value != 0:  # CU_GRAPH_NODE_TYPE_KERNEL
+                continue
+            p, func, name, registers = Params(), C.c_void_p(), C.c_char_p(), C.c_int()
+            check(driver.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)))
+            func.value = p.func
+            if not p.func:
+                check(driver.cuKernelGetFunction(C.byref(func), C.c_void_p(p.kern)))
+            check(driver.cuFuncGetName(C.byref(name), func))
+            check(driver.cuFuncGetAttribute(C.byref(registers), 4, func))  # CU_FUNC_ATTRIBUTE_NUM_REGS
+            text = name.value.decode()
+            out.append({"name": text, "arguments": [int(x) for x in re.findall(r"L[ib](\d+)E", text)], "grid": p.grid[0],
+                        "block": p.block[0], "registers": registers.value})
+        return out
 
     return run

@@ -298,4 +298,4 @@ def test_lookup_fetch_rows_a_warp(cuda_lib, kernels_of, mode, dim, n, per, lane)
         pytest.skip("the lines are those of 148 SMs")
     assert k["grid"] == min(-(-(-(-n // per) * 32) // k["block"]), 16 * sms), k
     if "lookup_fetch_kernel" in k["name"]:
-        assert k["name"].split("lookup_fetch_kernel<")[1].split(">")[0].split(", ")[3] in (("true", "1") if lane else ("false", "0")), k
+        assert k["arguments"][3] == lane, k

@@ -331,4 +331,4 @@ def test_values_a_lane_of_updates(cuda_lib, kernels_of, kind, n, dim, values):
     opt = (SparseAdam if kind == "adam" else SparseAdagrad)(ShardedEmbedding(n, dim), lr=0.01)
     ids, grads = torch.arange(n, device="cuda"), torch.zeros((n, dim), device="cuda")
     k, = [k for k in kernels_of(lambda: opt.update(ids, grads, None, is_unique=True)) if "sparse_update" in k["name"]]
-    assert k["name"].split("sparse_update_vec_kernel<")[1].split(">")[0].split(", ")[2] == str(values), k
+    assert k["arguments"][-1] == values, k
