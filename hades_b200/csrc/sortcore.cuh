@@ -67,13 +67,11 @@ constexpr int kSortGroups = 13;
 __host__ __device__ inline int sort_group_ctas(int ctas) { return (ctas + kSortGroups - 1) / kSortGroups; }
 static inline size_t sort_zero_words(int digit) { return kSortBarrierWords + ((size_t)kSortGroups << digit); }
 
-static inline int sort_grid_ctas(int64_t n, bool skips) {
+static inline int sort_grid_ctas(int64_t n) {
   // Fewer CTAs where the chunks would get short: a barrier over few CTAs is quicker, and a CTA takes all registers of its SM,
   // so that what runs on other streams meanwhile needs an SM without one.  Up to 128 CTAs an entry a thread (70,000 ids
   // 32.8 us, with two 33.7), then two.
-  // skips: the long lists of an add, which end in a walk by one thread a set: 2,048 always (80,000 ids with thousands of
-  // copies of some 4.74 -> 4.64 ms, 100,000 5.92 -> 5.74).
-  int64_t g = ceil_div(n, n <= 128 * (int64_t)kGridT && !skips ? kGridT : 2 * kGridT);
+  int64_t g = ceil_div(n, n <= 128 * (int64_t)kGridT ? kGridT : 2 * kGridT);
   const int64_t cap = sm_count();
   return (int)(g > cap ? cap : (g < 1 ? 1 : g));
 }
@@ -883,7 +881,7 @@ int sort_launch_grid(const Src& src, const Fin& fin, int64_t n, int max_digit, v
   if (early) HB_LAUNCH_NEXT(sort_grid_begin_kernel, (words + 1023) / 1024, 1024, 0, st, b.barrier, words);
   else HB_CUDA(cudaMemsetAsync(b.barrier, 0, words * sizeof(unsigned), st));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(sort_grid_ctas(n, Src::kSkips));
+  cfg.gridDim = dim3(sort_grid_ctas(n));
   cfg.blockDim = dim3(kGridT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -917,7 +915,7 @@ int sort_run(const Src& src, const Fin& fin, int64_t n, void* ws, cudaStream_t s
     if (n <= 32 * kClusterT) return sort_launch_cluster<Src, Fin, 2>(src, fin, 16, st);
     if (n <= 64 * kClusterT) return sort_launch_cluster<Src, Fin, 4>(src, fin, 16, st);
     if (n <= kSortClusterMax) return sort_launch_cluster<Src, Fin, 8>(src, fin, 16, st);
-    const int64_t per = ceil_div(n, sort_grid_ctas(n, Src::kSkips));
+    const int64_t per = ceil_div(n, sort_grid_ctas(n));
     if (per <= 2 * kGridT) return sort_launch_grid<Src, Fin, 2>(src, fin, n, kGridDigit, ws, st);
     if (per <= 4 * kGridT) return sort_launch_grid<Src, Fin, 4>(src, fin, n, kGridDigit, ws, st);
     if (per <= 8 * kGridT) return sort_launch_grid<Src, Fin, 8>(src, fin, n, kGridDigit, ws, st);

@@ -443,15 +443,3 @@ def test_host_lookups_with_one_id_beyond_32_bits(cuda_lib, n, at):
     ix.cuda_add(torch.arange(3000).cuda())
     want, _ = ix.cuda_lookup_found(torch.from_numpy(ids).cuda())
     _eq(ix.lookup(torch.from_numpy(ids)).numpy(), want.cpu().numpy(), "slots")
-
-
-@pytest.mark.parametrize("n", [65_537, 100_000, 131_072, 131_073])
-def test_blocks_of_the_sort_of_long_lists(cuda_lib, kernels_of, n):
-    """2,048 entries each, also where other sorts take 1,024."""
-    from hades_b200 import EmbCacheLib as E
-
-    index = E.IndexCache(500_000, f"long_lists_{n}", True, False)
-    ids = torch.randint(0, 1_000_000, (n,), device="cuda")
-    ids[::3] = 7
-    sort, = [k for k in kernels_of(lambda: index.cuda_add(ids)) if "sort_grid_kernel" in k["name"]]
-    assert sort["grid"] == -(-n // 2_048), sort
