@@ -531,8 +531,8 @@ __global__ void __launch_bounds__(kBlock) runs_keys_kernel(hb_runs_t r, int64_t 
 // RB: 512 = rows of exactly 512 bytes (128 fp32: the address arithmetic folds, no lane is idle);
 // 16 = any multiple of 16 bytes; 0 = words or bytes.  PEER: a source may be another GPU's memory
 // (runs that found no room in the stage), so rows are read with plain loads.
-// MAINTAIN: the first blocks of the launch bring the index up to date meanwhile (a chain of dependent
-// reads beside a stream of rows: a second launch of it costs more than it takes).
+// MAINTAIN: blocks that bring the index up to date meanwhile, the first of the launch or spread over it (a chain of
+// dependent reads beside a stream of rows: a second launch of it costs more than it takes).
 // FULL: 32 entries a warp and round, known here: the batches of rows in flight unroll over a fixed range, and
 // rows of 512 bytes take no spills at 64 registers (with a number known at run time 44 to 60 bytes: 2,000,000
 // distinct ids 0.376 -> 0.441 ms).  The other form is for lists that do not fill the GPU.

@@ -89,7 +89,8 @@ struct UpdateRows {
   const int8_t* dclass;       // [U]
   float* staged;              // [slots][dim]
   const int64_t* slots;       // [U] staging slot of a cold run, -1 = none
-  // the first blocks of the launch age the LRU counters by the lookup that found the slots
+  // blocks that age the LRU counters by the lookup that found the slots: the first of the sums' launch, the last of the
+  // second pass's
   int touch_blocks;
   RunsView touched;
   TouchMarks marks;
@@ -397,9 +398,8 @@ __device__ __forceinline__ void apply_runs(const UpdateRows<ADAM, true>& o, cons
 // in the shape of StoreRows (a captured step and an eager one may differ in which they use), and the CTA updates their rows
 // when it has them all.  An update where a run ends holds up the lane groups whose runs go on, and where runs are of
 // very different lengths most warps wait for a few; behind the sums every warp has its share (us a step without flushes,
-// in the walk / behind it: 10,000 x 64 63.1 / 58.9, 50,000 x 32 83.1 / 76.4, 65,536 x 128 111.0 / 107.5, 100,000 x 128
-// 148.2 / 144.6, 100,000 x 256 184 / 179.5; Adagrad, with half the values and half the arithmetic, 65,536 x 128 102.9 /
-// 103.7, 100,000 x 64 114.5 / 115.3.  With all lanes of a warp on one row and 32 warps an SM: 50,000 x 128 of next to no
+// in the walk / behind it: 10,000 x 64 63.1 / 58.9, 50,000 x 32 83.1 / 76.4, 65,536 x 128 111.0 / 107.5;
+// Adagrad, with half the values and half the arithmetic, 65,536 x 128 102.9 / 103.7.  With all lanes of a warp on one row and 32 warps an SM: 50,000 x 128 of next to no
 // duplicates 106.4 / 108.4, now 104.5).
 template <class Epi, int VEC, int G, int VPL> struct SegWalk {
   using Ops = EpiOps<Epi, VEC, G, VPL>;

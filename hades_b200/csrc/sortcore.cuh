@@ -69,8 +69,10 @@ static inline size_t sort_zero_words(int digit) { return kSortBarrierWords + ((s
 
 static inline int sort_grid_ctas(int64_t n) {
   // Fewer CTAs where the chunks would get short: a barrier over few CTAs is quicker, and a CTA takes all registers of its SM,
-  // so that what runs on other streams meanwhile needs an SM without one.  Up to 128 CTAs an entry a thread (70,000 ids
-  // 32.8 us, with two 33.7), then two.
+  // so that what runs on other streams meanwhile needs an SM without one.  Up to 128 CTAs of 1,024 entries, which are two a
+  // thread for half of its warps (70,000 ids 32.8 us, in half the CTAs 33.7), then of 2,048.  (A batch of add() with thousands
+  // of copies of some ids, whose sets a thread walks at the end, is 1 to 4 % behind: 80,000 ids 4.57 -> 4.74 ms; of distinct
+  // ids to few sets ahead: 80,000 to 20,000 places 95.9 -> 68.6 us, 100,000 to 50,000 102.7, with 2,048 for these lists 124.4.)
   int64_t g = ceil_div(n, n <= 128 * (int64_t)kGridT ? kGridT : 2 * kGridT);
   const int64_t cap = sm_count();
   return (int)(g > cap ? cap : (g < 1 ? 1 : g));
@@ -732,7 +734,8 @@ __global__ void __launch_bounds__(kGridT, 1) sort_grid_kernel(Src src, Fin fin, 
     auto load_tile = [&](int t) {
       const uint32_t first = ctx.first(t);
       // (the keys of a pass in a loop of their own, all on their way at once: 2,000,000 ids 111.0 -> 103.6 us, 1,048,576
-      // 64.5 -> 62.5; the ids four at a time 113, 68.6)
+      // 64.5 -> 62.5; the ids four at a time 113, 68.6.  At 64 registers, of ids: 152 bytes stored and 144 loaded with 16
+      // entries a thread, 24 and 16 with 8, 8 and 4 with 4, 16 and 56 with 2.)
       if (dig.wide || (!in && nt > 1)) {
 #pragma unroll
         for (int i = 0; i < I; ++i) {

@@ -34,11 +34,13 @@ constexpr int kCold = 2;
 // Small batches update rows as their sums become complete (one launch); large ones write the sums and
 // update in a second pass over the distinct ids: the sums then run at the speed of the copy, and the
 // update has many rows in flight whatever the lengths of the runs.
-// The line lies where the two cost the same (us a step with flushes, Adam, forward and backward called apart, at once / in
-// a second pass: 50,000 ids of 16 columns 72.4 / 72.0, of 64 80.2 / 81.6, of 128 96.6 / 98.6, of 256 128.8 / 127.4; 75,000: 85.9 /
-// 83.9, 100.8 / 97.8, 123.5 / 122.2, 165.0 / 160.9; 100,000: 96.3 / 93.9, 116.7 / 113.3, 139.0 / 133.2, 203.8 / 188.9; Adagrad 50,000
-// of 128 90.5 / 93.6, 75,000 116.5 / 116.4, 100,000 130.1 / 126.9).  In a captured step, and in one call above the line,
-// the fetch runs beside the sums.
+// The line lies where the two cost the same for 128 columns (us a step with flushes, Adam, forward and backward called apart,
+// at once / in a second pass: 50,000 ids of 16 columns 72.4 / 72.0, of 64 80.2 / 81.6, of 128 96.6 / 98.6, of 256 128.8 / 127.4;
+// 75,000: 85.9 / 83.9, 100.8 / 97.8, 123.5 / 122.2, 165.0 / 160.9; 100,000: 96.3 / 93.9, 116.7 / 113.3, 139.0 / 133.2, 203.8 /
+// 188.9; Adagrad 50,000 of 128 90.5 / 93.6, 75,000 116.5 / 116.4, 100,000 130.1 / 126.9).  By width it would lie lower: 65,000 of
+// 16 76.2 / 74.5, for Adagrad 74.8 / 70.8, of 64 87.1 / 85.8 and 85.6 / 82.6, of 128 104.8 / 106.3 and 99.8 / 100.2, of 256 142.9 /
+// 139.9 and 135.2 / 134.2; 20,000 of 64 63.6 / 65.3, of 256 78.1 / 84.7, of 16 for Adagrad 58.4 / 55.9.
+// In a captured step, and in one call above the line, the fetch runs beside the sums.
 constexpr int64_t kFuseMax = 70000;
 constexpr int64_t kFewRows = 100000;
 bool fuses_update(int64_t n) { return n <= kFuseMax; }
@@ -172,6 +174,11 @@ __global__ void __launch_bounds__(kBlock, step_lookup_blocks(MODE)) step_cold_ke
   }
 }
 
+// CTAs that run on an SM at once: 4 by 64 registers a thread, fewer where a lane holds more of a row.
+constexpr int step_apply_ctas(bool adam, int vec, int vpl) {
+  return vec * vpl <= (adam ? 4 : 8) ? 4 : 2;
+}
+
 // Summed gradients to where they belong: state and table rows of hot ids, staging rows of cold ones; then LRU
 // ageing by the lookup that found the staging rows.  A warp takes 32 distinct ids a round, a lane each for what is worked
 // out once per id, then G lanes per row.  Bound by HBM: rows read and written once.  As many warps as run at once, 32 an
@@ -180,11 +187,6 @@ __global__ void __launch_bounds__(kBlock, step_lookup_blocks(MODE)) step_cold_ke
 // ids of 128 columns for Adam (85,000 hot, 76,000 cold) 411 -> 403 us, of 2,000,000 (88,000, 80,000) 751 -> 748; with 24
 // warps and two rows in flight 427, with the ageing ahead of the rows 405.  (Two CTAs an SM where four fit, at other widths:
 // 1,000,000 x 47 for Adam 559 us, with four 538, for Adagrad 513 and 492, 282,624 x 256 for Adagrad 310 and 301.)
-// CTAs that run on an SM at once: 4 by 64 registers a thread, fewer where a lane holds more of a row.
-constexpr int step_apply_ctas(bool adam, int vec, int vpl) {
-  return vec * vpl <= (adam ? 4 : 8) ? 4 : 2;
-}
-
 template <bool ADAM, int VEC, int G, int VPL>
 __global__ void __launch_bounds__(kBlock, step_apply_ctas(ADAM, VEC, VPL)) step_apply_kernel(hb_runs_t r, SegArgs a,
                                                                                            UpdateRows<ADAM, true> epi,
@@ -410,7 +412,8 @@ int hb_step_forward(hb_step_t* s, const hb_step_desc_t* d, const int64_t* ids, i
   // Few rows: their blocks and those that bring the index up to date run at once, and what counts is the latter's chain
   // of reads: hits and misses to different blocks (2,000 ids 48.4 -> 48.0 us a step, 65,536 113.3 -> 112.6; 282,624 415.8 ->
   // 418.8).  Many: those blocks are spread among the rows', not ahead of them (282,624 415.8 -> 413, 2,000,000 750.4 ->
-  // 745.4; 65,536 113.3 -> 114.2).
+  // 745.4; 65,536 113.3 -> 114.2).  In between (us a step of 128 columns for Adam, apart / spread): 50,000 93.9 / 94.0, 65,000 105.0 /
+  // 105.4, 80,000 123.5 / 122.3, 100,000 132.4 / 131.7, 120,000 145.8 / 145.0, 150,000 163.0 / 159.9; 16 to 256 columns alike.
   const bool few_rows = n <= kFewRows;
   if (lists_used) h->sorted_stale = true;  // (ageing leaves the ids where they are)
   if (d->touch_lru || lists_used) {
